@@ -29,20 +29,20 @@ def listed():
     gpt = dict(kind="gpt", activation="relu", dtype="fp16", dense_mask=True, train=True)
     return [
         # smallest model of the configurations: launches and latency, not bandwidth, decide
-        dict(gpt, name="gpt d256 x2, 256 tokens", layers=2, vocab=10240, heads=4, dim_head=64, dim_ff=1024, batch=2, seq=128),
+        dict(gpt, name="gpt d256 x2 256 tokens", layers=2, vocab=10240, heads=4, dim_head=64, dim_ff=1024, batch=2, seq=128),
         # the benchmark model (half its layers): forward + backward with recomputation
-        dict(gpt, name="gpt d2560 x4, 1024 tokens", layers=4, vocab=10240, heads=32, dim_head=80, dim_ff=8192, batch=2, seq=512),
+        dict(gpt, name="gpt d2560 x4 1024 tokens", layers=4, vocab=10240, heads=32, dim_head=80, dim_ff=8192, batch=2, seq=512),
         # evaluation of the benchmark model on a ragged batch
-        dict(gpt, name="gpt d2560 x4 eval, 3x437", layers=4, vocab=10240, heads=32, dim_head=80, dim_ff=8192, batch=3, seq=437,
+        dict(gpt, name="gpt d2560 x4 eval 3x437", layers=4, vocab=10240, heads=32, dim_head=80, dim_ff=8192, batch=3, seq=437,
              dtype="bf16", train=False),
         # block and vocabulary of the larger GPT configuration: GELU, head dim 128, 2048 tokens a sequence, causal flag
-        dict(gpt, name="gpt d4096 gelu, 2x2048", layers=1, vocab=50304, heads=32, dim_head=128, dim_ff=16384, batch=2, seq=2048,
+        dict(gpt, name="gpt d4096 gelu 2x2048", layers=1, vocab=50304, heads=32, dim_head=128, dim_ff=16384, batch=2, seq=2048,
              activation="gelu", dtype="bf16", dense_mask=False),
         # 13B-shaped decoder layer at its training length
-        dict(kind="llama", name="llama d5120, 1x4096", layers=1, vocab=32000, heads=40, kv_heads=40, dim_head=128, dim_ff=13824,
+        dict(kind="llama", name="llama d5120 1x4096", layers=1, vocab=32000, heads=40, kv_heads=40, dim_head=128, dim_ff=13824,
              batch=1, seq=4096, dtype="bf16", train=True),
         # 70B-shaped decoder layer, grouped-query attention
-        dict(kind="llama", name="llama d8192 gqa, 1x2048", layers=1, vocab=32000, heads=64, kv_heads=8, dim_head=128, dim_ff=28672,
+        dict(kind="llama", name="llama d8192 gqa 1x2048", layers=1, vocab=32000, heads=64, kv_heads=8, dim_head=128, dim_ff=28672,
              batch=1, seq=2048, dtype="bf16", train=True),
         # padded batch of uneven lengths, head dim of the benchmark model
         dict(kind="attention", name="attention 4x1000 h32 d80 lens", batch=4, seq=1000, heads=32, kv_heads=32, dim_head=80,
