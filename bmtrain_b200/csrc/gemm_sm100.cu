@@ -8,7 +8,7 @@
 // * One CTA per SM, static persistent tile loop.  Warp roles:
 //       warp 0      TMA producer  (cp.async.bulk.tensor, 128-byte swizzle, S-stage mbarrier pipeline)
 //       warp 1      MMA issuer    (tcgen05.mma cta_group::1 kind::f16, 128 x BN x 16, one elected thread)
-//       warps 2..5  epilogue      (tcgen05.ld 32x32b -> registers -> alpha/bias/activation -> global)
+//       warps 2..9  epilogue      (tcgen05.ld 32x32b -> shared memory -> alpha/bias/activation -> global)
 //   Two TMEM accumulator buffers let the epilogue of tile i overlap the main loop of tile i+1.
 // * BN (16..256) is picked per problem to minimise wave quantisation on 148 SMs.
 // * Every wait on an mbarrier is bounded (about two seconds of polling); on expiry the kernel records a code in a
@@ -34,9 +34,12 @@ using namespace bmt_tc;
 constexpr int BM = 128;
 constexpr int BK = 64;          // 64 halves = 128 bytes = one swizzle row
 constexpr int UMMA_K = 16;
-constexpr int NUM_THREADS = 192;
+constexpr int NUM_THREADS = 192;                      // GEMM -> reduce-scatter kernel: producer, MMA issuer, 4 epilogue warps
+constexpr int epilogue_warps(int fused) { return fused == 1 ? 4 : 8; }
+constexpr int num_threads(int fused) { return 64 + 32 * epilogue_warps(fused); }
 constexpr int MAX_STAGES = 8;
-constexpr uint32_t SMEM_BUDGET = 222 * 1024;  // tiles; header, alignment slack and the kernels' small static arrays fit below the 227 KiB limit
+constexpr uint32_t SMEM_MAX = 227 * 1024;     // dynamic shared memory a CTA can ask for
+constexpr uint32_t SMEM_FIXED = 3 * 1024;     // header, alignment slack, small static arrays of the fused kernels
 
 __device__ int g_gemm_status = 0;  // 0 = fine; otherwise (code << 16) | blockIdx of the first CTA that gave up
 // Timing of the fused compute+collective kernels since the last read (nanoseconds of %globaltimer):
@@ -51,8 +54,7 @@ struct GemmParams {
     int bn;           // tile N
     int stages;
     uint32_t hdr_off;      // byte offset of the barrier header behind the tile stages (pusher CTAs need room for their ring)
-    uint32_t out_stage_off;  // byte offset of the epilogue's row staging area (128 rows x OUT_PITCH) when rows go out as bulk copies
-    int staged;              // plain GEMM: the epilogue stages rows in shared memory and writes them with bulk copies
+    uint32_t out_stage_off;  // byte offset of the epilogue's buffers: 4 KiB per warp, or 128 rows x OUT_PITCH when rows go out as bulk copies
     int a_mn, b_mn;   // 1 = MN-major operand
     int a_mn5, b_mn5; // the MN-major operand's tensor map has the 64-element chunks as a dimension of their own: one copy per
                       // stage brings all chunks of the tile (instead of one copy per chunk)
@@ -65,6 +67,7 @@ struct GemmParams {
     int bias_dtype;
     int act;
     int accumulate;
+    int epi;          // form of the epilogue: EXTRA of epilogue_rows, or -1: epilogue_rows_any
     float alpha;
     uint32_t idesc;
     const void* residual;  // optional (M x N, operand dtype, row pitch ldr): added after bias / activation
@@ -145,14 +148,13 @@ __device__ __forceinline__ void rs_reduce_all(const void* inbox, int64_t slot_el
 
 // Grouped raster: the CTAs that run at the same time cover a compact (group_m x ~#SM/group_m) patch of output tiles, so
 // every k-slice of A and B that one of them pulls from DRAM is found in L2 by the others.
-__device__ __forceinline__ void tile_coords(const GemmParams& p, int64_t rem, int& m_blk, int& n_blk) {
-    const int64_t per_group = (int64_t)p.group_m * p.n_blocks;
-    const int64_t group = rem / per_group;
-    const int first_m = (int)(group * p.group_m);
+__device__ __forceinline__ void tile_coords(const GemmParams& p, int rem, int& m_blk, int& n_blk) {
+    const int per_group = p.group_m * p.n_blocks;
+    const int group = rem / per_group, in_group = rem - group * per_group;
+    const int first_m = group * p.group_m;
     const int rows = p.m_blocks - first_m < p.group_m ? p.m_blocks - first_m : p.group_m;
-    const int64_t in_group = rem % per_group;
-    m_blk = first_m + (int)(in_group % rows);
-    n_blk = (int)(in_group / rows);
+    n_blk = in_group / rows;
+    m_blk = first_m + in_group - n_blk * rows;
 }
 
 struct SharedHeader {
@@ -168,126 +170,199 @@ __device__ __forceinline__ float gelu_grad_f(float x) {
     const float cdf = 0.5f * (1.f + erff(x * 0.70710678118654752f));
     return cdf + x * 0.3989422804014327f * __expf(-0.5f * x * x);
 }
-template <typename TA> __device__ __forceinline__ void apply_extras(const GemmParams& p, int64_t row, int64_t c, int64_t col_end, float* vv) {
-    if (p.aux_mode) {
-        const TA* ar = (const TA*)p.aux + row * p.ld_aux + c;
+// Eight consecutive elements of a row (the first `n` of them exist) as floats; one 16-byte load when `vec`.
+template <typename T> __device__ __forceinline__ void load_row8(const T* src, int n, bool vec, float (&v)[8]) {
+    if (vec && n >= 8) {
+        load8(src, v);
+    } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (c + i < col_end) {
-                const float a = bmt::Cvt<TA>::to_f(ar[i]);
-                vv[i] = p.aux_mode == 1 ? (a > 0.f ? vv[i] : 0.f) : vv[i] * gelu_grad_f(a);
-            }
+        for (int i = 0; i < 8; ++i) v[i] = i < n ? bmt::Cvt<T>::to_f(src[i]) : 0.f;
     }
-    if (p.residual) {
-        const TA* rr = (const TA*)p.residual + row * p.ldr + c;
+}
+__device__ __forceinline__ void load_row8_dt(const void* src, int dtype, int64_t idx, int n, bool vec, float (&v)[8]) {
+    if (dtype == BMT_DT_F16) load_row8((const __half*)src + idx, n, vec, v);
+    else if (dtype == BMT_DT_BF16) load_row8((const __nv_bfloat16*)src + idx, n, vec, v);
+    else load_row8((const float*)src + idx, n, false, v);
+}
+template <typename T> __device__ __forceinline__ void unpack8(const uint4& q, float (&v)[8]) {
+    bmt::Vec16<T> o;
+    *reinterpret_cast<uint4*>(&o) = q;
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (c + i < col_end) vv[i] += bmt::Cvt<TA>::to_f(rr[i]);
+    for (int i = 0; i < 8; ++i) v[i] = bmt::Cvt<T>::to_f(o.v[i]);
+}
+__device__ __forceinline__ uint4 ld_global_16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
+
+// Epilogue of one warp's 32 rows of a tile: tensor memory -> (alpha, bias, activation, mask, residual, old C) -> global.
+// tcgen05.ld hands every thread one row; written out that way, a store instruction touches 32 rows with 16 bytes each, which
+// cost 5.5 to 8 us per 128 x 256 tile and made every weight gradient of a 1024-token block epilogue-bound (2560 x 8192 x 1024:
+// 52.8 us, of which 16 us without the stores).  So 32 columns at a time go through a 4 KiB exchange buffer of the warp
+// (fp32, 16-byte units XOR-swizzled by the row: no bank conflicts either way) and come back as 8 columns per thread,
+// 4 threads per row: stores and the loads of residual / mask / old C move whole 32-byte sectors.  The next 32 columns are
+// read from tensor memory, and the matching piece of the residual, mask or old C from global memory, while the current
+// ones are worked on; `release` runs as soon as the last column has left tensor memory.  Two warps share 32 rows and take
+// the pieces of 32 columns in turn (`first` = 0 or 1).
+// Two warps per scheduler do this, so it is bound by their own instruction stream: the forms that the layers use are
+// compiled without run-time choices (EXTRA: 0 none, 1 add a 16-bit matrix (residual or old C), 2 / 3 ReLU / GELU gradient
+// mask; bias and ReLU stay run-time, they cost a few instructions), everything else takes epilogue_rows_any.
+constexpr uint32_t EPI_BYTES_PER_WARP = 32 * 128;
+
+__device__ __forceinline__ void epi_put(uint32_t sbuf, int lane, const uint32_t (&r)[32]) {
+    const uint32_t srow = sbuf + (uint32_t)lane * 128;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(srow + (uint32_t)((q ^ (lane & 7)) << 4)), "r"(r[4 * q]),
+                     "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3]) : "memory");
+}
+// columns 8 * (lane & 3) .. + 7 of row `rl` of the exchange buffer
+__device__ __forceinline__ void epi_get(uint32_t sbuf, int lane, int rl, float (&v)[8]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4 * h]), "=f"(v[4 * h + 1]), "=f"(v[4 * h + 2]), "=f"(v[4 * h + 3])
+                     : "r"(sbuf + (uint32_t)(rl * 128 + ((((lane & 3) * 2 + h) ^ (rl & 7)) << 4))) : "memory");
+}
+
+template <typename T, int EXTRA, typename Release>
+__device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, const T* ebase, int64_t e_ld, int64_t row0, int64_t n0,
+                                              int64_t col_end, uint32_t taddr, uint32_t sbuf, int lane, int first, Release release) {
+    const int sub = lane >> 2, cq = (lane & 3) * 8;
+    const int n_cols = (int)(col_end - n0), n_chunks = (n_cols + 31) / 32;
+    const int rows = (int)(p.M - row0 < 32 ? p.M - row0 : 32);     // may be <= 0: nothing is stored then
+    T* dst = cbase + (row0 + sub) * p.ldc + n0 + cq;
+    const T* src = EXTRA ? ebase + (row0 + sub) * e_ld + n0 + cq : nullptr;
+    const T* bias = p.bias ? (const T*)p.bias + n0 + cq : nullptr;
+    const int64_t d_step = 8 * p.ldc, e_step = 8 * e_ld;
+    const float alpha = p.alpha, floor = p.act == 1 ? 0.f : -INFINITY;
+    uint4 nx[4];
+    auto fetch = [&](int c) {
+        const bool col_ok = c * 32 + cq < n_cols;
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+            nx[it] = make_uint4(0u, 0u, 0u, 0u);
+            if (col_ok && it * 8 + sub < rows) nx[it] = ld_global_16(src + it * e_step + c * 32);
+        }
+    };
+    if (first >= n_chunks) { release(); return; }
+    uint32_t r[32];
+    tmem_ld32(taddr + first * 32, r);
+    if (EXTRA) fetch(first);
+    for (int c = first; c < n_chunks; c += 2) {
+        const bool col_ok = c * 32 + cq < n_cols;
+        float b[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (bias && col_ok) load8(bias + c * 32, b);
+        tmem_ld_wait();
+        epi_put(sbuf, lane, r);
+        if (c + 2 < n_chunks) tmem_ld32(taddr + (c + 2) * 32, r);
+        else release();
+        uint4 cur[4];
+        if (EXTRA) {
+#pragma unroll
+            for (int it = 0; it < 4; ++it) cur[it] = nx[it];
+            if (c + 2 < n_chunks) fetch(c + 2);
+        }
+        __syncwarp();
+        float v[4][8];
+#pragma unroll
+        for (int it = 0; it < 4; ++it) epi_get(sbuf, lane, it * 8 + sub, v[it]);
+        __syncwarp();    // the buffer has been read by all lanes
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[it][i] = fmaxf(v[it][i] * alpha + b[i], floor);
+            if (EXTRA) {
+                float e[8];
+                unpack8<T>(cur[it], e);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    v[it][i] = EXTRA == 1 ? v[it][i] + e[i] : EXTRA == 2 ? (e[i] > 0.f ? v[it][i] : 0.f) : v[it][i] * gelu_grad_f(e[i]);
+            }
+            if (col_ok && it * 8 + sub < rows && !(p.debug & 4)) store8(dst + it * d_step + c * 32, v[it]);
+        }
     }
 }
 
-// The arithmetic of epilogue_chunk without the store, for rows whose column count is a multiple of 8: v = final values of
-// the columns [col0, min(col0 + 32, col_end)) of this thread's row (alpha, bias, activation, mask / residual, old C).
-template <typename TC>
-__device__ __forceinline__ void epilogue_math(const GemmParams& p, const TC* crow, int64_t row, int64_t col0, int64_t col_end,
-                                              const uint32_t (&r)[32], float (&v)[32]) {
+// All other forms: fp32 output, odd pitches and widths, unaligned pointers, GELU, several extras at once.
+template <typename TC, typename Release>
+__device__ __forceinline__ void epilogue_rows_any(const GemmParams& p, TC* cbase, int64_t row0, int64_t n0, int64_t col_end, uint32_t taddr,
+                                               uint32_t sbuf, int lane, int first, Release release) {
+    const int sub = lane >> 2, cq = (lane & 3) * 8;
+    const int n_chunks = (int)((col_end - n0 + 31) / 32);
+    const bool c_vec = sizeof(TC) == 2 ? ((p.ldc & 7) == 0 && (((uintptr_t)cbase) & 15) == 0)
+                                       : ((p.ldc & 3) == 0 && (((uintptr_t)cbase) & 15) == 0);
+    const bool b_vec = (((uintptr_t)p.bias) & 15) == 0, r_vec = (p.ldr & 7) == 0 && (((uintptr_t)p.residual) & 15) == 0;
+    const bool a_vec = (p.ld_aux & 7) == 0 && (((uintptr_t)p.aux) & 15) == 0;
+    if (first >= n_chunks) { release(); return; }
+    for (int c = first; c < n_chunks; c += 2) {
+        uint32_t r[32];
+        tmem_ld32(taddr + c * 32, r);
+        tmem_ld_wait();
+        epi_put(sbuf, lane, r);
+        if (c + 2 >= n_chunks) release();
+        __syncwarp();
+        const int64_t col = n0 + c * 32 + cq;
+        const int n_ok = col_end - col >= 8 ? 8 : (int)(col_end - col);       // columns of this thread that exist (may be <= 0)
+        float bias[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (p.bias && n_ok > 0) load_row8_dt(p.bias, p.bias_dtype, col, n_ok, b_vec, bias);
+        for (int it = 0; it < 4; ++it) {
+            const int64_t row = row0 + it * 8 + sub;
+            if (row >= p.M || n_ok <= 0) continue;
+            float v[8], e[8];
+            epi_get(sbuf, lane, it * 8 + sub, v);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        const int64_t c = col0 + g * 8;
-        if (c >= col_end) break;
-        float* vv = v + g * 8;
-        if (p.bias) {
-            float b[8];
-            if (p.bias_dtype == BMT_DT_F16) load8((const __half*)p.bias + c, b);
-            else if (p.bias_dtype == BMT_DT_BF16) load8((const __nv_bfloat16*)p.bias + c, b);
-            else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) b[i] = ((const float*)p.bias)[c + i];
+            for (int i = 0; i < 8; ++i) {
+                v[i] = v[i] * p.alpha + bias[i];
+                if (p.act == 1) v[i] = fmaxf(v[i], 0.f);
+                else if (p.act == 2) v[i] = gelu_f(v[i]);
             }
+            if (p.aux_mode) {
+                load_row8_dt(p.aux, p.bias_dtype, row * p.ld_aux + col, n_ok, a_vec, e);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) vv[i] += b[i];
-        }
-        if (p.act == 1) {
+                for (int i = 0; i < 8; ++i) v[i] = p.aux_mode == 1 ? (e[i] > 0.f ? v[i] : 0.f) : v[i] * gelu_grad_f(e[i]);
+            }
+            if (p.residual) {
+                load_row8_dt(p.residual, p.bias_dtype, row * p.ldr + col, n_ok, r_vec, e);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) vv[i] = fmaxf(vv[i], 0.f);
-        } else if (p.act == 2) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) vv[i] = gelu_f(vv[i]);
-        }
-        if (p.aux_mode || p.residual) {
-            if (p.bias_dtype == BMT_DT_F16) apply_extras<__half>(p, row, c, col_end, vv);
-            else apply_extras<__nv_bfloat16>(p, row, c, col_end, vv);
-        }
-        if (p.accumulate) {
-            float old[8];
-            load8(crow + c, old);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) vv[i] += old[i];
-        }
-    }
-}
-
-template <typename TC>
-__device__ __forceinline__ void epilogue_chunk(const GemmParams& p, TC* crow, int64_t row, int64_t col0, int64_t col_end, const uint32_t (&r)[32], bool row_ok) {
-    // this thread owns one output row and the columns [col0, min(col0 + 32, col_end))
-    if (!row_ok) return;
-    float v[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
-    const bool vec = ((p.ldc & 7) == 0) && ((((uintptr_t)p.c) & 15) == 0) && (((p.c_bs0 | p.c_bs1) & 7) == 0) && sizeof(TC) == 2;
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        const int64_t c = col0 + g * 8;
-        if (c >= col_end) break;
-        float* vv = v + g * 8;
-        const bool full8 = c + 8 <= col_end;
-        if (p.bias) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (c + i < col_end)
-                    vv[i] += p.bias_dtype == BMT_DT_F16 ? __half2float(((const __half*)p.bias)[c + i])
-                           : p.bias_dtype == BMT_DT_BF16 ? __bfloat162float(((const __nv_bfloat16*)p.bias)[c + i])
-                                                         : ((const float*)p.bias)[c + i];
-        }
-        if (p.act == 1) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) vv[i] = fmaxf(vv[i], 0.f);
-        } else if (p.act == 2) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) vv[i] = gelu_f(vv[i]);
-        }
-        if (p.aux_mode || p.residual) {
-            if (p.bias_dtype == BMT_DT_F16) apply_extras<__half>(p, row, c, col_end, vv);
-            else apply_extras<__nv_bfloat16>(p, row, c, col_end, vv);
-        }
-        if (full8 && vec) {
+                for (int i = 0; i < 8; ++i) v[i] += e[i];
+            }
+            TC* dst = cbase + row * p.ldc + col;
             if (p.accumulate) {
-                float old[8];
-                load8(crow + c, old);
+                if constexpr (sizeof(TC) == 2) {
+                    load_row8(dst, n_ok, c_vec, e);
+                } else {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) vv[i] += old[i];
-            }
-            store8(crow + c, vv);
-        } else if (full8 && sizeof(TC) == 4 && ((p.ldc & 3) == 0) && ((((uintptr_t)p.c) & 15) == 0)) {
-            float4* d4 = reinterpret_cast<float4*>(crow + c);
-            if (p.accumulate) {
-                float4 o0 = d4[0], o1 = d4[1];
-                vv[0] += o0.x; vv[1] += o0.y; vv[2] += o0.z; vv[3] += o0.w; vv[4] += o1.x; vv[5] += o1.y; vv[6] += o1.z; vv[7] += o1.w;
-            }
-            d4[0] = make_float4(vv[0], vv[1], vv[2], vv[3]);
-            d4[1] = make_float4(vv[4], vv[5], vv[6], vv[7]);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (c + i < col_end) {
-                    float o = vv[i];
-                    if (p.accumulate) o += bmt::Cvt<TC>::to_f(crow[c + i]);
-                    crow[c + i] = bmt::Cvt<TC>::from_f(o);
+                    for (int i = 0; i < 8; ++i) e[i] = i < n_ok ? dst[i] : 0.f;
                 }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] += e[i];
+            }
+            if (p.debug & 4) continue;
+            if (n_ok == 8 && c_vec) {
+                if constexpr (sizeof(TC) == 2) {
+                    store8(dst, v);
+                } else {
+                    reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+                    reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (i < n_ok) dst[i] = bmt::Cvt<TC>::from_f(v[i]);
+            }
         }
+        __syncwarp();    // the buffer has been read by all lanes
     }
+}
+
+// Picks the form of the epilogue for a 16-bit output tile; `p.epi` is what launch_gemm found for the whole problem.
+template <typename T, typename Release>
+__device__ __forceinline__ void epilogue_tile(const GemmParams& p, T* cbase, int64_t row0, int64_t n0, int64_t col_end, uint32_t taddr,
+                                              uint32_t sbuf, int lane, int first, Release release) {
+    if (p.epi == 0) epilogue_rows<T, 0>(p, cbase, nullptr, 0, row0, n0, col_end, taddr, sbuf, lane, first, release);
+    else if (p.epi == 1)
+        epilogue_rows<T, 1>(p, cbase, p.accumulate ? cbase : (const T*)p.residual, p.accumulate ? p.ldc : p.ldr, row0, n0, col_end, taddr,
+                            sbuf, lane, first, release);
+    else if (p.epi == 2) epilogue_rows<T, 2>(p, cbase, (const T*)p.aux, p.ld_aux, row0, n0, col_end, taddr, sbuf, lane, first, release);
+    else if (p.epi == 3) epilogue_rows<T, 3>(p, cbase, (const T*)p.aux, p.ld_aux, row0, n0, col_end, taddr, sbuf, lane, first, release);
+    else epilogue_rows_any(p, cbase, row0, n0, col_end, taddr, sbuf, lane, first, release);
 }
 
 // ---- two-CTA (cta_group::2) helpers: the pair shares one 256 x BN accumulator tile, each CTA feeds its own
@@ -486,7 +561,7 @@ struct PushPipe {
 };
 
 template <bool CTA2, int FUSED>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(num_threads(FUSED), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const GemmParams p,
                     const FusedComm f) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -500,23 +575,23 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
     const uint32_t stage_bytes = a_bytes + b_bytes;
     SharedHeader* hdr = (SharedHeader*)(smem + p.hdr_off);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int k_blocks = (int)((p.K + BK - 1) / BK);
-    const int64_t tiles_per_batch = (int64_t)p.m_blocks * p.n_blocks;   // m_blocks counts (BM * NCTA)-row tiles
-    const int64_t num_tiles = tiles_per_batch * p.batch_inner * p.batch_outer;
+    const int tiles_per_batch = p.m_blocks * p.n_blocks;   // m_blocks counts (BM * NCTA)-row tiles
+    const int num_tiles = tiles_per_batch * (int)(p.batch_inner * p.batch_outer);
     // The pusher CTAs are the first CTAs of the grid: CTAs are handed to SMs in index order, so when another kernel keeps
     // part of the GPU busy it is compute CTAs that wait for an SM, never the CTAs the other ranks depend on.
     const int comm_first = (FUSED == 2 || FUSED == 3) ? f.ag_ctas : 0;
     const int compute_ctas = (int)gridDim.x - comm_first;
     const bool comm_cta = (int)blockIdx.x < comm_first;
-    const int64_t first_tile = comm_cta ? num_tiles : ((int)blockIdx.x - comm_first) / NCTA, tile_step = compute_ctas / NCTA;
+    const int first_tile = comm_cta ? num_tiles : ((int)blockIdx.x - comm_first) / NCTA, tile_step = compute_ctas / NCTA;
     const int blocks_per_rank = FUSED == 2 ? (int)(f.ag_rows / (BM * NCTA)) : 0;   // in tile rows (256 rows for a CTA pair)
     const int row_blocks_per_rank = FUSED == 2 ? (int)(f.ag_rows / BM) : 1;          // in 128-row blocks (counter granularity)
     const uint32_t tmem_cols = 2 * p.bn <= 32 ? 32 : 2 * p.bn <= 64 ? 64 : 2 * p.bn <= 128 ? 128 : 2 * p.bn <= 256 ? 256 : 512;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(&hdr->full[s], 1); mbar_init(&hdr->empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(&hdr->tmem_full[a], 1); mbar_init(&hdr->tmem_empty[a], 4 * NCTA); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&hdr->tmem_full[a], 1); mbar_init(&hdr->tmem_empty[a], epilogue_warps(FUSED) * NCTA); }
         hdr->failed = 0;
         fence_barrier_init();
     }
@@ -616,15 +691,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
         // the other threads of a pusher CTA have nothing to do
     } else if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (one per CTA)
-        if (lane == 0) {
+        {
             bool ok = true;
             uint64_t waited = 0;        // time spent waiting for data of other ranks (fused modes)
             uint32_t ps = 0, pph = 0;   // ring position and phase, carried across tiles
             const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(&hdr->full[0]), empty0 = smem_u32(&hdr->empty[0]);
             const uint32_t full_leader0 = CTA2 ? map_to_cta(full0, 0) : full0;
-            for (int64_t tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
-                const int64_t batch = tile / tiles_per_batch;
-                const int64_t rem = tile % tiles_per_batch;
+            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
+                const int batch = tile / tiles_per_batch;
+                const int rem = tile - batch * tiles_per_batch;
                 int m_blk, n_blk;
                 tile_coords(p, rem, m_blk, n_blk);
                 if (FUSED == 1 && f.rs_early) m_blk = (m_blk + (f.rank + 1) * f.rs_bpr) % p.m_blocks;   // own rows last
@@ -634,12 +709,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                     const int64_t r0 = (int64_t)n_blk * p.bn;
                     const int64_t r1 = (r0 + p.bn < p.N ? r0 + p.bn : p.N) - 1;
                     const uint64_t tw0 = global_ns();
-                    for (int64_t c = r0 / BM; c <= r1 / BM && ok; ++c) {
-                        const unsigned int target = f.epoch * f.bg_expected[c];
-                        if (!wait_counter(f.bg_cnt[f.rank] + c, target, f.limit_ns)) {
-                            ok = false; atomicCAS(f.status, 0, 0x900 | f.rank); atomicCAS(&g_gemm_status, 0, (10 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1;
+                    if (lane == 0) {
+                        for (int64_t c = r0 / BM; c <= r1 / BM && ok; ++c) {
+                            const unsigned int target = f.epoch * f.bg_expected[c];
+                            if (!wait_counter(f.bg_cnt[f.rank] + c, target, f.limit_ns)) {
+                                ok = false; atomicCAS(f.status, 0, 0x900 | f.rank); atomicCAS(&g_gemm_status, 0, (10 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1;
+                            }
                         }
                     }
+                    ok = __all_sync(0xffffffffu, ok) != 0;   // the other lanes follow lane 0, whose loads acquired the data
                     if (!ok) break;
                     waited += global_ns() - tw0;
                     asm volatile("fence.proxy.async.global;" ::: "memory");
@@ -651,108 +729,119 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                     const int row_block = m_blk * NCTA + (int)rank;
                     const bool mine = f.skip_local && row_block / row_blocks_per_rank == f.rank;   // copied before the launch
                     const uint64_t tw0 = global_ns();
-                    if (!mine && !wait_counter(f.ag_count[f.rank] + row_block, target, f.limit_ns)) {
-                        ok = false; atomicCAS(f.status, 0, 0x400 | f.rank); atomicCAS(&g_gemm_status, 0, (6 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; break;
+                    if (lane == 0 && !mine && !wait_counter(f.ag_count[f.rank] + row_block, target, f.limit_ns)) {
+                        ok = false; atomicCAS(f.status, 0, 0x400 | f.rank); atomicCAS(&g_gemm_status, 0, (6 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1;
                     }
+                    ok = __all_sync(0xffffffffu, ok) != 0;   // the other lanes follow lane 0, whose loads acquired the data
+                    if (!ok) break;
                     waited += global_ns() - tw0;
                     asm volatile("fence.proxy.async.global;" ::: "memory");  // the block was written by a peer's copies, TMA reads it
                 }
-                const int bi = (int)(batch % p.batch_inner), bo = (int)(batch / p.batch_inner);
-                const int bib = (int)(bi / p.b_inner_div);
+                const int bo = batch / (int)p.batch_inner, bi = batch - bo * (int)p.batch_inner;
+                const int bib = bi / (int)p.b_inner_div;
                 const int m0 = m_blk * (BM * NCTA) + (int)rank * BM;            // this CTA's rows of A
                 const int n0 = n_blk * p.bn + (int)(rank * bn_local);           // this CTA's rows of the B tile
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait_u32(empty0 + 8 * ps, pph ^ 1)) { ok = false; atomicCAS(&g_gemm_status, 0, (1 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; break; }
+                    if (!mbar_wait_warp(empty0 + 8 * ps, pph ^ 1)) { ok = false; if (lane == 0) { atomicCAS(&g_gemm_status, 0, (1 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; } break; }
                     const uint32_t sa = smem0 + ps * stage_bytes, sb = sa + a_bytes;
                     const int kx = kb * BK;
-                    if (p.debug & 1) {
-                        if (rank == 0) mbar_arrive_u32(full0 + 8 * ps);
-                    } else if (!CTA2) {
-                        const uint32_t bar = full0 + 8 * ps;
-                        mbar_expect_tx_u32(bar, stage_bytes);
-                        if (!p.a_mn) {
-                            tma_load_4d_u32(&tma_a, bar, sa, kx, m0, bi, bo);
-                        } else if (p.a_mn5) {
-                            tma_load_5d_u32(&tma_a, bar, sa, 0, kx, m0 / 64, bi, bo);
-                        } else {
+                    if (elect_one()) {
+                        if (p.debug & 1) {
+                            if (rank == 0) mbar_arrive_u32(full0 + 8 * ps);
+                        } else if (!CTA2) {
+                            const uint32_t bar = full0 + 8 * ps;
+                            mbar_expect_tx_u32(bar, stage_bytes);
+                            if (!p.a_mn) {
+                                tma_load_4d_u32(&tma_a, bar, sa, kx, m0, bi, bo);
+                            } else if (p.a_mn5) {
+                                tma_load_5d_u32(&tma_a, bar, sa, 0, kx, m0 / 64, bi, bo);
+                            } else {
 #pragma unroll
-                            for (int c = 0; c < BM / 64; ++c) tma_load_4d_u32(&tma_a, bar, sa + c * (64 * BK * 2), m0 + c * 64, kx, bi, bo);
-                        }
-                        if (!p.b_mn) {
-                            tma_load_4d_u32(&tma_b, bar, sb, kx, n0, bib, bo);
-                        } else if (p.b_mn5) {
-                            tma_load_5d_u32(&tma_b, bar, sb, 0, kx, n0 / 64, bib, bo);
+                                for (int c = 0; c < BM / 64; ++c) tma_load_4d_u32(&tma_a, bar, sa + c * (64 * BK * 2), m0 + c * 64, kx, bi, bo);
+                            }
+                            if (!p.b_mn) {
+                                tma_load_4d_u32(&tma_b, bar, sb, kx, n0, bib, bo);
+                            } else if (p.b_mn5) {
+                                tma_load_5d_u32(&tma_b, bar, sb, 0, kx, n0 / 64, bib, bo);
+                            } else {
+                                for (int c = 0; c < (int)bn_local / 64; ++c) tma_load_4d_u32(&tma_b, bar, sb + c * (64 * BK * 2), n0 + c * 64, kx, bib, bo);
+                            }
                         } else {
-                            for (int c = 0; c < (int)bn_local / 64; ++c) tma_load_4d_u32(&tma_b, bar, sb + c * (64 * BK * 2), n0 + c * 64, kx, bib, bo);
-                        }
-                    } else {
-                        // both CTAs report to the leader's barrier; the leader announces the bytes of the pair
-                        const uint32_t bar = full_leader0 + 8 * ps;
-                        if (rank == 0) mbar_expect_tx_u32(full0 + 8 * ps, 2 * stage_bytes);
-                        if (!p.a_mn) {
-                            tma_load_4d_2cta_u32(&tma_a, bar, sa, kx, m0, bi, bo);
-                        } else if (p.a_mn5) {
-                            tma_load_5d_2cta_u32(&tma_a, bar, sa, 0, kx, m0 / 64, bi, bo);
-                        } else {
+                            // both CTAs report to the leader's barrier; the leader announces the bytes of the pair
+                            const uint32_t bar = full_leader0 + 8 * ps;
+                            if (rank == 0) mbar_expect_tx_u32(full0 + 8 * ps, 2 * stage_bytes);
+                            if (!p.a_mn) {
+                                tma_load_4d_2cta_u32(&tma_a, bar, sa, kx, m0, bi, bo);
+                            } else if (p.a_mn5) {
+                                tma_load_5d_2cta_u32(&tma_a, bar, sa, 0, kx, m0 / 64, bi, bo);
+                            } else {
 #pragma unroll
-                            for (int c = 0; c < BM / 64; ++c) tma_load_4d_2cta_u32(&tma_a, bar, sa + c * (64 * BK * 2), m0 + c * 64, kx, bi, bo);
-                        }
-                        if (!p.b_mn) {
-                            tma_load_4d_2cta_u32(&tma_b, bar, sb, kx, n0, bib, bo);
-                        } else if (p.b_mn5) {
-                            tma_load_5d_2cta_u32(&tma_b, bar, sb, 0, kx, n0 / 64, bib, bo);
-                        } else {
-                            for (int c = 0; c < (int)bn_local / 64; ++c) tma_load_4d_2cta_u32(&tma_b, bar, sb + c * (64 * BK * 2), n0 + c * 64, kx, bib, bo);
+                                for (int c = 0; c < BM / 64; ++c) tma_load_4d_2cta_u32(&tma_a, bar, sa + c * (64 * BK * 2), m0 + c * 64, kx, bi, bo);
+                            }
+                            if (!p.b_mn) {
+                                tma_load_4d_2cta_u32(&tma_b, bar, sb, kx, n0, bib, bo);
+                            } else if (p.b_mn5) {
+                                tma_load_5d_2cta_u32(&tma_b, bar, sb, 0, kx, n0 / 64, bib, bo);
+                            } else {
+                                for (int c = 0; c < (int)bn_local / 64; ++c) tma_load_4d_2cta_u32(&tma_b, bar, sb + c * (64 * BK * 2), n0 + c * 64, kx, bib, bo);
+                            }
                         }
                     }
+                    __syncwarp();
                     if (++ps == (uint32_t)p.stages) { ps = 0; pph ^= 1; }
                 }
             }
-            if (FUSED == 2 || FUSED == 3) {
+            if ((FUSED == 2 || FUSED == 3) && lane == 0) {
                 atomicAdd(&g_fused_stats[0], (unsigned long long)waited);
                 atomicMax(&g_fused_stats[3], (unsigned long long)waited);
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (leader CTA only in pair mode)
-        if (lane == 0 && rank == 0) {
+        // The warp stays converged and one elected lane issues: with a single-lane branch around the loop a 64-deep step
+        // cost about 640 clocks of issue time whatever the tile width (the MMAs of a 128-wide tile take 256).
+        if (rank == 0) {
             uint32_t tcount = 0;
             bool ok = true;
             uint32_t cs = 0, cph = 0;
             const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(&hdr->full[0]), empty0 = smem_u32(&hdr->empty[0]);
+            const uint32_t tfull0 = smem_u32(&hdr->tmem_full[0]), tempty0 = smem_u32(&hdr->tmem_empty[0]);
             // descriptor halves that never change; per MMA only the start address moves: K-major steps 32 bytes inside
             // the 128-byte swizzle row, MN-major steps 16 K rows (2 KiB)
-            const uint32_t a_hi = desc_hi(1024), b_hi = desc_hi(1024);
+            const uint32_t d_hi = desc_hi(1024);
             const uint32_t a_lbo = p.a_mn ? 64 * BK * 2 : 0, b_lbo = p.b_mn ? 64 * BK * 2 : 0;
             const uint32_t a_kstep = (p.a_mn ? UMMA_K * 128 : UMMA_K * 2) >> 4, b_kstep = (p.b_mn ? UMMA_K * 128 : UMMA_K * 2) >> 4;
-            for (int64_t tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++tcount) {
+            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++tcount) {
                 const uint32_t acc = tcount & 1;
                 const uint32_t acc_ph = (tcount >> 1) & 1;
-                if (!mbar_wait(&hdr->tmem_empty[acc], acc_ph ^ 1)) { ok = false; atomicCAS(&g_gemm_status, 0, (2 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; break; }
+                if (!mbar_wait_warp(tempty0 + 8 * acc, acc_ph ^ 1)) { ok = false; if (lane == 0) { atomicCAS(&g_gemm_status, 0, (2 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; } break; }
                 tc_fence_after();
                 const uint32_t tmem_c = tmem_base + acc * p.bn;
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait_u32(full0 + 8 * cs, cph)) { ok = false; atomicCAS(&g_gemm_status, 0, (3 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; break; }
+                    if (!mbar_wait_warp(full0 + 8 * cs, cph)) { ok = false; if (lane == 0) { atomicCAS(&g_gemm_status, 0, (3 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; } break; }
                     tc_fence_after();
                     const uint32_t sa = smem0 + cs * stage_bytes;
                     const uint32_t a_lo = desc_lo(sa, a_lbo), b_lo = desc_lo(sa + a_bytes, b_lbo);
-                    if (!(p.debug & 2)) {
+                    if (elect_one()) {
+                        if (!(p.debug & 2)) {
 #pragma unroll
-                        for (int k = 0; k < BK / UMMA_K; ++k) {
-                            const uint64_t ad = pack_desc(a_lo + k * a_kstep, a_hi), bd = pack_desc(b_lo + k * b_kstep, b_hi);
-                            if (CTA2) umma_f16_2cta(tmem_c, ad, bd, p.idesc, (kb | k) != 0 ? 1u : 0u);
-                            else umma_f16(tmem_c, ad, bd, p.idesc, (kb | k) != 0 ? 1u : 0u);
+                            for (int k = 0; k < BK / UMMA_K; ++k) {
+                                const uint64_t ad = pack_desc(a_lo + k * a_kstep, d_hi), bd = pack_desc(b_lo + k * b_kstep, d_hi);
+                                if (CTA2) umma_f16_2cta(tmem_c, ad, bd, p.idesc, (kb | k) != 0 ? 1u : 0u);
+                                else umma_f16(tmem_c, ad, bd, p.idesc, (kb | k) != 0 ? 1u : 0u);
+                            }
                         }
+                        // frees the smem stage (in both CTAs) once these MMAs have read it
+                        if (CTA2) umma_commit_2cta_u32(empty0 + 8 * cs); else umma_commit_u32(empty0 + 8 * cs);
+                        if (kb + 1 == k_blocks) { if (CTA2) umma_commit_2cta_u32(tfull0 + 8 * acc); else umma_commit_u32(tfull0 + 8 * acc); }
                     }
-                    // frees the smem stage (in both CTAs) once these MMAs have read it
-                    if (CTA2) umma_commit_2cta_u32(empty0 + 8 * cs); else umma_commit_u32(empty0 + 8 * cs);
+                    __syncwarp();
                     if (++cs == (uint32_t)p.stages) { cs = 0; cph ^= 1; }
                 }
-                if (ok) { if (CTA2) umma_commit_2cta(&hdr->tmem_full[acc]); else umma_commit(&hdr->tmem_full[acc]); }
             }
         }
     } else {
-        // ------------------------------------------------------------------ epilogue (warps 2..5), own 128 rows
+        // ------------------------------------------------------------------ epilogue (warps 2..9), own 128 rows
         const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter + 32) are visible to this warp
         uint32_t tcount = 0;
         uint32_t rs_free_mask = 0;     // destinations whose inbox is known to be free (mode 1)
@@ -775,9 +864,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             }
             remote_open = false;
         };
-        for (int64_t tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++tcount) {
-            const int64_t batch = tile / tiles_per_batch;
-            const int64_t rem = tile % tiles_per_batch;
+        for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++tcount) {
+            const int batch = tile / tiles_per_batch;
+            const int rem = tile - batch * tiles_per_batch;
             int m_blk, n_blk;
             tile_coords(p, rem, m_blk, n_blk);
             if (FUSED == 1 && f.rs_early) {
@@ -786,7 +875,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             }
             if (FUSED == 2) m_blk = (m_blk + f.rank * blocks_per_rank) % p.m_blocks;
             if (FUSED == 3) n_blk = (n_blk + f.bg_first_block) % p.n_blocks;
-            const int64_t bi = batch % p.batch_inner, bo = batch / p.batch_inner;
+            const int bo = batch / (int)p.batch_inner, bi = batch - bo * (int)p.batch_inner;
             const uint32_t acc = tcount & 1;
             const uint32_t acc_ph = (tcount >> 1) & 1;
             // one lane per warp polls the barrier (128 pollers would compete with the producer / MMA threads for the
@@ -796,28 +885,37 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             got = __shfl_sync(0xffffffffu, got, 0);
             if (!got) { ok = false; if (lane == 0) atomicCAS(&g_gemm_status, 0, (4 << 16) | (blockIdx.x & 0xffff)); break; }
             tc_fence_after();
-            const int64_t row = (int64_t)m_blk * (BM * NCTA) + rank * BM + quarter * 32 + lane;
-            const bool row_ok = row < p.M;
-            int64_t coff = bi * p.c_bs0 + bo * p.c_bs1 + row * p.ldc;
-            char* cbase = (char*)p.c;
-            if (FUSED == 1 && row_ok) {
-                // route the row to the inbox of its owner; wait once per destination until that rank freed the inbox
-                const int owner = (int)(row / f.rs_rows);
-                if (owner != f.rank && !((rs_free_mask >> owner) & 1u)) {
-                    if (!wait_counter(f.flags[f.rank] + f.free_row * f.world + owner, f.epoch, f.limit_ns)) {
-                        atomicCAS(f.status, 0, 0x500 | f.rank); atomicCAS(&g_gemm_status, 0, (7 << 16) | (blockIdx.x & 0xffff));
-                    }
-                    rs_free_mask |= 1u << owner;
-                }
-                cbase = (char*)f.rs_inbox[owner];
-                coff = (row - (int64_t)owner * f.rs_rows) * p.N;
-            }
+            const int64_t row0 = (int64_t)m_blk * (BM * NCTA) + rank * BM + quarter * 32;
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * p.bn;
             const int64_t tile_end = (int64_t)(n_blk + 1) * p.bn;
             const int64_t col_end = tile_end < p.N ? tile_end : p.N;
-            if (FUSED == 1 || p.staged) {
-                // staged bulk-store epilogue: pack OUT_CHUNK columns of the row in shared memory, one bulk copy per row chunk
-                // (to the row's owner in the GEMM -> reduce-scatter kernel)
+            auto release = [&]() {      // this warp has read the accumulator
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (CTA2) mbar_arrive_cluster(map_to_cta(smem_u32(&hdr->tmem_empty[acc]), 0));
+                    else mbar_arrive(&hdr->tmem_empty[acc]);
+                }
+            };
+            if (FUSED == 1) {
+                const int64_t row = row0 + lane;
+                const bool row_ok = row < p.M;
+                char* cbase = (char*)p.c;
+                int64_t coff = 0;
+                if (row_ok) {
+                    // route the row to the inbox of its owner; wait once per destination until that rank freed the inbox
+                    const int owner = (int)(row / f.rs_rows);
+                    if (owner != f.rank && !((rs_free_mask >> owner) & 1u)) {
+                        if (!wait_counter(f.flags[f.rank] + f.free_row * f.world + owner, f.epoch, f.limit_ns)) {
+                            atomicCAS(f.status, 0, 0x500 | f.rank); atomicCAS(&g_gemm_status, 0, (7 << 16) | (blockIdx.x & 0xffff));
+                        }
+                        rs_free_mask |= 1u << owner;
+                    }
+                    cbase = (char*)f.rs_inbox[owner];
+                    coff = (row - (int64_t)owner * f.rs_rows) * p.N;
+                }
+                // bulk-store epilogue: pack OUT_CHUNK columns of the row in shared memory, one bulk copy per row chunk to the
+                // row's owner
                 const uint32_t srow = smem_u32(smem) + p.out_stage_off + (uint32_t)((quarter * 32 + lane) * OUT_PITCH);
                 for (int c0 = 0; c0 < p.bn; c0 += OUT_CHUNK) {
                     const int64_t col0 = (int64_t)n_blk * p.bn + c0;
@@ -829,18 +927,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                         uint32_t r[32];
                         tmem_ld32(taddr + c0 + sub, r);
                         tmem_ld_wait();
-                        float vals[32];
-                        if (FUSED == 1) {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) vals[i] = __uint_as_float(r[i]) * p.alpha;
-                        } else if (row_ok) {
-                            if (p.c_dtype == BMT_DT_F16) epilogue_math<__half>(p, (const __half*)cbase + coff, row, col0 + sub, col_end, r, vals);
-                            else epilogue_math<__nv_bfloat16>(p, (const __nv_bfloat16*)cbase + coff, row, col0 + sub, col_end, r, vals);
-                        }
                         uint32_t pk[16];
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
-                            const float a = vals[2 * i], b = vals[2 * i + 1];
+                            const float a = __uint_as_float(r[2 * i]) * p.alpha, b = __uint_as_float(r[2 * i + 1]) * p.alpha;
                             if (p.c_dtype == BMT_DT_F16) { __half2 h = __floats2half2_rn(a, b); pk[i] = *reinterpret_cast<uint32_t*>(&h); }
                             else { __nv_bfloat162 h = __floats2bfloat162_rn(a, b); pk[i] = *reinterpret_cast<uint32_t*>(&h); }
                         }
@@ -855,27 +945,18 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                                      ::"l"(cbase + (coff + col0) * 2), "r"(srow), "r"(ncols * 2) : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
-            } else
-            for (int c0 = 0; c0 < p.bn; c0 += 32) {
-                const int64_t col0 = (int64_t)n_blk * p.bn + c0;
-                if (col0 >= col_end) break;
-                uint32_t r[32];
-                tmem_ld32(taddr + c0, r);
-                tmem_ld_wait();
-                if (p.debug & 4) continue;
-                if (p.c_dtype == BMT_DT_F16) epilogue_chunk<__half>(p, (__half*)cbase + coff, row, col0, col_end, r, row_ok);
-                else if (p.c_dtype == BMT_DT_BF16) epilogue_chunk<__nv_bfloat16>(p, (__nv_bfloat16*)cbase + coff, row, col0, col_end, r, row_ok);
-                else epilogue_chunk<float>(p, (float*)cbase + coff, row, col0, col_end, r, row_ok);
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                if (CTA2) mbar_arrive_cluster(map_to_cta(smem_u32(&hdr->tmem_empty[acc]), 0));
-                else mbar_arrive(&hdr->tmem_empty[acc]);
+                release();
+            } else {
+                const uint32_t sbuf = smem_u32(smem) + p.out_stage_off + (uint32_t)(warp - 2) * EPI_BYTES_PER_WARP;
+                const int first = (warp - 2) >> 2;   // two warps see the same 32 rows: they take the 32-column pieces in turn
+                const int64_t coff = bi * p.c_bs0 + bo * p.c_bs1, n0 = (int64_t)n_blk * p.bn;
+                if (p.c_dtype == BMT_DT_F16) epilogue_tile(p, (__half*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, release);
+                else if (p.c_dtype == BMT_DT_BF16) epilogue_tile(p, (__nv_bfloat16*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, release);
+                else epilogue_rows_any(p, (float*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, release);
             }
         }
         if (remote_open) report_remote_done();
-        if (FUSED == 1 || p.staged) {
+        if (FUSED == 1) {
             // row copies read this CTA's shared memory and write the inboxes: complete them before the teardown barrier
             asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
             asm volatile("fence.proxy.async.global;" ::: "memory");
@@ -1123,14 +1204,14 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
         int dev = 0;
         BMT_CUDA_OK(cudaGetDevice(&dev));
         BMT_CUDA_OK(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET + 2048));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET + 2048));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET + 2048));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET + 2048));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET + 2048));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET + 2048));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET + 2048));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET + 2048));
+        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
+        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
+        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
+        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
+        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
+        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
+        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
+        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
     }
     static int force_bn = -1, force_cta2 = -2, debug_flags = -1;
     if (debug_flags < 0) { const char* e = getenv("BMT_GEMM_DEBUG"); debug_flags = e ? atoi(e) : 0; }
@@ -1153,18 +1234,8 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     p.bn = tc.bn;
     const int ncta = tc.cta2 ? 2 : 1;
     const uint32_t stage_bytes = BM * BK * 2 + (p.bn / ncta) * BK * 2;
-    // The staged bulk-store epilogue of the GEMM -> reduce-scatter kernel can also serve plain GEMMs with 16-bit output
-    // (BMT_GEMM_STAGED=1; =2: only for K <= 4096).  Off by default: measured on the transformer-block shapes it is slower
-    // than the direct stores (797 vs 734 us over the 15 GEMMs of a block) because it costs a pipeline stage and local
-    // stores do not need the 256-byte packets that peer stores do.
-    static int staged_env = -1;
-    if (staged_env < 0) { const char* e = getenv("BMT_GEMM_STAGED"); staged_env = e ? atoi(e) : 0; }
-    const bool c16 = c_dtype == BMT_DT_F16 || c_dtype == BMT_DT_BF16;
-    const bool can_stage = !fused && c16 && (ldc % 8 == 0) && (((uintptr_t)c & 15) == 0) && ((c_bs0 | c_bs1) % 8 == 0) && (n % 8 == 0) &&
-                           (!bias || ((uintptr_t)bias & 15) == 0);
-    p.staged = (can_stage && (staged_env == 1 || (staged_env == 2 && k <= 4096))) ? 1 : 0;
-    const uint32_t out_stage_bytes = ((fused && fused->mode == 1) || p.staged) ? BM * OUT_PITCH : 0;
-    int stages = (int)((SMEM_BUDGET - 1024 - out_stage_bytes) / stage_bytes);
+    const uint32_t out_stage_bytes = (fused && fused->mode == 1) ? BM * OUT_PITCH : epilogue_warps(0) * EPI_BYTES_PER_WARP;
+    int stages = (int)((SMEM_MAX - SMEM_FIXED - out_stage_bytes) / stage_bytes);
     p.stages = stages > MAX_STAGES ? MAX_STAGES : stages;
     p.m_blocks = (int)((m + BM * ncta - 1) / (BM * ncta));
     p.n_blocks = (int)((n + p.bn - 1) / p.bn);
@@ -1189,6 +1260,14 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     }
     p.residual = g.residual; p.ldr = g.ldr; p.aux = g.aux; p.ld_aux = g.ld_aux; p.aux_mode = g.aux ? g.aux_mode : 0;
     if ((p.residual || p.aux_mode) && batch_inner * batch_outer != 1) return -21;  // fused extras are for plain (unbatched) GEMMs
+    {
+        // the compiled forms of the epilogue move 16-byte vectors of the operand type: every pitch and pointer has to allow it
+        auto vec16 = [](const void* ptr, int64_t ld) { return (ld & 7) == 0 && ((uintptr_t)ptr & 15) == 0; };
+        const int extras = (accumulate ? 1 : 0) + (p.residual ? 1 : 0) + (p.aux_mode ? 1 : 0);
+        const bool ok = c_dtype == ab_dtype && n % 8 == 0 && vec16(c, ldc) && ((c_bs0 | c_bs1) & 7) == 0 && act != 2 && extras <= 1 &&
+                        vec16(bias, 0) && vec16(p.residual, p.residual ? p.ldr : 0) && vec16(p.aux, p.aux_mode ? p.ld_aux : 0);
+        p.epi = !ok ? -1 : (accumulate || p.residual) ? 1 : p.aux_mode == 1 ? 2 : p.aux_mode == 2 ? 3 : 0;
+    }
     const uint32_t fmt = ab_dtype == BMT_DT_F16 ? 0u : 1u;
     p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(a_major ? 1 : 0) << 15) | ((uint32_t)(b_major ? 1 : 0) << 16) |
               ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)((BM * ncta) >> 4) << 24);
@@ -1214,6 +1293,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     if (rc) return rc;
 
     const int64_t tiles = (int64_t)p.m_blocks * p.n_blocks * batch_inner * batch_outer;
+    if (tiles > 0x3fffffff) return -23;   // the kernel counts tiles in 32 bits (2^30 tiles are 3e13 elements of C)
     p.out_stage_off = (uint32_t)p.stages * stage_bytes;
     p.hdr_off = p.out_stage_off + out_stage_bytes;
     if (comm_ctas > 0 && p.hdr_off < PUSH_STAGES * PUSH_PIECE_BYTES) p.hdr_off = PUSH_STAGES * PUSH_PIECE_BYTES;
@@ -1232,15 +1312,15 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
         }
         if (!tc.cta2) {
             if (fc.mode == 1) gemm_tcgen05_kernel<false, 1><<<grid, NUM_THREADS, smem, stream>>>(ma, mb, p, fc);
-            else if (fc.mode == 2) gemm_tcgen05_kernel<false, 2><<<grid, NUM_THREADS, smem, stream>>>(ma, mb, p, fc);
-            else gemm_tcgen05_kernel<false, 3><<<grid, NUM_THREADS, smem, stream>>>(ma, mb, p, fc);
+            else if (fc.mode == 2) gemm_tcgen05_kernel<false, 2><<<grid, num_threads(2), smem, stream>>>(ma, mb, p, fc);
+            else gemm_tcgen05_kernel<false, 3><<<grid, num_threads(3), smem, stream>>>(ma, mb, p, fc);
             bmt_count_launch(1);
             return (int)cudaGetLastError();
         }
         cudaLaunchConfig_t cfg;
         memset(&cfg, 0, sizeof(cfg));
         cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(NUM_THREADS);
+        cfg.blockDim = dim3(num_threads(fc.mode));
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
         cudaLaunchAttribute attr[1];
@@ -1256,7 +1336,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     }
     if (!tc.cta2) {
         const unsigned grid = (unsigned)(tiles < g_num_sms ? tiles : g_num_sms);
-        gemm_tcgen05_kernel<false, 0><<<grid, NUM_THREADS, smem, stream>>>(ma, mb, p, none);
+        gemm_tcgen05_kernel<false, 0><<<grid, num_threads(0), smem, stream>>>(ma, mb, p, none);
         bmt_count_launch(1);
         return (int)cudaGetLastError();
     }
@@ -1264,7 +1344,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
-    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.blockDim = dim3(num_threads(0));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];

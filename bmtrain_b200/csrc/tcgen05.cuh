@@ -58,6 +58,22 @@ __device__ __forceinline__ bool mbar_wait_u32(uint32_t addr, uint32_t parity) {
         }
     }
 }
+// True in exactly one lane of a converged warp, always the same one.  Tensor-core and copy instructions take their operands
+// from uniform registers: a warp that stays together and elects the issuing lane lets the compiler keep descriptors and
+// addresses there, where a branch on the lane index makes it move them over for every instruction.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t pred;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(pred));
+    return pred != 0;
+}
+// Wait of a whole warp; the (bounded) result is the same in all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t addr, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait_u32(addr, parity)) != 0;
+}
 __device__ __forceinline__ void mbar_expect_tx_u32(uint32_t addr, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(addr), "r"(bytes) : "memory");
 }
