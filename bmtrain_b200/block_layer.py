@@ -134,13 +134,28 @@ def _get_param_kw(param: DistributedParameter) -> str:
 
 
 class _Slot:
-    """Where one inner parameter lives inside its bucket."""
+    """Where one inner parameter lives inside its bucket.
 
-    __slots__ = ("name", "param", "offset", "numel", "shape", "lo", "hi")
+    During the backward pass of the block it is also the place a kernel may write the parameter's gradient to
+    (``ops/grad_slot.py``): ``written`` tells whether the slot of the full gradient buffer holds a gradient yet."""
+
+    __slots__ = ("name", "param", "offset", "numel", "shape", "lo", "hi", "bucket", "written")
 
     def __init__(self, name, param, offset, numel, shape):
         self.name, self.param, self.offset, self.numel, self.shape = name, param, offset, numel, shape
         self.lo = self.hi = 0  # overlap with the local partition, in bucket coordinates
+        self.bucket = None
+        self.written = False
+
+    @property
+    def open(self) -> bool:
+        return self.bucket.grads_open and self.bucket.full_grad is not None
+
+    def grad_ptr(self) -> int:
+        return self.bucket.full_grad_ptr + self.offset * self.bucket.full_grad.element_size()
+
+    def grad_view(self) -> torch.Tensor:
+        return self.bucket.full_grad[self.offset:self.offset + self.numel].view(self.shape)
 
 
 class _Bucket:
@@ -153,8 +168,60 @@ class _Bucket:
         self.part = 0
         self.storage: Optional[torch.nn.Parameter] = None
         self.full: Optional[torch.Tensor] = None
+        self.aliased = False        # `full` is the partition itself
         self.full_grad: Optional[torch.Tensor] = None
+        self.full_grad_ptr = 0
+        self.grads_open = False     # the block's autograd backward is running: kernels may write into the slots
         self.work = None
+        self._views_of = None       # the storage memory `_local_views` / `_full_views` look at
+        self._layout = None
+
+    def layout(self):
+        """Sizes that cut the flat buffer into the slots and the alignment gaps between them, and the positions of the
+        gaps and of the slots: ``split_with_sizes`` makes all views of a buffer in one call."""
+        if self._layout is None:
+            sizes, gaps, where, at = [], [], [], 0
+            for s in self.slots + [None]:
+                start = self.total if s is None else s.offset
+                if start > at:
+                    gaps.append(len(sizes))
+                    sizes.append(start - at)
+                if s is not None:
+                    where.append(len(sizes))
+                    sizes.append(s.numel)
+                    at = s.offset + s.numel
+            self._layout = (sizes, gaps, where)
+        return self._layout
+
+    def _refresh_views(self) -> None:
+        data = self.storage.data
+        key = (data.data_ptr(), data.dtype, data.numel())
+        if self._views_of != key:
+            # the views keep the memory they look at alive, so an equal address is the same memory
+            self._local_views = [data[s.lo - self.begin:s.hi - self.begin] for s in self.slots]
+            self._full_views = None
+            if self.comm.size == 1:
+                sizes, _, where = self.layout()
+                parts = data.split_with_sizes(sizes)
+                self._full_views = [parts[i].view(s.shape) for i, s in zip(where, self.slots)]
+            self._views_of = key
+
+    def local_views(self):
+        """Local part of every slot (flat); views of the partition."""
+        self._refresh_views()
+        return self._local_views
+
+    def own_full_views(self):
+        """One rank: the partition is the whole bucket, seen as the parameters."""
+        self._refresh_views()
+        return self._full_views
+
+    def in_place(self) -> bool:
+        """Whether the block may compute on the partition itself instead of a gathered copy of it: one rank in the group
+        and no optimizer that uploads new values on its own stream (it would not wait for kernels that read them)."""
+        if self.comm.size != 1 or getattr(self.storage, "_bmt_grad_hook", None) is not None:
+            return False
+        return all(getattr(s.param, "_bmt_grad_hook", None) is None for s in self.slots)
 
     @property
     def begin(self) -> int:
@@ -261,7 +328,11 @@ class _BlockFunction(torch.autograd.Function):
                 outs.append(o)
                 grads.append(g)
         if outs:
-            torch.autograd.backward(outs, grads)
+            block._open_grads(True)
+            try:
+                torch.autograd.backward(outs, grads)
+            finally:
+                block._open_grads(False)
         block._exit_backward()
         ctx.detached = ctx.graph_out = ctx.inputs = None
         return (None, None, None) + tuple(d.grad if r else None for d, r in zip(detached, ctx.req))
@@ -364,6 +435,8 @@ class Block(torch.nn.Module):
             offset = round_up(b.total, align)
             numel = param._original_shape.numel()
             slot = _Slot(name, param, offset, numel, param._original_shape)
+            slot.bucket = b
+            param._bmt_grad_slot = slot
             b.slots.append(slot)
             b.total = offset + numel
         dev = config["device"]
@@ -428,8 +501,11 @@ class Block(torch.nn.Module):
                 continue
             if b.full is not None and b.work is not None:
                 b.work.wait()  # a stale prefetch: let it finish before its buffer is dropped
-            b.full = torch.empty(b.total, dtype=b.dtype, device=b.storage.device)
             b.full_epoch = _param_epoch[0]
+            if b.in_place():
+                b.full, b.work, b.aliased = b.storage.data, None, True
+                continue
+            b.full, b.aliased = torch.empty(b.total, dtype=b.dtype, device=b.storage.device), False
             b.work = b.comm.all_gather_into(b.full, b.storage.data, async_op=True)
 
     def _try_deferred_gather(self, args, backward: bool = False) -> bool:
@@ -502,7 +578,7 @@ class Block(torch.nn.Module):
                 state["ev_rest"] = ev
             return state["ev_rest"]
 
-        b.full = buf.tensor(b.dtype, b.total)
+        b.full, b.aliased = buf.tensor(b.dtype, b.total), False
         b.full_epoch = _param_epoch[0]
         b.full_sym = (rt, free_row, epoch)
         mod._bmt_deferred_gather = dict(rt=rt, buf=buf, bucket=b, slot=slot, epoch=epoch, key=key, free_row=free_row,
@@ -522,14 +598,20 @@ class Block(torch.nn.Module):
                 b.work.wait()
                 b.work = None
         for b in self._buckets.values():
-            for s in b.slots:
-                s.param.data = b.full[s.offset:s.offset + s.numel].view(s.shape)
+            if b.aliased:
+                for s, view in zip(b.slots, b.own_full_views()):
+                    s.param.data = view
+                continue
+            sizes, _, where = b.layout()
+            parts = b.full.split_with_sizes(sizes)
+            for s, i in zip(b.slots, where):
+                s.param.data = parts[i].view(s.shape)
         self._resident = True
 
     def _point_to_local(self) -> None:
         for b in self._buckets.values():
-            for s in b.slots:
-                s.param.data = b.storage.data[s.lo - b.begin:s.hi - b.begin]
+            for s, view in zip(b.slots, b.local_views()):
+                s.param.data = view
 
     def _release_params(self) -> None:
         self._point_to_local()
@@ -560,15 +642,22 @@ class Block(torch.nn.Module):
         # across all micro-batches, so each block needs a slot of its own.
         return ("grad", self._slot_parity, b.key, b.total, id(self) if self._mode == "PIPE" else 0)
 
-    def _prepare_grads(self) -> None:
-        """Full-size zeroed gradient buffers; inner ``.grad`` fields become views into them."""
+    def _prepare_grads(self, attach: bool = True) -> None:
+        """Full-size gradient buffers.
+
+        ``attach`` true: zeroed, and inner ``.grad`` fields become views into them.  False (the block's own backward pass):
+        left as they are apart from the gaps between the slots -- a kernel writes a gradient straight into its slot
+        (``ops/grad_slot.py``) or autograd leaves it in ``.grad``, and ``_scatter_grads`` fills in the rest, so that a
+        gradient is neither added to zeros nor written twice."""
         for b in self._buckets.values():
             needs = [s for s in b.slots if s.param.requires_grad]
-            for s in b.slots:
-                s.param.grad = None
+            fresh = b.full_grad is None
+            if fresh or attach:
+                for s in b.slots:
+                    s.param.grad = None
             if not needs:
                 continue
-            if b.full_grad is None:
+            if fresh:
                 rt = self._peer_runtime(b)
                 if rt is not None:
                     # staging buffer in peer-visible memory; peers must have finished reading its previous contents
@@ -577,17 +666,63 @@ class Block(torch.nn.Module):
                     done_row = rt.row(key + ("done",))
                     if rt.epochs.get(done_row, 0) > 0:
                         rt.signal_wait(done_row, rt.epochs[done_row], signal=False, wait=True)
-                    b.full_grad = buf.tensor(b.dtype, b.total).zero_()
+                    b.full_grad = buf.tensor(b.dtype, b.total)
                     b.full_grad_buf = buf
                 else:
-                    b.full_grad = torch.zeros(b.total, dtype=b.dtype, device=b.storage.device)
+                    b.full_grad = torch.empty(b.total, dtype=b.dtype, device=b.storage.device)
                     b.full_grad_buf = None
-            for s in needs:
-                s.param.grad = b.full_grad[s.offset:s.offset + s.numel].view(s.shape)
+                b.full_grad_ptr = b.full_grad.data_ptr()
+                if attach:
+                    b.full_grad.zero_()
+                else:
+                    sizes, gaps, _ = b.layout()
+                    if gaps:
+                        parts = b.full_grad.split_with_sizes(sizes)
+                        torch._foreach_zero_([parts[i] for i in gaps])
+                for s in b.slots:
+                    s.written = attach
+            if attach:
+                for s in needs:
+                    s.param.grad = s.grad_view()
+
+    def _open_grads(self, is_open: bool) -> None:
+        for b in self._buckets.values():
+            b.grads_open = is_open
+
+    @staticmethod
+    def _complete_grads(b: _Bucket) -> None:
+        """Bring every slot of the full gradient buffer up to date: what autograd left in ``.grad`` goes in, slots that
+        got no gradient are zero."""
+        parts, missing = None, []
+        sizes, _, where = b.layout()
+        for s, i in zip(b.slots, where):
+            g = s.param.grad
+            if g is None and s.written:
+                continue
+            if parts is None:
+                parts = b.full_grad.split_with_sizes(sizes)
+            flat = parts[i]
+            if g is None:
+                missing.append(flat)
+            elif g.is_sparse:
+                if not s.written:
+                    flat.zero_()
+                flat.view(s.shape).add_(g)
+            elif g.data_ptr() == flat.data_ptr() and g.numel() == flat.numel():
+                pass                                     # a view of the slot: nothing to move
+            elif s.written:
+                flat.view(s.shape).add_(g)
+            else:
+                flat.view(s.shape).copy_(g)
+            s.param.grad = None
+        if missing:
+            torch._foreach_zero_(missing)
 
     def _scatter_grads(self) -> None:
         """Reduce-scatter the full gradient buffers onto the partitions (asynchronously)."""
         for b in self._buckets.values():
+            if b.full_grad is not None:
+                self._complete_grads(b)
             for s in b.slots:
                 s.param.grad = None
         self._point_to_local()
@@ -630,15 +765,25 @@ class Block(torch.nn.Module):
                     ev.record(rt.stream)
                 work = StreamWork(ev)
                 fused = True
+            elif b.comm.size == 1:
+                piece, work, fused = full_grad, DONE, False      # the sum over one rank is the buffer itself
             else:
                 piece = torch.empty(b.part, dtype=b.dtype, device=full_grad.device)
                 work = b.comm.reduce_scatter_into(piece, full_grad, "sum", async_op=True)
                 fused = False
             if not accumulate:
                 b.storage.grad = piece
-            for s in b.slots:
-                if s.param.requires_grad:
-                    s.param.grad = b.storage.grad[s.lo - b.begin:s.hi - b.begin]
+            held = b.storage.grad
+            if b.comm.size == 1:
+                sizes, _, where = b.layout()
+                parts = held.split_with_sizes(sizes)
+                for s, i in zip(b.slots, where):
+                    if s.param.requires_grad:
+                        s.param.grad = parts[i]
+            else:
+                for s in b.slots:
+                    if s.param.requires_grad:
+                        s.param.grad = held[s.lo - b.begin:s.hi - b.begin]
 
             def finish(work=work, b=b, piece=piece, full_grad=full_grad, accumulate=accumulate, fused=fused):
                 work.wait()
@@ -675,7 +820,7 @@ class Block(torch.nn.Module):
 
     def _enter_backward(self, args=None) -> None:
         self._ensure_gathered(args, backward=True)
-        self._prepare_grads()
+        self._prepare_grads(attach=False)
         pre = self.pre_module()
         if pre is not None and pre._mode != "PIPE" and pre._zero_level == 3:
             pre._begin_gather(prefetch=True)

@@ -59,7 +59,7 @@ def ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
 
 
 def stream_handle() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def check(status: int, what: str) -> None:

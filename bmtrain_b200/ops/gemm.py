@@ -21,6 +21,7 @@ from typing import Optional
 import torch
 
 from . import _native
+from . import grad_slot as _grad_slot
 
 ACT_NONE, ACT_RELU, ACT_GELU = 0, 1, 2
 _ACT = {None: ACT_NONE, "none": ACT_NONE, "relu": ACT_RELU, "gelu": ACT_GELU}
@@ -181,7 +182,12 @@ class LinearFunction(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             grad_x = gemm_nn(g2, weight).view(x.shape)
         if ctx.needs_input_grad[1]:
-            grad_w = gemm_tn(g2, x2)
+            slot = _grad_slot.find(weight) if weight.is_cuda and weight.dtype == g2.dtype else None
+            if slot is None:
+                grad_w = gemm_tn(g2, x2)
+            else:
+                gemm_tn(g2, x2, out=slot.grad_view(), accumulate=slot.written)
+                slot.written = True
         if ctx.has_bias and ctx.needs_input_grad[2]:
             grad_b = bias_grad(g2)
         return grad_x, grad_w, grad_b

@@ -14,6 +14,7 @@ import torch
 
 from . import _native
 from . import gemm as _gemm
+from . import grad_slot as _grad_slot
 
 _c_void_p, _i64, _int, _f32 = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_float
 
@@ -48,6 +49,7 @@ class _Grad(ctypes.Structure):
 
 _PARAM_NAMES = ("ln1_w", "ln1_b", "qkv_w", "qkv_b", "out_w", "out_b", "ln2_w", "ln2_b", "fc1_w", "fc1_b", "fc2_w", "fc2_b")
 _WEIGHTS = ("qkv_w", "out_w", "fc1_w", "fc2_w")
+_SMALL = tuple(n for n in _PARAM_NAMES if n not in _WEIGHTS)
 
 
 def _as_bytes(mask: torch.Tensor) -> torch.Tensor:
@@ -149,22 +151,28 @@ class GPTBlockFunction(torch.autograd.Function):
         g = _Grad()
         dx = torch.empty_like(x)
         g.dy, g.dx = dy.data_ptr(), dx.data_ptr()
-        # gradients of the parameters: accumulate in place when the owner already attached same-dtype gradient buffers (no
-        # tensor goes back to autograd for them, so no add kernel per parameter either)
+        # gradients of the parameters go straight into the owning block's gradient buffer, or accumulate in place when the
+        # owner attached same-dtype gradient buffers (no tensor goes back to autograd for them then)
         def attached(p):
             return p.is_leaf and p.requires_grad and p.grad is not None and p.grad.dtype == dt and p.grad.is_contiguous()
 
-        acc_w = all(attached(p) for name, p in zip(_PARAM_NAMES, params) if name in _WEIGHTS)
-        acc_small = all(attached(p) for name, p in zip(_PARAM_NAMES, params) if name not in _WEIGHTS)
         grads = {}
-        for name, p in zip(_PARAM_NAMES, params):
-            if acc_w if name in _WEIGHTS else acc_small:
-                setattr(g, "d_" + name, p.grad.data_ptr())
-            else:
-                grads[name] = torch.empty_like(p)
-                setattr(g, "d_" + name, grads[name].data_ptr())
-        g.acc_w = 1 if acc_w else 0
-        g.acc_small = 1 if acc_small else 0
+        for names, flag in ((_WEIGHTS, "acc_w"), (_SMALL, "acc_small")):
+            mine = [(name, p) for name, p in zip(_PARAM_NAMES, params) if name in names]
+            slots = [_grad_slot.find(p) if p.dtype == dt else None for _, p in mine]
+            if all(s is not None for s in slots) and len({s.written for s in slots}) == 1:
+                # the owning ZeRO block's gradient buffer: written on first use, added to afterwards
+                setattr(g, flag, 1 if slots[0].written else 0)
+                for (name, _), slot in zip(mine, slots):
+                    setattr(g, "d_" + name, slot.grad_ptr())
+                    slot.written = True
+                continue
+            acc = all(attached(p) for _, p in mine)
+            setattr(g, flag, 1 if acc else 0)
+            for name, p in mine:
+                if not acc:
+                    grads[name] = torch.empty_like(p)
+                setattr(g, "d_" + name, (p.grad if acc else grads[name]).data_ptr())
         scratch = _gemm.colsum_scratch(dev)
         g.colsum_scratch, g.colsum_scratch_bytes = scratch.data_ptr(), scratch.numel() * 4
         nblk = min(T, 296)

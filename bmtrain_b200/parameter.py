@@ -92,7 +92,8 @@ class DistributedParameter(torch.nn.Parameter):
         """Full value over the ZeRO group (a new tensor; use :meth:`gather_all` to also undo TP)."""
         if self._in_block:
             raise RuntimeError("parameters inside a Block are gathered by the Block")
-        return OpAllGather.apply(self).detach()
+        full = OpAllGather.apply(self).detach()
+        return full.clone() if self._zero_comm.size == 1 else full
 
     def gather_all(self) -> torch.Tensor:
         """Full value with the tensor-parallel split undone as well."""
@@ -139,6 +140,10 @@ class OpAllGather(torch.autograd.Function):
         hook = getattr(value, "_bmt_pending_update", None)
         if hook is not None:
             hook(True)   # an asynchronous optimizer step is still rewriting this shard
+        if ctx.comm.size == 1 and getattr(value, "_bmt_grad_hook", None) is None:
+            # one rank: the shard is the whole value.  (An optimizer that uploads new values on a stream of its own does
+            # not wait for kernels that read them: those parameters are still copied.)
+            return value.detach().as_subclass(torch.Tensor).view(value._original_shape)
         full = gather_flat_shard(value.data, ctx.numel, ctx.comm)
         return full.view(value._original_shape)
 
@@ -147,6 +152,8 @@ class OpAllGather(torch.autograd.Function):
         comm: Communicator = ctx.comm
         per = (ctx.numel + comm.size - 1) // comm.size
         flat = grad_output.reshape(-1)
+        if comm.size == 1:
+            return flat
         if flat.numel() != per * comm.size:
             padded = torch.zeros(per * comm.size, dtype=flat.dtype, device=flat.device)
             padded[: flat.numel()].copy_(flat)
