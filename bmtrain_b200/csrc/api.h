@@ -128,6 +128,7 @@ typedef struct {
     void* pre;       // (T, d_ff) pre-activation, GELU only (NULL for ReLU)
     // fused attention (csrc/attn_sm100.cu): non-NULL lse selects it; probs is then unused and may be NULL
     void* lse;       // (batch, heads, seq) fp32
+    void* mask_packed;  // with lse and a mask: buffer for the packed mask (bmt_attn_mask_layout bytes), filled by forward
 } BmtGptBlock;
 
 typedef struct {
@@ -257,19 +258,23 @@ int bmt_rope_qkv(int64_t batch, int64_t seq, int hk, int g, int d, void* packed,
 // Fused attention forward (csrc/attn_sm100.cu): o = softmax(scale * q k^T + masks) v, lse = log-sum-exp per row.
 // q (b, sq, h, d), k / v (b, sk, hk, d), o (b, sq, h, d); *_strides = element strides {token, head, batch}, head dim
 // contiguous; d a multiple of 16 up to 128; strides multiples of 8; pointers 16-byte aligned.  lse (b, h, sq) fp32 or
-// NULL; mask (b, sq, sk) bytes (non-zero = attend) or NULL; kv_lens (b) int32 or NULL.
+// NULL; mask_bits / mask_cls: parts of a dense mask packed by bmt_attn_mask_pack, or NULL; kv_lens (b) int32 or NULL.
 int bmt_flash_attn_fwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const void* q, const int64_t* q_strides,
                        const void* k, const int64_t* k_strides, const void* v, const int64_t* v_strides, void* o,
-                       const int64_t* o_strides, void* lse, float scale, int causal, const void* mask, const void* kv_lens,
-                       int dtype, void* stream);
+                       const int64_t* o_strides, void* lse, float scale, int causal, const void* mask_bits,
+                       const void* mask_cls, const void* kv_lens, int dtype, void* stream);
 // Backward of bmt_flash_attn_fwd: o / lse from the forward, dout = gradient of o; dq, dk, dv receive the gradients (strided
 // like q, k, v).  Scratch from the caller: dq_acc = batch * sq * h * d floats, delta = batch * h * sq floats.
 int bmt_flash_attn_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const void* q, const int64_t* q_strides,
                        const void* k, const int64_t* k_strides, const void* v, const int64_t* v_strides, const void* o,
                        const int64_t* o_strides, const void* dout, const int64_t* do_strides, const void* lse, void* dq,
                        const int64_t* dq_strides, void* dk, const int64_t* dk_strides, void* dv, const int64_t* dv_strides,
-                       void* dq_acc, void* delta, float scale, int causal, const void* mask, const void* kv_lens, int dtype,
-                       void* stream);
+                       void* dq_acc, void* delta, float scale, int causal, const void* mask_bits_t, const void* mask_cls,
+                       const void* kv_lens, int dtype, void* stream);
+// A dense mask (batch, sq, sk) of bytes (non-zero = attend) as bits: by query (bits, at offset 0), by key (bits_t) and a
+// class per 128 x 128 tile (cls).  The layout call returns the bytes needed and the offsets of the last two parts.
+int64_t bmt_attn_mask_layout(int64_t batch, int64_t sq, int64_t sk, int64_t* bits_t_off, int64_t* cls_off);
+int bmt_attn_mask_pack(int64_t batch, int64_t sq, int64_t sk, const void* mask, void* packed, void* stream);
 // 0, or (wait code << 16 | CTA) of the first attention CTA whose bounded wait ran out; reading clears it
 int bmt_attn_status(void);
 

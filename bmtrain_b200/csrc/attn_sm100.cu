@@ -1,15 +1,6 @@
 // Fused attention for sm_100a (B200): softmax(scale * Q K^T + mask) V without the score matrix ever leaving the SM.
 //
-// Forward, one CTA per (128 query rows, head, sample):
-//   warp 0      TMA producer: Q once, then the K and V tiles of 128 keys through two-stage rings
-//   warp 1      MMA issuer (one thread): S_j = Q K_j^T into tensor memory (two S buffers), O += P_j V_j into one fp32
-//               accumulator in tensor memory; S_{j+1} is issued before P_j V_j so that the tensor core works while the
-//               softmax warps are busy with S_j
-//   warps 2..5  softmax: one thread per query row reads its whole row of S_j from tensor memory in one round trip
-//               (tcgen05.ld), applies the masks, keeps the sum and a reference maximum, writes P_j = exp2(..) as
-//               fp16/bf16 into shared memory in the 128-byte-swizzled K-major layout the MMA reads.  The reference
-//               maximum follows the true one lazily; only when it moves is the accumulator rescaled (tcgen05.ld / st).
-//               The epilogue normalises and stores the row and its log-sum-exp.
+// Forward, backward and the packing of dense masks; the kernels' comments say how each is organised and what bounds it.
 // Masks: causal (key j visible to query i iff j <= i + sk - sq), per-sample key counts, dense boolean (b, sq, sk).
 // Grouped-query attention: kv head = head / (h / hk).  Head dims up to 128 (multiples of 16); tiles are padded with
 // zeros by TMA.  Every mbarrier wait is bounded; on expiry a status word is set and the CTA winds down.
@@ -29,7 +20,7 @@ namespace {
 
 using namespace bmt_tc;
 
-constexpr int ATT_THREADS = 192;
+constexpr int FWD_THREADS = 320;                 // producer, MMA issuer, two groups of four softmax warps
 constexpr int TILE = 128;                        // query rows per CTA and keys per step
 constexpr uint32_t CHUNK = TILE * 64 * 2;        // one [128 rows][64 columns] swizzled chunk of 16-bit elements: 16 KiB
 
@@ -41,17 +32,20 @@ struct AttnParams {
     float sl2;                  // scale * log2(e)
     int causal;
     int64_t causal_off;         // sk - sq
-    const uint8_t* mask;        // (b, sq, sk) or null; non-zero = attend
+    const uint32_t* bits;       // packed mask (b, sq, key tiles, 4 words) or null; a set bit = attend
+    const uint8_t* cls;         // its summary (b, query tiles, key tiles): 0 nothing visible, 1 mixed, 2 everything visible
     const int32_t* kv_lens;     // (b) or null
     void* o;                    // (b, sq, h, d) by strides
     int64_t o_tok, o_head, o_batch;
     float* lse;                 // (b, h, sq), natural log; -inf for rows without a visible key
     uint32_t idesc_s, idesc_pv;
+    int q_tiles, k_tiles;       // 128-row tiles of the queries / keys
+    int per_cta;                // query tiles per CTA: 2, or 1 when there are too few to fill the GPU with pairs
 };
 
 struct AttnShared {
     uint64_t q_full, k_full[2], v_full[2], k_empty[2], v_empty[2];
-    uint64_t s_full[2], s_free[2], p_ready, p_free, o_full;
+    uint64_t s_full[2], p_ready[2], o_full[2];
     uint32_t tmem_base;
     int failed;
 };
@@ -60,6 +54,31 @@ __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+// Two fp32 multiply-adds / adds in one instruction.
+__device__ __forceinline__ uint64_t pack_f2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack_f2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// A from tensor memory: lane = row, every column holds two consecutive 16-bit elements of the reduction dimension.
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_c, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_c), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
 
 __device__ __forceinline__ void fail(AttnShared* sh, int code) {
@@ -71,32 +90,13 @@ __device__ __forceinline__ void fail(AttnShared* sh, int code) {
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int lane) {
     int got = 1;
     if (lane == 0) got = mbar_wait(bar, parity) ? 1 : 0;
-    return __shfl_sync(0xffffffffu, got, 0) != 0;
+    got = __shfl_sync(0xffffffffu, got, 0);
+    __syncwarp();
+    return got != 0;
 }
 
-// Which of the 32 keys [col0, col0 + 32) one query row may attend to, as a bit mask: keys below `limit` (the smaller of
-// the valid key count and the causal boundary + 1), and, with a dense mask row, keys whose mask byte is non-zero.
-__device__ __forceinline__ uint32_t visible_bits(int64_t col0, int64_t limit, const uint8_t* mrow) {
-    const int64_t n = limit - col0;
-    uint32_t bits = n >= 32 ? 0xffffffffu : n <= 0 ? 0u : ((1u << (int)n) - 1u);
-    if (mrow != nullptr && bits != 0u) {
-        const uint8_t* m = mrow + col0;
-        uint32_t mb = 0u;
-        if ((((uintptr_t)m) & 15) == 0 && n >= 32) {
-            const uint4 a = *reinterpret_cast<const uint4*>(m), b = *reinterpret_cast<const uint4*>(m + 16);
-            const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint32_t nz = __vcmpne4(w[i], 0u);     // 0xff per non-zero byte
-                mb |= ((nz & 1u) | ((nz >> 7) & 2u) | ((nz >> 14) & 4u) | ((nz >> 21) & 8u)) << (4 * i);
-            }
-        } else {
-            for (int i = 0; i < 32 && i < n; ++i) mb |= (m[i] != 0 ? 1u : 0u) << i;
-        }
-        bits &= mb;
-    }
-    return bits;
-}
+// The lowest `n` of 32 bits (n may be outside [0, 32]).
+__device__ __forceinline__ uint32_t low_bits(int64_t n) { return n >= 32 ? 0xffffffffu : n <= 0 ? 0u : ((1u << (int)n) - 1u); }
 
 template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
@@ -108,36 +108,113 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
+// Packs a dense mask (b, sq, sk) of bytes into bits, once per call instead of once per head: one block per 128 x 128 tile.
+//   bits   (b, sq, key tiles, 4 words): the 128 keys of a tile as seen by one query (forward)
+//   bits_t (b, sk, query tiles, 4 words): the 128 queries of a tile as seen by one key (backward)
+//   cls    (b, query tiles, key tiles): 0 nothing visible, 1 mixed, 2 everything visible -- tiles of class 0 are skipped
+// Read per head and row, the bytes of a 437-key mask (rows not 16-byte aligned) took 3/4 of the attention kernel's time.
+constexpr int MASK_THREADS = 256;
+__global__ void __launch_bounds__(MASK_THREADS)
+attn_mask_pack_kernel(const uint8_t* mask, int64_t sq, int64_t sk, uint32_t* bits, uint32_t* bits_t, uint8_t* cls) {
+    __shared__ uint32_t w[TILE][4];
+    __shared__ int any, full;
+    const int kt = blockIdx.x, qt = blockIdx.y, b = blockIdx.z, n_kt = gridDim.x, n_qt = gridDim.y;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t q0 = (int64_t)qt * TILE, k0 = (int64_t)kt * TILE;
+    if (threadIdx.x == 0) { any = 0; full = 1; }
+    __syncthreads();
+    for (int r = warp; r < TILE; r += MASK_THREADS / 32) {
+        const int64_t q = q0 + r;
+        uint32_t word[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int64_t k = k0 + c * 32 + lane;
+            const bool on = q < sq && k < sk && mask[((int64_t)b * sq + q) * sk + k] != 0;
+            word[c] = __ballot_sync(0xffffffffu, on);
+        }
+        if (lane == 0) {
+            uint32_t seen = 0;
+            bool all = true;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                w[r][c] = word[c];
+                seen |= word[c];
+                all = all && word[c] == low_bits(sk - (k0 + c * 32));
+            }
+            if (q < sq) {
+                if (seen) any = 1;
+                if (!all) full = 0;
+                *reinterpret_cast<uint4*>(bits + ((((int64_t)b * sq + q) * n_kt) + kt) * 4) = make_uint4(word[0], word[1], word[2], word[3]);
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) cls[((int64_t)b * n_qt + qt) * n_kt + kt] = (uint8_t)(!any ? 0 : full ? 2 : 1);
+    // the 32 x 32 bit blocks transposed: lane = query, one ballot per key
+    for (int blk = warp; blk < 16; blk += MASK_THREADS / 32) {
+        const int qw = blk >> 2, kw = blk & 3;
+        const uint32_t mine = w[qw * 32 + lane][kw];
+        uint32_t out = 0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const uint32_t t = __ballot_sync(0xffffffffu, (mine >> i) & 1u);
+            if (lane == i) out = t;
+        }
+        const int64_t k = k0 + kw * 32 + lane;
+        if (k < sk) bits_t[((((int64_t)b * sk + k) * n_qt) + qt) * 4 + qw] = out;
+    }
+}
+
+// Forward.  A CTA works on two tiles of 128 query rows (one when the grid would not fill the GPU) with a group of four
+// softmax warps each, so that the tensor core multiplies for one tile while the other one is in its softmax:
+//   warp 0      TMA producer: both Q tiles once, then K and V tiles of 128 keys through two-stage rings (shared by both)
+//   warp 1      MMA issuer: S_t = Q_t K^T into tensor memory, O_t += P_t V with P_t read from tensor memory
+//   warps 2..5 / 6..9   softmax of tile 0 / 1: one thread per query row reads its row of S from tensor memory, applies the
+//               masks, and writes the probabilities back over it as packed 16-bit pairs, where the MMA takes them from.
+// What bounds it: a 128 x 128 tile at head dim 128 is 1024 clocks of MMA and 1024 clocks of ex2 (16 per clock and SM); with
+// one tile per CTA, and P going through shared memory, the two and everything in between took turns (about 4500 clocks).
+// The commit behind S_t(j) also covers P V of the tile before (the tensor pipe works in issue order), so a softmax group that
+// has seen S_t(j) may rescale O_t without another wait.
 template <int HD, typename T>
-__global__ void __launch_bounds__(ATT_THREADS, 1)
+__global__ void __launch_bounds__(FWD_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                  const AttnParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     constexpr int DC = HD / 64;                     // 64-column chunks of the (padded) head dim
     constexpr uint32_t TB = DC * CHUNK;             // bytes of one Q / K / V tile
-    const uint32_t sQ = smem_u32(smem), sK = sQ + TB, sV = sK + 2 * TB, sP = sV + 2 * TB;
-    AttnShared* sh = (AttnShared*)(smem + 5 * TB + 2 * CHUNK);
+    const uint32_t sQ = smem_u32(smem), sK = sQ + 2 * TB, sV = sK + 2 * TB;
+    AttnShared* sh = (AttnShared*)(smem + 6 * TB);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;       // under a causal mask the long rows start first
-    const int head = blockIdx.y, b = blockIdx.z, kvh = head / (p.h / p.hk);
-    const int64_t q0 = (int64_t)qt * TILE;
-    int64_t kv_end = p.sk;
-    if (p.causal && q0 + TILE + p.causal_off < kv_end) kv_end = q0 + TILE + p.causal_off;
-    if (p.kv_lens && p.kv_lens[b] < kv_end) kv_end = p.kv_lens[b];
-    if (kv_end < 0) kv_end = 0;
-    const int J = (int)((kv_end + TILE - 1) / TILE);           // key tiles this CTA visits
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int head = blockIdx.x % p.h, b = blockIdx.x / p.h, kvh = head / (p.h / p.hk);
+    const int qt0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * p.per_cta;   // under a causal mask the long rows start first
+    int64_t kv_lim = p.sk;
+    if (p.kv_lens && p.kv_lens[b] < kv_lim) kv_lim = p.kv_lens[b];
+    if (kv_lim < 0) kv_lim = 0;
+    int J[2];                                       // key tiles that query tile t can see
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int64_t q_end = (int64_t)(qt0 + t + 1) * TILE;
+        int64_t end = kv_lim;
+        if (p.causal && q_end + p.causal_off < end) end = q_end + p.causal_off;
+        if (end < 0 || t >= p.per_cta || qt0 + t >= p.q_tiles) end = 0;
+        J[t] = (int)((end + TILE - 1) / TILE);
+    }
+    const int J_max = J[0] > J[1] ? J[0] : J[1];
+    const uint8_t* cls0 = p.cls ? p.cls + ((int64_t)b * p.q_tiles + qt0) * p.k_tiles : nullptr;
+    auto active = [&](int t, int j) -> bool { return j < J[t] && (!cls0 || cls0[t * p.k_tiles + j] != 0); };
+    auto next_step = [&](int j) -> int {
+        do ++j; while (j < J_max && !active(0, j) && !active(1, j));
+        return j;
+    };
 
     if (threadIdx.x == 0) {
         mbar_init(&sh->q_full, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&sh->k_full[i], 1); mbar_init(&sh->v_full[i], 1); mbar_init(&sh->k_empty[i], 1); mbar_init(&sh->v_empty[i], 1);
-            mbar_init(&sh->s_full[i], 1); mbar_init(&sh->s_free[i], 4);
+            mbar_init(&sh->s_full[i], 1); mbar_init(&sh->p_ready[i], 4); mbar_init(&sh->o_full[i], 1);
         }
-        mbar_init(&sh->p_ready, 4);
-        mbar_init(&sh->p_free, 1);
-        mbar_init(&sh->o_full, 1);
         sh->failed = 0;
         fence_barrier_init();
     }
@@ -145,128 +222,169 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = sh->tmem_base;
-    const uint32_t tmem_o = tmem + 256;             // S buffers: columns [0,128) and [128,256); the O accumulator behind them
+    const uint32_t tmem = sh->tmem_base;            // S_0 / P_0 [0,128), S_1 / P_1 [128,256), O_0 [256,384), O_1 [384,512)
+    const int first = next_step(-1);
 
     if (warp == 0) {
         // ------------------------------------------------------------------------------------------ TMA producer
-        if (lane == 0 && J > 0) {
+        if (first < J_max) {
             const uint32_t qbar = smem_u32(&sh->q_full);
-            mbar_expect_tx_u32(qbar, TB);
+            if (elect_one()) {
+                mbar_expect_tx_u32(qbar, (J[0] > 0 ? TB : 0) + (J[1] > 0 ? TB : 0));
 #pragma unroll
-            for (int c = 0; c < DC; ++c) tma_load_4d_u32(&tq, qbar, sQ + c * CHUNK, c * 64, (int)q0, head, b);
-            for (int j = 0; j < J; ++j) {
-                const int st = j & 1;
-                const uint32_t ph = (uint32_t)((j >> 1) & 1);
-                if (!mbar_wait(&sh->k_empty[st], ph ^ 1)) { fail(sh, 1); break; }
-                const uint32_t kbar = smem_u32(&sh->k_full[st]);
-                mbar_expect_tx_u32(kbar, TB);
+                for (int t = 0; t < 2; ++t)
+                    if (J[t] > 0) {
 #pragma unroll
-                for (int c = 0; c < DC; ++c) tma_load_4d_u32(&tk, kbar, sK + st * TB + c * CHUNK, c * 64, j * TILE, kvh, b);
-                if (!mbar_wait(&sh->v_empty[st], ph ^ 1)) { fail(sh, 2); break; }
-                const uint32_t vbar = smem_u32(&sh->v_full[st]);
-                mbar_expect_tx_u32(vbar, TB);
+                        for (int c = 0; c < DC; ++c) tma_load_4d_u32(&tq, qbar, sQ + t * TB + c * CHUNK, c * 64, (qt0 + t) * TILE, head, b);
+                    }
+            }
+            __syncwarp();
+            int n = 0;
+            for (int j = first; j < J_max; j = next_step(j), ++n) {
+                const int st = n & 1;
+                const uint32_t ph = (uint32_t)((n >> 1) & 1);
+                if (!mbar_wait_warp(smem_u32(&sh->k_empty[st]), ph ^ 1)) { if (lane == 0) fail(sh, 1); break; }
+                const uint32_t kbar = smem_u32(&sh->k_full[st]), vbar = smem_u32(&sh->v_full[st]);
+                if (elect_one()) {
+                    mbar_expect_tx_u32(kbar, TB);
 #pragma unroll
-                for (int c = 0; c < DC; ++c) tma_load_4d_u32(&tv, vbar, sV + st * TB + c * CHUNK, c * 64, j * TILE, kvh, b);
+                    for (int c = 0; c < DC; ++c) tma_load_4d_u32(&tk, kbar, sK + st * TB + c * CHUNK, c * 64, j * TILE, kvh, b);
+                }
+                __syncwarp();
+                if (!mbar_wait_warp(smem_u32(&sh->v_empty[st]), ph ^ 1)) { if (lane == 0) fail(sh, 2); break; }
+                if (elect_one()) {
+                    mbar_expect_tx_u32(vbar, TB);
+#pragma unroll
+                    for (int c = 0; c < DC; ++c) tma_load_4d_u32(&tv, vbar, sV + st * TB + c * CHUNK, c * 64, j * TILE, kvh, b);
+                }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------------------------------ MMA issuer
-        if (lane == 0 && J > 0) {
+        // the warp stays converged and one elected lane issues (operands in uniform registers)
+        if (first < J_max) {
             const uint32_t hi = desc_hi(1024);
-            const int ks_s = (p.d + 15) / 16;            // 16-deep steps of the Q K^T contraction
-            bool ok = mbar_wait(&sh->q_full, 0);
-            if (!ok) fail(sh, 3);
-            auto issue_pv = [&](int i) -> bool {
-                const int st = i & 1;
-                const uint32_t ph = (uint32_t)((i >> 1) & 1);
-                if (!mbar_wait(&sh->v_full[st], ph)) { fail(sh, 4); return false; }
-                // P_i is in shared memory and, if the row maxima moved, the accumulator has been rescaled by its owners
-                if (!mbar_wait(&sh->p_ready, (uint32_t)(i & 1))) { fail(sh, 5); return false; }
-                tc_fence_after();
-                const uint32_t d_tmem = tmem_o;
+            const int ks_s = p.d / 16;                   // 16-deep steps of the Q K^T contraction
+            bool ok = mbar_wait_warp(smem_u32(&sh->q_full), 0);
+            if (!ok && lane == 0) fail(sh, 3);
+            uint32_t done[2] = {0u, 0u};                 // tiles of P V issued per query tile
+            int last[2] = {J[0] - 1, J[1] - 1};          // its last key tile
 #pragma unroll
-                for (int ks = 0; ks < TILE / 16; ++ks) {
-                    // A = P (128 x 128 keys, K-major): chunk ks / 4, 32 bytes per step inside the swizzle row
-                    // B = V (128 keys x HD, head dim contiguous = MN-major): 16 key rows per step, chunks of 64 columns apart by CHUNK
-                    const uint64_t ad = pack_desc(desc_lo(sP + (ks >> 2) * CHUNK + (ks & 3) * 32, 0), hi);
-                    const uint64_t bd = pack_desc(desc_lo(sV + st * TB + ks * 2048, CHUNK), hi);
-                    umma_f16(d_tmem, ad, bd, p.idesc_pv, (i | ks) != 0 ? 1u : 0u);   // O accumulates over all key tiles
+            for (int t = 0; t < 2; ++t)
+                while (last[t] >= 0 && !active(t, last[t])) --last[t];
+            auto issue_s = [&](int t, int st) {          // S_t = Q_t K^T
+                if (elect_one()) {
+                    for (int ks = 0; ks < ks_s; ++ks) {
+                        const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32);
+                        umma_f16(tmem + t * TILE, pack_desc(desc_lo(sQ + t * TB + off, 0), hi), pack_desc(desc_lo(sK + st * TB + off, 0), hi),
+                                 p.idesc_s, ks != 0 ? 1u : 0u);
+                    }
+                    umma_commit(&sh->s_full[t]);
                 }
-                umma_commit(&sh->v_empty[st]);
-                umma_commit(&sh->p_free);
-                umma_commit(&sh->o_full);
-                return true;
+                __syncwarp();
             };
-            for (int j = 0; j < J && ok; ++j) {
-                const int st = j & 1;
-                const uint32_t ph = (uint32_t)((j >> 1) & 1);
-                if (!mbar_wait(&sh->k_full[st], ph)) { fail(sh, 7); ok = false; break; }
-                if (!mbar_wait(&sh->s_free[st], ph ^ 1)) { fail(sh, 8); ok = false; break; }
+            int j = first, n = 0;
+            if (ok && !mbar_wait_warp(smem_u32(&sh->k_full[0]), 0)) { if (lane == 0) fail(sh, 4); ok = false; }
+            if (ok) {
                 tc_fence_after();
-                for (int ks = 0; ks < ks_s; ++ks) {
-                    const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32);
-                    const uint64_t ad = pack_desc(desc_lo(sQ + off, 0), hi);
-                    const uint64_t bd = pack_desc(desc_lo(sK + st * TB + off, 0), hi);
-                    umma_f16(tmem + st * TILE, ad, bd, p.idesc_s, ks != 0 ? 1u : 0u);
-                }
-                umma_commit(&sh->k_empty[st]);
-                umma_commit(&sh->s_full[st]);
-                if (j >= 1) ok = issue_pv(j - 1);
+                if (active(0, j)) issue_s(0, 0);
+                if (active(1, j)) issue_s(1, 0);
+                if (elect_one()) umma_commit(&sh->k_empty[0]);
+                __syncwarp();
             }
-            if (ok) issue_pv(J - 1);
+            while (ok && j < J_max) {
+                const int jn = next_step(j), st = n & 1, sn = (n + 1) & 1;
+                const uint32_t ph = (uint32_t)((n >> 1) & 1), phn = (uint32_t)(((n + 1) >> 1) & 1);
+                if (!mbar_wait_warp(smem_u32(&sh->v_full[st]), ph)) { if (lane == 0) fail(sh, 5); ok = false; break; }
+                bool k_seen = false;
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    if (active(t, j)) {
+                        // P_t is in tensor memory and, if row maxima moved, O_t has been rescaled by its owners
+                        if (!mbar_wait_warp(smem_u32(&sh->p_ready[t]), done[t] & 1u)) { if (lane == 0) fail(sh, 6); ok = false; break; }
+                        tc_fence_after();
+                        if (elect_one()) {
+#pragma unroll
+                            for (int ks = 0; ks < TILE / 16; ++ks)
+                                // B = V (128 keys x head dim, head dim contiguous = MN-major): 16 key rows per step, 64-column chunks CHUNK apart
+                                umma_f16_ts(tmem + 256 + t * TILE, tmem + t * TILE + ks * 8, pack_desc(desc_lo(sV + st * TB + ks * 2048, CHUNK), hi),
+                                            p.idesc_pv, (done[t] | ks) != 0 ? 1u : 0u);
+                            if (j == last[t]) umma_commit(&sh->o_full[t]);
+                        }
+                        __syncwarp();
+                        ++done[t];
+                    }
+                    if (jn < J_max && active(t, jn)) {
+                        if (!k_seen) {
+                            if (!mbar_wait_warp(smem_u32(&sh->k_full[sn]), phn)) { if (lane == 0) fail(sh, 7); ok = false; break; }
+                            tc_fence_after();
+                            k_seen = true;
+                        }
+                        issue_s(t, sn);
+                    }
+                }
+                if (!ok) break;
+                if (elect_one()) {
+                    umma_commit(&sh->v_empty[st]);
+                    if (jn < J_max) umma_commit(&sh->k_empty[sn]);
+                }
+                __syncwarp();
+                j = jn;
+                ++n;
+            }
         }
     } else {
         // ------------------------------------------------------------------------------------------ softmax + epilogue
-        const int quarter = warp & 3;                 // TMEM lanes [32 * quarter, 32 * quarter + 32) belong to this warp
+        const int t = (warp - 2) >> 2, quarter = warp & 3;      // TMEM lanes [32 * quarter, 32 * quarter + 32) belong to this warp
         const int row = quarter * 32 + lane;
-        const int64_t qi = q0 + row;                  // query index of this thread
+        const int64_t q0 = (int64_t)(qt0 + t) * TILE, qi = q0 + row;
         const bool row_ok = qi < p.sq;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        const uint8_t* mrow = (p.mask && row_ok) ? p.mask + ((int64_t)b * p.sq + qi) * p.sk : nullptr;
-        const int64_t causal_last = p.causal ? qi + p.causal_off : p.sk;   // last visible key of this row under the causal rule
+        const uint32_t s_addr = tmem + lane_addr + t * TILE, o_addr = tmem + lane_addr + 256 + t * TILE;
+        const uint4* brow = (p.bits && row_ok) ? reinterpret_cast<const uint4*>(p.bits) + ((int64_t)b * p.sq + qi) * p.k_tiles : nullptr;
+        const uint8_t* crow = cls0 ? cls0 + t * p.k_tiles : nullptr;
+        const int64_t limit = p.causal && qi + p.causal_off + 1 < kv_lim ? qi + p.causal_off + 1 : kv_lim;   // keys below it are visible
         // m_ref: the maximum the exponents are taken against.  It follows the running maximum lazily: only when that
         // has grown by more than 8 (in base-2 exponent units) is the accumulator in tensor memory rescaled -- probabilities
         // stay below 2^8, sums are fp32 -- so that after the first few tiles a tile costs one round trip to tensor memory.
         float m_ref = -INFINITY, l_run = 0.f;
+        uint32_t n = 0;
         bool ok = true;
-        for (int j = 0; j < J && ok; ++j) {
-            const int sb = j & 1;
-            if (!warp_wait(&sh->s_full[sb], (uint32_t)((j >> 1) & 1), lane)) { if (lane == 0) fail(sh, 9); ok = false; break; }
-            tc_fence_after();
+        for (int j = 0; j < J[t] && ok; ++j) {
+            const int kind = crow ? crow[j] : 2;
+            if (kind == 0) continue;
             const int64_t kv0 = (int64_t)j * TILE;
-            const bool need_mask = (kv0 + TILE > kv_end) || (p.causal && kv0 + TILE - 1 > q0 + p.causal_off) || mrow != nullptr;
-            const uint32_t s_addr = tmem + lane_addr + sb * TILE;
+            const bool need_mask = kind == 1 || kv0 + TILE > kv_lim || (p.causal && kv0 + TILE - 1 > q0 + p.causal_off);
+            uint32_t vis[TILE / 32];
+            if (need_mask) {
+                uint4 w = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+                if (kind == 1 && brow) w = brow[j];
+                vis[0] = w.x & low_bits(limit - kv0); vis[1] = w.y & low_bits(limit - kv0 - 32);
+                vis[2] = w.z & low_bits(limit - kv0 - 64); vis[3] = w.w & low_bits(limit - kv0 - 96);
+            }
+            if (!warp_wait(&sh->s_full[t], n & 1u, lane)) { if (lane == 0) fail(sh, 9); ok = false; break; }
+            tc_fence_after();
             uint32_t r[TILE / 32][32];
 #pragma unroll
             for (int c4 = 0; c4 < TILE / 32; ++c4) tmem_ld32(s_addr + c4 * 32, r[c4]);
             tmem_ld_wait();
-            // the scores are in registers: the S buffer may take the tile after next
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh->s_free[sb]);
-            uint32_t vis[TILE / 32];
-#pragma unroll
-            for (int c4 = 0; c4 < TILE / 32; ++c4) vis[c4] = 0xffffffffu;
-            if (need_mask) {
-                const int64_t limit = kv_end < causal_last + 1 ? kv_end : causal_last + 1;
-#pragma unroll
-                for (int c4 = 0; c4 < TILE / 32; ++c4) vis[c4] = visible_bits(kv0 + c4 * 32, limit, mrow);
-            }
             // tiles away from the diagonal and the ragged edge (the common case) skip the per-element visibility tests
-            float mt = -INFINITY;
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
             if (need_mask) {
 #pragma unroll
                 for (int c4 = 0; c4 < TILE / 32; ++c4)
 #pragma unroll
                     for (int i = 0; i < 32; ++i)
-                        if ((vis[c4] >> i) & 1u) mt = fmaxf(mt, __uint_as_float(r[c4][i]));
+                        if ((vis[c4] >> i) & 1u) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(r[c4][i]));
             } else {
 #pragma unroll
                 for (int c4 = 0; c4 < TILE / 32; ++c4)
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) mt = fmaxf(mt, __uint_as_float(r[c4][i]));
+                    for (int i = 0; i < 32; i += 2)
+                        mx[(i >> 1) & 3] = fmaxf(fmaxf(mx[(i >> 1) & 3], __uint_as_float(r[c4][i])), __uint_as_float(r[c4][i + 1]));
             }
+            const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
             // move the reference maximum?  (first visible score of the row, or growth beyond the threshold)
             float alpha = 1.f;
             bool move = false;
@@ -274,56 +392,55 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 if (m_ref == -INFINITY) { m_ref = mt; }               // nothing accumulated yet: O and l are zero
                 else if ((mt - m_ref) * p.sl2 > 8.f) { alpha = ex2((m_ref - mt) * p.sl2); m_ref = mt; move = true; }
             }
-            // the previous tile's MMAs have read P (and, when rescaling, must have finished adding into O)
-            if (!warp_wait(&sh->p_free, (uint32_t)((j & 1) ^ 1), lane)) { if (lane == 0) fail(sh, 10); ok = false; break; }
-            if (j > 0 && __any_sync(0xffffffffu, move)) {
+            if (n > 0 && __any_sync(0xffffffffu, move)) {
                 // rescale this warp's 32 rows of the accumulator (lanes whose maximum did not move multiply by one)
-                tc_fence_after();
-                l_run *= alpha;
 #pragma unroll
-                for (int c4 = 0; c4 < HD / 32; ++c4) {
-                    uint32_t o[32];
-                    tmem_ld32(tmem_o + lane_addr + c4 * 32, o);
-                    tmem_ld_wait();
+                for (int c8 = 0; c8 < HD / 8; ++c8) {
+                    if (c8 * 8 < p.d) {
+                        uint32_t o[8];
+                        tmem_ld8(o_addr + c8 * 8, o);
+                        tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                    tmem_st32(tmem_o + lane_addr + c4 * 32, o);
+                        for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st8(o_addr + c8 * 8, o);
+                    }
                 }
-                tmem_st_wait();
-            } else {
-                l_run *= alpha;
             }
             const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref * p.sl2;
-            float rowsum = 0.f;
+            const uint64_t sl2_2 = pack_f2(p.sl2, p.sl2), neg_2 = pack_f2(neg_m, neg_m);
+            uint64_t sum2[2] = {0ull, 0ull};
 #pragma unroll
-            for (int c4 = 0; c4 < TILE / 32; ++c4) {
-                const uint32_t base = sP + (uint32_t)(c4 >> 1) * CHUNK + (uint32_t)row * 128;
+            for (int half = 0; half < 2; ++half) {
+                uint32_t pk[32];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    float pv[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        float e = ex2(fmaf(__uint_as_float(r[c4][8 * t + i]), p.sl2, neg_m));
-                        if (need_mask && !((vis[c4] >> (8 * t + i)) & 1u)) e = 0.f;
-                        pv[i] = e;
-                        rowsum += e;
+                for (int i = 0; i < 32; ++i) {
+                    const int e = half * 64 + 2 * i, c4 = e >> 5, k = e & 31;
+                    float x, y;
+                    unpack_f2(fma_f2(pack_f2(__uint_as_float(r[c4][k]), __uint_as_float(r[c4][k + 1])), sl2_2, neg_2), x, y);
+                    x = ex2(x);
+                    y = ex2(y);
+                    if (need_mask) {
+                        if (!((vis[c4] >> k) & 1u)) x = 0.f;
+                        if (!((vis[c4] >> (k + 1)) & 1u)) y = 0.f;
                     }
-                    const uint32_t piece = (uint32_t)(((c4 & 1) * 4 + t) ^ (row & 7));
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(base + (piece << 4)),
-                                 "r"(pack2<T>(pv[0], pv[1])), "r"(pack2<T>(pv[2], pv[3])),
-                                 "r"(pack2<T>(pv[4], pv[5])), "r"(pack2<T>(pv[6], pv[7])) : "memory");
+                    sum2[i & 1] = add_f2(sum2[i & 1], pack_f2(x, y));
+                    pk[i] = pack2<T>(x, y);
                 }
+                tmem_st32(s_addr + half * 32, pk);     // over the scores: this thread's row, already in registers
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores before the MMA's async-proxy reads
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sh->p_ready);
-            l_run += rowsum;
+            if (lane == 0) mbar_arrive(&sh->p_ready[t]);
+            float s0, s1;
+            unpack_f2(add_f2(sum2[0], sum2[1]), s0, s1);
+            l_run = l_run * alpha + (s0 + s1);
+            ++n;
         }
-        if (ok && J > 0) {
-            if (!warp_wait(&sh->o_full, (uint32_t)((J - 1) & 1), lane)) { if (lane == 0) fail(sh, 12); ok = false; }
+        if (ok && n > 0) {
+            if (!warp_wait(&sh->o_full[t], 0u, lane)) { if (lane == 0) fail(sh, 12); ok = false; }
         }
-        if (ok) {
+        if (ok && t < p.per_cta && qt0 + t < p.q_tiles) {
             // normalise and store the row (the tensor-memory loads are warp-wide; only the stores depend on the row)
             const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
             T* orow = (T*)p.o + (int64_t)b * p.o_batch + qi * p.o_tok + (int64_t)head * p.o_head;
@@ -331,8 +448,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
 #pragma unroll
             for (int c4 = 0; c4 < HD / 32; ++c4) {
                 uint32_t o[32];
-                if (J > 0) {
-                    tmem_ld32(tmem_o + lane_addr + c4 * 32, o);
+                if (n > 0) {
+                    tmem_ld32(o_addr + c4 * 32, o);
                     tmem_ld_wait();
                 } else {
 #pragma unroll
@@ -340,12 +457,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 }
                 if (row_ok) {
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        if (c4 * 32 + t * 8 < p.d) {
+                    for (int q = 0; q < 4; ++q) {
+                        if (c4 * 32 + q * 8 < p.d) {
                             bmt::Vec16<T> ov;
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) ov.v[i] = bmt::Cvt<T>::from_f(__uint_as_float(o[t * 8 + i]) * inv);
-                            bmt::st16(orow + c4 * 32 + t * 8, ov);
+                            for (int i = 0; i < 8; ++i) ov.v[i] = bmt::Cvt<T>::from_f(__uint_as_float(o[q * 8 + i]) * inv);
+                            bmt::st16(orow + c4 * 32 + q * 8, ov);
                         }
                     }
                 }
@@ -368,50 +485,73 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
+int sm_count() {
+    static int sms[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (sms[dev] == 0 && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+    return sms[dev];
+}
+
 template <int HD, typename T>
-int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, int64_t batch, cudaStream_t stream) {
+int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, AttnParams& p, int64_t batch, cudaStream_t stream) {
     constexpr uint32_t TB = (HD / 64) * CHUNK;
-    const size_t smem = 5 * TB + 2 * CHUNK + sizeof(AttnShared) + 1024;
+    const size_t smem = 6 * TB + sizeof(AttnShared) + 1024;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(flash_fwd_kernel<HD, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -30;
         configured = true;
     }
-    dim3 grid((unsigned)((p.sq + TILE - 1) / TILE), (unsigned)p.h, (unsigned)batch);
-    flash_fwd_kernel<HD, T><<<grid, ATT_THREADS, smem, stream>>>(tq, tk, tv, p);
+    // pairs of query tiles unless single tiles still find an SM each: a pair shares its K / V loads and hides one tile's
+    // softmax behind the other's MMAs, two SMs are faster still
+    p.per_cta = (int64_t)p.q_tiles * p.h * batch > sm_count() ? 2 : 1;
+    dim3 grid((unsigned)(p.h * batch), (unsigned)((p.q_tiles + p.per_cta - 1) / p.per_cta));
+    flash_fwd_kernel<HD, T><<<grid, FWD_THREADS, smem, stream>>>(tq, tk, tv, p);
     bmt_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
 
-
 // ================================================================================================ backward
 // One CTA per (128 keys, kv head, sample).  K and V tiles stay in shared memory; the CTA walks over the query heads that
-// share the kv head and over the query tiles that can see its keys.  Per (query tile, key tile) pair:
-//   MMA   S = Q K^T and dP = dO V^T into tensor memory
-//   warps P = exp2(S * scale * log2e - lse * log2e) (masked), dS = P * (dP - delta) * scale; both written to shared
-//         memory as fp16/bf16 in the swizzled [query][key] layout, which serves as a K-major operand (dQ) and,
-//         read "transposed", as an MN-major operand (dV, dK)
-//   MMA   dV += P^T dO, dK += dS^T Q (accumulating in tensor memory over the whole walk), dQ = dS K
-//   warps dQ rows are added to an fp32 accumulator in global memory (vector reductions); a small kernel converts it
+// share the kv head and over the query tiles that can see its keys.  Scores are held transposed (lane = key, column =
+// query), so that P^T and dS^T are the A operands of dV += P^T dO and dK += dS^T Q as they stand.  Per (query, key) tile:
+//   MMA   S^T = K Q^T and dP^T = V dO^T into tensor memory
+//   softmax warps (8, two per 32 keys, 64 queries each): P = exp2(S * scale * log2e - lse * log2e) (masked) back into
+//         tensor memory as packed 16-bit pairs, over S^T; dS = P * (dP - delta) * scale as 16 bits into shared memory,
+//         [key][query] swizzled: K-major A for dK and, read "transposed", MN-major A for dQ = dS K
+//   MMA   dV += P^T dO (P from tensor memory), dK += dS^T Q, dQ = dS K
+//   dQ warps (4): add the tile of dQ to an fp32 accumulator in global memory (vector reductions); a small kernel converts it
 // delta = rowsum(dO * O) comes from a pre-pass.  dK / dV are written once at the end, already summed over the group.
+// Order on the tensor pipe, which bounds a tile at 5 x 512 clocks (head dim 128): dP(i), dV(i), S(i+1), dK(i), dQ(i), dP(i+1):
+// while the softmax warps turn dP(i) into dS(i) the pipe has dV(i) and S(i+1) to do, and while it does dK(i) and dQ(i) they
+// exponentiate S(i+1).  dQ(i) shares its columns with dP, so dP(i+1) waits until the dQ warps have read them; with head
+// dims up to 80 dQ has columns of its own.  All five products in turn with one group of four warps doing everything in
+// between took 13 600 clocks a tile.
 struct AttnBwdParams {
     int64_t sq, sk;
     int h, hk, d;
     float sl2, scale;
     int causal;
     int64_t causal_off;
-    const uint8_t* mask;
+    const uint32_t* bits_t;     // packed mask by key (b, sk, query tiles, 4 words) or null
+    const uint8_t* cls;         // (b, query tiles, key tiles), see the forward kernel
     const int32_t* kv_lens;
     const float* lse;
     const float* delta;
-    float* dq_acc;              // (b, sq, h, d) fp32, zero on entry
+    float* dq_acc;              // (b, h, sq, d) fp32, zero on entry
     void* dk; void* dv;         // (b, sk, hk, d) by strides {token, head, batch}
     int64_t dk_tok, dk_head, dk_batch, dv_tok, dv_head, dv_batch;
-    uint32_t idesc_s, idesc_tn, idesc_dq;
+    uint32_t idesc_s, idesc_dv, idesc_dq;
+    int q_tiles, k_tiles;
 };
 
+constexpr int BWD_THREADS = 448;                 // producer, MMA issuer, 8 softmax warps, 4 dQ warps
+
 struct BwdShared {
-    uint64_t kv_full, qdo_full, qdo_empty, sdp_full, pds_ready, dq_full, tmem_free;
+    uint64_t kv_full, q_full[2], q_empty[2], do_full, do_empty, s_full, dp_full, p_ready, ds_ready, dq_full, dq_empty, all_done;
+    uint64_t row_full[2], row_empty[2], pair[4];
+    float nlse[2][TILE], delta[2][TILE];         // per query of a tile: -lse * log2(e) (0 for rows that take no part), delta
+    uint32_t live[2][4];                         // queries of the tile that exist and see at least one key
     uint32_t tmem_base;
     int failed;
 };
@@ -425,35 +565,58 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
+// Walks the (head, query tile) pairs of a CTA in order, leaving out tiles without a visible pair.
+struct BwdWalk {
+    int head, qt, head_end, qt_first, q_tiles, k_tiles;
+    const uint8_t* cls;        // class of (query tile, this key tile), row pitch k_tiles; or null
+    __device__ __forceinline__ void settle() {
+        while (head < head_end) {
+            while (qt < q_tiles && cls && cls[(int64_t)qt * k_tiles] == 0) ++qt;
+            if (qt < q_tiles) return;
+            ++head;
+            qt = qt_first;
+        }
+    }
+    __device__ __forceinline__ bool more() const { return head < head_end; }
+    __device__ __forceinline__ void next() { ++qt; settle(); }
+};
+
 template <int HD, typename T>
-__global__ void __launch_bounds__(ATT_THREADS, 1)
+__global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                  const __grid_constant__ CUtensorMap tdo, const AttnBwdParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     constexpr int DC = HD / 64;
     constexpr uint32_t TB = DC * CHUNK;
-    const uint32_t sK = smem_u32(smem), sV = sK + TB, sQ = sV + TB, sdO = sQ + TB, sP = sdO + TB, sdS = sP + 2 * CHUNK;
-    BwdShared* sh = (BwdShared*)(smem + 4 * TB + 4 * CHUNK);
-    // tensor memory columns: S [0,128), dP [128,256), dV, dK behind them; dQ has columns of its own when they fit,
-    // otherwise it reuses the S columns (S has been read by the time dS exists)
-    constexpr uint32_t C_DP = 128, C_DV = 256, C_DK = 256 + HD, C_DQ = (256 + 3 * HD <= 512) ? 256 + 2 * HD : 0;
+    constexpr uint32_t DQ_BUF = 32 * 128;           // exchange buffer of one dQ warp: 32 rows x 32 floats
+    const uint32_t sK = smem_u32(smem), sV = sK + TB, sQ = sV + TB, sdO = sQ + 2 * TB, sdS = sdO + TB, sX = sdS + 2 * CHUNK;
+    BwdShared* sh = (BwdShared*)(smem + 5 * TB + 2 * CHUNK + 4 * DQ_BUF);
+    // tensor memory columns: S^T / P^T [0,128), dP^T [128,256), dV, dK, dQ each of d columns; above head dim 80 dQ takes dP's
+    const uint32_t C_DP = 128, C_DV = 256, C_DK = C_DV + p.d, C_DQ = p.d <= 80 ? C_DK + p.d : C_DP;
+    const bool dq_shared = p.d > 80;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kt = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int kvh = blockIdx.x % p.hk, b = blockIdx.x / p.hk, kt = blockIdx.y;   // under a causal mask the long columns start first
     const int group = p.h / p.hk;
     const int64_t kv0 = (int64_t)kt * TILE;
     int64_t kv_valid = p.sk;
     if (p.kv_lens && p.kv_lens[b] < kv_valid) kv_valid = p.kv_lens[b];
-    const int n_qt = (int)((p.sq + TILE - 1) / TILE);
-    int qt_first = 0;
-    if (p.causal && kv0 - p.causal_off > 0) qt_first = (int)((kv0 - p.causal_off) / TILE);
-    const int per_head = (kv0 < kv_valid && qt_first < n_qt) ? n_qt - qt_first : 0;
-    const int n_it = per_head * group;
+    BwdWalk walk;
+    walk.qt_first = 0;
+    if (p.causal && kv0 - p.causal_off > 0) walk.qt_first = (int)((kv0 - p.causal_off) / TILE);
+    walk.qt = walk.qt_first; walk.q_tiles = p.q_tiles; walk.k_tiles = p.k_tiles;
+    walk.head = kvh * group; walk.head_end = kv0 < kv_valid ? walk.head + group : walk.head;
+    walk.cls = p.cls ? p.cls + (int64_t)b * p.q_tiles * p.k_tiles + kt : nullptr;
+    walk.settle();
+    const bool work = walk.more();
 
     if (threadIdx.x == 0) {
-        mbar_init(&sh->kv_full, 1); mbar_init(&sh->qdo_full, 1); mbar_init(&sh->qdo_empty, 1); mbar_init(&sh->sdp_full, 1);
-        mbar_init(&sh->pds_ready, 4); mbar_init(&sh->dq_full, 1); mbar_init(&sh->tmem_free, 4);
+        mbar_init(&sh->kv_full, 1); mbar_init(&sh->do_full, 1); mbar_init(&sh->do_empty, 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(&sh->q_full[i], 1); mbar_init(&sh->q_empty[i], 1); mbar_init(&sh->row_full[i], 4); mbar_init(&sh->row_empty[i], 8); }
+        mbar_init(&sh->s_full, 1); mbar_init(&sh->dp_full, 1); mbar_init(&sh->p_ready, 8); mbar_init(&sh->ds_ready, 8);
+        for (int i = 0; i < 4; ++i) mbar_init(&sh->pair[i], 2);
+        mbar_init(&sh->dq_full, 1); mbar_init(&sh->dq_empty, 4); mbar_init(&sh->all_done, 1);
         sh->failed = 0;
         fence_barrier_init();
     }
@@ -464,185 +627,299 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     const uint32_t tmem = sh->tmem_base;
 
     if (warp == 0) {
-        if (lane == 0 && n_it > 0) {
+        // ------------------------------------------------------------------------------------------ TMA producer
+        if (work) {
             const uint32_t kvbar = smem_u32(&sh->kv_full);
-            mbar_expect_tx_u32(kvbar, 2 * TB);
-#pragma unroll
-            for (int c = 0; c < DC; ++c) {
-                tma_load_4d_u32(&tk, kvbar, sK + c * CHUNK, c * 64, (int)kv0, kvh, b);
-                tma_load_4d_u32(&tv, kvbar, sV + c * CHUNK, c * 64, (int)kv0, kvh, b);
-            }
-            for (int it = 0; it < n_it; ++it) {
-                const int head = kvh * group + it / per_head, qt = qt_first + it % per_head;
-                if (!mbar_wait(&sh->qdo_empty, (uint32_t)((it & 1) ^ 1))) { fail_bwd(sh, 1); break; }
-                const uint32_t bar = smem_u32(&sh->qdo_full);
-                mbar_expect_tx_u32(bar, 2 * TB);
+            if (elect_one()) {
+                mbar_expect_tx_u32(kvbar, 2 * TB);
 #pragma unroll
                 for (int c = 0; c < DC; ++c) {
-                    tma_load_4d_u32(&tq, bar, sQ + c * CHUNK, c * 64, qt * TILE, head, b);
-                    tma_load_4d_u32(&tdo, bar, sdO + c * CHUNK, c * 64, qt * TILE, head, b);
+                    tma_load_4d_u32(&tk, kvbar, sK + c * CHUNK, c * 64, (int)kv0, kvh, b);
+                    tma_load_4d_u32(&tv, kvbar, sV + c * CHUNK, c * 64, (int)kv0, kvh, b);
                 }
+            }
+            __syncwarp();
+            for (uint32_t it = 0; walk.more(); walk.next(), ++it) {
+                const uint32_t st = it & 1, ph = (it >> 1) & 1;
+                if (!mbar_wait_warp(smem_u32(&sh->q_empty[st]), ph ^ 1)) { if (lane == 0) fail_bwd(sh, 1); break; }
+                if (elect_one()) {
+                    const uint32_t bar = smem_u32(&sh->q_full[st]);
+                    mbar_expect_tx_u32(bar, TB);
+#pragma unroll
+                    for (int c = 0; c < DC; ++c) tma_load_4d_u32(&tq, bar, sQ + st * TB + c * CHUNK, c * 64, walk.qt * TILE, walk.head, b);
+                }
+                __syncwarp();
+                if (!mbar_wait_warp(smem_u32(&sh->do_empty), (it & 1) ^ 1)) { if (lane == 0) fail_bwd(sh, 2); break; }
+                if (elect_one()) {
+                    const uint32_t bar = smem_u32(&sh->do_full);
+                    mbar_expect_tx_u32(bar, TB);
+#pragma unroll
+                    for (int c = 0; c < DC; ++c) tma_load_4d_u32(&tdo, bar, sdO + c * CHUNK, c * 64, walk.qt * TILE, walk.head, b);
+                }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && n_it > 0) {
+        // ------------------------------------------------------------------------------------------ MMA issuer
+        if (work) {
             const uint32_t hi = desc_hi(1024);
-            const int ks_d = (p.d + 15) / 16;
-            bool ok = mbar_wait(&sh->kv_full, 0);
-            if (!ok) fail_bwd(sh, 2);
-            for (int it = 0; it < n_it && ok; ++it) {
-                const uint32_t ph = (uint32_t)(it & 1);
-                if (!mbar_wait(&sh->qdo_full, ph)) { fail_bwd(sh, 3); break; }
-                if (!mbar_wait(&sh->tmem_free, ph ^ 1)) { fail_bwd(sh, 4); break; }
+            const int ks_d = p.d / 16;
+            bool ok = mbar_wait_warp(smem_u32(&sh->kv_full), 0);
+            if (!ok && lane == 0) fail_bwd(sh, 3);
+            auto issue_s = [&](uint32_t it) -> bool {       // S^T = K Q^T of tile `it`
+                const uint32_t st = it & 1;
+                if (!mbar_wait_warp(smem_u32(&sh->q_full[st]), (it >> 1) & 1)) { if (lane == 0) fail_bwd(sh, 4); return false; }
                 tc_fence_after();
-                for (int ks = 0; ks < ks_d; ++ks) {
-                    const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32);
-                    umma_f16(tmem, pack_desc(desc_lo(sQ + off, 0), hi), pack_desc(desc_lo(sK + off, 0), hi), p.idesc_s, ks != 0 ? 1u : 0u);
+                if (elect_one()) {
+                    for (int ks = 0; ks < ks_d; ++ks) {
+                        const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32);
+                        umma_f16(tmem, pack_desc(desc_lo(sK + off, 0), hi), pack_desc(desc_lo(sQ + st * TB + off, 0), hi), p.idesc_s, ks != 0 ? 1u : 0u);
+                    }
+                    umma_commit(&sh->s_full);
                 }
-                for (int ks = 0; ks < ks_d; ++ks) {
-                    const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32);
-                    umma_f16(tmem + C_DP, pack_desc(desc_lo(sdO + off, 0), hi), pack_desc(desc_lo(sV + off, 0), hi), p.idesc_s, ks != 0 ? 1u : 0u);
-                }
-                umma_commit(&sh->sdp_full);
-                if (!mbar_wait(&sh->pds_ready, ph)) { fail_bwd(sh, 5); break; }
+                __syncwarp();
+                return true;
+            };
+            ok = ok && issue_s(0);
+            for (uint32_t it = 0; ok && walk.more(); ++it) {
+                const uint32_t ph = it & 1, st = it & 1;
+                walk.next();
+                if (!mbar_wait_warp(smem_u32(&sh->do_full), ph)) { if (lane == 0) fail_bwd(sh, 5); break; }
+                // dP's columns: dS(it-1) was computed from them before dK(it-1) could be issued; dQ(it-1) has to be out of them
+                if (dq_shared && !mbar_wait_warp(smem_u32(&sh->dq_empty), ph ^ 1)) { if (lane == 0) fail_bwd(sh, 6); break; }
                 tc_fence_after();
+                if (elect_one()) {
+                    for (int ks = 0; ks < ks_d; ++ks) {
+                        const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32);
+                        umma_f16(tmem + C_DP, pack_desc(desc_lo(sV + off, 0), hi), pack_desc(desc_lo(sdO + off, 0), hi), p.idesc_s, ks != 0 ? 1u : 0u);
+                    }
+                    umma_commit(&sh->dp_full);
+                }
+                __syncwarp();
+                if (!mbar_wait_warp(smem_u32(&sh->p_ready), ph)) { if (lane == 0) fail_bwd(sh, 7); break; }
+                tc_fence_after();
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < TILE / 16; ++ks)      // dV += P^T dO: 16 query rows per step, both operands MN-major
-                    umma_f16(tmem + C_DV, pack_desc(desc_lo(sP + ks * 2048, CHUNK), hi), pack_desc(desc_lo(sdO + ks * 2048, CHUNK), hi),
-                             p.idesc_tn, (it | ks) != 0 ? 1u : 0u);
+                    for (int ks = 0; ks < TILE / 16; ++ks)      // dV += P^T dO: 16 queries per step, dO MN-major
+                        umma_f16_ts(tmem + C_DV, tmem + ks * 8, pack_desc(desc_lo(sdO + ks * 2048, CHUNK), hi), p.idesc_dv, (it | (uint32_t)ks) != 0 ? 1u : 0u);
+                    umma_commit(&sh->do_empty);
+                }
+                __syncwarp();
+                if (walk.more() && !issue_s(it + 1)) break;
+                if (!mbar_wait_warp(smem_u32(&sh->ds_ready), ph)) { if (lane == 0) fail_bwd(sh, 8); break; }
+                if (!dq_shared && !mbar_wait_warp(smem_u32(&sh->dq_empty), ph ^ 1)) { if (lane == 0) fail_bwd(sh, 9); break; }
+                tc_fence_after();
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < TILE / 16; ++ks)      // dK += dS^T Q
-                    umma_f16(tmem + C_DK, pack_desc(desc_lo(sdS + ks * 2048, CHUNK), hi), pack_desc(desc_lo(sQ + ks * 2048, CHUNK), hi),
-                             p.idesc_tn, (it | ks) != 0 ? 1u : 0u);
-                umma_commit(&sh->qdo_empty);
+                    for (int ks = 0; ks < TILE / 16; ++ks)      // dQ = dS K: 16 keys per step, both operands MN-major
+                        umma_f16(tmem + C_DQ, pack_desc(desc_lo(sdS + ks * 2048, CHUNK), hi), pack_desc(desc_lo(sK + ks * 2048, CHUNK), hi),
+                                 p.idesc_dq, ks != 0 ? 1u : 0u);
+                    umma_commit(&sh->dq_full);
 #pragma unroll
-                for (int ks = 0; ks < TILE / 16; ++ks)      // dQ = dS K: 16 keys per step, A K-major, B (K tile) MN-major
-                    umma_f16(tmem + C_DQ, pack_desc(desc_lo(sdS + (ks >> 2) * CHUNK + (ks & 3) * 32, 0), hi),
-                             pack_desc(desc_lo(sK + ks * 2048, CHUNK), hi), p.idesc_dq, ks != 0 ? 1u : 0u);
-                umma_commit(&sh->dq_full);
+                    for (int ks = 0; ks < TILE / 16; ++ks)      // dK += dS^T Q: 16 queries per step, A K-major, Q MN-major
+                        umma_f16(tmem + C_DK, pack_desc(desc_lo(sdS + (ks >> 2) * CHUNK + (ks & 3) * 32, 0), hi),
+                                 pack_desc(desc_lo(sQ + st * TB + ks * 2048, CHUNK), hi), p.idesc_dv, (it | (uint32_t)ks) != 0 ? 1u : 0u);
+                    umma_commit(&sh->q_empty[st]);
+                    if (!walk.more()) umma_commit(&sh->all_done);
+                }
+                __syncwarp();
             }
         }
-    } else {
-        const int quarter = warp & 3;
+    } else if (warp < 10) {
+        // ------------------------------------------------------------------------------------------ softmax: P and dS
+        const int quarter = warp & 3, part = (warp - 2) >> 2;       // 32 keys, 64 queries of the tile
         const int row = quarter * 32 + lane;
+        const int64_t kj = kv0 + row;                                // this thread's key
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+        const uint4* brow = (p.bits_t && kj < p.sk) ? reinterpret_cast<const uint4*>(p.bits_t) + ((int64_t)b * p.sk + kj) * p.q_tiles : nullptr;
+        const uint64_t sl2_2 = pack_f2(p.sl2, p.sl2);
         bool ok = true;
-        for (int it = 0; it < n_it && ok; ++it) {
-            const uint32_t ph = (uint32_t)(it & 1);
-            const int head = kvh * group + it / per_head, qt = qt_first + it % per_head;
-            const int64_t q0 = (int64_t)qt * TILE, qi = q0 + row;
-            const bool row_ok = qi < p.sq;
-            float lse_r = -INFINITY, delta_r = 0.f;
-            if (row_ok) {
-                lse_r = p.lse[((int64_t)b * p.h + head) * p.sq + qi];
-                delta_r = p.delta[((int64_t)b * p.h + head) * p.sq + qi];
+        uint32_t it = 0;
+        for (; walk.more() && ok; walk.next(), ++it) {
+            const uint32_t ph = it & 1, st = it & 1;
+            const int64_t q0 = (int64_t)walk.qt * TILE;
+            const int kind = walk.cls ? walk.cls[(int64_t)walk.qt * p.k_tiles] : 2;
+            if (!warp_wait(&sh->row_full[st], (it >> 1) & 1, lane)) { if (lane == 0) fail_bwd(sh, 10); ok = false; break; }
+            uint32_t vis[2];
+            vis[0] = sh->live[st][part * 2]; vis[1] = sh->live[st][part * 2 + 1];
+            bool need_mask = kind == 1 || kv0 + TILE > kv_valid || (p.causal && kv0 + TILE - 1 > q0 + p.causal_off) ||
+                             (vis[0] & vis[1]) != 0xffffffffu;
+            if (need_mask) {
+                if (kj >= kv_valid) vis[0] = vis[1] = 0u;
+                if (p.causal) {          // query q0 + c sees this key from c = kj - causal_off - q0 on
+                    const int64_t c0 = kj - p.causal_off - q0 - part * 64;
+                    vis[0] &= ~low_bits(c0);
+                    vis[1] &= ~low_bits(c0 - 32);
+                }
+                if (kind == 1 && brow) {
+                    const uint4 w = brow[walk.qt];
+                    vis[0] &= part ? w.z : w.x;
+                    vis[1] &= part ? w.w : w.y;
+                }
             }
-            const bool alive = row_ok && lse_r != -INFINITY;
-            const float nlse = alive ? -lse_r * 1.4426950408889634f : 0.f;
-            const uint8_t* mrow = (p.mask && row_ok) ? p.mask + ((int64_t)b * p.sq + qi) * p.sk : nullptr;
-            const int64_t causal_last = p.causal ? qi + p.causal_off : p.sk;
-            const bool need_mask = (kv0 + TILE > kv_valid) || (p.causal && kv0 + TILE - 1 > q0 + p.causal_off) || mrow != nullptr;
-            if (!warp_wait(&sh->sdp_full, ph, lane)) { if (lane == 0) fail_bwd(sh, 6); ok = false; break; }
+            if (!warp_wait(&sh->s_full, ph, lane)) { if (lane == 0) fail_bwd(sh, 11); ok = false; break; }
             tc_fence_after();
-            // A tensor-memory load costs a round trip of a few hundred nanoseconds however wide it is, so the loads of 64
-            // columns of S and of dP are issued together and waited for once (two round trips per tile).
+            uint32_t s[2][32];
+            tmem_ld32(tmem + lane_addr + part * 64, s[0]);
+            tmem_ld32(tmem + lane_addr + part * 64 + 32, s[1]);
+            tmem_ld_wait();
+            // the other warp of these 32 keys still reads S^T columns that P^T goes over (packed columns [0,64) are queries
+            // [0,64) of S^T): both halves have to be in registers before either is written
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->pair[quarter]);
+            if (!warp_wait(&sh->pair[quarter], ph, lane)) { if (lane == 0) fail_bwd(sh, 17); ok = false; break; }
+            tc_fence_after();
+            float pr[64];
+            uint32_t pk[32];
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t rs[2][32], rd[2][32];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    tmem_ld32(tmem + lane_addr + (half * 2 + u) * 32, rs[u]);
-                    tmem_ld32(tmem + lane_addr + C_DP + (half * 2 + u) * 32, rd[u]);
+            for (int i = 0; i < 32; ++i) {
+                const int u = i >> 4, k = (2 * i) & 31;
+                const float2 nl = *reinterpret_cast<const float2*>(&sh->nlse[st][part * 64 + 2 * i]);
+                float x, y;
+                unpack_f2(fma_f2(pack_f2(__uint_as_float(s[u][k]), __uint_as_float(s[u][k + 1])), sl2_2, pack_f2(nl.x, nl.y)), x, y);
+                x = ex2(x);
+                y = ex2(y);
+                if (need_mask) {
+                    if (!((vis[u] >> k) & 1u)) x = 0.f;
+                    if (!((vis[u] >> (k + 1)) & 1u)) y = 0.f;
                 }
-                tmem_ld_wait();
+                pr[2 * i] = x;
+                pr[2 * i + 1] = y;
+                pk[i] = pack2<T>(x, y);
+            }
+            tmem_st32(tmem + lane_addr + part * 32, pk);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->p_ready);
+            if (!warp_wait(&sh->dp_full, ph, lane)) { if (lane == 0) fail_bwd(sh, 12); ok = false; break; }
+            tc_fence_after();
+            tmem_ld32(tmem + lane_addr + C_DP + part * 64, s[0]);
+            // dS(it-1) in shared memory may still be read by dQ / dK(it-1): wait for the commit behind both
+            if (it > 0 && !warp_wait(&sh->q_empty[st ^ 1], ((it - 1) >> 1) & 1, lane)) { if (lane == 0) fail_bwd(sh, 13); ok = false; break; }
+            const uint32_t base = sdS + (uint32_t)part * CHUNK + (uint32_t)row * 128;
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int c4 = half * 2 + u;
-                    uint32_t bits = alive ? 0xffffffffu : 0u;
-                    if (need_mask && alive) bits = visible_bits(kv0 + c4 * 32, kv_valid < causal_last + 1 ? kv_valid : causal_last + 1, mrow);
-                    const uint32_t off = (uint32_t)half * CHUNK + (uint32_t)row * 128;
+            for (int u = 0; u < 2; ++u) {
+                tmem_ld_wait_for(s[0]);
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        float pv[8], ds[8];
+                for (int t = 0; t < 4; ++t) {
+                    uint32_t w[4];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const float e = ((bits >> (8 * t + i)) & 1u) ? ex2(fmaf(__uint_as_float(rs[u][8 * t + i]), p.sl2, nlse)) : 0.f;
-                            pv[i] = e;
-                            ds[i] = e * (__uint_as_float(rd[u][8 * t + i]) - delta_r) * p.scale;
-                        }
-                        const uint32_t piece = (uint32_t)((u * 4 + t) ^ (row & 7)) << 4;
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sP + off + piece),
-                                     "r"(pack2<T>(pv[0], pv[1])), "r"(pack2<T>(pv[2], pv[3])),
-                                     "r"(pack2<T>(pv[4], pv[5])), "r"(pack2<T>(pv[6], pv[7])) : "memory");
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sdS + off + piece),
-                                     "r"(pack2<T>(ds[0], ds[1])), "r"(pack2<T>(ds[2], ds[3])),
-                                     "r"(pack2<T>(ds[4], ds[5])), "r"(pack2<T>(ds[6], ds[7])) : "memory");
+                    for (int i = 0; i < 4; ++i) {
+                        const int k = t * 8 + 2 * i, e = u * 32 + k;
+                        const float2 dl = *reinterpret_cast<const float2*>(&sh->delta[st][part * 64 + e]);
+                        w[i] = pack2<T>(pr[e] * (__uint_as_float(s[0][k]) - dl.x) * p.scale, pr[e + 1] * (__uint_as_float(s[0][k + 1]) - dl.y) * p.scale);
                     }
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(base + (uint32_t)(((u * 4 + t) ^ (row & 7)) << 4)), "r"(w[0]),
+                                 "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
                 }
+                if (u == 0) tmem_ld32(tmem + lane_addr + C_DP + part * 64 + 32, s[0]);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sh->pds_ready);
-            if (!warp_wait(&sh->dq_full, ph, lane)) { if (lane == 0) fail_bwd(sh, 7); ok = false; break; }
-            tc_fence_after();
-            float* dq_row = p.dq_acc + (((int64_t)b * p.sq + qi) * p.h + head) * p.d;
-            {
-                uint32_t r[HD / 32][32];
-#pragma unroll
-                for (int c4 = 0; c4 < HD / 32; ++c4) tmem_ld32(tmem + lane_addr + C_DQ + c4 * 32, r[c4]);
-                tmem_ld_wait();
-                // the values are in registers: the tensor memory may be overwritten by the next tile's MMAs while the
-                // reductions below are still being issued
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sh->tmem_free);
-                if (row_ok) {
-#pragma unroll
-                    for (int c4 = 0; c4 < HD / 32; ++c4)
-#pragma unroll
-                        for (int t = 0; t < 8; ++t)
-                            if (c4 * 32 + t * 4 < p.d)
-                                red_add_v4(dq_row + c4 * 32 + t * 4, __uint_as_float(r[c4][4 * t]), __uint_as_float(r[c4][4 * t + 1]),
-                                           __uint_as_float(r[c4][4 * t + 2]), __uint_as_float(r[c4][4 * t + 3]));
-                }
-            }
+            if (lane == 0) { mbar_arrive(&sh->ds_ready); mbar_arrive(&sh->row_empty[st]); }
         }
-        // dK, dV rows of this CTA's keys (zeros when no query sees them).  The tensor-memory loads are warp-wide, so every
-        // lane takes part in them; only the stores depend on the row.
-        const int64_t kj = kv0 + row;
+        // dK, dV rows of this CTA's keys (zeros when no query sees them): part 0 writes dK, part 1 dV.  The tensor-memory
+        // loads are warp-wide, so every lane takes part in them; only the stores depend on the row.
+        if (ok && it > 0 && !warp_wait(&sh->all_done, 0, lane)) { if (lane == 0) fail_bwd(sh, 14); ok = false; }
         if (ok) {
-            T* dkr = (T*)p.dk + (int64_t)b * p.dk_batch + kj * p.dk_tok + (int64_t)kvh * p.dk_head;
-            T* dvr = (T*)p.dv + (int64_t)b * p.dv_batch + kj * p.dv_tok + (int64_t)kvh * p.dv_head;
+            tc_fence_after();
+            T* dst = part == 0 ? (T*)p.dk + (int64_t)b * p.dk_batch + kj * p.dk_tok + (int64_t)kvh * p.dk_head
+                               : (T*)p.dv + (int64_t)b * p.dv_batch + kj * p.dv_tok + (int64_t)kvh * p.dv_head;
+            const uint32_t src = tmem + lane_addr + (part == 0 ? C_DK : C_DV);
 #pragma unroll
-            for (int c4 = 0; c4 < HD / 32; ++c4) {
-                uint32_t rk[32], rv[32];
-                if (n_it > 0) {
-                    tmem_ld32(tmem + lane_addr + C_DK + c4 * 32, rk);
-                    tmem_ld32(tmem + lane_addr + C_DV + c4 * 32, rv);
-                    tmem_ld_wait();
-                } else {
+            for (int c16 = 0; c16 < HD / 16; ++c16) {
+                if (c16 * 16 < p.d) {
+                    uint32_t r[16];
+                    if (it > 0) {
+                        tmem_ld16(src + c16 * 16, r);
+                        tmem_ld_wait();
+                    } else {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) rk[i] = rv[i] = 0u;
-                }
-                if (kj < p.sk) {
+                        for (int i = 0; i < 16; ++i) r[i] = 0u;
+                    }
+                    if (kj < p.sk) {
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        if (c4 * 32 + t * 8 < p.d) {
-                            bmt::Vec16<T> ok8, ov8;
+                        for (int q = 0; q < 2; ++q) {
+                            bmt::Vec16<T> ov;
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) {
-                                ok8.v[i] = bmt::Cvt<T>::from_f(__uint_as_float(rk[t * 8 + i]));
-                                ov8.v[i] = bmt::Cvt<T>::from_f(__uint_as_float(rv[t * 8 + i]));
-                            }
-                            bmt::st16(dkr + c4 * 32 + t * 8, ok8);
-                            bmt::st16(dvr + c4 * 32 + t * 8, ov8);
+                            for (int i = 0; i < 8; ++i) ov.v[i] = bmt::Cvt<T>::from_f(__uint_as_float(r[q * 8 + i]));
+                            bmt::st16(dst + c16 * 16 + q * 8, ov);
                         }
                     }
                 }
             }
+            tc_fence_before();
         }
-        tc_fence_before();
+    } else {
+        // ------------------------------------------------------------------------------------------ row statistics, dQ
+        const int quarter = warp & 3, r0 = quarter * 32;
+        const uint32_t lane_addr = (uint32_t)r0 << 16, xbuf = sX + (uint32_t)(warp - 10) * DQ_BUF;
+        bool ok = true;
+        BwdWalk ahead = walk;                    // the tile whose row statistics are fetched next: one ahead of the dQ tile
+        uint32_t n_rows = 0;
+        auto fetch_rows = [&]() -> bool {
+            const uint32_t st = n_rows & 1;
+            if (!warp_wait(&sh->row_empty[st], ((n_rows >> 1) & 1) ^ 1, lane)) { if (lane == 0) fail_bwd(sh, 15); return false; }
+            const int64_t qi = (int64_t)ahead.qt * TILE + r0 + lane;
+            float l = -INFINITY, dl = 0.f;
+            if (qi < p.sq) {
+                const int64_t at = ((int64_t)b * p.h + ahead.head) * p.sq + qi;
+                l = p.lse[at];
+                dl = p.delta[at];
+            }
+            const bool alive = l != -INFINITY;
+            sh->nlse[st][r0 + lane] = alive ? -l * 1.4426950408889634f : 0.f;
+            sh->delta[st][r0 + lane] = dl;
+            const uint32_t bits = __ballot_sync(0xffffffffu, alive);
+            if (lane == 0) sh->live[st][quarter] = bits;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->row_full[st]);
+            ++n_rows;
+            ahead.next();
+            return true;
+        };
+        if (work) ok = fetch_rows();
+        for (uint32_t it = 0; walk.more() && ok; walk.next(), ++it) {
+            if (ahead.more() && !fetch_rows()) { ok = false; break; }
+            if (!warp_wait(&sh->dq_full, it & 1, lane)) { if (lane == 0) fail_bwd(sh, 16); ok = false; break; }
+            tc_fence_after();
+            // 32 columns at a time through the exchange buffer: a reduction then covers 4 rows x 128 bytes
+            const int64_t q0 = (int64_t)walk.qt * TILE + r0;
+            const int sub = lane >> 3, col = (lane & 7) * 4;
+            float* acc = p.dq_acc + (((int64_t)b * p.h + walk.head) * p.sq + q0) * p.d + col;
+            uint32_t r[2][32];
+            tmem_ld32(tmem + lane_addr + C_DQ, r[0]);
+#pragma unroll
+            for (int c4 = 0; c4 < HD / 32; ++c4) {
+                if (c4 * 32 >= p.d) break;
+                tmem_ld_wait();
+                if ((c4 + 1) * 32 < p.d) {
+                    if (c4 + 1 < HD / 32) tmem_ld32(tmem + lane_addr + C_DQ + (c4 + 1) * 32, r[(c4 + 1) & 1]);
+                } else {                     // all columns have left the tensor memory
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh->dq_empty);
+                }
+                const uint32_t srow = xbuf + (uint32_t)lane * 128;
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(srow + (uint32_t)((q ^ (lane & 7)) << 4)), "r"(r[c4 & 1][4 * q]),
+                                 "r"(r[c4 & 1][4 * q + 1]), "r"(r[c4 & 1][4 * q + 2]), "r"(r[c4 & 1][4 * q + 3]) : "memory");
+                __syncwarp();
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    const int rl = g * 4 + sub;
+                    float v0, v1, v2, v3;
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v0), "=f"(v1), "=f"(v2), "=f"(v3)
+                                 : "r"(xbuf + (uint32_t)(rl * 128 + (((lane & 7) ^ (rl & 7)) << 4))) : "memory");
+                    if (q0 + rl < p.sq && c4 * 32 + col < p.d) red_add_v4(acc + (int64_t)rl * p.d + c4 * 32, v0, v1, v2, v3);
+                }
+                __syncwarp();
+            }
+        }
     }
 
     __syncthreads();
@@ -655,40 +932,42 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-// delta[b, h, q] = sum_d dO[b, q, h, d] * O[b, q, h, d]; one warp per row
+// delta[b, h, q] = sum_d dO[b, q, h, d] * O[b, q, h, d], and zeros in the same row of the dQ accumulator (b, h, sq, d); 16
+// lanes per row (head dims up to 128 are 16 vectors of 8), two rows per warp.
 template <typename T>
 __global__ void attn_delta_kernel(const T* o, int64_t o_tok, int64_t o_head, int64_t o_batch, const T* dout, int64_t g_tok, int64_t g_head,
-                                  int64_t g_batch, float* delta, int64_t batch, int64_t sq, int h, int d) {
-    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= batch * sq * h) return;
-    const int head = (int)(w % h);
-    const int64_t qi = (w / h) % sq, bb = w / ((int64_t)h * sq);
-    const T* orow = o + bb * o_batch + qi * o_tok + head * o_head;
-    const T* grow = dout + bb * g_batch + qi * g_tok + head * g_head;
+                                  int64_t g_batch, float* delta, float* dq_acc, int64_t rows, int64_t sq, int h, int d) {
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+    const int c = (threadIdx.x & 15) * 8;
+    const bool ok = w < rows;
+    const int64_t tok = ok ? w / h : 0;
+    const int head = ok ? (int)(w - tok * h) : 0;
+    const int64_t bb = tok / sq, qi = tok - bb * sq, row = (bb * h + head) * sq + qi;
     float acc = 0.f;
-    for (int c = lane * 8; c < d; c += 256) {
-        const bmt::Vec16<T> a = bmt::ld16(orow + c), g = bmt::ld16(grow + c);
+    if (ok && c < d) {
+        const bmt::Vec16<T> a = bmt::ld16(o + bb * o_batch + qi * o_tok + head * o_head + c), g = bmt::ld16(dout + bb * g_batch + qi * g_tok + head * g_head + c);
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc += bmt::Cvt<T>::to_f(a.v[i]) * bmt::Cvt<T>::to_f(g.v[i]);
+        float4* z = reinterpret_cast<float4*>(dq_acc + row * d + c);
+        z[0] = z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-    if (lane == 0) delta[(bb * h + head) * sq + qi] = acc;
+    for (int s = 8; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    if (ok && c == 0) delta[row] = acc;
 }
 
-// dq[b, q, h, :] (strided, T) <- dq_acc (b, sq, h, d) fp32
+// dq[b, q, h, :] (strided, T) <- dq_acc (b, h, sq, d) fp32
 template <typename T>
-__global__ void attn_dq_convert_kernel(const float* acc, T* dq, int64_t q_tok, int64_t q_head, int64_t q_batch, int64_t batch, int64_t sq,
+__global__ void attn_dq_convert_kernel(const float* acc, T* dq, int64_t q_tok, int64_t q_head, int64_t q_batch, int64_t rows, int64_t sq,
                                        int h, int d) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;   // one 8-element vector per thread
-    const int per_row = d / 8;
-    if (v >= batch * sq * h * per_row) return;
-    const int c = (int)(v % per_row) * 8;
-    const int64_t r = v / per_row;
-    const int head = (int)(r % h);
-    const int64_t qi = (r / h) % sq, bb = r / ((int64_t)h * sq);
-    const float4 a0 = *reinterpret_cast<const float4*>(acc + r * d + c), a1 = *reinterpret_cast<const float4*>(acc + r * d + c + 4);
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+    const int c = (threadIdx.x & 15) * 8;
+    if (w >= rows || c >= d) return;
+    const int64_t tok = w / h;
+    const int head = (int)(w - tok * h);
+    const int64_t bb = tok / sq, qi = tok - bb * sq;
+    const float4* src = reinterpret_cast<const float4*>(acc + ((bb * h + head) * sq + qi) * d + c);
+    const float4 a0 = src[0], a1 = src[1];
     bmt::Vec16<T> o;
     o.v[0] = bmt::Cvt<T>::from_f(a0.x); o.v[1] = bmt::Cvt<T>::from_f(a0.y); o.v[2] = bmt::Cvt<T>::from_f(a0.z); o.v[3] = bmt::Cvt<T>::from_f(a0.w);
     o.v[4] = bmt::Cvt<T>::from_f(a1.x); o.v[5] = bmt::Cvt<T>::from_f(a1.y); o.v[6] = bmt::Cvt<T>::from_f(a1.z); o.v[7] = bmt::Cvt<T>::from_f(a1.w);
@@ -699,14 +978,14 @@ template <int HD, typename T>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const AttnBwdParams& p,
                int64_t batch, cudaStream_t stream) {
     constexpr uint32_t TB = (HD / 64) * CHUNK;
-    const size_t smem = 4 * TB + 4 * CHUNK + sizeof(BwdShared) + 1024;
+    const size_t smem = 5 * TB + 2 * CHUNK + 4 * 32 * 128 + sizeof(BwdShared) + 1024;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(flash_bwd_kernel<HD, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -30;
         configured = true;
     }
-    dim3 grid((unsigned)((p.sk + TILE - 1) / TILE), (unsigned)p.hk, (unsigned)batch);
-    flash_bwd_kernel<HD, T><<<grid, ATT_THREADS, smem, stream>>>(tq, tk, tv, tdo, p);
+    dim3 grid((unsigned)(p.hk * batch), (unsigned)p.k_tiles);
+    flash_bwd_kernel<HD, T><<<grid, BWD_THREADS, smem, stream>>>(tq, tk, tv, tdo, p);
     bmt_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
@@ -715,7 +994,7 @@ template <typename T>
 int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const void* q, const int64_t* qs, const void* k, const int64_t* ks,
             const void* v, const int64_t* vs, const void* o, const int64_t* os, const void* dout, const int64_t* gs, const void* lse,
             void* dq, const int64_t* dqs, void* dk, const int64_t* dks, void* dv, const int64_t* dvs, void* dq_acc, void* delta, float scale,
-            int causal, const void* mask, const void* kv_lens, int dtype, cudaStream_t st) {
+            int causal, const void* mask_bits_t, const void* mask_cls, const void* kv_lens, int dtype, cudaStream_t st) {
     const int hd = d <= 64 ? 64 : 128;
     CUtensorMap tq, tk, tv, tdo;
     int rc;
@@ -724,28 +1003,28 @@ int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const v
     if ((rc = bmt_tma_map_4d(&tv, v, dtype, d, sk, vs[0], hk, vs[1], batch, vs[2], 64, TILE)) != 0) return rc;
     if ((rc = bmt_tma_map_4d(&tdo, dout, dtype, d, sq, gs[0], h, gs[1], batch, gs[2], 64, TILE)) != 0) return rc;
     const int64_t rows = batch * sq * h;
-    if (cudaMemsetAsync(dq_acc, 0, (size_t)rows * d * sizeof(float), st) != cudaSuccess) return -32;
-    attn_delta_kernel<T><<<(unsigned)((rows * 32 + 255) / 256), 256, 0, st>>>((const T*)o, os[0], os[1], os[2], (const T*)dout, gs[0], gs[1],
-                                                                                gs[2], (float*)delta, batch, sq, h, d);
+    const unsigned row_blocks = (unsigned)((rows * 16 + 255) / 256);
+    attn_delta_kernel<T><<<row_blocks, 256, 0, st>>>((const T*)o, os[0], os[1], os[2], (const T*)dout, gs[0], gs[1], gs[2], (float*)delta,
+                                                     (float*)dq_acc, rows, sq, h, d);
     AttnBwdParams p;
     memset(&p, 0, sizeof(p));
     p.sq = sq; p.sk = sk; p.h = h; p.hk = hk; p.d = d;
     p.scale = scale; p.sl2 = scale * 1.4426950408889634f;
     p.causal = causal; p.causal_off = sk - sq;
-    p.mask = (const uint8_t*)mask; p.kv_lens = (const int32_t*)kv_lens;
+    p.bits_t = (const uint32_t*)mask_bits_t; p.cls = (const uint8_t*)mask_cls; p.kv_lens = (const int32_t*)kv_lens;
+    p.q_tiles = (int)((sq + TILE - 1) / TILE); p.k_tiles = (int)((sk + TILE - 1) / TILE);
     p.lse = (const float*)lse; p.delta = (const float*)delta; p.dq_acc = (float*)dq_acc;
     p.dk = dk; p.dk_tok = dks[0]; p.dk_head = dks[1]; p.dk_batch = dks[2];
     p.dv = dv; p.dv_tok = dvs[0]; p.dv_head = dvs[1]; p.dv_batch = dvs[2];
     const uint32_t fmt = dtype == BMT_DT_F16 ? 0u : 1u;
     const uint32_t common = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(TILE >> 4) << 24);
     p.idesc_s = common | ((uint32_t)(TILE >> 3) << 17);
-    p.idesc_tn = common | (1u << 15) | (1u << 16) | ((uint32_t)(hd >> 3) << 17);
-    p.idesc_dq = common | (1u << 16) | ((uint32_t)(hd >> 3) << 17);
+    p.idesc_dv = common | (1u << 16) | ((uint32_t)(d >> 3) << 17);              // A K-major (or tensor memory), B MN-major, N = head dim
+    p.idesc_dq = common | (1u << 15) | (1u << 16) | ((uint32_t)(d >> 3) << 17);  // A and B MN-major
     rc = hd == 64 ? launch_bwd<64, T>(tq, tk, tv, tdo, p, batch, st) : launch_bwd<128, T>(tq, tk, tv, tdo, p, batch, st);
     if (rc != 0) return rc;
-    const int64_t vecs = rows * (d / 8);
-    attn_dq_convert_kernel<T><<<(unsigned)((vecs + 255) / 256), 256, 0, st>>>((const float*)dq_acc, (T*)dq, dqs[0], dqs[1], dqs[2], batch, sq, h, d);
-    bmt_count_launch(3);
+    attn_dq_convert_kernel<T><<<row_blocks, 256, 0, st>>>((const float*)dq_acc, (T*)dq, dqs[0], dqs[1], dqs[2], rows, sq, h, d);
+    bmt_count_launch(2);
     return cudaGetLastError() == cudaSuccess ? 0 : -33;
 }
 
@@ -753,11 +1032,12 @@ int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const v
 
 // q (b, sq, h, d), k / v (b, sk, hk, d), o (b, sq, h, d): element strides given per tensor as {token, head, batch}, the
 // head dim is contiguous.  d: multiple of 16, at most 128; every stride a multiple of 8, pointers 16-byte aligned.
-// lse (b, h, sq) fp32 or NULL.  mask: (b, sq, sk) bytes or NULL; kv_lens: (b) int32 or NULL.
+// lse (b, h, sq) fp32 or NULL.  mask_bits, mask_cls: a dense mask as bmt_attn_mask_pack wrote it, or NULL; kv_lens: (b) int32
+// or NULL.
 extern "C" int bmt_flash_attn_fwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const void* q, const int64_t* q_strides,
                                   const void* k, const int64_t* k_strides, const void* v, const int64_t* v_strides, void* o,
-                                  const int64_t* o_strides, void* lse, float scale, int causal, const void* mask, const void* kv_lens,
-                                  int dtype, void* stream) {
+                                  const int64_t* o_strides, void* lse, float scale, int causal, const void* mask_bits,
+                                  const void* mask_cls, const void* kv_lens, int dtype, void* stream) {
     if (d <= 0 || d > 128 || (d & 15) || h % hk || batch <= 0 || sq <= 0 || sk <= 0) return -1;
     if (((uintptr_t)o & 15) || (o_strides[0] & 7) || (o_strides[1] & 7) || (o_strides[2] & 7)) return -2;
     const int hd = d <= 64 ? 64 : 128;
@@ -771,17 +1051,41 @@ extern "C" int bmt_flash_attn_fwd(int64_t batch, int64_t sq, int64_t sk, int h, 
     p.sq = sq; p.sk = sk; p.h = h; p.hk = hk; p.d = d;
     p.sl2 = scale * 1.4426950408889634f;
     p.causal = causal; p.causal_off = sk - sq;
-    p.mask = (const uint8_t*)mask; p.kv_lens = (const int32_t*)kv_lens;
+    p.bits = (const uint32_t*)mask_bits; p.cls = (const uint8_t*)mask_cls; p.kv_lens = (const int32_t*)kv_lens;
+    p.q_tiles = (int)((sq + TILE - 1) / TILE); p.k_tiles = (int)((sk + TILE - 1) / TILE);
     p.o = o; p.o_tok = o_strides[0]; p.o_head = o_strides[1]; p.o_batch = o_strides[2];
     p.lse = (float*)lse;
     const uint32_t fmt = dtype == BMT_DT_F16 ? 0u : 1u;
     const uint32_t common = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(TILE >> 4) << 24);
     p.idesc_s = common | ((uint32_t)(TILE >> 3) << 17);                       // A, B K-major; N = 128 keys
-    p.idesc_pv = common | (1u << 16) | ((uint32_t)(hd >> 3) << 17);           // B (V) MN-major; N = padded head dim
+    p.idesc_pv = common | (1u << 16) | ((uint32_t)(d >> 3) << 17);            // B (V) MN-major; N = head dim
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == BMT_DT_F16) return hd == 64 ? launch_fwd<64, __half>(tq, tk, tv, p, batch, st) : launch_fwd<128, __half>(tq, tk, tv, p, batch, st);
     if (dtype == BMT_DT_BF16) return hd == 64 ? launch_fwd<64, __nv_bfloat16>(tq, tk, tv, p, batch, st) : launch_fwd<128, __nv_bfloat16>(tq, tk, tv, p, batch, st);
     return -3;
+}
+
+// Bytes of a packed mask, and where its three parts start: bits at 0, bits_t and cls at the returned offsets.
+extern "C" int64_t bmt_attn_mask_layout(int64_t batch, int64_t sq, int64_t sk, int64_t* bits_t_off, int64_t* cls_off) {
+    const int64_t qt = (sq + TILE - 1) / TILE, kt = (sk + TILE - 1) / TILE;
+    const int64_t t_off = batch * sq * kt * 16, c_off = t_off + batch * sk * qt * 16;
+    if (bits_t_off) *bits_t_off = t_off;
+    if (cls_off) *cls_off = c_off;
+    return c_off + batch * qt * kt;
+}
+
+// Packs a dense mask (batch, sq, sk) of bytes (non-zero = attend) for the attention kernels; `packed` is 16-byte aligned and
+// has the size that bmt_attn_mask_layout gives.
+extern "C" int bmt_attn_mask_pack(int64_t batch, int64_t sq, int64_t sk, const void* mask, void* packed, void* stream) {
+    if (batch <= 0 || sq <= 0 || sk <= 0 || ((uintptr_t)packed & 15)) return -1;
+    const int64_t qt = (sq + TILE - 1) / TILE, kt = (sk + TILE - 1) / TILE;
+    if (qt > 65535 || batch > 65535) return -2;
+    int64_t t_off, c_off;
+    bmt_attn_mask_layout(batch, sq, sk, &t_off, &c_off);
+    attn_mask_pack_kernel<<<dim3((unsigned)kt, (unsigned)qt, (unsigned)batch), MASK_THREADS, 0, (cudaStream_t)stream>>>(
+        (const uint8_t*)mask, sq, sk, (uint32_t*)packed, (uint32_t*)((char*)packed + t_off), (uint8_t*)packed + c_off);
+    bmt_count_launch(1);
+    return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
 
 // status of the attention kernels: 0, or (wait code << 16 | CTA) of the first CTA that gave up; reading clears it
@@ -799,8 +1103,8 @@ extern "C" int bmt_flash_attn_bwd(int64_t batch, int64_t sq, int64_t sk, int h, 
                                   const void* k, const int64_t* k_strides, const void* v, const int64_t* v_strides, const void* o,
                                   const int64_t* o_strides, const void* dout, const int64_t* do_strides, const void* lse, void* dq,
                                   const int64_t* dq_strides, void* dk, const int64_t* dk_strides, void* dv, const int64_t* dv_strides,
-                                  void* dq_acc, void* delta, float scale, int causal, const void* mask, const void* kv_lens, int dtype,
-                                  void* stream) {
+                                  void* dq_acc, void* delta, float scale, int causal, const void* mask_bits_t,
+                                  const void* mask_cls, const void* kv_lens, int dtype, void* stream) {
     if (d <= 0 || d > 128 || (d & 15) || h % hk || batch <= 0 || sq <= 0 || sk <= 0) return -1;
     const int64_t* all[] = {o_strides, dq_strides, dk_strides, dv_strides};
     for (const int64_t* s3 : all)
@@ -809,9 +1113,9 @@ extern "C" int bmt_flash_attn_bwd(int64_t batch, int64_t sq, int64_t sk, int h, 
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == BMT_DT_F16)
         return run_bwd<__half>(batch, sq, sk, h, hk, d, q, q_strides, k, k_strides, v, v_strides, o, o_strides, dout, do_strides, lse, dq,
-                               dq_strides, dk, dk_strides, dv, dv_strides, dq_acc, delta, scale, causal, mask, kv_lens, dtype, st);
+                               dq_strides, dk, dk_strides, dv, dv_strides, dq_acc, delta, scale, causal, mask_bits_t, mask_cls, kv_lens, dtype, st);
     if (dtype == BMT_DT_BF16)
         return run_bwd<__nv_bfloat16>(batch, sq, sk, h, hk, d, q, q_strides, k, k_strides, v, v_strides, o, o_strides, dout, do_strides, lse,
-                                      dq, dq_strides, dk, dk_strides, dv, dv_strides, dq_acc, delta, scale, causal, mask, kv_lens, dtype, st);
+                                      dq, dq_strides, dk, dk_strides, dv, dv_strides, dq_acc, delta, scale, causal, mask_bits_t, mask_cls, kv_lens, dtype, st);
     return -3;
 }

@@ -41,6 +41,14 @@ Dims dims_of(const BmtGptBlock& k) {
 const char* off(const void* p, int64_t elems) { return (const char*)p + elems * 2; }
 char* off(void* p, int64_t elems) { return (char*)p + elems * 2; }
 
+// Part 0 (by query), 1 (by key) or 2 (tile classes) of the packed mask of the fused attention, or null.
+const void* mask_part(const BmtGptBlock& k, const Dims& q, int part) {
+    if (!k.mask_packed) return nullptr;
+    int64_t at[3] = {0, 0, 0};
+    bmt_attn_mask_layout(q.b, q.s, q.s, &at[1], &at[2]);
+    return (const char*)k.mask_packed + at[part];
+}
+
 }  // namespace
 
 // Steps [first_step, last_step] of the forward (1 = LN1, 2 = QKV projection, 3..5 attention core, 6 = output
@@ -63,10 +71,11 @@ extern "C" int bmt_gpt_block_forward_steps(const BmtGptBlock* blk, int first_ste
     // 3-5 as one fused attention kernel: q, k, v are strided views of the packed projection, nothing of size s x s is stored
     if (k.lse) {
         STEP(3) {
+            if (k.mask_packed) RUN(bmt_attn_mask_pack(q.b, q.s, q.s, k.mask, k.mask_packed, stream));
             const int64_t in_str[3] = {tok, head, q.s * tok}, out_str[3] = {q.hd, q.dh, q.s * q.hd};
             RUN(bmt_flash_attn_fwd(q.b, q.s, q.s, (int)q.h, (int)q.h, (int)q.dh, k.qkv, in_str, off(k.qkv, q.dh), in_str,
-                                   off(k.qkv, 2 * q.dh), in_str, k.ctx, out_str, k.lse, 1.f / sqrtf((float)q.dh), k.causal, k.mask,
-                                   nullptr, dt, stream));
+                                   off(k.qkv, 2 * q.dh), in_str, k.ctx, out_str, k.lse, 1.f / sqrtf((float)q.dh), k.causal,
+                                   mask_part(k, q, 0), mask_part(k, q, 2), nullptr, dt, stream));
         }
     } else {
     // 3. scores = q k^T / sqrt(d_head)   -> probs (b, h, s, ld)
@@ -165,7 +174,7 @@ extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockG
         RUN(bmt_flash_attn_bwd(q.b, q.s, q.s, (int)q.h, (int)q.h, (int)q.dh, k.qkv, in_str, off(k.qkv, q.dh), in_str,
                                off(k.qkv, 2 * q.dh), in_str, k.ctx, out_str, w.d_ctx, out_str, k.lse, w.d_qkv, in_str,
                                off(w.d_qkv, q.dh), in_str, off(w.d_qkv, 2 * q.dh), in_str, w.dq_acc, w.delta,
-                               1.f / sqrtf((float)q.dh), k.causal, k.mask, nullptr, dt, stream));
+                               1.f / sqrtf((float)q.dh), k.causal, mask_part(k, q, 1), mask_part(k, q, 2), nullptr, dt, stream));
     } else {
     {   // dP = d_ctx v^T
         BmtGemmDesc g = plain(q.s, q.s, q.dh, w.d_ctx, q.hd, 0, off(k.qkv, 2 * q.dh), tok, 0, w.d_probs, pl, dt);

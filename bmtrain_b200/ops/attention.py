@@ -66,26 +66,59 @@ def flash_usable(q, k, v) -> bool:
     return True
 
 
-def flash_forward(q, k, v, scale, causal, mask8, lens32):
-    """Fused forward: returns ``(o (b, sq, h, d), lse (b, h, sq) fp32)``."""
+def packed_mask_buffer(b: int, sq: int, sk: int, device) -> torch.Tensor:
+    """Room for a dense mask as bits: by query, by key, and a class per 128 x 128 tile (``bmt_attn_mask_pack``)."""
+    qt, kt = (sq + 127) // 128, (sk + 127) // 128
+    return torch.empty(b * (16 * (sq * kt + sk * qt) + qt * kt), dtype=torch.uint8, device=device)
+
+
+def pack_mask(mask8: Optional[torch.Tensor], b: int, sq: int, sk: int) -> Optional[torch.Tensor]:
+    """A (b, sq, sk) byte mask in the form the fused kernels read (once per call instead of once per head), or None."""
+    if mask8 is None:
+        return None
+    mask8 = mask8.reshape(b, sq, sk).contiguous()
+    packed = packed_mask_buffer(b, sq, sk, mask8.device)
+    _native.check(_native.cuda_lib().bmt_attn_mask_pack(
+        ctypes.c_int64(b), ctypes.c_int64(sq), ctypes.c_int64(sk), _native.ptr(mask8), _native.ptr(packed),
+        _native.stream_handle()), "attention mask packing")
+    return packed
+
+
+def _mask_parts(packed, b, sq, sk):
+    """Pointers to the three parts of a packed mask (null without one)."""
+    if packed is None:
+        return (ctypes.c_void_p(0),) * 3
+    qt, kt = (sq + 127) // 128, (sk + 127) // 128
+    at = packed.data_ptr()
+    by_key = at + b * sq * kt * 16
+    return ctypes.c_void_p(at), ctypes.c_void_p(by_key), ctypes.c_void_p(by_key + b * sk * qt * 16)
+
+
+def flash_forward(q, k, v, scale, causal, mask8, lens32, packed=None):
+    """Fused forward: returns ``(o (b, sq, h, d), lse (b, h, sq) fp32)``.  ``packed``: what ``pack_mask`` made of it when the caller
+    has it already."""
     lib = _native.cuda_lib()
     b, sq, h, d = q.shape
     sk, hk = k.shape[1], k.shape[2]
+    packed = pack_mask(mask8, b, sq, sk) if packed is None else packed
+    bits, _, classes = _mask_parts(packed, b, sq, sk)
     o = torch.empty(b, sq, h, d, dtype=q.dtype, device=q.device)
     lse = torch.empty(b, h, sq, dtype=torch.float32, device=q.device)
     _native.check(lib.bmt_flash_attn_fwd(
         ctypes.c_int64(b), ctypes.c_int64(sq), ctypes.c_int64(sk), ctypes.c_int(h), ctypes.c_int(hk), ctypes.c_int(d),
         _native.ptr(q), _strides3(q), _native.ptr(k), _strides3(k), _native.ptr(v), _strides3(v), _native.ptr(o), _strides3(o),
-        _native.ptr(lse), ctypes.c_float(scale), ctypes.c_int(1 if causal else 0), _native.ptr(mask8), _native.ptr(lens32),
+        _native.ptr(lse), ctypes.c_float(scale), ctypes.c_int(1 if causal else 0), bits, classes, _native.ptr(lens32),
         ctypes.c_int(_DT[q.dtype]), _native.stream_handle()), "fused attention forward")
     return o, lse
 
 
-def flash_backward(q, k, v, o, lse, do, scale, causal, mask8, lens32):
+def flash_backward(q, k, v, o, lse, do, scale, causal, mask8, lens32, packed=None):
     """Fused backward: returns ``(dq, dk, dv)`` shaped like ``q, k, v`` (contiguous)."""
     lib = _native.cuda_lib()
     b, sq, h, d = q.shape
     sk, hk = k.shape[1], k.shape[2]
+    packed = pack_mask(mask8, b, sq, sk) if packed is None else packed
+    _, bits_t, classes = _mask_parts(packed, b, sq, sk)
     dq = torch.empty(b, sq, h, d, dtype=q.dtype, device=q.device)
     dk = torch.empty(b, sk, hk, d, dtype=q.dtype, device=q.device)
     dv = torch.empty(b, sk, hk, d, dtype=q.dtype, device=q.device)
@@ -96,7 +129,7 @@ def flash_backward(q, k, v, o, lse, do, scale, causal, mask8, lens32):
         _native.ptr(q), _strides3(q), _native.ptr(k), _strides3(k), _native.ptr(v), _strides3(v), _native.ptr(o), _strides3(o),
         _native.ptr(do), _strides3(do), _native.ptr(lse), _native.ptr(dq), _strides3(dq), _native.ptr(dk), _strides3(dk),
         _native.ptr(dv), _strides3(dv), _native.ptr(dq_acc), _native.ptr(delta), ctypes.c_float(scale),
-        ctypes.c_int(1 if causal else 0), _native.ptr(mask8), _native.ptr(lens32), ctypes.c_int(_DT[q.dtype]),
+        ctypes.c_int(1 if causal else 0), bits_t, classes, _native.ptr(lens32), ctypes.c_int(_DT[q.dtype]),
         _native.stream_handle()), "fused attention backward")
     return dq, dk, dv
 
@@ -118,9 +151,11 @@ class AttentionFunction(torch.autograd.Function):
         m8, l32 = _softmax_args(mask, kv_lens)
         ctx.scale, ctx.group, ctx.causal = scale, group, causal
         if flash_usable(q, k, v):
-            o, lse = flash_forward(q, k, v, scale, causal, m8, l32)
-            # nothing of size sq x sk is kept: backward rebuilds the probabilities tile by tile from q, k and lse
-            ctx.save_for_backward(q, k, v, o, lse, m8, l32)
+            packed = pack_mask(m8, b, sq, sk)
+            o, lse = flash_forward(q, k, v, scale, causal, None, l32, packed)
+            # nothing of size sq x sk is kept (a dense mask as bits): backward rebuilds the probabilities tile by tile from
+            # q, k and lse
+            ctx.save_for_backward(q, k, v, o, lse, packed, l32)
             ctx.fused = True
             return o
         assert d % 8 == 0, "head dimension must be a multiple of 8"
@@ -149,11 +184,11 @@ class AttentionFunction(torch.autograd.Function):
     def backward(ctx, do):
         lib = _native.cuda_lib()
         if ctx.fused:
-            q, k, v, o, lse, m8, l32 = ctx.saved_tensors
+            q, k, v, o, lse, packed, l32 = ctx.saved_tensors
             do = do.contiguous()
             if do.data_ptr() % 16:
                 do = do.clone()
-            dq, dk, dv = flash_backward(q, k, v, o, lse, do, ctx.scale, ctx.causal, m8, l32)
+            dq, dk, dv = flash_backward(q, k, v, o, lse, do, ctx.scale, ctx.causal, None, l32, packed)
             return dq, dk, dv, None, None, None, None
         q, k, v, p = ctx.saved_tensors
         b, sq, h, d = q.shape

@@ -13,6 +13,7 @@ from typing import Optional
 import torch
 
 from . import _native
+from . import attention as _attn
 from . import gemm as _gemm
 from . import grad_slot as _grad_slot
 
@@ -29,7 +30,7 @@ class _Block(ctypes.Structure):
         ("x", _c_void_p), ("y", _c_void_p),
         ("ln1", _c_void_p), ("stats1", _c_void_p), ("qkv", _c_void_p), ("probs", _c_void_p), ("probs_ld", _i64),
         ("ctx", _c_void_p), ("h1", _c_void_p), ("ln2", _c_void_p), ("stats2", _c_void_p), ("ff", _c_void_p), ("pre", _c_void_p),
-        ("lse", _c_void_p),
+        ("lse", _c_void_p), ("mask_packed", _c_void_p),
     ]
 
 
@@ -77,6 +78,8 @@ def _fill(blk: _Block, x, y, mask, params, saved, n_heads, d_head, act, eps, cau
         blk.lse, blk.probs, blk.probs_ld = saved["lse"].data_ptr(), None, 0
     else:
         blk.lse, blk.probs, blk.probs_ld = None, saved["probs"].data_ptr(), saved["probs"].stride(2)
+    packed = saved.get("mask_packed")
+    blk.mask_packed = None if packed is None else packed.data_ptr()
     blk.pre = saved["pre"].data_ptr() if saved.get("pre") is not None else None
 
 
@@ -102,6 +105,7 @@ class GPTBlockFunction(torch.autograd.Function):
             "ln2": torch.empty(T, d, dtype=dt, device=dev), "stats2": torch.empty(2, T, dtype=torch.float32, device=dev),
             "ff": torch.empty(T, dff, dtype=dt, device=dev),
             "pre": torch.empty(T, dff, dtype=dt, device=dev) if act == "gelu" else None,
+            "mask_packed": _attn.packed_mask_buffer(b, s, s, dev) if fused_attn and mask8 is not None else None,
         }
         y = torch.empty_like(x)
         blk = _Block()
