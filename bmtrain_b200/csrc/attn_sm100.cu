@@ -20,7 +20,7 @@ namespace {
 
 using namespace bmt_tc;
 
-constexpr int FWD_THREADS = 320;                 // producer, MMA issuer, two groups of four softmax warps
+constexpr int FWD_THREADS = 384;                 // two groups of four softmax warps, producer, MMA issuer (a warpgroup of their own)
 constexpr int TILE = 128;                        // query rows per CTA and keys per step
 constexpr uint32_t CHUNK = TILE * 64 * 2;        // one [128 rows][64 columns] swizzled chunk of 16-bit elements: 16 KiB
 
@@ -72,6 +72,11 @@ __device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 // A from tensor memory: lane = row, every column holds two consecutive 16-bit elements of the reduction dimension.
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_c, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -85,6 +90,11 @@ __device__ __forceinline__ void fail(AttnShared* sh, int code) {
     sh->failed = 1;
     atomicCAS(&g_attn_status, 0, (code << 16) | (int)(blockIdx.x & 0xffff));
 }
+
+// Register split: a warpgroup hands registers back or takes more.  The shares of all warpgroups stay within what the block was
+// launched with.
+template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // one lane polls, the warp follows
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int lane) {
@@ -167,9 +177,10 @@ attn_mask_pack_kernel(const uint8_t* mask, int64_t sq, int64_t sk, uint32_t* bit
 
 // Forward.  A CTA works on two tiles of 128 query rows (one when the grid would not fill the GPU) with a group of four
 // softmax warps each, so that the tensor core multiplies for one tile while the other one is in its softmax:
-//   warp 0      TMA producer: both Q tiles once, then K and V tiles of 128 keys through two-stage rings (shared by both)
-//   warp 1      MMA issuer: S_t = Q_t K^T into tensor memory, O_t += P_t V with P_t read from tensor memory
-//   warps 2..5 / 6..9   softmax of tile 0 / 1: one thread per query row reads its row of S from tensor memory, applies the
+//   warps 0..3 / 4..7   softmax of tile 0 / 1 (below)
+//   warp 8      TMA producer: both Q tiles once, then K and V tiles of 128 keys through two-stage rings (shared by both)
+//   warp 9      MMA issuer: S_t = Q_t K^T into tensor memory, O_t += P_t V with P_t read from tensor memory
+//   softmax     one thread per query row reads its row of S from tensor memory, applies the
 //               masks, and writes the probabilities back over it as packed 16-bit pairs, where the MMA takes them from.
 // What bounds it: a 128 x 128 tile at head dim 128 is 1024 clocks of MMA and 1024 clocks of ex2 (16 per clock and SM); with
 // one tile per CTA, and P going through shared memory, the two and everything in between took turns (about 4500 clocks).
@@ -218,14 +229,16 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         sh->failed = 0;
         fence_barrier_init();
     }
-    if (warp == 1) { tmem_alloc(&sh->tmem_base, 512); tmem_relinquish(); }
+    if (warp == 9) { tmem_alloc(&sh->tmem_base, 512); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;            // S_0 / P_0 [0,128), S_1 / P_1 [128,256), O_0 [256,384), O_1 [384,512)
     const int first = next_step(-1);
 
-    if (warp == 0) {
+    if (warp >= 8) {
+    regs_down<56>();             // 128 x 56 + 256 x 216 of the 384 x 168 registers at launch
+    if (warp == 8) {
         // ------------------------------------------------------------------------------------------ TMA producer
         if (first < J_max) {
             const uint32_t qbar = smem_u32(&sh->q_full);
@@ -260,7 +273,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 __syncwarp();
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == 9) {
         // ------------------------------------------------------------------------------------------ MMA issuer
         // the warp stays converged and one elected lane issues (operands in uniform registers)
         if (first < J_max) {
@@ -334,9 +347,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 ++n;
             }
         }
+    }
     } else {
         // ------------------------------------------------------------------------------------------ softmax + epilogue
-        const int t = (warp - 2) >> 2, quarter = warp & 3;      // TMEM lanes [32 * quarter, 32 * quarter + 32) belong to this warp
+        regs_up<216>();
+        const int t = warp >> 2, quarter = warp & 3;      // TMEM lanes [32 * quarter, 32 * quarter + 32) belong to this warp
         const int row = quarter * 32 + lane;
         const int64_t q0 = (int64_t)(qt0 + t) * TILE, qi = q0 + row;
         const bool row_ok = qi < p.sq;
@@ -482,7 +497,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         __syncthreads();
     }
     tc_fence_after();
-    if (warp == 1) tmem_dealloc(tmem, 512);
+    if (warp == 9) tmem_dealloc(tmem, 512);
 }
 
 int sm_count() {
@@ -520,7 +535,8 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
 //         tensor memory as packed 16-bit pairs, over S^T; dS = P * (dP - delta) * scale as 16 bits into shared memory,
 //         [key][query] swizzled: K-major A for dK and, read "transposed", MN-major A for dQ = dS K
 //   MMA   dV += P^T dO (P from tensor memory), dK += dS^T Q, dQ = dS K
-//   dQ warps (4): add the tile of dQ to an fp32 accumulator in global memory (vector reductions); a small kernel converts it
+//   dQ warps (4): add the tile of dQ to an fp32 accumulator in global memory (bulk reductions out of shared memory, 32 columns
+//         at a time; vector reductions by the threads themselves took 4300 clocks a tile); a small kernel converts it
 // delta = rowsum(dO * O) comes from a pre-pass.  dK / dV are written once at the end, already summed over the group.
 // Order on the tensor pipe, which bounds a tile at 5 x 512 clocks (head dim 128): dP(i), dV(i), S(i+1), dK(i), dQ(i), dP(i+1):
 // while the softmax warps turn dP(i) into dS(i) the pipe has dV(i) and S(i+1) to do, and while it does dK(i) and dQ(i) they
@@ -545,12 +561,12 @@ struct AttnBwdParams {
     int q_tiles, k_tiles;
 };
 
-constexpr int BWD_THREADS = 448;                 // producer, MMA issuer, 8 softmax warps, 4 dQ warps
+constexpr int BWD_THREADS = 512;                 // 8 softmax warps, 4 dQ warps, producer and MMA issuer (a warpgroup of their own)
 
 struct BwdShared {
-    uint64_t kv_full, q_full[2], q_empty[2], do_full, do_empty, s_full, dp_full, p_ready, ds_ready, dq_full, dq_empty, all_done;
+    alignas(16) uint64_t kv_full; uint64_t q_full[2], q_empty[2], do_full, do_empty, s_full, dp_full, p_ready, ds_ready, dq_full, dq_empty, all_done;
     uint64_t row_full[2], row_empty[2], pair[4];
-    float nlse[2][TILE], delta[2][TILE];         // per query of a tile: -lse * log2(e) (0 for rows that take no part), delta
+    float nlse[2][TILE], ndelta[2][TILE];        // per query of a tile: -lse * log2(e) (0 for rows that take no part), -delta * scale
     uint32_t live[2][4];                         // queries of the tile that exist and see at least one key
     uint32_t tmem_base;
     int failed;
@@ -559,10 +575,6 @@ struct BwdShared {
 __device__ __forceinline__ void fail_bwd(BwdShared* sh, int code) {
     sh->failed = 1;
     atomicCAS(&g_attn_status, 0, ((0x40 | code) << 16) | (int)(blockIdx.x & 0xffff));
-}
-
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
 // Walks the (head, query tile) pairs of a CTA in order, leaving out tiles without a visible pair.
@@ -584,7 +596,7 @@ struct BwdWalk {
 template <int HD, typename T>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
-                 const __grid_constant__ CUtensorMap tdo, const AttnBwdParams p) {
+                 const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdq, const AttnBwdParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     constexpr int DC = HD / 64;
@@ -620,13 +632,15 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         sh->failed = 0;
         fence_barrier_init();
     }
-    if (warp == 1) { tmem_alloc(&sh->tmem_base, 512); tmem_relinquish(); }
+    if (warp == 13) { tmem_alloc(&sh->tmem_base, 512); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
 
-    if (warp == 0) {
+    if (warp >= 12) {
+    regs_down<48>();             // 128 x 48 + 384 x 152 of the 512 x 128 registers at launch
+    if (warp == 12) {
         // ------------------------------------------------------------------------------------------ TMA producer
         if (work) {
             const uint32_t kvbar = smem_u32(&sh->kv_full);
@@ -659,7 +673,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 __syncwarp();
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == 13) {
         // ------------------------------------------------------------------------------------------ MMA issuer
         if (work) {
             const uint32_t hi = desc_hi(1024);
@@ -725,14 +739,16 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 __syncwarp();
             }
         }
-    } else if (warp < 10) {
+    }
+    } else if (warp < 8) {
         // ------------------------------------------------------------------------------------------ softmax: P and dS
-        const int quarter = warp & 3, part = (warp - 2) >> 2;       // 32 keys, 64 queries of the tile
+        regs_up<152>();
+        const int quarter = warp & 3, part = warp >> 2;             // 32 keys, 64 queries of the tile
         const int row = quarter * 32 + lane;
         const int64_t kj = kv0 + row;                                // this thread's key
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         const uint4* brow = (p.bits_t && kj < p.sk) ? reinterpret_cast<const uint4*>(p.bits_t) + ((int64_t)b * p.sk + kj) * p.q_tiles : nullptr;
-        const uint64_t sl2_2 = pack_f2(p.sl2, p.sl2);
+        const uint64_t sl2_2 = pack_f2(p.sl2, p.sl2), scale_2 = pack_f2(p.scale, p.scale);
         bool ok = true;
         uint32_t it = 0;
         for (; walk.more() && ok; walk.next(), ++it) {
@@ -773,20 +789,20 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             float pr[64];
             uint32_t pk[32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const int u = i >> 4, k = (2 * i) & 31;
-                const float2 nl = *reinterpret_cast<const float2*>(&sh->nlse[st][part * 64 + 2 * i]);
-                float x, y;
-                unpack_f2(fma_f2(pack_f2(__uint_as_float(s[u][k]), __uint_as_float(s[u][k + 1])), sl2_2, pack_f2(nl.x, nl.y)), x, y);
-                x = ex2(x);
-                y = ex2(y);
-                if (need_mask) {
-                    if (!((vis[u] >> k) & 1u)) x = 0.f;
-                    if (!((vis[u] >> (k + 1)) & 1u)) y = 0.f;
+            for (int i = 0; i < 16; ++i) {
+                const int u = i >> 3, k = (4 * i) & 31;
+                const float4 nl = *reinterpret_cast<const float4*>(&sh->nlse[st][part * 64 + 4 * i]);
+                float x[4];
+                unpack_f2(fma_f2(pack_f2(__uint_as_float(s[u][k]), __uint_as_float(s[u][k + 1])), sl2_2, pack_f2(nl.x, nl.y)), x[0], x[1]);
+                unpack_f2(fma_f2(pack_f2(__uint_as_float(s[u][k + 2]), __uint_as_float(s[u][k + 3])), sl2_2, pack_f2(nl.z, nl.w)), x[2], x[3]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    x[e] = ex2(x[e]);
+                    if (need_mask && !((vis[u] >> (k + e)) & 1u)) x[e] = 0.f;
+                    pr[4 * i + e] = x[e];
                 }
-                pr[2 * i] = x;
-                pr[2 * i + 1] = y;
-                pk[i] = pack2<T>(x, y);
+                pk[2 * i] = pack2<T>(x[0], x[1]);
+                pk[2 * i + 1] = pack2<T>(x[2], x[3]);
             }
             tmem_st32(tmem + lane_addr + part * 32, pk);
             tmem_st_wait();
@@ -806,10 +822,15 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 for (int t = 0; t < 4; ++t) {
                     uint32_t w[4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int k = t * 8 + 2 * i, e = u * 32 + k;
-                        const float2 dl = *reinterpret_cast<const float2*>(&sh->delta[st][part * 64 + e]);
-                        w[i] = pack2<T>(pr[e] * (__uint_as_float(s[0][k]) - dl.x) * p.scale, pr[e + 1] * (__uint_as_float(s[0][k + 1]) - dl.y) * p.scale);
+                    for (int i = 0; i < 2; ++i) {
+                        const int k = t * 8 + 4 * i, e = u * 32 + k;
+                        const float4 nd = *reinterpret_cast<const float4*>(&sh->ndelta[st][part * 64 + e]);
+                        float a, c;
+                        // dS = P * (dP * scale - delta * scale)
+                        unpack_f2(mul_f2(pack_f2(pr[e], pr[e + 1]), fma_f2(pack_f2(__uint_as_float(s[0][k]), __uint_as_float(s[0][k + 1])), scale_2, pack_f2(nd.x, nd.y))), a, c);
+                        w[2 * i] = pack2<T>(a, c);
+                        unpack_f2(mul_f2(pack_f2(pr[e + 2], pr[e + 3]), fma_f2(pack_f2(__uint_as_float(s[0][k + 2]), __uint_as_float(s[0][k + 3])), scale_2, pack_f2(nd.z, nd.w))), a, c);
+                        w[2 * i + 1] = pack2<T>(a, c);
                     }
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(base + (uint32_t)(((u * 4 + t) ^ (row & 7)) << 4)), "r"(w[0]),
                                  "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
@@ -855,8 +876,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         }
     } else {
         // ------------------------------------------------------------------------------------------ row statistics, dQ
+        regs_up<152>();
         const int quarter = warp & 3, r0 = quarter * 32;
-        const uint32_t lane_addr = (uint32_t)r0 << 16, xbuf = sX + (uint32_t)(warp - 10) * DQ_BUF;
+        const uint32_t lane_addr = (uint32_t)r0 << 16, xbuf = sX + (uint32_t)(warp - 8) * DQ_BUF;
         bool ok = true;
         BwdWalk ahead = walk;                    // the tile whose row statistics are fetched next: one ahead of the dQ tile
         uint32_t n_rows = 0;
@@ -872,7 +894,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             }
             const bool alive = l != -INFINITY;
             sh->nlse[st][r0 + lane] = alive ? -l * 1.4426950408889634f : 0.f;
-            sh->delta[st][r0 + lane] = dl;
+            sh->ndelta[st][r0 + lane] = -dl * p.scale;
             const uint32_t bits = __ballot_sync(0xffffffffu, alive);
             if (lane == 0) sh->live[st][quarter] = bits;
             __syncwarp();
@@ -886,40 +908,35 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             if (ahead.more() && !fetch_rows()) { ok = false; break; }
             if (!warp_wait(&sh->dq_full, it & 1, lane)) { if (lane == 0) fail_bwd(sh, 16); ok = false; break; }
             tc_fence_after();
-            // 32 columns at a time through the exchange buffer: a reduction then covers 4 rows x 128 bytes
-            const int64_t q0 = (int64_t)walk.qt * TILE + r0;
-            const int sub = lane >> 3, col = (lane & 7) * 4;
-            float* acc = p.dq_acc + (((int64_t)b * p.h + walk.head) * p.sq + q0) * p.d + col;
-            uint32_t r[2][32];
-            tmem_ld32(tmem + lane_addr + C_DQ, r[0]);
+            uint32_t r[HD / 32][32];
+#pragma unroll
+            for (int c4 = 0; c4 < HD / 32; ++c4)
+                if (c4 * 32 < p.d) tmem_ld32(tmem + lane_addr + C_DQ + c4 * 32, r[c4]);
+            tmem_ld_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->dq_empty);
+            // 32 columns at a time into the buffer (16-byte units swizzled as the tensor map says), one bulk reduction each
 #pragma unroll
             for (int c4 = 0; c4 < HD / 32; ++c4) {
                 if (c4 * 32 >= p.d) break;
-                tmem_ld_wait();
-                if ((c4 + 1) * 32 < p.d) {
-                    if (c4 + 1 < HD / 32) tmem_ld32(tmem + lane_addr + C_DQ + (c4 + 1) * 32, r[(c4 + 1) & 1]);
-                } else {                     // all columns have left the tensor memory
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sh->dq_empty);
-                }
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the one before has read the buffer
+                __syncwarp();
                 const uint32_t srow = xbuf + (uint32_t)lane * 128;
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(srow + (uint32_t)((q ^ (lane & 7)) << 4)), "r"(r[c4 & 1][4 * q]),
-                                 "r"(r[c4 & 1][4 * q + 1]), "r"(r[c4 & 1][4 * q + 2]), "r"(r[c4 & 1][4 * q + 3]) : "memory");
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(srow + (uint32_t)((q ^ (lane & 7)) << 4)), "r"(r[c4][4 * q]),
+                                 "r"(r[c4][4 * q + 1]), "r"(r[c4][4 * q + 2]), "r"(r[c4][4 * q + 3]) : "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
-#pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    const int rl = g * 4 + sub;
-                    float v0, v1, v2, v3;
-                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v0), "=f"(v1), "=f"(v2), "=f"(v3)
-                                 : "r"(xbuf + (uint32_t)(rl * 128 + (((lane & 7) ^ (rl & 7)) << 4))) : "memory");
-                    if (q0 + rl < p.sq && c4 * 32 + col < p.d) red_add_v4(acc + (int64_t)rl * p.d + c4 * 32, v0, v1, v2, v3);
+                if (lane == 0) {
+                    asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+                                 ::"l"(&tdq), "r"(xbuf), "r"(c4 * 32), "r"(walk.qt * TILE + r0), "r"(b * p.h + walk.head) : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
-                __syncwarp();
             }
         }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // the reductions read this CTA's shared memory
     }
 
     __syncthreads();
@@ -929,7 +946,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         __syncthreads();
     }
     tc_fence_after();
-    if (warp == 1) tmem_dealloc(tmem, 512);
+    if (warp == 13) tmem_dealloc(tmem, 512);
 }
 
 // delta[b, h, q] = sum_d dO[b, q, h, d] * O[b, q, h, d], and zeros in the same row of the dQ accumulator (b, h, sq, d); 16
@@ -975,7 +992,7 @@ __global__ void attn_dq_convert_kernel(const float* acc, T* dq, int64_t q_tok, i
 }
 
 template <int HD, typename T>
-int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const AttnBwdParams& p,
+int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdParams& p,
                int64_t batch, cudaStream_t stream) {
     constexpr uint32_t TB = (HD / 64) * CHUNK;
     const size_t smem = 5 * TB + 2 * CHUNK + 4 * 32 * 128 + sizeof(BwdShared) + 1024;
@@ -985,7 +1002,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
         configured = true;
     }
     dim3 grid((unsigned)(p.hk * batch), (unsigned)p.k_tiles);
-    flash_bwd_kernel<HD, T><<<grid, BWD_THREADS, smem, stream>>>(tq, tk, tv, tdo, p);
+    flash_bwd_kernel<HD, T><<<grid, BWD_THREADS, smem, stream>>>(tq, tk, tv, tdo, tdq, p);
     bmt_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
@@ -996,12 +1013,13 @@ int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const v
             void* dq, const int64_t* dqs, void* dk, const int64_t* dks, void* dv, const int64_t* dvs, void* dq_acc, void* delta, float scale,
             int causal, const void* mask_bits_t, const void* mask_cls, const void* kv_lens, int dtype, cudaStream_t st) {
     const int hd = d <= 64 ? 64 : 128;
-    CUtensorMap tq, tk, tv, tdo;
+    CUtensorMap tq, tk, tv, tdo, tdq;
     int rc;
     if ((rc = bmt_tma_map_4d(&tq, q, dtype, d, sq, qs[0], h, qs[1], batch, qs[2], 64, TILE)) != 0) return rc;
     if ((rc = bmt_tma_map_4d(&tk, k, dtype, d, sk, ks[0], hk, ks[1], batch, ks[2], 64, TILE)) != 0) return rc;
     if ((rc = bmt_tma_map_4d(&tv, v, dtype, d, sk, vs[0], hk, vs[1], batch, vs[2], 64, TILE)) != 0) return rc;
     if ((rc = bmt_tma_map_4d(&tdo, dout, dtype, d, sq, gs[0], h, gs[1], batch, gs[2], 64, TILE)) != 0) return rc;
+    if ((rc = bmt_tma_map_f32_3d(&tdq, dq_acc, d, sq, batch * h, 32, 32)) != 0) return rc;
     const int64_t rows = batch * sq * h;
     const unsigned row_blocks = (unsigned)((rows * 16 + 255) / 256);
     attn_delta_kernel<T><<<row_blocks, 256, 0, st>>>((const T*)o, os[0], os[1], os[2], (const T*)dout, gs[0], gs[1], gs[2], (float*)delta,
@@ -1021,7 +1039,7 @@ int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const v
     p.idesc_s = common | ((uint32_t)(TILE >> 3) << 17);
     p.idesc_dv = common | (1u << 16) | ((uint32_t)(d >> 3) << 17);              // A K-major (or tensor memory), B MN-major, N = head dim
     p.idesc_dq = common | (1u << 15) | (1u << 16) | ((uint32_t)(d >> 3) << 17);  // A and B MN-major
-    rc = hd == 64 ? launch_bwd<64, T>(tq, tk, tv, tdo, p, batch, st) : launch_bwd<128, T>(tq, tk, tv, tdo, p, batch, st);
+    rc = hd == 64 ? launch_bwd<64, T>(tq, tk, tv, tdo, tdq, p, batch, st) : launch_bwd<128, T>(tq, tk, tv, tdo, tdq, p, batch, st);
     if (rc != 0) return rc;
     attn_dq_convert_kernel<T><<<row_blocks, 256, 0, st>>>((const float*)dq_acc, (T*)dq, dqs[0], dqs[1], dqs[2], rows, sq, h, d);
     bmt_count_launch(2);

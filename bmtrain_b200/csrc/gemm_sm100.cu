@@ -1115,6 +1115,20 @@ int bmt_tma_map_4d(CUtensorMap* out, const void* ptr, int dtype, int64_t inner, 
     return make_map(out, ptr, dtype, inner, rows, ld, nb0, bs0, nb1, bs1, box_inner, box_rows);
 }
 
+int bmt_tma_map_f32_3d(CUtensorMap* out, const void* ptr, int64_t inner, int64_t rows, int64_t nb, int box_inner, int box_rows) {
+    EncodeTiledFn enc = get_encode();
+    if (!enc) return -10;
+    if (((uintptr_t)ptr & 15) || (inner & 3)) return -11;
+    cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)nb};
+    cuuint64_t st[2] = {(cuuint64_t)inner * 4, (cuuint64_t)(inner * rows) * 4};
+    cuuint32_t box[3] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1};
+    cuuint32_t es[3] = {1, 1, 1};
+    cudaFree(0);  // see make_map
+    const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)ptr, dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : -12;
+}
+
 namespace {
 
 // 5-D map of an MN-major operand (element (k, mn) at ptr + k * ld + mn, mn contiguous): dims {64, k rows, mn / 64 chunks,

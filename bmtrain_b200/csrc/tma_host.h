@@ -8,3 +8,7 @@
 // (-10 driver entry point missing, -11 alignment, -12 encode failed).
 int bmt_tma_map_4d(CUtensorMap* out, const void* ptr, int dtype, int64_t inner, int64_t rows, int64_t ld, int64_t nb0, int64_t bs0,
                    int64_t nb1, int64_t bs1, int box_inner, int box_rows);
+
+// 3-D fp32 map of a dense (nb, rows, inner) array (inner a multiple of 4, base 16-byte aligned), box {box_inner, box_rows, 1},
+// 128-byte swizzle (box_inner * 4 <= 128).  Not cached: for scratch whose address changes from call to call.
+int bmt_tma_map_f32_3d(CUtensorMap* out, const void* ptr, int64_t inner, int64_t rows, int64_t nb, int box_inner, int box_rows);
