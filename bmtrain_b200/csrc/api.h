@@ -44,6 +44,12 @@ int bmt_ce_row_stats(int64_t m, int64_t n, const void* logits, int dtype, const 
                      void* out_3xm_f32, void* stream);
 int bmt_ce_backward(int64_t m, int64_t n, const void* logits, int dtype, const void* target_i64, const void* lse_f32,
                     const void* grad_loss_f32, int64_t vocab_start, int64_t ignore_index, void* out, void* stream);
+// Mean (or sum) of the cross-entropy over the rows whose target is not ignore_index, and its gradient.  scratch: 3 * m floats,
+// lse: m floats; loss, divisor (what the gradient is divided by), grad: one float each.
+int bmt_ce_reduced_forward(int64_t m, int64_t n, const void* logits, int dtype, const void* target, int64_t ignore_index, int mean,
+                           void* scratch, void* lse, void* loss, void* divisor, void* stream);
+int bmt_ce_reduced_backward(int64_t m, int64_t n, const void* logits, int dtype, const void* target, const void* lse,
+                            const void* grad, const void* divisor, int64_t ignore_index, void* out, void* stream);
 
 int bmt_norm_fwd(int64_t rows, int64_t d, const void* x, const void* w, const void* b, float eps, int rms, int dtype,
                  void* y, void* stats_2xrows_f32, void* stream);
@@ -58,7 +64,9 @@ int bmt_norm_bwd_ex(int64_t rows, int64_t d, const void* x, const void* dy, cons
                     int accumulate, void* stream);
 
 int bmt_embedding_fwd(int64_t tokens, int64_t d, const void* ids_i64, const void* weight, int dtype, void* out, void* stream);
-int bmt_embedding_bwd(int64_t tokens, int64_t d, const void* ids_i64, const void* grad, int dtype, void* acc_f32, void* stream);
+int64_t bmt_embedding_bwd_scratch(int64_t tokens, int64_t rows);   // 32-bit words of scratch
+int bmt_embedding_bwd(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out, void* scratch,
+                      void* stream);
 
 int bmt_masked_softmax(int64_t b, int64_t h, int64_t sq, int64_t sk, int64_t ld, void* scores, int dtype, int causal,
                        const void* mask_u8_b_sq_sk, const void* kv_lens_i32, void* stream);

@@ -7,6 +7,8 @@
 #include "api.h"
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace {
 
 // 2^x on the special-function unit (one instruction; the C library's exp2f adds range handling around it)
@@ -169,11 +171,32 @@ __global__ void __launch_bounds__(256) ce_row_stats_stream_kernel(int64_t m, int
     }
 }
 
+// The reduced loss from the row statistics (3 x m: maximum, sum, target logit): lse of every row, the loss (sum over the rows
+// whose target counts, divided by their number when `mean`) and that divisor.  One block, fixed order: a
+// few microseconds in the place of the dozen elementwise launches that cost the host more than the device.
+constexpr int CE_FINISH_THREADS = 1024;
+__global__ void __launch_bounds__(CE_FINISH_THREADS) ce_finish_kernel(int64_t m, const float* __restrict__ rows, const int64_t* __restrict__ target,
+                                                                      int64_t ignore_index, int mean, float* __restrict__ lse,
+                                                                      float* __restrict__ loss, float* __restrict__ divisor) {
+    __shared__ float scratch[33];
+    float sum = 0.f, count = 0.f;
+#pragma unroll 4
+    for (int64_t i = threadIdx.x; i < m; i += CE_FINISH_THREADS) {
+        const float l = rows[i] + logf(rows[m + i] + 1e-10f);
+        lse[i] = l;
+        if (target[i] != ignore_index) { sum += l - rows[2 * m + i]; count += 1.f; }
+    }
+    sum = bmt::block_allreduce<false>(sum, scratch);
+    count = bmt::block_allreduce<false>(count, scratch);
+    if (threadIdx.x == 0) { *loss = mean ? sum / count : sum; *divisor = mean ? count : 1.f; }
+}
+
+// `divisor` null: grad holds one value per row; else one value for all rows, to be divided by *divisor.
 template <typename T>
 __global__ void __launch_bounds__(256) ce_backward_kernel(int64_t m, int64_t n, const T* __restrict__ x,
                                                           const int64_t* __restrict__ target, const float* __restrict__ lse,
-                                                          const float* __restrict__ grad, int64_t vocab_start,
-                                                          int64_t ignore_index, T* __restrict__ out) {
+                                                          const float* __restrict__ grad, const float* __restrict__ divisor,
+                                                          int64_t vocab_start, int64_t ignore_index, T* __restrict__ out) {
     const int64_t row = blockIdx.x;
     const T* __restrict__ xr = x + row * n;
     T* __restrict__ orow = out + row * n;
@@ -181,7 +204,7 @@ __global__ void __launch_bounds__(256) ce_backward_kernel(int64_t m, int64_t n, 
     const bool ignored = tg == ignore_index;
     const int64_t t = tg - vocab_start;
     const float l = lse[row];
-    const float g = ignored ? 0.f : grad[row];
+    const float g = ignored ? 0.f : divisor ? grad[0] / divisor[0] : grad[row];
     constexpr int V = bmt::Vec16<T>::N;
     const bool vec_ok = (n % V == 0) && (((uintptr_t)xr & 15) == 0) && (((uintptr_t)orow & 15) == 0);
     if (vec_ok) {
@@ -252,13 +275,40 @@ extern "C" int bmt_ce_row_stats(int64_t m, int64_t n, const void* logits, int dt
     return (int)cudaGetLastError();
 }
 
-extern "C" int bmt_ce_backward(int64_t m, int64_t n, const void* logits, int dtype, const void* target, const void* lse,
-                               const void* grad, int64_t vocab_start, int64_t ignore_index, void* out, void* stream) {
+static int ce_backward(int64_t m, int64_t n, const void* logits, int dtype, const void* target, const void* lse, const void* grad,
+                       const void* divisor, int64_t vocab_start, int64_t ignore_index, void* out, void* stream) {
     if (m <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == BMT_DT_F16) ce_backward_kernel<__half><<<(unsigned)m, 256, 0, s>>>(m, n, (const __half*)logits, (const int64_t*)target, (const float*)lse, (const float*)grad, vocab_start, ignore_index, (__half*)out);
-    else if (dtype == BMT_DT_BF16) ce_backward_kernel<__nv_bfloat16><<<(unsigned)m, 256, 0, s>>>(m, n, (const __nv_bfloat16*)logits, (const int64_t*)target, (const float*)lse, (const float*)grad, vocab_start, ignore_index, (__nv_bfloat16*)out);
-    else ce_backward_kernel<float><<<(unsigned)m, 256, 0, s>>>(m, n, (const float*)logits, (const int64_t*)target, (const float*)lse, (const float*)grad, vocab_start, ignore_index, (float*)out);
+    const auto run = [&](auto* zero) {
+        using T = std::remove_pointer_t<decltype(zero)>;
+        ce_backward_kernel<T><<<(unsigned)m, 256, 0, s>>>(m, n, (const T*)logits, (const int64_t*)target, (const float*)lse, (const float*)grad,
+                                                          (const float*)divisor, vocab_start, ignore_index, (T*)out);
+    };
+    if (dtype == BMT_DT_F16) run((__half*)nullptr);
+    else if (dtype == BMT_DT_BF16) run((__nv_bfloat16*)nullptr);
+    else run((float*)nullptr);
     bmt_count_launch(1);
     return (int)cudaGetLastError();
+}
+
+extern "C" int bmt_ce_backward(int64_t m, int64_t n, const void* logits, int dtype, const void* target, const void* lse,
+                               const void* grad, int64_t vocab_start, int64_t ignore_index, void* out, void* stream) {
+    return ce_backward(m, n, logits, dtype, target, lse, grad, nullptr, vocab_start, ignore_index, out, stream);
+}
+
+// Forward and backward of the reduced loss (mean or sum over the rows whose target is not ignore_index).  scratch: 3 * m floats;
+// lse: m floats; loss, divisor: one float each (the divisor is what the gradient is divided by).
+extern "C" int bmt_ce_reduced_forward(int64_t m, int64_t n, const void* logits, int dtype, const void* target, int64_t ignore_index,
+                                      int mean, void* scratch, void* lse, void* loss, void* divisor, void* stream) {
+    const int rc = bmt_ce_row_stats(m, n, logits, dtype, target, 0, scratch, stream);
+    if (rc != 0) return rc;
+    ce_finish_kernel<<<1, CE_FINISH_THREADS, 0, (cudaStream_t)stream>>>(m, (const float*)scratch, (const int64_t*)target, ignore_index, mean,
+                                                                        (float*)lse, (float*)loss, (float*)divisor);
+    bmt_count_launch(1);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int bmt_ce_reduced_backward(int64_t m, int64_t n, const void* logits, int dtype, const void* target, const void* lse,
+                                       const void* grad, const void* divisor, int64_t ignore_index, void* out, void* stream) {
+    return ce_backward(m, n, logits, dtype, target, lse, grad, divisor, 0, ignore_index, out, stream);
 }

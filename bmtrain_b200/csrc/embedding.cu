@@ -1,4 +1,4 @@
-// Embedding gather and fp32 scatter-add (ids < 0: zeros in forward, skipped in backward).
+// Embedding gather and its gradient (ids < 0: zeros in forward, skipped in backward).
 #include "api.h"
 #include "common.cuh"
 
@@ -21,19 +21,118 @@ __global__ void __launch_bounds__(128) emb_fwd_kernel(int64_t d, const int64_t* 
     for (int64_t c = threadIdx.x * V; c < d; c += blockDim.x * V) bmt::st16(o + c, bmt::ld16(src + c));
 }
 
-template <typename T>
-__global__ void __launch_bounds__(128) emb_bwd_kernel(int64_t d, const int64_t* __restrict__ ids, const T* __restrict__ g, float* __restrict__ acc) {
-    const int64_t t = blockIdx.x;
+// Gradient of the table: row r = sum of the gradients of the tokens with id r, added in fp32, rounded once.
+// A table has far more rows than a batch has tokens, so what bounds it is writing the table (50304 x 4096 bf16: 63 us at the
+// copy rate).  Zeroing an fp32 table, adding to it atomically and converting it moved five times that (490 us there).  So the
+// tokens are ordered by id first -- three small kernels over tokens or rows: count and rank, a start for every row that has
+// tokens, order -- and every row is then written once, by a team of threads that adds up its tokens.  Rows with more than
+// EMB_HOT tokens (padding) are left to a kernel that spreads one row's tokens over warps and its columns over blocks.
+constexpr int EMB_HOT = 64;
+
+struct EmbScratch {                 // one int32 array: total, hot rows | count[rows] | start[rows] | hot[hot_cap] | rank[tokens] | order[tokens]
+    int *total, *n_hot, *count, *start, *hot, *rank, *order;
+};
+__host__ __device__ __forceinline__ int64_t emb_hot_cap(int64_t tokens) { return tokens / EMB_HOT + 1; }
+EmbScratch emb_scratch(void* base, int64_t tokens, int64_t rows) {
+    EmbScratch e;
+    int* p = (int*)base;
+    e.total = p; e.n_hot = p + 1; e.count = p + 2; e.start = e.count + rows; e.hot = e.start + rows; e.rank = e.hot + emb_hot_cap(tokens);
+    e.order = e.rank + tokens;
+    return e;
+}
+
+__global__ void __launch_bounds__(256) emb_count_kernel(int64_t tokens, int64_t rows, const int64_t* __restrict__ ids, EmbScratch e) {
+    const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (t >= tokens) return;
     const int64_t id = ids[t];
-    if (id < 0) return;
-    const T* __restrict__ gr = g + t * d;
-    float* __restrict__ a = acc + id * d;
+    if (id >= 0 && id < rows) e.rank[t] = atomicAdd(e.count + id, 1);
+}
+__global__ void __launch_bounds__(256) emb_start_kernel(int64_t rows, EmbScratch e) {
+    const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (r >= rows) return;
+    const int c = e.count[r];
+    if (c == 0) return;
+    e.start[r] = atomicAdd(e.total, c);
+    if (c > EMB_HOT) e.hot[atomicAdd(e.n_hot, 1)] = (int)r;
+}
+__global__ void __launch_bounds__(256) emb_order_kernel(int64_t tokens, int64_t rows, const int64_t* __restrict__ ids, EmbScratch e) {
+    const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (t >= tokens) return;
+    const int64_t id = ids[t];
+    if (id >= 0 && id < rows) e.order[e.start[id] + e.rank[t]] = (int)t;
+}
+// `team` threads (32 .. 256) per row
+template <typename T>
+__global__ void __launch_bounds__(256) emb_rows_kernel(int64_t rows, int64_t d, int team, const T* __restrict__ g, EmbScratch e, T* __restrict__ out) {
     constexpr int V = bmt::Vec16<T>::N;
-    for (int64_t c = threadIdx.x * V; c < d; c += blockDim.x * V) {
-        bmt::Vec16<T> v = bmt::ld16(gr + c);
+    const int64_t r = (int64_t)blockIdx.x * (256 / team) + threadIdx.x / team;
+    if (r >= rows) return;
+    const int c = e.count[r];
+    if (c > EMB_HOT) return;
+    const int* __restrict__ tok = e.order + (c ? e.start[r] : 0);
+    for (int64_t col = (threadIdx.x % team) * V; col < d; col += (int64_t)team * V) {
+        float acc[V];
 #pragma unroll
-        for (int k = 0; k < V; ++k) atomicAdd(a + c + k, bmt::Cvt<T>::to_f(v.v[k]));
+        for (int k = 0; k < V; ++k) acc[k] = 0.f;
+#pragma unroll 4
+        for (int i = 0; i < c; ++i) {
+            const bmt::Vec16<T> v = bmt::ld16(g + (int64_t)tok[i] * d + col);
+#pragma unroll
+            for (int k = 0; k < V; ++k) acc[k] += bmt::Cvt<T>::to_f(v.v[k]);
+        }
+        bmt::Vec16<T> o;
+#pragma unroll
+        for (int k = 0; k < V; ++k) o.v[k] = bmt::Cvt<T>::from_f(acc[k]);
+        bmt::st16(out + r * d + col, o);
     }
+}
+template <typename T>
+__global__ void __launch_bounds__(256) emb_hot_kernel(int64_t d, const T* __restrict__ g, EmbScratch e, T* __restrict__ out) {
+    constexpr int V = bmt::Vec16<T>::N;
+    __shared__ float part[8][32 * V];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t segs = (d + 32 * V - 1) / (32 * V), items = (int64_t)*e.n_hot * segs;
+    for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+        const int64_t r = e.hot[it / segs], col = (it % segs) * 32 * V + lane * V;
+        const int c = e.count[r];
+        const int* __restrict__ tok = e.order + e.start[r];
+        float acc[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) acc[k] = 0.f;
+        if (col < d) {
+#pragma unroll 4
+            for (int i = warp; i < c; i += 8) {
+                const bmt::Vec16<T> v = bmt::ld16(g + (int64_t)tok[i] * d + col);
+#pragma unroll
+                for (int k = 0; k < V; ++k) acc[k] += bmt::Cvt<T>::to_f(v.v[k]);
+            }
+        }
+        __syncthreads();                       // the previous item's sums have been read
+#pragma unroll
+        for (int k = 0; k < V; ++k) part[warp][lane * V + k] = acc[k];
+        __syncthreads();
+        if (warp == 0 && col < d) {
+            bmt::Vec16<T> o;
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+                float s = 0.f;
+#pragma unroll
+                for (int w = 0; w < 8; ++w) s += part[w][lane * V + k];
+                o.v[k] = bmt::Cvt<T>::from_f(s);
+            }
+            bmt::st16(out + r * d + col, o);
+        }
+    }
+}
+
+template <typename T>
+void launch_rows(int64_t rows, int64_t d, const void* g, const EmbScratch& e, void* out, bool any_hot, cudaStream_t s) {
+    constexpr int V = bmt::Vec16<T>::N;
+    int team = 32;
+    while (team < 256 && (int64_t)team * V < d) team *= 2;
+    const int per = 256 / team;
+    emb_rows_kernel<T><<<(unsigned)((rows + per - 1) / per), 256, 0, s>>>(rows, d, team, (const T*)g, e, (T*)out);
+    if (any_hot) emb_hot_kernel<T><<<296, 256, 0, s>>>(d, (const T*)g, e, (T*)out);
 }
 
 }  // namespace
@@ -49,13 +148,27 @@ extern "C" int bmt_embedding_fwd(int64_t tokens, int64_t d, const void* ids, con
     return (int)cudaGetLastError();
 }
 
-extern "C" int bmt_embedding_bwd(int64_t tokens, int64_t d, const void* ids, const void* grad, int dtype, void* acc, void* stream) {
-    if (tokens <= 0) return 0;
+// 32-bit words of scratch that bmt_embedding_bwd needs.
+extern "C" int64_t bmt_embedding_bwd_scratch(int64_t tokens, int64_t rows) { return 2 + 2 * rows + emb_hot_cap(tokens) + 2 * tokens; }
+
+extern "C" int bmt_embedding_bwd(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out,
+                                 void* scratch, void* stream) {
+    if (rows <= 0) return 0;
+    if (d % (dtype == BMT_DT_F32 ? 4 : 8) || tokens > 0x7fffffff || rows > 0x7fffffff) return -3;
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == BMT_DT_F32) { if (d % 4) return -3; emb_bwd_kernel<float><<<(unsigned)tokens, 128, 0, s>>>(d, (const int64_t*)ids, (const float*)grad, (float*)acc); }
-    else { if (d % 8) return -3;
-        if (dtype == BMT_DT_F16) emb_bwd_kernel<__half><<<(unsigned)tokens, 128, 0, s>>>(d, (const int64_t*)ids, (const __half*)grad, (float*)acc);
-        else emb_bwd_kernel<__nv_bfloat16><<<(unsigned)tokens, 128, 0, s>>>(d, (const int64_t*)ids, (const __nv_bfloat16*)grad, (float*)acc); }
-    bmt_count_launch(1);
+    const EmbScratch e = emb_scratch(scratch, tokens, rows);
+    BMT_CUDA_OK(cudaMemsetAsync(e.total, 0, (size_t)(2 + rows) * sizeof(int), s));
+    if (tokens > 0) {
+        const unsigned tb = (unsigned)((tokens + 255) / 256);
+        emb_count_kernel<<<tb, 256, 0, s>>>(tokens, rows, (const int64_t*)ids, e);
+        emb_start_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, s>>>(rows, e);
+        emb_order_kernel<<<tb, 256, 0, s>>>(tokens, rows, (const int64_t*)ids, e);
+        bmt_count_launch(3);
+    }
+    const bool any_hot = tokens > EMB_HOT;
+    if (dtype == BMT_DT_F32) launch_rows<float>(rows, d, grad, e, out, any_hot, s);
+    else if (dtype == BMT_DT_F16) launch_rows<__half>(rows, d, grad, e, out, any_hot, s);
+    else launch_rows<__nv_bfloat16>(rows, d, grad, e, out, any_hot, s);
+    bmt_count_launch(any_hot ? 2 : 1);
     return (int)cudaGetLastError();
 }

@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(1024) norm_fold_kernel(int d, int nblk, const 
     if (c < d) {
         for (int i = ty; i < nblk; i += 32) {
             a += partial[(int64_t)i * d + c];
-            bsum += partial[((int64_t)nblk + i) * d + c];
+            if (db) bsum += partial[((int64_t)nblk + i) * d + c];
         }
     }
     sa[ty][tx] = a; sb[ty][tx] = bsum;
@@ -374,83 +374,117 @@ int fwd(int64_t rows, int64_t d, const void* x, const void* w, const void* b, fl
     return (int)cudaGetLastError();
 }
 
-// Backward with the same work split as norm_fwd_reg_kernel: a team of WPR warps per row, every lane owns fixed columns.
-// x and dy are read once (kept as packed 16-byte vectors in registers between the statistics and the dx pass), the
-// per-column sums of dy * xhat and dy accumulate in registers over all rows a lane sees and are combined once per CTA
-// through shared memory into the (nblk x d) scratch that norm_fold_kernel reduces.  No block-wide barrier per row
-// unless a row is shared by several warps.
-template <typename T, int VPL, int WPR>
-__global__ void __launch_bounds__(NT, 1) norm_bwd_reg_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __restrict__ dy,
-                                                             const T* __restrict__ w, const float* __restrict__ stats, int rms,
-                                                             T* __restrict__ dx, float* __restrict__ partial,
-                                                             const T* __restrict__ dres) {
-    constexpr int RPC = 8 / WPR;
-    __shared__ float ex[2][8];
-    extern __shared__ float fold[];                    // [RPC][2][d / ... ] reused for the final combination
+// Backward: a team of WPR warps per row, every lane owns fixed columns (VPL vectors of 8).  x and dy of the next row are on
+// their way while the current one is worked on, both are kept as packed 16-byte vectors between the statistics and the dx
+// pass, and the per-column sums of dy * xhat and dy accumulate in registers over all rows a lane sees; they are combined once
+// per CTA through shared memory into the scratch that norm_fold_kernel reduces.
+// HBM bytes bound it (x, dy in, dx out), so what counts is rows in flight: with up to 8 vectors a lane and no prefetch the
+// accumulators alone took 249 registers, eight warps a SM waited for their loads and the kernel ran at 0.41 of the copy rate
+// (16384 x 5120 RMS 180 us).  Wide teams keep a lane at 2 or 3 vectors, which leaves room for the prefetch and for 16 warps a SM;
+// RMSNorm (RMS) has no bias and drops the second accumulator.  One barrier per row: the partial sums alternate between two
+// sets of slots.
+template <int WPR> struct BwdTeam {
+    static constexpr int THREADS = WPR == 16 ? 512 : 256, CTAS = WPR == 16 ? 1 : 2, RPC = THREADS / 32 / WPR;
+};
+
+template <typename T, int VPL, int WPR, bool RMS>
+__global__ void __launch_bounds__(BwdTeam<WPR>::THREADS, BwdTeam<WPR>::CTAS)
+norm_bwd_stream_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ w,
+                       const float* __restrict__ stats, T* __restrict__ dx, float* __restrict__ partial, const T* __restrict__ dres) {
+    constexpr int RPC = BwdTeam<WPR>::RPC, WARPS = BwdTeam<WPR>::THREADS / 32;
+    constexpr bool AHEAD = VPL <= 3;                   // the next row's loads are issued before this row's arithmetic
+    __shared__ float ex[2][2][WARPS];
+    extern __shared__ float fold[];                    // 2 * d floats, for the final combination
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = warp % WPR, slot = warp / WPR;
-    float dg[VPL][8], db[VPL][8];
+    float dg[VPL][8], db[RMS ? 1 : VPL][8];
+    bmt::Vec16<T> wv[VPL], xv[VPL], gv[VPL], xn[VPL], gn[VPL];
 #pragma unroll
-    for (int v = 0; v < VPL; ++v)
+    for (int v = 0; v < VPL; ++v) {
+        const int c = ((v * WPR + sub) * 32 + lane) * 8;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) dg[v][k] = db[v][k] = 0.f;
+        for (int k = 0; k < 8; ++k) { dg[v][k] = 0.f; if (!RMS) db[v][k] = 0.f; }
+        if (c < d) wv[v] = bmt::ld16(w + c);
+    }
     const int64_t groups = (rows + RPC - 1) / RPC;
-    for (int64_t gi = blockIdx.x; gi < groups; gi += gridDim.x) {
+    float mean, rstd, mean_n, rstd_n;
+    auto load = [&](int64_t gi, bmt::Vec16<T>(&xx)[VPL], bmt::Vec16<T>(&gg)[VPL], float& mu, float& rs) {
         const int64_t r = gi * RPC + slot;
-        const bool live = r < rows;
-        const float mean = live ? stats[r] : 0.f, rstd = live ? stats[rows + r] : 0.f;
-        bmt::Vec16<T> xv[VPL], gv[VPL];
+        const bool live = gi < groups && r < rows;
+        mu = live && !RMS ? stats[r] : 0.f;
+        rs = live ? stats[rows + r] : 0.f;
 #pragma unroll
         for (int v = 0; v < VPL; ++v) {
             const int c = ((v * WPR + sub) * 32 + lane) * 8;
-            if (live && c < d) { xv[v] = bmt::ld16(x + r * d + c); gv[v] = bmt::ld16(dy + r * d + c); }
+            if (live && c < d) { xx[v] = bmt::ld16(x + r * d + c); gg[v] = bmt::ld16(dy + r * d + c); }
+        }
+    };
+    load(blockIdx.x, xv, gv, mean, rstd);
+    int par = 0;
+    for (int64_t gi = blockIdx.x; gi < groups; gi += gridDim.x, par ^= 1) {
+        const int64_t r = gi * RPC + slot;
+        const bool live = r < rows;
+        if (AHEAD) load(gi + gridDim.x, xn, gn, mean_n, rstd_n);
+        bmt::Vec16<T> rv[VPL];
+        if (dres) {
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) {
+                const int c = ((v * WPR + sub) * 32 + lane) * 8;
+                if (live && c < d) rv[v] = bmt::ld16(dres + r * d + c);
+            }
         }
         float s1 = 0.f, s2 = 0.f;
 #pragma unroll
         for (int v = 0; v < VPL; ++v) {
             const int c = ((v * WPR + sub) * 32 + lane) * 8;
             if (live && c < d) {
-                const bmt::Vec16<T> wv = bmt::ld16(w + c);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const float xh = (bmt::Cvt<T>::to_f(xv[v].v[k]) - mean) * rstd;
                     const float g = bmt::Cvt<T>::to_f(gv[v].v[k]);
-                    const float wg = g * bmt::Cvt<T>::to_f(wv.v[k]);
-                    s1 += wg; s2 += wg * xh;
-                    dg[v][k] += g * xh; db[v][k] += g;
+                    const float wg = g * bmt::Cvt<T>::to_f(wv[v].v[k]);
+                    if (!RMS) s1 += wg;
+                    s2 += wg * xh;
+                    dg[v][k] += g * xh;
+                    if (!RMS) db[v][k] += g;
                 }
             }
         }
-        s1 = bmt::warp_sum(s1);
+        if (!RMS) s1 = bmt::warp_sum(s1);
         s2 = bmt::warp_sum(s2);
         if (WPR > 1) {
-            if (lane == 0) { ex[0][warp] = s1; ex[1][warp] = s2; }
+            if (lane == 0) { ex[par][0][warp] = s1; ex[par][1][warp] = s2; }
             __syncthreads();
             s1 = s2 = 0.f;
 #pragma unroll
-            for (int i = 0; i < WPR; ++i) { s1 += ex[0][slot * WPR + i]; s2 += ex[1][slot * WPR + i]; }
+            for (int i = 0; i < WPR; ++i) { if (!RMS) s1 += ex[par][0][slot * WPR + i]; s2 += ex[par][1][slot * WPR + i]; }
         }
-        s1 = rms ? 0.f : s1 / d;
+        s1 = s1 / d;
         s2 = s2 / d;
 #pragma unroll
         for (int v = 0; v < VPL; ++v) {
             const int c = ((v * WPR + sub) * 32 + lane) * 8;
             if (live && c < d) {
-                const bmt::Vec16<T> wv = bmt::ld16(w + c);
-                bmt::Vec16<T> o, rv;
-                if (dres) rv = bmt::ld16(dres + r * d + c);
+                bmt::Vec16<T> o;
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const float xh = (bmt::Cvt<T>::to_f(xv[v].v[k]) - mean) * rstd;
-                    const float wg = bmt::Cvt<T>::to_f(gv[v].v[k]) * bmt::Cvt<T>::to_f(wv.v[k]);
+                    const float wg = bmt::Cvt<T>::to_f(gv[v].v[k]) * bmt::Cvt<T>::to_f(wv[v].v[k]);
                     float val = rstd * (wg - s1 - xh * s2);
-                    if (dres) val += bmt::Cvt<T>::to_f(rv.v[k]);
+                    if (dres) val += bmt::Cvt<T>::to_f(rv[v].v[k]);
                     o.v[k] = bmt::Cvt<T>::from_f(val);
                 }
                 bmt::st16(dx + r * d + c, o);
             }
         }
-        if (WPR > 1) __syncthreads();
+        if (AHEAD) {
+            mean = mean_n;
+            rstd = rstd_n;
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) { xv[v] = xn[v]; gv[v] = gn[v]; }
+        } else {
+            load(gi + gridDim.x, xv, gv, mean, rstd);
+        }
     }
     // combine the RPC row slots of this CTA: slot 0 ends up with the CTA's column sums
     float* pg = partial + (int64_t)blockIdx.x * d;
@@ -463,7 +497,7 @@ __global__ void __launch_bounds__(NT, 1) norm_bwd_reg_kernel(int64_t rows, int d
                 const int c = ((v * WPR + sub) * 32 + lane) * 8;
                 if (c < d) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) { fold[c + k] = dg[v][k]; fold[d + c + k] = db[v][k]; }
+                    for (int k = 0; k < 8; ++k) { fold[c + k] = dg[v][k]; if (!RMS) fold[d + c + k] = db[v][k]; }
                 }
             }
         }
@@ -474,7 +508,7 @@ __global__ void __launch_bounds__(NT, 1) norm_bwd_reg_kernel(int64_t rows, int d
                 const int c = ((v * WPR + sub) * 32 + lane) * 8;
                 if (c < d) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) { dg[v][k] += fold[c + k]; db[v][k] += fold[d + c + k]; }
+                    for (int k = 0; k < 8; ++k) { dg[v][k] += fold[c + k]; if (!RMS) db[v][k] += fold[d + c + k]; }
                 }
             }
         }
@@ -485,58 +519,66 @@ __global__ void __launch_bounds__(NT, 1) norm_bwd_reg_kernel(int64_t rows, int d
             const int c = ((v * WPR + sub) * 32 + lane) * 8;
             if (c < d) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) { pg[c + k] = dg[v][k]; pb[c + k] = db[v][k]; }
+                for (int k = 0; k < 8; k += 4) {
+                    *reinterpret_cast<float4*>(pg + c + k) = make_float4(dg[v][k], dg[v][k + 1], dg[v][k + 2], dg[v][k + 3]);
+                    if (!RMS) *reinterpret_cast<float4*>(pb + c + k) = make_float4(db[v][k], db[v][k + 1], db[v][k + 2], db[v][k + 3]);
+                }
             }
         }
     }
 }
 
-template <typename T, int WPR>
-bool bwd_reg_vpl(int vpl, int64_t rows, int d, const void* x, const void* dy, const void* w, const void* stats, int rms, int nblk,
-                 void* dx, void* partial, const void* dres, cudaStream_t s) {
-    const size_t smem = (size_t)2 * d * sizeof(float);
-#define BMT_BWD_REG(V)                                                                                                          \
-    do {                                                                                                                        \
-        static bool cfg = false;                                                                                                \
-        if (!cfg) { cudaFuncSetAttribute(norm_bwd_reg_kernel<T, V, WPR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 16384 * 4); cfg = true; } \
-        norm_bwd_reg_kernel<T, V, WPR><<<nblk, NT, smem, s>>>(rows, d, (const T*)x, (const T*)dy, (const T*)w, (const float*)stats, rms, \
-                                                              (T*)dx, (float*)partial, (const T*)dres);                         \
-    } while (0)
-    if (vpl <= 2) BMT_BWD_REG(2);
-    else if (vpl <= 4) BMT_BWD_REG(4);
-    else if (vpl <= 6) BMT_BWD_REG(6);
-    else if (vpl <= 8) BMT_BWD_REG(8);
-    else return false;
-#undef BMT_BWD_REG
-    return true;
+// Returns the number of CTAs (rows of partial sums per accumulator) that were launched.
+template <typename T, int VPL, int WPR>
+int launch_bwd_stream(int64_t rows, int d, const void* x, const void* dy, const void* w, const void* stats, int rms, int nblk, void* dx,
+                      void* partial, const void* dres, cudaStream_t s) {
+    using Team = BwdTeam<WPR>;
+    const size_t smem = Team::RPC > 1 ? (size_t)2 * d * sizeof(float) : 0;   // at most 2 * 3072 floats where rows share a CTA
+    int64_t grid = (rows + Team::RPC - 1) / Team::RPC;
+    if (grid > 148 * Team::CTAS) grid = 148 * Team::CTAS;
+    if (grid > nblk) grid = nblk;
+    if (rms) norm_bwd_stream_kernel<T, VPL, WPR, true><<<(unsigned)grid, Team::THREADS, smem, s>>>(rows, d, (const T*)x, (const T*)dy, (const T*)w,
+                                                                                                (const float*)stats, (T*)dx, (float*)partial, (const T*)dres);
+    else if constexpr (VPL != 3 || WPR == 16)   // narrower teams have at most 2 vectors a lane here
+        norm_bwd_stream_kernel<T, VPL, WPR, false><<<(unsigned)grid, Team::THREADS, smem, s>>>(rows, d, (const T*)x, (const T*)dy, (const T*)w,
+                                                                                               (const float*)stats, (T*)dx, (float*)partial, (const T*)dres);
+    return (int)grid;
+}
+
+template <typename T, int WPR, typename... Args>
+int bwd_stream_vpl(int vpl, Args... args) {
+    if (vpl <= 1) return launch_bwd_stream<T, 1, WPR>(args...);
+    if (vpl == 2) return launch_bwd_stream<T, 2, WPR>(args...);
+    if constexpr (WPR == 16) if (vpl > 3) return launch_bwd_stream<T, 4, WPR>(args...);
+    return launch_bwd_stream<T, 3, WPR>(args...);
 }
 
 template <typename T>
 int bwd(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, const void* stats, int rms, int nblk, void* dx,
         void* partial, void* dw, void* db, cudaStream_t s, const void* dres = nullptr, bool acc = false) {
-    const auto fold = [&] {
+    const auto fold = [&](int blocks) {
         const unsigned g = (unsigned)((d + 31) / 32);
-        if (acc) norm_fold_kernel<T, true><<<g, dim3(32, 32), 0, s>>>((int)d, nblk, (const float*)partial, (T*)dw, (T*)db);
-        else norm_fold_kernel<T><<<g, dim3(32, 32), 0, s>>>((int)d, nblk, (const float*)partial, (T*)dw, (T*)db);
+        if (acc) norm_fold_kernel<T, true><<<g, dim3(32, 32), 0, s>>>((int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
+        else norm_fold_kernel<T><<<g, dim3(32, 32), 0, s>>>((int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
     };
     static const bool use_reg = [] { const char* e = getenv("BMT_NORM_STAGED"); return !(e && atoi(e) == 1); }();
-    if (use_reg && d <= 16384) {
-        // the backward keeps two column-sum accumulators per value: at most 6 vectors per lane where the row length allows
-        const int wpr = d <= 1536 ? 1 : d <= 3072 ? 2 : d <= 6144 ? 4 : 8;
-        const int vpl = (int)((d + 256 * wpr - 1) / (256 * wpr));
-        bool done = false;
-        if (wpr == 1) done = bwd_reg_vpl<T, 1>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s);
-        else if (wpr == 2) done = bwd_reg_vpl<T, 2>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s);
-        else if (wpr == 4) done = bwd_reg_vpl<T, 4>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s);
-        else done = bwd_reg_vpl<T, 8>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s);
-        if (done) {
-            fold();
-            bmt_count_launch(2);
-            return (int)cudaGetLastError();
-        }
+    if (use_reg && d <= 16384 && !(rms && db)) {
+        // the narrowest team whose lanes need no register spills: 3 vectors for RMSNorm, 2 with the bias sums; beyond that
+        // (above 12288 / 8192 columns) the widest team
+        const int64_t nv = (d + 255) / 256, most = rms ? 3 : 2;   // nv: vectors a lane of one warp would have
+        const int wpr = nv <= most ? 1 : nv <= 2 * most ? 2 : nv <= 4 * most ? 4 : nv <= 8 * most ? 8 : 16;
+        const int vpl = (int)((nv + wpr - 1) / wpr);
+        const int blocks = wpr == 1 ? bwd_stream_vpl<T, 1>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s)
+                         : wpr == 2 ? bwd_stream_vpl<T, 2>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s)
+                         : wpr == 4 ? bwd_stream_vpl<T, 4>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s)
+                         : wpr == 8 ? bwd_stream_vpl<T, 8>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s)
+                                    : bwd_stream_vpl<T, 16>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s);
+        fold(blocks);
+        bmt_count_launch(2);
+        return (int)cudaGetLastError();
     }
     norm_bwd_kernel<T><<<nblk, NT, 0, s>>>(rows, (int)d, (const T*)x, (const T*)dy, (const T*)w, (const float*)stats, rms, (T*)dx, (float*)partial, (const T*)dres);
-    fold();
+    fold(nblk);
     bmt_count_launch(2);
     return (int)cudaGetLastError();
 }

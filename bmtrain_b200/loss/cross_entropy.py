@@ -38,6 +38,24 @@ class OpFusedCrossEntropy(torch.autograd.Function):
         return grad, None, None
 
 
+class OpReducedCrossEntropy(torch.autograd.Function):
+    """Mean or sum of the cross entropy over the rows whose target counts, on the GPU: row statistics and one small kernel
+    forward, one kernel backward."""
+
+    @staticmethod
+    def forward(ctx, x: torch.Tensor, target: torch.Tensor, ignore_index: int, mean: bool):
+        x, target = x.contiguous(), target.contiguous()
+        loss, lse, divisor = _ce.reduced_forward(x, target, ignore_index, mean)
+        ctx.ignore_index = ignore_index
+        ctx.save_for_backward(x, target, lse, divisor)
+        return loss
+
+    @staticmethod
+    def backward(ctx, grad_output: torch.Tensor):
+        x, target, lse, divisor = ctx.saved_tensors
+        return _ce.reduced_backward(x, target, lse, divisor, grad_output, ctx.ignore_index), None, None, None
+
+
 class VPFusedCrossEntropy(torch.autograd.Function):
     """Cross entropy over a vocabulary sharded across the tensor-parallel group."""
 
@@ -107,6 +125,8 @@ class FusedCrossEntropy(torch.nn.Module):
                     reduction=self.reduction, label_smoothing=self.label_smoothing)
             if self.label_smoothing != 0.0:
                 raise NotImplementedError("label_smoothing is not supported by the fused cross entropy")
+            if self.weight is None and self.reduction in ("mean", "sum") and input.is_cuda and input.ndim == 2 and target.ndim == 1:
+                return OpReducedCrossEntropy.apply(input, target.long(), self.ignore_index, self.reduction == "mean")
             ret = OpFusedCrossEntropy.apply(input, target.long(), self.ignore_index)
 
         ignored = target == self.ignore_index

@@ -66,3 +66,30 @@ def ce_backward(logits: torch.Tensor, target: torch.Tensor, lse: torch.Tensor, g
         _native.ptr(lse.contiguous()), _native.ptr(grad_loss.float().contiguous()), ctypes.c_int64(vocab_start),
         ctypes.c_int64(ignore_index), _native.ptr(out), _native.stream_handle()), "cross-entropy backward kernel")
     return out
+
+
+def reduced_forward(logits: torch.Tensor, target: torch.Tensor, ignore_index: int, mean: bool):
+    """Mean or sum of the cross entropy over the rows whose target is not ``ignore_index``: ``(loss scalar, log-sum-exp per
+    row, divisor of its gradient)``, all fp32.  GPU only."""
+    m, n = logits.shape
+    assert logits.is_cuda and logits.is_contiguous() and target.is_contiguous() and target.dtype == torch.int64 and target.numel() == m
+    scratch = torch.empty(3 * m, dtype=torch.float32, device=logits.device)
+    kept = torch.empty(m + 1, dtype=torch.float32, device=logits.device)
+    loss, lse, divisor = torch.empty((), dtype=torch.float32, device=logits.device), kept[:m], kept[m:]
+    _native.check(_native.cuda_lib().bmt_ce_reduced_forward(
+        ctypes.c_int64(m), ctypes.c_int64(n), _native.ptr(logits), ctypes.c_int(_DT[logits.dtype]), _native.ptr(target),
+        ctypes.c_int64(ignore_index), ctypes.c_int(1 if mean else 0), _native.ptr(scratch), _native.ptr(lse), _native.ptr(loss), _native.ptr(divisor),
+        _native.stream_handle()), "cross-entropy forward kernels")
+    return loss, lse, divisor
+
+
+def reduced_backward(logits: torch.Tensor, target: torch.Tensor, lse: torch.Tensor, divisor: torch.Tensor, grad_loss: torch.Tensor,
+                     ignore_index: int) -> torch.Tensor:
+    """Gradient of :func:`reduced_forward`'s loss for the scalar ``grad_loss``."""
+    m, n = logits.shape
+    out = torch.empty_like(logits)
+    _native.check(_native.cuda_lib().bmt_ce_reduced_backward(
+        ctypes.c_int64(m), ctypes.c_int64(n), _native.ptr(logits), ctypes.c_int(_DT[logits.dtype]), _native.ptr(target),
+        _native.ptr(lse), _native.ptr(grad_loss.float().contiguous()), _native.ptr(divisor), ctypes.c_int64(ignore_index),
+        _native.ptr(out), _native.stream_handle()), "cross-entropy backward kernel")
+    return out

@@ -38,12 +38,17 @@ def embedding_backward(ids: torch.Tensor, grad: torch.Tensor, rows: int) -> torc
         keep = flat >= 0
         acc.index_add_(0, flat[keep], g2[keep].float())
         return acc.to(grad.dtype)
-    acc = torch.zeros(rows, d, dtype=torch.float32, device=grad.device)
-    ids64 = flat.to(torch.int64).contiguous()
-    _native.check(_native.cuda_lib().bmt_embedding_bwd(
-        ctypes.c_int64(ids64.numel()), ctypes.c_int64(d), _native.ptr(ids64), _native.ptr(g2.contiguous()),
-        ctypes.c_int(_DT[grad.dtype]), _native.ptr(acc), _native.stream_handle()), "embedding backward kernel")
-    return acc.to(grad.dtype)
+    if flat.numel() == 0:
+        return torch.zeros(rows, d, dtype=grad.dtype, device=grad.device)
+    lib = _native.cuda_lib()
+    ids64, g2 = flat.to(torch.int64).contiguous(), g2.contiguous()
+    out = torch.empty(rows, d, dtype=grad.dtype, device=grad.device)
+    words = 2 + 2 * rows + ids64.numel() // 64 + 1 + 2 * ids64.numel()     # bmt_embedding_bwd_scratch
+    scratch = torch.empty(words, dtype=torch.int32, device=grad.device)
+    _native.check(lib.bmt_embedding_bwd(
+        ctypes.c_int64(ids64.numel()), ctypes.c_int64(d), ctypes.c_int64(rows), _native.ptr(ids64), _native.ptr(g2),
+        ctypes.c_int(_DT[grad.dtype]), _native.ptr(out), _native.ptr(scratch), _native.stream_handle()), "embedding backward kernels")
+    return out
 
 
 class EmbeddingFunction(torch.autograd.Function):

@@ -1,0 +1,85 @@
+"""Row kernels at the edges of their work splits, against float64: norm backward (every team width, ragged lanes, fewer rows
+than CTAs), the reduced cross-entropy, the embedding gradient (ids that repeat up to and beyond the hot-row limit)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+_UNIT = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2.0 ** -24}
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("rows,d", [(1, 8), (3, 256), (37, 264), (700, 512), (5, 520), (33, 768), (9, 776), (64, 1536), (300, 1544),
+                                    (17, 2048), (1000, 2560), (2, 3072), (11, 4104), (600, 5120), (7, 6152), (149, 8192), (5, 8200),
+                                    (3, 12288), (150, 12296), (4, 16384)])
+def test_norm_backward(bmt_gpu, dtype, rms, rows, d):
+    from bmtrain_b200.ops import norm as N
+
+    gen = torch.Generator(device="cuda").manual_seed(rows + d)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    x, dy = (2 * rand(rows, d) + 0.5).to(dtype), rand(rows, d).to(dtype)
+    w, b = (1 + 0.2 * rand(d)).to(dtype), (0.2 * rand(d)).to(dtype)
+    leaves = [t.clone().requires_grad_() for t in ((x, w) if rms else (x, w, b))]
+    y = N.rms_norm(*leaves, 1e-5) if rms else N.layer_norm(*leaves, 1e-5)
+    got = torch.autograd.grad(y, leaves, dy)
+    exact = [t.double().requires_grad_() for t in ((x, w) if rms else (x, w, b))]
+    if rms:
+        ref = exact[0] * torch.rsqrt(exact[0].square().mean(-1, keepdim=True) + 1e-5) * exact[1]
+    else:
+        ref = torch.nn.functional.layer_norm(exact[0], (d,), exact[1], exact[2], 1e-5)
+    want = torch.autograd.grad(ref, exact, dy.double())
+    for name, a, e in zip(("dx", "dw", "db"), got, want):
+        # one rounding of the result; fp32 inside (sums over a row or a column: relative 1e-5 of the norm)
+        assert (a.double() - e).norm() <= (_UNIT[dtype] + 2e-5) * e.norm() + 1e-6, (name, float((a.double() - e).norm() / e.norm()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,classes", [(1, 8), (3, 1000), (1023, 33), (1025, 2048), (130, 32003), (2049, 4096)])
+@pytest.mark.parametrize("reduction", ["mean", "sum"])
+def test_reduced_cross_entropy(bmt_gpu, dtype, rows, classes, reduction):
+    gen = torch.Generator(device="cuda").manual_seed(rows + classes)
+    x = (2 * torch.randn(rows, classes, generator=gen, device="cuda")).to(dtype).requires_grad_()
+    t = torch.randint(0, classes, (rows,), generator=gen, device="cuda")
+    t[1::5] = -100
+    loss = bmt_gpu.loss.FusedCrossEntropy(ignore_index=-100, reduction=reduction)(x, t)
+    assert loss.dtype == torch.float32 and loss.dim() == 0
+    (gx,) = torch.autograd.grad(loss * 64.0, (x,))
+    xe = x.detach().double().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(xe, t, ignore_index=-100, reduction=reduction)
+    (ge,) = torch.autograd.grad(ref * 64.0, (xe,))
+    assert abs(float(loss) - float(ref)) <= 3e-6 * abs(float(ref)) + 1e-6
+    # half types: one rounding, gradients below the smallest normal fp16 number lose bits
+    bound = 1.5 * _UNIT[dtype] * ge.norm() + (3e-8 * ge.numel() ** 0.5 if dtype == torch.float16 else 0) + 3e-6 * ge.norm()
+    assert (gx.double() - ge).norm() <= bound
+
+
+def test_reduced_cross_entropy_without_rows(bmt_gpu):
+    x = torch.randn(4, 64, device="cuda", dtype=torch.float16, requires_grad=True)
+    t = torch.full((4,), -100, device="cuda")
+    loss = bmt_gpu.loss.FusedCrossEntropy()(x, t)
+    assert torch.isnan(loss)
+    (g,) = torch.autograd.grad(loss, (x,))
+    assert not g.any()
+    assert float(bmt_gpu.loss.FusedCrossEntropy(reduction="sum")(x, t)) == 0.0
+    empty = torch.empty(0, 64, device="cuda", dtype=torch.float16)
+    assert torch.isnan(bmt_gpu.loss.FusedCrossEntropy()(empty, t[:0]))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens,rows,d", [(1, 1, 8), (65, 3, 8), (64, 1, 264), (700, 5, 2056), (2000, 4099, 512), (129, 70000, 64), (5000, 300, 96)])
+def test_embedding_gradient(bmt_gpu, dtype, tokens, rows, d):
+    from bmtrain_b200.ops import embedding as E
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens + rows)
+    ids = torch.randint(0, rows, (tokens,), generator=gen, device="cuda")
+    ids[torch.rand(tokens, generator=gen, device="cuda") < 0.1] = -1        # not in this shard
+    if tokens > 1000:
+        ids[:tokens // 3] = rows - 1                                        # one row far above the hot-row limit
+    g = torch.randn(tokens, d, generator=gen, device="cuda").to(dtype)
+    got = E.embedding_backward(ids, g, rows)
+    keep = ids >= 0
+    want = torch.zeros(rows, d, dtype=torch.float64, device="cuda").index_add_(0, ids[keep], g[keep].double())
+    size = torch.zeros(rows, d, dtype=torch.float64, device="cuda").index_add_(0, ids[keep], g[keep].double().abs())
+    assert got.dtype == dtype
+    assert (got.double() - want).abs().le(_UNIT[dtype] * want.abs() + tokens * 2.0 ** -24 * size + 1e-7).all()
