@@ -11,6 +11,7 @@
 
 #include "api.h"
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace {
 
@@ -374,31 +375,57 @@ int fwd(int64_t rows, int64_t d, const void* x, const void* w, const void* b, fl
     return (int)cudaGetLastError();
 }
 
-// Backward: a team of WPR warps per row, every lane owns fixed columns (VPL vectors of 8).  x and dy of the next row are on
-// their way while the current one is worked on, both are kept as packed 16-byte vectors between the statistics and the dx
-// pass, and the per-column sums of dy * xhat and dy accumulate in registers over all rows a lane sees; they are combined once
-// per CTA through shared memory into the scratch that norm_fold_kernel reduces.
-// HBM bytes bound it (x, dy in, dx out), so what counts is rows in flight: with up to 8 vectors a lane and no prefetch the
-// accumulators alone took 249 registers, eight warps a SM waited for their loads and the kernel ran at 0.41 of the copy rate
-// (16384 x 5120 RMS 180 us).  Wide teams keep a lane at 2 or 3 vectors, which leaves room for the prefetch and for 16 warps a SM;
-// RMSNorm (RMS) has no bias and drops the second accumulator.  One barrier per row: the partial sums alternate between two
-// sets of slots.
+// Backward: a team of WPR warps per row, every lane owns fixed columns (VPL vectors of 8).  The per-column sums of dy * xhat
+// and dy accumulate in registers over all rows a lane sees; they are combined once per CTA through shared memory into the
+// scratch that norm_fold_kernel reduces.
+// HBM bytes bound it (x, dy and the residual's gradient in, dx out), so what counts is bytes in flight.  Loading a row into
+// registers and then working on it ran at 0.41 of the copy rate (16384 x 5120 RMS 193 us), one row ahead in registers at 0.48
+// (160 us): a load takes longer than a row's arithmetic; it is 124 us now (LayerNorm 194 -> 171, bound by its arithmetic).  So whole rows come as bulk copies into a ring of up to BWD_STAGES
+// stages in shared memory, refilled by one thread right behind the barrier that every row has anyway; the rows' statistics
+// are fetched for BWD_BATCH rows at a time.  RMSNorm (RMS) has no bias and drops the second accumulator.
+constexpr int BWD_STAGES = 8, BWD_BATCH = 32;
+__device__ int g_norm_status = 0;   // 1 after a bounded wait for a bulk copy ran out
+
 template <int WPR> struct BwdTeam {
     static constexpr int THREADS = WPR == 16 ? 512 : 256, CTAS = WPR == 16 ? 1 : 2, RPC = THREADS / 32 / WPR;
 };
 
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
 template <typename T, int VPL, int WPR, bool RMS>
 __global__ void __launch_bounds__(BwdTeam<WPR>::THREADS, BwdTeam<WPR>::CTAS)
-norm_bwd_stream_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ w,
+norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ w,
                        const float* __restrict__ stats, T* __restrict__ dx, float* __restrict__ partial, const T* __restrict__ dres) {
     constexpr int RPC = BwdTeam<WPR>::RPC, WARPS = BwdTeam<WPR>::THREADS / 32;
-    constexpr bool AHEAD = VPL <= 3;                   // the next row's loads are issued before this row's arithmetic
-    __shared__ float ex[2][2][WARPS];
-    extern __shared__ float fold[];                    // 2 * d floats, for the final combination
+    extern __shared__ __align__(128) uint8_t ring[];   // stages x {x, dy[, dres]} x RPC rows; 2 * d floats at the end of the kernel
+    __shared__ __align__(8) uint64_t full[BWD_STAGES];
+    __shared__ float ex[2][2][WARPS], mu[BWD_BATCH * RPC], rs[BWD_BATCH * RPC];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = warp % WPR, slot = warp / WPR;
+    const uint32_t part_bytes = (uint32_t)(RPC * d * 2), stage_bytes = part_bytes * (dres ? 3 : 2);
+    const int64_t groups = (rows + RPC - 1) / RPC;
+    const int64_t n_it = (int64_t)blockIdx.x < groups ? (groups - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    auto refill = [&](int64_t it) {                    // one thread: the rows of iteration `it` into its stage
+        const int st = (int)(it % stages);
+        const int64_t r0 = (blockIdx.x + it * gridDim.x) * RPC;
+        const uint32_t bytes = (uint32_t)((rows - r0 < RPC ? rows - r0 : RPC) * d * 2);
+        const uint32_t bar = bmt_tc::smem_u32(&full[st]), dst = bmt_tc::smem_u32(ring) + st * stage_bytes;
+        bmt_tc::mbar_expect_tx_u32(bar, bytes * (dres ? 3u : 2u));
+        bulk_load(dst, x + r0 * d, bytes, bar);
+        bulk_load(dst + part_bytes, dy + r0 * d, bytes, bar);
+        if (dres) bulk_load(dst + 2 * part_bytes, dres + r0 * d, bytes, bar);
+    };
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < stages; ++i) bmt_tc::mbar_init(&full[i], 1);
+        bmt_tc::fence_barrier_init();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        for (int64_t it = 0; it < stages && it < n_it; ++it) refill(it);
+    }
     float dg[VPL][8], db[RMS ? 1 : VPL][8];
-    bmt::Vec16<T> wv[VPL], xv[VPL], gv[VPL], xn[VPL], gn[VPL];
+    bmt::Vec16<T> wv[VPL];
 #pragma unroll
     for (int v = 0; v < VPL; ++v) {
         const int c = ((v * WPR + sub) * 32 + lane) * 8;
@@ -406,38 +433,33 @@ norm_bwd_stream_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __
         for (int k = 0; k < 8; ++k) { dg[v][k] = 0.f; if (!RMS) db[v][k] = 0.f; }
         if (c < d) wv[v] = bmt::ld16(w + c);
     }
-    const int64_t groups = (rows + RPC - 1) / RPC;
-    float mean, rstd, mean_n, rstd_n;
-    auto load = [&](int64_t gi, bmt::Vec16<T>(&xx)[VPL], bmt::Vec16<T>(&gg)[VPL], float& mu, float& rs) {
-        const int64_t r = gi * RPC + slot;
-        const bool live = gi < groups && r < rows;
-        mu = live && !RMS ? stats[r] : 0.f;
-        rs = live ? stats[rows + r] : 0.f;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-            const int c = ((v * WPR + sub) * 32 + lane) * 8;
-            if (live && c < d) { xx[v] = bmt::ld16(x + r * d + c); gg[v] = bmt::ld16(dy + r * d + c); }
-        }
-    };
-    load(blockIdx.x, xv, gv, mean, rstd);
-    int par = 0;
-    for (int64_t gi = blockIdx.x; gi < groups; gi += gridDim.x, par ^= 1) {
-        const int64_t r = gi * RPC + slot;
+    __syncthreads();
+    int st = 0;
+    uint32_t phase = 0;
+    for (int64_t it = 0; it < n_it; ++it) {
+        const int64_t r = (blockIdx.x + it * gridDim.x) * RPC + slot;
         const bool live = r < rows;
-        if (AHEAD) load(gi + gridDim.x, xn, gn, mean_n, rstd_n);
-        bmt::Vec16<T> rv[VPL];
-        if (dres) {
-#pragma unroll
-            for (int v = 0; v < VPL; ++v) {
-                const int c = ((v * WPR + sub) * 32 + lane) * 8;
-                if (live && c < d) rv[v] = bmt::ld16(dres + r * d + c);
+        if (it % BWD_BATCH == 0) {
+            __syncthreads();                           // the previous batch has been read
+            for (int i = threadIdx.x; i < BWD_BATCH * RPC; i += BwdTeam<WPR>::THREADS) {
+                const int64_t rr = (blockIdx.x + (it + i / RPC) * gridDim.x) * RPC + i % RPC;
+                mu[i] = rr < rows && !RMS ? stats[rr] : 0.f;
+                rs[i] = rr < rows ? stats[rows + rr] : 0.f;
             }
+            __syncthreads();
         }
+        const float mean = mu[(it % BWD_BATCH) * RPC + slot], rstd = rs[(it % BWD_BATCH) * RPC + slot];
+        if (!bmt_tc::mbar_wait(&full[st], phase)) atomicExch(&g_norm_status, 1);
+        const T* xs = reinterpret_cast<const T*>(ring + st * stage_bytes) + slot * d;
+        const T* gs = reinterpret_cast<const T*>(ring + st * stage_bytes + part_bytes) + slot * d;
+        bmt::Vec16<T> xv[VPL], gv[VPL];
         float s1 = 0.f, s2 = 0.f;
 #pragma unroll
         for (int v = 0; v < VPL; ++v) {
             const int c = ((v * WPR + sub) * 32 + lane) * 8;
             if (live && c < d) {
+                xv[v] = bmt::ld16(xs + c);
+                gv[v] = bmt::ld16(gs + c);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const float xh = (bmt::Cvt<T>::to_f(xv[v].v[k]) - mean) * rstd;
@@ -452,41 +474,41 @@ norm_bwd_stream_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __
         }
         if (!RMS) s1 = bmt::warp_sum(s1);
         s2 = bmt::warp_sum(s2);
+        const int par = (int)(it & 1);
+        if (WPR > 1 && lane == 0) { ex[par][0][warp] = s1; ex[par][1][warp] = s2; }
+        __syncthreads();
+        // every warp is through with the previous row: its stage takes the row `stages - 1` ahead of this one
+        if (threadIdx.x == 0 && it > 0 && it - 1 + stages < n_it) refill(it - 1 + stages);
         if (WPR > 1) {
-            if (lane == 0) { ex[par][0][warp] = s1; ex[par][1][warp] = s2; }
-            __syncthreads();
             s1 = s2 = 0.f;
 #pragma unroll
             for (int i = 0; i < WPR; ++i) { if (!RMS) s1 += ex[par][0][slot * WPR + i]; s2 += ex[par][1][slot * WPR + i]; }
         }
         s1 = s1 / d;
         s2 = s2 / d;
+        const T* ds = reinterpret_cast<const T*>(ring + st * stage_bytes + 2 * part_bytes) + slot * d;
 #pragma unroll
         for (int v = 0; v < VPL; ++v) {
             const int c = ((v * WPR + sub) * 32 + lane) * 8;
             if (live && c < d) {
-                bmt::Vec16<T> o;
+                bmt::Vec16<T> o, rv;
+                if (dres) rv = bmt::ld16(ds + c);
+                const bmt::Vec16<T> xc = VPL > 3 ? bmt::ld16(xs + c) : xv[v], gc = VPL > 3 ? bmt::ld16(gs + c) : gv[v];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
-                    const float xh = (bmt::Cvt<T>::to_f(xv[v].v[k]) - mean) * rstd;
-                    const float wg = bmt::Cvt<T>::to_f(gv[v].v[k]) * bmt::Cvt<T>::to_f(wv[v].v[k]);
+                    const float xh = (bmt::Cvt<T>::to_f(xc.v[k]) - mean) * rstd;
+                    const float wg = bmt::Cvt<T>::to_f(gc.v[k]) * bmt::Cvt<T>::to_f(wv[v].v[k]);
                     float val = rstd * (wg - s1 - xh * s2);
-                    if (dres) val += bmt::Cvt<T>::to_f(rv[v].v[k]);
+                    if (dres) val += bmt::Cvt<T>::to_f(rv.v[k]);
                     o.v[k] = bmt::Cvt<T>::from_f(val);
                 }
                 bmt::st16(dx + r * d + c, o);
             }
         }
-        if (AHEAD) {
-            mean = mean_n;
-            rstd = rstd_n;
-#pragma unroll
-            for (int v = 0; v < VPL; ++v) { xv[v] = xn[v]; gv[v] = gn[v]; }
-        } else {
-            load(gi + gridDim.x, xv, gv, mean, rstd);
-        }
+        if (++st == stages) { st = 0; phase ^= 1; }
     }
-    // combine the RPC row slots of this CTA: slot 0 ends up with the CTA's column sums
+    // combine the RPC row slots of this CTA (slot 0 ends up with the CTA's column sums); every copy into the ring has landed
+    float* fold = reinterpret_cast<float*>(ring);
     float* pg = partial + (int64_t)blockIdx.x * d;
     float* pb = partial + ((int64_t)gridDim.x + blockIdx.x) * d;
     for (int s_ = 1; s_ < RPC; ++s_) {
@@ -528,21 +550,27 @@ norm_bwd_stream_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __
     }
 }
 
-// Returns the number of CTAs (rows of partial sums per accumulator) that were launched.
+// Returns the number of CTAs (rows of partial sums per accumulator) that were launched, or a negative code.
 template <typename T, int VPL, int WPR>
 int launch_bwd_stream(int64_t rows, int d, const void* x, const void* dy, const void* w, const void* stats, int rms, int nblk, void* dx,
                       void* partial, const void* dres, cudaStream_t s) {
     using Team = BwdTeam<WPR>;
-    const size_t smem = Team::RPC > 1 ? (size_t)2 * d * sizeof(float) : 0;   // at most 2 * 3072 floats where rows share a CTA
+    // the ring: as many stages as fit the CTA's share of the shared memory; at least two (16384 columns with a residual: 192 KiB)
+    const size_t budget = (size_t)(Team::CTAS == 1 ? 208 : 100) * 1024, stage = (size_t)Team::RPC * d * 2 * (dres ? 3 : 2);
+    int stages = (int)(budget / stage);
+    if (stages > BWD_STAGES) stages = BWD_STAGES;
+    size_t smem = stages * stage;
+    if (Team::RPC > 1 && smem < (size_t)2 * d * sizeof(float)) smem = (size_t)2 * d * sizeof(float);
     int64_t grid = (rows + Team::RPC - 1) / Team::RPC;
     if (grid > 148 * Team::CTAS) grid = 148 * Team::CTAS;
     if (grid > nblk) grid = nblk;
-    if (rms) norm_bwd_stream_kernel<T, VPL, WPR, true><<<(unsigned)grid, Team::THREADS, smem, s>>>(rows, d, (const T*)x, (const T*)dy, (const T*)w,
-                                                                                                (const float*)stats, (T*)dx, (float*)partial, (const T*)dres);
-    else if constexpr (VPL != 3 || WPR == 16)   // narrower teams have at most 2 vectors a lane here
-        norm_bwd_stream_kernel<T, VPL, WPR, false><<<(unsigned)grid, Team::THREADS, smem, s>>>(rows, d, (const T*)x, (const T*)dy, (const T*)w,
-                                                                                               (const float*)stats, (T*)dx, (float*)partial, (const T*)dres);
-    return (int)grid;
+    const auto run = [&](auto kernel) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) != cudaSuccess) return -30;
+        kernel<<<(unsigned)grid, Team::THREADS, smem, s>>>(rows, d, stages, (const T*)x, (const T*)dy, (const T*)w, (const float*)stats, (T*)dx,
+                                                           (float*)partial, (const T*)dres);
+        return (int)grid;
+    };
+    return rms ? run(norm_bwd_stream_kernel<T, VPL, WPR, true>) : run(norm_bwd_stream_kernel<T, VPL, WPR, false>);
 }
 
 template <typename T, int WPR, typename... Args>
@@ -563,8 +591,8 @@ int bwd(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, c
     };
     static const bool use_reg = [] { const char* e = getenv("BMT_NORM_STAGED"); return !(e && atoi(e) == 1); }();
     if (use_reg && d <= 16384 && !(rms && db)) {
-        // the narrowest team whose lanes need no register spills: 3 vectors for RMSNorm, 2 with the bias sums; beyond that
-        // (above 12288 / 8192 columns) the widest team
+        // the narrowest team with at most 3 vectors a lane, 2 with the bias sums (LayerNorm 16384 x 5120: 223 us with 3,
+        // 171 with 2); above 12288 / 8192 columns the widest team
         const int64_t nv = (d + 255) / 256, most = rms ? 3 : 2;   // nv: vectors a lane of one warp would have
         const int wpr = nv <= most ? 1 : nv <= 2 * most ? 2 : nv <= 4 * most ? 4 : nv <= 8 * most ? 8 : 16;
         const int vpl = (int)((nv + wpr - 1) / wpr);
@@ -573,6 +601,7 @@ int bwd(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, c
                          : wpr == 4 ? bwd_stream_vpl<T, 4>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s)
                          : wpr == 8 ? bwd_stream_vpl<T, 8>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s)
                                     : bwd_stream_vpl<T, 16>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s);
+        if (blocks < 0) return blocks;
         fold(blocks);
         bmt_count_launch(2);
         return (int)cudaGetLastError();
