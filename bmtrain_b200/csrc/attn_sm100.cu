@@ -45,7 +45,7 @@ struct AttnParams {
 
 struct AttnShared {
     uint64_t q_full, k_full[2], v_full[2], k_empty[2], v_empty[2];
-    uint64_t s_full[2], p_ready[2], o_full[2];
+    uint64_t s_full[2], p_half[2], p_ready[2], o_full[2];
     uint32_t tmem_base;
     int failed;
 };
@@ -133,28 +133,31 @@ attn_mask_pack_kernel(const uint8_t* mask, int64_t sq, int64_t sk, uint32_t* bit
     const int64_t q0 = (int64_t)qt * TILE, k0 = (int64_t)kt * TILE;
     if (threadIdx.x == 0) { any = 0; full = 1; }
     __syncthreads();
-    for (int r = warp; r < TILE; r += MASK_THREADS / 32) {
-        const int64_t q = q0 + r;
-        uint32_t word[4];
+    // a warp takes 16 rows, 8 at a time: 32 loads in flight, then the ballots
+    for (int r0 = warp * 16; r0 < warp * 16 + 16; r0 += 8) {
+        uint8_t byte[8][4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int64_t k = k0 + c * 32 + lane;
-            const bool on = q < sq && k < sk && mask[((int64_t)b * sq + q) * sk + k] != 0;
-            word[c] = __ballot_sync(0xffffffffu, on);
-        }
-        if (lane == 0) {
-            uint32_t seen = 0;
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int64_t q = q0 + r0 + i, k = k0 + c * 32 + lane;
+                byte[i][c] = q < sq && k < sk ? mask[((int64_t)b * sq + q) * sk + k] : 0;
+            }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            uint32_t word[4], seen = 0;
             bool all = true;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                w[r][c] = word[c];
+                word[c] = __ballot_sync(0xffffffffu, byte[i][c] != 0);
                 seen |= word[c];
                 all = all && word[c] == low_bits(sk - (k0 + c * 32));
             }
-            if (q < sq) {
+            if (lane < 4) w[r0 + i][lane] = lane == 0 ? word[0] : lane == 1 ? word[1] : lane == 2 ? word[2] : word[3];
+            if (lane == 0 && q0 + r0 + i < sq) {
                 if (seen) any = 1;
                 if (!all) full = 0;
-                *reinterpret_cast<uint4*>(bits + ((((int64_t)b * sq + q) * n_kt) + kt) * 4) = make_uint4(word[0], word[1], word[2], word[3]);
+                *reinterpret_cast<uint4*>(bits + ((((int64_t)b * sq + q0 + r0 + i) * n_kt) + kt) * 4) = make_uint4(word[0], word[1], word[2], word[3]);
             }
         }
     }
@@ -224,7 +227,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         mbar_init(&sh->q_full, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&sh->k_full[i], 1); mbar_init(&sh->v_full[i], 1); mbar_init(&sh->k_empty[i], 1); mbar_init(&sh->v_empty[i], 1);
-            mbar_init(&sh->s_full[i], 1); mbar_init(&sh->p_ready[i], 4); mbar_init(&sh->o_full[i], 1);
+            mbar_init(&sh->s_full[i], 1); mbar_init(&sh->p_half[i], 4); mbar_init(&sh->p_ready[i], 4); mbar_init(&sh->o_full[i], 1);
         }
         sh->failed = 0;
         fence_barrier_init();
@@ -314,18 +317,23 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
                     if (active(t, j)) {
-                        // P_t is in tensor memory and, if row maxima moved, O_t has been rescaled by its owners
-                        if (!mbar_wait_warp(smem_u32(&sh->p_ready[t]), done[t] & 1u)) { if (lane == 0) fail(sh, 6); ok = false; break; }
-                        tc_fence_after();
-                        if (elect_one()) {
+                        // the first 64 keys of P_t are in tensor memory and, if row maxima moved, O_t has been rescaled by its
+                        // owners; the second half of the softmax runs under the first half of the MMAs
 #pragma unroll
-                            for (int ks = 0; ks < TILE / 16; ++ks)
-                                // B = V (128 keys x head dim, head dim contiguous = MN-major): 16 key rows per step, 64-column chunks CHUNK apart
-                                umma_f16_ts(tmem + 256 + t * TILE, tmem + t * TILE + ks * 8, pack_desc(desc_lo(sV + st * TB + ks * 2048, CHUNK), hi),
-                                            p.idesc_pv, (done[t] | ks) != 0 ? 1u : 0u);
-                            if (j == last[t]) umma_commit(&sh->o_full[t]);
+                        for (int half = 0; half < 2; ++half) {
+                            if (!mbar_wait_warp(smem_u32(half ? &sh->p_ready[t] : &sh->p_half[t]), done[t] & 1u)) { if (lane == 0) fail(sh, 6); ok = false; break; }
+                            tc_fence_after();
+                            if (elect_one()) {
+#pragma unroll
+                                for (int ks = half * 4; ks < half * 4 + 4; ++ks)
+                                    // B = V (128 keys x head dim, head dim contiguous = MN-major): 16 key rows per step, 64-column chunks CHUNK apart
+                                    umma_f16_ts(tmem + 256 + t * TILE, tmem + t * TILE + ks * 8, pack_desc(desc_lo(sV + st * TB + ks * 2048, CHUNK), hi),
+                                                p.idesc_pv, (done[t] | ks) != 0 ? 1u : 0u);
+                                if (half == 1 && j == last[t]) umma_commit(&sh->o_full[t]);
+                            }
+                            __syncwarp();
                         }
-                        __syncwarp();
+                        if (!ok) break;
                         ++done[t];
                     }
                     if (jn < J_max && active(t, jn)) {
@@ -442,11 +450,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                     pk[i] = pack2<T>(x, y);
                 }
                 tmem_st32(s_addr + half * 32, pk);     // over the scores: this thread's row, already in registers
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(half ? &sh->p_ready[t] : &sh->p_half[t]);
             }
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh->p_ready[t]);
             float s0, s1;
             unpack_f2(add_f2(sum2[0], sum2[1]), s0, s1);
             l_run = l_run * alpha + (s0 + s1);
@@ -535,6 +543,7 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
 //         tensor memory as packed 16-bit pairs, over S^T; dS = P * (dP - delta) * scale as 16 bits into shared memory,
 //         [key][query] swizzled: K-major A for dK and, read "transposed", MN-major A for dQ = dS K
 //   MMA   dV += P^T dO (P from tensor memory), dK += dS^T Q, dQ = dS K
+//   one warp fetches lse and delta of the tiles to come
 //   dQ warps (4): add the tile of dQ to an fp32 accumulator in global memory (bulk reductions out of shared memory, 32 columns
 //         at a time; vector reductions by the threads themselves took 4300 clocks a tile); a small kernel converts it
 // delta = rowsum(dO * O) comes from a pre-pass.  dK / dV are written once at the end, already summed over the group.
@@ -565,7 +574,7 @@ constexpr int BWD_THREADS = 512;                 // 8 softmax warps, 4 dQ warps,
 
 struct BwdShared {
     alignas(16) uint64_t kv_full; uint64_t q_full[2], q_empty[2], do_full, do_empty, s_full, dp_full, p_ready, ds_ready, dq_full, dq_empty, all_done;
-    uint64_t row_full[2], row_empty[2], pair[4];
+    uint64_t row_full[2], row_empty[2];
     float nlse[2][TILE], ndelta[2][TILE];        // per query of a tile: -lse * log2(e) (0 for rows that take no part), -delta * scale
     uint32_t live[2][4];                         // queries of the tile that exist and see at least one key
     uint32_t tmem_base;
@@ -625,9 +634,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
 
     if (threadIdx.x == 0) {
         mbar_init(&sh->kv_full, 1); mbar_init(&sh->do_full, 1); mbar_init(&sh->do_empty, 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(&sh->q_full[i], 1); mbar_init(&sh->q_empty[i], 1); mbar_init(&sh->row_full[i], 4); mbar_init(&sh->row_empty[i], 8); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&sh->q_full[i], 1); mbar_init(&sh->q_empty[i], 1); mbar_init(&sh->row_full[i], 1); mbar_init(&sh->row_empty[i], 8); }
         mbar_init(&sh->s_full, 1); mbar_init(&sh->dp_full, 1); mbar_init(&sh->p_ready, 8); mbar_init(&sh->ds_ready, 8);
-        for (int i = 0; i < 4; ++i) mbar_init(&sh->pair[i], 2);
         mbar_init(&sh->dq_full, 1); mbar_init(&sh->dq_empty, 4); mbar_init(&sh->all_done, 1);
         sh->failed = 0;
         fence_barrier_init();
@@ -715,7 +723,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 if (elect_one()) {
 #pragma unroll
                     for (int ks = 0; ks < TILE / 16; ++ks)      // dV += P^T dO: 16 queries per step, dO MN-major
-                        umma_f16_ts(tmem + C_DV, tmem + ks * 8, pack_desc(desc_lo(sdO + ks * 2048, CHUNK), hi), p.idesc_dv, (it | (uint32_t)ks) != 0 ? 1u : 0u);
+                        umma_f16_ts(tmem + C_DV, tmem + (ks >> 2) * 64 + (ks & 3) * 8, pack_desc(desc_lo(sdO + ks * 2048, CHUNK), hi), p.idesc_dv, (it | (uint32_t)ks) != 0 ? 1u : 0u);
                     umma_commit(&sh->do_empty);
                 }
                 __syncwarp();
@@ -738,6 +746,30 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 }
                 __syncwarp();
             }
+        }
+    } else if (warp == 14) {
+        // ------------------------------------------------------------------------------------------ row statistics, up to two tiles ahead
+        for (uint32_t it = 0; walk.more(); walk.next(), ++it) {
+            const uint32_t st = it & 1;
+            if (!mbar_wait_warp(smem_u32(&sh->row_empty[st]), ((it >> 1) & 1) ^ 1)) { if (lane == 0) fail_bwd(sh, 15); break; }
+            const int64_t q0 = (int64_t)walk.qt * TILE + lane, at = ((int64_t)b * p.h + walk.head) * p.sq + q0;
+            float l[4], dl[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const bool in = q0 + i * 32 < p.sq;
+                l[i] = in ? p.lse[at + i * 32] : -INFINITY;
+                dl[i] = in ? p.delta[at + i * 32] : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const bool alive = l[i] != -INFINITY;
+                sh->nlse[st][i * 32 + lane] = alive ? -l[i] * 1.4426950408889634f : 0.f;
+                sh->ndelta[st][i * 32 + lane] = -dl[i] * p.scale;
+                const uint32_t bits = __ballot_sync(0xffffffffu, alive);
+                if (lane == 0) sh->live[st][i] = bits;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->row_full[st]);
         }
     }
     } else if (warp < 8) {
@@ -779,13 +811,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             tmem_ld32(tmem + lane_addr + part * 64, s[0]);
             tmem_ld32(tmem + lane_addr + part * 64 + 32, s[1]);
             tmem_ld_wait();
-            // the other warp of these 32 keys still reads S^T columns that P^T goes over (packed columns [0,64) are queries
-            // [0,64) of S^T): both halves have to be in registers before either is written
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh->pair[quarter]);
-            if (!warp_wait(&sh->pair[quarter], ph, lane)) { if (lane == 0) fail_bwd(sh, 17); ok = false; break; }
-            tc_fence_after();
             float pr[64];
             uint32_t pk[32];
 #pragma unroll
@@ -804,7 +829,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 pk[2 * i] = pack2<T>(x[0], x[1]);
                 pk[2 * i + 1] = pack2<T>(x[2], x[3]);
             }
-            tmem_st32(tmem + lane_addr + part * 32, pk);
+            // over this warp's own half of the scores: queries [0,64) go to columns [0,32), queries [64,128) to [64,96)
+            tmem_st32(tmem + lane_addr + part * 64, pk);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -875,37 +901,12 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             tc_fence_before();
         }
     } else {
-        // ------------------------------------------------------------------------------------------ row statistics, dQ
+        // ------------------------------------------------------------------------------------------ dQ
         regs_up<152>();
         const int quarter = warp & 3, r0 = quarter * 32;
         const uint32_t lane_addr = (uint32_t)r0 << 16, xbuf = sX + (uint32_t)(warp - 8) * DQ_BUF;
         bool ok = true;
-        BwdWalk ahead = walk;                    // the tile whose row statistics are fetched next: one ahead of the dQ tile
-        uint32_t n_rows = 0;
-        auto fetch_rows = [&]() -> bool {
-            const uint32_t st = n_rows & 1;
-            if (!warp_wait(&sh->row_empty[st], ((n_rows >> 1) & 1) ^ 1, lane)) { if (lane == 0) fail_bwd(sh, 15); return false; }
-            const int64_t qi = (int64_t)ahead.qt * TILE + r0 + lane;
-            float l = -INFINITY, dl = 0.f;
-            if (qi < p.sq) {
-                const int64_t at = ((int64_t)b * p.h + ahead.head) * p.sq + qi;
-                l = p.lse[at];
-                dl = p.delta[at];
-            }
-            const bool alive = l != -INFINITY;
-            sh->nlse[st][r0 + lane] = alive ? -l * 1.4426950408889634f : 0.f;
-            sh->ndelta[st][r0 + lane] = -dl * p.scale;
-            const uint32_t bits = __ballot_sync(0xffffffffu, alive);
-            if (lane == 0) sh->live[st][quarter] = bits;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh->row_full[st]);
-            ++n_rows;
-            ahead.next();
-            return true;
-        };
-        if (work) ok = fetch_rows();
         for (uint32_t it = 0; walk.more() && ok; walk.next(), ++it) {
-            if (ahead.more() && !fetch_rows()) { ok = false; break; }
             if (!warp_wait(&sh->dq_full, it & 1, lane)) { if (lane == 0) fail_bwd(sh, 16); ok = false; break; }
             tc_fence_after();
             uint32_t r[HD / 32][32];
