@@ -570,7 +570,8 @@ int launch_bwd_stream(int64_t rows, int d, const void* x, const void* dy, const 
                                                            (float*)partial, (const T*)dres);
         return (int)grid;
     };
-    return rms ? run(norm_bwd_stream_kernel<T, VPL, WPR, true>) : run(norm_bwd_stream_kernel<T, VPL, WPR, false>);
+    if constexpr (VPL == 3 && WPR < 16) return rms ? run(norm_bwd_stream_kernel<T, VPL, WPR, true>) : -31;   // LayerNorm: 2 vectors at most
+    else return rms ? run(norm_bwd_stream_kernel<T, VPL, WPR, true>) : run(norm_bwd_stream_kernel<T, VPL, WPR, false>);
 }
 
 template <typename T, int WPR, typename... Args>

@@ -66,10 +66,14 @@ def flash_usable(q, k, v) -> bool:
     return True
 
 
+def packed_mask_bytes(b: int, sq: int, sk: int) -> int:
+    qt, kt = (sq + 127) // 128, (sk + 127) // 128
+    return b * (16 * (sq * kt + sk * qt) + qt * kt)
+
+
 def packed_mask_buffer(b: int, sq: int, sk: int, device) -> torch.Tensor:
     """Room for a dense mask as bits: by query, by key, and a class per 128 x 128 tile (``bmt_attn_mask_pack``)."""
-    qt, kt = (sq + 127) // 128, (sk + 127) // 128
-    return torch.empty(b * (16 * (sq * kt + sk * qt) + qt * kt), dtype=torch.uint8, device=device)
+    return torch.empty(packed_mask_bytes(b, sq, sk), dtype=torch.uint8, device=device)
 
 
 def pack_mask(mask8: Optional[torch.Tensor], b: int, sq: int, sk: int) -> Optional[torch.Tensor]:

@@ -139,7 +139,8 @@ _scratch = {}
 def colsum_scratch(dev) -> torch.Tensor:
     """Work space of the row-split column sums (4 KB of ticket counters + partial sums), one per device and stream, zeroed
     once: the kernel leaves the counters at zero, and calls that share it are ordered on their stream."""
-    key = (str(dev), torch.cuda.current_stream(dev).cuda_stream)
+    index = dev.index if dev.index is not None else torch.cuda.current_device()
+    key = (index, torch._C._cuda_getCurrentRawStream(index))
     buf = _scratch.get(key)
     if buf is None:
         buf = _scratch[key] = torch.zeros(1024 + 2 * 1024 * 1024, dtype=torch.float32, device=dev)

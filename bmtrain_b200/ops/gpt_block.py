@@ -8,6 +8,8 @@ does before backward), which removes the separate accumulate pass.
 from __future__ import annotations
 
 import ctypes
+import functools
+import os
 from typing import Optional
 
 import torch
@@ -60,27 +62,55 @@ def _as_bytes(mask: torch.Tensor) -> torch.Tensor:
     return mask.to(torch.uint8).contiguous()
 
 
-def _fill(blk: _Block, x, y, mask, params, saved, n_heads, d_head, act, eps, causal):
-    b, s, d = x.shape
-    blk.batch, blk.seq, blk.d_model, blk.n_heads, blk.d_head = b, s, d, n_heads, d_head
-    blk.d_ff = params[8].shape[0]
-    blk.dtype = 0 if x.dtype == torch.float16 else 1
-    blk.act = 1 if act == "relu" else 2
-    blk.eps, blk.causal = eps, 1 if causal else 0
-    blk.mask = None if mask is None else mask.data_ptr()
-    for name, p in zip(_PARAM_NAMES, params):
-        setattr(blk, name, p.data_ptr())
-    blk.x, blk.y = x.data_ptr(), y.data_ptr()
-    for name in ("ln1", "stats1", "qkv", "ctx", "h1", "ln2", "stats2", "ff"):
-        setattr(blk, name, saved[name].data_ptr())
-    if saved.get("lse") is not None:
-        # fused attention: scores and probabilities never reach memory, one log-sum-exp per row is kept instead
-        blk.lse, blk.probs, blk.probs_ld = saved["lse"].data_ptr(), None, 0
+def _carve(sizes):
+    """Offsets of buffers of the given byte sizes inside one allocation (256-byte aligned), and its size.  One allocation per
+    pass: at 1024 tokens the host is what bounds a block, and twenty tensors cost it 40 us a block."""
+    offsets, at = {}, 0
+    for name, n in sizes:
+        offsets[name] = at
+        at += (n + 255) // 256 * 256
+    return offsets, at
+
+
+@functools.lru_cache(maxsize=256)
+def _saved_plan(b, s, d, n_heads, d_head, dff, gelu, fused_attn, masked):
+    """What forward keeps for backward (16-bit activations, fp32 statistics)."""
+    T, hd = b * s, n_heads * d_head
+    sizes = [("ln1", 2 * T * d), ("stats1", 8 * T), ("qkv", 6 * T * hd), ("ctx", 2 * T * hd), ("h1", 2 * T * d), ("ln2", 2 * T * d),
+             ("stats2", 8 * T), ("ff", 2 * T * dff)]
+    if fused_attn:
+        sizes.append(("lse", 4 * b * n_heads * s))
+        if masked:
+            sizes.append(("mask_packed", _attn.packed_mask_bytes(b, s, s)))
     else:
-        blk.lse, blk.probs, blk.probs_ld = None, saved["probs"].data_ptr(), saved["probs"].stride(2)
-    packed = saved.get("mask_packed")
-    blk.mask_packed = None if packed is None else packed.data_ptr()
-    blk.pre = saved["pre"].data_ptr() if saved.get("pre") is not None else None
+        sizes.append(("probs", 2 * b * n_heads * s * ((s + 7) // 8 * 8)))
+    if gelu:
+        sizes.append(("pre", 2 * T * dff))
+    return _carve(sizes)
+
+
+@functools.lru_cache(maxsize=256)
+def _work_plan(b, s, d, n_heads, d_head, dff, fused_attn, nblk):
+    """Scratch of a backward pass."""
+    T, hd = b * s, n_heads * d_head
+    sizes = [("d_ff", 2 * T * dff), ("d_ln2", 2 * T * d), ("d_h1", 2 * T * d), ("d_ctx", 2 * T * hd), ("d_qkv", 6 * T * hd),
+             ("norm_partial", 8 * nblk * d)]
+    if fused_attn:
+        sizes += [("dq_acc", 4 * T * hd), ("delta", 4 * b * n_heads * s)]
+    else:
+        sizes.append(("d_probs", 2 * b * n_heads * s * ((s + 7) // 8 * 8)))
+    return _carve(sizes)
+
+
+def _describe(x, y, mask, params, saved, plan, n_heads, d_head, act, eps, causal):
+    """The block as the native executor takes it; ``saved``: address of the buffer that ``plan`` divides."""
+    b, s, d = x.shape
+    at = lambda name: saved + plan[name] if name in plan else None  # noqa: E731
+    # fused attention: scores and probabilities never reach memory, one log-sum-exp per row is kept instead
+    return _Block(b, s, d, n_heads, d_head, params[8].shape[0], 0 if x.dtype == torch.float16 else 1, 1 if act == "relu" else 2, eps,
+                  1 if causal else 0, None if mask is None else mask.data_ptr(), *[p.data_ptr() for p in params], x.data_ptr(),
+                  y.data_ptr(), at("ln1"), at("stats1"), at("qkv"), at("probs"), (s + 7) // 8 * 8 if "probs" in plan else 0,
+                  at("ctx"), at("h1"), at("ln2"), at("stats2"), at("ff"), at("pre"), at("lse"), at("mask_packed"))
 
 
 class GPTBlockFunction(torch.autograd.Function):
@@ -89,27 +119,13 @@ class GPTBlockFunction(torch.autograd.Function):
         lib = _native.cuda_lib()
         x = x.contiguous()
         b, s, d = x.shape
-        T, hd, dff = b * s, n_heads * d_head, params[8].shape[0]
-        dev, dt = x.device, x.dtype
-        sp = (s + 7) // 8 * 8
+        dff = params[8].shape[0]
         mask8 = None if mask is None else _as_bytes(mask)
-        import os
-
         fused_attn = d_head % 16 == 0 and d_head <= 128 and os.environ.get("BMT_FLASH_ATTN", "1") != "0"
-        saved = {
-            "ln1": torch.empty(T, d, dtype=dt, device=dev), "stats1": torch.empty(2, T, dtype=torch.float32, device=dev),
-            "qkv": torch.empty(T, 3 * hd, dtype=dt, device=dev),
-            "probs": None if fused_attn else torch.empty(b, n_heads, s, sp, dtype=dt, device=dev),
-            "lse": torch.empty(b, n_heads, s, dtype=torch.float32, device=dev) if fused_attn else None,
-            "ctx": torch.empty(T, hd, dtype=dt, device=dev), "h1": torch.empty(T, d, dtype=dt, device=dev),
-            "ln2": torch.empty(T, d, dtype=dt, device=dev), "stats2": torch.empty(2, T, dtype=torch.float32, device=dev),
-            "ff": torch.empty(T, dff, dtype=dt, device=dev),
-            "pre": torch.empty(T, dff, dtype=dt, device=dev) if act == "gelu" else None,
-            "mask_packed": _attn.packed_mask_buffer(b, s, s, dev) if fused_attn and mask8 is not None else None,
-        }
+        plan, total = _saved_plan(b, s, d, n_heads, d_head, dff, act == "gelu", fused_attn, mask8 is not None)
+        saved = torch.empty(total, dtype=torch.uint8, device=x.device)
         y = torch.empty_like(x)
-        blk = _Block()
-        _fill(blk, x, y, mask8, params, saved, n_heads, d_head, act, eps, causal)
+        blk = _describe(x, y, mask8, params, saved.data_ptr(), plan, n_heads, d_head, act, eps, causal)
         if deferred is None:
             _native.check(lib.bmt_gpt_block_forward(ctypes.byref(blk), _native.stream_handle()), "GPT block forward")
         else:
@@ -117,9 +133,11 @@ class GPTBlockFunction(torch.autograd.Function):
             # that consumes it; the other big weights travel on the peer stream and have the attention core's duration to
             # arrive before the output projection.  They start together with the GEMM ("before") or when it is done
             # ("after", so that the QKV weight has the links to itself): BMT_REST_PUSH, default by group size.
-            import os
-
             from ..parallel import fused_ops
+
+            T, hd = b * s, n_heads * d_head
+            ln1 = saved[plan["ln1"]:plan["ln1"] + 2 * T * d].view(x.dtype).view(T, d)
+            qkv = saved[plan["qkv"]:plan["qkv"] + 6 * T * hd].view(x.dtype).view(T, 3 * hd)
 
             cur = torch.cuda.current_stream()
             cur.wait_event(deferred["ev_small"])
@@ -127,31 +145,29 @@ class GPTBlockFunction(torch.autograd.Function):
             when = os.environ.get("BMT_REST_PUSH") or ("before" if deferred["bucket"].comm.size <= 2 else "after")
             if when == "before":
                 ev_rest = deferred["push_rest"]()
-                fused_ops.zero_gather_gemm(saved["ln1"], saved["qkv"], params[3], deferred)
+                fused_ops.zero_gather_gemm(ln1, qkv, params[3], deferred)
             else:
-                fused_ops.zero_gather_gemm(saved["ln1"], saved["qkv"], params[3], deferred)
+                fused_ops.zero_gather_gemm(ln1, qkv, params[3], deferred)
                 ev_gemm = torch.cuda.Event()
                 ev_gemm.record(cur)
                 ev_rest = deferred["push_rest"](ev_gemm)
             _native.check(lib.bmt_gpt_block_forward_steps(ctypes.byref(blk), 3, 5, _native.stream_handle()), "GPT block forward")
             cur.wait_event(ev_rest)
             _native.check(lib.bmt_gpt_block_forward_steps(ctypes.byref(blk), 6, 9, _native.stream_handle()), "GPT block forward")
-        ctx.saved, ctx.x, ctx.mask8, ctx.params = saved, x, mask8, params
-        ctx.cfg = (n_heads, d_head, act, eps, causal)
+        ctx.saved, ctx.plan, ctx.x, ctx.mask8, ctx.params = saved, plan, x, mask8, params
+        ctx.cfg = (n_heads, d_head, act, eps, causal, fused_attn)
         return y
 
     @staticmethod
     def backward(ctx, dy):
         lib = _native.cuda_lib()
         x, saved, params = ctx.x, ctx.saved, ctx.params
-        n_heads, d_head, act, eps, causal = ctx.cfg
+        n_heads, d_head, act, eps, causal, fused_attn = ctx.cfg
         b, s, d = x.shape
-        T, hd, dff = b * s, n_heads * d_head, params[8].shape[0]
         dev, dt = x.device, x.dtype
         dy = dy.contiguous()
-        blk = _Block()
-        y_dummy = dy  # forward output pointer is not read by backward
-        _fill(blk, x, y_dummy, ctx.mask8, params, saved, n_heads, d_head, act, eps, causal)
+        # (the forward output's pointer is not read by backward)
+        blk = _describe(x, dy, ctx.mask8, params, saved.data_ptr(), ctx.plan, n_heads, d_head, act, eps, causal)
         g = _Grad()
         dx = torch.empty_like(x)
         g.dy, g.dx = dy.data_ptr(), dx.data_ptr()
@@ -179,18 +195,12 @@ class GPTBlockFunction(torch.autograd.Function):
                 setattr(g, "d_" + name, (p.grad if acc else grads[name]).data_ptr())
         scratch = _gemm.colsum_scratch(dev)
         g.colsum_scratch, g.colsum_scratch_bytes = scratch.data_ptr(), scratch.numel() * 4
-        nblk = min(T, 296)
-        work = {
-            "d_ff": torch.empty(T, dff, dtype=dt, device=dev), "d_ln2": torch.empty(T, d, dtype=dt, device=dev),
-            "d_h1": torch.empty(T, d, dtype=dt, device=dev), "d_ctx": torch.empty(T, hd, dtype=dt, device=dev),
-            "d_probs": None if saved["probs"] is None else torch.empty_like(saved["probs"]),
-            "d_qkv": torch.empty(T, 3 * hd, dtype=dt, device=dev),
-            "norm_partial": torch.empty(2, nblk, d, dtype=torch.float32, device=dev),
-            "dq_acc": torch.empty(T * hd, dtype=torch.float32, device=dev) if saved["probs"] is None else None,
-            "delta": torch.empty(b * n_heads * s, dtype=torch.float32, device=dev) if saved["probs"] is None else None,
-        }
-        for name, t in work.items():
-            setattr(g, name, None if t is None else t.data_ptr())
+        nblk = min(b * s, 296)
+        plan, total = _work_plan(b, s, d, n_heads, d_head, params[8].shape[0], fused_attn, nblk)
+        work = torch.empty(total, dtype=torch.uint8, device=dev)
+        base = work.data_ptr()
+        for name, at in plan.items():
+            setattr(g, name, base + at)
         g.nblk = nblk
         _native.check(lib.bmt_gpt_block_backward(ctypes.byref(blk), ctypes.byref(g), _native.stream_handle()), "GPT block backward")
         ctx.saved = None
