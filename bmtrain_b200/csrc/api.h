@@ -278,7 +278,8 @@ int bmt_flash_attn_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int
                        const int64_t* o_strides, const void* dout, const int64_t* do_strides, const void* lse, void* dq,
                        const int64_t* dq_strides, void* dk, const int64_t* dk_strides, void* dv, const int64_t* dv_strides,
                        void* dq_acc, void* delta, float scale, int causal, const void* mask_bits_t, const void* mask_cls,
-                       const void* kv_lens, int dtype, void* stream);
+                       const void* kv_lens, void* dkv_part, int dtype, void* stream);
+int64_t bmt_flash_attn_bwd_parts(int64_t batch, int64_t sk, int h, int hk, int d);   // floats of dkv_part (0: NULL will do)
 // A dense mask (batch, sq, sk) of bytes (non-zero = attend) as bits: by query (bits, at offset 0), by key (bits_t) and a
 // class per 128 x 128 tile (cls).  The layout call returns the bytes needed and the offsets of the last two parts.
 int64_t bmt_attn_mask_layout(int64_t batch, int64_t sq, int64_t sk, int64_t* bits_t_off, int64_t* cls_off);

@@ -568,6 +568,9 @@ struct AttnBwdParams {
     int64_t dk_tok, dk_head, dk_batch, dv_tok, dv_head, dv_batch;
     uint32_t idesc_s, idesc_dv, idesc_dq;
     int q_tiles, k_tiles;
+    int splits;                 // CTAs that share the query heads of one kv head; above 1 they leave fp32 parts in dkv_part
+    float* dkv_part;            // (splits, 2: dK / dV, b, sk, hk, d)
+    int64_t part_elems;         // b * sk * hk * d
 };
 
 constexpr int BWD_THREADS = 512;                 // 8 softmax warps, 4 dQ warps, producer and MMA issuer (a warpgroup of their own)
@@ -619,7 +622,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int kvh = blockIdx.x % p.hk, b = blockIdx.x / p.hk, kt = blockIdx.y;   // under a causal mask the long columns start first
-    const int group = p.h / p.hk;
+    const int group = p.h / p.hk / p.splits;     // query heads of this CTA
     const int64_t kv0 = (int64_t)kt * TILE;
     int64_t kv_valid = p.sk;
     if (p.kv_lens && p.kv_lens[b] < kv_valid) kv_valid = p.kv_lens[b];
@@ -627,7 +630,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     walk.qt_first = 0;
     if (p.causal && kv0 - p.causal_off > 0) walk.qt_first = (int)((kv0 - p.causal_off) / TILE);
     walk.qt = walk.qt_first; walk.q_tiles = p.q_tiles; walk.k_tiles = p.k_tiles;
-    walk.head = kvh * group; walk.head_end = kv0 < kv_valid ? walk.head + group : walk.head;
+    walk.head = (kvh * p.splits + (int)blockIdx.z) * group; walk.head_end = kv0 < kv_valid ? walk.head + group : walk.head;
     walk.cls = p.cls ? p.cls + (int64_t)b * p.q_tiles * p.k_tiles + kt : nullptr;
     walk.settle();
     const bool work = walk.more();
@@ -887,7 +890,13 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
 #pragma unroll
                         for (int i = 0; i < 16; ++i) r[i] = 0u;
                     }
-                    if (kj < p.sk) {
+                    if (kj < p.sk && p.splits > 1) {
+                        float* part_dst = p.dkv_part + ((int64_t)blockIdx.z * 2 + part) * p.part_elems + (((int64_t)b * p.sk + kj) * p.hk + kvh) * p.d + c16 * 16;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            reinterpret_cast<float4*>(part_dst)[q] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
+                                                                                 __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+                    } else if (kj < p.sk) {
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {
                             bmt::Vec16<T> ov;
@@ -992,6 +1001,43 @@ __global__ void attn_dq_convert_kernel(const float* acc, T* dq, int64_t q_tok, i
     bmt::st16(dq + bb * q_batch + qi * q_tok + head * q_head + c, o);
 }
 
+// dk / dv (strided, T) <- sum of the parts in split order; one 8-element vector per thread, dK in the first half of the grid
+template <typename T>
+__global__ void attn_dkv_sum_kernel(const float* part, int splits, int64_t elems, int64_t sk, int hk, int d, T* dk, int64_t k_tok, int64_t k_head,
+                                    int64_t k_batch, T* dv, int64_t v_tok, int64_t v_head, int64_t v_batch) {
+    const int64_t vecs = elems / 8;
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 2 * vecs) return;
+    const int which = i >= vecs ? 1 : 0;
+    i -= which * vecs;
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int sp = 0; sp < splits; ++sp) {
+        const float4* src = reinterpret_cast<const float4*>(part + ((int64_t)sp * 2 + which) * elems + i * 8);
+        const float4 a = src[0], c = src[1];
+        acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w; acc[4] += c.x; acc[5] += c.y; acc[6] += c.z; acc[7] += c.w;
+    }
+    const int per = d / 8;
+    const int64_t row = i / per, tok = row / hk;
+    const int col = (int)(i - row * per) * 8, head = (int)(row - tok * hk);
+    const int64_t bb = tok / sk, kj = tok - bb * sk;
+    bmt::Vec16<T> o;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o.v[e] = bmt::Cvt<T>::from_f(acc[e]);
+    T* dst = which ? dv + bb * v_batch + kj * v_tok + head * v_head : dk + bb * k_batch + kj * k_tok + head * k_head;
+    bmt::st16(dst + col, o);
+}
+
+// CTAs that share the query heads of a kv head.  Without a split there is a CTA per key tile, kv head and sample, which walks
+// over all query heads of the group: one kv head leaves most SMs idle, and under a causal mask the CTA of the first keys sets
+// the pace (1x2048, 64 / 8 heads x 128: 128 CTAs, 408 us).  The heads are shared out until there are two CTAs per SM.
+int bwd_splits(int64_t batch, int64_t sk, int h, int hk) {
+    const int group = h / hk;
+    const int64_t ctas = (sk + TILE - 1) / TILE * hk * batch;
+    for (int s = 1; s < group; ++s)
+        if (group % s == 0 && ctas * s >= 2 * 148) return s;
+    return group;
+}
+
 template <int HD, typename T>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdParams& p,
                int64_t batch, cudaStream_t stream) {
@@ -1002,7 +1048,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
         if (cudaFuncSetAttribute(flash_bwd_kernel<HD, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -30;
         configured = true;
     }
-    dim3 grid((unsigned)(p.hk * batch), (unsigned)p.k_tiles);
+    dim3 grid((unsigned)(p.hk * batch), (unsigned)p.k_tiles, (unsigned)p.splits);
     flash_bwd_kernel<HD, T><<<grid, BWD_THREADS, smem, stream>>>(tq, tk, tv, tdo, tdq, p);
     bmt_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -31;
@@ -1012,7 +1058,7 @@ template <typename T>
 int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const void* q, const int64_t* qs, const void* k, const int64_t* ks,
             const void* v, const int64_t* vs, const void* o, const int64_t* os, const void* dout, const int64_t* gs, const void* lse,
             void* dq, const int64_t* dqs, void* dk, const int64_t* dks, void* dv, const int64_t* dvs, void* dq_acc, void* delta, float scale,
-            int causal, const void* mask_bits_t, const void* mask_cls, const void* kv_lens, int dtype, cudaStream_t st) {
+            int causal, const void* mask_bits_t, const void* mask_cls, const void* kv_lens, void* dkv_part, int dtype, cudaStream_t st) {
     const int hd = d <= 64 ? 64 : 128;
     CUtensorMap tq, tk, tv, tdo, tdq;
     int rc;
@@ -1032,6 +1078,7 @@ int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const v
     p.causal = causal; p.causal_off = sk - sq;
     p.bits_t = (const uint32_t*)mask_bits_t; p.cls = (const uint8_t*)mask_cls; p.kv_lens = (const int32_t*)kv_lens;
     p.q_tiles = (int)((sq + TILE - 1) / TILE); p.k_tiles = (int)((sk + TILE - 1) / TILE);
+    p.splits = dkv_part ? bwd_splits(batch, sk, h, hk) : 1; p.dkv_part = (float*)dkv_part; p.part_elems = batch * sk * hk * d;
     p.lse = (const float*)lse; p.delta = (const float*)delta; p.dq_acc = (float*)dq_acc;
     p.dk = dk; p.dk_tok = dks[0]; p.dk_head = dks[1]; p.dk_batch = dks[2];
     p.dv = dv; p.dv_tok = dvs[0]; p.dv_head = dvs[1]; p.dv_batch = dvs[2];
@@ -1042,6 +1089,12 @@ int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const v
     p.idesc_dq = common | (1u << 15) | (1u << 16) | ((uint32_t)(d >> 3) << 17);  // A and B MN-major
     rc = hd == 64 ? launch_bwd<64, T>(tq, tk, tv, tdo, tdq, p, batch, st) : launch_bwd<128, T>(tq, tk, tv, tdo, tdq, p, batch, st);
     if (rc != 0) return rc;
+    if (p.splits > 1) {
+        const int64_t vecs = p.part_elems / 4;   // 8-element vectors of dK and dV
+        attn_dkv_sum_kernel<T><<<(unsigned)((vecs + 255) / 256), 256, 0, st>>>(p.dkv_part, p.splits, p.part_elems, sk, hk, d, (T*)dk, dks[0], dks[1],
+                                                                              dks[2], (T*)dv, dvs[0], dvs[1], dvs[2]);
+        bmt_count_launch(1);
+    }
     attn_dq_convert_kernel<T><<<row_blocks, 256, 0, st>>>((const float*)dq_acc, (T*)dq, dqs[0], dqs[1], dqs[2], rows, sq, h, d);
     bmt_count_launch(2);
     return cudaGetLastError() == cudaSuccess ? 0 : -33;
@@ -1115,26 +1168,33 @@ extern "C" int bmt_attn_status(void) {
     return v;
 }
 
+// Floats of dkv_part that the backward takes for this problem; 0: none needed.
+extern "C" int64_t bmt_flash_attn_bwd_parts(int64_t batch, int64_t sk, int h, int hk, int d) {
+    const int splits = bwd_splits(batch, sk, h, hk);
+    return splits > 1 ? (int64_t)splits * 2 * batch * sk * hk * d : 0;
+}
+
 // Backward of bmt_flash_attn_fwd.  o / lse are the forward's results, dout the gradient of o; dq, dk, dv receive the
-// gradients (strided like their operands).  dq_acc: scratch of batch * sq * h * d floats, delta: batch * h * sq floats.
+// gradients (strided like their operands).  dq_acc: scratch of batch * sq * h * d floats, delta: batch * h * sq floats,
+// dkv_part: bmt_flash_attn_bwd_parts floats, or NULL (the query heads of a kv head then share one CTA).
 // All tensors follow the forward's stride and alignment rules.
 extern "C" int bmt_flash_attn_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const void* q, const int64_t* q_strides,
                                   const void* k, const int64_t* k_strides, const void* v, const int64_t* v_strides, const void* o,
                                   const int64_t* o_strides, const void* dout, const int64_t* do_strides, const void* lse, void* dq,
                                   const int64_t* dq_strides, void* dk, const int64_t* dk_strides, void* dv, const int64_t* dv_strides,
                                   void* dq_acc, void* delta, float scale, int causal, const void* mask_bits_t,
-                                  const void* mask_cls, const void* kv_lens, int dtype, void* stream) {
+                                  const void* mask_cls, const void* kv_lens, void* dkv_part, int dtype, void* stream) {
     if (d <= 0 || d > 128 || (d & 15) || h % hk || batch <= 0 || sq <= 0 || sk <= 0) return -1;
     const int64_t* all[] = {o_strides, dq_strides, dk_strides, dv_strides};
     for (const int64_t* s3 : all)
         if ((s3[0] & 7) || (s3[1] & 7) || (s3[2] & 7)) return -2;
-    if (((uintptr_t)o | (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv | (uintptr_t)dq_acc) & 15) return -2;
+    if (((uintptr_t)o | (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv | (uintptr_t)dq_acc | (uintptr_t)dkv_part) & 15) return -2;
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == BMT_DT_F16)
         return run_bwd<__half>(batch, sq, sk, h, hk, d, q, q_strides, k, k_strides, v, v_strides, o, o_strides, dout, do_strides, lse, dq,
-                               dq_strides, dk, dk_strides, dv, dv_strides, dq_acc, delta, scale, causal, mask_bits_t, mask_cls, kv_lens, dtype, st);
+                               dq_strides, dk, dk_strides, dv, dv_strides, dq_acc, delta, scale, causal, mask_bits_t, mask_cls, kv_lens, dkv_part, dtype, st);
     if (dtype == BMT_DT_BF16)
         return run_bwd<__nv_bfloat16>(batch, sq, sk, h, hk, d, q, q_strides, k, k_strides, v, v_strides, o, o_strides, dout, do_strides, lse,
-                                      dq, dq_strides, dk, dk_strides, dv, dv_strides, dq_acc, delta, scale, causal, mask_bits_t, mask_cls, kv_lens, dtype, st);
+                                      dq, dq_strides, dk, dk_strides, dv, dv_strides, dq_acc, delta, scale, causal, mask_bits_t, mask_cls, kv_lens, dkv_part, dtype, st);
     return -3;
 }

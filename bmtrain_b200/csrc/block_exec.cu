@@ -174,7 +174,7 @@ extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockG
         RUN(bmt_flash_attn_bwd(q.b, q.s, q.s, (int)q.h, (int)q.h, (int)q.dh, k.qkv, in_str, off(k.qkv, q.dh), in_str,
                                off(k.qkv, 2 * q.dh), in_str, k.ctx, out_str, w.d_ctx, out_str, k.lse, w.d_qkv, in_str,
                                off(w.d_qkv, q.dh), in_str, off(w.d_qkv, 2 * q.dh), in_str, w.dq_acc, w.delta,
-                               1.f / sqrtf((float)q.dh), k.causal, mask_part(k, q, 1), mask_part(k, q, 2), nullptr, dt, stream));
+                               1.f / sqrtf((float)q.dh), k.causal, mask_part(k, q, 1), mask_part(k, q, 2), nullptr, nullptr, dt, stream));
     } else {
     {   // dP = d_ctx v^T
         BmtGemmDesc g = plain(q.s, q.s, q.dh, w.d_ctx, q.hd, 0, off(k.qkv, 2 * q.dh), tok, 0, w.d_probs, pl, dt);

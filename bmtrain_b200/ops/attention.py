@@ -128,12 +128,17 @@ def flash_backward(q, k, v, o, lse, do, scale, causal, mask8, lens32, packed=Non
     dv = torch.empty(b, sk, hk, d, dtype=q.dtype, device=q.device)
     dq_acc = torch.empty(b * sq * h * d, dtype=torch.float32, device=q.device)
     delta = torch.empty(b * h * sq, dtype=torch.float32, device=q.device)
+    parts = None
+    if hk != h:
+        lib.bmt_flash_attn_bwd_parts.restype = ctypes.c_int64
+        n = lib.bmt_flash_attn_bwd_parts(ctypes.c_int64(b), ctypes.c_int64(sk), ctypes.c_int(h), ctypes.c_int(hk), ctypes.c_int(d))
+        parts = torch.empty(n, dtype=torch.float32, device=q.device) if n else None
     _native.check(lib.bmt_flash_attn_bwd(
         ctypes.c_int64(b), ctypes.c_int64(sq), ctypes.c_int64(sk), ctypes.c_int(h), ctypes.c_int(hk), ctypes.c_int(d),
         _native.ptr(q), _strides3(q), _native.ptr(k), _strides3(k), _native.ptr(v), _strides3(v), _native.ptr(o), _strides3(o),
         _native.ptr(do), _strides3(do), _native.ptr(lse), _native.ptr(dq), _strides3(dq), _native.ptr(dk), _strides3(dk),
         _native.ptr(dv), _strides3(dv), _native.ptr(dq_acc), _native.ptr(delta), ctypes.c_float(scale),
-        ctypes.c_int(1 if causal else 0), bits_t, classes, _native.ptr(lens32), ctypes.c_int(_DT[q.dtype]),
+        ctypes.c_int(1 if causal else 0), bits_t, classes, _native.ptr(lens32), _native.ptr(parts), ctypes.c_int(_DT[q.dtype]),
         _native.stream_handle()), "fused attention backward")
     return dq, dk, dv
 
