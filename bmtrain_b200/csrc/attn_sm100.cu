@@ -11,6 +11,8 @@
 #include <math.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "api.h"
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -96,14 +98,6 @@ __device__ __forceinline__ void fail(AttnShared* sh, int code) {
 template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
-// one lane polls, the warp follows
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int lane) {
-    int got = 1;
-    if (lane == 0) got = mbar_wait(bar, parity) ? 1 : 0;
-    got = __shfl_sync(0xffffffffu, got, 0);
-    __syncwarp();
-    return got != 0;
-}
 
 // The lowest `n` of 32 bits (n may be outside [0, 32]).
 __device__ __forceinline__ uint32_t low_bits(int64_t n) { return n >= 32 ? 0xffffffffu : n <= 0 ? 0u : ((1u << (int)n) - 1u); }
@@ -187,6 +181,9 @@ attn_mask_pack_kernel(const uint8_t* mask, int64_t sq, int64_t sk, uint32_t* bit
 //               masks, and writes the probabilities back over it as packed 16-bit pairs, where the MMA takes them from.
 // What bounds it: a 128 x 128 tile at head dim 128 is 1024 clocks of MMA and 1024 clocks of ex2 (16 per clock and SM); with
 // one tile per CTA, and P going through shared memory, the two and everything in between took turns (about 4500 clocks).
+// Now a group's tile takes about 3500 clocks (two groups: 1750 a tile): 550 for reading the row and its maximum, 1600 for the
+// exponentials of both groups (2048 clocks of ex2 between them), 1200 from handing over P to the next scores, of which the MMAs are 770:
+// P lies over the scores, and with two accumulators there is no tensor memory for a second set at head dim 128.
 // The commit behind S_t(j) also covers P V of the tile before (the tensor pipe works in issue order), so a softmax group that
 // has seen S_t(j) may rescale O_t without another wait.
 template <int HD, typename T>
@@ -290,60 +287,60 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             for (int t = 0; t < 2; ++t)
                 while (last[t] >= 0 && !active(t, last[t])) --last[t];
             auto issue_s = [&](int t, int st) {          // S_t = Q_t K^T
-                if (elect_one()) {
-                    for (int ks = 0; ks < ks_s; ++ks) {
-                        const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32);
-                        umma_f16(tmem + t * TILE, pack_desc(desc_lo(sQ + t * TB + off, 0), hi), pack_desc(desc_lo(sK + st * TB + off, 0), hi),
-                                 p.idesc_s, ks != 0 ? 1u : 0u);
-                    }
-                    umma_commit(&sh->s_full[t]);
+                // unrolled: a loop of unknown length took 70 clocks an instruction, more than its 64 of multiplying
+                const uint32_t qd = desc_lo(sQ + t * TB, 0), kd = desc_lo(sK + st * TB, 0);
+#pragma unroll
+                for (int ks = 0; ks < HD / 16; ++ks) {
+                    const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32) >> 4;
+                    if (ks < ks_s) umma_f16(tmem + t * TILE, pack_desc(qd + off, hi), pack_desc(kd + off, hi), p.idesc_s, ks != 0 ? 1u : 0u);
                 }
-                __syncwarp();
+                umma_commit(&sh->s_full[t]);
             };
             int j = first, n = 0;
             if (ok && !mbar_wait_warp(smem_u32(&sh->k_full[0]), 0)) { if (lane == 0) fail(sh, 4); ok = false; }
             if (ok) {
                 tc_fence_after();
-                if (active(0, j)) issue_s(0, 0);
-                if (active(1, j)) issue_s(1, 0);
-                if (elect_one()) umma_commit(&sh->k_empty[0]);
+                if (elect_one()) {
+                    if (active(0, j)) issue_s(0, 0);
+                    if (active(1, j)) issue_s(1, 0);
+                    umma_commit(&sh->k_empty[0]);
+                }
                 __syncwarp();
             }
             while (ok && j < J_max) {
                 const int jn = next_step(j), st = n & 1, sn = (n + 1) & 1;
                 const uint32_t ph = (uint32_t)((n >> 1) & 1), phn = (uint32_t)(((n + 1) >> 1) & 1);
                 if (!mbar_wait_warp(smem_u32(&sh->v_full[st]), ph)) { if (lane == 0) fail(sh, 5); ok = false; break; }
-                bool k_seen = false;
+                if (jn < J_max && !mbar_wait_warp(smem_u32(&sh->k_full[sn]), phn)) { if (lane == 0) fail(sh, 7); ok = false; break; }
+                const uint32_t vd = desc_lo(sV + st * TB, CHUNK);
+                // P V: B = V (128 keys x head dim, head dim contiguous = MN-major), 16 key rows per step, 64-column chunks CHUNK apart
+                auto issue_pv = [&](int t, int half) {
+#pragma unroll
+                    for (int ks = half * 4; ks < half * 4 + 4; ++ks)
+                        umma_f16_ts(tmem + 256 + t * TILE, tmem + t * TILE + ks * 8, pack_desc(vd + ks * 128, hi), p.idesc_pv, (done[t] | ks) != 0 ? 1u : 0u);
+                };
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
-                    if (active(t, j)) {
+                    const bool now = active(t, j), next = jn < J_max && active(t, jn);
+                    if (now) {
                         // the first 64 keys of P_t are in tensor memory and, if row maxima moved, O_t has been rescaled by its
                         // owners; the second half of the softmax runs under the first half of the MMAs
-#pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            if (!mbar_wait_warp(smem_u32(half ? &sh->p_ready[t] : &sh->p_half[t]), done[t] & 1u)) { if (lane == 0) fail(sh, 6); ok = false; break; }
-                            tc_fence_after();
-                            if (elect_one()) {
-#pragma unroll
-                                for (int ks = half * 4; ks < half * 4 + 4; ++ks)
-                                    // B = V (128 keys x head dim, head dim contiguous = MN-major): 16 key rows per step, 64-column chunks CHUNK apart
-                                    umma_f16_ts(tmem + 256 + t * TILE, tmem + t * TILE + ks * 8, pack_desc(desc_lo(sV + st * TB + ks * 2048, CHUNK), hi),
-                                                p.idesc_pv, (done[t] | ks) != 0 ? 1u : 0u);
-                                if (half == 1 && j == last[t]) umma_commit(&sh->o_full[t]);
-                            }
-                            __syncwarp();
-                        }
-                        if (!ok) break;
-                        ++done[t];
+                        if (!mbar_wait_warp(smem_u32(&sh->p_half[t]), done[t] & 1u)) { if (lane == 0) fail(sh, 6); ok = false; break; }
+                        tc_fence_after();
+                        if (elect_one()) issue_pv(t, 0);
+                        __syncwarp();
+                        if (!mbar_wait_warp(smem_u32(&sh->p_ready[t]), done[t] & 1u)) { if (lane == 0) fail(sh, 6); ok = false; break; }
                     }
-                    if (jn < J_max && active(t, jn)) {
-                        if (!k_seen) {
-                            if (!mbar_wait_warp(smem_u32(&sh->k_full[sn]), phn)) { if (lane == 0) fail(sh, 7); ok = false; break; }
-                            tc_fence_after();
-                            k_seen = true;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        if (now) {
+                            issue_pv(t, 1);
+                            if (j == last[t]) umma_commit(&sh->o_full[t]);
                         }
-                        issue_s(t, sn);
+                        if (next) issue_s(t, sn);
                     }
+                    __syncwarp();
+                    if (now) ++done[t];
                 }
                 if (!ok) break;
                 if (elect_one()) {
@@ -386,37 +383,42 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 vis[0] = w.x & low_bits(limit - kv0); vis[1] = w.y & low_bits(limit - kv0 - 32);
                 vis[2] = w.z & low_bits(limit - kv0 - 64); vis[3] = w.w & low_bits(limit - kv0 - 96);
             }
-            if (!warp_wait(&sh->s_full[t], n & 1u, lane)) { if (lane == 0) fail(sh, 9); ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&sh->s_full[t]), n & 1u)) { if (lane == 0) fail(sh, 9); ok = false; break; }
             tc_fence_after();
             uint32_t r[TILE / 32][32];
-#pragma unroll
-            for (int c4 = 0; c4 < TILE / 32; ++c4) tmem_ld32(s_addr + c4 * 32, r[c4]);
-            tmem_ld_wait();
+            tmem_ld32(s_addr, r[0]);
+            tmem_ld32(s_addr + 32, r[1]);
+            tmem_ld_wait_for(r[0]);
+            tmem_ld_wait_for(r[1]);
+            tmem_ld32(s_addr + 64, r[2]);        // on its way while the maximum of the first half is taken
+            tmem_ld32(s_addr + 96, r[3]);
             // tiles away from the diagonal and the ragged edge (the common case) skip the per-element visibility tests
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
             if (need_mask) {
 #pragma unroll
-                for (int c4 = 0; c4 < TILE / 32; ++c4)
+                for (int c4 = 0; c4 < TILE / 32; ++c4) {
+                    if (c4 == 2) { tmem_ld_wait_for(r[2]); tmem_ld_wait_for(r[3]); }
 #pragma unroll
                     for (int i = 0; i < 32; ++i)
                         if ((vis[c4] >> i) & 1u) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(r[c4][i]));
+                }
             } else {
 #pragma unroll
-                for (int c4 = 0; c4 < TILE / 32; ++c4)
+                for (int c4 = 0; c4 < TILE / 32; ++c4) {
+                    if (c4 == 2) { tmem_ld_wait_for(r[2]); tmem_ld_wait_for(r[3]); }
 #pragma unroll
                     for (int i = 0; i < 32; i += 2)
                         mx[(i >> 1) & 3] = fmaxf(fmaxf(mx[(i >> 1) & 3], __uint_as_float(r[c4][i])), __uint_as_float(r[c4][i + 1]));
+                }
             }
             const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
             // move the reference maximum?  (first visible score of the row, or growth beyond the threshold)
-            float alpha = 1.f;
-            bool move = false;
-            if (mt != -INFINITY) {
-                if (m_ref == -INFINITY) { m_ref = mt; }               // nothing accumulated yet: O and l are zero
-                else if ((mt - m_ref) * p.sl2 > 8.f) { alpha = ex2((m_ref - mt) * p.sl2); m_ref = mt; move = true; }
-            }
-            if (n > 0 && __any_sync(0xffffffffu, move)) {
+            const bool fresh = m_ref == -INFINITY;                        // nothing accumulated yet: O and l are zero
+            const bool move = !fresh && mt != -INFINITY && (mt - m_ref) * p.sl2 > 8.f;
+            if (__any_sync(0xffffffffu, move)) {
                 // rescale this warp's 32 rows of the accumulator (lanes whose maximum did not move multiply by one)
+                const float alpha = move ? ex2((m_ref - mt) * p.sl2) : 1.f;
+                l_run *= alpha;
 #pragma unroll
                 for (int c8 = 0; c8 < HD / 8; ++c8) {
                     if (c8 * 8 < p.d) {
@@ -429,39 +431,44 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                     }
                 }
             }
+            if (fresh || move) m_ref = mt;
             const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref * p.sl2;
             const uint64_t sl2_2 = pack_f2(p.sl2, p.sl2), neg_2 = pack_f2(neg_m, neg_m);
             uint64_t sum2[2] = {0ull, 0ull};
+            // compiled with and without masks: tests that are predicated off still take an issue slot each
+            auto exps = [&](auto masked) {
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t pk[32];
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t pk[32];
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int e = half * 64 + 2 * i, c4 = e >> 5, k = e & 31;
-                    float x, y;
-                    unpack_f2(fma_f2(pack_f2(__uint_as_float(r[c4][k]), __uint_as_float(r[c4][k + 1])), sl2_2, neg_2), x, y);
-                    x = ex2(x);
-                    y = ex2(y);
-                    if (need_mask) {
-                        if (!((vis[c4] >> k) & 1u)) x = 0.f;
-                        if (!((vis[c4] >> (k + 1)) & 1u)) y = 0.f;
+                    for (int i = 0; i < 32; ++i) {
+                        const int e = half * 64 + 2 * i, c4 = e >> 5, k = e & 31;
+                        float x, y;
+                        unpack_f2(fma_f2(pack_f2(__uint_as_float(r[c4][k]), __uint_as_float(r[c4][k + 1])), sl2_2, neg_2), x, y);
+                        x = ex2(x);
+                        y = ex2(y);
+                        if constexpr (decltype(masked)::value) {
+                            if (!((vis[c4] >> k) & 1u)) x = 0.f;
+                            if (!((vis[c4] >> (k + 1)) & 1u)) y = 0.f;
+                        }
+                        sum2[i & 1] = add_f2(sum2[i & 1], pack_f2(x, y));
+                        pk[i] = pack2<T>(x, y);
                     }
-                    sum2[i & 1] = add_f2(sum2[i & 1], pack_f2(x, y));
-                    pk[i] = pack2<T>(x, y);
+                    tmem_st32(s_addr + half * 32, pk);     // over the scores: this thread's row, already in registers
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(half ? &sh->p_ready[t] : &sh->p_half[t]);
                 }
-                tmem_st32(s_addr + half * 32, pk);     // over the scores: this thread's row, already in registers
-                tmem_st_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(half ? &sh->p_ready[t] : &sh->p_half[t]);
-            }
+            };
+            if (need_mask) exps(std::true_type{}); else exps(std::false_type{});
             float s0, s1;
             unpack_f2(add_f2(sum2[0], sum2[1]), s0, s1);
-            l_run = l_run * alpha + (s0 + s1);
+            l_run += s0 + s1;
             ++n;
         }
         if (ok && n > 0) {
-            if (!warp_wait(&sh->o_full[t], 0u, lane)) { if (lane == 0) fail(sh, 12); ok = false; }
+            if (!mbar_wait_warp(smem_u32(&sh->o_full[t]), 0u)) { if (lane == 0) fail(sh, 12); ok = false; }
         }
         if (ok && t < p.per_cta && qt0 + t < p.q_tiles) {
             // normalise and store the row (the tensor-memory loads are warp-wide; only the stores depend on the row)
@@ -696,9 +703,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 if (!mbar_wait_warp(smem_u32(&sh->q_full[st]), (it >> 1) & 1)) { if (lane == 0) fail_bwd(sh, 4); return false; }
                 tc_fence_after();
                 if (elect_one()) {
-                    for (int ks = 0; ks < ks_d; ++ks) {
-                        const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32);
-                        umma_f16(tmem, pack_desc(desc_lo(sK + off, 0), hi), pack_desc(desc_lo(sQ + st * TB + off, 0), hi), p.idesc_s, ks != 0 ? 1u : 0u);
+                    const uint32_t kd = desc_lo(sK, 0), qd = desc_lo(sQ + st * TB, 0);
+#pragma unroll
+                    for (int ks = 0; ks < HD / 16; ++ks) {       // unrolled, see the forward kernel
+                        const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32) >> 4;
+                        if (ks < ks_d) umma_f16(tmem, pack_desc(kd + off, hi), pack_desc(qd + off, hi), p.idesc_s, ks != 0 ? 1u : 0u);
                     }
                     umma_commit(&sh->s_full);
                 }
@@ -714,9 +723,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                 if (dq_shared && !mbar_wait_warp(smem_u32(&sh->dq_empty), ph ^ 1)) { if (lane == 0) fail_bwd(sh, 6); break; }
                 tc_fence_after();
                 if (elect_one()) {
-                    for (int ks = 0; ks < ks_d; ++ks) {
-                        const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32);
-                        umma_f16(tmem + C_DP, pack_desc(desc_lo(sV + off, 0), hi), pack_desc(desc_lo(sdO + off, 0), hi), p.idesc_s, ks != 0 ? 1u : 0u);
+                    const uint32_t vd = desc_lo(sV, 0), od = desc_lo(sdO, 0);
+#pragma unroll
+                    for (int ks = 0; ks < HD / 16; ++ks) {
+                        const uint32_t off = (uint32_t)((ks >> 2) * CHUNK + (ks & 3) * 32) >> 4;
+                        if (ks < ks_d) umma_f16(tmem + C_DP, pack_desc(vd + off, hi), pack_desc(od + off, hi), p.idesc_s, ks != 0 ? 1u : 0u);
                     }
                     umma_commit(&sh->dp_full);
                 }
@@ -790,7 +801,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             const uint32_t ph = it & 1, st = it & 1;
             const int64_t q0 = (int64_t)walk.qt * TILE;
             const int kind = walk.cls ? walk.cls[(int64_t)walk.qt * p.k_tiles] : 2;
-            if (!warp_wait(&sh->row_full[st], (it >> 1) & 1, lane)) { if (lane == 0) fail_bwd(sh, 10); ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&sh->row_full[st]), (it >> 1) & 1)) { if (lane == 0) fail_bwd(sh, 10); ok = false; break; }
             uint32_t vis[2];
             vis[0] = sh->live[st][part * 2]; vis[1] = sh->live[st][part * 2 + 1];
             bool need_mask = kind == 1 || kv0 + TILE > kv_valid || (p.causal && kv0 + TILE - 1 > q0 + p.causal_off) ||
@@ -808,7 +819,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
                     vis[1] &= part ? w.w : w.y;
                 }
             }
-            if (!warp_wait(&sh->s_full, ph, lane)) { if (lane == 0) fail_bwd(sh, 11); ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&sh->s_full), ph)) { if (lane == 0) fail_bwd(sh, 11); ok = false; break; }
             tc_fence_after();
             uint32_t s[2][32];
             tmem_ld32(tmem + lane_addr + part * 64, s[0]);
@@ -838,11 +849,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh->p_ready);
-            if (!warp_wait(&sh->dp_full, ph, lane)) { if (lane == 0) fail_bwd(sh, 12); ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&sh->dp_full), ph)) { if (lane == 0) fail_bwd(sh, 12); ok = false; break; }
             tc_fence_after();
             tmem_ld32(tmem + lane_addr + C_DP + part * 64, s[0]);
             // dS(it-1) in shared memory may still be read by dQ / dK(it-1): wait for the commit behind both
-            if (it > 0 && !warp_wait(&sh->q_empty[st ^ 1], ((it - 1) >> 1) & 1, lane)) { if (lane == 0) fail_bwd(sh, 13); ok = false; break; }
+            if (it > 0 && !mbar_wait_warp(smem_u32(&sh->q_empty[st ^ 1]), ((it - 1) >> 1) & 1)) { if (lane == 0) fail_bwd(sh, 13); ok = false; break; }
             const uint32_t base = sdS + (uint32_t)part * CHUNK + (uint32_t)row * 128;
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -873,7 +884,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         }
         // dK, dV rows of this CTA's keys (zeros when no query sees them): part 0 writes dK, part 1 dV.  The tensor-memory
         // loads are warp-wide, so every lane takes part in them; only the stores depend on the row.
-        if (ok && it > 0 && !warp_wait(&sh->all_done, 0, lane)) { if (lane == 0) fail_bwd(sh, 14); ok = false; }
+        if (ok && it > 0 && !mbar_wait_warp(smem_u32(&sh->all_done), 0)) { if (lane == 0) fail_bwd(sh, 14); ok = false; }
         if (ok) {
             tc_fence_after();
             T* dst = part == 0 ? (T*)p.dk + (int64_t)b * p.dk_batch + kj * p.dk_tok + (int64_t)kvh * p.dk_head
@@ -916,7 +927,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         const uint32_t lane_addr = (uint32_t)r0 << 16, xbuf = sX + (uint32_t)(warp - 8) * DQ_BUF;
         bool ok = true;
         for (uint32_t it = 0; walk.more() && ok; walk.next(), ++it) {
-            if (!warp_wait(&sh->dq_full, it & 1, lane)) { if (lane == 0) fail_bwd(sh, 16); ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&sh->dq_full), it & 1)) { if (lane == 0) fail_bwd(sh, 16); ok = false; break; }
             tc_fence_after();
             uint32_t r[HD / 32][32];
 #pragma unroll

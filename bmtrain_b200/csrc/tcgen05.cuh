@@ -70,7 +70,9 @@ __device__ __forceinline__ bool elect_one() {
         : "=r"(pred));
     return pred != 0;
 }
-// Wait of a whole warp; the (bounded) result is the same in all lanes.
+// Wait of a whole warp; the (bounded) result is the same in all lanes.  All lanes poll (one request a warp): one lane polling
+// inside a branch, with a shuffle behind it, cost about 300 clocks more per wait -- attention forward, 2x4096, 20 x 128 causal,
+// 199 us against 170.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t addr, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_wait_u32(addr, parity)) != 0;
 }
