@@ -878,12 +878,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             const int bo = batch / (int)p.batch_inner, bi = batch - bo * (int)p.batch_inner;
             const uint32_t acc = tcount & 1;
             const uint32_t acc_ph = (tcount >> 1) & 1;
-            // one lane per warp polls the barrier (128 pollers would compete with the producer / MMA threads for the
-            // barrier unit during the whole main loop); the warp then re-converges
-            int got = 1;
-            if (lane == 0) got = mbar_wait(&hdr->tmem_full[acc], acc_ph) ? 1 : 0;
-            got = __shfl_sync(0xffffffffu, got, 0);
-            if (!got) { ok = false; if (lane == 0) atomicCAS(&g_gemm_status, 0, (4 << 16) | (blockIdx.x & 0xffff)); break; }
+            if (!mbar_wait_warp(smem_u32(&hdr->tmem_full[acc]), acc_ph)) { ok = false; if (lane == 0) atomicCAS(&g_gemm_status, 0, (4 << 16) | (blockIdx.x & 0xffff)); break; }
             tc_fence_after();
             const int64_t row0 = (int64_t)m_blk * (BM * NCTA) + rank * BM + quarter * 32;
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * p.bn;
