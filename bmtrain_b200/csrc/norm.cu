@@ -1,11 +1,10 @@
 // LayerNorm / RMSNorm forward and backward for sm_100a.
 //
-// Forward: one CTA per row; the row is staged once in shared memory as fp32, mean and
-// variance are exact two-pass statistics over that copy, the output is written with
-// 128-bit stores.  Saves (mean, rstd) per row.
-// Backward: a persistent grid (nblk CTAs) strides over the rows; each CTA produces dx for
-// its rows and keeps per-thread partial dgamma / dbeta in registers, written once to a
-// (nblk x d) fp32 scratch that a second kernel folds over nblk.
+// Forward: persistent grids whose warp teams hold a row in registers, take exact two-pass statistics over it and issue the
+// next row's loads ahead of the arithmetic.  Saves (mean, rstd) per row.
+// Backward: persistent grids (at most nblk CTAs) that get whole rows as bulk copies through a ring in shared memory, produce dx
+// and keep partial dgamma / dbeta in registers, written once to a (blocks x d) fp32 scratch that a second kernel folds.
+// Both also exist with one CTA per row, staged in shared memory (BMT_NORM_STAGED=1, and the combinations the others do not take).
 // (The reference calls F.layer_norm: example/layers/layernorm.py:29.)
 #include <stdlib.h>
 
@@ -380,9 +379,10 @@ int fwd(int64_t rows, int64_t d, const void* x, const void* w, const void* b, fl
 // scratch that norm_fold_kernel reduces.
 // HBM bytes bound it (x, dy and the residual's gradient in, dx out), so what counts is bytes in flight.  Loading a row into
 // registers and then working on it ran at 0.41 of the copy rate (16384 x 5120 RMS 193 us), one row ahead in registers at 0.48
-// (160 us): a load takes longer than a row's arithmetic; it is 124 us now (LayerNorm 194 -> 171, bound by its arithmetic).  So whole rows come as bulk copies into a ring of up to BWD_STAGES
+// (160 us): a load takes longer than a row's arithmetic.  So whole rows come as bulk copies into a ring of up to BWD_STAGES
 // stages in shared memory, refilled by one thread right behind the barrier that every row has anyway; the rows' statistics
-// are fetched for BWD_BATCH rows at a time.  RMSNorm (RMS) has no bias and drops the second accumulator.
+// are fetched for BWD_BATCH rows at a time: 124 us (LayerNorm 194 -> 171, bound by its arithmetic).  RMSNorm (RMS) has no bias
+// and drops the second accumulator.
 constexpr int BWD_STAGES = 8, BWD_BATCH = 32;
 __device__ int g_norm_status = 0;   // 1 after a bounded wait for a bulk copy ran out
 

@@ -3,9 +3,10 @@
 The reference example materialises the scores with two ``bmm`` calls and a
 ``(b, S, S)`` boolean mask (``example/layers/attention.py:78-104``).  Here the
 forward pass is one fused tcgen05 kernel (``csrc/attn_sm100.cu``): scores and
-probabilities stay in tensor memory / shared memory, only the output and one
-log-sum-exp per row reach HBM.  Causal flag, per-sample key lengths and a
-dense boolean mask are applied inside the kernel; grouped-query attention is
+probabilities stay in tensor memory, only the output and one log-sum-exp per
+row reach HBM.  Causal flag, per-sample key lengths and a dense boolean mask
+are applied inside the kernel; a dense mask is packed to bits first, by query,
+by key and with a class per 128 x 128 tile, once for both directions; grouped-query attention is
 supported (``kv heads`` divides ``heads``).  Head dims that the fused kernel
 does not take (not a multiple of 16, or above 128) use the two-GEMM form:
 batched tcgen05 GEMMs on the strided ``(b, s, heads, dim)`` views plus a fused

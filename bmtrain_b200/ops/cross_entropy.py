@@ -7,6 +7,8 @@ The reference materialises a full softmax (``csrc/cuda/cross_entropy.cu:9-121``,
 three passes per row); the interface functions with its names are kept in
 ``bmtrain_b200/loss/_function.py``.
 
+Mean and sum losses without class weights (``reduced_forward`` / ``reduced_backward``) add one block that turns the
+row statistics into the loss and the gradient's factor, so that a pass is three launches.
 The same two kernels serve the vocab-parallel loss: ``row_stats`` returns the
 local (max, sum-exp relative to that max, target logit) triple of a vocabulary
 shard, the caller combines them over the tensor-parallel group, and

@@ -1,6 +1,7 @@
 """Embedding gather / scatter-add kernels (the reference uses ``F.embedding``).
 
-Index ``-1`` means "not in this shard": forward writes zeros, backward skips the row.
+Index ``-1`` means "not in this shard": forward writes zeros, backward skips the row.  Backward orders the tokens by id
+and writes every row of the table's gradient once, added in fp32 and rounded once.
 """
 from __future__ import annotations
 

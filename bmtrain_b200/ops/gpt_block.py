@@ -1,9 +1,10 @@
 """Whole pre-LN GPT block as one autograd node on the native block executor (``csrc/block_exec.cu``).
 
-Forward issues 9 kernel launches and backward 21 from C++ in a single call each, all contractions on the tcgen05
-GEMM with fused epilogues (bias, ReLU, residual add, ReLU-mask on dgrad).  The big weight gradients are written
-straight into ``param.grad`` when a gradient buffer of the right dtype is already attached (as the ZeRO block
-does before backward), which removes the separate accumulate pass.
+Each direction is one C++ call that issues all of the block's launches; what a pass keeps for backward, and what backward
+scratches, is one allocation each, divided by a plan of the sizes.  All contractions run on the tcgen05 GEMM with fused
+epilogues (bias, ReLU, residual add, ReLU-mask on dgrad) or in the fused attention kernels.  The big weight gradients are
+written straight into the parameter's slot of the ZeRO block's gradient buffer, or into ``param.grad`` when a gradient of the
+right dtype is already attached, which removes the separate accumulate pass.
 """
 from __future__ import annotations
 

@@ -1,9 +1,10 @@
 """LayerNorm and RMSNorm, forward and backward (the reference calls ``F.layer_norm``:
 ``example/layers/layernorm.py:29``; RMSNorm is needed by the Llama-shaped models).
 
-One row per warp-group, single pass: the row is held in registers, statistics
-in fp32; backward produces dx and per-CTA partial dgamma/dbeta that a second
-tiny kernel folds.  CPU tensors use the PyTorch definition.
+A team of warps per row, statistics in fp32: forward holds the row in
+registers, backward gets rows through a ring of bulk copies in shared memory
+and produces dx and per-CTA partial dgamma/dbeta that a second tiny kernel
+folds.  CPU tensors use the PyTorch definition.
 """
 from __future__ import annotations
 
