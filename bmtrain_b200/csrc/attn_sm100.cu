@@ -552,7 +552,8 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
 //   MMA   dV += P^T dO (P from tensor memory), dK += dS^T Q, dQ = dS K
 //   one warp fetches lse and delta of the tiles to come
 //   dQ warps (4): add the tile of dQ to an fp32 accumulator in global memory (bulk reductions out of shared memory, 32 columns
-//         at a time; vector reductions by the threads themselves took 4300 clocks a tile); a small kernel converts it
+//         at a time through two buffers a warp: with one, waiting for it to be read made a tile 4065 clocks of their time; vector
+//         reductions by the threads themselves took 4300); a small kernel converts it
 // delta = rowsum(dO * O) comes from a pre-pass.  dK / dV are written once at the end, already summed over the group.
 // Order on the tensor pipe, which bounds a tile at 5 x 512 clocks (head dim 128): dP(i), dV(i), S(i+1), dK(i), dQ(i), dP(i+1):
 // while the softmax warps turn dP(i) into dS(i) the pipe has dV(i) and S(i+1) to do, and while it does dK(i) and dQ(i) they
@@ -580,6 +581,7 @@ struct AttnBwdParams {
     int64_t part_elems;         // b * sk * hk * d
 };
 
+constexpr uint32_t DQ_BUF = 32 * 128;            // exchange buffer of a dQ warp: 32 rows x 32 floats; each warp has two
 constexpr int BWD_THREADS = 512;                 // 8 softmax warps, 4 dQ warps, producer and MMA issuer (a warpgroup of their own)
 
 struct BwdShared {
@@ -617,12 +619,16 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                  const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdq, const AttnBwdParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    // swizzled tiles want 1024-byte alignment; there is no static shared memory in front of the block's own and no room to round up
+    uint8_t* smem = smem_raw;
+    if (smem_u32(smem_raw) & 1023u) {
+        if (threadIdx.x == 0) atomicCAS(&g_attn_status, 0, (0x7f << 16) | (int)(blockIdx.x & 0xffff));
+        return;
+    }
     constexpr int DC = HD / 64;
     constexpr uint32_t TB = DC * CHUNK;
-    constexpr uint32_t DQ_BUF = 32 * 128;           // exchange buffer of one dQ warp: 32 rows x 32 floats
     const uint32_t sK = smem_u32(smem), sV = sK + TB, sQ = sV + TB, sdO = sQ + 2 * TB, sdS = sdO + TB, sX = sdS + 2 * CHUNK;
-    BwdShared* sh = (BwdShared*)(smem + 5 * TB + 2 * CHUNK + 4 * DQ_BUF);
+    BwdShared* sh = (BwdShared*)(smem + 5 * TB + 2 * CHUNK + 8 * DQ_BUF);
     // tensor memory columns: S^T / P^T [0,128), dP^T [128,256), dV, dK, dQ each of d columns; above head dim 80 dQ takes dP's
     const uint32_t C_DP = 128, C_DV = 256, C_DK = C_DV + p.d, C_DQ = p.d <= 80 ? C_DK + p.d : C_DP;
     const bool dq_shared = p.d > 80;
@@ -924,7 +930,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         // ------------------------------------------------------------------------------------------ dQ
         regs_up<152>();
         const int quarter = warp & 3, r0 = quarter * 32;
-        const uint32_t lane_addr = (uint32_t)r0 << 16, xbuf = sX + (uint32_t)(warp - 8) * DQ_BUF;
+        const uint32_t lane_addr = (uint32_t)r0 << 16, xbufs = sX + (uint32_t)(warp - 8) * 2 * DQ_BUF;
         bool ok = true;
         for (uint32_t it = 0; walk.more() && ok; walk.next(), ++it) {
             if (!mbar_wait_warp(smem_u32(&sh->dq_full), it & 1)) { if (lane == 0) fail_bwd(sh, 16); ok = false; break; }
@@ -941,7 +947,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
 #pragma unroll
             for (int c4 = 0; c4 < HD / 32; ++c4) {
                 if (c4 * 32 >= p.d) break;
-                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the one before has read the buffer
+                const uint32_t xbuf = xbufs + (c4 & 1) * DQ_BUF;
+                // the buffers in turn: all of the previous tile have been read by now, from the third on the last but one has
+                if (lane == 0 && c4 == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                if (lane == 0 && c4 >= 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                 __syncwarp();
                 const uint32_t srow = xbuf + (uint32_t)lane * 128;
 #pragma unroll
@@ -1053,7 +1062,8 @@ template <int HD, typename T>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdParams& p,
                int64_t batch, cudaStream_t stream) {
     constexpr uint32_t TB = (HD / 64) * CHUNK;
-    const size_t smem = 5 * TB + 2 * CHUNK + 4 * 32 * 128 + sizeof(BwdShared) + 1024;
+    const size_t smem = 5 * TB + 2 * CHUNK + 8 * DQ_BUF + sizeof(BwdShared);
+    static_assert(5 * 2 * CHUNK + 2 * CHUNK + 8 * DQ_BUF + sizeof(BwdShared) <= 227 * 1024, "shared memory of a block");
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(flash_bwd_kernel<HD, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -30;
