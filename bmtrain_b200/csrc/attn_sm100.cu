@@ -632,6 +632,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     // tensor memory columns: S^T / P^T [0,128), dP^T [128,256), dV, dK, dQ each of d columns; above head dim 80 dQ takes dP's
     const uint32_t C_DP = 128, C_DV = 256, C_DK = C_DV + p.d, C_DQ = p.d <= 80 ? C_DK + p.d : C_DP;
     const bool dq_shared = p.d > 80;
+    // Registers of the producer / issuer warpgroup and of the other three, of the 512 x 128 at launch.  The unrolled issue of 8-step
+    // products wants more than 48 (2x4096, 20 x 128 causal: 505 us with 48 / 152, 493 with 72 / 144); with 4 steps 48 do, and the
+    // softmax has use for the rest (1x8192, 16 x 64 causal: 460 against 464).
+    constexpr int FEW = HD == 128 ? 72 : 48, MANY = HD == 128 ? 144 : 152;
+    static_assert(128 * FEW + 384 * MANY <= 512 * 128, "registers of a block");
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int kvh = blockIdx.x % p.hk, b = blockIdx.x / p.hk, kt = blockIdx.y;   // under a causal mask the long columns start first
@@ -663,7 +668,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     const uint32_t tmem = sh->tmem_base;
 
     if (warp >= 12) {
-    regs_down<48>();             // 128 x 48 + 384 x 152 of the 512 x 128 registers at launch
+    regs_down<FEW>();
     if (warp == 12) {
         // ------------------------------------------------------------------------------------------ TMA producer
         if (work) {
@@ -794,7 +799,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     }
     } else if (warp < 8) {
         // ------------------------------------------------------------------------------------------ softmax: P and dS
-        regs_up<152>();
+        regs_up<MANY>();
         const int quarter = warp & 3, part = warp >> 2;             // 32 keys, 64 queries of the tile
         const int row = quarter * 32 + lane;
         const int64_t kj = kv0 + row;                                // this thread's key
@@ -928,7 +933,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         }
     } else {
         // ------------------------------------------------------------------------------------------ dQ
-        regs_up<152>();
+        regs_up<MANY>();
         const int quarter = warp & 3, r0 = quarter * 32;
         const uint32_t lane_addr = (uint32_t)r0 << 16, xbufs = sX + (uint32_t)(warp - 8) * 2 * DQ_BUF;
         bool ok = true;
