@@ -231,7 +231,8 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, con
     const T* src = EXTRA ? ebase + (row0 + sub) * e_ld + n0 + cq : nullptr;
     const T* bias = p.bias ? (const T*)p.bias + n0 + cq : nullptr;
     const int64_t d_step = 8 * p.ldc, e_step = 8 * e_ld;
-    const float alpha = p.alpha, floor = p.act == 1 ? 0.f : -INFINITY;
+    const float alpha = p.alpha;
+    const bool relu = p.act == 1;
     uint4 nx[4];
     auto fetch = [&](int c) {
         const bool col_ok = c * 32 + cq < n_cols;
@@ -267,7 +268,11 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, con
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[it][i] = fmaxf(v[it][i] * alpha + b[i], floor);
+            for (int i = 0; i < 8; ++i) v[it][i] = v[it][i] * alpha + b[i];
+            if (relu) {      // a branch, not a floor of -inf: fmaxf(NaN, -inf) is -inf
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[it][i] = fmaxf(v[it][i], 0.f);
+            }
             if (EXTRA) {
                 float e[8];
                 unpack8<T>(cur[it], e);

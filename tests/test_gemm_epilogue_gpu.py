@@ -61,3 +61,50 @@ def test_epilogue_forms(bmt_gpu, dtype, shape, form):
     assert (got - ref).abs().le(bound).all(), float(((got - ref).abs() - bound).max())
     assert torch.equal(store[:, n:], before[:, n:])      # columns behind the matrix are left alone
     assert lib.bmt_gemm_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,ldc", [(264, 264), (267, 272)])      # the compiled forms and the general one
+@pytest.mark.parametrize("form", ["plain", "bias", "bias_relu", "bias_gelu", "residual", "relu_mask", "gelu_mask", "accumulate", "float_out"])
+def test_epilogue_keeps_nan_and_inf(bmt_gpu, dtype, n, ldc, form):
+    """A product that is not a number, or infinite, arrives as such in every form (a ReLU maps NaN to zero, as fmaxf does)."""
+    from bmtrain_b200.ops import _native
+    from bmtrain_b200.parallel.fused_ops import _GemmDesc
+
+    m, k = 130, 64
+    a, b = torch.ones(m, k, device="cuda", dtype=dtype), torch.ones(n, k, device="cuda", dtype=dtype)
+    bad = {3: float("nan"), 64: float("inf"), 129: float("-inf")}
+    for row, value in bad.items():
+        a[row, 5] = value
+    out_dt = torch.float32 if form == "float_out" else dtype
+    store = torch.ones(m, ldc, device="cuda", dtype=out_dt)
+    ones, bias = torch.ones(m, n, device="cuda", dtype=dtype), torch.ones(n, device="cuda", dtype=dtype)
+    g = _GemmDesc()
+    g.m, g.n, g.k = m, n, k
+    g.a, g.lda, g.b, g.ldb = a.data_ptr(), k, b.data_ptr(), k
+    g.c, g.ldc, g.c_dtype, g.ab_dtype, g.alpha = store.data_ptr(), ldc, _DT[out_dt], _DT[dtype], 1.0
+    g.batch_inner = g.batch_outer = g.b_inner_div = 1
+    if form.startswith("bias"):
+        g.bias, g.act = bias.data_ptr(), {"bias": 0, "bias_relu": 1, "bias_gelu": 2}[form]
+    if "mask" in form:
+        g.aux, g.ld_aux, g.aux_mode = ones.data_ptr(), n, 1 if form == "relu_mask" else 2
+    if form == "residual":
+        g.residual, g.ldr = ones.data_ptr(), n
+    if form == "accumulate":
+        g.accumulate = 1
+    lib = _native.cuda_lib()
+    _native.check(lib.bmt_gemm_ex(ctypes.byref(g), _native.stream_handle()), "gemm")
+    got = store[:, :n].float()
+    finite = torch.ones(m, dtype=torch.bool, device="cuda")
+    finite[list(bad)] = False
+    assert torch.isfinite(got[finite]).all()
+    if form == "bias_relu":
+        assert not got[3].any() and not got[129].any()
+    else:
+        assert torch.isnan(got[3]).all()
+        if form == "bias_gelu":
+            assert not torch.isposinf(got[129]).any()        # -inf * 0 or -0, as the formula gives it
+        else:
+            assert torch.isneginf(got[129]).all()
+    assert torch.isposinf(got[64]).all()
+    assert lib.bmt_gemm_status() == 0
