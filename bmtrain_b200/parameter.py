@@ -152,12 +152,11 @@ class OpAllGather(torch.autograd.Function):
         comm: Communicator = ctx.comm
         per = (ctx.numel + comm.size - 1) // comm.size
         flat = grad_output.reshape(-1)
-        if comm.size == 1:
-            return flat
         if flat.numel() != per * comm.size:
             padded = torch.zeros(per * comm.size, dtype=flat.dtype, device=flat.device)
             padded[: flat.numel()].copy_(flat)
             flat = padded
+        # a tensor of its own on one rank too: autograd hands one tensor to several parameters, and each keeps what it gets
         out = torch.empty(per, dtype=flat.dtype, device=flat.device)
         comm.reduce_scatter_into(out, flat, "sum")
         start, end = ctx.bounds

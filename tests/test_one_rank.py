@@ -1,0 +1,45 @@
+"""One rank in the group: what a user's program may do with gathered parameters and gradients is what it may do on several
+ranks, although there is nothing to gather or to reduce."""
+import pytest
+import torch
+
+
+@pytest.fixture
+def bmt(bmt_cpu):
+    return bmt_cpu
+
+
+def _two(bmt):
+    class Two(bmt.DistributedModule):
+        def __init__(self):
+            super().__init__()
+            self.a = bmt.DistributedParameter(torch.arange(6.0).view(2, 3))
+            self.b = bmt.DistributedParameter(torch.ones(2, 3))
+
+        def forward(self, x):
+            return ((self.a + self.b + x) ** 2).sum()
+
+    return Two()
+
+
+def test_gradients_of_two_parameters_are_two_tensors(bmt):
+    """The operands of an addition get the same gradient from autograd; each parameter keeps one of its own."""
+    m, x = _two(bmt), torch.randn(2, 3)
+    m(x).backward()
+    once = m._parameters["a"].grad.clone()
+    assert torch.equal(m._parameters["b"].grad, once) and once.any()
+    assert m._parameters["a"].grad.data_ptr() != m._parameters["b"].grad.data_ptr()
+    m(x).backward()                                              # accumulates
+    for name in ("a", "b"):
+        assert torch.equal(m._parameters[name].grad, 2 * once)
+
+
+def test_clipping_scales_every_gradient_once(bmt):
+    m = _two(bmt)
+    opt = bmt.optim.AdamOptimizer(m.parameters(), lr=1e-3)
+    manager = bmt.optim.OptimManager(loss_scale=None)
+    manager.add_optimizer(opt)
+    manager.backward(m(torch.randn(2, 3) + 3))
+    manager.clip_grad_norm(opt.param_groups, 1.0)
+    norm = torch.stack([p.grad.norm() for p in m.parameters()]).norm()
+    assert abs(float(norm) - 1.0) < 1e-4
