@@ -92,8 +92,7 @@ class DistributedParameter(torch.nn.Parameter):
         """Full value over the ZeRO group (a new tensor; use :meth:`gather_all` to also undo TP)."""
         if self._in_block:
             raise RuntimeError("parameters inside a Block are gathered by the Block")
-        full = OpAllGather.apply(self).detach()
-        return full.clone() if self._zero_comm.size == 1 else full
+        return OpAllGather.apply(self).detach()
 
     def gather_all(self) -> torch.Tensor:
         """Full value with the tensor-parallel split undone as well."""
@@ -140,10 +139,8 @@ class OpAllGather(torch.autograd.Function):
         hook = getattr(value, "_bmt_pending_update", None)
         if hook is not None:
             hook(True)   # an asynchronous optimizer step is still rewriting this shard
-        if ctx.comm.size == 1 and getattr(value, "_bmt_grad_hook", None) is None:
-            # one rank: the shard is the whole value.  (An optimizer that uploads new values on a stream of its own does
-            # not wait for kernels that read them: those parameters are still copied.)
-            return value.detach().as_subclass(torch.Tensor).view(value._original_shape)
+        # a copy on one rank too: the caller may write to what it reads here, and backward uses the value of the forward pass
+        # although the shard may have been updated in between
         full = gather_flat_shard(value.data, ctx.numel, ctx.comm)
         return full.view(value._original_shape)
 

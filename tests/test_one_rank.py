@@ -43,3 +43,23 @@ def test_clipping_scales_every_gradient_once(bmt):
     manager.clip_grad_norm(opt.param_groups, 1.0)
     norm = torch.stack([p.grad.norm() for p in m.parameters()]).norm()
     assert abs(float(norm) - 1.0) < 1e-4
+
+
+def test_what_is_done_to_a_gathered_value_stays_there(bmt):
+    m = _two(bmt)
+    before = m._parameters["a"].detach().clone()
+    with torch.no_grad():
+        m.a.mul_(2)
+        m.a.data.add_(1)
+    m._parameters["a"].gather().zero_()
+    assert torch.equal(m._parameters["a"].detach(), before)
+
+
+def test_backward_uses_the_value_of_the_forward_pass(bmt):
+    m = _two(bmt)
+    x = torch.randn(2, 3, requires_grad=True)
+    y = (m.a * x).sum()
+    value = m._parameters["a"].detach().clone().view(2, 3)
+    m._parameters["a"].data.add_(20)                             # an update between the two passes
+    y.backward()
+    assert torch.equal(x.grad, value)
