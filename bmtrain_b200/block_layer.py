@@ -290,7 +290,7 @@ class _BlockFunction(torch.autograd.Function):
         ctx.arg_spec = arg_spec
         ctx.req = [t.requires_grad for t in tensors]
         ctx.checkpoint = block._use_checkpoint and not debug.get("_inspect_tensor", False)
-        block._enter_forward(_fill(arg_spec, tensors))
+        block._enter_forward(_fill(arg_spec, tensors), in_place=True)
         if ctx.checkpoint:
             ctx.rng = _rng_state()
             ctx.inputs = tensors
@@ -314,7 +314,7 @@ class _BlockFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *grad_outs):
         block: Block = ctx.block
-        block._enter_backward(_fill(ctx.arg_spec, ctx.inputs) if ctx.checkpoint else None)
+        block._enter_backward(_fill(ctx.arg_spec, ctx.inputs) if ctx.checkpoint else None, in_place=True)
         if ctx.checkpoint:
             detached = [t.detach().requires_grad_(r) for t, r in zip(ctx.inputs, ctx.req)]
             with _restore_rng(ctx.rng), torch.enable_grad():
@@ -488,12 +488,13 @@ class Block(torch.nn.Module):
             b.storage.data[s.lo - b.begin:s.hi - b.begin].copy_(flat[s.lo - s.offset:s.hi - s.offset])
 
     # ------------------------------------------------------ gather / release
-    def _begin_gather(self, prefetch: bool = False) -> None:
+    def _begin_gather(self, prefetch: bool = False, in_place: bool = False) -> None:
         """Start the all-gather of every bucket (no-op when resident or already in flight).  ``prefetch``: called on behalf
         of a neighbouring block; a bucket whose optimizer update has not landed yet is then left for later instead of
-        making the caller wait."""
+        making the caller wait.  ``in_place``: for a pass of the block; where ``_Bucket.in_place`` allows it the partition
+        itself will do.  Whoever looks at the parameters or keeps them (state dicts, ``ZeroContext``) gets a copy."""
         for b in self._buckets.values():
-            if b.full is not None and getattr(b, "full_epoch", -1) == _param_epoch[0]:
+            if b.full is not None and getattr(b, "full_epoch", -1) == _param_epoch[0] and (in_place or not b.aliased):
                 continue
             # the optimizer may hold the flat partition or the parameters that are views of it
             holders = [b.storage] + [s.param for s in b.slots]
@@ -502,7 +503,7 @@ class Block(torch.nn.Module):
             if b.full is not None and b.work is not None:
                 b.work.wait()  # a stale prefetch: let it finish before its buffer is dropped
             b.full_epoch = _param_epoch[0]
-            if b.in_place():
+            if in_place and b.in_place():
                 b.full, b.work, b.aliased = b.storage.data, None, True
                 continue
             b.full, b.aliased = torch.empty(b.total, dtype=b.dtype, device=b.storage.device), False
@@ -585,14 +586,14 @@ class Block(torch.nn.Module):
                                         ev_small=ev_small, push_rest=push_rest)
         return True
 
-    def _ensure_gathered(self, args=None, backward: bool = False) -> None:
+    def _ensure_gathered(self, args=None, backward: bool = False, in_place: bool = False) -> None:
         if args is not None:
             for b in self._buckets.values():
                 if b.full is None:
                     for h in [b.storage] + [s.param for s in b.slots]:
                         update_ready(h)
             self._try_deferred_gather(args, backward)
-        self._begin_gather()
+        self._begin_gather(in_place=in_place)
         for b in self._buckets.values():
             if b.work is not None:
                 b.work.wait()
@@ -802,11 +803,11 @@ class Block(torch.nn.Module):
                     hook(holder, None if accumulate else work)
 
     # ------------------------------------------------------------- scheduling
-    def _enter_forward(self, args=None) -> None:
-        self._ensure_gathered(args)
+    def _enter_forward(self, args=None, in_place: bool = False) -> None:
+        self._ensure_gathered(args, in_place=in_place)
         nxt = self.next_module()
         if nxt is not None and nxt._mode != "PIPE":
-            nxt._begin_gather(prefetch=True)
+            nxt._begin_gather(prefetch=True, in_place=in_place)
 
     def _exit_forward(self) -> None:
         if self._mode == "PIPE" and self._micro_idx != config["micros"] - 1:
@@ -818,12 +819,12 @@ class Block(torch.nn.Module):
         else:
             self._release_params()
 
-    def _enter_backward(self, args=None) -> None:
-        self._ensure_gathered(args, backward=True)
+    def _enter_backward(self, args=None, in_place: bool = False) -> None:
+        self._ensure_gathered(args, backward=True, in_place=in_place)
         self._prepare_grads(attach=False)
         pre = self.pre_module()
         if pre is not None and pre._mode != "PIPE" and pre._zero_level == 3:
-            pre._begin_gather(prefetch=True)
+            pre._begin_gather(prefetch=True, in_place=in_place)
 
     def _exit_backward(self) -> None:
         if self._mode == "PIPE":
@@ -866,7 +867,7 @@ class Block(torch.nn.Module):
 
         if not self._grad_mode:
             # nothing to differentiate: gather, run once, release
-            self._enter_forward()
+            self._enter_forward(in_place=True)
             try:
                 out = self._module(*args)
             finally:

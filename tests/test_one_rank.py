@@ -63,3 +63,32 @@ def test_backward_uses_the_value_of_the_forward_pass(bmt):
     m._parameters["a"].data.add_(20)                             # an update between the two passes
     y.backward()
     assert torch.equal(x.grad, value)
+
+
+def _gpt_block(bmt):
+    from bmtrain_b200.models.gpt import TransformerEncoder
+
+    torch.manual_seed(3)
+    blk = bmt.Block(TransformerEncoder(16, 8, 2, 32, dtype=torch.float32))
+    bmt.init_parameters(blk)
+    return blk
+
+
+def test_state_dict_is_a_snapshot(bmt):
+    blk = _gpt_block(bmt)
+    saved = blk.state_dict()
+    kept = {k: v.clone() for k, v in saved.items()}
+    for b in blk._buckets.values():
+        b.storage.data.add_(1)                                   # the next optimizer step
+    assert all(torch.equal(saved[k], kept[k]) for k in kept)
+
+
+def test_zero_context_hands_out_a_copy(bmt):
+    from bmtrain_b200.zero_context import ZeroContext
+
+    blk = _gpt_block(bmt)
+    before = [b.storage.data.clone() for b in blk._buckets.values()]
+    with ZeroContext(blk):
+        for p in blk._module.parameters():
+            p.data.add_(1)
+    assert all(torch.equal(b.storage.data, was) for b, was in zip(blk._buckets.values(), before))
