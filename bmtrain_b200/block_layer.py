@@ -31,6 +31,7 @@ import torch
 from . import debug
 from .comm import Communicator, DONE
 from .global_var import config
+from .layer import only_reads_parameters
 from .parameter import DistributedParameter, gather_flat_shard
 from .utils import round_up, tp_split_tensor
 
@@ -290,7 +291,7 @@ class _BlockFunction(torch.autograd.Function):
         ctx.arg_spec = arg_spec
         ctx.req = [t.requires_grad for t in tensors]
         ctx.checkpoint = block._use_checkpoint and not debug.get("_inspect_tensor", False)
-        block._enter_forward(_fill(arg_spec, tensors), in_place=True)
+        block._enter_forward(_fill(arg_spec, tensors), in_place=block._may_run_in_place())
         if ctx.checkpoint:
             ctx.rng = _rng_state()
             ctx.inputs = tensors
@@ -314,7 +315,8 @@ class _BlockFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *grad_outs):
         block: Block = ctx.block
-        block._enter_backward(_fill(ctx.arg_spec, ctx.inputs) if ctx.checkpoint else None, in_place=True)
+        block._enter_backward(_fill(ctx.arg_spec, ctx.inputs) if ctx.checkpoint else None,
+                              in_place=ctx.checkpoint and block._may_run_in_place())
         if ctx.checkpoint:
             detached = [t.detach().requires_grad_(r) for t, r in zip(ctx.inputs, ctx.req)]
             with _restore_rng(ctx.rng), torch.enable_grad():
@@ -491,8 +493,9 @@ class Block(torch.nn.Module):
     def _begin_gather(self, prefetch: bool = False, in_place: bool = False) -> None:
         """Start the all-gather of every bucket (no-op when resident or already in flight).  ``prefetch``: called on behalf
         of a neighbouring block; a bucket whose optimizer update has not landed yet is then left for later instead of
-        making the caller wait.  ``in_place``: for a pass of the block; where ``_Bucket.in_place`` allows it the partition
-        itself will do.  Whoever looks at the parameters or keeps them (state dicts, ``ZeroContext``) gets a copy."""
+        making the caller wait.  ``in_place``: for a pass of the block that is known to read its parameters only
+        (``_may_run_in_place``); where ``_Bucket.in_place`` allows it the partition itself will do.  Whoever else looks at
+        the parameters or keeps them (state dicts, ``ZeroContext``) gets a copy."""
         for b in self._buckets.values():
             if b.full is not None and getattr(b, "full_epoch", -1) == _param_epoch[0] and (in_place or not b.aliased):
                 continue
@@ -803,11 +806,19 @@ class Block(torch.nn.Module):
                     hook(holder, None if accumulate else work)
 
     # ------------------------------------------------------------- scheduling
+    def _may_run_in_place(self) -> bool:
+        """Whether a pass may compute on the partition itself (if ``_Bucket.in_place``) instead of a copy.  Code that is not
+        known may write to what it is given, which changes a copy that is dropped afterwards and must not change the
+        parameters.  And nothing that forward read may be used after it: ZeRO-2 keeps its copy for backward, a block
+        without recomputation saves views for autograd, and an optimizer step may come in between."""
+        return (self._zero_level == 3 and self._use_checkpoint and not debug.get("_inspect_tensor", False)
+                and all(b.comm.size == 1 for b in self._buckets.values()) and only_reads_parameters(self._module))
+
     def _enter_forward(self, args=None, in_place: bool = False) -> None:
         self._ensure_gathered(args, in_place=in_place)
         nxt = self.next_module()
         if nxt is not None and nxt._mode != "PIPE":
-            nxt._begin_gather(prefetch=True, in_place=in_place)
+            nxt._begin_gather(prefetch=True, in_place=nxt._may_run_in_place())
 
     def _exit_forward(self) -> None:
         if self._mode == "PIPE" and self._micro_idx != config["micros"] - 1:
@@ -824,7 +835,7 @@ class Block(torch.nn.Module):
         self._prepare_grads(attach=False)
         pre = self.pre_module()
         if pre is not None and pre._mode != "PIPE" and pre._zero_level == 3:
-            pre._begin_gather(prefetch=True, in_place=in_place)
+            pre._begin_gather(prefetch=True, in_place=pre._may_run_in_place())
 
     def _exit_backward(self) -> None:
         if self._mode == "PIPE":
@@ -867,7 +878,7 @@ class Block(torch.nn.Module):
 
         if not self._grad_mode:
             # nothing to differentiate: gather, run once, release
-            self._enter_forward(in_place=True)
+            self._enter_forward(in_place=self._may_run_in_place())
             try:
                 out = self._module(*args)
             finally:

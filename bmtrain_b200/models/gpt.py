@@ -17,7 +17,7 @@ import torch
 from .. import inspect as bmt_inspect
 from ..block_layer import Block, TransformerBlockList
 from ..global_var import config
-from ..layer import DistributedModule
+from ..layer import DistributedModule, reads_parameters_only
 from ..nn import ColumnParallelLinear, Embedding, LayerNorm, Linear, RowParallelLinear, VPEmbedding
 from ..ops import attention as _attn
 from ..ops import gpt_block as _gpt_block
@@ -27,6 +27,7 @@ from ..ops import gpt_block as _gpt_block
 _FUSED_BLOCK = os.environ.get("BMT_FUSED_BLOCK", "1") != "0"
 
 
+@reads_parameters_only
 class Attention(DistributedModule):
     """Multi-head self attention with a fused QKV projection."""
 
@@ -65,6 +66,7 @@ class Attention(DistributedModule):
         return self.project_out(out)
 
 
+@reads_parameters_only
 class Feedforward(DistributedModule):
     def __init__(self, dim_model: int, dim_ff: int, bias: bool = True, dtype=None, activation: str = "relu"):
         super().__init__()
@@ -82,6 +84,7 @@ class Feedforward(DistributedModule):
         return self.w_out(h)
 
 
+@reads_parameters_only
 class TransformerEncoder(DistributedModule):
     """One pre-LN block."""
 

@@ -13,12 +13,13 @@ import torch
 
 from ..block_layer import Block, TransformerBlockList
 from ..global_var import config
-from ..layer import DistributedModule
+from ..layer import DistributedModule, reads_parameters_only
 from ..nn import ColumnParallelLinear, Embedding, Linear, RMSNorm, RowParallelLinear, VPEmbedding
 from ..ops import attention as _attn
 from ..ops import elementwise as _ew
 
 
+@reads_parameters_only
 class LlamaAttention(DistributedModule):
     def __init__(self, dim_model: int, num_heads: int, num_kv_heads: int, dim_head: int, dtype=None, rope_theta: float = 10000.0):
         super().__init__()
@@ -52,6 +53,7 @@ class LlamaAttention(DistributedModule):
         return self.project_out(out)
 
 
+@reads_parameters_only
 class LlamaMLP(DistributedModule):
     """``w_out(silu(gate) * up)`` with gate and up projections fused into one GEMM (interleaved per TP rank)."""
 
@@ -68,6 +70,7 @@ class LlamaMLP(DistributedModule):
         return self.w_out(_ew.swiglu(self.w_gate_up(x)))
 
 
+@reads_parameters_only
 class LlamaBlock(DistributedModule):
     def __init__(self, dim_model, num_heads, num_kv_heads, dim_head, dim_ff, dtype=None, eps=1e-5):
         super().__init__()

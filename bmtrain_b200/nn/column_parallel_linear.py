@@ -1,10 +1,12 @@
 """Column-parallel linear: the output features are split over the tensor-parallel group
 (reference: ``bmtrain/nn/column_parallel_linear.py:9-80``)."""
 from ..global_var import config
+from ..layer import reads_parameters_only
 from ._tp_linear import ShardedLinearBase
 from .parallel_linear_func import OpParallelLinear
 
 
+@reads_parameters_only
 class ColumnParallelLinear(ShardedLinearBase):
     """``y_local = gather_tokens(x) W_r^T + b_r`` with ``W_r`` = rows ``[r*out/tp, (r+1)*out/tp)`` of the full weight.
 

@@ -10,13 +10,14 @@ from typing import Optional
 
 import torch
 
-from ..layer import DistributedModule
+from ..layer import DistributedModule, reads_parameters_only
 from ..ops import embedding as _emb
 from ..ops import gemm as _gemm
 from ..ops import norm as _norm
 from ..parameter import DistributedParameter, ParameterInitializer
 
 
+@reads_parameters_only
 class Embedding(DistributedModule):
     """Token embedding; ``forward(x, projection=True)`` multiplies by the transposed table (tied LM head)."""
 
@@ -37,6 +38,7 @@ class Embedding(DistributedModule):
         return f"{self.num_embeddings}, {self.embedding_dim}"
 
 
+@reads_parameters_only
 class LayerNorm(DistributedModule):
     """LayerNorm over the last dimension."""
 
@@ -63,6 +65,7 @@ class LayerNorm(DistributedModule):
 Layernorm = LayerNorm
 
 
+@reads_parameters_only
 class RMSNorm(DistributedModule):
     """Root-mean-square norm over the last dimension (Llama style)."""
 

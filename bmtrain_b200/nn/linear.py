@@ -1,7 +1,7 @@
 """Plain (non tensor-parallel) linear layer on sharded parameters (reference: ``bmtrain/nn/linear.py:6-56``)."""
 import torch
 
-from ..layer import DistributedModule
+from ..layer import DistributedModule, reads_parameters_only
 from ..ops import gemm as _gemm
 from ..parameter import DistributedParameter
 
@@ -18,6 +18,7 @@ class OpLinear(torch.autograd.Function):
         return _gemm.LinearFunction.backward(ctx, grad_output)
 
 
+@reads_parameters_only
 class Linear(DistributedModule):
     """``y = x W^T + b`` with ``W`` of shape (out_features, in_features), Xavier-normal initialised."""
 

@@ -11,7 +11,7 @@ multiplied by the local vocabulary shard, giving logits ``(..., vocab / tp)``.
 import torch
 
 from ..global_var import config
-from ..layer import DistributedModule
+from ..layer import DistributedModule, reads_parameters_only
 from ..ops import embedding as _emb
 from ..parameter import DistributedParameter, ParameterInitializer
 from .parallel_linear_func import OpParallelLinear
@@ -61,6 +61,7 @@ class _VocabParallelLookup(torch.autograd.Function):
         return None, _emb.embedding_backward(idx, g_all, ctx.rows), None
 
 
+@reads_parameters_only
 class VPEmbedding(DistributedModule):
     """Embedding whose vocabulary is sharded over the tensor-parallel group."""
 

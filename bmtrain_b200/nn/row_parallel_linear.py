@@ -3,6 +3,7 @@
 import torch
 
 from ..global_var import config
+from ..layer import reads_parameters_only
 from ._tp_linear import ShardedLinearBase
 from .parallel_linear_func import OpParallelLinear, ReduceType
 
@@ -25,6 +26,7 @@ class _AddReplicatedBias(torch.autograd.Function):
         return grad, gb
 
 
+@reads_parameters_only
 class RowParallelLinear(ShardedLinearBase):
     """``y = reduce(x_r W_r^T) + b`` with ``W_r`` = columns ``[r*in/tp, (r+1)*in/tp)`` of the full weight.
 
