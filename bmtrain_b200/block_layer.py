@@ -172,6 +172,7 @@ class _Bucket:
         self.aliased = False        # `full` is the partition itself
         self.full_grad: Optional[torch.Tensor] = None
         self.full_grad_ptr = 0
+        self.attached = False       # the inner `.grad` fields are views of `full_grad`
         self.grads_open = False     # the block's autograd backward is running: kernels may write into the slots
         self.work = None
         self._views_of = None       # the storage memory `_local_views` / `_full_views` look at
@@ -315,8 +316,9 @@ class _BlockFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *grad_outs):
         block: Block = ctx.block
+        plain = only_reads_parameters(block._module)
         block._enter_backward(_fill(ctx.arg_spec, ctx.inputs) if ctx.checkpoint else None,
-                              in_place=ctx.checkpoint and block._may_run_in_place())
+                              in_place=plain and ctx.checkpoint and block._may_run_in_place(plain), attach=not plain)
         if ctx.checkpoint:
             detached = [t.detach().requires_grad_(r) for t, r in zip(ctx.inputs, ctx.req)]
             with _restore_rng(ctx.rng), torch.enable_grad():
@@ -330,7 +332,7 @@ class _BlockFunction(torch.autograd.Function):
                 outs.append(o)
                 grads.append(g)
         if outs:
-            block._open_grads(True)
+            block._open_grads(plain)
             try:
                 torch.autograd.backward(outs, grads)
             finally:
@@ -649,13 +651,17 @@ class Block(torch.nn.Module):
     def _prepare_grads(self, attach: bool = True) -> None:
         """Full-size gradient buffers.
 
-        ``attach`` true: zeroed, and inner ``.grad`` fields become views into them.  False (the block's own backward pass):
-        left as they are apart from the gaps between the slots -- a kernel writes a gradient straight into its slot
+        ``attach`` true: zeroed, and inner ``.grad`` fields become views into them, which an autograd function inside the
+        block may add to in place.  False (backward of a block whose code is known, ``only_reads_parameters``): left as
+        they are apart from the gaps between the slots -- a kernel writes a gradient straight into its slot
         (``ops/grad_slot.py``) or autograd leaves it in ``.grad``, and ``_scatter_grads`` fills in the rest, so that a
         gradient is neither added to zeros nor written twice."""
         for b in self._buckets.values():
             needs = [s for s in b.slots if s.param.requires_grad]
             fresh = b.full_grad is None
+            if attach and not fresh and not b.attached:
+                self._complete_grads(b)      # an earlier micro-batch ran without
+            b.attached = attach
             if fresh or attach:
                 for s in b.slots:
                     s.param.grad = None
@@ -687,6 +693,7 @@ class Block(torch.nn.Module):
                     s.written = attach
             if attach:
                 for s in needs:
+                    s.written = True
                     s.param.grad = s.grad_view()
 
     def _open_grads(self, is_open: bool) -> None:
@@ -725,7 +732,7 @@ class Block(torch.nn.Module):
     def _scatter_grads(self) -> None:
         """Reduce-scatter the full gradient buffers onto the partitions (asynchronously)."""
         for b in self._buckets.values():
-            if b.full_grad is not None:
+            if b.full_grad is not None and not b.attached:
                 self._complete_grads(b)
             for s in b.slots:
                 s.param.grad = None
@@ -806,13 +813,14 @@ class Block(torch.nn.Module):
                     hook(holder, None if accumulate else work)
 
     # ------------------------------------------------------------- scheduling
-    def _may_run_in_place(self) -> bool:
+    def _may_run_in_place(self, plain: Optional[bool] = None) -> bool:
         """Whether a pass may compute on the partition itself (if ``_Bucket.in_place``) instead of a copy.  Code that is not
         known may write to what it is given, which changes a copy that is dropped afterwards and must not change the
         parameters.  And nothing that forward read may be used after it: ZeRO-2 keeps its copy for backward, a block
-        without recomputation saves views for autograd, and an optimizer step may come in between."""
+        without recomputation saves views for autograd, and an optimizer step may come in between.  ``plain``: what ``only_reads_parameters`` says of the module, if the caller knows."""
         return (self._zero_level == 3 and self._use_checkpoint and not debug.get("_inspect_tensor", False)
-                and all(b.comm.size == 1 for b in self._buckets.values()) and only_reads_parameters(self._module))
+                and all(b.comm.size == 1 for b in self._buckets.values())
+                and (only_reads_parameters(self._module) if plain is None else plain))
 
     def _enter_forward(self, args=None, in_place: bool = False) -> None:
         self._ensure_gathered(args, in_place=in_place)
@@ -830,9 +838,9 @@ class Block(torch.nn.Module):
         else:
             self._release_params()
 
-    def _enter_backward(self, args=None, in_place: bool = False) -> None:
+    def _enter_backward(self, args=None, in_place: bool = False, attach: bool = True) -> None:
         self._ensure_gathered(args, backward=True, in_place=in_place)
-        self._prepare_grads(attach=False)
+        self._prepare_grads(attach)
         pre = self.pre_module()
         if pre is not None and pre._mode != "PIPE" and pre._zero_level == 3:
             pre._begin_gather(prefetch=True, in_place=pre._may_run_in_place())

@@ -16,6 +16,7 @@ import itertools
 import torch
 
 from .global_var import config
+from .ops import grad_slot
 from .parameter import DistributedParameter, OpAllGather
 from .utils import tp_split_tensor
 
@@ -38,7 +39,7 @@ def only_reads_parameters(module: torch.nn.Module) -> bool:
         if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks:
             return False
         for p in m._parameters.values():
-            if p is not None and (p._backward_hooks or p._post_accumulate_grad_hooks):
+            if p is not None and grad_slot.watched(p):
                 return False
         return all(plain(c) for c in m._modules.values() if c is not None)
 

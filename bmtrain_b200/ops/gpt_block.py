@@ -175,7 +175,8 @@ class GPTBlockFunction(torch.autograd.Function):
         # gradients of the parameters go straight into the owning block's gradient buffer, or accumulate in place when the
         # owner attached same-dtype gradient buffers (no tensor goes back to autograd for them then)
         def attached(p):
-            return p.is_leaf and p.requires_grad and p.grad is not None and p.grad.dtype == dt and p.grad.is_contiguous()
+            return (p.is_leaf and p.requires_grad and p.grad is not None and p.grad.dtype == dt and p.grad.is_contiguous()
+                    and not _grad_slot.watched(p))
 
         grads = {}
         for names, flag in ((_WEIGHTS, "acc_w"), (_SMALL, "acc_small")):
