@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(256) ce_row_stats_kernel(int64_t m, int64_t n,
     for (int64_t i = threadIdx.x; i < head + n - tail; i += blockDim.x) {
         const float f = bmt::Cvt<T>::to_f(xr[i < head ? i : tail + i - head]);
         if (f > mx) { se *= ex2((mx - f) * L2E); mx = f; }
-        se += ex2((f - mx) * L2E);
+        if (f != -INFINITY) se += ex2((f - mx) * L2E);      // a hidden class adds nothing, also before the first finite one
     }
     for (int64_t i0 = threadIdx.x; i0 < nv; i0 += (int64_t)blockDim.x * U) {
         bmt::Vec16<T> v[U];
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256) ce_row_stats_kernel(int64_t m, int64_t n,
                 for (int k = 0; k < V; ++k) lm = fmaxf(lm, bmt::Cvt<T>::to_f(v[u].v[k]));
             }
         if (lm > mx) { se *= ex2((mx - lm) * L2E); mx = lm; }
-        const float off = -mx * L2E;
+        const float off = mx == -INFINITY ? 0.f : -mx * L2E;   // all classes so far hidden: 2^-inf, not 2^(inf - inf)
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (i0 + (int64_t)u * blockDim.x < nv) {
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(256) ce_row_stats_kernel(int64_t m, int64_t n,
             }
     }
     const float gmx = bmt::block_allreduce<true>(mx, scratch);
-    const float contrib = (mx == -INFINITY) ? 0.f : se * __expf(mx - gmx);
+    const float contrib = se == 0.f ? 0.f : se * __expf(mx - gmx);   // zero: no class that counts (a NaN is not lost)
     const float gse = bmt::block_allreduce<false>(contrib, scratch);
     if (threadIdx.x == 0) {
         const int64_t t = target[row] - vocab_start;
@@ -95,8 +95,8 @@ __device__ __forceinline__ float packet_max(const bmt::Vec16<__nv_bfloat16>& v) 
 __device__ __forceinline__ void lse_combine(float& m, float& s, float m2, float s2) {
     constexpr float L2E = 1.4426950408889634f;
     const float nm = fmaxf(m, m2);
-    const float a = (m == -INFINITY) ? 0.f : s * ex2((m - nm) * L2E);
-    const float b = (m2 == -INFINITY) ? 0.f : s2 * ex2((m2 - nm) * L2E);
+    const float a = s == 0.f ? 0.f : s * ex2((m - nm) * L2E);       // zero: no class that counts yet
+    const float b = s2 == 0.f ? 0.f : s2 * ex2((m2 - nm) * L2E);
     m = nm;
     s = a + b;
 }
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) ce_row_stats_stream_kernel(int64_t m, int
         for (int u = 0; u < U; ++u)
             if (base + u * 256 < nv) lm = fmaxf(lm, packet_max(v[u]));
         if (lm > mx) { se *= ex2((mx - lm) * L2E); mx = lm; }   // mx = -inf: se is 0 and stays 0 (0 * 2^-inf)
-        const float off = -mx * L2E;
+        const float off = mx == -INFINITY ? 0.f : -mx * L2E;
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (base + u * 256 < nv) {

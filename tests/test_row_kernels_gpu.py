@@ -83,3 +83,34 @@ def test_embedding_gradient(bmt_gpu, dtype, tokens, rows, d):
     size = torch.zeros(rows, d, dtype=torch.float64, device="cuda").index_add_(0, ids[keep], g[keep].double().abs())
     assert got.dtype == dtype
     assert (got.double() - want).abs().le(_UNIT[dtype] * want.abs() + tokens * 2.0 ** -24 * size + 1e-7).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("classes", [33, 1000, 2047, 4096, 12289, 12296])       # odd and even, scalar, vector and streaming rows
+def test_cross_entropy_of_hidden_classes(bmt_gpu, dtype, classes):
+    """Classes hidden with -inf: the first ones, the last ones, all but one, a thread's whole first trip, everything a thread
+    sees; and rows with a NaN, which must not come out finite."""
+    gen = torch.Generator(device="cuda").manual_seed(classes)
+    x = torch.randn(8, classes, generator=gen, device="cuda").to(dtype)
+    inf = float("inf")
+    x[0, :9] = -inf
+    x[1, -9:] = -inf
+    x[2, :] = -inf
+    x[2, classes // 2] = 1.0
+    x[3, : min(classes - 1, 8 * 256 * 4 + 5)] = -inf
+    x[4, (torch.arange(classes, device="cuda") // 8) % 3 != 1] = -inf
+    x[5, classes - 1] = float("nan")
+    x[6, 0] = float("nan")
+    t = torch.full((8,), classes - 1, device="cuda")
+    t[1], t[2], t[4] = classes // 2, classes // 2, 9
+    x = x.requires_grad_()
+    loss = bmt_gpu.loss.FusedCrossEntropy(reduction="none")(x, t)
+    (gx,) = torch.autograd.grad(loss, (x,), torch.ones_like(loss))
+    xe = x.detach().double().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(xe, t, reduction="none")
+    (ge,) = torch.autograd.grad(ref, (xe,), torch.ones_like(ref))
+    good = [0, 1, 2, 3, 4, 7]
+    assert torch.isnan(loss[[5, 6]]).all()
+    assert (loss[good].double() - ref[good]).abs().le(3e-6 * ref[good].abs() + 2e-6).all()
+    assert (gx[good].double() - ge[good]).abs().le(1.5 * _UNIT[dtype] * ge[good].abs() + 2e-6 + (6e-8 if dtype == torch.float16 else 0)).all()
+    assert torch.isnan(gx[[5, 6]]).any(1).all()
