@@ -32,19 +32,30 @@ __global__ void __launch_bounds__(256) ce_row_stats_kernel(int64_t m, int64_t n,
     const int64_t row = blockIdx.x;
     const T* __restrict__ xr = x + row * n;
     constexpr int V = bmt::Vec16<T>::N;
-    float mx = -INFINITY, se = 0.f;
+    // mx: largest logit so far; se: sum of 2^(x * log2e - ref) with ref = mx * log2e as it is rounded.  Taking the rounded product
+    // as the reference keeps the exponent exact to one rounding of the FMA; its distance from mx * log2e is made up for once, at
+    // the end.
+    float mx = -INFINITY, ref = 0.f, se = 0.f;
     // Rows of an odd number of classes start anywhere: the few elements before the first 16-byte boundary and behind the last
-    // whole vector go one by one, the rest as vectors (4096 x 50257 bf16 element by element: 242 us forward, 356 us backward; 97 and 141 us now).
+    // whole vector go one by one, the rest as vectors (4096 x 50257 bf16 element by element: 242 us forward, 356 us backward;
+    // 104 and 141 us so).
     // U vectors per thread and trip: all loads are issued before the first use, the running maximum moves at most
-    // once per trip, and every element costs one FMA and one ex2 (base-2 exponent of x * log2e - max * log2e)
+    // once per trip, and every element costs one FMA and one ex2
     constexpr int U = 4;
     constexpr float L2E = 1.4426950408889634f;
     const int64_t head = row_head<T>(xr, n), nv = (n - head) / V, tail = head + nv * V;
     const T* __restrict__ xv = xr + head;
+    const auto move_to = [&](float v) {
+        if (!(v > mx)) return;
+        const float r = v * L2E;
+        if (mx != -INFINITY) se *= ex2(ref - r);
+        mx = v;
+        ref = r;
+    };
     for (int64_t i = threadIdx.x; i < head + n - tail; i += blockDim.x) {
         const float f = bmt::Cvt<T>::to_f(xr[i < head ? i : tail + i - head]);
-        if (f > mx) { se *= ex2((mx - f) * L2E); mx = f; }
-        if (f != -INFINITY) se += ex2((f - mx) * L2E);      // a hidden class adds nothing, also before the first finite one
+        move_to(f);
+        se += ex2(fmaf(f, L2E, -ref));       // ref is 0 as long as all classes are hidden (-inf): they add nothing
     }
     for (int64_t i0 = threadIdx.x; i0 < nv; i0 += (int64_t)blockDim.x * U) {
         bmt::Vec16<T> v[U];
@@ -58,8 +69,8 @@ __global__ void __launch_bounds__(256) ce_row_stats_kernel(int64_t m, int64_t n,
 #pragma unroll
                 for (int k = 0; k < V; ++k) lm = fmaxf(lm, bmt::Cvt<T>::to_f(v[u].v[k]));
             }
-        if (lm > mx) { se *= ex2((mx - lm) * L2E); mx = lm; }
-        const float off = mx == -INFINITY ? 0.f : -mx * L2E;   // all classes so far hidden: 2^-inf, not 2^(inf - inf)
+        move_to(lm);
+        const float off = -ref;
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (i0 + (int64_t)u * blockDim.x < nv) {
@@ -68,7 +79,7 @@ __global__ void __launch_bounds__(256) ce_row_stats_kernel(int64_t m, int64_t n,
             }
     }
     const float gmx = bmt::block_allreduce<true>(mx, scratch);
-    const float contrib = se == 0.f ? 0.f : se * __expf(mx - gmx);   // zero: no class that counts (a NaN is not lost)
+    const float contrib = se == 0.f ? 0.f : se * ex2(-fmaf(gmx, L2E, -ref));   // zero: no class that counts (a NaN is not lost)
     const float gse = bmt::block_allreduce<false>(contrib, scratch);
     if (threadIdx.x == 0) {
         const int64_t t = target[row] - vocab_start;
@@ -212,15 +223,17 @@ __global__ void __launch_bounds__(256) ce_backward_kernel(int64_t m, int64_t n, 
     const float g = ignored ? 0.f : divisor ? grad[0] / divisor[0] : grad[row];
     constexpr int V = bmt::Vec16<T>::N;
     constexpr float L2E = 1.4426950408889634f;
-    const float off = -l * L2E;
+    // p = 2^(x * log2e + off) * 2^rest: `off` is -l * log2e as it is rounded, which near p = 1 is not exact enough, `rest` what
+    // the rounding dropped (exact); the second factor goes into the multiplication by g
+    const float off = -l * L2E, rest = fmaf(-l, L2E, -off);
+    const float pg = fabsf(l) < INFINITY ? g * ex2(rest) : g;
     // as in the forward kernel; vectors need the logits and the gradient to be off the 16-byte boundary by the same amount
     const bool same = (((uintptr_t)xr ^ (uintptr_t)orow) & 15) == 0;
     const int64_t head = same ? row_head<T>(xr, n) : n, nv = (n - head) / V, tail = head + nv * V;
     for (int64_t i = threadIdx.x; i < head + n - tail; i += blockDim.x) {
         const int64_t c = i < head ? i : tail + i - head;
-        float p = ex2(fmaf(bmt::Cvt<T>::to_f(xr[c]), L2E, off));
-        if (c == t) p -= 1.f;
-        orow[c] = bmt::Cvt<T>::from_f(p * g);
+        const float p = ex2(fmaf(bmt::Cvt<T>::to_f(xr[c]), L2E, off));
+        orow[c] = bmt::Cvt<T>::from_f(fmaf(p, pg, c == t ? -g : 0.f));
     }
     constexpr int U = 4;
     for (int64_t i0 = threadIdx.x; i0 < nv; i0 += (int64_t)blockDim.x * U) {
@@ -235,9 +248,8 @@ __global__ void __launch_bounds__(256) ce_backward_kernel(int64_t m, int64_t n, 
             bmt::Vec16<T> o;
 #pragma unroll
             for (int k = 0; k < V; ++k) {
-                float p = ex2(fmaf(bmt::Cvt<T>::to_f(v[u].v[k]), L2E, off));
-                if (head + i * V + k == t) p -= 1.f;
-                o.v[k] = bmt::Cvt<T>::from_f(p * g);
+                const float p = ex2(fmaf(bmt::Cvt<T>::to_f(v[u].v[k]), L2E, off));
+                o.v[k] = bmt::Cvt<T>::from_f(fmaf(p, pg, head + i * V + k == t ? -g : 0.f));
             }
             bmt::st16(orow + head + i * V, o);
         }

@@ -114,3 +114,30 @@ def test_cross_entropy_of_hidden_classes(bmt_gpu, dtype, classes):
     assert (loss[good].double() - ref[good]).abs().le(3e-6 * ref[good].abs() + 2e-6).all()
     assert (gx[good].double() - ge[good]).abs().le(1.5 * _UNIT[dtype] * ge[good].abs() + 2e-6 + (6e-8 if dtype == torch.float16 else 0)).all()
     assert torch.isnan(gx[[5, 6]]).any(1).all()
+
+
+@pytest.mark.parametrize("classes", [33, 1024, 5001])
+@pytest.mark.parametrize("level", [0.0, 14.0, 65.0, 700.0])
+def test_cross_entropy_is_exact_near_the_target(bmt_gpu, classes, level):
+    """fp32 logits around ``level``, one class far above the others.  The exponent is x - lse up to one rounding of that
+    difference and the 1.3e-8 that the fp32 log2(e) is off; each 2^x is good to 2 ulp (4 units), each product to one unit."""
+    from bmtrain_b200.ops import cross_entropy as C
+
+    gen = torch.Generator(device="cuda").manual_seed(classes)
+    x = torch.randn(64, classes, generator=gen, device="cuda") * 3 + level
+    t = torch.randint(0, classes, (64,), generator=gen, device="cuda")
+    x[torch.arange(32), t[:32]] = level + 30.0
+    lse = torch.logsumexp(x.double(), 1).float()
+    g = torch.rand(64, generator=gen, device="cuda") + 0.5
+    got = C.ce_backward(x, t, lse, g, ignore_index=-100)
+    gap = x.double() - lse.double()[:, None]
+    p = gap.exp()
+    want = (p - torch.nn.functional.one_hot(t, classes)) * g.double()[:, None]
+    unit = 2.0 ** -24
+    bound = g[:, None] * p * (10 * unit + 2 * unit * gap.abs()) + unit * want.abs() + 1e-37
+    assert (got.double() - want).abs().le(bound).all(), float(((got.double() - want).abs() - bound).max())
+    mx, se, _ = C.row_stats(x, t)
+    top = x.double().max(1).values
+    exact = (x.double() - top[:, None]).exp().sum(1)
+    assert torch.equal(mx.double(), top)
+    assert (se.double() - exact).abs().le((16 + classes / 256 + 8) * unit * exact).all()
