@@ -63,6 +63,9 @@ int bmt_norm_bwd_ex(int64_t rows, int64_t d, const void* x, const void* dy, cons
                     int dtype, int nblk, void* dx, void* partial_2xnblkxd_f32, void* dw, void* db, const void* dres,
                     int accumulate, void* stream);
 
+// 0, or (1 << 16 | CTA) of the first CTA of a norm backward whose bounded wait ran out (its weight gradient is NaN then); reading clears it
+int bmt_norm_status(void);
+
 int bmt_embedding_fwd(int64_t tokens, int64_t d, const void* ids_i64, const void* weight, int dtype, void* out, void* stream);
 int64_t bmt_embedding_bwd_scratch(int64_t tokens, int64_t rows);   // 32-bit words of scratch
 int bmt_embedding_bwd(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out, void* scratch,

@@ -6,6 +6,7 @@
 // and keep partial dgamma / dbeta in registers, written once to a (blocks x d) fp32 scratch that a second kernel folds.
 // Both also exist with one CTA per row, staged in shared memory (BMT_NORM_STAGED=1, and the combinations the others do not take).
 // (The reference calls F.layer_norm: example/layers/layernorm.py:29.)
+#include <math.h>
 #include <stdlib.h>
 
 #include "api.h"
@@ -384,7 +385,7 @@ int fwd(int64_t rows, int64_t d, const void* x, const void* w, const void* b, fl
 // are fetched for BWD_BATCH rows at a time: 124 us (LayerNorm 194 -> 171, bound by its arithmetic).  RMSNorm (RMS) has no bias
 // and drops the second accumulator.
 constexpr int BWD_STAGES = 8, BWD_BATCH = 32;
-__device__ int g_norm_status = 0;   // 1 after a bounded wait for a bulk copy ran out
+__device__ int g_norm_status = 0;   // 0, or (1 << 16) | blockIdx.x of the first CTA whose wait for a bulk copy ran out
 
 template <int WPR> struct BwdTeam {
     static constexpr int THREADS = WPR == 16 ? 512 : 256, CTAS = WPR == 16 ? 1 : 2, RPC = THREADS / 32 / WPR;
@@ -402,6 +403,7 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
     constexpr int RPC = BwdTeam<WPR>::RPC, WARPS = BwdTeam<WPR>::THREADS / 32;
     extern __shared__ __align__(128) uint8_t ring[];   // stages x {x, dy[, dres]} x RPC rows; 2 * d floats at the end of the kernel
     __shared__ __align__(8) uint64_t full[BWD_STAGES];
+    __shared__ int late[2];                            // by parity of the row: a thread's wait for its copy ran out
     __shared__ float ex[2][2][WARPS], mu[BWD_BATCH * RPC], rs[BWD_BATCH * RPC];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = warp % WPR, slot = warp / WPR;
@@ -423,6 +425,7 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
         bmt_tc::fence_barrier_init();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         for (int64_t it = 0; it < stages && it < n_it; ++it) refill(it);
+        late[0] = late[1] = 0;
     }
     float dg[VPL][8], db[RMS ? 1 : VPL][8];
     bmt::Vec16<T> wv[VPL];
@@ -436,6 +439,7 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
     __syncthreads();
     int st = 0;
     uint32_t phase = 0;
+    bool failed = false;                               // the same in all threads
     for (int64_t it = 0; it < n_it; ++it) {
         const int64_t r = (blockIdx.x + it * gridDim.x) * RPC + slot;
         const bool live = r < rows;
@@ -449,7 +453,7 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
             __syncthreads();
         }
         const float mean = mu[(it % BWD_BATCH) * RPC + slot], rstd = rs[(it % BWD_BATCH) * RPC + slot];
-        if (!bmt_tc::mbar_wait(&full[st], phase)) atomicExch(&g_norm_status, 1);
+        if (!bmt_tc::mbar_wait(&full[st], phase)) late[it & 1] = 1;   // bounded
         const T* xs = reinterpret_cast<const T*>(ring + st * stage_bytes) + slot * d;
         const T* gs = reinterpret_cast<const T*>(ring + st * stage_bytes + part_bytes) + slot * d;
         bmt::Vec16<T> xv[VPL], gv[VPL];
@@ -477,6 +481,8 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
         const int par = (int)(it & 1);
         if (WPR > 1 && lane == 0) { ex[par][0][warp] = s1; ex[par][1][warp] = s2; }
         __syncthreads();
+        failed = late[par] != 0;                       // not written again before all have passed the next row's barrier
+        if (failed) break;
         // every warp is through with the previous row: its stage takes the row `stages - 1` ahead of this one
         if (threadIdx.x == 0 && it > 0 && it - 1 + stages < n_it) refill(it - 1 + stages);
         if (WPR > 1) {
@@ -506,6 +512,18 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
             }
         }
         if (++st == stages) { st = 0; phase ^= 1; }
+    }
+    if (failed) {
+        // a copy did not arrive: report it, give those in flight time to land before the ring is used again, and let the column sums
+        // say that they are none
+        if (threadIdx.x == 0) atomicCAS(&g_norm_status, 0, (1 << 16) | (int)(blockIdx.x & 0xffff));
+        const uint64_t t0 = bmt_tc::global_ns();
+        while (bmt_tc::global_ns() - t0 < 2000000ull) __nanosleep(1000);
+        __syncthreads();
+#pragma unroll
+        for (int v = 0; v < VPL; ++v)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) { dg[v][k] = NAN; if (!RMS) db[v][k] = NAN; }
     }
     // combine the RPC row slots of this CTA (slot 0 ends up with the CTA's column sums); every copy into the ring has landed
     float* fold = reinterpret_cast<float*>(ring);
@@ -652,6 +670,14 @@ extern "C" int bmt_norm_bwd_ex(int64_t rows, int64_t d, const void* x, const voi
     cudaStream_t s = (cudaStream_t)stream;
     return dtype == BMT_DT_F16 ? bwd<__half>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, dw, db, s, dres, accumulate != 0)
                                : bwd<__nv_bfloat16>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, dw, db, s, dres, accumulate != 0);
+}
+
+// status of the norm backward: 0, or (1 << 16 | CTA) of the first CTA that gave up waiting for its rows; reading clears it
+extern "C" int bmt_norm_status(void) {
+    int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_norm_status, sizeof(int)) != cudaSuccess) return -1;
+    if (v != 0) cudaMemcpyToSymbol(g_norm_status, &zero, sizeof(int));
+    return v;
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -14,6 +14,7 @@ _UNIT = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2.
                                     (17, 2048), (1000, 2560), (2, 3072), (11, 4104), (600, 5120), (7, 6152), (149, 8192), (5, 8200),
                                     (3, 12288), (150, 12296), (4, 16384)])
 def test_norm_backward(bmt_gpu, dtype, rms, rows, d):
+    from bmtrain_b200.ops import _native
     from bmtrain_b200.ops import norm as N
 
     gen = torch.Generator(device="cuda").manual_seed(rows + d)
@@ -23,6 +24,7 @@ def test_norm_backward(bmt_gpu, dtype, rms, rows, d):
     leaves = [t.clone().requires_grad_() for t in ((x, w) if rms else (x, w, b))]
     y = N.rms_norm(*leaves, 1e-5) if rms else N.layer_norm(*leaves, 1e-5)
     got = torch.autograd.grad(y, leaves, dy)
+    assert _native.cuda_lib().bmt_norm_status() == 0
     exact = [t.double().requires_grad_() for t in ((x, w) if rms else (x, w, b))]
     if rms:
         ref = exact[0] * torch.rsqrt(exact[0].square().mean(-1, keepdim=True) + 1e-5) * exact[1]
