@@ -139,7 +139,8 @@ typedef struct {
     void* pre;       // (T, d_ff) pre-activation, GELU only (NULL for ReLU)
     // fused attention (csrc/attn_sm100.cu): non-NULL lse selects it; probs is then unused and may be NULL
     void* lse;       // (batch, heads, seq) fp32
-    void* mask_packed;  // with lse and a mask: buffer for the packed mask (bmt_attn_mask_layout bytes), filled by forward
+    void* mask_packed;  // with lse and a mask: buffer for the packed mask (bmt_attn_mask_layout bytes), filled by forward; one
+                        // without the other is refused (-40)
 } BmtGptBlock;
 
 typedef struct {

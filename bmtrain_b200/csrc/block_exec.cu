@@ -41,6 +41,9 @@ Dims dims_of(const BmtGptBlock& k) {
 const char* off(const void* p, int64_t elems) { return (const char*)p + elems * 2; }
 char* off(void* p, int64_t elems) { return (char*)p + elems * 2; }
 
+// The fused attention takes a dense mask in its packed form: one without room for the other would attend everywhere.
+bool mask_complete(const BmtGptBlock& k) { return !k.lse || (k.mask != nullptr) == (k.mask_packed != nullptr); }
+
 // Part 0 (by query), 1 (by key) or 2 (tile classes) of the packed mask of the fused attention, or null.
 const void* mask_part(const BmtGptBlock& k, const Dims& q, int part) {
     if (!k.mask_packed) return nullptr;
@@ -56,6 +59,7 @@ const void* mask_part(const BmtGptBlock& k, const Dims& q, int part) {
 // caller put its own QKV GEMM (fused with the parameter gather) or a stream wait between the steps.
 extern "C" int bmt_gpt_block_forward_steps(const BmtGptBlock* blk, int first_step, int last_step, void* stream) {
     const BmtGptBlock& k = *blk;
+    if (!mask_complete(k)) return -40;
     const Dims q = dims_of(k);
     const int dt = k.dtype;
 #define STEP(n) if (first_step <= (n) && (n) <= last_step)
@@ -127,6 +131,7 @@ extern "C" int bmt_gpt_block_forward(const BmtGptBlock* blk, void* stream) { ret
 extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockGrad* grad, void* stream) {
     const BmtGptBlock& k = *blk;
     const BmtGptBlockGrad& w = *grad;
+    if (!mask_complete(k)) return -40;
     const Dims q = dims_of(k);
     const int dt = k.dtype;
     const int64_t tok = 3 * q.hd, head = 3 * q.dh;
