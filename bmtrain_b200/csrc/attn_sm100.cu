@@ -619,12 +619,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                  const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdq, const AttnBwdParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    // swizzled tiles want 1024-byte alignment; there is no static shared memory in front of the block's own and no room to round up
-    uint8_t* smem = smem_raw;
-    if (smem_u32(smem_raw) & 1023u) {
-        if (threadIdx.x == 0) atomicCAS(&g_attn_status, 0, (0x7f << 16) | (int)(blockIdx.x & 0xffff));
-        return;
-    }
+    uint8_t* smem = smem_raw;         // swizzled tiles want 1024-byte alignment, there is no room to round up: launch_bwd looks after it
     constexpr int DC = HD / 64;
     constexpr uint32_t TB = DC * CHUNK;
     const uint32_t sK = smem_u32(smem), sV = sK + TB, sQ = sV + TB, sdO = sQ + 2 * TB, sdS = sdO + TB, sX = sdS + 2 * CHUNK;
@@ -1071,6 +1066,12 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     static_assert(5 * 2 * CHUNK + 2 * CHUNK + 8 * DQ_BUF + sizeof(BwdShared) <= 227 * 1024, "shared memory of a block");
     static bool configured = false;
     if (!configured) {
+        // what lies in front of the kernel's own shared memory: the system's share and static arrays
+        int dev = 0, reserved = 0;
+        cudaFuncAttributes attr;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaFuncGetAttributes(&attr, flash_bwd_kernel<HD, T>) != cudaSuccess ||
+            cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess) return -30;
+        if ((reserved + attr.sharedSizeBytes) % 1024 != 0) return -34;
         if (cudaFuncSetAttribute(flash_bwd_kernel<HD, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -30;
         configured = true;
     }
