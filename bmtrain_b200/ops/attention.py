@@ -67,9 +67,16 @@ def flash_usable(q, k, v) -> bool:
     return True
 
 
+def packed_mask_layout(b: int, sq: int, sk: int):
+    """Bytes of a packed mask, and where its parts by key and by tile start (the part by query starts at 0)."""
+    lib, by_key, classes = _native.cuda_lib(), ctypes.c_int64(), ctypes.c_int64()
+    lib.bmt_attn_mask_layout.restype = ctypes.c_int64
+    size = lib.bmt_attn_mask_layout(ctypes.c_int64(b), ctypes.c_int64(sq), ctypes.c_int64(sk), ctypes.byref(by_key), ctypes.byref(classes))
+    return size, by_key.value, classes.value
+
+
 def packed_mask_bytes(b: int, sq: int, sk: int) -> int:
-    qt, kt = (sq + 127) // 128, (sk + 127) // 128
-    return b * (16 * (sq * kt + sk * qt) + qt * kt)
+    return packed_mask_layout(b, sq, sk)[0]
 
 
 def packed_mask_buffer(b: int, sq: int, sk: int, device) -> torch.Tensor:
@@ -93,10 +100,9 @@ def _mask_parts(packed, b, sq, sk):
     """Pointers to the three parts of a packed mask (null without one)."""
     if packed is None:
         return (ctypes.c_void_p(0),) * 3
-    qt, kt = (sq + 127) // 128, (sk + 127) // 128
+    _, by_key, classes = packed_mask_layout(b, sq, sk)
     at = packed.data_ptr()
-    by_key = at + b * sq * kt * 16
-    return ctypes.c_void_p(at), ctypes.c_void_p(by_key), ctypes.c_void_p(by_key + b * sk * qt * 16)
+    return ctypes.c_void_p(at), ctypes.c_void_p(at + by_key), ctypes.c_void_p(at + classes)
 
 
 def flash_forward(q, k, v, scale, causal, mask8, lens32, packed=None):

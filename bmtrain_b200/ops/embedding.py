@@ -44,7 +44,8 @@ def embedding_backward(ids: torch.Tensor, grad: torch.Tensor, rows: int) -> torc
     lib = _native.cuda_lib()
     ids64, g2 = flat.to(torch.int64).contiguous(), g2.contiguous()
     out = torch.empty(rows, d, dtype=grad.dtype, device=grad.device)
-    words = 2 + 2 * rows + ids64.numel() // 64 + 1 + 2 * ids64.numel()     # bmt_embedding_bwd_scratch
+    lib.bmt_embedding_bwd_scratch.restype = ctypes.c_int64
+    words = lib.bmt_embedding_bwd_scratch(ctypes.c_int64(ids64.numel()), ctypes.c_int64(rows))
     scratch = torch.empty(words, dtype=torch.int32, device=grad.device)
     _native.check(lib.bmt_embedding_bwd(
         ctypes.c_int64(ids64.numel()), ctypes.c_int64(d), ctypes.c_int64(rows), _native.ptr(ids64), _native.ptr(g2),
