@@ -515,14 +515,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     if (warp == 9) tmem_dealloc(tmem, 512);
 }
 
-int sm_count() {
-    static int sms[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (sms[dev] == 0 && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
-    return sms[dev];
-}
-
 template <int HD, typename T>
 int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, AttnParams& p, int64_t batch, cudaStream_t stream) {
     constexpr uint32_t TB = (HD / 64) * CHUNK;
@@ -534,7 +526,7 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     }
     // pairs of query tiles unless single tiles still find an SM each: a pair shares its K / V loads and hides one tile's
     // softmax behind the other's MMAs, two SMs are faster still
-    p.per_cta = (int64_t)p.q_tiles * p.h * batch > sm_count() ? 2 : 1;
+    p.per_cta = (int64_t)p.q_tiles * p.h * batch > bmt::sm_count() ? 2 : 1;
     dim3 grid((unsigned)(p.h * batch), (unsigned)((p.q_tiles + p.per_cta - 1) / p.per_cta));
     flash_fwd_kernel<HD, T><<<grid, FWD_THREADS, smem, stream>>>(tq, tk, tv, p);
     bmt_count_launch(1);
@@ -1054,7 +1046,7 @@ int bwd_splits(int64_t batch, int64_t sk, int h, int hk) {
     const int group = h / hk;
     const int64_t ctas = (sk + TILE - 1) / TILE * hk * batch;
     for (int s = 1; s < group; ++s)
-        if (group % s == 0 && ctas * s >= 2 * 148) return s;
+        if (group % s == 0 && ctas * s >= 2 * bmt::sm_count()) return s;
     return group;
 }
 

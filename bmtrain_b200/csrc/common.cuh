@@ -63,6 +63,15 @@ template <bool IsMax> __device__ __forceinline__ float block_allreduce(float v, 
     return r;
 }
 
+// SMs of the current device (148 on a B200, also where there is none to ask).
+inline int sm_count() {
+    static int sms[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (sms[dev] == 0 && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+    return sms[dev];
+}
+
 __host__ __device__ __forceinline__ int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 }  // namespace bmt

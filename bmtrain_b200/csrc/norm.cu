@@ -580,7 +580,7 @@ int launch_bwd_stream(int64_t rows, int d, const void* x, const void* dy, const 
     size_t smem = stages * stage;
     if (Team::RPC > 1 && smem < (size_t)2 * d * sizeof(float)) smem = (size_t)2 * d * sizeof(float);
     int64_t grid = (rows + Team::RPC - 1) / Team::RPC;
-    if (grid > 148 * Team::CTAS) grid = 148 * Team::CTAS;
+    if (grid > (int64_t)bmt::sm_count() * Team::CTAS) grid = (int64_t)bmt::sm_count() * Team::CTAS;
     if (grid > nblk) grid = nblk;
     const auto run = [&](auto kernel) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget) != cudaSuccess) return -30;
