@@ -499,6 +499,8 @@ class Block(torch.nn.Module):
         (``_may_run_in_place``); where ``_Bucket.in_place`` allows it the partition itself will do.  Whoever else looks at
         the parameters or keeps them (state dicts, ``ZeroContext``) gets a copy."""
         for b in self._buckets.values():
+            if prefetch and b.comm.size == 1:
+                continue                     # nothing to wait for later
             if b.full is not None and getattr(b, "full_epoch", -1) == _param_epoch[0] and (in_place or not b.aliased):
                 continue
             # the optimizer may hold the flat partition or the parameters that are views of it
@@ -826,7 +828,7 @@ class Block(torch.nn.Module):
         self._ensure_gathered(args, in_place=in_place)
         nxt = self.next_module()
         if nxt is not None and nxt._mode != "PIPE":
-            nxt._begin_gather(prefetch=True, in_place=nxt._may_run_in_place())
+            nxt._begin_gather(prefetch=True)
 
     def _exit_forward(self) -> None:
         if self._mode == "PIPE" and self._micro_idx != config["micros"] - 1:
@@ -843,7 +845,7 @@ class Block(torch.nn.Module):
         self._prepare_grads(attach)
         pre = self.pre_module()
         if pre is not None and pre._mode != "PIPE" and pre._zero_level == 3:
-            pre._begin_gather(prefetch=True, in_place=pre._may_run_in_place())
+            pre._begin_gather(prefetch=True)
 
     def _exit_backward(self) -> None:
         if self._mode == "PIPE":

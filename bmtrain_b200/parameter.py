@@ -116,6 +116,8 @@ class DistributedParameter(torch.nn.Parameter):
 
 def gather_flat_shard(local: torch.Tensor, numel: int, comm: Communicator) -> torch.Tensor:
     """All-gather equal-capacity 1-D shards (the last ones may be short or empty) into ``numel`` elements."""
+    if comm.size == 1:
+        return local.clone(memory_format=torch.contiguous_format).view(-1)
     per = (numel + comm.size - 1) // comm.size
     if local.numel() != per:
         padded = torch.zeros(per, dtype=local.dtype, device=local.device)
@@ -147,13 +149,15 @@ class OpAllGather(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_output: torch.Tensor):
         comm: Communicator = ctx.comm
+        if comm.size == 1:
+            # a tensor of its own here too: autograd hands one tensor to several parameters, and each keeps what it gets
+            return grad_output.clone(memory_format=torch.contiguous_format).view(-1)
         per = (ctx.numel + comm.size - 1) // comm.size
         flat = grad_output.reshape(-1)
         if flat.numel() != per * comm.size:
             padded = torch.zeros(per * comm.size, dtype=flat.dtype, device=flat.device)
             padded[: flat.numel()].copy_(flat)
             flat = padded
-        # a tensor of its own on one rank too: autograd hands one tensor to several parameters, and each keeps what it gets
         out = torch.empty(per, dtype=flat.dtype, device=flat.device)
         comm.reduce_scatter_into(out, flat, "sum")
         start, end = ctx.bounds
