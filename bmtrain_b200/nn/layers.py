@@ -14,7 +14,38 @@ from ..layer import DistributedModule, reads_parameters_only
 from ..ops import embedding as _emb
 from ..ops import gemm as _gemm
 from ..ops import norm as _norm
-from ..parameter import DistributedParameter, ParameterInitializer
+from ..parameter import DistributedParameter, ParameterInitializer, await_update, private_value, shard_is_value
+
+
+class _ShardLookup(torch.autograd.Function):
+    """Lookup in a table whose shard is the whole table: the kernel has read it before anything behind the call can write to
+    it, backward does not need it, and its gradient is a fresh tensor.  So neither is copied."""
+
+    @staticmethod
+    def forward(ctx, ids, table):
+        await_update(table)
+        ctx.save_for_backward(ids)
+        ctx.rows = table._original_shape[0]
+        return _emb.embedding_forward(ids, table.data.reshape(table._original_shape))
+
+    @staticmethod
+    def backward(ctx, grad):
+        (ids,) = ctx.saved_tensors
+        return None, _emb.embedding_backward(ids, grad.contiguous(), ctx.rows).view(-1)
+
+
+class _ShardProjection(torch.autograd.Function):
+    """Multiplication by such a table: backward multiplies by the value of the forward pass, which is therefore a copy; the
+    table's gradient is a fresh tensor and is not copied."""
+
+    @staticmethod
+    def forward(ctx, x, table):
+        return _gemm.LinearFunction.forward(ctx, x, private_value(table), None)
+
+    @staticmethod
+    def backward(ctx, grad):
+        grad_x, grad_w, _ = _gemm.LinearFunction.backward(ctx, grad)
+        return grad_x, None if grad_w is None else grad_w.view(-1)
 
 
 @reads_parameters_only
@@ -30,6 +61,12 @@ class Embedding(DistributedModule):
             init_method=ParameterInitializer(torch.nn.init.normal_, mean=init_mean, std=init_std))
 
     def forward(self, input: torch.Tensor, projection: bool = False) -> torch.Tensor:
+        table = self._parameters.get("weight")
+        if type(self) is Embedding and isinstance(table, DistributedParameter) and shard_is_value(table):
+            if not projection:
+                return _ShardLookup.apply(input, table)
+            if input.is_cuda or input.dtype != torch.float32:
+                return _ShardProjection.apply(input, table)
         if projection:
             return _gemm.linear(input, self.weight)
         return _emb.embedding(input, self.weight)

@@ -129,6 +129,25 @@ def gather_flat_shard(local: torch.Tensor, numel: int, comm: Communicator) -> to
     return out[:numel]
 
 
+def await_update(param: "DistributedParameter") -> None:
+    """Wait until an asynchronous optimizer step is through with the shard of ``param``."""
+    hook = getattr(param, "_bmt_pending_update", None)
+    if hook is not None:
+        hook(True)
+
+
+def private_value(param: "DistributedParameter") -> torch.Tensor:
+    """Full value of a stand-alone parameter in memory of its own, without autograd."""
+    await_update(param)
+    return gather_flat_shard(param.data, param._original_shape.numel(), param._zero_comm).view(param._original_shape)
+
+
+def shard_is_value(param: "DistributedParameter") -> bool:
+    """Whether the shard of ``param`` is its whole value and stays as it is until kernels on the current stream have read it:
+    stand-alone, one rank, no optimizer that uploads new values on a stream of its own."""
+    return not param._in_block and param._zero_comm.size == 1 and getattr(param, "_bmt_grad_hook", None) is None
+
+
 class OpAllGather(torch.autograd.Function):
     """Full value of a stand-alone sharded parameter; backward reduce-scatters the gradient onto the shards."""
 
@@ -138,13 +157,9 @@ class OpAllGather(torch.autograd.Function):
         ctx.comm = value._zero_comm
         ctx.numel = value._original_shape.numel()
         ctx.bounds = (value._start_partition, value._end_partition)
-        hook = getattr(value, "_bmt_pending_update", None)
-        if hook is not None:
-            hook(True)   # an asynchronous optimizer step is still rewriting this shard
         # a copy on one rank too: the caller may write to what it reads here, and backward uses the value of the forward pass
         # although the shard may have been updated in between
-        full = gather_flat_shard(value.data, ctx.numel, ctx.comm)
-        return full.view(value._original_shape)
+        return private_value(value)
 
     @staticmethod
     def backward(ctx, grad_output: torch.Tensor):

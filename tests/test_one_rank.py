@@ -187,3 +187,76 @@ def test_zero_2_keeps_the_parameters_of_the_forward_pass(bmt):
         return a.grad
 
     assert torch.equal(grad(0.0), grad(0.5))
+
+
+def _check_tables(bmt, dev, projection):
+    """Lookup and projection of a stand-alone table: gradients of a table used twice, of two tables, with hooks, accumulated over
+    passes; an update between the two passes; results that share no memory with the table."""
+    torch.manual_seed(5)
+    dtype = torch.bfloat16 if projection or dev == "cuda" else torch.float32      # fp32 projections on the CPU go through torch
+    a, b = (bmt.nn.Embedding(12, 8, dtype=dtype) for _ in range(2))
+    bmt.init_parameters(a)
+    bmt.init_parameters(b)
+    pa, pb = a._parameters["weight"], b._parameters["weight"]
+    x = torch.randn(5, 8).to(dtype).to(dev).requires_grad_() if projection else torch.tensor([3, 3, 0, 11, 7], device=dev)
+    seen = []
+    pa.register_hook(lambda g: seen.append(g))
+
+    def loss():
+        return (a(x, projection=projection) * 2 + a(x, projection=projection) + b(x, projection=projection)).float().sum()
+
+    def want():
+        wa, wb = (p.detach().clone().view(12, 8).float().requires_grad_() for p in (pa, pb))
+        xs = x.detach().float().requires_grad_() if projection else x
+        f = lambda w: xs @ w.t() if projection else w[xs]  # noqa: E731
+        (f(wa) * 3 + f(wb)).sum().backward()
+        return wa.grad.reshape(-1), wb.grad.reshape(-1), xs.grad
+
+    ga, gb, gx = want()
+    value = loss()
+    for p in (pa, pb):
+        p.data.add_(1)                                           # an update between the two passes
+    value.backward()
+    for p in (pa, pb):
+        p.data.sub_(1)
+    # bf16: three results of magnitude up to 20 are rounded and added
+    tol = dict(rtol=2e-2, atol=2e-1) if dtype == torch.bfloat16 else dict(rtol=1e-6, atol=1e-6)
+    assert torch.allclose(pa.grad.float(), ga, **tol) and torch.allclose(pb.grad.float(), gb, **tol)
+    if projection:
+        assert torch.allclose(x.grad.float(), gx, **tol)
+    assert len(seen) == 1 and pa.grad.data_ptr() != pb.grad.data_ptr()
+    kept = seen[0].clone()
+    once = pb.grad.clone()
+    loss().backward()
+    assert torch.allclose(pb.grad.float(), 2 * once.float(), **tol)
+    assert torch.equal(seen[0], kept)                            # what a hook kept is not added to
+    before = pa.detach().clone()
+    with torch.no_grad():
+        a(x, projection=projection).zero_()
+    assert torch.equal(pa.detach(), before)
+
+
+@pytest.mark.parametrize("projection", [False, True])
+def test_tables_are_used_in_place_without_showing(bmt, projection):
+    _check_tables(bmt, "cpu", projection)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("projection", [False, True])
+def test_tables_are_used_in_place_without_showing_gpu(bmt_gpu, projection):
+    _check_tables(bmt_gpu, "cuda", projection)
+
+
+def test_a_table_with_a_weight_of_its_own_making(bmt):
+    class Scaled(bmt.nn.Embedding):
+        @property
+        def weight(self):
+            return self.__getattr__("weight") * 3
+
+    e = Scaled.__new__(Scaled)
+    torch.nn.Module.__init__(e)
+    e.num_embeddings, e.embedding_dim = 4, 8
+    e.register_parameter("weight_", None)
+    e._parameters["weight"] = bmt.DistributedParameter(torch.randn(4, 8))
+    ids = torch.tensor([1, 2])
+    assert torch.allclose(e(ids), 3 * e._parameters["weight"].gather()[ids])
