@@ -140,23 +140,25 @@ class _Slot:
     During the backward pass of the block it is also the place a kernel may write the parameter's gradient to
     (``ops/grad_slot.py``): ``written`` tells whether the slot of the full gradient buffer holds a gradient yet."""
 
-    __slots__ = ("name", "param", "offset", "numel", "shape", "lo", "hi", "bucket", "written")
+    __slots__ = ("name", "param", "offset", "numel", "shape", "lo", "hi", "bucket", "written", "__weakref__")
 
     def __init__(self, name, param, offset, numel, shape):
         self.name, self.param, self.offset, self.numel, self.shape = name, param, offset, numel, shape
         self.lo = self.hi = 0  # overlap with the local partition, in bucket coordinates
-        self.bucket = None
+        self.bucket = None     # weak, as is the parameter's reference to its slot: a dropped block is freed at once
         self.written = False
 
     @property
     def open(self) -> bool:
-        return self.bucket.grads_open and self.bucket.full_grad is not None
+        b = self.bucket()
+        return b is not None and b.grads_open and b.full_grad is not None
 
     def grad_ptr(self) -> int:
-        return self.bucket.full_grad_ptr + self.offset * self.bucket.full_grad.element_size()
+        b = self.bucket()
+        return b.full_grad_ptr + self.offset * b.full_grad.element_size()
 
     def grad_view(self) -> torch.Tensor:
-        return self.bucket.full_grad[self.offset:self.offset + self.numel].view(self.shape)
+        return self.bucket().full_grad[self.offset:self.offset + self.numel].view(self.shape)
 
 
 class _Bucket:
@@ -439,8 +441,8 @@ class Block(torch.nn.Module):
             offset = round_up(b.total, align)
             numel = param._original_shape.numel()
             slot = _Slot(name, param, offset, numel, param._original_shape)
-            slot.bucket = b
-            param._bmt_grad_slot = slot
+            slot.bucket = weakref.ref(b)
+            param._bmt_grad_slot = weakref.ref(slot)
             b.slots.append(slot)
             b.total = offset + numel
         dev = config["device"]

@@ -260,3 +260,22 @@ def test_a_table_with_a_weight_of_its_own_making(bmt):
     e._parameters["weight"] = bmt.DistributedParameter(torch.randn(4, 8))
     ids = torch.tensor([1, 2])
     assert torch.allclose(e(ids), 3 * e._parameters["weight"].gather()[ids])
+
+
+def test_a_dropped_block_is_freed_at_once(bmt):
+    """No reference cycle keeps the partition or the gradients of a block until the next garbage collection."""
+    import gc
+    import weakref
+
+    blk = _gpt_block(bmt)
+    blk(torch.randn(2, 4, 16, requires_grad=True)).sum().backward()
+    bmt.synchronize()
+    gc.collect()
+    gc.disable()
+    try:
+        refs = [weakref.ref(b.storage) for b in blk._buckets.values()] + [weakref.ref(b.storage.grad) for b in blk._buckets.values()]
+        refs += [weakref.ref(p) for p in blk._module.parameters()] + [weakref.ref(blk._module)]
+        del blk
+        assert all(r() is None for r in refs)
+    finally:
+        gc.enable()
