@@ -1051,6 +1051,22 @@ EncodeTiledFn get_encode() {
     return fn;
 }
 
+// Makes the primary context current on this thread (autograd worker threads may not have one yet).  cudaFree does that, but
+// it invalidates a stream capture, so it is called only where there is none.
+void bind_context() {
+    typedef CUresult (*GetCurrentFn)(CUcontext*);
+    static GetCurrentFn fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = (GetCurrentFn)p;
+    });
+    CUcontext ctx = nullptr;
+    if (!fn || fn(&ctx) != CUDA_SUCCESS || !ctx) cudaFree(0);
+}
+
 struct MapKey {
     const void* ptr;
     int64_t d[4], s[3];
@@ -1091,7 +1107,7 @@ int make_map(CUtensorMap* out, const void* ptr, int dtype, int64_t inner, int64_
     if (st[2] == 0) st[2] = 16;
     cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
     cuuint32_t es[4] = {1, 1, 1, 1};
-    cudaFree(0);  // binds the primary context to this thread (autograd worker threads may not have one current yet)
+    bind_context();
     CUresult r = enc(out, dtype == BMT_DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)ptr,
                      dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1123,7 +1139,7 @@ int bmt_tma_map_f32_3d(CUtensorMap* out, const void* ptr, int64_t inner, int64_t
     cuuint64_t st[2] = {(cuuint64_t)inner * 4, (cuuint64_t)(inner * rows) * 4};
     cuuint32_t box[3] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1};
     cuuint32_t es[3] = {1, 1, 1};
-    cudaFree(0);  // see make_map
+    bind_context();
     const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)ptr, dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : -12;
@@ -1157,7 +1173,7 @@ int make_map_mn5(CUtensorMap* out, const void* ptr, int dtype, int64_t mn, int64
     if (st[3] == 0) st[3] = 16;
     cuuint32_t box[5] = {64, (cuuint32_t)box_rows, (cuuint32_t)chunks, 1, 1};
     cuuint32_t es[5] = {1, 1, 1, 1, 1};
-    cudaFree(0);
+    bind_context();
     CUresult r = enc(out, dtype == BMT_DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, (void*)ptr,
                      dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

@@ -68,3 +68,39 @@ def test_tiles(bmt_gpu, dtype, cfg):
     for name, a, w in zip(("o", "dq", "dk", "dv"), got, want):
         assert torch.isfinite(a).all(), name
         assert (a.double() - w).norm() <= tol * w.norm() + 1e-6, (name, float((a.double() - w).norm() / w.norm()))
+
+
+@pytest.mark.parametrize("hk,masking", [(8, None), (2, None), (8, "mask"), (8, "lens")])
+def test_forward_and_backward_under_capture(bmt_gpu, hk, masking):
+    """Both directions are captured into a graph on addresses that they have not seen, and replay on new inputs."""
+    from bmtrain_b200.ops import attention as AT
+
+    gen = torch.Generator(device="cuda").manual_seed(hk)
+    fresh = lambda h: torch.randn(2, 200, h, 64, generator=gen, device="cuda").half()  # noqa: E731
+    q, k, v, do = (fresh(h) for h in (8, hk, hk, 8))
+    mask = torch.rand(2, 200, 200, generator=gen, device="cuda") > 0.3 if masking == "mask" else None
+    lens = torch.tensor([77, 200], device="cuda") if masking == "lens" else None
+    for t in (q, k, v):
+        t.requires_grad_()
+
+    def run():
+        o = AT.attention(q, k, v, mask=mask, kv_lens=lens)
+        return [o.detach(), *torch.autograd.grad(o, (q, k, v), do)]
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        got = run()
+    with torch.no_grad():
+        for t in (q, k, v, do):
+            t.copy_(fresh(t.shape[2]))
+    graph.replay()
+    torch.cuda.synchronize()
+    got = [t.clone() for t in got]
+    for a, b in zip(got, run()):
+        # dQ is added up in another order
+        assert (a - b).float().norm() <= 1e-3 * b.float().norm()
