@@ -188,23 +188,43 @@ __global__ void __launch_bounds__(256) ce_row_stats_stream_kernel(int64_t m, int
 }
 
 // The reduced loss from the row statistics (3 x m: maximum, sum, target logit): lse of every row, the loss (sum over the rows
-// whose target counts, divided by their number when `mean`) and that divisor.  One block, fixed order: a
-// few microseconds in the place of the dozen elementwise launches that cost the host more than the device.
+// whose target counts, divided by their number when `mean`) and that divisor.  One block up to CE_FINISH_ROWS rows, in the
+// place of the dozen elementwise launches that cost the host more than the device.  It takes a fifth of a microsecond per 1024
+// rows; above, every block leaves the sum of its rows and their number in the place of its first row's maximum and target
+// logit, and a second launch adds them up.  The order is fixed either way.
 constexpr int CE_FINISH_THREADS = 1024;
-__global__ void __launch_bounds__(CE_FINISH_THREADS) ce_finish_kernel(int64_t m, const float* __restrict__ rows, const int64_t* __restrict__ target,
-                                                                      int64_t ignore_index, int mean, float* __restrict__ lse,
-                                                                      float* __restrict__ loss, float* __restrict__ divisor) {
+constexpr int64_t CE_FINISH_ROWS = 8192;
+__device__ __forceinline__ void ce_result(float sum, float count, int mean, float* loss, float* divisor) {
+    *loss = mean ? sum / count : sum;
+    *divisor = mean ? count : 1.f;
+}
+__global__ void __launch_bounds__(CE_FINISH_THREADS) ce_finish_kernel(int64_t m, int64_t chunk, float* __restrict__ rows,
+                                                                      const int64_t* __restrict__ target, int64_t ignore_index, int mean,
+                                                                      float* __restrict__ lse, float* __restrict__ loss,
+                                                                      float* __restrict__ divisor) {
     __shared__ float scratch[33];
+    const int64_t first = blockIdx.x * chunk, end = first + chunk < m ? first + chunk : m;
     float sum = 0.f, count = 0.f;
 #pragma unroll 4
-    for (int64_t i = threadIdx.x; i < m; i += CE_FINISH_THREADS) {
+    for (int64_t i = first + threadIdx.x; i < end; i += CE_FINISH_THREADS) {
         const float l = rows[i] + logf(rows[m + i] + 1e-10f);
         lse[i] = l;
         if (target[i] != ignore_index) { sum += l - rows[2 * m + i]; count += 1.f; }
     }
+    sum = bmt::block_allreduce<false>(sum, scratch);       // (barriers inside: all maxima of the block have been read)
+    count = bmt::block_allreduce<false>(count, scratch);
+    if (threadIdx.x != 0) return;
+    if (gridDim.x == 1) ce_result(sum, count, mean, loss, divisor);
+    else { rows[first] = sum; rows[2 * m + first] = count; }
+}
+__global__ void __launch_bounds__(256) ce_total_kernel(int64_t m, int blocks, int64_t chunk, const float* __restrict__ rows,
+                                                       int mean, float* __restrict__ loss, float* __restrict__ divisor) {
+    __shared__ float scratch[33];
+    float sum = 0.f, count = 0.f;
+    for (int b = threadIdx.x; b < blocks; b += 256) { sum += rows[b * chunk]; count += rows[2 * m + b * chunk]; }
     sum = bmt::block_allreduce<false>(sum, scratch);
     count = bmt::block_allreduce<false>(count, scratch);
-    if (threadIdx.x == 0) { *loss = mean ? sum / count : sum; *divisor = mean ? count : 1.f; }
+    if (threadIdx.x == 0) ce_result(sum, count, mean, loss, divisor);
 }
 
 // `divisor` null: grad holds one value per row; else one value for all rows, to be divided by *divisor.
@@ -323,9 +343,13 @@ extern "C" int bmt_ce_reduced_forward(int64_t m, int64_t n, const void* logits, 
                                       int mean, void* scratch, void* lse, void* loss, void* divisor, void* stream) {
     const int rc = bmt_ce_row_stats(m, n, logits, dtype, target, 0, scratch, stream);
     if (rc != 0) return rc;
-    ce_finish_kernel<<<1, CE_FINISH_THREADS, 0, (cudaStream_t)stream>>>(m, (const float*)scratch, (const int64_t*)target, ignore_index, mean,
-                                                                        (float*)lse, (float*)loss, (float*)divisor);
-    bmt_count_launch(1);
+    const int64_t share = (m + bmt::sm_count() - 1) / bmt::sm_count();     // a block per SM, of at least 1024 rows
+    const int64_t chunk = m <= CE_FINISH_ROWS ? CE_FINISH_ROWS : share > 1024 ? share : 1024;
+    const int64_t blocks = m <= CE_FINISH_ROWS ? 1 : (m + chunk - 1) / chunk;
+    ce_finish_kernel<<<(unsigned)blocks, CE_FINISH_THREADS, 0, (cudaStream_t)stream>>>(m, chunk, (float*)scratch, (const int64_t*)target, ignore_index, mean,
+                                                                                       (float*)lse, (float*)loss, (float*)divisor);
+    if (blocks > 1) ce_total_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(m, (int)blocks, chunk, (const float*)scratch, mean, (float*)loss, (float*)divisor);
+    bmt_count_launch(blocks > 1 ? 2 : 1);
     return (int)cudaGetLastError();
 }
 

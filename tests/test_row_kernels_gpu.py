@@ -37,7 +37,8 @@ def test_norm_backward(bmt_gpu, dtype, rms, rows, d):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("rows,classes", [(1, 8), (3, 1000), (1023, 33), (1025, 2048), (130, 32003), (2049, 4096)])
+@pytest.mark.parametrize("rows,classes", [(1, 8), (3, 1000), (1023, 33), (1025, 2048), (130, 32003), (2049, 4096), (8192, 16), (8193, 16),
+                                          (9217, 9), (151553, 8), (200000, 24)])       # from 8193 rows on several blocks
 @pytest.mark.parametrize("reduction", ["mean", "sum"])
 def test_reduced_cross_entropy(bmt_gpu, dtype, rows, classes, reduction):
     gen = torch.Generator(device="cuda").manual_seed(rows + classes)
