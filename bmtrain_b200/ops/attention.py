@@ -18,6 +18,7 @@ saved log-sum-exp and accumulates dK / dV in tensor memory.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 from typing import Optional
 
@@ -67,6 +68,7 @@ def flash_usable(q, k, v) -> bool:
     return True
 
 
+@functools.lru_cache(maxsize=256)
 def packed_mask_layout(b: int, sq: int, sk: int):
     """Bytes of a packed mask, and where its parts by key and by tile start (the part by query starts at 0)."""
     lib, by_key, classes = _native.cuda_lib(), ctypes.c_int64(), ctypes.c_int64()
