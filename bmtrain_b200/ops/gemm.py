@@ -183,7 +183,7 @@ class LinearFunction(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             grad_x = gemm_nn(g2, weight).view(x.shape)
         if ctx.needs_input_grad[1]:
-            slot = _grad_slot.find(weight) if weight.is_cuda and weight.dtype == g2.dtype else None
+            slot = _grad_slot.find(weight) if weight.dtype == g2.dtype else None
             if slot is None:
                 grad_w = gemm_tn(g2, x2)
             else:
