@@ -18,6 +18,10 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
+// Logits are multiplied by log2(e) before the exponent is taken.  The lowest finite numbers of fp32 and bf16, which classes
+// are hidden with, overflow in that product: as a reference it is kept finite, so that they count for nothing beside others.
+constexpr float LOWEST = -3.402823466e38f;
+
 // Elements of a row before its first 16-byte boundary.
 template <typename T> __device__ __forceinline__ int64_t row_head(const T* row, int64_t n) {
     const int64_t h = ((16 - ((uintptr_t)row & 15)) & 15) / sizeof(T);
@@ -47,7 +51,7 @@ __global__ void __launch_bounds__(256) ce_row_stats_kernel(int64_t m, int64_t n,
     const T* __restrict__ xv = xr + head;
     const auto move_to = [&](float v) {
         if (!(v > mx)) return;
-        const float r = v * L2E;
+        const float r = fmaxf(v * L2E, LOWEST);
         if (mx != -INFINITY) se *= ex2(ref - r);
         mx = v;
         ref = r;
@@ -147,7 +151,7 @@ __global__ void __launch_bounds__(256) ce_row_stats_stream_kernel(int64_t m, int
         for (int u = 0; u < U; ++u)
             if (base + u * 256 < nv) lm = fmaxf(lm, packet_max(v[u]));
         if (lm > mx) { se *= ex2((mx - lm) * L2E); mx = lm; }   // mx = -inf: se is 0 and stays 0 (0 * 2^-inf)
-        const float off = mx == -INFINITY ? 0.f : -mx * L2E;
+        const float off = mx == -INFINITY ? 0.f : -fmaxf(mx * L2E, LOWEST);
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (base + u * 256 < nv) {
@@ -245,8 +249,9 @@ __global__ void __launch_bounds__(256) ce_backward_kernel(int64_t m, int64_t n, 
     constexpr float L2E = 1.4426950408889634f;
     // p = 2^(x * log2e + off) * 2^rest: `off` is -l * log2e as it is rounded, which near p = 1 is not exact enough, `rest` what
     // the rounding dropped (exact); the second factor goes into the multiplication by g
-    const float off = -l * L2E, rest = fmaf(-l, L2E, -off);
-    const float pg = fabsf(l) < INFINITY ? g * ex2(rest) : g;
+    const bool huge = fabsf(l) > 1e38f;
+    const float off = huge && l > -INFINITY ? fminf(-l * L2E, -LOWEST) : -l * L2E, rest = huge ? 0.f : fmaf(-l, L2E, -off);
+    const float pg = g * ex2(rest);
     // as in the forward kernel; vectors need the logits and the gradient to be off the 16-byte boundary by the same amount
     const bool same = (((uintptr_t)xr ^ (uintptr_t)orow) & 15) == 0;
     const int64_t head = same ? row_head<T>(xr, n) : n, nv = (n - head) / V, tail = head + nv * V;

@@ -90,12 +90,13 @@ def test_embedding_gradient(bmt_gpu, dtype, tokens, rows, d):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("classes", [33, 1000, 2047, 4096, 12289, 12296])       # odd and even, scalar, vector and streaming rows
-def test_cross_entropy_of_hidden_classes(bmt_gpu, dtype, classes):
-    """Classes hidden with -inf: the first ones, the last ones, all but one, a thread's whole first trip, everything a thread
+@pytest.mark.parametrize("hide", ["inf", "lowest"])
+def test_cross_entropy_of_hidden_classes(bmt_gpu, dtype, classes, hide):
+    """Classes hidden with -inf or with the lowest number of the type: the first ones, the last ones, all but one, a thread's whole first trip, everything a thread
     sees; and rows with a NaN, which must not come out finite."""
     gen = torch.Generator(device="cuda").manual_seed(classes)
     x = torch.randn(8, classes, generator=gen, device="cuda").to(dtype)
-    inf = float("inf")
+    inf = float("inf") if hide == "inf" else torch.finfo(dtype).max
     x[0, :9] = -inf
     x[1, -9:] = -inf
     x[2, :] = -inf
