@@ -166,6 +166,8 @@ def _check_known(bmt, dev, dtype, kind, tol):
         blk.load_state_dict({k: v.to(dev) for k, v in state.items()})
     list(blocks[1].parameters())[0].register_hook(lambda g: seen.append(g.shape))
     x, g = torch.randn(2, 24, 64).to(dtype).to(dev), torch.randn(2, 24, 64).to(dtype).to(dev)
+    with torch.no_grad():
+        assert torch.equal(blocks[0](x), blocks[1](x))
     grads = []
     for blk in blocks:
         for _ in range(2):                                       # the second pass accumulates
