@@ -20,9 +20,9 @@ def watched(param: torch.Tensor) -> bool:
 
 def find(param: Optional[torch.Tensor]):
     """The slot a kernel may write the gradient of ``param`` to, or None: not a parameter of a block whose backward pass
-    of known code is running, not trained, or watched by hooks."""
+    of known code is running (which includes that nothing watches its parameters), or not trained."""
     ref = getattr(param, "_bmt_grad_slot", None)
     slot = None if ref is None else ref()
     if slot is None or slot.param is not param or not slot.open or not param.requires_grad:
         return None
-    return None if watched(param) else slot
+    return slot
