@@ -243,9 +243,18 @@ __global__ void __launch_bounds__(256) ce_backward_kernel(int64_t m, int64_t n, 
     const int64_t tg = target[row];
     const bool ignored = tg == ignore_index;
     const int64_t t = tg - vocab_start;
-    const float l = lse[row];
-    const float g = ignored ? 0.f : divisor ? grad[0] / divisor[0] : grad[row];
     constexpr int V = bmt::Vec16<T>::N;
+    if (ignored) {       // zeros whatever the logits are: 0 * NaN is none
+        const int64_t head = row_head<T>(orow, n), nv = (n - head) / V, tail = head + nv * V;
+        bmt::Vec16<T> zero;
+#pragma unroll
+        for (int k = 0; k < V; ++k) zero.v[k] = bmt::Cvt<T>::from_f(0.f);
+        for (int64_t i = threadIdx.x; i < head + n - tail; i += blockDim.x) orow[i < head ? i : tail + i - head] = zero.v[0];
+        for (int64_t i = threadIdx.x; i < nv; i += blockDim.x) bmt::st16(orow + head + i * V, zero);
+        return;
+    }
+    const float l = lse[row];
+    const float g = divisor ? grad[0] / divisor[0] : grad[row];
     constexpr float L2E = 1.4426950408889634f;
     // p = 2^(x * log2e + off) * 2^rest: `off` is -l * log2e as it is rounded, which near p = 1 is not exact enough, `rest` what
     // the rounding dropped (exact); the second factor goes into the multiplication by g

@@ -279,3 +279,24 @@ def test_a_dropped_block_is_freed_at_once(bmt):
         assert all(r() is None for r in refs)
     finally:
         gc.enable()
+
+
+def test_hook_functions_attach_gradient_buffers(bmt):
+    """The four moments for code that brackets a block by hand: full-size parameters and gradients are in place in between."""
+    from bmtrain_b200 import hook_func
+
+    blk = _gpt_block(bmt)
+    before = _partitions(blk)
+    hook_func.zero_pre_forward(blk, ())
+    for p in blk._module.parameters():
+        p.data.mul_(2)                                           # on a copy
+    hook_func.zero_post_forward(blk, None, None)
+    hook_func.zero_pre_backward(blk, None)
+    for s in blk._slots:
+        assert s.param.shape == s.shape and s.param.grad.shape == s.shape and not s.param.grad.any()
+        s.param.grad.add_(1)
+    hook_func.zero_post_backward(blk, None, None)
+    bmt.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(before, _partitions(blk)))
+    for p in blk.parameters():
+        assert torch.equal(p.grad, torch.ones_like(p.grad))

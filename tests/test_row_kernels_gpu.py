@@ -145,3 +145,18 @@ def test_cross_entropy_is_exact_near_the_target(bmt_gpu, classes, level):
     exact = (x.double() - top[:, None]).exp().sum(1)
     assert torch.equal(mx.double(), top)
     assert (se.double() - exact).abs().le((16 + classes / 256 + 8) * unit * exact).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("classes", [7, 100, 1001, 4096])
+@pytest.mark.parametrize("reduction", ["mean", "none"])
+def test_ignored_rows_get_no_gradient(bmt_gpu, dtype, classes, reduction):
+    """... whatever their logits are."""
+    x = torch.randn(5, classes, device="cuda").to(dtype)
+    x[1, 3], x[2, classes - 1], x[3] = float("nan"), float("inf"), float("-inf")
+    t = torch.tensor([0, -100, -100, -100, classes - 1], device="cuda")
+    x = x.requires_grad_()
+    loss = bmt_gpu.loss.FusedCrossEntropy(ignore_index=-100, reduction=reduction)(x, t)
+    (g,) = torch.autograd.grad(loss, (x,), torch.ones_like(loss))
+    assert torch.equal(g[1:4], torch.zeros_like(g[1:4]))
+    assert torch.isfinite(g).all() and g[0].any() and g[4].any()
