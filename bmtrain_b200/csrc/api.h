@@ -98,16 +98,21 @@ typedef struct {
     int ab_dtype;
     const void* residual; int64_t ldr;                                // + residual (m x n, operand dtype)
     const void* aux; int64_t ld_aux; int aux_mode;                    // 1: *= (aux > 0), 2: *= gelu'(aux)
+    void* scratch; int64_t scratch_bytes;                             // optional: bmt_gemm_scratch_bytes(), the start of it zeros
 } BmtGemmDesc;
 // Fused GEMM + collective kernels launched from now on leave `n` SMs (even, at most 64) out of their grids, so that a kernel
 // of another parallel dimension can start while their CTAs wait for other ranks; 0 restores full grids.
 int bmt_gemm_reserve_sms(int n);
 int bmt_gemm_ex(const BmtGemmDesc* desc, void* stream);
+// Scratch with which a GEMM may divide tiles over several CTAs: bytes of it, zeroed once; kernels that use it at the same time need
+// one each (a stream's launches take turns).
+int64_t bmt_gemm_scratch_bytes(void);
+int bmt_gemm_plan(int64_t m, int64_t n, int64_t k, int b_major, int worker, int64_t* plan6, int* items5, int most);
 
 // C[M,N] (+)= alpha * op(A) op(B) (+ bias) with optional activation; majors: 0 = reduction dim contiguous, 1 = output dim contiguous.
 int bmt_gemm(int64_t m, int64_t n, int64_t k, const void* a, int64_t lda, int a_major, const void* b, int64_t ldb,
              int b_major, void* c, int64_t ldc, int c_dtype, const void* bias, int act, int accumulate, int ab_dtype,
-             void* stream);
+             void* scratch, int64_t scratch_bytes, void* stream);
 int bmt_gemm_batched(int64_t m, int64_t n, int64_t k, const void* a, int64_t lda, int a_major, int64_t a_bs0, int64_t a_bs1,
                      const void* b, int64_t ldb, int b_major, int64_t b_bs0, int64_t b_bs1, void* c, int64_t ldc,
                      int c_dtype, int64_t c_bs0, int64_t c_bs1, int64_t batch_inner, int64_t batch_outer,
@@ -141,6 +146,9 @@ typedef struct {
     void* lse;       // (batch, heads, seq) fp32
     void* mask_packed;  // with lse and a mask: buffer for the packed mask (bmt_attn_mask_layout bytes), filled by forward; one
                         // without the other is refused (-40)
+    // work space of bmt_colsum_ex and of the GEMMs (BmtGemmDesc.scratch), both optional and zeroed once
+    void* colsum_scratch; int64_t colsum_scratch_bytes;
+    void* gemm_scratch; int64_t gemm_scratch_bytes;
 } BmtGptBlock;
 
 typedef struct {
@@ -161,8 +169,6 @@ typedef struct {
     void* dq_acc;
     void* delta;
     int acc_small;            // bias and norm gradients are added to what d_*_b / d_ln*_w already hold
-    void* colsum_scratch;     // optional work space of bmt_colsum_ex (zero-initialised once), colsum_scratch_bytes large
-    int64_t colsum_scratch_bytes;
 } BmtGptBlockGrad;
 
 int bmt_gpt_block_forward(const BmtGptBlock* blk, void* stream);

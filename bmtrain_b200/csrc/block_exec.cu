@@ -27,6 +27,11 @@ BmtGemmDesc plain(int64_t m, int64_t n, int64_t k, const void* a, int64_t lda, i
     return g;
 }
 
+int gemm(const BmtGptBlock& k, BmtGemmDesc& g, void* stream) {
+    g.scratch = k.gemm_scratch; g.scratch_bytes = k.gemm_scratch_bytes;
+    return bmt_gemm_ex(&g, stream);
+}
+
 struct Dims {
     int64_t T, d, h, dh, hd, dff, s, b, es;  // es = element size
 };
@@ -69,7 +74,7 @@ extern "C" int bmt_gpt_block_forward_steps(const BmtGptBlock* blk, int first_ste
     STEP(2) {
         BmtGemmDesc g = plain(q.T, 3 * q.hd, q.d, k.ln1, q.d, 0, k.qkv_w, q.d, 0, k.qkv, 3 * q.hd, dt);
         g.bias = k.qkv_b;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     const int64_t tok = 3 * q.hd, head = 3 * q.dh;
     // 3-5 as one fused attention kernel: q, k, v are strided views of the packed projection, nothing of size s x s is stored
@@ -88,7 +93,7 @@ extern "C" int bmt_gpt_block_forward_steps(const BmtGptBlock* blk, int first_ste
         g.a_bs0 = head; g.a_bs1 = q.s * tok; g.b_bs0 = head; g.b_bs1 = q.s * tok;
         g.c_bs0 = q.s * k.probs_ld; g.c_bs1 = q.h * q.s * k.probs_ld;
         g.batch_inner = q.h; g.batch_outer = q.b; g.alpha = 1.f / sqrtf((float)q.dh);
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     // 4. masked softmax in place
     STEP(4) RUN(bmt_masked_softmax(q.b, q.h, q.s, q.s, k.probs_ld, k.probs, dt, k.causal, k.mask, nullptr, stream));
@@ -98,14 +103,14 @@ extern "C" int bmt_gpt_block_forward_steps(const BmtGptBlock* blk, int first_ste
         g.a_bs0 = q.s * k.probs_ld; g.a_bs1 = q.h * q.s * k.probs_ld; g.b_bs0 = head; g.b_bs1 = q.s * tok;
         g.c_bs0 = q.dh; g.c_bs1 = q.s * q.hd;
         g.batch_inner = q.h; g.batch_outer = q.b;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     }
     // 6. h1 = ctx W_o^T + b_o + x
     STEP(6) {
         BmtGemmDesc g = plain(q.T, q.d, q.hd, k.ctx, q.hd, 0, k.out_w, q.hd, 0, k.h1, q.d, dt);
         g.bias = k.out_b; g.residual = k.x; g.ldr = q.d;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     // 7. LN2
     STEP(7) RUN(bmt_norm_fwd(q.T, q.d, k.h1, k.ln2_w, k.ln2_b, k.eps, 0, dt, k.ln2, k.stats2, stream));
@@ -113,14 +118,14 @@ extern "C" int bmt_gpt_block_forward_steps(const BmtGptBlock* blk, int first_ste
     STEP(8) {
         BmtGemmDesc g = plain(q.T, q.dff, q.d, k.ln2, q.d, 0, k.fc1_w, q.d, 0, k.act == 2 ? k.pre : k.ff, q.dff, dt);
         g.bias = k.fc1_b; g.act = k.act == 1 ? 1 : 0;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
         if (k.act == 2) RUN(bmt_gelu_fwd(q.T * q.dff, k.pre, dt, k.ff, stream));
     }
     // 9. y = ff W_2^T + b_2 + h1
     STEP(9) {
         BmtGemmDesc g = plain(q.T, q.d, q.dff, k.ff, q.dff, 0, k.fc2_w, q.dff, 0, k.y, q.d, dt);
         g.bias = k.fc2_b; g.residual = k.h1; g.ldr = q.d;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
 #undef STEP
     return 0;
@@ -139,38 +144,38 @@ extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockG
     {   // d_ff = (dy W_2) * act'(.)
         BmtGemmDesc g = plain(q.T, q.dff, q.d, w.dy, q.d, 0, k.fc2_w, q.dff, 1, w.d_ff, q.dff, dt);
         g.aux = k.act == 2 ? k.pre : k.ff; g.ld_aux = q.dff; g.aux_mode = k.act == 2 ? 2 : 1;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     {   // dW_2 = dy^T ff
         BmtGemmDesc g = plain(q.d, q.dff, q.T, w.dy, q.d, 1, k.ff, q.dff, 1, w.d_fc2_w, q.dff, dt);
         g.accumulate = w.acc_w;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
-    RUN(bmt_colsum_ex(q.T, q.d, w.dy, dt, w.d_fc2_b, w.acc_small, w.colsum_scratch, w.colsum_scratch_bytes, stream));
+    RUN(bmt_colsum_ex(q.T, q.d, w.dy, dt, w.d_fc2_b, w.acc_small, k.colsum_scratch, k.colsum_scratch_bytes, stream));
     {   // d_ln2 = d_ff W_1
         BmtGemmDesc g = plain(q.T, q.d, q.dff, w.d_ff, q.dff, 0, k.fc1_w, q.d, 1, w.d_ln2, q.d, dt);
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     {   // dW_1 = d_ff^T ln2
         BmtGemmDesc g = plain(q.dff, q.d, q.T, w.d_ff, q.dff, 1, k.ln2, q.d, 1, w.d_fc1_w, q.d, dt);
         g.accumulate = w.acc_w;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
-    RUN(bmt_colsum_ex(q.T, q.dff, w.d_ff, dt, w.d_fc1_b, w.acc_small, w.colsum_scratch, w.colsum_scratch_bytes, stream));
+    RUN(bmt_colsum_ex(q.T, q.dff, w.d_ff, dt, w.d_fc1_b, w.acc_small, k.colsum_scratch, k.colsum_scratch_bytes, stream));
     // d_h1 = dy + LN2'(d_ln2)
     RUN(bmt_norm_bwd_ex(q.T, q.d, k.h1, w.d_ln2, k.ln2_w, k.stats2, 0, dt, w.nblk, w.d_h1, w.norm_partial, w.d_ln2_w, w.d_ln2_b,
                         w.dy, w.acc_small, stream));
     // ---- attention output projection
     {   // d_ctx = d_h1 W_o
         BmtGemmDesc g = plain(q.T, q.hd, q.d, w.d_h1, q.d, 0, k.out_w, q.hd, 1, w.d_ctx, q.hd, dt);
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     {   // dW_o = d_h1^T ctx
         BmtGemmDesc g = plain(q.d, q.hd, q.T, w.d_h1, q.d, 1, k.ctx, q.hd, 1, w.d_out_w, q.hd, dt);
         g.accumulate = w.acc_w;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
-    RUN(bmt_colsum_ex(q.T, q.d, w.d_h1, dt, w.d_out_b, w.acc_small, w.colsum_scratch, w.colsum_scratch_bytes, stream));
+    RUN(bmt_colsum_ex(q.T, q.d, w.d_h1, dt, w.d_out_b, w.acc_small, k.colsum_scratch, k.colsum_scratch_bytes, stream));
     // ---- attention core
     const int64_t pl = k.probs_ld;
     if (k.lse) {
@@ -185,39 +190,39 @@ extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockG
         BmtGemmDesc g = plain(q.s, q.s, q.dh, w.d_ctx, q.hd, 0, off(k.qkv, 2 * q.dh), tok, 0, w.d_probs, pl, dt);
         g.a_bs0 = q.dh; g.a_bs1 = q.s * q.hd; g.b_bs0 = head; g.b_bs1 = q.s * tok;
         g.c_bs0 = q.s * pl; g.c_bs1 = q.h * q.s * pl; g.batch_inner = q.h; g.batch_outer = q.b;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     RUN(bmt_softmax_bwd(q.b * q.h * q.s, q.s, pl, k.probs, w.d_probs, 1.f / sqrtf((float)q.dh), dt, stream));
     {   // dq = dS k
         BmtGemmDesc g = plain(q.s, q.dh, q.s, w.d_probs, pl, 0, off(k.qkv, q.dh), tok, 1, w.d_qkv, tok, dt);
         g.a_bs0 = q.s * pl; g.a_bs1 = q.h * q.s * pl; g.b_bs0 = head; g.b_bs1 = q.s * tok;
         g.c_bs0 = head; g.c_bs1 = q.s * tok; g.batch_inner = q.h; g.batch_outer = q.b;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     {   // dk = dS^T q
         BmtGemmDesc g = plain(q.s, q.dh, q.s, w.d_probs, pl, 1, k.qkv, tok, 1, off(w.d_qkv, q.dh), tok, dt);
         g.a_bs0 = q.s * pl; g.a_bs1 = q.h * q.s * pl; g.b_bs0 = head; g.b_bs1 = q.s * tok;
         g.c_bs0 = head; g.c_bs1 = q.s * tok; g.batch_inner = q.h; g.batch_outer = q.b;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     {   // dv = P^T d_ctx
         BmtGemmDesc g = plain(q.s, q.dh, q.s, k.probs, pl, 1, w.d_ctx, q.hd, 1, off(w.d_qkv, 2 * q.dh), tok, dt);
         g.a_bs0 = q.s * pl; g.a_bs1 = q.h * q.s * pl; g.b_bs0 = q.dh; g.b_bs1 = q.s * q.hd;
         g.c_bs0 = head; g.c_bs1 = q.s * tok; g.batch_inner = q.h; g.batch_outer = q.b;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     }
     // ---- QKV projection
     {   // d_ln1 = d_qkv W_qkv   (reuses the d_ln2 buffer)
         BmtGemmDesc g = plain(q.T, q.d, 3 * q.hd, w.d_qkv, tok, 0, k.qkv_w, q.d, 1, w.d_ln2, q.d, dt);
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
     {   // dW_qkv = d_qkv^T ln1
         BmtGemmDesc g = plain(3 * q.hd, q.d, q.T, w.d_qkv, tok, 1, k.ln1, q.d, 1, w.d_qkv_w, q.d, dt);
         g.accumulate = w.acc_w;
-        RUN(bmt_gemm_ex(&g, stream));
+        RUN(gemm(k, g, stream));
     }
-    RUN(bmt_colsum_ex(q.T, 3 * q.hd, w.d_qkv, dt, w.d_qkv_b, w.acc_small, w.colsum_scratch, w.colsum_scratch_bytes, stream));
+    RUN(bmt_colsum_ex(q.T, 3 * q.hd, w.d_qkv, dt, w.d_qkv_b, w.acc_small, k.colsum_scratch, k.colsum_scratch_bytes, stream));
     // dx = d_h1 + LN1'(d_ln1)
     RUN(bmt_norm_bwd_ex(q.T, q.d, k.x, w.d_ln2, k.ln1_w, k.stats1, 0, dt, w.nblk, w.dx, w.norm_partial, w.d_ln1_w, w.d_ln1_b,
                         w.d_h1, w.acc_small, stream));

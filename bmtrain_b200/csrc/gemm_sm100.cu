@@ -17,6 +17,7 @@
 //
 // The reference has no GEMM kernel: all matmuls go through cuBLAS (bmtrain/nn/linear.py:10-24).
 #include <cuda.h>
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
 #include <vector>
@@ -76,7 +77,12 @@ struct GemmParams {
     int64_t ld_aux;
     int aux_mode;          // 0 none, 1: out *= (aux > 0)  (ReLU backward), 2: out *= gelu'(aux)
     int group_m;           // tile raster: consecutive tiles walk down `group_m` row blocks before moving to the next column block
-    int debug;             // measurement only (BMT_GEMM_DEBUG): 1 = no TMA loads, 2 = no MMAs, 4 = no epilogue stores
+    // Split tiles: the first `sk_tiles` tiles of the raster are cut along K over the first `sk_workers` CTAs (or CTA pairs), see Work.
+    int sk_tiles, sk_workers, sk_snap;
+    uint32_t sk_tag;       // what a flag holds when the partial sums behind it are complete (another one for each launch)
+    uint32_t* sk_flags;    // SK_WARPS words per CTA, zero between launches
+    float4* sk_part;       // sk_slot 16-byte units per CTA
+    uint32_t sk_slot;
 };
 
 __device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
@@ -192,6 +198,171 @@ template <typename T> __device__ __forceinline__ void unpack8(const uint4& q, fl
 }
 __device__ __forceinline__ uint4 ld_global_16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 
+// ---- split tiles --------------------------------------------------------------------------------------------------------
+// Whole tiles leave SMs idle when their number is not a multiple of the CTAs: outputs of 1024 x 2560 are 40 tiles of 256 x 256 for 74
+// pairs, and smaller tiles pay in bytes from L2 per multiplication.  So the tiles of the last, partial wave (and of the wave before, when
+// there is one) are laid end to end along K and cut into equal ranges, one per CTA (pair).  After its whole tiles a CTA works on the
+// part of its range that ends inside a tile and leaves the fp32 accumulators in its slot of the scratch; last, the CTA whose range
+// holds the end of a tile adds the slots of the others to its own accumulators, in a fixed order, and stores the tile.  It waits only
+// for CTAs with a lower index, which have been given an SM before it and wait for nobody before they deliver.
+constexpr int SK_WARPS = 8;
+struct Item { int tile, kb0, kb1, kind; };        // kind: 0 whole tile, 1 leaves partial sums, 2 adds the others' and stores
+struct Work {
+    int begin, end, k_blocks, phase, whole, whole_end, tile, step, tiles;
+    __host__ __device__ __forceinline__ static int bound(const GemmParams& p, int worker, int k_blocks) {
+        const int total = p.sk_tiles * k_blocks;
+        if (worker >= p.sk_workers) return total;
+        int at = (int)((int64_t)worker * total / p.sk_workers);
+        const int in = at % k_blocks;             // no slivers of a tile
+        if (in < p.sk_snap) at -= in;
+        else if (k_blocks - in < p.sk_snap) at += k_blocks - in;
+        return at;
+    }
+    // First of the workers whose ranges reach into the tile that `worker` finishes; it and those up to worker - 1 leave sums of it.
+    __host__ __device__ __forceinline__ static int first_of(const GemmParams& p, int worker, int tile, int k_blocks) {
+        int low = worker - 1;
+        while (low > 0 && bound(p, low, k_blocks) > tile * k_blocks) --low;
+        return low;
+    }
+    // `worker` takes the whole tiles sk_tiles + worker, + step, ... and the range [bound(worker), bound(worker + 1)) of the split ones
+    __host__ __device__ __forceinline__ Work(const GemmParams& p, int worker, int step_, int tiles_, int k_blocks_, bool split)
+        : begin(0), end(0), k_blocks(k_blocks_), phase(3), whole(0), whole_end(0), tile(worker), step(step_), tiles(tiles_) {
+        if (!split) return;
+        tile += p.sk_tiles;
+        if (worker >= p.sk_workers) return;
+        begin = bound(p, worker, k_blocks);
+        end = bound(p, worker + 1, k_blocks);
+        whole = (begin + k_blocks - 1) / k_blocks;
+        whole_end = end / k_blocks;
+        phase = begin < end ? 1 : 3;
+    }
+    __host__ __device__ __forceinline__ bool next(Item& it) {
+        if (tile < tiles) {
+            it = Item{tile, 0, k_blocks, 0};
+            tile += step;
+            return true;
+        }
+        if (whole < whole_end) { it = Item{whole++, 0, k_blocks, 0}; return true; }
+        if (phase == 1) {
+            phase = 2;
+            const int t = end / k_blocks, at = t * k_blocks;
+            if (end > at) { it = Item{t, (begin > at ? begin : at) - at, end - at, 1}; return true; }
+        }
+        if (phase == 2) {
+            phase = 3;
+            const int t = begin / k_blocks, in = begin - t * k_blocks;
+            if (in && (t + 1) * k_blocks <= end) { it = Item{t, in, k_blocks, 2}; return true; }
+        }
+        return false;
+    }
+};
+
+// The next item of a whole warp, in a form that tells the compiler that it is the same in all lanes: the descriptors and coordinates
+// that depend on it stay in uniform registers (without, a k-block of a single-CTA tile took 120 ns more).
+__device__ __forceinline__ bool next_item(Work& work, Item& it) {
+    const bool more = __all_sync(0xffffffffu, work.next(it)) != 0;
+    if (more) {
+        it.tile = __shfl_sync(0xffffffffu, it.tile, 0);
+        it.kb0 = __shfl_sync(0xffffffffu, it.kb0, 0);
+        it.kb1 = __shfl_sync(0xffffffffu, it.kb1, 0);
+        it.kind = __shfl_sync(0xffffffffu, it.kind, 0);
+    }
+    return more;
+}
+
+// The slots a storing warp adds: `count` of them, from `at` down, `slot` units apart.  In a slot, piece c (32 columns) of the 32 rows of
+// a quarter is 256 units of 16 bytes, unit q * 32 + r being the columns 4q .. 4q + 3 of row r: what a lane holds in registers, and 512
+// consecutive bytes per access.  The tile is the CTA's last, so the pipeline's shared memory is free: the units are fetched SK_AHEAD
+// pieces ahead (every lane its own, so nobody has to be waited for); read when needed, a piece took 1 us.
+constexpr int SK_AHEAD = 4;
+struct Partials {
+    const float4* at;
+    int64_t slot;
+    int count;
+    uint32_t ring;                    // this lane's first unit of SK_AHEAD buffers of 4 KiB
+    int c, i, step, n_chunks;         // next piece to fetch
+    uint32_t put, get;
+
+    __device__ __forceinline__ void fetch() {
+        if (c < n_chunks) {
+            const float4* src = at - i * slot + c * 256;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring + put * 4096 + q * 512), "l"(src + q * 32) : "memory");
+            if (++put == SK_AHEAD) put = 0;
+            if (++i == count) { i = 0; c += step; }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    __device__ __forceinline__ void start(uint32_t ring_, int first, int step_, int n_chunks_) {
+        ring = ring_; c = first; i = 0; step = step_; n_chunks = n_chunks_; put = get = 0;
+#pragma unroll
+        for (int k = 0; k < SK_AHEAD; ++k) fetch();
+    }
+    // r += the next piece of all slots
+    __device__ __forceinline__ void add(uint32_t (&r)[32]) {
+        for (int k = 0; k < count; ++k) {
+            float4 v[8];
+            asm volatile("cp.async.wait_group %0;" ::"n"(SK_AHEAD - 1) : "memory");
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[q].x), "=f"(v[q].y), "=f"(v[q].z), "=f"(v[q].w)
+                             : "r"(ring + get * 4096 + q * 512) : "memory");
+            if (++get == SK_AHEAD) get = 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                r[4 * q] = __float_as_uint(__uint_as_float(r[4 * q]) + v[q].x);
+                r[4 * q + 1] = __float_as_uint(__uint_as_float(r[4 * q + 1]) + v[q].y);
+                r[4 * q + 2] = __float_as_uint(__uint_as_float(r[4 * q + 2]) + v[q].z);
+                r[4 * q + 3] = __float_as_uint(__uint_as_float(r[4 * q + 3]) + v[q].w);
+            }
+            fetch();
+        }
+    }
+};
+
+// This warp's pieces of the accumulator into the slot, then its flag.
+template <typename Release>
+__device__ __forceinline__ void store_partials(float4* slot, uint32_t* flag, uint32_t tag, int n_chunks, uint32_t taddr, int lane, int first,
+                                               Release release) {
+    if (first >= n_chunks) release();
+    for (int c = first; c < n_chunks; c += 2) {
+        uint32_t r[32];
+        tmem_ld32(taddr + c * 32, r);
+        tmem_ld_wait();
+        if (c + 2 >= n_chunks) release();
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            __stcg(slot + c * 256 + q * 32, make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
+                                                          __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3])));
+    }
+    __syncwarp();       // the release of lane 0 covers what the others have stored
+    if (lane == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(tag) : "memory");
+}
+
+// Bounded wait for the same warp of `count` other CTAs; takes the flags back.
+__device__ __forceinline__ bool wait_partials(uint32_t* flag, int64_t pitch, int count, uint32_t tag, int lane) {
+    bool ok = true;
+    if (lane == 0)
+        for (int i = 0; i < count && ok; ++i, flag -= pitch) {
+            uint64_t t0 = 0;
+            for (uint32_t spin = 0;; ++spin) {
+                uint32_t v;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+                if (v == tag) break;
+                if ((spin & 255u) == 255u) {
+                    const uint64_t now = global_ns();
+                    if (t0 == 0) t0 = now;
+                    else if (now - t0 > 2000000000ull) { ok = false; break; }
+                }
+            }
+            asm volatile("st.relaxed.gpu.global.u32 [%0], 0;" ::"l"(flag) : "memory");
+        }
+    ok = __all_sync(0xffffffffu, ok) != 0;
+    __syncwarp();       // what lane 0 has acquired is there for the others
+    return ok;
+}
+
 // Epilogue of one warp's 32 rows of a tile: tensor memory -> (alpha, bias, activation, mask, residual, old C) -> global.
 // tcgen05.ld hands every thread one row; written out that way, a store instruction touches 32 rows with 16 bytes each, which
 // cost 5.5 to 8 us per 128 x 256 tile and made every weight gradient of a 1024-token block epilogue-bound (2560 x 8192 x 1024:
@@ -223,7 +394,8 @@ __device__ __forceinline__ void epi_get(uint32_t sbuf, int lane, int rl, float (
 
 template <typename T, int EXTRA, typename Release>
 __device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, const T* ebase, int64_t e_ld, int64_t row0, int64_t n0,
-                                              int64_t col_end, uint32_t taddr, uint32_t sbuf, int lane, int first, Release release) {
+                                              int64_t col_end, uint32_t taddr, uint32_t sbuf, int lane, int first, Partials& sk,
+                                              Release release) {
     const int sub = lane >> 2, cq = (lane & 3) * 8;
     const int n_cols = (int)(col_end - n0), n_chunks = (n_cols + 31) / 32;
     const int rows = (int)(p.M - row0 < 32 ? p.M - row0 : 32);     // may be <= 0: nothing is stored then
@@ -251,6 +423,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, con
         float b[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         if (bias && col_ok) load8(bias + c * 32, b);
         tmem_ld_wait();
+        if (sk.count) sk.add(r);
         epi_put(sbuf, lane, r);
         if (c + 2 < n_chunks) tmem_ld32(taddr + (c + 2) * 32, r);
         else release();
@@ -280,7 +453,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, con
                 for (int i = 0; i < 8; ++i)
                     v[it][i] = EXTRA == 1 ? v[it][i] + e[i] : EXTRA == 2 ? (e[i] > 0.f ? v[it][i] : 0.f) : v[it][i] * gelu_grad_f(e[i]);
             }
-            if (col_ok && it * 8 + sub < rows && !(p.debug & 4)) store8(dst + it * d_step + c * 32, v[it]);
+            if (col_ok && it * 8 + sub < rows) store8(dst + it * d_step + c * 32, v[it]);
         }
     }
 }
@@ -288,7 +461,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, con
 // All other forms: fp32 output, odd pitches and widths, unaligned pointers, GELU, several extras at once.
 template <typename TC, typename Release>
 __device__ __forceinline__ void epilogue_rows_any(const GemmParams& p, TC* cbase, int64_t row0, int64_t n0, int64_t col_end, uint32_t taddr,
-                                               uint32_t sbuf, int lane, int first, Release release) {
+                                               uint32_t sbuf, int lane, int first, Partials& sk, Release release) {
     const int sub = lane >> 2, cq = (lane & 3) * 8;
     const int n_chunks = (int)((col_end - n0 + 31) / 32);
     const bool c_vec = sizeof(TC) == 2 ? ((p.ldc & 7) == 0 && (((uintptr_t)cbase) & 15) == 0)
@@ -300,6 +473,7 @@ __device__ __forceinline__ void epilogue_rows_any(const GemmParams& p, TC* cbase
         uint32_t r[32];
         tmem_ld32(taddr + c * 32, r);
         tmem_ld_wait();
+        if (sk.count) sk.add(r);
         epi_put(sbuf, lane, r);
         if (c + 2 >= n_chunks) release();
         __syncwarp();
@@ -339,7 +513,6 @@ __device__ __forceinline__ void epilogue_rows_any(const GemmParams& p, TC* cbase
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] += e[i];
             }
-            if (p.debug & 4) continue;
             if (n_ok == 8 && c_vec) {
                 if constexpr (sizeof(TC) == 2) {
                     store8(dst, v);
@@ -360,14 +533,14 @@ __device__ __forceinline__ void epilogue_rows_any(const GemmParams& p, TC* cbase
 // Picks the form of the epilogue for a 16-bit output tile; `p.epi` is what launch_gemm found for the whole problem.
 template <typename T, typename Release>
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, T* cbase, int64_t row0, int64_t n0, int64_t col_end, uint32_t taddr,
-                                              uint32_t sbuf, int lane, int first, Release release) {
-    if (p.epi == 0) epilogue_rows<T, 0>(p, cbase, nullptr, 0, row0, n0, col_end, taddr, sbuf, lane, first, release);
+                                              uint32_t sbuf, int lane, int first, Partials& sk, Release release) {
+    if (p.epi == 0) epilogue_rows<T, 0>(p, cbase, nullptr, 0, row0, n0, col_end, taddr, sbuf, lane, first, sk, release);
     else if (p.epi == 1)
         epilogue_rows<T, 1>(p, cbase, p.accumulate ? cbase : (const T*)p.residual, p.accumulate ? p.ldc : p.ldr, row0, n0, col_end, taddr,
-                            sbuf, lane, first, release);
-    else if (p.epi == 2) epilogue_rows<T, 2>(p, cbase, (const T*)p.aux, p.ld_aux, row0, n0, col_end, taddr, sbuf, lane, first, release);
-    else if (p.epi == 3) epilogue_rows<T, 3>(p, cbase, (const T*)p.aux, p.ld_aux, row0, n0, col_end, taddr, sbuf, lane, first, release);
-    else epilogue_rows_any(p, cbase, row0, n0, col_end, taddr, sbuf, lane, first, release);
+                            sbuf, lane, first, sk, release);
+    else if (p.epi == 2) epilogue_rows<T, 2>(p, cbase, (const T*)p.aux, p.ld_aux, row0, n0, col_end, taddr, sbuf, lane, first, sk, release);
+    else if (p.epi == 3) epilogue_rows<T, 3>(p, cbase, (const T*)p.aux, p.ld_aux, row0, n0, col_end, taddr, sbuf, lane, first, sk, release);
+    else epilogue_rows_any(p, cbase, row0, n0, col_end, taddr, sbuf, lane, first, sk, release);
 }
 
 // ---- two-CTA (cta_group::2) helpers: the pair shares one 256 x BN accumulator tile, each CTA feeds its own
@@ -385,8 +558,10 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_smem_addr, uint32_
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Relaxed: what has to come before it is the warp's reading of tensor memory, which tcgen05.wait::ld and the fence have completed.  A
+// release would also wait for the warp's stores to global memory, about 1000 clocks.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_2cta(uint32_t* dst_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
@@ -702,7 +877,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             uint32_t ps = 0, pph = 0;   // ring position and phase, carried across tiles
             const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(&hdr->full[0]), empty0 = smem_u32(&hdr->empty[0]);
             const uint32_t full_leader0 = CTA2 ? map_to_cta(full0, 0) : full0;
-            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
+            Work work(p, first_tile, tile_step, num_tiles, k_blocks, FUSED == 0 && p.sk_tiles > 0);
+            for (Item it; ok && next_item(work, it);) {
+                const int tile = it.tile;
                 const int batch = tile / tiles_per_batch;
                 const int rem = tile - batch * tiles_per_batch;
                 int m_blk, n_blk;
@@ -746,14 +923,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                 const int bib = bi / (int)p.b_inner_div;
                 const int m0 = m_blk * (BM * NCTA) + (int)rank * BM;            // this CTA's rows of A
                 const int n0 = n_blk * p.bn + (int)(rank * bn_local);           // this CTA's rows of the B tile
-                for (int kb = 0; kb < k_blocks; ++kb) {
+                for (int kb = it.kb0; kb < it.kb1; ++kb) {
                     if (!mbar_wait_warp(empty0 + 8 * ps, pph ^ 1)) { ok = false; if (lane == 0) { atomicCAS(&g_gemm_status, 0, (1 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; } break; }
                     const uint32_t sa = smem0 + ps * stage_bytes, sb = sa + a_bytes;
                     const int kx = kb * BK;
                     if (elect_one()) {
-                        if (p.debug & 1) {
-                            if (rank == 0) mbar_arrive_u32(full0 + 8 * ps);
-                        } else if (!CTA2) {
+                        if (!CTA2) {
                             const uint32_t bar = full0 + 8 * ps;
                             mbar_expect_tx_u32(bar, stage_bytes);
                             if (!p.a_mn) {
@@ -816,29 +991,29 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             const uint32_t d_hi = desc_hi(1024);
             const uint32_t a_lbo = p.a_mn ? 64 * BK * 2 : 0, b_lbo = p.b_mn ? 64 * BK * 2 : 0;
             const uint32_t a_kstep = (p.a_mn ? UMMA_K * 128 : UMMA_K * 2) >> 4, b_kstep = (p.b_mn ? UMMA_K * 128 : UMMA_K * 2) >> 4;
-            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++tcount) {
+            Work work(p, first_tile, tile_step, num_tiles, k_blocks, FUSED == 0 && p.sk_tiles > 0);
+            for (Item it; ok && next_item(work, it); ++tcount) {
                 const uint32_t acc = tcount & 1;
                 const uint32_t acc_ph = (tcount >> 1) & 1;
                 if (!mbar_wait_warp(tempty0 + 8 * acc, acc_ph ^ 1)) { ok = false; if (lane == 0) { atomicCAS(&g_gemm_status, 0, (2 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; } break; }
                 tc_fence_after();
                 const uint32_t tmem_c = tmem_base + acc * p.bn;
-                for (int kb = 0; kb < k_blocks; ++kb) {
+                for (int kb = it.kb0; kb < it.kb1; ++kb) {
                     if (!mbar_wait_warp(full0 + 8 * cs, cph)) { ok = false; if (lane == 0) { atomicCAS(&g_gemm_status, 0, (3 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; } break; }
                     tc_fence_after();
                     const uint32_t sa = smem0 + cs * stage_bytes;
                     const uint32_t a_lo = desc_lo(sa, a_lbo), b_lo = desc_lo(sa + a_bytes, b_lbo);
                     if (elect_one()) {
-                        if (!(p.debug & 2)) {
 #pragma unroll
-                            for (int k = 0; k < BK / UMMA_K; ++k) {
-                                const uint64_t ad = pack_desc(a_lo + k * a_kstep, d_hi), bd = pack_desc(b_lo + k * b_kstep, d_hi);
-                                if (CTA2) umma_f16_2cta(tmem_c, ad, bd, p.idesc, (kb | k) != 0 ? 1u : 0u);
-                                else umma_f16(tmem_c, ad, bd, p.idesc, (kb | k) != 0 ? 1u : 0u);
-                            }
+                        for (int k = 0; k < BK / UMMA_K; ++k) {
+                            const uint64_t ad = pack_desc(a_lo + k * a_kstep, d_hi), bd = pack_desc(b_lo + k * b_kstep, d_hi);
+                            const uint32_t add = (kb > it.kb0 || k != 0) ? 1u : 0u;
+                            if (CTA2) umma_f16_2cta(tmem_c, ad, bd, p.idesc, add);
+                            else umma_f16(tmem_c, ad, bd, p.idesc, add);
                         }
                         // frees the smem stage (in both CTAs) once these MMAs have read it
                         if (CTA2) umma_commit_2cta_u32(empty0 + 8 * cs); else umma_commit_u32(empty0 + 8 * cs);
-                        if (kb + 1 == k_blocks) { if (CTA2) umma_commit_2cta_u32(tfull0 + 8 * acc); else umma_commit_u32(tfull0 + 8 * acc); }
+                        if (kb + 1 == it.kb1) { if (CTA2) umma_commit_2cta_u32(tfull0 + 8 * acc); else umma_commit_u32(tfull0 + 8 * acc); }
                     }
                     __syncwarp();
                     if (++cs == (uint32_t)p.stages) { cs = 0; cph ^= 1; }
@@ -869,7 +1044,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             }
             remote_open = false;
         };
-        for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++tcount) {
+        Work work(p, first_tile, tile_step, num_tiles, k_blocks, FUSED == 0 && p.sk_tiles > 0);
+        for (Item it; ok && next_item(work, it); ++tcount) {
+            const int tile = it.tile;
             const int batch = tile / tiles_per_batch;
             const int rem = tile - batch * tiles_per_batch;
             int m_blk, n_blk;
@@ -940,7 +1117,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                                          "r"(pk[4 * q + 1]), "r"(pk[4 * q + 2]), "r"(pk[4 * q + 3]) : "memory");
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    if (row_ok && !(p.debug & 4))
+                    if (row_ok)
                         asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
                                      ::"l"(cbase + (coff + col0) * 2), "r"(srow), "r"(ncols * 2) : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -950,9 +1127,31 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                 const uint32_t sbuf = smem_u32(smem) + p.out_stage_off + (uint32_t)(warp - 2) * EPI_BYTES_PER_WARP;
                 const int first = (warp - 2) >> 2;   // two warps see the same 32 rows: they take the 32-column pieces in turn
                 const int64_t coff = bi * p.c_bs0 + bo * p.c_bs1, n0 = (int64_t)n_blk * p.bn;
-                if (p.c_dtype == BMT_DT_F16) epilogue_tile(p, (__half*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, release);
-                else if (p.c_dtype == BMT_DT_BF16) epilogue_tile(p, (__nv_bfloat16*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, release);
-                else epilogue_rows_any(p, (float*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, release);
+                Partials sk;
+                sk.count = 0;
+                if (it.kind != 0) {
+                    const int cta = first_tile * NCTA + (int)rank;
+                    uint32_t* flag = p.sk_flags + cta * SK_WARPS + (warp - 2);
+                    const int n_chunks = (int)((col_end - n0 + 31) / 32);
+                    float4* slot = p.sk_part + (int64_t)cta * p.sk_slot + (uint32_t)quarter * (p.sk_slot / 4) + lane;
+                    if (it.kind == 1) {
+                        store_partials(slot, flag, p.sk_tag, n_chunks, taddr, lane, first, release);
+                        continue;
+                    }
+                    sk.slot = (int64_t)NCTA * p.sk_slot;
+                    sk.at = slot - sk.slot;
+                    sk.count = first_tile - Work::first_of(p, first_tile, tile, k_blocks);
+                    if (!wait_partials(flag - NCTA * SK_WARPS, NCTA * SK_WARPS, sk.count, p.sk_tag, lane)) {
+                        ok = false;
+                        if (lane == 0) { atomicCAS(&g_gemm_status, 0, (12 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; }
+                        break;
+                    }
+                    // the last item of this CTA: its loads have landed and its MMAs have read them
+                    sk.start(smem_u32(smem) + (uint32_t)(warp - 2) * (SK_AHEAD * 4096) + lane * 16, first, 2, n_chunks);
+                }
+                if (p.c_dtype == BMT_DT_F16) epilogue_tile(p, (__half*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, sk, release);
+                else if (p.c_dtype == BMT_DT_BF16) epilogue_tile(p, (__nv_bfloat16*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, sk, release);
+                else epilogue_rows_any(p, (float*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, sk, release);
             }
         }
         if (remote_open) report_remote_done();
@@ -1194,12 +1393,21 @@ int g_reserved_sms = 0;
 // and has to pull (128 + BN / ncta) * 128 bytes from L2 at about 64 bytes per clock; the slower of the two sets
 // the pace.  A CTA pair (cta_group::2, 256 x BN tile) halves the B bytes per SM, which is what lifts large
 // problems off the L2->SM limit.  The cost also counts waves on the available SMs and a fixed per-tile overhead.
-struct TileChoice { int bn; int cta2; };
+//
+// Split tiles (`split`) spread the tiles of the partial wave, with the wave before it if there is one, evenly over all CTAs, or over
+// as many as leave a range SK_MIN k-blocks.  Handing the sums over costs about SK_COST clocks, mostly waiting and fp32 through L2: 3 us
+// behind a long reduction and up to 10 where all SMs write and read their slots at once.  So the estimate has to win by 12 %
+// where there is less than a wave (1024 x 2560 x 8192 in the dgrad layout: 50 -> 43 us; 56 x 720 x 9144: 41 -> 19; 777 x 2560 x 7680,
+// estimated 11 % better, took 41 instead of 40) and by 2 % behind whole waves (4096 x 5120 x 27648: 807 -> 738 us;
+// 2048 x 57344 x 8192: 1256 -> 1208; 2560 x 8192 x 1024, not chosen, would take 44 instead of 38).
+struct TileChoice { int bn, cta2, sk_tiles, sk_workers; };
+constexpr int SK_MIN = 4, SK_MOST = 8;      // k-blocks of a range at least, CTAs per tile at most
+constexpr double SK_COST = 16000.0;
 
-TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn, int force_bn, int force_cta2) {
-    TileChoice best{0, 0};
-    double best_cost = 1e30;
-    const double kblocks = (double)((K + BK - 1) / BK);
+TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn, int force_bn, int force_cta2, bool split) {
+    TileChoice best{0, 0, 0, 0}, best_split{0, 0, 0, 0};
+    double best_cost = 1e30, best_split_cost = 1e30;
+    const int64_t kblocks = (K + BK - 1) / BK;
     for (int cta2 = 0; cta2 <= 1; ++cta2) {
         if (force_cta2 >= 0 && cta2 != force_cta2) continue;
         if (cta2 && M <= BM) continue;
@@ -1211,13 +1419,38 @@ TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn
             const int64_t slots = g_num_sms / ncta;
             const int64_t waves = (tiles + slots - 1) / slots;
             const double mma = 2.05 * bn, load = 2.0 * (128 + bn / ncta);
-            const double per_tile = kblocks * (mma > load ? mma : load) + 600.0 + 6.0 * bn;  // + fill/drain and epilogue
-            const double cost = (double)waves * per_tile;
-            if (cost < best_cost * 0.999) { best_cost = cost; best = TileChoice{bn, cta2}; }
+            const double per_block = mma > load ? mma : load, fixed = 600.0 + 6.0 * bn;   // + fill/drain and epilogue
+            const double cost = (double)waves * (kblocks * per_block + fixed);
+            if (cost < best_cost * 0.999) { best_cost = cost; best = TileChoice{bn, cta2, 0, 0}; }
+            if (!split || tiles % slots == 0) continue;
+            const bool behind = tiles > slots;              // behind whole waves
+            const int64_t sk_tiles = tiles % slots + (behind ? slots : 0), total = sk_tiles * kblocks;
+            int64_t workers = slots;
+            if (workers > sk_tiles * SK_MOST) workers = sk_tiles * SK_MOST;
+            if (workers > total / SK_MIN) workers = total / SK_MIN;
+            if (workers <= sk_tiles && !behind) continue;
+            const int64_t whole_waves = (tiles - sk_tiles) / slots;
+            const double parts = (double)workers / sk_tiles;        // a CTA adds what the others left of its tile: 8 * bn clocks a slot
+            const double estimate = (whole_waves * kblocks + (double)total / workers) * per_block + (whole_waves + 2) * fixed + SK_COST +
+                                    (parts > 1 ? (parts - 1) * 8 * bn : 0);
+            const double c = estimate / (behind ? 0.98 : 0.88);
+            if (c < best_split_cost) { best_split_cost = c; best_split = TileChoice{bn, cta2, (int)sk_tiles, (int)workers}; }
         }
     }
-    return best;
+    return best_split_cost < best_cost ? best_split : best;
 }
+
+// Tensor of a scratch: flags of all CTAs, then their slots.
+int64_t sk_bytes(int ctas, int bn) { return (int64_t)ctas * (SK_WARPS * 4 + 128 * ((bn + 31) / 32 * 32) * 4); }
+std::atomic<uint32_t> g_sk_tag{0};
+
+void set_split(GemmParams& p, const TileChoice& tc, int k_blocks) {
+    p.sk_tiles = tc.sk_tiles; p.sk_workers = tc.sk_workers;
+    p.sk_snap = (int64_t)tc.sk_tiles * k_blocks / tc.sk_workers >= 16 ? 3 : 1;     // ranges stay longer than two snaps
+}
+
+// CTAs (pairs) of a launch with split tiles: whole tiles come only in full waves.
+int64_t whole_or_split(int64_t tiles, int64_t slots, const TileChoice& tc) { return tiles > tc.sk_tiles ? slots : tc.sk_workers; }
 
 int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fused = nullptr) {
     const int64_t m = g.m, n = g.n, k = g.k;
@@ -1243,8 +1476,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
         BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
         BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
     }
-    static int force_bn = -1, force_cta2 = -2, debug_flags = -1;
-    if (debug_flags < 0) { const char* e = getenv("BMT_GEMM_DEBUG"); debug_flags = e ? atoi(e) : 0; }
+    static int force_bn = -1, force_cta2 = -2;
     if (force_bn < 0) { const char* e = getenv("BMT_GEMM_BN"); force_bn = e ? atoi(e) : 0; }
     if (force_cta2 == -2) { const char* e = getenv("BMT_GEMM_CTA2"); force_cta2 = e ? atoi(e) : -1; }
 
@@ -1257,9 +1489,16 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     if (fused) g_num_sms -= held_back;  // tile choice for the CTAs that do math
     // a fused kernel can run as CTA pairs when its pusher CTAs pair up too and (mode 2) a rank's rows fill whole 256-row tiles
     const bool pair_ok = !fused || (comm_ctas % 2 == 0 && (fused->mode != 2 || fused->ag_rows % (2 * BM) == 0));
-    TileChoice tc = pick_tile(m, n, k, batch_inner * batch_outer, b_major != 0, force_bn, pair_ok ? force_cta2 : 0);
+    // Split tiles need scratch whose flags nobody else uses.  A captured launch may be replayed next to any other, on any stream: there
+    // the tiles stay whole.
+    bool split = !fused && g.scratch && k < (1 << 26) && g.scratch_bytes >= sk_bytes(g_num_sms, 256);
+    if (split) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) { cudaGetLastError(); split = false; }
+    }
+    TileChoice tc = pick_tile(m, n, k, batch_inner * batch_outer, b_major != 0, force_bn, pair_ok ? force_cta2 : 0, split);
     if (fused) g_num_sms += held_back;
-    if (tc.bn == 0) tc = pick_tile(m, n, k, batch_inner * batch_outer, b_major != 0, 0, -1);  // forced shape not applicable here
+    if (tc.bn == 0) tc = pick_tile(m, n, k, batch_inner * batch_outer, b_major != 0, 0, -1, split);  // forced shape not applicable here
     if (tc.bn == 0) return -22;
     p.bn = tc.bn;
     const int ncta = tc.cta2 ? 2 : 1;
@@ -1272,10 +1511,16 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     p.batch_inner = batch_inner; p.batch_outer = batch_outer; p.b_inner_div = b_inner_div > 0 ? b_inner_div : 1;
     p.c = c; p.ldc = ldc; p.c_bs0 = c_bs0; p.c_bs1 = c_bs1; p.c_dtype = c_dtype;
     p.bias = bias; p.bias_dtype = ab_dtype; p.act = act; p.accumulate = accumulate; p.alpha = alpha;
-    p.debug = debug_flags;
     static int group_env = -1;
     if (group_env < 0) { const char* e = getenv("BMT_GEMM_GROUP_M"); group_env = e ? atoi(e) : 0; }
     p.group_m = group_env > 0 ? group_env : 16;
+    if (tc.sk_tiles) {
+        set_split(p, tc, (int)((k + BK - 1) / BK));
+        do p.sk_tag = g_sk_tag.fetch_add(1, std::memory_order_relaxed) + 1; while (p.sk_tag == 0);
+        p.sk_flags = (uint32_t*)g.scratch;
+        p.sk_part = (float4*)((char*)g.scratch + (int64_t)g_num_sms * SK_WARPS * 4);
+        p.sk_slot = (uint32_t)(128 * ((p.bn + 31) / 32 * 32) / 4);
+    }
     if (p.group_m > p.m_blocks) p.group_m = p.m_blocks;
     if (fused && fused->mode == 3) p.group_m = p.m_blocks;  // all row tiles of one weight chunk in a row: chunks are needed in order
     const bool rs_early = fused && fused->mode == 1 && fused->rs_rows % (BM * ncta) == 0;
@@ -1365,7 +1610,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
         return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
     }
     if (!tc.cta2) {
-        const unsigned grid = (unsigned)(tiles < g_num_sms ? tiles : g_num_sms);
+        const unsigned grid = (unsigned)(tc.sk_tiles ? whole_or_split(tiles, g_num_sms, tc) : tiles < g_num_sms ? tiles : g_num_sms);
         gemm_tcgen05_kernel<false, 0><<<grid, num_threads(0), smem, stream>>>(ma, mb, p, none);
         bmt_count_launch(1);
         return (int)cudaGetLastError();
@@ -1373,7 +1618,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     const int64_t pairs = g_num_sms / 2;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
+    cfg.gridDim = dim3((unsigned)(2 * (tc.sk_tiles ? whole_or_split(tiles, pairs, tc) : tiles < pairs ? tiles : pairs)));
     cfg.blockDim = dim3(num_threads(0));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -1393,16 +1638,48 @@ extern "C" int bmt_gemm_reserve_sms(int n) {
     return 0;
 }
 
+// How a GEMM that has scratch is divided: plan = {tile width, CTAs per tile, tiles, split tiles, CTAs (pairs) that share them, CTAs
+// (pairs) of the grid}; the items of `worker` (tile, first and last k-block, kind, first of the workers that leave sums) go to `items`.
+// Returns their number.  Host arithmetic only.
+extern "C" int bmt_gemm_plan(int64_t m, int64_t n, int64_t k, int b_major, int worker, int64_t* plan, int* items, int most) {
+    const int sms = bmt::sm_count();
+    if (g_num_sms != 0 && g_num_sms != sms) return -1;
+    const int was = g_num_sms;
+    g_num_sms = sms;
+    const TileChoice tc = pick_tile(m, n, k, 1, b_major != 0, 0, -1, true);
+    g_num_sms = was;
+    const int ncta = tc.cta2 ? 2 : 1, k_blocks = (int)((k + BK - 1) / BK);
+    const int64_t tiles = ((m + BM * ncta - 1) / (BM * ncta)) * ((n + tc.bn - 1) / tc.bn), slots = sms / ncta;
+    const int64_t grid = tc.sk_tiles ? whole_or_split(tiles, slots, tc) : tiles < slots ? tiles : slots;
+    const int64_t out[6] = {tc.bn, ncta, tiles, tc.sk_tiles, tc.sk_workers, grid};
+    memcpy(plan, out, sizeof(out));
+    GemmParams p;
+    memset(&p, 0, sizeof(p));
+    if (tc.sk_tiles) set_split(p, tc, k_blocks);
+    Work work(p, worker, (int)grid, (int)tiles, k_blocks, tc.sk_tiles > 0);
+    int count = 0;
+    for (Item it; work.next(it); ++count) {
+        if (count >= most) return -2;
+        const int row[5] = {it.tile, it.kb0, it.kb1, it.kind, it.kind == 2 ? Work::first_of(p, worker, it.tile, k_blocks) : worker};
+        memcpy(items + 5 * count, row, sizeof(row));
+    }
+    return count;
+}
+
+extern "C" int64_t bmt_gemm_scratch_bytes(void) {
+    return sk_bytes(bmt::sm_count(), 256);
+}
+
 extern "C" int bmt_gemm_ex(const BmtGemmDesc* desc, void* stream) { return launch_gemm(*desc, (cudaStream_t)stream); }
 
 extern "C" int bmt_gemm(int64_t m, int64_t n, int64_t k, const void* a, int64_t lda, int a_major, const void* b, int64_t ldb,
                         int b_major, void* c, int64_t ldc, int c_dtype, const void* bias, int act, int accumulate, int ab_dtype,
-                        void* stream) {
+                        void* scratch, int64_t scratch_bytes, void* stream) {
     BmtGemmDesc g;
     memset(&g, 0, sizeof(g));
     g.m = m; g.n = n; g.k = k; g.a = a; g.lda = lda; g.a_major = a_major; g.b = b; g.ldb = ldb; g.b_major = b_major;
     g.c = c; g.ldc = ldc; g.c_dtype = c_dtype; g.bias = bias; g.act = act; g.accumulate = accumulate; g.ab_dtype = ab_dtype;
-    g.batch_inner = g.batch_outer = g.b_inner_div = 1; g.alpha = 1.0f;
+    g.batch_inner = g.batch_outer = g.b_inner_div = 1; g.alpha = 1.0f; g.scratch = scratch; g.scratch_bytes = scratch_bytes;
     return launch_gemm(g, (cudaStream_t)stream);
 }
 
@@ -1493,7 +1770,7 @@ extern "C" int bmt_gemm_rs_grid(int64_t m, int64_t n, int64_t k, int b_major) {
         if (cudaGetDevice(&dev) != cudaSuccess) return -1;
         if (cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
     }
-    const TileChoice tc = pick_tile(m, n, k, 1, b_major != 0, 0, 0);
+    const TileChoice tc = pick_tile(m, n, k, 1, b_major != 0, 0, 0, false);
     const int64_t tiles = ((m + BM - 1) / BM) * ((n + tc.bn - 1) / tc.bn);
     return (int)(tiles < g_num_sms ? tiles : g_num_sms);
 }

@@ -45,13 +45,14 @@ def _launch(a, b, out, m, n, k, a_major, b_major, bias, act, accumulate, lda, ld
     lib = _native.cuda_lib()
     assert a.dtype == b.dtype and a.dtype in _DT, "tensor-core GEMM takes fp16 or bf16 operands"
     out_dt = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}[out.dtype]
+    work = scratch()
     status = lib.bmt_gemm(
         ctypes.c_int64(m), ctypes.c_int64(n), ctypes.c_int64(k),
         _native.ptr(a), ctypes.c_int64(lda), ctypes.c_int(a_major),
         _native.ptr(b), ctypes.c_int64(ldb), ctypes.c_int(b_major),
         _native.ptr(out), ctypes.c_int64(out.stride(0)), ctypes.c_int(out_dt),
         _native.ptr(bias), ctypes.c_int(_ACT[act]), ctypes.c_int(1 if accumulate else 0),
-        ctypes.c_int(_DT[a.dtype]), _native.stream_handle())
+        ctypes.c_int(_DT[a.dtype]), *work.gemm, work.stream)
     _native.check(status, f"tcgen05 GEMM (m={m}, n={n}, k={k})")
 
 
@@ -133,18 +134,40 @@ def gemm_tn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
     return out
 
 
+_COLSUM_BYTES = 4 * (1024 + 2 * 1024 * 1024)
+_MOST_SCRATCH = 16
 _scratch = {}
 
 
-def colsum_scratch(dev) -> torch.Tensor:
-    """Work space of the row-split column sums (4 KB of ticket counters + partial sums), one per device and stream, zeroed
-    once: the kernel leaves the counters at zero, and calls that share it are ordered on their stream."""
-    index = dev.index if dev.index is not None else torch.cuda.current_device()
-    key = (index, torch._C._cuda_getCurrentRawStream(index))
-    buf = _scratch.get(key)
-    if buf is None:
-        buf = _scratch[key] = torch.zeros(1024 + 2 * 1024 * 1024, dtype=torch.float32, device=dev)
-    return buf
+class _Scratch:
+    """Work space of the kernels that add partial sums, one per device and stream, zeroed once: the kernels leave counters and flags
+    at zero, and launches that share it take turns on their stream.  The first part belongs to the column sums (4 KB of ticket
+    counters and the sums), the second to the GEMMs that divide tiles over several CTAs.  Both as C arguments, with the stream."""
+
+    __slots__ = ("buf", "colsum", "gemm", "stream")
+
+    def __init__(self, index, stream):
+        lib = _native.cuda_lib()
+        lib.bmt_gemm_scratch_bytes.restype = ctypes.c_int64
+        size = lib.bmt_gemm_scratch_bytes()
+        self.buf = torch.zeros(_COLSUM_BYTES + size, dtype=torch.uint8, device=torch.device("cuda", index))
+        base = self.buf.data_ptr()
+        self.colsum = (ctypes.c_void_p(base), ctypes.c_int64(_COLSUM_BYTES))
+        self.gemm = (ctypes.c_void_p(base + _COLSUM_BYTES), ctypes.c_int64(size))
+        self.stream = ctypes.c_void_p(stream)
+
+
+def scratch() -> _Scratch:
+    """The current stream's.  Streams beyond the last ``_MOST_SCRATCH`` that came to have one give theirs back: to the allocator, which
+    hands it out again in the order of the same stream."""
+    index = torch._C._cuda_getDevice()
+    stream = torch._C._cuda_getCurrentRawStream(index)
+    got = _scratch.get((index, stream))
+    if got is None:
+        if len(_scratch) >= _MOST_SCRATCH:
+            _scratch.pop(next(iter(_scratch)), None)
+        got = _scratch[(index, stream)] = _Scratch(index, stream)
+    return got
 
 
 def bias_grad(grad_out: torch.Tensor) -> torch.Tensor:
@@ -155,11 +178,10 @@ def bias_grad(grad_out: torch.Tensor) -> torch.Tensor:
     g = grad_out.contiguous()
     m, n = g.shape
     out = torch.empty(n, dtype=g.dtype, device=g.device)
+    work = scratch()
     dt = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}[g.dtype]
-    scratch = colsum_scratch(g.device)
     _native.check(lib.bmt_colsum_ex(ctypes.c_int64(m), ctypes.c_int64(n), _native.ptr(g), ctypes.c_int(dt), _native.ptr(out),
-                                    ctypes.c_int(0), _native.ptr(scratch), ctypes.c_int64(scratch.numel() * 4),
-                                    _native.stream_handle()), "column-sum kernel")
+                                    ctypes.c_int(0), *work.colsum, work.stream), "column-sum kernel")
     return out
 
 

@@ -34,6 +34,7 @@ class _Block(ctypes.Structure):
         ("ln1", _c_void_p), ("stats1", _c_void_p), ("qkv", _c_void_p), ("probs", _c_void_p), ("probs_ld", _i64),
         ("ctx", _c_void_p), ("h1", _c_void_p), ("ln2", _c_void_p), ("stats2", _c_void_p), ("ff", _c_void_p), ("pre", _c_void_p),
         ("lse", _c_void_p), ("mask_packed", _c_void_p),
+        ("colsum_scratch", _c_void_p), ("colsum_scratch_bytes", _i64), ("gemm_scratch", _c_void_p), ("gemm_scratch_bytes", _i64),
     ]
 
 
@@ -47,7 +48,7 @@ class _Grad(ctypes.Structure):
         ("d_ff", _c_void_p), ("d_ln2", _c_void_p), ("d_h1", _c_void_p), ("d_ctx", _c_void_p), ("d_probs", _c_void_p),
         ("d_qkv", _c_void_p), ("norm_partial", _c_void_p), ("nblk", _int),
         ("dq_acc", _c_void_p), ("delta", _c_void_p),
-        ("acc_small", _int), ("colsum_scratch", _c_void_p), ("colsum_scratch_bytes", ctypes.c_int64),
+        ("acc_small", _int),
     ]
 
 
@@ -106,12 +107,14 @@ def _work_plan(b, s, d, n_heads, d_head, dff, fused_attn, nblk):
 def _describe(x, y, mask, params, saved, plan, n_heads, d_head, act, eps, causal):
     """The block as the native executor takes it; ``saved``: address of the buffer that ``plan`` divides."""
     b, s, d = x.shape
+    work = _gemm.scratch()
     at = lambda name: saved + plan[name] if name in plan else None  # noqa: E731
     # fused attention: scores and probabilities never reach memory, one log-sum-exp per row is kept instead
     return _Block(b, s, d, n_heads, d_head, params[8].shape[0], 0 if x.dtype == torch.float16 else 1, 1 if act == "relu" else 2, eps,
                   1 if causal else 0, None if mask is None else mask.data_ptr(), *[p.data_ptr() for p in params], x.data_ptr(),
                   y.data_ptr(), at("ln1"), at("stats1"), at("qkv"), at("probs"), (s + 7) // 8 * 8 if "probs" in plan else 0,
-                  at("ctx"), at("h1"), at("ln2"), at("stats2"), at("ff"), at("pre"), at("lse"), at("mask_packed"))
+                  at("ctx"), at("h1"), at("ln2"), at("stats2"), at("ff"), at("pre"), at("lse"), at("mask_packed"),
+                  *work.colsum, *work.gemm)
 
 
 class GPTBlockFunction(torch.autograd.Function):
@@ -195,8 +198,6 @@ class GPTBlockFunction(torch.autograd.Function):
                 if not acc:
                     grads[name] = torch.empty_like(p)
                 setattr(g, "d_" + name, (p.grad if acc else grads[name]).data_ptr())
-        scratch = _gemm.colsum_scratch(dev)
-        g.colsum_scratch, g.colsum_scratch_bytes = scratch.data_ptr(), scratch.numel() * 4
         nblk = min(b * s, 296)
         plan, total = _work_plan(b, s, d, n_heads, d_head, params[8].shape[0], fused_attn, nblk)
         work = torch.empty(total, dtype=torch.uint8, device=dev)
