@@ -120,6 +120,7 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
 constexpr int MASK_THREADS = 256;
 __global__ void __launch_bounds__(MASK_THREADS)
 attn_mask_pack_kernel(const uint8_t* mask, int64_t sq, int64_t sk, uint32_t* bits, uint32_t* bits_t, uint8_t* cls) {
+    bmt::after_previous();
     __shared__ uint32_t w[TILE][4];
     __shared__ int any, full;
     const int kt = blockIdx.x, qt = blockIdx.y, b = blockIdx.z, n_kt = gridDim.x, n_qt = gridDim.y;
@@ -198,6 +199,20 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     AttnShared* sh = (AttnShared*)(smem + 6 * TB);
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        mbar_init(&sh->q_full, 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&sh->k_full[i], 1); mbar_init(&sh->v_full[i], 1); mbar_init(&sh->k_empty[i], 1); mbar_init(&sh->v_empty[i], 1);
+            mbar_init(&sh->s_full[i], 1); mbar_init(&sh->p_half[i], 4); mbar_init(&sh->p_ready[i], 4); mbar_init(&sh->o_full[i], 1);
+        }
+        sh->failed = 0;
+        fence_barrier_init();
+    }
+    if (warp == 9) { tmem_alloc(&sh->tmem_base, 512); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    bmt::after_previous();
     const int head = blockIdx.x % p.h, b = blockIdx.x / p.h, kvh = head / (p.h / p.hk);
     const int qt0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * p.per_cta;   // under a causal mask the long rows start first
     int64_t kv_lim = p.sk;
@@ -220,19 +235,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         return j;
     };
 
-    if (threadIdx.x == 0) {
-        mbar_init(&sh->q_full, 1);
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&sh->k_full[i], 1); mbar_init(&sh->v_full[i], 1); mbar_init(&sh->k_empty[i], 1); mbar_init(&sh->v_empty[i], 1);
-            mbar_init(&sh->s_full[i], 1); mbar_init(&sh->p_half[i], 4); mbar_init(&sh->p_ready[i], 4); mbar_init(&sh->o_full[i], 1);
-        }
-        sh->failed = 0;
-        fence_barrier_init();
-    }
-    if (warp == 9) { tmem_alloc(&sh->tmem_base, 512); tmem_relinquish(); }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
     const uint32_t tmem = sh->tmem_base;            // S_0 / P_0 [0,128), S_1 / P_1 [128,256), O_0 [256,384), O_1 [384,512)
     const int first = next_step(-1);
 
@@ -528,7 +530,7 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     // softmax behind the other's MMAs, two SMs are faster still
     p.per_cta = (int64_t)p.q_tiles * p.h * batch > bmt::sm_count() ? 2 : 1;
     dim3 grid((unsigned)(p.h * batch), (unsigned)((p.q_tiles + p.per_cta - 1) / p.per_cta));
-    flash_fwd_kernel<HD, T><<<grid, FWD_THREADS, smem, stream>>>(tq, tk, tv, p);
+    bmt::launch(flash_fwd_kernel<HD, T>, grid, FWD_THREADS, smem, stream, 1, tq, tk, tv, p);
     bmt_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
@@ -626,6 +628,19 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     static_assert(128 * FEW + 384 * MANY <= 512 * 128, "registers of a block");
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        mbar_init(&sh->kv_full, 1); mbar_init(&sh->do_full, 1); mbar_init(&sh->do_empty, 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(&sh->q_full[i], 1); mbar_init(&sh->q_empty[i], 1); mbar_init(&sh->row_full[i], 1); mbar_init(&sh->row_empty[i], 8); }
+        mbar_init(&sh->s_full, 1); mbar_init(&sh->dp_full, 1); mbar_init(&sh->p_ready, 8); mbar_init(&sh->ds_ready, 8);
+        mbar_init(&sh->dq_full, 1); mbar_init(&sh->dq_empty, 4); mbar_init(&sh->all_done, 1);
+        sh->failed = 0;
+        fence_barrier_init();
+    }
+    if (warp == 13) { tmem_alloc(&sh->tmem_base, 512); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    bmt::after_previous();
     const int kvh = blockIdx.x % p.hk, b = blockIdx.x / p.hk, kt = blockIdx.y;   // under a causal mask the long columns start first
     const int group = p.h / p.hk / p.splits;     // query heads of this CTA
     const int64_t kv0 = (int64_t)kt * TILE;
@@ -640,18 +655,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     walk.settle();
     const bool work = walk.more();
 
-    if (threadIdx.x == 0) {
-        mbar_init(&sh->kv_full, 1); mbar_init(&sh->do_full, 1); mbar_init(&sh->do_empty, 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(&sh->q_full[i], 1); mbar_init(&sh->q_empty[i], 1); mbar_init(&sh->row_full[i], 1); mbar_init(&sh->row_empty[i], 8); }
-        mbar_init(&sh->s_full, 1); mbar_init(&sh->dp_full, 1); mbar_init(&sh->p_ready, 8); mbar_init(&sh->ds_ready, 8);
-        mbar_init(&sh->dq_full, 1); mbar_init(&sh->dq_empty, 4); mbar_init(&sh->all_done, 1);
-        sh->failed = 0;
-        fence_barrier_init();
-    }
-    if (warp == 13) { tmem_alloc(&sh->tmem_base, 512); tmem_relinquish(); }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
 
     if (warp >= 12) {
@@ -976,6 +979,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
 template <typename T>
 __global__ void attn_delta_kernel(const T* o, int64_t o_tok, int64_t o_head, int64_t o_batch, const T* dout, int64_t g_tok, int64_t g_head,
                                   int64_t g_batch, float* delta, float* dq_acc, int64_t rows, int64_t sq, int h, int d) {
+    bmt::after_previous();
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
     const int c = (threadIdx.x & 15) * 8;
     const bool ok = w < rows;
@@ -999,6 +1003,7 @@ __global__ void attn_delta_kernel(const T* o, int64_t o_tok, int64_t o_head, int
 template <typename T>
 __global__ void attn_dq_convert_kernel(const float* acc, T* dq, int64_t q_tok, int64_t q_head, int64_t q_batch, int64_t rows, int64_t sq,
                                        int h, int d) {
+    bmt::after_previous();
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
     const int c = (threadIdx.x & 15) * 8;
     if (w >= rows || c >= d) return;
@@ -1017,6 +1022,7 @@ __global__ void attn_dq_convert_kernel(const float* acc, T* dq, int64_t q_tok, i
 template <typename T>
 __global__ void attn_dkv_sum_kernel(const float* part, int splits, int64_t elems, int64_t sk, int hk, int d, T* dk, int64_t k_tok, int64_t k_head,
                                     int64_t k_batch, T* dv, int64_t v_tok, int64_t v_head, int64_t v_batch) {
+    bmt::after_previous();
     const int64_t vecs = elems / 8;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 2 * vecs) return;
@@ -1068,7 +1074,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
         configured = true;
     }
     dim3 grid((unsigned)(p.hk * batch), (unsigned)p.k_tiles, (unsigned)p.splits);
-    flash_bwd_kernel<HD, T><<<grid, BWD_THREADS, smem, stream>>>(tq, tk, tv, tdo, tdq, p);
+    bmt::launch(flash_bwd_kernel<HD, T>, grid, BWD_THREADS, smem, stream, 1, tq, tk, tv, tdo, tdq, p);
     bmt_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
@@ -1088,7 +1094,7 @@ int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const v
     if ((rc = bmt_tma_map_f32_3d(&tdq, dq_acc, d, sq, batch * h, 32, 32)) != 0) return rc;
     const int64_t rows = batch * sq * h;
     const unsigned row_blocks = (unsigned)((rows * 16 + 255) / 256);
-    attn_delta_kernel<T><<<row_blocks, 256, 0, st>>>((const T*)o, os[0], os[1], os[2], (const T*)dout, gs[0], gs[1], gs[2], (float*)delta,
+    bmt::launch(attn_delta_kernel<T>, row_blocks, 256, 0, st, 1, (const T*)o, os[0], os[1], os[2], (const T*)dout, gs[0], gs[1], gs[2], (float*)delta,
                                                      (float*)dq_acc, rows, sq, h, d);
     AttnBwdParams p;
     memset(&p, 0, sizeof(p));
@@ -1110,11 +1116,11 @@ int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const v
     if (rc != 0) return rc;
     if (p.splits > 1) {
         const int64_t vecs = p.part_elems / 4;   // 8-element vectors of dK and dV
-        attn_dkv_sum_kernel<T><<<(unsigned)((vecs + 255) / 256), 256, 0, st>>>(p.dkv_part, p.splits, p.part_elems, sk, hk, d, (T*)dk, dks[0], dks[1],
+        bmt::launch(attn_dkv_sum_kernel<T>, (unsigned)((vecs + 255) / 256), 256, 0, st, 1, p.dkv_part, p.splits, p.part_elems, sk, hk, d, (T*)dk, dks[0], dks[1],
                                                                               dks[2], (T*)dv, dvs[0], dvs[1], dvs[2]);
         bmt_count_launch(1);
     }
-    attn_dq_convert_kernel<T><<<row_blocks, 256, 0, st>>>((const float*)dq_acc, (T*)dq, dqs[0], dqs[1], dqs[2], rows, sq, h, d);
+    bmt::launch(attn_dq_convert_kernel<T>, row_blocks, 256, 0, st, 1, (const float*)dq_acc, (T*)dq, dqs[0], dqs[1], dqs[2], rows, sq, h, d);
     bmt_count_launch(2);
     return cudaGetLastError() == cudaSuccess ? 0 : -33;
 }
@@ -1173,7 +1179,7 @@ extern "C" int bmt_attn_mask_pack(int64_t batch, int64_t sq, int64_t sk, const v
     if (qt > 65535 || batch > 65535) return -2;
     int64_t t_off, c_off;
     bmt_attn_mask_layout(batch, sq, sk, &t_off, &c_off);
-    attn_mask_pack_kernel<<<dim3((unsigned)kt, (unsigned)qt, (unsigned)batch), MASK_THREADS, 0, (cudaStream_t)stream>>>(
+    bmt::launch(attn_mask_pack_kernel, dim3((unsigned)kt, (unsigned)qt, (unsigned)batch), MASK_THREADS, 0, (cudaStream_t)stream, 1, 
         (const uint8_t*)mask, sq, sk, (uint32_t*)packed, (uint32_t*)((char*)packed + t_off), (uint8_t*)packed + c_off);
     bmt_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -31;

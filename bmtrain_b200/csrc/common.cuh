@@ -63,6 +63,32 @@ template <bool IsMax> __device__ __forceinline__ float block_allreduce(float v, 
     return r;
 }
 
+// ---- dependent launches -------------------------------------------------------------------------------------------------------
+// Kernels launched with `launch` may start while the kernel before them on the stream is still running: their CTAs take the SMs that
+// it leaves, set up what does not touch global memory, and wait in `after_previous` until it has completed and its writes are visible.
+// Every thread of such a kernel calls `after_previous` before its first access to global memory, and after it has allocated what it
+// needs of the SM (tensor memory), since it also lets the next kernel begin.  A GEMM after a GEMM begins 2 us earlier this way
+// (256 x 768 x 256: 6.2 -> 4.8 us from start to start, 1024 x 2560 x 2560: 18.5 -> 16.0).  Not for grids of resident CTAs that stride over
+// their work with several to an SM: they count on being spread evenly, and CTAs that arrive while others still hold SMs pile up
+// on the free ones (RMSNorm 16384 x 5120, both directions: 187 -> 204 us).  Those are launched normally and only let the next begin.
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // SMs of the current device (148 on a B200, also where there is none to ask).
 inline int sm_count() {
     static int sms[64] = {0};

@@ -124,6 +124,7 @@ template <typename T, int U>
 __global__ void __launch_bounds__(256) ce_row_stats_stream_kernel(int64_t m, int64_t n, int trips, const T* __restrict__ x,
                                                                   const int64_t* __restrict__ target, int64_t vocab_start,
                                                                   float* __restrict__ out) {
+    bmt::after_previous();
     constexpr int V = bmt::Vec16<T>::N;
     constexpr float L2E = 1.4426950408889634f;
     __shared__ float sm_m[2][8], sm_s[2][8];
@@ -206,6 +207,7 @@ __global__ void __launch_bounds__(CE_FINISH_THREADS) ce_finish_kernel(int64_t m,
                                                                       const int64_t* __restrict__ target, int64_t ignore_index, int mean,
                                                                       float* __restrict__ lse, float* __restrict__ loss,
                                                                       float* __restrict__ divisor) {
+    bmt::after_previous();
     __shared__ float scratch[33];
     const int64_t first = blockIdx.x * chunk, end = first + chunk < m ? first + chunk : m;
     float sum = 0.f, count = 0.f;
@@ -237,6 +239,7 @@ __global__ void __launch_bounds__(256) ce_backward_kernel(int64_t m, int64_t n, 
                                                           const int64_t* __restrict__ target, const float* __restrict__ lse,
                                                           const float* __restrict__ grad, const float* __restrict__ divisor,
                                                           int64_t vocab_start, int64_t ignore_index, T* __restrict__ out) {
+    bmt::after_previous();
     const int64_t row = blockIdx.x;
     const T* __restrict__ xr = x + row * n;
     T* __restrict__ orow = out + row * n;
@@ -312,7 +315,7 @@ extern "C" int bmt_ce_row_stats(int64_t m, int64_t n, const void* logits, int dt
             if (!per_sm && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ce_row_stats_stream_kernel<T, UU>, 256, 0) != cudaSuccess || per_sm < 1)) \
                 per_sm = 2;                                                                                                    \
             const int64_t cap = (int64_t)148 * per_sm;                                                                         \
-            ce_row_stats_stream_kernel<T, UU><<<(unsigned)(m < cap ? m : cap), 256, 0, s>>>(                                   \
+            bmt::launch(ce_row_stats_stream_kernel<T, UU>, (unsigned)(m < cap ? m : cap), 256, 0, s, 1,                                    \
                 m, n, trips, (const T*)logits, (const int64_t*)target, vocab_start, (float*)out);                              \
         } while (0)
 #define BMT_CE_STREAM_U(T) \
@@ -336,7 +339,7 @@ static int ce_backward(int64_t m, int64_t n, const void* logits, int dtype, cons
     cudaStream_t s = (cudaStream_t)stream;
     const auto run = [&](auto* zero) {
         using T = std::remove_pointer_t<decltype(zero)>;
-        ce_backward_kernel<T><<<(unsigned)m, 256, 0, s>>>(m, n, (const T*)logits, (const int64_t*)target, (const float*)lse, (const float*)grad,
+        bmt::launch(ce_backward_kernel<T>, (unsigned)m, 256, 0, s, 1, m, n, (const T*)logits, (const int64_t*)target, (const float*)lse, (const float*)grad,
                                                           (const float*)divisor, vocab_start, ignore_index, (T*)out);
     };
     if (dtype == BMT_DT_F16) run((__half*)nullptr);
@@ -360,7 +363,7 @@ extern "C" int bmt_ce_reduced_forward(int64_t m, int64_t n, const void* logits, 
     const int64_t share = (m + bmt::sm_count() - 1) / bmt::sm_count();     // a block per SM, of at least 1024 rows
     const int64_t chunk = m <= CE_FINISH_ROWS ? CE_FINISH_ROWS : share > 1024 ? share : 1024;
     const int64_t blocks = m <= CE_FINISH_ROWS ? 1 : (m + chunk - 1) / chunk;
-    ce_finish_kernel<<<(unsigned)blocks, CE_FINISH_THREADS, 0, (cudaStream_t)stream>>>(m, chunk, (float*)scratch, (const int64_t*)target, ignore_index, mean,
+    bmt::launch(ce_finish_kernel, (unsigned)blocks, CE_FINISH_THREADS, 0, (cudaStream_t)stream, 1, m, chunk, (float*)scratch, (const int64_t*)target, ignore_index, mean,
                                                                                        (float*)lse, (float*)loss, (float*)divisor);
     if (blocks > 1) ce_total_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(m, (int)blocks, chunk, (const float*)scratch, mean, (float*)loss, (float*)divisor);
     bmt_count_launch(blocks > 1 ? 2 : 1);

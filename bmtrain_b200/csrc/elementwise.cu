@@ -6,6 +6,7 @@ namespace {
 
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(int64_t rows, int64_t f, const T* __restrict__ x, T* __restrict__ out) {
+    bmt::after_previous();
     const int64_t per_row = f / 8;
     const int64_t total = rows * per_row;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -22,6 +23,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(int64_t rows, int64_t f
 
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(int64_t rows, int64_t f, const T* __restrict__ x, const T* __restrict__ go, T* __restrict__ dx) {
+    bmt::after_previous();
     const int64_t per_row = f / 8;
     const int64_t total = rows * per_row;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -47,6 +49,7 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(int64_t rows, int64_t f
 template <typename T>
 __global__ void __launch_bounds__(256) colsum_kernel(int64_t m, int64_t n, const T* __restrict__ x, T* __restrict__ out, int acc,
                                                      float* __restrict__ scratch, unsigned int* __restrict__ tickets) {
+    bmt::after_previous();
     __shared__ float red[32][65];
     __shared__ unsigned int last_s;
     const int cv = threadIdx.x & 7, lane = threadIdx.x >> 3;
@@ -100,6 +103,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(int64_t m, int64_t n, const
 
 template <typename T>
 __global__ void __launch_bounds__(256) gelu_kernel(int64_t n8, const T* __restrict__ x, T* __restrict__ out) {
+    bmt::after_previous();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (int64_t)gridDim.x * blockDim.x) {
         bmt::Vec16<T> v = bmt::ld16(x + i * 8), o;
 #pragma unroll
@@ -121,6 +125,7 @@ template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(256) rope_qkv_kernel(int64_t batch, int64_t seq, int hk, int g, int d, T* __restrict__ packed,
                                                        int64_t p_tok, int64_t p_batch, T* __restrict__ q, T* __restrict__ k,
                                                        T* __restrict__ v, const float* __restrict__ cs, int64_t pos0) {
+    bmt::after_previous();
     const int half = d / 2, vecs = half / 8, slots = hk * (g + 2);
     const int64_t total = batch * seq * slots * vecs;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -171,8 +176,8 @@ extern "C" int bmt_swiglu_fwd(int64_t rows, int64_t f, const void* x, int dtype,
     if (rows <= 0) return 0;
     if (f % 8 || dtype == BMT_DT_F32) return -3;
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == BMT_DT_F16) swiglu_fwd_kernel<__half><<<grid1d(rows * f / 8), 256, 0, s>>>(rows, f, (const __half*)x, (__half*)out);
-    else swiglu_fwd_kernel<__nv_bfloat16><<<grid1d(rows * f / 8), 256, 0, s>>>(rows, f, (const __nv_bfloat16*)x, (__nv_bfloat16*)out);
+    if (dtype == BMT_DT_F16) bmt::launch(swiglu_fwd_kernel<__half>, grid1d(rows * f / 8), 256, 0, s, 1, rows, f, (const __half*)x, (__half*)out);
+    else bmt::launch(swiglu_fwd_kernel<__nv_bfloat16>, grid1d(rows * f / 8), 256, 0, s, 1, rows, f, (const __nv_bfloat16*)x, (__nv_bfloat16*)out);
     bmt_count_launch(1);
     return (int)cudaGetLastError();
 }
@@ -181,8 +186,8 @@ extern "C" int bmt_swiglu_bwd(int64_t rows, int64_t f, const void* x, const void
     if (rows <= 0) return 0;
     if (f % 8 || dtype == BMT_DT_F32) return -3;
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == BMT_DT_F16) swiglu_bwd_kernel<__half><<<grid1d(rows * f / 8), 256, 0, s>>>(rows, f, (const __half*)x, (const __half*)g, (__half*)dx);
-    else swiglu_bwd_kernel<__nv_bfloat16><<<grid1d(rows * f / 8), 256, 0, s>>>(rows, f, (const __nv_bfloat16*)x, (const __nv_bfloat16*)g, (__nv_bfloat16*)dx);
+    if (dtype == BMT_DT_F16) bmt::launch(swiglu_bwd_kernel<__half>, grid1d(rows * f / 8), 256, 0, s, 1, rows, f, (const __half*)x, (const __half*)g, (__half*)dx);
+    else bmt::launch(swiglu_bwd_kernel<__nv_bfloat16>, grid1d(rows * f / 8), 256, 0, s, 1, rows, f, (const __nv_bfloat16*)x, (const __nv_bfloat16*)g, (__nv_bfloat16*)dx);
     bmt_count_launch(1);
     return (int)cudaGetLastError();
 }
@@ -208,8 +213,8 @@ extern "C" int bmt_colsum_ex(int64_t m, int64_t n, const void* x, int dtype, voi
     const dim3 g((unsigned)cb, (unsigned)splits);
     unsigned int* tickets = (unsigned int*)scratch;
     float* partial = scratch ? (float*)((char*)scratch + 4096) : nullptr;
-    if (dtype == BMT_DT_F16) colsum_kernel<__half><<<g, 256, 0, s>>>(m, n, (const __half*)x, (__half*)out, accumulate, partial, tickets);
-    else colsum_kernel<__nv_bfloat16><<<g, 256, 0, s>>>(m, n, (const __nv_bfloat16*)x, (__nv_bfloat16*)out, accumulate, partial, tickets);
+    if (dtype == BMT_DT_F16) bmt::launch(colsum_kernel<__half>, g, 256, 0, s, 1, m, n, (const __half*)x, (__half*)out, accumulate, partial, tickets);
+    else bmt::launch(colsum_kernel<__nv_bfloat16>, g, 256, 0, s, 1, m, n, (const __nv_bfloat16*)x, (__nv_bfloat16*)out, accumulate, partial, tickets);
     bmt_count_launch(1);
     return (int)cudaGetLastError();
 }
@@ -223,8 +228,8 @@ extern "C" int bmt_gelu_fwd(int64_t n, const void* x, int dtype, void* out, void
     if (n <= 0) return 0;
     if (n % 8 || dtype == BMT_DT_F32) return -3;
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == BMT_DT_F16) gelu_kernel<__half><<<grid1d(n / 8), 256, 0, s>>>(n / 8, (const __half*)x, (__half*)out);
-    else gelu_kernel<__nv_bfloat16><<<grid1d(n / 8), 256, 0, s>>>(n / 8, (const __nv_bfloat16*)x, (__nv_bfloat16*)out);
+    if (dtype == BMT_DT_F16) bmt::launch(gelu_kernel<__half>, grid1d(n / 8), 256, 0, s, 1, n / 8, (const __half*)x, (__half*)out);
+    else bmt::launch(gelu_kernel<__nv_bfloat16>, grid1d(n / 8), 256, 0, s, 1, n / 8, (const __nv_bfloat16*)x, (__nv_bfloat16*)out);
     bmt_count_launch(1);
     return (int)cudaGetLastError();
 }
@@ -241,11 +246,11 @@ extern "C" int bmt_rope_qkv(int64_t batch, int64_t seq, int hk, int g, int d, vo
     const int64_t work = batch * seq * hk * (g + 2) * (d / 16);
     const float* table = (const float*)cos_sin;
     if (dtype == BMT_DT_F16) {
-        if (split) rope_qkv_kernel<__half, true><<<grid1d(work), 256, 0, s>>>(batch, seq, hk, g, d, (__half*)packed, p_tok, p_batch, (__half*)q, (__half*)k, (__half*)v, table, pos0);
-        else rope_qkv_kernel<__half, false><<<grid1d(work), 256, 0, s>>>(batch, seq, hk, g, d, (__half*)packed, p_tok, p_batch, (__half*)q, (__half*)k, (__half*)v, table, pos0);
+        if (split) bmt::launch(rope_qkv_kernel<__half, true>, grid1d(work), 256, 0, s, 1, batch, seq, hk, g, d, (__half*)packed, p_tok, p_batch, (__half*)q, (__half*)k, (__half*)v, table, pos0);
+        else bmt::launch(rope_qkv_kernel<__half, false>, grid1d(work), 256, 0, s, 1, batch, seq, hk, g, d, (__half*)packed, p_tok, p_batch, (__half*)q, (__half*)k, (__half*)v, table, pos0);
     } else {
-        if (split) rope_qkv_kernel<__nv_bfloat16, true><<<grid1d(work), 256, 0, s>>>(batch, seq, hk, g, d, (__nv_bfloat16*)packed, p_tok, p_batch, (__nv_bfloat16*)q, (__nv_bfloat16*)k, (__nv_bfloat16*)v, table, pos0);
-        else rope_qkv_kernel<__nv_bfloat16, false><<<grid1d(work), 256, 0, s>>>(batch, seq, hk, g, d, (__nv_bfloat16*)packed, p_tok, p_batch, (__nv_bfloat16*)q, (__nv_bfloat16*)k, (__nv_bfloat16*)v, table, pos0);
+        if (split) bmt::launch(rope_qkv_kernel<__nv_bfloat16, true>, grid1d(work), 256, 0, s, 1, batch, seq, hk, g, d, (__nv_bfloat16*)packed, p_tok, p_batch, (__nv_bfloat16*)q, (__nv_bfloat16*)k, (__nv_bfloat16*)v, table, pos0);
+        else bmt::launch(rope_qkv_kernel<__nv_bfloat16, false>, grid1d(work), 256, 0, s, 1, batch, seq, hk, g, d, (__nv_bfloat16*)packed, p_tok, p_batch, (__nv_bfloat16*)q, (__nv_bfloat16*)k, (__nv_bfloat16*)v, table, pos0);
     }
     bmt_count_launch(1);
     return (int)cudaGetLastError();

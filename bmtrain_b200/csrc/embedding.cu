@@ -6,6 +6,7 @@ namespace {
 
 template <typename T>
 __global__ void __launch_bounds__(128) emb_fwd_kernel(int64_t d, const int64_t* __restrict__ ids, const T* __restrict__ w, T* __restrict__ out) {
+    bmt::after_previous();
     const int64_t t = blockIdx.x;
     const int64_t id = ids[t];
     T* __restrict__ o = out + t * d;
@@ -42,12 +43,14 @@ EmbScratch emb_scratch(void* base, int64_t tokens, int64_t rows) {
 }
 
 __global__ void __launch_bounds__(256) emb_count_kernel(int64_t tokens, int64_t rows, const int64_t* __restrict__ ids, EmbScratch e) {
+    bmt::after_previous();
     const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (t >= tokens) return;
     const int64_t id = ids[t];
     if (id >= 0 && id < rows) e.rank[t] = atomicAdd(e.count + id, 1);
 }
 __global__ void __launch_bounds__(256) emb_start_kernel(int64_t rows, EmbScratch e) {
+    bmt::after_previous();
     const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (r >= rows) return;
     const int c = e.count[r];
@@ -56,6 +59,7 @@ __global__ void __launch_bounds__(256) emb_start_kernel(int64_t rows, EmbScratch
     if (c > EMB_HOT) e.hot[atomicAdd(e.n_hot, 1)] = (int)r;
 }
 __global__ void __launch_bounds__(256) emb_order_kernel(int64_t tokens, int64_t rows, const int64_t* __restrict__ ids, EmbScratch e) {
+    bmt::after_previous();
     const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (t >= tokens) return;
     const int64_t id = ids[t];
@@ -64,6 +68,7 @@ __global__ void __launch_bounds__(256) emb_order_kernel(int64_t tokens, int64_t 
 // `team` threads (32 .. 256) per row
 template <typename T>
 __global__ void __launch_bounds__(256) emb_rows_kernel(int64_t rows, int64_t d, int team, const T* __restrict__ g, EmbScratch e, T* __restrict__ out) {
+    bmt::after_previous();
     constexpr int V = bmt::Vec16<T>::N;
     const int64_t r = (int64_t)blockIdx.x * (256 / team) + threadIdx.x / team;
     if (r >= rows) return;
@@ -88,6 +93,7 @@ __global__ void __launch_bounds__(256) emb_rows_kernel(int64_t rows, int64_t d, 
 }
 template <typename T>
 __global__ void __launch_bounds__(256) emb_hot_kernel(int64_t d, const T* __restrict__ g, EmbScratch e, T* __restrict__ out) {
+    bmt::after_previous();
     constexpr int V = bmt::Vec16<T>::N;
     __shared__ float part[8][32 * V];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -131,8 +137,8 @@ void launch_rows(int64_t rows, int64_t d, const void* g, const EmbScratch& e, vo
     int team = 32;
     while (team < 256 && (int64_t)team * V < d) team *= 2;
     const int per = 256 / team;
-    emb_rows_kernel<T><<<(unsigned)((rows + per - 1) / per), 256, 0, s>>>(rows, d, team, (const T*)g, e, (T*)out);
-    if (any_hot) emb_hot_kernel<T><<<296, 256, 0, s>>>(d, (const T*)g, e, (T*)out);
+    bmt::launch(emb_rows_kernel<T>, (unsigned)((rows + per - 1) / per), 256, 0, s, 1, rows, d, team, (const T*)g, e, (T*)out);
+    if (any_hot) bmt::launch(emb_hot_kernel<T>, 296, 256, 0, s, 1, d, (const T*)g, e, (T*)out);
 }
 
 }  // namespace
@@ -140,10 +146,10 @@ void launch_rows(int64_t rows, int64_t d, const void* g, const EmbScratch& e, vo
 extern "C" int bmt_embedding_fwd(int64_t tokens, int64_t d, const void* ids, const void* weight, int dtype, void* out, void* stream) {
     if (tokens <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == BMT_DT_F32) { if (d % 4) return -3; emb_fwd_kernel<float><<<(unsigned)tokens, 128, 0, s>>>(d, (const int64_t*)ids, (const float*)weight, (float*)out); }
+    if (dtype == BMT_DT_F32) { if (d % 4) return -3; bmt::launch(emb_fwd_kernel<float>, (unsigned)tokens, 128, 0, s, 1, d, (const int64_t*)ids, (const float*)weight, (float*)out); }
     else { if (d % 8) return -3;
-        if (dtype == BMT_DT_F16) emb_fwd_kernel<__half><<<(unsigned)tokens, 128, 0, s>>>(d, (const int64_t*)ids, (const __half*)weight, (__half*)out);
-        else emb_fwd_kernel<__nv_bfloat16><<<(unsigned)tokens, 128, 0, s>>>(d, (const int64_t*)ids, (const __nv_bfloat16*)weight, (__nv_bfloat16*)out); }
+        if (dtype == BMT_DT_F16) bmt::launch(emb_fwd_kernel<__half>, (unsigned)tokens, 128, 0, s, 1, d, (const int64_t*)ids, (const __half*)weight, (__half*)out);
+        else bmt::launch(emb_fwd_kernel<__nv_bfloat16>, (unsigned)tokens, 128, 0, s, 1, d, (const int64_t*)ids, (const __nv_bfloat16*)weight, (__nv_bfloat16*)out); }
     bmt_count_launch(1);
     return (int)cudaGetLastError();
 }
@@ -160,9 +166,9 @@ extern "C" int bmt_embedding_bwd(int64_t tokens, int64_t d, int64_t rows, const 
     BMT_CUDA_OK(cudaMemsetAsync(e.total, 0, (size_t)(2 + rows) * sizeof(int), s));
     if (tokens > 0) {
         const unsigned tb = (unsigned)((tokens + 255) / 256);
-        emb_count_kernel<<<tb, 256, 0, s>>>(tokens, rows, (const int64_t*)ids, e);
-        emb_start_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, s>>>(rows, e);
-        emb_order_kernel<<<tb, 256, 0, s>>>(tokens, rows, (const int64_t*)ids, e);
+        bmt::launch(emb_count_kernel, tb, 256, 0, s, 1, tokens, rows, (const int64_t*)ids, e);
+        bmt::launch(emb_start_kernel, (unsigned)((rows + 255) / 256), 256, 0, s, 1, rows, e);
+        bmt::launch(emb_order_kernel, tb, 256, 0, s, 1, tokens, rows, (const int64_t*)ids, e);
         bmt_count_launch(3);
     }
     const bool any_hot = tokens > EMB_HOT;

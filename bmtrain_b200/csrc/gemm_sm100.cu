@@ -783,6 +783,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
     __syncthreads();
     if (CTA2) cluster_sync();   // the peer's barriers must be initialised before anything is signalled across
     tc_fence_after();
+    if (FUSED == 0) bmt::after_previous();
     const uint32_t tmem_base = hdr->tmem_base;
 
     const uint64_t t_kernel0 = (FUSED != 0 && threadIdx.x == 0) ? global_ns() : 0;
@@ -1440,6 +1441,19 @@ TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn
     return best_split_cost < best_cost ? best_split : best;
 }
 
+// The choice for a problem costs 2 to 4 us of divisions; a thread keeps its last ones.
+TileChoice planned_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn, int force_bn, int force_cta2, bool split) {
+    struct Plan { int64_t m, n, k, batches; int how, sms; TileChoice tc; };
+    static thread_local Plan plans[256];
+    const int how = 1 + (b_mn ? 1 : 0) + (split ? 2 : 0) + 4 * (force_cta2 + 1) + 16 * force_bn;
+    const uint64_t hash = ((uint64_t)M * 0x9e3779b97f4a7c15ull) ^ ((uint64_t)N * 0xc2b2ae3d27d4eb4full) ^ ((uint64_t)K * 0x165667b19e3779f9ull) ^
+                          ((uint64_t)batches * 0x27d4eb2f165667c5ull) ^ ((uint64_t)how * 0x85ebca77c2b2ae63ull);
+    Plan& p = plans[(hash >> 40) & 255];
+    if (p.how != how || p.m != M || p.n != N || p.k != K || p.batches != batches || p.sms != g_num_sms)
+        p = Plan{M, N, K, batches, how, g_num_sms, pick_tile(M, N, K, batches, b_mn, force_bn, force_cta2, split)};
+    return p.tc;
+}
+
 // Tensor of a scratch: flags of all CTAs, then their slots.
 int64_t sk_bytes(int ctas, int bn) { return (int64_t)ctas * (SK_WARPS * 4 + 128 * ((bn + 31) / 32 * 32) * 4); }
 std::atomic<uint32_t> g_sk_tag{0};
@@ -1496,7 +1510,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) { cudaGetLastError(); split = false; }
     }
-    TileChoice tc = pick_tile(m, n, k, batch_inner * batch_outer, b_major != 0, force_bn, pair_ok ? force_cta2 : 0, split);
+    TileChoice tc = planned_tile(m, n, k, batch_inner * batch_outer, b_major != 0, force_bn, pair_ok ? force_cta2 : 0, split);
     if (fused) g_num_sms += held_back;
     if (tc.bn == 0) tc = pick_tile(m, n, k, batch_inner * batch_outer, b_major != 0, 0, -1, split);  // forced shape not applicable here
     if (tc.bn == 0) return -22;
@@ -1611,22 +1625,13 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     }
     if (!tc.cta2) {
         const unsigned grid = (unsigned)(tc.sk_tiles ? whole_or_split(tiles, g_num_sms, tc) : tiles < g_num_sms ? tiles : g_num_sms);
-        gemm_tcgen05_kernel<false, 0><<<grid, num_threads(0), smem, stream>>>(ma, mb, p, none);
+        const cudaError_t e = bmt::launch(gemm_tcgen05_kernel<false, 0>, grid, num_threads(0), smem, stream, 1, ma, mb, p, none);
         bmt_count_launch(1);
-        return (int)cudaGetLastError();
+        return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
     }
     const int64_t pairs = g_num_sms / 2;
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)(2 * (tc.sk_tiles ? whole_or_split(tiles, pairs, tc) : tiles < pairs ? tiles : pairs)));
-    cfg.blockDim = dim3(num_threads(0));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<true, 0>, ma, mb, p, none);
+    const unsigned grid = (unsigned)(2 * (tc.sk_tiles ? whole_or_split(tiles, pairs, tc) : tiles < pairs ? tiles : pairs));
+    const cudaError_t e = bmt::launch(gemm_tcgen05_kernel<true, 0>, grid, num_threads(0), smem, stream, 2, ma, mb, p, none);
     bmt_count_launch(1);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }

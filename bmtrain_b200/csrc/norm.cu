@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(NT) norm_bwd_kernel(int64_t rows, int d, const
 // Fold the per-CTA partial sums: block = 32 columns x 32 row lanes, rows strided over the lanes, smem tree at the end.
 template <typename T, bool ACC = false>
 __global__ void __launch_bounds__(1024) norm_fold_kernel(int d, int nblk, const float* __restrict__ partial, T* __restrict__ dw, T* __restrict__ db) {
+    bmt::after_previous();
     // ACC: dw / db already hold gradients of earlier passes and are added to
     __shared__ float sa[32][33], sb[32][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -241,6 +242,7 @@ template <typename T, int VPL, int WPR>
 __global__ void __launch_bounds__(NT, VPL <= 4 ? 3 : 2) norm_fwd_stream_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __restrict__ w,
                                                              const T* __restrict__ b, float eps, int rms, T* __restrict__ y,
                                                              float* __restrict__ stats) {
+    bmt::after_previous();
     constexpr int RPC = 8 / WPR;
     __shared__ float ex[2][2][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -333,8 +335,12 @@ void launch_fwd_reg(int64_t rows, int d, const void* x, const void* w, const voi
     if (stream) {
         const int64_t cap = 148 * (VPL <= 4 ? 3 : 2);
         const int64_t grid = groups < cap ? groups : cap;
-        norm_fwd_stream_kernel<T, VPL, WPR><<<(unsigned)grid, NT, 0, s>>>(rows, d, (const T*)x, (const T*)w, (const T*)b, eps, rms,
-                                                                           (T*)y, (float*)stats);
+        if (groups <= cap)      // no striding: see `launch`
+            bmt::launch(norm_fwd_stream_kernel<T, VPL, WPR>, (unsigned)grid, NT, 0, s, 1, rows, d, (const T*)x, (const T*)w, (const T*)b, eps,
+                        rms, (T*)y, (float*)stats);
+        else
+            norm_fwd_stream_kernel<T, VPL, WPR><<<(unsigned)grid, NT, 0, s>>>(rows, d, (const T*)x, (const T*)w, (const T*)b, eps, rms,
+                                                                              (T*)y, (float*)stats);
         return;
     }
     const int64_t grid = groups < 148 * 2 ? groups : 148 * 2;
@@ -400,6 +406,7 @@ template <typename T, int VPL, int WPR, bool RMS>
 __global__ void __launch_bounds__(BwdTeam<WPR>::THREADS, BwdTeam<WPR>::CTAS)
 norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ w,
                        const float* __restrict__ stats, T* __restrict__ dx, float* __restrict__ partial, const T* __restrict__ dres) {
+    bmt::after_previous();
     constexpr int RPC = BwdTeam<WPR>::RPC, WARPS = BwdTeam<WPR>::THREADS / 32;
     extern __shared__ __align__(128) uint8_t ring[];   // stages x {x, dy[, dres]} x RPC rows; 2 * d floats at the end of the kernel
     __shared__ __align__(8) uint64_t full[BWD_STAGES];
@@ -605,8 +612,8 @@ int bwd(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, c
         void* partial, void* dw, void* db, cudaStream_t s, const void* dres = nullptr, bool acc = false) {
     const auto fold = [&](int blocks) {
         const unsigned g = (unsigned)((d + 31) / 32);
-        if (acc) norm_fold_kernel<T, true><<<g, dim3(32, 32), 0, s>>>((int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
-        else norm_fold_kernel<T><<<g, dim3(32, 32), 0, s>>>((int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
+        if (acc) bmt::launch(norm_fold_kernel<T, true>, g, dim3(32, 32), 0, s, 1, (int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
+        else bmt::launch(norm_fold_kernel<T>, g, dim3(32, 32), 0, s, 1, (int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
     };
     static const bool use_reg = [] { const char* e = getenv("BMT_NORM_STAGED"); return !(e && atoi(e) == 1); }();
     if (use_reg && d <= 16384 && !(rms && db)) {
