@@ -197,6 +197,10 @@ class _Bucket:
             self._layout = (sizes, gaps, where)
         return self._layout
 
+    def views_current(self) -> bool:
+        data = self.storage.data
+        return self._views_of == (data.data_ptr(), data.dtype, data.numel())
+
     def _refresh_views(self) -> None:
         data = self.storage.data
         key = (data.data_ptr(), data.dtype, data.numel())
@@ -294,7 +298,14 @@ class _BlockFunction(torch.autograd.Function):
         ctx.arg_spec = arg_spec
         ctx.req = [t.requires_grad for t in tensors]
         ctx.checkpoint = block._use_checkpoint and not debug.get("_inspect_tensor", False)
-        block._enter_forward(_fill(arg_spec, tensors), in_place=block._may_run_in_place())
+        args = _fill(arg_spec, tensors)
+        plain = ctx.checkpoint and only_reads_parameters(block._module)
+        native = block._native_module(args, plain)
+        if native is not None:
+            ctx.inputs, ctx.out_spec, ctx.rng = tensors, None, None       # this package's blocks draw no random numbers
+            block._last_out_spec = None
+            return (block._native_forward(native, args),)
+        block._enter_forward(args, in_place=block._may_run_in_place(plain))
         if ctx.checkpoint:
             ctx.rng = _rng_state()
             ctx.inputs = tensors
@@ -319,11 +330,20 @@ class _BlockFunction(torch.autograd.Function):
     def backward(ctx, *grad_outs):
         block: Block = ctx.block
         plain = only_reads_parameters(block._module)
+        if ctx.checkpoint and len(grad_outs) == 1 and grad_outs[0] is not None:
+            args = _fill(ctx.arg_spec, ctx.inputs)
+            native = block._native_module(args, plain, training=True)
+            if native is not None:
+                dx = block._native_backward(native, args, grad_outs[0])
+                req = ctx.req
+                ctx.inputs = None
+                # the hidden state is the first tensor of the arguments; masks get no gradient
+                return (None, None, None) + tuple(dx if i == 0 and r else None for i, r in enumerate(req))
         block._enter_backward(_fill(ctx.arg_spec, ctx.inputs) if ctx.checkpoint else None,
                               in_place=plain and ctx.checkpoint and block._may_run_in_place(plain), attach=not plain)
         if ctx.checkpoint:
             detached = [t.detach().requires_grad_(r) for t, r in zip(ctx.inputs, ctx.req)]
-            with _restore_rng(ctx.rng), torch.enable_grad():
+            with _restore_rng(ctx.rng if ctx.rng is not None else _rng_state()), torch.enable_grad():
                 out = block._module(*_fill(ctx.arg_spec, detached))
             graph_out, _ = _flatten_out(out)
         else:
@@ -379,6 +399,7 @@ class Block(torch.nn.Module):
         self._mode = mode
         self._micro_idx = 0
         self._resident = False
+        self._pointing = True       # parameters may point at something else than the local partition
         self._need_release = True
         self.all_input_no_grad = False
         self.all_param_no_grad = False
@@ -616,9 +637,12 @@ class Block(torch.nn.Module):
             parts = b.full.split_with_sizes(sizes)
             for s, i in zip(b.slots, where):
                 s.param.data = parts[i].view(s.shape)
-        self._resident = True
+        self._resident = self._pointing = True
 
     def _point_to_local(self) -> None:
+        if not self._pointing and all(b.views_current() for b in self._buckets.values()):
+            return                               # they have not been made to point anywhere else
+        self._pointing = False
         for b in self._buckets.values():
             for s, view in zip(b.slots, b.local_views()):
                 s.param.data = view
@@ -826,6 +850,62 @@ class Block(torch.nn.Module):
                 and all(b.comm.size == 1 for b in self._buckets.values())
                 and (only_reads_parameters(self._module) if plain is None else plain))
 
+    # A block of known code with a native executor (``models/gpt.py``, ``models/llama.py``: ``_bmt_native_*``) is not run through its
+    # modules: the executor gets addresses inside the gathered buffer and inside the gradient buffer.  There is no autograd graph inside
+    # the block, no parameter is made to point at gathered values, and the recomputation leaves out what only the output needs.  A
+    # block of the benchmark model cost the host 600 us a training step through modules and autograd.
+    def _native_module(self, args, plain: bool, training: bool = False):
+        """(inner module, bucket, slots in the executor's order) if the module's native executor may compute this pass, else None.  One
+        rank, one bucket with exactly the executor's parameters, values nobody holds on to (``_may_run_in_place``); ``training``: every
+        parameter gets a gradient."""
+        mod = self._module
+        takes = getattr(type(mod), "_bmt_native_takes", None)
+        if takes is None or not plain or self._mode == "PIPE" or len(self._buckets) != 1 or not self._may_run_in_place(plain):
+            return None
+        (b,) = self._buckets.values()
+        if b.full is not None or b.full_grad is not None or not args or getattr(args[0], "dtype", None) != b.dtype:
+            return None
+        params = takes(mod, *args)
+        if params is None or len(params) != len(b.slots):
+            return None
+        slots = []
+        for p in params:
+            ref = getattr(p, "_bmt_grad_slot", None)
+            slot = None if ref is None else ref()
+            if slot is None or slot.param is not p or slot.bucket() is not b or (training and not p.requires_grad):
+                return None
+            slots.append(slot)
+        return mod, b, slots
+
+    def _native_pass(self, native, args):
+        """The executor's pass, on the gathered values."""
+        mod, b, slots = native
+        self._begin_gather(in_place=True)
+        if b.work is not None:
+            b.work.wait()
+            b.work = None
+        base, size = b.full.data_ptr(), b.full.element_size()
+        return mod._bmt_native_pass([base + s.offset * size for s in slots], *args)
+
+    def _native_forward(self, native, args):
+        b = native[1]
+        try:
+            return self._native_pass(native, args).forward()
+        finally:
+            b.full = b.work = None
+
+    def _native_backward(self, native, args, grad_out):
+        _, b, slots = native
+        run = self._native_pass(native, args)
+        self._prepare_grads(attach=False)
+        run.recompute()
+        size = b.full_grad.element_size()
+        dx = run.backward(grad_out.contiguous(), [b.full_grad_ptr + s.offset * size for s in slots])
+        for s in slots:
+            s.written = True
+        self._exit_backward()
+        return dx
+
     def _enter_forward(self, args=None, in_place: bool = False) -> None:
         self._ensure_gathered(args, in_place=in_place)
         nxt = self.next_module()
@@ -890,7 +970,11 @@ class Block(torch.nn.Module):
 
         if not self._grad_mode:
             # nothing to differentiate: gather, run once, release
-            self._enter_forward(in_place=self._may_run_in_place())
+            plain = only_reads_parameters(self._module)
+            native = self._native_module(args, plain)
+            if native is not None:
+                return self._native_forward(native, args)
+            self._enter_forward(in_place=self._may_run_in_place(plain))
             try:
                 out = self._module(*args)
             finally:
@@ -910,10 +994,13 @@ class Block(torch.nn.Module):
     def __setattr__(self, name, value):
         object.__setattr__(self, name, value)
 
-    def __getattribute__(self, name: str):
-        if name == "_parameters":
-            return object.__getattribute__(self, "_module")._parameters
-        return super().__getattribute__(name)
+    @property
+    def _parameters(self):
+        return object.__getattribute__(self, "_module")._parameters
+
+    @_parameters.setter
+    def _parameters(self, value):
+        self.__dict__["_parameters"] = value      # nn.Module's own, empty
 
     def __delattr__(self, name):
         object.__delattr__(self, name)

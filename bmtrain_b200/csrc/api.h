@@ -99,6 +99,7 @@ typedef struct {
     const void* residual; int64_t ldr;                                // + residual (m x n, operand dtype)
     const void* aux; int64_t ld_aux; int aux_mode;                    // 1: *= (aux > 0), 2: *= gelu'(aux)
     void* scratch; int64_t scratch_bytes;                             // optional: bmt_gemm_scratch_bytes(), the start of it zeros
+    int round_first;                                                  // the product is rounded to C's type before the residual is added
 } BmtGemmDesc;
 // Fused GEMM + collective kernels launched from now on leave `n` SMs (even, at most 64) out of their grids, so that a kernel
 // of another parallel dimension can start while their CTAs wait for other ranks; 0 restores full grids.
@@ -174,6 +175,55 @@ typedef struct {
 int bmt_gpt_block_forward(const BmtGptBlock* blk, void* stream);
 int bmt_gpt_block_forward_steps(const BmtGptBlock* blk, int first_step, int last_step, void* stream);
 int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockGrad* g, void* stream);
+
+// ---- whole Llama-shaped block (RMSNorm, rotary embedding, grouped-query attention, SwiGLU; no biases) --------------------------
+// h1 = x + out(attention(rope(qkv(RMS1(x))))),  y = h1 + w_out(silu(gate) * up),  (gate, up) = gate_up(RMS2(h1))
+typedef struct {
+    int64_t batch, seq, d_model, n_heads, n_kv, d_head, d_ff;
+    int dtype;       // 0 fp16, 1 bf16
+    float eps1, eps2;
+    int reserved;
+    const void *ln1_w, *qkv_w, *out_w, *ln2_w, *gate_up_w, *w_out;
+    const void* x;       // (T, d_model)
+    void* y;             // (T, d_model)
+    const void* rope;    // (cos, sin) table of bmt_rope_qkv, positions from 0
+    // what backward reads
+    void* ln1;           // (T, d)
+    void* stats1;        // (2, T) fp32
+    void* q;             // (batch, seq, n_heads, d_head), rotated
+    void* k;             // (batch, seq, n_kv, d_head), rotated
+    void* v;             // (batch, seq, n_kv, d_head)
+    void* ctx;           // (T, n_heads * d_head)
+    void* lse;           // (batch, n_heads, seq) fp32
+    void* h1;            // (T, d)
+    void* ln2;           // (T, d)
+    void* stats2;        // (2, T) fp32
+    void* gate_up;       // (T, 2 d_ff)
+    void* ff;            // (T, d_ff)
+    void* packed;        // (T, (n_heads + 2 n_kv) * d_head): work space of the forward
+    void* gemm_scratch; int64_t gemm_scratch_bytes;     // BmtGemmDesc.scratch
+} BmtLlamaBlock;
+typedef struct {
+    const void* dy;      // (T, d)
+    void* dx;            // (T, d)
+    void *d_ln1_w, *d_qkv_w, *d_out_w, *d_ln2_w, *d_gate_up_w, *d_w_out;
+    // work space
+    void* d_ff;          // (T, d_ff)
+    void* d_gate_up;     // (T, 2 d_ff)
+    void* d_ln;          // (T, d)
+    void* d_h1;          // (T, d)
+    void* d_ctx;         // (T, n_heads * d_head)
+    void *dq, *dk, *dv;  // like q, k, v
+    void* d_packed;      // like packed
+    void* norm_partial;  // (2, nblk, d) fp32
+    void* dq_acc;        // batch * seq * n_heads * d_head fp32
+    void* delta;         // batch * n_heads * seq fp32
+    void* dkv_part;      // bmt_flash_attn_bwd_parts floats, or NULL
+    int64_t nblk;
+} BmtLlamaBlockGrad;
+// last_step 8 leaves out the GEMM that computes y (a recomputation for backward)
+int bmt_llama_block_forward(const BmtLlamaBlock* blk, int last_step, void* stream);
+int bmt_llama_block_backward(const BmtLlamaBlock* blk, const BmtLlamaBlockGrad* g, void* stream);
 
 // ---- peer memory (one NVLink domain) ------------------------------------------------------------------------------
 int bmt_symm_alloc(int64_t bytes, void** out);

@@ -1,4 +1,4 @@
-// Native executor for one pre-LN GPT block: the whole forward (9 launches) or backward (21 launches) of a
+// Native executors for whole transformer blocks: pre-LN GPT and, below, the Llama-shaped one.  GPT: the whole forward (9 launches) or backward (21 launches) of a
 // transformer layer is issued from C++ by a single call, so the host cost per layer is a few microseconds instead
 // of one Python/autograd round trip per operator.  Every contraction goes to the tcgen05 GEMM (gemm_sm100.cu) with
 // fused epilogues: bias, ReLU, residual add, ReLU-mask / GELU-derivative on the dgrad path.
@@ -226,5 +226,87 @@ extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockG
     // dx = d_h1 + LN1'(d_ln1)
     RUN(bmt_norm_bwd_ex(q.T, q.d, k.x, w.d_ln2, k.ln1_w, k.stats1, 0, dt, w.nblk, w.dx, w.norm_partial, w.d_ln1_w, w.d_ln1_b,
                         w.d_h1, w.acc_small, stream));
+    return 0;
+}
+
+// ------------------------------------------------------------------------------------------------- Llama-shaped block
+// 9 launches forward, 16 to 17 backward.  The residual additions happen in the epilogues of the projections and in the norms'
+// backward (as operators of their own: six passes over (T, d) per block and step, 4 % of a block at 2048 x 8192).
+namespace {
+
+struct LlamaDims { int64_t T, d, h, hk, dh, hd, kd, qkv, dff; };
+LlamaDims dims_of(const BmtLlamaBlock& k) {
+    LlamaDims q;
+    q.T = k.batch * k.seq; q.d = k.d_model; q.h = k.n_heads; q.hk = k.n_kv; q.dh = k.d_head; q.hd = q.h * q.dh; q.kd = q.hk * q.dh;
+    q.qkv = q.hd + 2 * q.kd; q.dff = k.d_ff;
+    return q;
+}
+
+}  // namespace
+
+extern "C" int bmt_llama_block_forward(const BmtLlamaBlock* blk, int last_step, void* stream) {
+    const BmtLlamaBlock& k = *blk;
+    const LlamaDims q = dims_of(k);
+    const int dt = k.dtype;
+    auto gemm = [&](BmtGemmDesc g) {
+        g.scratch = k.gemm_scratch; g.scratch_bytes = k.gemm_scratch_bytes;
+        return bmt_gemm_ex(&g, stream);
+    };
+    RUN(bmt_norm_fwd(q.T, q.d, k.x, k.ln1_w, nullptr, k.eps1, 1, dt, k.ln1, k.stats1, stream));
+    RUN(gemm(plain(q.T, q.qkv, q.d, k.ln1, q.d, 0, k.qkv_w, q.d, 0, k.packed, q.qkv, dt)));
+    RUN(bmt_rope_qkv(k.batch, k.seq, (int)q.hk, (int)(q.h / q.hk), (int)q.dh, k.packed, q.qkv, k.seq * q.qkv, k.q, k.k, k.v, k.rope, 0, 1, dt,
+                     stream));
+    const int64_t qs[3] = {q.hd, q.dh, k.seq * q.hd}, ks[3] = {q.kd, q.dh, k.seq * q.kd};
+    RUN(bmt_flash_attn_fwd(k.batch, k.seq, k.seq, (int)q.h, (int)q.hk, (int)q.dh, k.q, qs, k.k, ks, k.v, ks, k.ctx, qs, k.lse,
+                           1.f / sqrtf((float)q.dh), 1, nullptr, nullptr, nullptr, dt, stream));
+    {
+        BmtGemmDesc g = plain(q.T, q.d, q.hd, k.ctx, q.hd, 0, k.out_w, q.hd, 0, k.h1, q.d, dt);
+        g.residual = k.x; g.ldr = q.d; g.round_first = 1;      // the modules round the projection, and so does this
+        RUN(gemm(g));
+    }
+    RUN(bmt_norm_fwd(q.T, q.d, k.h1, k.ln2_w, nullptr, k.eps2, 1, dt, k.ln2, k.stats2, stream));
+    RUN(gemm(plain(q.T, 2 * q.dff, q.d, k.ln2, q.d, 0, k.gate_up_w, q.d, 0, k.gate_up, 2 * q.dff, dt)));
+    RUN(bmt_swiglu_fwd(q.T, q.dff, k.gate_up, dt, k.ff, stream));
+    if (last_step >= 9) {
+        BmtGemmDesc g = plain(q.T, q.d, q.dff, k.ff, q.dff, 0, k.w_out, q.dff, 0, k.y, q.d, dt);
+        g.residual = k.h1; g.ldr = q.d; g.round_first = 1;
+        RUN(gemm(g));
+    }
+    return 0;
+}
+
+extern "C" int bmt_llama_block_backward(const BmtLlamaBlock* blk, const BmtLlamaBlockGrad* grad, void* stream) {
+    const BmtLlamaBlock& k = *blk;
+    const BmtLlamaBlockGrad& w = *grad;
+    const LlamaDims q = dims_of(k);
+    const int dt = k.dtype;
+    auto gemm = [&](BmtGemmDesc g) {
+        g.scratch = k.gemm_scratch; g.scratch_bytes = k.gemm_scratch_bytes;
+        return bmt_gemm_ex(&g, stream);
+    };
+    // (T, n) gradient times an (n, m) weight; transposed (T, n) gradient times the (T, m) input of the layer
+    auto dgrad = [&](const void* dy, int64_t n, const void* weight, int64_t m, void* dx) {
+        return gemm(plain(q.T, m, n, dy, n, 0, weight, m, 1, dx, m, dt));
+    };
+    auto wgrad = [&](const void* dy, int64_t n, const void* x, int64_t m, void* dw) {
+        return gemm(plain(n, m, q.T, dy, n, 1, x, m, 1, dw, m, dt));
+    };
+    RUN(dgrad(w.dy, q.d, k.w_out, q.dff, w.d_ff));
+    RUN(wgrad(w.dy, q.d, k.ff, q.dff, w.d_w_out));
+    RUN(bmt_swiglu_bwd(q.T, q.dff, k.gate_up, w.d_ff, dt, w.d_gate_up, stream));
+    RUN(dgrad(w.d_gate_up, 2 * q.dff, k.gate_up_w, q.d, w.d_ln));
+    RUN(wgrad(w.d_gate_up, 2 * q.dff, k.ln2, q.d, w.d_gate_up_w));
+    RUN(bmt_norm_bwd_ex(q.T, q.d, k.h1, w.d_ln, k.ln2_w, k.stats2, 1, dt, (int)w.nblk, w.d_h1, w.norm_partial, w.d_ln2_w, nullptr, w.dy, 0, stream));
+    RUN(dgrad(w.d_h1, q.d, k.out_w, q.hd, w.d_ctx));
+    RUN(wgrad(w.d_h1, q.d, k.ctx, q.hd, w.d_out_w));
+    const int64_t qs[3] = {q.hd, q.dh, k.seq * q.hd}, ks[3] = {q.kd, q.dh, k.seq * q.kd};
+    RUN(bmt_flash_attn_bwd(k.batch, k.seq, k.seq, (int)q.h, (int)q.hk, (int)q.dh, k.q, qs, k.k, ks, k.v, ks, k.ctx, qs, w.d_ctx, qs, k.lse, w.dq,
+                           qs, w.dk, ks, w.dv, ks, w.dq_acc, w.delta, 1.f / sqrtf((float)q.dh), 1, nullptr, nullptr, nullptr, w.dkv_part, dt,
+                           stream));
+    RUN(bmt_rope_qkv(k.batch, k.seq, (int)q.hk, (int)(q.h / q.hk), (int)q.dh, w.d_packed, q.qkv, k.seq * q.qkv, w.dq, w.dk, w.dv, k.rope, 0, 0, dt,
+                     stream));
+    RUN(dgrad(w.d_packed, q.qkv, k.qkv_w, q.d, w.d_ln));
+    RUN(wgrad(w.d_packed, q.qkv, k.ln1, q.d, w.d_qkv_w));
+    RUN(bmt_norm_bwd_ex(q.T, q.d, k.x, w.d_ln, k.ln1_w, k.stats1, 1, dt, (int)w.nblk, w.dx, w.norm_partial, w.d_ln1_w, nullptr, w.d_h1, 0, stream));
     return 0;
 }

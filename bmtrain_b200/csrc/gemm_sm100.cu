@@ -73,6 +73,7 @@ struct GemmParams {
     uint32_t idesc;
     const void* residual;  // optional (M x N, operand dtype, row pitch ldr): added after bias / activation
     int64_t ldr;
+    int round_first;       // the product is rounded to C's type before the residual is added, as two operators do it
     const void* aux;       // optional (M x N, operand dtype, row pitch ld_aux) for the multiplicative epilogues
     int64_t ld_aux;
     int aux_mode;          // 0 none, 1: out *= (aux > 0)  (ReLU backward), 2: out *= gelu'(aux)
@@ -451,7 +452,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, con
                 unpack8<T>(cur[it], e);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    v[it][i] = EXTRA == 1 ? v[it][i] + e[i] : EXTRA == 2 ? (e[i] > 0.f ? v[it][i] : 0.f) : v[it][i] * gelu_grad_f(e[i]);
+                    v[it][i] = EXTRA == 1 ? (p.round_first ? bmt::Cvt<T>::to_f(bmt::Cvt<T>::from_f(v[it][i])) : v[it][i]) + e[i] : EXTRA == 2 ? (e[i] > 0.f ? v[it][i] : 0.f) : v[it][i] * gelu_grad_f(e[i]);
             }
             if (col_ok && it * 8 + sub < rows) store8(dst + it * d_step + c * 32, v[it]);
         }
@@ -500,7 +501,7 @@ __device__ __forceinline__ void epilogue_rows_any(const GemmParams& p, TC* cbase
             if (p.residual) {
                 load_row8_dt(p.residual, p.bias_dtype, row * p.ldr + col, n_ok, r_vec, e);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] += e[i];
+                for (int i = 0; i < 8; ++i) v[i] = (p.round_first ? bmt::Cvt<TC>::to_f(bmt::Cvt<TC>::from_f(v[i])) : v[i]) + e[i];
             }
             TC* dst = cbase + row * p.ldc + col;
             if (p.accumulate) {
@@ -1547,7 +1548,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
         const int per_rank = (int)(fused->ag_rows / (BM * ncta));
         while (per_rank % p.group_m) --p.group_m;
     }
-    p.residual = g.residual; p.ldr = g.ldr; p.aux = g.aux; p.ld_aux = g.ld_aux; p.aux_mode = g.aux ? g.aux_mode : 0;
+    p.residual = g.residual; p.ldr = g.ldr; p.round_first = g.residual ? g.round_first : 0; p.aux = g.aux; p.ld_aux = g.ld_aux; p.aux_mode = g.aux ? g.aux_mode : 0;
     if ((p.residual || p.aux_mode) && batch_inner * batch_outer != 1) return -21;  // fused extras are for plain (unbatched) GEMMs
     {
         // the compiled forms of the epilogue move 16-byte vectors of the operand type: every pitch and pointer has to allow it

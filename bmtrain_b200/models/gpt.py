@@ -105,8 +105,34 @@ class TransformerEncoder(DistributedModule):
         return torch.is_tensor(hidden) and self._fused_ok(hidden) and not bmt_inspect.tensor.debug.get("_inspect_tensor", False)
 
     def _fused_ok(self, hidden: torch.Tensor) -> bool:
-        return (hidden.is_cuda and hidden.dim() == 3 and config["tp_size"] == 1 and _FUSED_BLOCK and self.attn.project_qkv.bias is not None
-                and hidden.dtype in (torch.float16, torch.bfloat16) and self.attn.dim_head % 8 == 0)
+        attn = self._modules["attn"]
+        return (hidden.is_cuda and hidden.dim() == 3 and config["tp_size"] == 1 and _FUSED_BLOCK
+                and attn._modules["project_qkv"]._parameters["bias"] is not None
+                and hidden.dtype in (torch.float16, torch.bfloat16) and attn.dim_head % 8 == 0)
+
+    # A ``Block`` whose module is this one, as it stands, has it computed by the native executor without autograd inside (see
+    # ``Block._native_module``): the parameters as addresses in this order, the recomputation and the gradients in one call.
+    def _bmt_native_takes(self, hidden, mask=None, position_bias=None):
+        """The parameters in the executor's order if it takes these arguments, else None."""
+        if not (torch.is_tensor(hidden) and self._fused_ok(hidden) and hidden.numel() > 0 and self._bmt_deferred_gather is None):
+            return None
+        m, a = self._modules, self._modules["attn"]
+        attn, ff, (b, s, d), inner = a._modules, m["ff"]._modules, hidden.shape, a.num_heads * a.dim_head
+        if mask is not None and (not torch.is_tensor(mask) or mask.shape != (b, s, s) or mask.device != hidden.device):
+            return None
+        params = [p for mod in (m["ln_attn"], attn["project_qkv"], attn["project_out"], m["ln_ff"], ff["w_in"], ff["w_out"])
+                  for p in (mod._parameters["weight"], mod._parameters["bias"])]
+        if any(p is None for p in params):
+            return None
+        shapes = [tuple(p._original_shape) for p in params]
+        f = shapes[8][0]
+        return params if shapes == [(d,), (d,), (3 * inner, d), (3 * inner,), (d, inner), (d,), (d,), (d,), (f, d), (f,), (d, f), (d,)] else None
+
+    def _bmt_native_pass(self, addresses, hidden, mask=None, position_bias=None):
+        m = self._modules
+        a, f = m["attn"], m["ff"]
+        return _gpt_block.Pass(hidden.contiguous(), mask, addresses, a.num_heads, a.dim_head, f._modules["w_in"]._parameters["weight"]._original_shape[0],
+                               f.activation, m["ln_attn"].eps, self.causal)
 
     def forward(self, hidden: torch.Tensor, mask: Optional[torch.Tensor] = None, position_bias=None):
         bmt_inspect.record_tensor(hidden, "hidden")

@@ -7,6 +7,7 @@ configurations need one.  Built from the same sharded-parameter modules as
 from __future__ import annotations
 
 import math
+import os
 from typing import Optional
 
 import torch
@@ -17,6 +18,10 @@ from ..layer import DistributedModule, reads_parameters_only
 from ..nn import ColumnParallelLinear, Embedding, Linear, RMSNorm, RowParallelLinear, VPEmbedding
 from ..ops import attention as _attn
 from ..ops import elementwise as _ew
+from ..ops import llama_block as _llama_block
+
+
+_FUSED_BLOCK = os.environ.get("BMT_FUSED_BLOCK", "1") != "0"
 
 
 @reads_parameters_only
@@ -78,6 +83,32 @@ class LlamaBlock(DistributedModule):
         self.attn = LlamaAttention(dim_model, num_heads, num_kv_heads, dim_head, dtype=dtype)
         self.ln_ff = RMSNorm(dim_model, eps=eps, dtype=dtype)
         self.ff = LlamaMLP(dim_model, dim_ff, dtype=dtype)
+
+    # A ``Block`` whose module is this one, as it stands, has it computed by the native executor (see ``Block._native_module``).
+    def _bmt_native_takes(self, hidden):
+        """The parameters in the executor's order if it takes these arguments, else None."""
+        if not (torch.is_tensor(hidden) and hidden.is_cuda and hidden.dim() == 3 and hidden.numel() > 0 and config["tp_size"] == 1
+                and hidden.dtype in (torch.float16, torch.bfloat16) and _FUSED_BLOCK and os.environ.get("BMT_FLASH_ATTN", "1") != "0"):
+            return None
+        m, a = self._modules, self._modules["attn"]
+        attn, ff, d = a._modules, m["ff"]._modules, hidden.shape[-1]
+        linears = (attn["project_qkv"], attn["project_out"], ff["w_gate_up"], ff["w_out"])
+        if any(mod._parameters["bias"] is not None for mod in linears):
+            return None
+        params = [mod._parameters["weight"] for mod in (m["ln_attn"], *linears[:2], m["ln_ff"], *linears[2:])]
+        shapes = [tuple(p._original_shape) for p in params]
+        f = shapes[5][1]
+        if shapes != [(d,), ((a.h + 2 * a.hk) * a.dh, d), (d, a.h * a.dh), (d,), (2 * f, d), (d, f)]:
+            return None
+        # what the kernels take: head dims of the fused attention, rows of the norms, whole 16-byte vectors
+        return params if a.dh % 16 == 0 and a.dh <= 128 and d % 8 == 0 and d <= 16384 and f % 8 == 0 else None
+
+    def _bmt_native_pass(self, addresses, hidden):
+        m = self._modules
+        attn = m["attn"]
+        return _llama_block.Pass(hidden.contiguous(), addresses, attn.h, attn.hk, attn.dh,
+                                 m["ff"]._modules["w_out"]._parameters["weight"]._original_shape[1], m["ln_attn"].eps, m["ln_ff"].eps,
+                                 attn.rope_theta)
 
     def forward(self, hidden: torch.Tensor) -> torch.Tensor:
         hidden = hidden + self.attn(self.ln_attn(hidden))

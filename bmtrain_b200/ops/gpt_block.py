@@ -11,6 +11,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import os
+import struct
 from typing import Optional
 
 import torch
@@ -19,6 +20,7 @@ from . import _native
 from . import attention as _attn
 from . import gemm as _gemm
 from . import grad_slot as _grad_slot
+
 
 _c_void_p, _i64, _int, _f32 = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_float
 
@@ -50,6 +52,13 @@ class _Grad(ctypes.Structure):
         ("dq_acc", _c_void_p), ("delta", _c_void_p),
         ("acc_small", _int),
     ]
+
+
+# The same in one go: packing the block costs the host 2 us, filling the structure field by field 12.
+_BLOCK = struct.Struct("@6q2ifi15Q4Qq8QQqQq")
+_GRAD = struct.Struct("@14Qi4x7Qi4x2Qi4x")
+assert _BLOCK.size == ctypes.sizeof(_Block) and _GRAD.size == ctypes.sizeof(_Grad)
+_WORK = ("d_ff", "d_ln2", "d_h1", "d_ctx", "d_probs", "d_qkv", "norm_partial")
 
 
 _PARAM_NAMES = ("ln1_w", "ln1_b", "qkv_w", "qkv_b", "out_w", "out_b", "ln2_w", "ln2_b", "fc1_w", "fc1_b", "fc2_w", "fc2_b")
@@ -104,34 +113,76 @@ def _work_plan(b, s, d, n_heads, d_head, dff, fused_attn, nblk):
     return _carve(sizes)
 
 
-def _describe(x, y, mask, params, saved, plan, n_heads, d_head, act, eps, causal):
-    """The block as the native executor takes it; ``saved``: address of the buffer that ``plan`` divides."""
-    b, s, d = x.shape
-    work = _gemm.scratch()
-    at = lambda name: saved + plan[name] if name in plan else None  # noqa: E731
-    # fused attention: scores and probabilities never reach memory, one log-sum-exp per row is kept instead
-    return _Block(b, s, d, n_heads, d_head, params[8].shape[0], 0 if x.dtype == torch.float16 else 1, 1 if act == "relu" else 2, eps,
-                  1 if causal else 0, None if mask is None else mask.data_ptr(), *[p.data_ptr() for p in params], x.data_ptr(),
-                  y.data_ptr(), at("ln1"), at("stats1"), at("qkv"), at("probs"), (s + 7) // 8 * 8 if "probs" in plan else 0,
-                  at("ctx"), at("h1"), at("ln2"), at("stats2"), at("ff"), at("pre"), at("lse"), at("mask_packed"),
-                  *work.colsum, *work.gemm)
+class Pass:
+    """One forward (or recomputation) of a block by the native executor and what backward needs of it.  ``addresses``: of the parameters,
+    in the order of ``_PARAM_NAMES``."""
+
+    def __init__(self, x, mask, addresses, n_heads, d_head, d_ff, act, eps, causal):
+        b, s, d = self.shape = x.shape
+        self.x = x
+        self.mask8 = None if mask is None else _as_bytes(mask)
+        self.fused_attn = d_head % 16 == 0 and d_head <= 128 and os.environ.get("BMT_FLASH_ATTN", "1") != "0"
+        self.cfg = (n_heads, d_head, d_ff)
+        self.plan, total = _saved_plan(b, s, d, n_heads, d_head, d_ff, act == "gelu", self.fused_attn, self.mask8 is not None)
+        self.saved = torch.empty(total, dtype=torch.uint8, device=x.device)
+        base = self.saved.data_ptr()
+        at = {name: base + offset for name, offset in self.plan.items()}
+        work = self.scratch = _gemm.scratch()
+        self.addresses = addresses
+        self.head = (b, s, d, n_heads, d_head, d_ff, 0 if x.dtype == torch.float16 else 1, 1 if act == "relu" else 2, eps, 1 if causal else 0,
+                     0 if self.mask8 is None else self.mask8.data_ptr())
+        get = at.get
+        # fused attention: scores and probabilities never reach memory, one log-sum-exp per row is kept instead
+        self.tail = (at["ln1"], at["stats1"], at["qkv"], get("probs", 0), (s + 7) // 8 * 8 if "probs" in at else 0, at["ctx"], at["h1"], at["ln2"],
+                     at["stats2"], at["ff"], get("pre", 0), get("lse", 0), get("mask_packed", 0),
+                     work.colsum[0].value, work.colsum[1].value, work.gemm[0].value, work.gemm[1].value)
+
+    def forward(self) -> torch.Tensor:
+        y = torch.empty_like(self.x)
+        self.run(1, 9, y)
+        return y
+
+    def recompute(self) -> None:
+        """Forward again for ``backward``: without the last GEMM, whose result nothing reads."""
+        self.run(1, 8)
+
+    def describe(self, y: int = 0) -> bytes:
+        return _BLOCK.pack(*self.head, *self.addresses, self.x.data_ptr(), y, *self.tail)
+
+    def run(self, first: int, last: int, y: Optional[torch.Tensor] = None) -> None:
+        """Steps of the forward (``bmt_gpt_block_forward_steps``); the last one, 9, is what computes ``y``."""
+        _native.check(_native.cuda_lib().bmt_gpt_block_forward_steps(self.describe(0 if y is None else y.data_ptr()), first, last,
+                                                                     self.scratch.stream), "GPT block forward")
+
+    def backward(self, dy: torch.Tensor, grads, acc_weights: bool = False, acc_small: bool = False) -> torch.Tensor:
+        """``grads``: addresses for the gradients of the parameters, in their order; ``acc_*``: added to what is there."""
+        b, s, d = self.shape
+        nblk = min(b * s, 296)
+        plan, total = _work_plan(b, s, d, *self.cfg, self.fused_attn, nblk)
+        work = torch.empty(total, dtype=torch.uint8, device=dy.device)
+        base = work.data_ptr()
+        at = lambda name: base + plan[name] if name in plan else 0  # noqa: E731
+        dx = torch.empty_like(self.x)
+        g = _GRAD.pack(dy.data_ptr(), dx.data_ptr(), *grads, 1 if acc_weights else 0, *[at(n) for n in _WORK], nblk, at("dq_acc"), at("delta"),
+                       1 if acc_small else 0)
+        scratch = _gemm.scratch()
+        if scratch is not self.scratch:         # another stream than the forward's
+            self.tail = self.tail[:-4] + (scratch.colsum[0].value, scratch.colsum[1].value, scratch.gemm[0].value, scratch.gemm[1].value)
+        _native.check(_native.cuda_lib().bmt_gpt_block_backward(self.describe(), g, scratch.stream), "GPT block backward")
+        return dx
+
+
 
 
 class GPTBlockFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, mask, n_heads, d_head, act, eps, causal, deferred, *params):
-        lib = _native.cuda_lib()
         x = x.contiguous()
         b, s, d = x.shape
-        dff = params[8].shape[0]
-        mask8 = None if mask is None else _as_bytes(mask)
-        fused_attn = d_head % 16 == 0 and d_head <= 128 and os.environ.get("BMT_FLASH_ATTN", "1") != "0"
-        plan, total = _saved_plan(b, s, d, n_heads, d_head, dff, act == "gelu", fused_attn, mask8 is not None)
-        saved = torch.empty(total, dtype=torch.uint8, device=x.device)
+        run = Pass(x, mask, [p.data_ptr() for p in params], n_heads, d_head, params[8].shape[0], act, eps, causal)
         y = torch.empty_like(x)
-        blk = _describe(x, y, mask8, params, saved.data_ptr(), plan, n_heads, d_head, act, eps, causal)
         if deferred is None:
-            _native.check(lib.bmt_gpt_block_forward(ctypes.byref(blk), _native.stream_handle()), "GPT block forward")
+            run.run(1, 9, y)
         else:
             # the block's parameters are still on their way: norms and biases first; the QKV weight is gathered by the GEMM
             # that consumes it; the other big weights travel on the peer stream and have the attention core's duration to
@@ -140,12 +191,13 @@ class GPTBlockFunction(torch.autograd.Function):
             from ..parallel import fused_ops
 
             T, hd = b * s, n_heads * d_head
+            plan, saved = run.plan, run.saved
             ln1 = saved[plan["ln1"]:plan["ln1"] + 2 * T * d].view(x.dtype).view(T, d)
             qkv = saved[plan["qkv"]:plan["qkv"] + 6 * T * hd].view(x.dtype).view(T, 3 * hd)
 
             cur = torch.cuda.current_stream()
             cur.wait_event(deferred["ev_small"])
-            _native.check(lib.bmt_gpt_block_forward_steps(ctypes.byref(blk), 1, 1, _native.stream_handle()), "GPT block forward")
+            run.run(1, 1, y)
             when = os.environ.get("BMT_REST_PUSH") or ("before" if deferred["bucket"].comm.size <= 2 else "after")
             if when == "before":
                 ev_rest = deferred["push_rest"]()
@@ -155,58 +207,43 @@ class GPTBlockFunction(torch.autograd.Function):
                 ev_gemm = torch.cuda.Event()
                 ev_gemm.record(cur)
                 ev_rest = deferred["push_rest"](ev_gemm)
-            _native.check(lib.bmt_gpt_block_forward_steps(ctypes.byref(blk), 3, 5, _native.stream_handle()), "GPT block forward")
+            run.run(3, 5, y)
             cur.wait_event(ev_rest)
-            _native.check(lib.bmt_gpt_block_forward_steps(ctypes.byref(blk), 6, 9, _native.stream_handle()), "GPT block forward")
-        ctx.saved, ctx.plan, ctx.x, ctx.mask8, ctx.params = saved, plan, x, mask8, params
-        ctx.cfg = (n_heads, d_head, act, eps, causal, fused_attn)
+            run.run(6, 9, y)
+        ctx.run, ctx.params = run, params
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        lib = _native.cuda_lib()
-        x, saved, params = ctx.x, ctx.saved, ctx.params
-        n_heads, d_head, act, eps, causal, fused_attn = ctx.cfg
-        b, s, d = x.shape
-        dev, dt = x.device, x.dtype
+        run, params = ctx.run, ctx.params
+        dt = run.x.dtype
         dy = dy.contiguous()
-        # (the forward output's pointer is not read by backward)
-        blk = _describe(x, dy, ctx.mask8, params, saved.data_ptr(), ctx.plan, n_heads, d_head, act, eps, causal)
-        g = _Grad()
-        dx = torch.empty_like(x)
-        g.dy, g.dx = dy.data_ptr(), dx.data_ptr()
+        run.addresses = [p.data_ptr() for p in params]
+
         # gradients of the parameters go straight into the owning block's gradient buffer, or accumulate in place when the
         # owner attached same-dtype gradient buffers (no tensor goes back to autograd for them then)
         def attached(p):
             return (p.is_leaf and p.requires_grad and p.grad is not None and p.grad.dtype == dt and p.grad.is_contiguous()
                     and not _grad_slot.watched(p))
 
-        grads = {}
-        for names, flag in ((_WEIGHTS, "acc_w"), (_SMALL, "acc_small")):
+        grads, where, acc = {}, {}, {}
+        for names in (_WEIGHTS, _SMALL):
             mine = [(name, p) for name, p in zip(_PARAM_NAMES, params) if name in names]
             slots = [_grad_slot.find(p) if p.dtype == dt else None for _, p in mine]
             if all(s is not None for s in slots) and len({s.written for s in slots}) == 1:
                 # the owning ZeRO block's gradient buffer: written on first use, added to afterwards
-                setattr(g, flag, 1 if slots[0].written else 0)
+                acc[names] = slots[0].written
                 for (name, _), slot in zip(mine, slots):
-                    setattr(g, "d_" + name, slot.grad_ptr())
+                    where[name] = slot.grad_ptr()
                     slot.written = True
                 continue
-            acc = all(attached(p) for _, p in mine)
-            setattr(g, flag, 1 if acc else 0)
+            acc[names] = all(attached(p) for _, p in mine)
             for name, p in mine:
-                if not acc:
+                if not acc[names]:
                     grads[name] = torch.empty_like(p)
-                setattr(g, "d_" + name, (p.grad if acc else grads[name]).data_ptr())
-        nblk = min(b * s, 296)
-        plan, total = _work_plan(b, s, d, n_heads, d_head, params[8].shape[0], fused_attn, nblk)
-        work = torch.empty(total, dtype=torch.uint8, device=dev)
-        base = work.data_ptr()
-        for name, at in plan.items():
-            setattr(g, name, base + at)
-        g.nblk = nblk
-        _native.check(lib.bmt_gpt_block_backward(ctypes.byref(blk), ctypes.byref(g), _native.stream_handle()), "GPT block backward")
-        ctx.saved = None
+                where[name] = (p.grad if acc[names] else grads[name]).data_ptr()
+        dx = run.backward(dy, [where[n] for n in _PARAM_NAMES], acc[_WEIGHTS], acc[_SMALL])
+        ctx.run = None
         out = [grads.get(name) if p.requires_grad else None for name, p in zip(_PARAM_NAMES, params)]
         return (dx, None, None, None, None, None, None, None) + tuple(out)
 

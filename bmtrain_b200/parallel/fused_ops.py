@@ -42,7 +42,7 @@ class _GemmDesc(ctypes.Structure):
         ("batch_inner", _i64), ("batch_outer", _i64), ("b_inner_div", _i64),
         ("bias", _c_void_p), ("act", _int), ("accumulate", _int), ("alpha", _f32), ("ab_dtype", _int),
         ("residual", _c_void_p), ("ldr", _i64), ("aux", _c_void_p), ("ld_aux", _i64), ("aux_mode", _int),
-        ("scratch", _c_void_p), ("scratch_bytes", _i64),
+        ("scratch", _c_void_p), ("scratch_bytes", _i64), ("round_first", _int),
     ]
 
 

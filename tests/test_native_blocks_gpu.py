@@ -1,0 +1,100 @@
+"""Blocks computed by the native executors against the same blocks run through their modules: outputs, gradients of the input and of
+every parameter, with recomputation; what makes a block go through its modules again."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+_UNIT = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+
+
+def _llama(bmt, dtype, dim, heads, kv, dh, ff):
+    from bmtrain_b200.models.llama import LlamaBlock
+
+    return LlamaBlock(dim, heads, kv, dh, ff, dtype=dtype)
+
+
+def _gpt(bmt, dtype, dim, heads, dh, ff, act, causal):
+    from bmtrain_b200.models.gpt import TransformerEncoder
+
+    return TransformerEncoder(dim, dh, heads, ff, True, dtype, act, causal=causal)
+
+
+def _step(block, args, gy):
+    x = args[0].detach().clone().requires_grad_()
+    y = block(x, *args[1:])
+    y.backward(gy)
+    grads = {n: p.grad.clone() for n, p in block.named_parameters()}
+    for b in block._buckets.values():
+        b.storage.grad = None
+    for p in block.parameters():
+        p.grad = None
+    return y.detach(), x.grad, grads
+
+
+CASES = [("llama", dict(dim=256, heads=4, kv=4, dh=64, ff=704), (2, 128)), ("llama", dict(dim=264, heads=3, kv=1, dh=80, ff=328), (1, 77)),
+         ("llama", dict(dim=512, heads=8, kv=2, dh=128, ff=1024), (3, 200)),
+         ("gpt", dict(dim=256, heads=4, dh=64, ff=1024, act="relu", causal=True), (2, 128)),
+         ("gpt", dict(dim=240, heads=3, dh=80, ff=520, act="gelu", causal=False), (2, 77)),
+         ("gpt", dict(dim=256, heads=2, dh=8, ff=256, act="relu", causal=True), (1, 40))]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kind,cfg,tokens", CASES)
+def test_native_block(bmt_gpu, dtype, kind, cfg, tokens, monkeypatch):
+    bmt = bmt_gpu
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    block = bmt.Block((_llama if kind == "llama" else _gpt)(bmt, dtype, **cfg))
+    with torch.no_grad():
+        for name, p in block._module.named_parameters():
+            shape = p._original_shape
+            value = torch.randn(*shape, generator=gen, device="cuda") * (0.1 if len(shape) == 1 else shape[-1] ** -0.5) + (
+                1.0 if len(shape) == 1 and name.endswith("weight") else 0.0)
+            block._load_param(p, value.to(dtype))
+    b, s = tokens
+    x = torch.randn(b, s, cfg["dim"], generator=gen, device="cuda").to(dtype)
+    gy = torch.randn(b, s, cfg["dim"], generator=gen, device="cuda").to(dtype)
+    args = [x]
+    if kind == "gpt" and not cfg["causal"]:
+        mask = torch.rand(b, s, s, generator=gen, device="cuda") < 0.6
+        mask[:, :, 0] = True
+        args.append(mask)
+    calls = []
+    real = type(block)._native_backward
+    monkeypatch.setattr(type(block), "_native_backward", lambda *a: calls.append(1) or real(*a))
+    native = _step(block, args, gy)
+    assert len(calls) == 1
+    again = _step(block, args, gy)
+    assert torch.equal(native[0], again[0])
+    with torch.no_grad():
+        assert torch.equal(block(*args), native[0])
+    monkeypatch.setattr(type(block), "_native_module", lambda *a, **k: None)
+    modules = _step(block, args, gy)
+    assert len(calls) == 2
+    assert torch.equal(native[0], modules[0])              # the same roundings forward
+    # each is a few roundings of 16-bit intermediates away from the exact block; a chain of a dozen of them on either side
+    for a, e in [(native[0], modules[0]), (native[1], modules[1])] + [(native[2][n], modules[2][n]) for n in modules[2]]:
+        assert (a.double() - e.double()).norm() <= 12 * _UNIT[dtype] * e.double().norm() + 1e-6
+    assert set(native[2]) == set(modules[2])
+
+
+def test_hooks_and_partial_training_go_through_the_modules(bmt_gpu):
+    bmt = bmt_gpu
+    block = bmt.Block(_llama(bmt, torch.bfloat16, 256, 4, 4, 64, 512))
+    bmt.init_parameters(block)
+    x = torch.randn(1, 64, 256, device="cuda", dtype=torch.bfloat16)
+    args = [x]
+    assert block._native_module(args, True) is not None
+    seen = []
+    handle = block._module.ff.register_forward_hook(lambda m, i, o: seen.append(o))
+    block(x.requires_grad_()).sum().backward()
+    assert len(seen) == 2                                  # forward and recomputation
+    handle.remove()
+    block(x).sum().backward()
+    assert len(seen) == 2
+    p = block._module.attn.project_out.weight
+    p.requires_grad_(False)
+    from bmtrain_b200.layer import only_reads_parameters
+
+    assert block._native_module(args, only_reads_parameters(block._module), training=True) is None
+    assert block._native_module([x.float()], True) is None
