@@ -20,6 +20,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import math
+import struct
 from typing import Optional
 
 import torch
@@ -50,9 +51,13 @@ def _reference_attention(q, k, v, scale, causal, mask, kv_lens):
     return torch.einsum("bhqk,bkhd->bqhd", p, v.float()).to(q.dtype)
 
 
+_STRIDES = struct.Struct("@3q")
+
+
 def _strides3(t):
-    """{token, head, batch} element strides of a (b, s, h, d) tensor as a ctypes array."""
-    return (ctypes.c_int64 * 3)(t.stride(1), t.stride(2), t.stride(0))
+    """{token, head, batch} element strides of a (b, s, h, d) tensor as three int64 in memory."""
+    batch, token, head, _ = t.stride()
+    return _STRIDES.pack(token, head, batch)
 
 
 def flash_usable(q, k, v) -> bool:
@@ -101,27 +106,26 @@ def pack_mask(mask8: Optional[torch.Tensor], b: int, sq: int, sk: int) -> Option
 def _mask_parts(packed, b, sq, sk):
     """Pointers to the three parts of a packed mask (null without one)."""
     if packed is None:
-        return (ctypes.c_void_p(0),) * 3
+        return 0, 0, 0
     _, by_key, classes = packed_mask_layout(b, sq, sk)
     at = packed.data_ptr()
-    return ctypes.c_void_p(at), ctypes.c_void_p(at + by_key), ctypes.c_void_p(at + classes)
+    return at, at + by_key, at + classes
 
 
 def flash_forward(q, k, v, scale, causal, mask8, lens32, packed=None):
     """Fused forward: returns ``(o (b, sq, h, d), lse (b, h, sq) fp32)``.  ``packed``: what ``pack_mask`` made of it when the caller
     has it already."""
-    lib = _native.cuda_lib()
     b, sq, h, d = q.shape
     sk, hk = k.shape[1], k.shape[2]
     packed = pack_mask(mask8, b, sq, sk) if packed is None else packed
     bits, _, classes = _mask_parts(packed, b, sq, sk)
     o = torch.empty(b, sq, h, d, dtype=q.dtype, device=q.device)
     lse = torch.empty(b, h, sq, dtype=torch.float32, device=q.device)
-    _native.check(lib.bmt_flash_attn_fwd(
-        ctypes.c_int64(b), ctypes.c_int64(sq), ctypes.c_int64(sk), ctypes.c_int(h), ctypes.c_int(hk), ctypes.c_int(d),
-        _native.ptr(q), _strides3(q), _native.ptr(k), _strides3(k), _native.ptr(v), _strides3(v), _native.ptr(o), _strides3(o),
-        _native.ptr(lse), ctypes.c_float(scale), ctypes.c_int(1 if causal else 0), bits, classes, _native.ptr(lens32),
-        ctypes.c_int(_DT[q.dtype]), _native.stream_handle()), "fused attention forward")
+    out_str = _strides3(o)
+    _native.check(_native.entry("bmt_flash_attn_fwd", "qqqiiipbpbpbpbpfipppip")(
+        b, sq, sk, h, hk, d, q.data_ptr(), _strides3(q), k.data_ptr(), _strides3(k), v.data_ptr(), _strides3(v), o.data_ptr(), out_str,
+        lse.data_ptr(), scale, 1 if causal else 0, bits, classes, 0 if lens32 is None else lens32.data_ptr(), _DT[q.dtype],
+        _native.stream()), "fused attention forward")
     return o, lse
 
 
@@ -142,13 +146,12 @@ def flash_backward(q, k, v, o, lse, do, scale, causal, mask8, lens32, packed=Non
         lib.bmt_flash_attn_bwd_parts.restype = ctypes.c_int64
         n = lib.bmt_flash_attn_bwd_parts(ctypes.c_int64(b), ctypes.c_int64(sk), ctypes.c_int(h), ctypes.c_int(hk), ctypes.c_int(d))
         parts = torch.empty(n, dtype=torch.float32, device=q.device) if n else None
-    _native.check(lib.bmt_flash_attn_bwd(
-        ctypes.c_int64(b), ctypes.c_int64(sq), ctypes.c_int64(sk), ctypes.c_int(h), ctypes.c_int(hk), ctypes.c_int(d),
-        _native.ptr(q), _strides3(q), _native.ptr(k), _strides3(k), _native.ptr(v), _strides3(v), _native.ptr(o), _strides3(o),
-        _native.ptr(do), _strides3(do), _native.ptr(lse), _native.ptr(dq), _strides3(dq), _native.ptr(dk), _strides3(dk),
-        _native.ptr(dv), _strides3(dv), _native.ptr(dq_acc), _native.ptr(delta), ctypes.c_float(scale),
-        ctypes.c_int(1 if causal else 0), bits_t, classes, _native.ptr(lens32), _native.ptr(parts), ctypes.c_int(_DT[q.dtype]),
-        _native.stream_handle()), "fused attention backward")
+    dq_str, kv_str = _strides3(dq), _strides3(dk)
+    _native.check(_native.entry("bmt_flash_attn_bwd", "qqqiiipbpbpbpbpbppbpbpbppfippppip")(
+        b, sq, sk, h, hk, d, q.data_ptr(), _strides3(q), k.data_ptr(), _strides3(k), v.data_ptr(), _strides3(v), o.data_ptr(), _strides3(o),
+        do.data_ptr(), _strides3(do), lse.data_ptr(), dq.data_ptr(), dq_str, dk.data_ptr(), kv_str, dv.data_ptr(), kv_str, dq_acc.data_ptr(),
+        delta.data_ptr(), scale, 1 if causal else 0, bits_t, classes, 0 if lens32 is None else lens32.data_ptr(),
+        0 if parts is None else parts.data_ptr(), _DT[q.dtype], _native.stream()), "fused attention backward")
     return dq, dk, dv
 
 

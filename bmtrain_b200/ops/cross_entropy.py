@@ -78,10 +78,9 @@ def reduced_forward(logits: torch.Tensor, target: torch.Tensor, ignore_index: in
     scratch = torch.empty(3 * m, dtype=torch.float32, device=logits.device)
     kept = torch.empty(m + 1, dtype=torch.float32, device=logits.device)
     loss, lse, divisor = torch.empty((), dtype=torch.float32, device=logits.device), kept[:m], kept[m:]
-    _native.check(_native.cuda_lib().bmt_ce_reduced_forward(
-        ctypes.c_int64(m), ctypes.c_int64(n), _native.ptr(logits), ctypes.c_int(_DT[logits.dtype]), _native.ptr(target),
-        ctypes.c_int64(ignore_index), ctypes.c_int(1 if mean else 0), _native.ptr(scratch), _native.ptr(lse), _native.ptr(loss), _native.ptr(divisor),
-        _native.stream_handle()), "cross-entropy forward kernels")
+    _native.check(_native.entry("bmt_ce_reduced_forward", "qqpipqippppp")(
+        m, n, logits.data_ptr(), _DT[logits.dtype], target.data_ptr(), ignore_index, 1 if mean else 0, scratch.data_ptr(), lse.data_ptr(),
+        loss.data_ptr(), divisor.data_ptr(), _native.stream()), "cross-entropy forward kernels")
     return loss, lse, divisor
 
 
@@ -90,8 +89,7 @@ def reduced_backward(logits: torch.Tensor, target: torch.Tensor, lse: torch.Tens
     """Gradient of :func:`reduced_forward`'s loss for the scalar ``grad_loss``."""
     m, n = logits.shape
     out = torch.empty_like(logits)
-    _native.check(_native.cuda_lib().bmt_ce_reduced_backward(
-        ctypes.c_int64(m), ctypes.c_int64(n), _native.ptr(logits), ctypes.c_int(_DT[logits.dtype]), _native.ptr(target),
-        _native.ptr(lse), _native.ptr(grad_loss.float().contiguous()), _native.ptr(divisor), ctypes.c_int64(ignore_index),
-        _native.ptr(out), _native.stream_handle()), "cross-entropy backward kernel")
+    _native.check(_native.entry("bmt_ce_reduced_backward", "qqpippppqpp")(
+        m, n, logits.data_ptr(), _DT[logits.dtype], target.data_ptr(), lse.data_ptr(), grad_loss.float().contiguous().data_ptr(),
+        divisor.data_ptr(), ignore_index, out.data_ptr(), _native.stream()), "cross-entropy backward kernel")
     return out

@@ -41,19 +41,18 @@ def _apply_act(x: torch.Tensor, act) -> torch.Tensor:
     raise ValueError(act)
 
 
+_OUT_DT = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}
+
+
 def _launch(a, b, out, m, n, k, a_major, b_major, bias, act, accumulate, lda, ldb):
-    lib = _native.cuda_lib()
-    assert a.dtype == b.dtype and a.dtype in _DT, "tensor-core GEMM takes fp16 or bf16 operands"
-    out_dt = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}[out.dtype]
+    dt = a.dtype
+    assert dt == b.dtype and dt in _DT, "tensor-core GEMM takes fp16 or bf16 operands"
     work = scratch()
-    status = lib.bmt_gemm(
-        ctypes.c_int64(m), ctypes.c_int64(n), ctypes.c_int64(k),
-        _native.ptr(a), ctypes.c_int64(lda), ctypes.c_int(a_major),
-        _native.ptr(b), ctypes.c_int64(ldb), ctypes.c_int(b_major),
-        _native.ptr(out), ctypes.c_int64(out.stride(0)), ctypes.c_int(out_dt),
-        _native.ptr(bias), ctypes.c_int(_ACT[act]), ctypes.c_int(1 if accumulate else 0),
-        ctypes.c_int(_DT[a.dtype]), *work.gemm, work.stream)
-    _native.check(status, f"tcgen05 GEMM (m={m}, n={n}, k={k})")
+    status = _native.entry("bmt_gemm", "qqqpqipqipqipiiipqp")(
+        m, n, k, a.data_ptr(), lda, a_major, b.data_ptr(), ldb, b_major, out.data_ptr(), out.stride(0), _OUT_DT[out.dtype],
+        0 if bias is None else bias.data_ptr(), _ACT[act], 1 if accumulate else 0, _DT[dt], work.gemm[0], work.gemm[1], work.stream)
+    if status != 0:
+        _native.check(status, f"tcgen05 GEMM (m={m}, n={n}, k={k})")
 
 
 def _use_torch(t: torch.Tensor) -> bool:
@@ -62,13 +61,14 @@ def _use_torch(t: torch.Tensor) -> bool:
 
 def _rowmajor(t: torch.Tensor) -> torch.Tensor:
     """A view TMA can read: unit inner stride, 16-byte aligned base and row pitch (pads a copy when needed)."""
-    if t.stride(-1) == 1 and t.stride(0) >= t.shape[1] and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0:
+    (rows, cols), (pitch, step) = t.shape, t.stride()
+    if step == 1 and pitch >= cols and pitch % 8 == 0 and t.data_ptr() % 16 == 0:
         return t
-    if t.shape[1] % 8 == 0:
+    if cols % 8 == 0:
         return t.contiguous()
-    padded = torch.zeros(t.shape[0], (t.shape[1] + 7) // 8 * 8, dtype=t.dtype, device=t.device)
-    padded[:, : t.shape[1]].copy_(t)
-    return padded[:, : t.shape[1]]
+    padded = torch.zeros(rows, (cols + 7) // 8 * 8, dtype=t.dtype, device=t.device)
+    padded[:, :cols].copy_(t)
+    return padded[:, :cols]
 
 
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, act=None,
@@ -142,7 +142,7 @@ _scratch = {}
 class _Scratch:
     """Work space of the kernels that add partial sums, one per device and stream, zeroed once: the kernels leave counters and flags
     at zero, and launches that share it take turns on their stream.  The first part belongs to the column sums (4 KB of ticket
-    counters and the sums), the second to the GEMMs that divide tiles over several CTAs.  Both as C arguments, with the stream."""
+    counters and the sums), the second to the GEMMs that divide tiles over several CTAs: (address, bytes) each."""
 
     __slots__ = ("buf", "colsum", "gemm", "stream")
 
@@ -152,9 +152,9 @@ class _Scratch:
         size = lib.bmt_gemm_scratch_bytes()
         self.buf = torch.zeros(_COLSUM_BYTES + size, dtype=torch.uint8, device=torch.device("cuda", index))
         base = self.buf.data_ptr()
-        self.colsum = (ctypes.c_void_p(base), ctypes.c_int64(_COLSUM_BYTES))
-        self.gemm = (ctypes.c_void_p(base + _COLSUM_BYTES), ctypes.c_int64(size))
-        self.stream = ctypes.c_void_p(stream)
+        self.colsum = (base, _COLSUM_BYTES)
+        self.gemm = (base + _COLSUM_BYTES, size)
+        self.stream = stream
 
 
 def scratch() -> _Scratch:
@@ -174,14 +174,12 @@ def bias_grad(grad_out: torch.Tensor) -> torch.Tensor:
     """Column sums of ``grad_out`` (M, N), accumulated in fp32, returned in the input dtype."""
     if not grad_out.is_cuda:
         return grad_out.float().sum(0).to(grad_out.dtype)
-    lib = _native.cuda_lib()
     g = grad_out.contiguous()
     m, n = g.shape
     out = torch.empty(n, dtype=g.dtype, device=g.device)
     work = scratch()
-    dt = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}[g.dtype]
-    _native.check(lib.bmt_colsum_ex(ctypes.c_int64(m), ctypes.c_int64(n), _native.ptr(g), ctypes.c_int(dt), _native.ptr(out),
-                                    ctypes.c_int(0), *work.colsum, work.stream), "column-sum kernel")
+    _native.check(_native.entry("bmt_colsum_ex", "qqpipipqp")(m, n, g.data_ptr(), _OUT_DT[g.dtype], out.data_ptr(), 0, *work.colsum, work.stream),
+                  "column-sum kernel")
     return out
 
 
@@ -192,15 +190,16 @@ class LinearFunction(torch.autograd.Function):
     def forward(ctx, x, weight, bias):
         ctx.save_for_backward(x, weight)
         ctx.has_bias = bias is not None
-        x2 = x.reshape(-1, x.shape[-1])
-        y = gemm_nt(x2, weight, bias)
+        if x.dim() == 2:
+            return gemm_nt(x, weight, bias)
+        y = gemm_nt(x.reshape(-1, x.shape[-1]), weight, bias)
         return y.view(*x.shape[:-1], weight.shape[0])
 
     @staticmethod
     def backward(ctx, grad_output):
         x, weight = ctx.saved_tensors
-        g2 = grad_output.reshape(-1, grad_output.shape[-1])
-        x2 = x.reshape(-1, x.shape[-1])
+        g2 = grad_output if grad_output.dim() == 2 else grad_output.reshape(-1, grad_output.shape[-1])
+        x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
         grad_x = grad_w = grad_b = None
         if ctx.needs_input_grad[0]:
             grad_x = gemm_nn(g2, weight).view(x.shape)

@@ -135,7 +135,7 @@ class Pass:
         # fused attention: scores and probabilities never reach memory, one log-sum-exp per row is kept instead
         self.tail = (at["ln1"], at["stats1"], at["qkv"], get("probs", 0), (s + 7) // 8 * 8 if "probs" in at else 0, at["ctx"], at["h1"], at["ln2"],
                      at["stats2"], at["ff"], get("pre", 0), get("lse", 0), get("mask_packed", 0),
-                     work.colsum[0].value, work.colsum[1].value, work.gemm[0].value, work.gemm[1].value)
+                     *work.colsum, *work.gemm)
 
     def forward(self) -> torch.Tensor:
         y = torch.empty_like(self.x)
@@ -151,8 +151,8 @@ class Pass:
 
     def run(self, first: int, last: int, y: Optional[torch.Tensor] = None) -> None:
         """Steps of the forward (``bmt_gpt_block_forward_steps``); the last one, 9, is what computes ``y``."""
-        _native.check(_native.cuda_lib().bmt_gpt_block_forward_steps(self.describe(0 if y is None else y.data_ptr()), first, last,
-                                                                     self.scratch.stream), "GPT block forward")
+        _native.check(_native.entry("bmt_gpt_block_forward_steps", "biip")(self.describe(0 if y is None else y.data_ptr()), first, last,
+                                                                           self.scratch.stream), "GPT block forward")
 
     def backward(self, dy: torch.Tensor, grads, acc_weights: bool = False, acc_small: bool = False) -> torch.Tensor:
         """``grads``: addresses for the gradients of the parameters, in their order; ``acc_*``: added to what is there."""
@@ -167,8 +167,8 @@ class Pass:
                        1 if acc_small else 0)
         scratch = _gemm.scratch()
         if scratch is not self.scratch:         # another stream than the forward's
-            self.tail = self.tail[:-4] + (scratch.colsum[0].value, scratch.colsum[1].value, scratch.gemm[0].value, scratch.gemm[1].value)
-        _native.check(_native.cuda_lib().bmt_gpt_block_backward(self.describe(), g, scratch.stream), "GPT block backward")
+            self.tail = self.tail[:-4] + (*scratch.colsum, *scratch.gemm)
+        _native.check(_native.entry("bmt_gpt_block_backward", "bbp")(self.describe(), g, scratch.stream), "GPT block backward")
         return dx
 
 

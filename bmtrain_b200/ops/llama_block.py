@@ -58,18 +58,18 @@ class Pass:
         self.tail = (self.table.data_ptr(), *[base + plan[n] for n in _SAVED])
 
     def _describe(self, y, scratch):
-        return _BLOCK.pack(*self.head, self.x.data_ptr(), y, *self.tail, scratch.gemm[0].value, scratch.gemm[1].value)
+        return _BLOCK.pack(*self.head, self.x.data_ptr(), y, *self.tail, *scratch.gemm)
 
     def forward(self) -> torch.Tensor:
         y = torch.empty_like(self.x)
         scratch = _gemm.scratch()
-        _native.check(_native.cuda_lib().bmt_llama_block_forward(self._describe(y.data_ptr(), scratch), 9, scratch.stream), "Llama block forward")
+        _native.check(_native.entry("bmt_llama_block_forward", "bip")(self._describe(y.data_ptr(), scratch), 9, scratch.stream), "Llama block forward")
         return y
 
     def recompute(self) -> None:
         """Forward again for ``backward``: without the last GEMM, whose result nothing reads."""
         scratch = _gemm.scratch()
-        _native.check(_native.cuda_lib().bmt_llama_block_forward(self._describe(0, scratch), 8, scratch.stream), "Llama block forward")
+        _native.check(_native.entry("bmt_llama_block_forward", "bip")(self._describe(0, scratch), 8, scratch.stream), "Llama block forward")
 
     def backward(self, dy: torch.Tensor, grads) -> torch.Tensor:
         """``grads``: addresses for the gradients of the parameters, in their order."""
@@ -81,5 +81,5 @@ class Pass:
         dx = torch.empty_like(self.x)
         scratch = _gemm.scratch()
         g = _GRAD.pack(dy.data_ptr(), dx.data_ptr(), *grads, *[base + plan[n] if n in plan else 0 for n in _WORK], nblk)
-        _native.check(_native.cuda_lib().bmt_llama_block_backward(self._describe(0, scratch), g, scratch.stream), "Llama block backward")
+        _native.check(_native.entry("bmt_llama_block_backward", "bbp")(self._describe(0, scratch), g, scratch.stream), "Llama block backward")
         return dx

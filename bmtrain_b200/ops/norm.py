@@ -8,7 +8,6 @@ folds.  CPU tensors use the PyTorch definition.
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Optional
 
 import torch
@@ -27,10 +26,9 @@ class LayerNormFunction(torch.autograd.Function):
         rows = x2.shape[0]
         y = torch.empty_like(x2)
         stats = torch.empty(2, rows, dtype=torch.float32, device=x.device)  # mean, rstd
-        _native.check(_native.cuda_lib().bmt_norm_fwd(
-            ctypes.c_int64(rows), ctypes.c_int64(d), _native.ptr(x2), _native.ptr(weight), _native.ptr(bias),
-            ctypes.c_float(eps), ctypes.c_int(1 if rms else 0), ctypes.c_int(_DT[x.dtype]),
-            _native.ptr(y), _native.ptr(stats), _native.stream_handle()), "norm forward kernel")
+        _native.check(_native.entry("bmt_norm_fwd", "qqpppfiippp")(
+            rows, d, x2.data_ptr(), weight.data_ptr(), 0 if bias is None else bias.data_ptr(), eps, 1 if rms else 0, _DT[x.dtype], y.data_ptr(),
+            stats.data_ptr(), _native.stream()), "norm forward kernel")
         ctx.save_for_backward(x2, weight, stats)
         ctx.rms, ctx.has_bias, ctx.shape = rms, bias is not None, shape
         return y.view(shape)
@@ -45,11 +43,9 @@ class LayerNormFunction(torch.autograd.Function):
         partial = torch.empty(2, nblk, d, dtype=torch.float32, device=x2.device)
         dw = torch.empty(d, dtype=weight.dtype, device=x2.device)
         db = torch.empty(d, dtype=weight.dtype, device=x2.device) if ctx.has_bias else None
-        _native.check(_native.cuda_lib().bmt_norm_bwd(
-            ctypes.c_int64(rows), ctypes.c_int64(d), _native.ptr(x2), _native.ptr(g2), _native.ptr(weight),
-            _native.ptr(stats), ctypes.c_int(1 if ctx.rms else 0), ctypes.c_int(_DT[x2.dtype]), ctypes.c_int(nblk),
-            _native.ptr(dx), _native.ptr(partial), _native.ptr(dw), _native.ptr(db),
-            _native.stream_handle()), "norm backward kernel")
+        _native.check(_native.entry("bmt_norm_bwd", "qqppppiiippppp")(
+            rows, d, x2.data_ptr(), g2.data_ptr(), weight.data_ptr(), stats.data_ptr(), 1 if ctx.rms else 0, _DT[x2.dtype], nblk, dx.data_ptr(),
+            partial.data_ptr(), dw.data_ptr(), 0 if db is None else db.data_ptr(), _native.stream()), "norm backward kernel")
         return dx.view(ctx.shape), dw, db, None, None
 
 
