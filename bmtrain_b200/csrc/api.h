@@ -70,6 +70,9 @@ int bmt_embedding_fwd(int64_t tokens, int64_t d, const void* ids_i64, const void
 int64_t bmt_embedding_bwd_scratch(int64_t tokens, int64_t rows);   // 32-bit words of scratch
 int bmt_embedding_bwd(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out, void* scratch,
                       void* stream);
+// accumulate: added to what `out` holds
+int bmt_embedding_bwd_ex(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out, int accumulate,
+                         void* scratch, void* stream);
 
 int bmt_masked_softmax(int64_t b, int64_t h, int64_t sq, int64_t sk, int64_t ld, void* scores, int dtype, int causal,
                        const void* mask_u8_b_sq_sk, const void* kv_lens_i32, void* stream);

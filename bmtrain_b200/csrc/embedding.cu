@@ -65,13 +65,21 @@ __global__ void __launch_bounds__(256) emb_order_kernel(int64_t tokens, int64_t 
     const int64_t id = ids[t];
     if (id >= 0 && id < rows) e.order[e.start[id] + e.rank[t]] = (int)t;
 }
-// `team` threads (32 .. 256) per row
-template <typename T>
-__global__ void __launch_bounds__(256) emb_rows_kernel(int64_t rows, int64_t d, int team, const T* __restrict__ g, EmbScratch e, T* __restrict__ out) {
+// `team` threads (32 .. 256) per row.  ADD: the sums are added to what the table's gradient holds already (in fp32, rounded once).
+// Then only rows that have tokens are touched, and there is a team per token instead, which works if its token is the first of its
+// row: 4096 tokens, 50304 x 4096 bf16: 68 us for the whole table, and 190 us of autograd adding that up, became 14 us.
+template <typename T, bool ADD>
+__global__ void __launch_bounds__(256) emb_rows_kernel(int64_t items, int64_t rows, int64_t d, int team, const int64_t* __restrict__ ids,
+                                                       const T* __restrict__ g, EmbScratch e, T* __restrict__ out) {
     bmt::after_previous();
     constexpr int V = bmt::Vec16<T>::N;
-    const int64_t r = (int64_t)blockIdx.x * (256 / team) + threadIdx.x / team;
-    if (r >= rows) return;
+    int64_t r = (int64_t)blockIdx.x * (256 / team) + threadIdx.x / team;
+    if (r >= items) return;
+    if (ADD) {
+        const int64_t id = ids[r];
+        if (id < 0 || id >= rows || e.rank[r] != 0) return;
+        r = id;
+    }
     const int c = e.count[r];
     if (c > EMB_HOT) return;
     const int* __restrict__ tok = e.order + (c ? e.start[r] : 0);
@@ -86,12 +94,13 @@ __global__ void __launch_bounds__(256) emb_rows_kernel(int64_t rows, int64_t d, 
             for (int k = 0; k < V; ++k) acc[k] += bmt::Cvt<T>::to_f(v.v[k]);
         }
         bmt::Vec16<T> o;
+        if (ADD) o = bmt::ld16(out + r * d + col);
 #pragma unroll
-        for (int k = 0; k < V; ++k) o.v[k] = bmt::Cvt<T>::from_f(acc[k]);
+        for (int k = 0; k < V; ++k) o.v[k] = bmt::Cvt<T>::from_f(ADD ? bmt::Cvt<T>::to_f(o.v[k]) + acc[k] : acc[k]);
         bmt::st16(out + r * d + col, o);
     }
 }
-template <typename T>
+template <typename T, bool ADD>
 __global__ void __launch_bounds__(256) emb_hot_kernel(int64_t d, const T* __restrict__ g, EmbScratch e, T* __restrict__ out) {
     bmt::after_previous();
     constexpr int V = bmt::Vec16<T>::N;
@@ -119,9 +128,10 @@ __global__ void __launch_bounds__(256) emb_hot_kernel(int64_t d, const T* __rest
         __syncthreads();
         if (warp == 0 && col < d) {
             bmt::Vec16<T> o;
+            if (ADD) o = bmt::ld16(out + r * d + col);
 #pragma unroll
             for (int k = 0; k < V; ++k) {
-                float s = 0.f;
+                float s = ADD ? bmt::Cvt<T>::to_f(o.v[k]) : 0.f;
 #pragma unroll
                 for (int w = 0; w < 8; ++w) s += part[w][lane * V + k];
                 o.v[k] = bmt::Cvt<T>::from_f(s);
@@ -131,14 +141,15 @@ __global__ void __launch_bounds__(256) emb_hot_kernel(int64_t d, const T* __rest
     }
 }
 
-template <typename T>
-void launch_rows(int64_t rows, int64_t d, const void* g, const EmbScratch& e, void* out, bool any_hot, cudaStream_t s) {
+template <typename T, bool ADD>
+void launch_rows(int64_t tokens, int64_t rows, int64_t d, const int64_t* ids, const void* g, const EmbScratch& e, void* out, cudaStream_t s) {
     constexpr int V = bmt::Vec16<T>::N;
     int team = 32;
     while (team < 256 && (int64_t)team * V < d) team *= 2;
     const int per = 256 / team;
-    bmt::launch(emb_rows_kernel<T>, (unsigned)((rows + per - 1) / per), 256, 0, s, 1, rows, d, team, (const T*)g, e, (T*)out);
-    if (any_hot) bmt::launch(emb_hot_kernel<T>, 296, 256, 0, s, 1, d, (const T*)g, e, (T*)out);
+    const int64_t items = ADD ? tokens : rows;
+    bmt::launch(emb_rows_kernel<T, ADD>, (unsigned)((items + per - 1) / per), 256, 0, s, 1, items, rows, d, team, ids, (const T*)g, e, (T*)out);
+    if (tokens > EMB_HOT) bmt::launch(emb_hot_kernel<T, ADD>, 296, 256, 0, s, 1, d, (const T*)g, e, (T*)out);
 }
 
 }  // namespace
@@ -157,9 +168,9 @@ extern "C" int bmt_embedding_fwd(int64_t tokens, int64_t d, const void* ids, con
 // 32-bit words of scratch that bmt_embedding_bwd needs.
 extern "C" int64_t bmt_embedding_bwd_scratch(int64_t tokens, int64_t rows) { return 2 + 2 * rows + emb_hot_cap(tokens) + 2 * tokens; }
 
-extern "C" int bmt_embedding_bwd(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out,
-                                 void* scratch, void* stream) {
-    if (rows <= 0) return 0;
+extern "C" int bmt_embedding_bwd_ex(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out,
+                                    int accumulate, void* scratch, void* stream) {
+    if (rows <= 0 || (accumulate && tokens <= 0)) return 0;
     if (d % (dtype == BMT_DT_F32 ? 4 : 8) || tokens > 0x7fffffff || rows > 0x7fffffff) return -3;
     cudaStream_t s = (cudaStream_t)stream;
     const EmbScratch e = emb_scratch(scratch, tokens, rows);
@@ -171,10 +182,19 @@ extern "C" int bmt_embedding_bwd(int64_t tokens, int64_t d, int64_t rows, const 
         bmt::launch(emb_order_kernel, tb, 256, 0, s, 1, tokens, rows, (const int64_t*)ids, e);
         bmt_count_launch(3);
     }
-    const bool any_hot = tokens > EMB_HOT;
-    if (dtype == BMT_DT_F32) launch_rows<float>(rows, d, grad, e, out, any_hot, s);
-    else if (dtype == BMT_DT_F16) launch_rows<__half>(rows, d, grad, e, out, any_hot, s);
-    else launch_rows<__nv_bfloat16>(rows, d, grad, e, out, any_hot, s);
-    bmt_count_launch(any_hot ? 2 : 1);
+    const auto run = [&](auto zero) {
+        using T = decltype(zero);
+        if (accumulate) launch_rows<T, true>(tokens, rows, d, (const int64_t*)ids, grad, e, out, s);
+        else launch_rows<T, false>(tokens, rows, d, (const int64_t*)ids, grad, e, out, s);
+    };
+    if (dtype == BMT_DT_F32) run(0.f);
+    else if (dtype == BMT_DT_F16) run(__half());
+    else run(__nv_bfloat16());
+    bmt_count_launch(tokens > EMB_HOT ? 2 : 1);
     return (int)cudaGetLastError();
+}
+
+extern "C" int bmt_embedding_bwd(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out,
+                                 void* scratch, void* stream) {
+    return bmt_embedding_bwd_ex(tokens, d, rows, ids, grad, dtype, out, 0, scratch, stream);
 }

@@ -13,39 +13,53 @@ import torch
 from ..layer import DistributedModule, reads_parameters_only
 from ..ops import embedding as _emb
 from ..ops import gemm as _gemm
+from ..ops import grad_slot as _grad_slot
 from ..ops import norm as _norm
 from ..parameter import DistributedParameter, ParameterInitializer, await_update, private_value, shard_is_value
 
 
 class _ShardLookup(torch.autograd.Function):
     """Lookup in a table whose shard is the whole table: the kernel has read it before anything behind the call can write to
-    it, backward does not need it, and its gradient is a fresh tensor.  So neither is copied."""
+    it, backward does not need it, and its gradient is a fresh tensor.  So neither is copied; a gradient that is attached is added to."""
 
     @staticmethod
     def forward(ctx, ids, table):
         await_update(table)
         ctx.save_for_backward(ids)
-        ctx.rows = table._original_shape[0]
+        ctx.table = table
         return _emb.embedding_forward(ids, table.data.reshape(table._original_shape))
 
     @staticmethod
     def backward(ctx, grad):
         (ids,) = ctx.saved_tensors
-        return None, _emb.embedding_backward(ids, grad.contiguous(), ctx.rows).view(-1)
+        shape = ctx.table._original_shape
+        held = _grad_slot.attached(ctx, 1, ctx.table) if grad.dtype == ctx.table.dtype else None
+        if held is not None:
+            _emb.embedding_backward(ids, grad.contiguous(), shape[0], add_to=held.view(shape))
+            return None, None
+        return None, _emb.embedding_backward(ids, grad.contiguous(), shape[0]).view(-1)
 
 
 class _ShardProjection(torch.autograd.Function):
     """Multiplication by such a table: backward multiplies by the value of the forward pass, which is therefore a copy; the
-    table's gradient is a fresh tensor and is not copied."""
+    table's gradient is a fresh tensor and is not copied, or added to the one that is attached."""
 
     @staticmethod
     def forward(ctx, x, table):
+        ctx.table = table
         return _gemm.LinearFunction.forward(ctx, x, private_value(table), None)
 
     @staticmethod
     def backward(ctx, grad):
-        grad_x, grad_w, _ = _gemm.LinearFunction.backward(ctx, grad)
-        return grad_x, None if grad_w is None else grad_w.view(-1)
+        x, weight = ctx.saved_tensors
+        held = _grad_slot.attached(ctx, 1, ctx.table) if ctx.needs_input_grad[1] and grad.dtype == weight.dtype else None
+        if held is None:
+            grad_x, grad_w, _ = _gemm.LinearFunction.backward(ctx, grad)
+            return grad_x, None if grad_w is None else grad_w.view(-1)
+        g2 = grad.reshape(-1, grad.shape[-1])
+        grad_x = _gemm.gemm_nn(g2, weight).view(x.shape) if ctx.needs_input_grad[0] else None
+        _gemm.gemm_tn(g2, x.reshape(-1, x.shape[-1]), out=held.view(weight.shape), accumulate=True)
+        return grad_x, None
 
 
 @reads_parameters_only

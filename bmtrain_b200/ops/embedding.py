@@ -6,6 +6,7 @@ and writes every row of the table's gradient once, added in fp32 and rounded onc
 from __future__ import annotations
 
 import ctypes
+from typing import Optional
 
 import torch
 
@@ -29,8 +30,9 @@ def embedding_forward(ids: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def embedding_backward(ids: torch.Tensor, grad: torch.Tensor, rows: int) -> torch.Tensor:
-    """``grad_weight[ids[t]] += grad[t]`` accumulated in fp32, returned in ``grad``'s dtype."""
+def embedding_backward(ids: torch.Tensor, grad: torch.Tensor, rows: int, add_to: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``grad_weight[ids[t]] += grad[t]`` accumulated in fp32, returned in ``grad``'s dtype.  ``add_to`` (GPU): a gradient of the table,
+    (rows, d) and contiguous, that the sums are added to; only its rows that occur in ``ids`` are touched."""
     d = grad.shape[-1]
     g2 = grad.reshape(-1, d)
     flat = ids.reshape(-1)
@@ -40,16 +42,16 @@ def embedding_backward(ids: torch.Tensor, grad: torch.Tensor, rows: int) -> torc
         acc.index_add_(0, flat[keep], g2[keep].float())
         return acc.to(grad.dtype)
     if flat.numel() == 0:
-        return torch.zeros(rows, d, dtype=grad.dtype, device=grad.device)
+        return torch.zeros(rows, d, dtype=grad.dtype, device=grad.device) if add_to is None else add_to
     lib = _native.cuda_lib()
     ids64, g2 = flat.to(torch.int64).contiguous(), g2.contiguous()
-    out = torch.empty(rows, d, dtype=grad.dtype, device=grad.device)
+    out = torch.empty(rows, d, dtype=grad.dtype, device=grad.device) if add_to is None else add_to
     lib.bmt_embedding_bwd_scratch.restype = ctypes.c_int64
     words = lib.bmt_embedding_bwd_scratch(ctypes.c_int64(ids64.numel()), ctypes.c_int64(rows))
     scratch = torch.empty(words, dtype=torch.int32, device=grad.device)
-    _native.check(lib.bmt_embedding_bwd(
-        ctypes.c_int64(ids64.numel()), ctypes.c_int64(d), ctypes.c_int64(rows), _native.ptr(ids64), _native.ptr(g2),
-        ctypes.c_int(_DT[grad.dtype]), _native.ptr(out), _native.ptr(scratch), _native.stream_handle()), "embedding backward kernels")
+    _native.check(_native.entry("bmt_embedding_bwd_ex", "qqqppipipp")(
+        ids64.numel(), d, rows, ids64.data_ptr(), g2.data_ptr(), _DT[grad.dtype], out.data_ptr(), 0 if add_to is None else 1, scratch.data_ptr(),
+        _native.stream()), "embedding backward kernels")
     return out
 
 
