@@ -86,8 +86,6 @@ struct GemmParams {
     uint32_t sk_slot;
 };
 
-__device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
-
 template <typename T> __device__ __forceinline__ void store8(T* dst, const float* v) {
     bmt::Vec16<T> o;
 #pragma unroll
@@ -173,10 +171,6 @@ struct SharedHeader {
     int failed;
 };
 
-__device__ __forceinline__ float gelu_grad_f(float x) {
-    const float cdf = 0.5f * (1.f + erff(x * 0.70710678118654752f));
-    return cdf + x * 0.3989422804014327f * __expf(-0.5f * x * x);
-}
 // Eight consecutive elements of a row (the first `n` of them exist) as floats; one 16-byte load when `vec`.
 template <typename T> __device__ __forceinline__ void load_row8(const T* src, int n, bool vec, float (&v)[8]) {
     if (vec && n >= 8) {
@@ -452,7 +446,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, con
                 unpack8<T>(cur[it], e);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    v[it][i] = EXTRA == 1 ? (p.round_first ? bmt::Cvt<T>::to_f(bmt::Cvt<T>::from_f(v[it][i])) : v[it][i]) + e[i] : EXTRA == 2 ? (e[i] > 0.f ? v[it][i] : 0.f) : v[it][i] * gelu_grad_f(e[i]);
+                    v[it][i] = EXTRA == 1 ? (p.round_first ? bmt::Cvt<T>::to_f(bmt::Cvt<T>::from_f(v[it][i])) : v[it][i]) + e[i] : EXTRA == 2 ? (e[i] > 0.f ? v[it][i] : 0.f) : v[it][i] * bmt::gelu_grad(e[i]);
             }
             if (col_ok && it * 8 + sub < rows) store8(dst + it * d_step + c * 32, v[it]);
         }
@@ -491,12 +485,12 @@ __device__ __forceinline__ void epilogue_rows_any(const GemmParams& p, TC* cbase
             for (int i = 0; i < 8; ++i) {
                 v[i] = v[i] * p.alpha + bias[i];
                 if (p.act == 1) v[i] = fmaxf(v[i], 0.f);
-                else if (p.act == 2) v[i] = gelu_f(v[i]);
+                else if (p.act == 2) v[i] = bmt::gelu(v[i]);
             }
             if (p.aux_mode) {
                 load_row8_dt(p.aux, p.bias_dtype, row * p.ld_aux + col, n_ok, a_vec, e);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = p.aux_mode == 1 ? (e[i] > 0.f ? v[i] : 0.f) : v[i] * gelu_grad_f(e[i]);
+                for (int i = 0; i < 8; ++i) v[i] = p.aux_mode == 1 ? (e[i] > 0.f ? v[i] : 0.f) : v[i] * bmt::gelu_grad(e[i]);
             }
             if (p.residual) {
                 load_row8_dt(p.residual, p.bias_dtype, row * p.ldr + col, n_ok, r_vec, e);
