@@ -87,6 +87,22 @@ int bmt_colsum(int64_t m, int64_t n, const void* x, int dtype, void* out, void* 
 int bmt_colsum_ex(int64_t m, int64_t n, const void* x, int dtype, void* out, int accumulate, void* scratch,
                   int64_t scratch_bytes, void* stream);
 
+// Column sums of several matrices at once: the bias gradients of a block and the sums that the norms' backward leaves.
+typedef struct {
+    const void* x;          // (m, n) contiguous: of the call's 16-bit type, or fp32
+    int64_t m, n;
+    void* out;              // n elements of the call's type
+    int f32;
+    int first;              // set by the call
+} BmtColsum;
+#define BMT_MAX_COLSUMS 12
+// At most BMT_MAX_COLSUMS, n multiples of 8; scratch as of bmt_colsum_ex; accumulate: added to what the outputs hold.
+int bmt_colsum_multi(const BmtColsum* items, int count, int dtype, int accumulate, void* scratch, int64_t scratch_bytes, void* stream);
+// bmt_norm_bwd_ex without its last kernel: the weight's gradient is the column sums of the first *blocks rows of `partial` (fp32, d columns),
+// the bias's of the *blocks rows behind them.
+int bmt_norm_bwd_partial(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, const void* stats, int rms, int dtype, int nblk,
+                         void* dx, void* partial, const void* dres, int* blocks, void* stream);
+
 // Full description of one (optionally batched) GEMM launch; zero-initialise, then fill what is needed.
 typedef struct {
     int64_t m, n, k;
@@ -173,6 +189,7 @@ typedef struct {
     void* dq_acc;
     void* delta;
     int acc_small;            // bias and norm gradients are added to what d_*_b / d_ln*_w already hold
+    void* norm_partial2;      // like norm_partial: one for each norm
 } BmtGptBlockGrad;
 
 int bmt_gpt_block_forward(const BmtGptBlock* blk, void* stream);
@@ -218,7 +235,7 @@ typedef struct {
     void* d_ctx;         // (T, n_heads * d_head)
     void *dq, *dk, *dv;  // like q, k, v
     void* d_packed;      // like packed
-    void* norm_partial;  // (2, nblk, d) fp32
+    void* norm_partial;  // (2, nblk, d) fp32, twice
     void* dq_acc;        // batch * seq * n_heads * d_head fp32
     void* delta;         // batch * n_heads * seq fp32
     void* dkv_part;      // bmt_flash_attn_bwd_parts floats, or NULL

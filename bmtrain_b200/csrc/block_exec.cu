@@ -1,4 +1,4 @@
-// Native executors for whole transformer blocks: pre-LN GPT and, below, the Llama-shaped one.  GPT: the whole forward (9 launches) or backward (21 launches) of a
+// Native executors for whole transformer blocks: pre-LN GPT and, below, the Llama-shaped one.  GPT: the whole forward (9 launches) or backward (15 launches) of a
 // transformer layer is issued from C++ by a single call, so the host cost per layer is a few microseconds instead
 // of one Python/autograd round trip per operator.  Every contraction goes to the tcgen05 GEMM (gemm_sm100.cu) with
 // fused epilogues: bias, ReLU, residual add, ReLU-mask / GELU-derivative on the dgrad path.
@@ -151,7 +151,6 @@ extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockG
         g.accumulate = w.acc_w;
         RUN(gemm(k, g, stream));
     }
-    RUN(bmt_colsum_ex(q.T, q.d, w.dy, dt, w.d_fc2_b, w.acc_small, k.colsum_scratch, k.colsum_scratch_bytes, stream));
     {   // d_ln2 = d_ff W_1
         BmtGemmDesc g = plain(q.T, q.d, q.dff, w.d_ff, q.dff, 0, k.fc1_w, q.d, 1, w.d_ln2, q.d, dt);
         RUN(gemm(k, g, stream));
@@ -161,10 +160,9 @@ extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockG
         g.accumulate = w.acc_w;
         RUN(gemm(k, g, stream));
     }
-    RUN(bmt_colsum_ex(q.T, q.dff, w.d_ff, dt, w.d_fc1_b, w.acc_small, k.colsum_scratch, k.colsum_scratch_bytes, stream));
     // d_h1 = dy + LN2'(d_ln2)
-    RUN(bmt_norm_bwd_ex(q.T, q.d, k.h1, w.d_ln2, k.ln2_w, k.stats2, 0, dt, w.nblk, w.d_h1, w.norm_partial, w.d_ln2_w, w.d_ln2_b,
-                        w.dy, w.acc_small, stream));
+    int rows2 = 0, rows1 = 0;
+    RUN(bmt_norm_bwd_partial(q.T, q.d, k.h1, w.d_ln2, k.ln2_w, k.stats2, 0, dt, w.nblk, w.d_h1, w.norm_partial, w.dy, &rows2, stream));
     // ---- attention output projection
     {   // d_ctx = d_h1 W_o
         BmtGemmDesc g = plain(q.T, q.hd, q.d, w.d_h1, q.d, 0, k.out_w, q.hd, 1, w.d_ctx, q.hd, dt);
@@ -175,7 +173,6 @@ extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockG
         g.accumulate = w.acc_w;
         RUN(gemm(k, g, stream));
     }
-    RUN(bmt_colsum_ex(q.T, q.d, w.d_h1, dt, w.d_out_b, w.acc_small, k.colsum_scratch, k.colsum_scratch_bytes, stream));
     // ---- attention core
     const int64_t pl = k.probs_ld;
     if (k.lse) {
@@ -222,15 +219,20 @@ extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockG
         g.accumulate = w.acc_w;
         RUN(gemm(k, g, stream));
     }
-    RUN(bmt_colsum_ex(q.T, 3 * q.hd, w.d_qkv, dt, w.d_qkv_b, w.acc_small, k.colsum_scratch, k.colsum_scratch_bytes, stream));
     // dx = d_h1 + LN1'(d_ln1)
-    RUN(bmt_norm_bwd_ex(q.T, q.d, k.x, w.d_ln2, k.ln1_w, k.stats1, 0, dt, w.nblk, w.dx, w.norm_partial, w.d_ln1_w, w.d_ln1_b,
-                        w.d_h1, w.acc_small, stream));
+    RUN(bmt_norm_bwd_partial(q.T, q.d, k.x, w.d_ln2, k.ln1_w, k.stats1, 0, dt, w.nblk, w.dx, w.norm_partial2, w.d_h1, &rows1, stream));
+    // everything that is a column sum, in one launch
+    const float *p2 = (const float*)w.norm_partial, *p1 = (const float*)w.norm_partial2;
+    const BmtColsum sums[8] = {{w.dy, q.T, q.d, w.d_fc2_b, 0, 0}, {w.d_ff, q.T, q.dff, w.d_fc1_b, 0, 0},
+                               {w.d_h1, q.T, q.d, w.d_out_b, 0, 0}, {w.d_qkv, q.T, 3 * q.hd, w.d_qkv_b, 0, 0},
+                               {p2, rows2, q.d, w.d_ln2_w, 1, 0}, {p2 + rows2 * q.d, rows2, q.d, w.d_ln2_b, 1, 0},
+                               {p1, rows1, q.d, w.d_ln1_w, 1, 0}, {p1 + rows1 * q.d, rows1, q.d, w.d_ln1_b, 1, 0}};
+    RUN(bmt_colsum_multi(sums, 8, dt, w.acc_small, k.colsum_scratch, k.colsum_scratch_bytes, stream));
     return 0;
 }
 
 // ------------------------------------------------------------------------------------------------- Llama-shaped block
-// 9 launches forward, 16 to 17 backward.  The residual additions happen in the epilogues of the projections and in the norms'
+// 9 launches forward, 17 to 18 backward.  The residual additions happen in the epilogues of the projections and in the norms'
 // backward (as operators of their own: six passes over (T, d) per block and step, 4 % of a block at 2048 x 8192).
 namespace {
 
@@ -296,7 +298,9 @@ extern "C" int bmt_llama_block_backward(const BmtLlamaBlock* blk, const BmtLlama
     RUN(bmt_swiglu_bwd(q.T, q.dff, k.gate_up, w.d_ff, dt, w.d_gate_up, stream));
     RUN(dgrad(w.d_gate_up, 2 * q.dff, k.gate_up_w, q.d, w.d_ln));
     RUN(wgrad(w.d_gate_up, 2 * q.dff, k.ln2, q.d, w.d_gate_up_w));
-    RUN(bmt_norm_bwd_ex(q.T, q.d, k.h1, w.d_ln, k.ln2_w, k.stats2, 1, dt, (int)w.nblk, w.d_h1, w.norm_partial, w.d_ln2_w, nullptr, w.dy, 0, stream));
+    int rows2 = 0, rows1 = 0;
+    float *p2 = (float*)w.norm_partial, *p1 = p2 + 2 * w.nblk * q.d;
+    RUN(bmt_norm_bwd_partial(q.T, q.d, k.h1, w.d_ln, k.ln2_w, k.stats2, 1, dt, (int)w.nblk, w.d_h1, p2, w.dy, &rows2, stream));
     RUN(dgrad(w.d_h1, q.d, k.out_w, q.hd, w.d_ctx));
     RUN(wgrad(w.d_h1, q.d, k.ctx, q.hd, w.d_out_w));
     const int64_t qs[3] = {q.hd, q.dh, k.seq * q.hd}, ks[3] = {q.kd, q.dh, k.seq * q.kd};
@@ -307,6 +311,8 @@ extern "C" int bmt_llama_block_backward(const BmtLlamaBlock* blk, const BmtLlama
                      stream));
     RUN(dgrad(w.d_packed, q.qkv, k.qkv_w, q.d, w.d_ln));
     RUN(wgrad(w.d_packed, q.qkv, k.ln1, q.d, w.d_qkv_w));
-    RUN(bmt_norm_bwd_ex(q.T, q.d, k.x, w.d_ln, k.ln1_w, k.stats1, 1, dt, (int)w.nblk, w.dx, w.norm_partial, w.d_ln1_w, nullptr, w.d_h1, 0, stream));
+    RUN(bmt_norm_bwd_partial(q.T, q.d, k.x, w.d_ln, k.ln1_w, k.stats1, 1, dt, (int)w.nblk, w.dx, p1, w.d_h1, &rows1, stream));
+    const BmtColsum sums[2] = {{p2, rows2, q.d, w.d_ln2_w, 1, 0}, {p1, rows1, q.d, w.d_ln1_w, 1, 0}};
+    RUN(bmt_colsum_multi(sums, 2, dt, 0, nullptr, 0, stream));
     return 0;
 }

@@ -609,8 +609,10 @@ int bwd_stream_vpl(int vpl, Args... args) {
 
 template <typename T>
 int bwd(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, const void* stats, int rms, int nblk, void* dx,
-        void* partial, void* dw, void* db, cudaStream_t s, const void* dres = nullptr, bool acc = false) {
+        void* partial, void* dw, void* db, cudaStream_t s, const void* dres = nullptr, bool acc = false, int* left = nullptr) {
+    // `left`: the sums are left in `partial`, as so many rows of them
     const auto fold = [&](int blocks) {
+        if (left) { *left = blocks; return; }
         const unsigned g = (unsigned)((d + 31) / 32);
         if (acc) bmt::launch(norm_fold_kernel<T, true>, g, dim3(32, 32), 0, s, 1, (int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
         else bmt::launch(norm_fold_kernel<T>, g, dim3(32, 32), 0, s, 1, (int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
@@ -629,12 +631,12 @@ int bwd(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, c
                                     : bwd_stream_vpl<T, 16>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s);
         if (blocks < 0) return blocks;
         fold(blocks);
-        bmt_count_launch(2);
+        bmt_count_launch(left ? 1 : 2);
         return (int)cudaGetLastError();
     }
     norm_bwd_kernel<T><<<nblk, NT, 0, s>>>(rows, (int)d, (const T*)x, (const T*)dy, (const T*)w, (const float*)stats, rms, (T*)dx, (float*)partial, (const T*)dres);
     fold(nblk);
-    bmt_count_launch(2);
+    bmt_count_launch(left ? 1 : 2);
     return (int)cudaGetLastError();
 }
 
@@ -677,6 +679,16 @@ extern "C" int bmt_norm_bwd_ex(int64_t rows, int64_t d, const void* x, const voi
     cudaStream_t s = (cudaStream_t)stream;
     return dtype == BMT_DT_F16 ? bwd<__half>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, dw, db, s, dres, accumulate != 0)
                                : bwd<__nv_bfloat16>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, dw, db, s, dres, accumulate != 0);
+}
+
+extern "C" int bmt_norm_bwd_partial(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, const void* stats, int rms, int dtype,
+                                    int nblk, void* dx, void* partial, const void* dres, int* blocks, void* stream) {
+    *blocks = 0;
+    if (rows <= 0) return 0;
+    if (d % 8 != 0 || d > NT * 8 * MAXIT || dtype == BMT_DT_F32) return -3;
+    cudaStream_t s = (cudaStream_t)stream;
+    return dtype == BMT_DT_F16 ? bwd<__half>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, nullptr, nullptr, s, dres, false, blocks)
+                               : bwd<__nv_bfloat16>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, nullptr, nullptr, s, dres, false, blocks);
 }
 
 // status of the norm backward: 0, or (1 << 16 | CTA) of the first CTA that gave up waiting for its rows; reading clears it

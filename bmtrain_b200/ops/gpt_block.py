@@ -50,13 +50,13 @@ class _Grad(ctypes.Structure):
         ("d_ff", _c_void_p), ("d_ln2", _c_void_p), ("d_h1", _c_void_p), ("d_ctx", _c_void_p), ("d_probs", _c_void_p),
         ("d_qkv", _c_void_p), ("norm_partial", _c_void_p), ("nblk", _int),
         ("dq_acc", _c_void_p), ("delta", _c_void_p),
-        ("acc_small", _int),
+        ("acc_small", _int), ("norm_partial2", _c_void_p),
     ]
 
 
 # The same in one go: packing the block costs the host 2 us, filling the structure field by field 12.
 _BLOCK = struct.Struct("@6q2ifi15Q4Qq8QQqQq")
-_GRAD = struct.Struct("@14Qi4x7Qi4x2Qi4x")
+_GRAD = struct.Struct("@14Qi4x7Qi4x2Qi4xQ")
 assert _BLOCK.size == ctypes.sizeof(_Block) and _GRAD.size == ctypes.sizeof(_Grad)
 _WORK = ("d_ff", "d_ln2", "d_h1", "d_ctx", "d_probs", "d_qkv", "norm_partial")
 
@@ -105,7 +105,7 @@ def _work_plan(b, s, d, n_heads, d_head, dff, fused_attn, nblk):
     """Scratch of a backward pass."""
     T, hd = b * s, n_heads * d_head
     sizes = [("d_ff", 2 * T * dff), ("d_ln2", 2 * T * d), ("d_h1", 2 * T * d), ("d_ctx", 2 * T * hd), ("d_qkv", 6 * T * hd),
-             ("norm_partial", 8 * nblk * d)]
+             ("norm_partial", 8 * nblk * d), ("norm_partial2", 8 * nblk * d)]
     if fused_attn:
         sizes += [("dq_acc", 4 * T * hd), ("delta", 4 * b * n_heads * s)]
     else:
@@ -164,7 +164,7 @@ class Pass:
         at = lambda name: base + plan[name] if name in plan else 0  # noqa: E731
         dx = torch.empty_like(self.x)
         g = _GRAD.pack(dy.data_ptr(), dx.data_ptr(), *grads, 1 if acc_weights else 0, *[at(n) for n in _WORK], nblk, at("dq_acc"), at("delta"),
-                       1 if acc_small else 0)
+                       1 if acc_small else 0, at("norm_partial2"))
         scratch = _gemm.scratch()
         if scratch is not self.scratch:         # another stream than the forward's
             self.tail = self.tail[:-4] + (*scratch.colsum, *scratch.gemm)

@@ -39,7 +39,7 @@ def _work_plan(b, s, d, h, hk, dh, dff, nblk):
     parts = lib.bmt_flash_attn_bwd_parts(i64(b), i64(s), c_int(h), c_int(hk), c_int(dh)) if hk != h else 0
     sizes = [("d_ff", 2 * T * dff), ("d_gate_up", 4 * T * dff), ("d_ln", 2 * T * d), ("d_h1", 2 * T * d), ("d_ctx", 2 * T * h * dh),
              ("dq", 2 * T * h * dh), ("dk", 2 * T * hk * dh), ("dv", 2 * T * hk * dh), ("d_packed", 2 * T * (h + 2 * hk) * dh),
-             ("norm_partial", 8 * nblk * d), ("dq_acc", 4 * T * h * dh), ("delta", 4 * T * h)]
+             ("norm_partial", 16 * nblk * d), ("dq_acc", 4 * T * h * dh), ("delta", 4 * T * h)]
     return _carve(sizes + [("dkv_part", 4 * parts)] if parts else sizes)
 
 
