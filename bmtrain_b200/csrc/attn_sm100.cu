@@ -117,60 +117,64 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
 //   bits_t (b, sk, query tiles, 4 words): the 128 queries of a tile as seen by one key (backward)
 //   cls    (b, query tiles, key tiles): 0 nothing visible, 1 mixed, 2 everything visible -- tiles of class 0 are skipped
 // Read per head and row, the bytes of a 437-key mask (rows not 16-byte aligned) took 3/4 of the attention kernel's time.
-constexpr int MASK_THREADS = 256;
+// A warp packs 32 queries x 32 keys with all its bytes in flight: a lane its query's keys from two 16-byte pieces, where the rows are
+// made of such, or else its key's queries; the other direction is the same 32 x 32 bits transposed in five shuffles.  Latency bounds
+// it up to some 500 tokens, then the bytes (1.8 - 2.1 TB/s).  With a vote per word and per key, and stores of single words:
+// 2 x 512 x 512 10.4 us, now 2.9; 3 x 437 x 437 10.4, now 3.8; 4096 x 4096 39, now 9.1; 8 x 2048 x 2048 71, now 16.
+constexpr int MASK_THREADS = 512;
+// Bit i of lane l <-> bit l of lane i.
+__device__ __forceinline__ uint32_t transpose_bits(uint32_t x, int lane) {
+#pragma unroll
+    for (int j = 16; j; j >>= 1) {
+        const uint32_t low = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu : j == 2 ? 0x33333333u : 0x55555555u;
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = lane & j ? (x & ~low) | ((y & ~low) >> j) : (x & low) | ((y & low) << j);
+    }
+    return x;
+}
 __global__ void __launch_bounds__(MASK_THREADS)
 attn_mask_pack_kernel(const uint8_t* mask, int64_t sq, int64_t sk, uint32_t* bits, uint32_t* bits_t, uint8_t* cls) {
     bmt::after_previous();
-    __shared__ uint32_t w[TILE][4];
-    __shared__ int any, full;
+    __shared__ __align__(16) uint32_t w[TILE][4], wt[TILE][4];      // of a query, of a key
     const int kt = blockIdx.x, qt = blockIdx.y, b = blockIdx.z, n_kt = gridDim.x, n_qt = gridDim.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t q0 = (int64_t)qt * TILE, k0 = (int64_t)kt * TILE;
-    if (threadIdx.x == 0) { any = 0; full = 1; }
-    __syncthreads();
-    // a warp takes 16 rows, 8 at a time: 32 loads in flight, then the ballots
-    for (int r0 = warp * 16; r0 < warp * 16 + 16; r0 += 8) {
-        uint8_t byte[8][4];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qw = warp >> 2, kw = warp & 3;
+    const int rows = (int)min((int64_t)TILE, sq - (int64_t)qt * TILE), keys = (int)min((int64_t)TILE, sk - (int64_t)kt * TILE);
+    const uint8_t* tile = mask + ((int64_t)b * sq + (int64_t)qt * TILE) * sk + (int64_t)kt * TILE;
+    // warp (qw, kw): 32 queries x 32 keys
+    uint32_t by_query, by_key;
+    if (sk % 16 == 0 && (reinterpret_cast<uintptr_t>(mask) & 15) == 0) {
+        const int row = qw * 32 + lane, key = kw * 32;
+        uint4 v[2];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int u = 0; u < 2; ++u)
+            v[u] = row < rows && key + u * 16 < keys ? *reinterpret_cast<const uint4*>(tile + row * sk + key + u * 16) : make_uint4(0, 0, 0, 0);
+        // one bit per byte that is not 0: the product moves the lowest bits of the four bytes next to one another, without carries
+        const auto nibble = [](uint32_t x) { return ((__vcmpne4(x, 0u) & 0x01010101u) * 0x10204080u) >> 28; };
+        by_query = 0;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int64_t q = q0 + r0 + i, k = k0 + c * 32 + lane;
-                byte[i][c] = q < sq && k < sk ? mask[((int64_t)b * sq + q) * sk + k] : 0;
-            }
+        for (int u = 0; u < 2; ++u)
+            by_query |= (nibble(v[u].x) | nibble(v[u].y) << 4 | nibble(v[u].z) << 8 | nibble(v[u].w) << 12) << (16 * u);
+        by_key = transpose_bits(by_query, lane);
+    } else {
+        const int row = qw * 32, key = kw * 32 + lane;
+        uint8_t byte[32];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            uint32_t word[4], seen = 0;
-            bool all = true;
+        for (int i = 0; i < 32; ++i) byte[i] = row + i < rows && key < keys ? tile[(row + i) * sk + key] : 0;
+        by_key = 0;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                word[c] = __ballot_sync(0xffffffffu, byte[i][c] != 0);
-                seen |= word[c];
-                all = all && word[c] == low_bits(sk - (k0 + c * 32));
-            }
-            if (lane < 4) w[r0 + i][lane] = lane == 0 ? word[0] : lane == 1 ? word[1] : lane == 2 ? word[2] : word[3];
-            if (lane == 0 && q0 + r0 + i < sq) {
-                if (seen) any = 1;
-                if (!all) full = 0;
-                *reinterpret_cast<uint4*>(bits + ((((int64_t)b * sq + q0 + r0 + i) * n_kt) + kt) * 4) = make_uint4(word[0], word[1], word[2], word[3]);
-            }
-        }
+        for (int i = 0; i < 32; ++i) by_key |= (byte[i] ? 1u : 0u) << i;
+        by_query = transpose_bits(by_key, lane);
     }
-    __syncthreads();
+    w[qw * 32 + lane][kw] = by_query;
+    wt[kw * 32 + lane][qw] = by_key;
+    const bool any = __syncthreads_or(by_query != 0);
+    const bool full = __syncthreads_and(qw * 32 + lane >= rows || by_query == low_bits(keys - kw * 32));
     if (threadIdx.x == 0) cls[((int64_t)b * n_qt + qt) * n_kt + kt] = (uint8_t)(!any ? 0 : full ? 2 : 1);
-    // the 32 x 32 bit blocks transposed: lane = query, one ballot per key
-    for (int blk = warp; blk < 16; blk += MASK_THREADS / 32) {
-        const int qw = blk >> 2, kw = blk & 3;
-        const uint32_t mine = w[qw * 32 + lane][kw];
-        uint32_t out = 0;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const uint32_t t = __ballot_sync(0xffffffffu, (mine >> i) & 1u);
-            if (lane == i) out = t;
-        }
-        const int64_t k = k0 + kw * 32 + lane;
-        if (k < sk) bits_t[((((int64_t)b * sk + k) * n_qt) + qt) * 4 + qw] = out;
-    }
+    const int i = threadIdx.x;
+    if (i < rows)
+        *reinterpret_cast<uint4*>(bits + ((((int64_t)b * sq + (int64_t)qt * TILE + i) * n_kt) + kt) * 4) = *reinterpret_cast<const uint4*>(w[i]);
+    else if (i >= TILE && i - TILE < keys)
+        *reinterpret_cast<uint4*>(bits_t + ((((int64_t)b * sk + (int64_t)kt * TILE + i - TILE) * n_qt) + qt) * 4) = *reinterpret_cast<const uint4*>(wt[i - TILE]);
 }
 
 // Forward.  A CTA works on two tiles of 128 query rows (one when the grid would not fill the GPU) with a group of four
