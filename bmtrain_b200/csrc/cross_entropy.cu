@@ -28,71 +28,6 @@ template <typename T> __device__ __forceinline__ int64_t row_head(const T* row, 
     return h < n ? h : n;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) ce_row_stats_kernel(int64_t m, int64_t n, const T* __restrict__ x,
-                                                           const int64_t* __restrict__ target, int64_t vocab_start,
-                                                           float* __restrict__ out) {
-    __shared__ float scratch[33];
-    const int64_t row = blockIdx.x;
-    const T* __restrict__ xr = x + row * n;
-    constexpr int V = bmt::Vec16<T>::N;
-    // mx: largest logit so far; se: sum of 2^(x * log2e - ref) with ref = mx * log2e as it is rounded.  Taking the rounded product
-    // as the reference keeps the exponent exact to one rounding of the FMA; its distance from mx * log2e is made up for once, at
-    // the end.
-    float mx = -INFINITY, ref = 0.f, se = 0.f;
-    // Rows of an odd number of classes start anywhere: the few elements before the first 16-byte boundary and behind the last
-    // whole vector go one by one, the rest as vectors (4096 x 50257 bf16 element by element: 242 us forward, 356 us backward;
-    // 104 and 141 us so).
-    // U vectors per thread and trip: all loads are issued before the first use, the running maximum moves at most
-    // once per trip, and every element costs one FMA and one ex2
-    constexpr int U = 4;
-    constexpr float L2E = 1.4426950408889634f;
-    const int64_t head = row_head<T>(xr, n), nv = (n - head) / V, tail = head + nv * V;
-    const T* __restrict__ xv = xr + head;
-    const auto move_to = [&](float v) {
-        if (!(v > mx)) return;
-        const float r = fmaxf(v * L2E, LOWEST);
-        if (mx != -INFINITY) se *= ex2(ref - r);
-        mx = v;
-        ref = r;
-    };
-    for (int64_t i = threadIdx.x; i < head + n - tail; i += blockDim.x) {
-        const float f = bmt::Cvt<T>::to_f(xr[i < head ? i : tail + i - head]);
-        move_to(f);
-        se += ex2(fmaf(f, L2E, -ref));       // ref is 0 as long as all classes are hidden (-inf): they add nothing
-    }
-    for (int64_t i0 = threadIdx.x; i0 < nv; i0 += (int64_t)blockDim.x * U) {
-        bmt::Vec16<T> v[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (i0 + (int64_t)u * blockDim.x < nv) v[u] = bmt::ld16(xv + (i0 + (int64_t)u * blockDim.x) * V);
-        float lm = -INFINITY;
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (i0 + (int64_t)u * blockDim.x < nv) {
-#pragma unroll
-                for (int k = 0; k < V; ++k) lm = fmaxf(lm, bmt::Cvt<T>::to_f(v[u].v[k]));
-            }
-        move_to(lm);
-        const float off = -ref;
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (i0 + (int64_t)u * blockDim.x < nv) {
-#pragma unroll
-                for (int k = 0; k < V; ++k) se += ex2(fmaf(bmt::Cvt<T>::to_f(v[u].v[k]), L2E, off));
-            }
-    }
-    const float gmx = bmt::block_allreduce<true>(mx, scratch);
-    const float contrib = se == 0.f ? 0.f : se * ex2(-fmaf(gmx, L2E, -ref));   // zero: no class that counts (a NaN is not lost)
-    const float gse = bmt::block_allreduce<false>(contrib, scratch);
-    if (threadIdx.x == 0) {
-        const int64_t t = target[row] - vocab_start;
-        out[row] = gmx;
-        out[m + row] = gse;
-        out[2 * m + row] = (t >= 0 && t < n) ? bmt::Cvt<T>::to_f(xr[t]) : 0.f;
-    }
-}
-
 // Largest of the 8 values of a packet, found on packed pairs (no conversion to fp32 per element, so the compiler has no
 // reason to keep 8 converted values per packet alive between the maximum pass and the exponent pass).
 __device__ __forceinline__ float packet_max(const bmt::Vec16<__half>& v) {
@@ -106,89 +41,97 @@ __device__ __forceinline__ float packet_max(const bmt::Vec16<__nv_bfloat16>& v) 
     return __bfloat162float(__hmax(__low2bfloat16(m), __high2bfloat16(m)));
 }
 
-// (max, sum of exp relative to max) pairs combine associatively
-__device__ __forceinline__ void lse_combine(float& m, float& s, float m2, float s2) {
-    constexpr float L2E = 1.4426950408889634f;
-    const float nm = fmaxf(m, m2);
-    const float a = s == 0.f ? 0.f : s * ex2((m - nm) * L2E);       // zero: no class that counts yet
-    const float b = s2 == 0.f ? 0.f : s2 * ex2((m2 - nm) * L2E);
-    m = nm;
-    s = a + b;
-}
+__device__ __forceinline__ float packet_max(const bmt::Vec16<float>& v) { return fmaxf(fmaxf(v.v[0], v.v[1]), fmaxf(v.v[2], v.v[3])); }
 
-// Streaming form for rows of 16-byte vectors: a persistent grid walks over (row, trip) chunks of 256 * U vectors; the
-// loads of the next chunk are issued before the arithmetic on the current one, so every thread has U loads in flight all
-// the time.  One barrier per row: warps leave their (max, sum) pair in one of two alternating slot sets and thread 0
-// combines them.
+// Statistics of a row, one block each: its maximum, the sum of exp relative to it, the logit of its target.  Every thread has U
+// vectors in flight while it works on the U before them; the few elements before the first 16-byte boundary of a row (rows of an odd
+// number of classes start anywhere) and behind its last whole vector go one by one.  The bytes bound it, because little is issued for
+// an element beyond a conversion, an FMA, an ex2 and an addition; a persistent grid whose chunks were found by 64-bit divisions issued
+// twice as much, and held rows back for its last wave.  4096 x 50304 bf16: 91 us, now 66
+// (6.2 TB/s); 4096 x 50257, element by element at the edges in a kernel of its own: 88, now 67; 16384 x 10240: 93, now 68.
+// The rows go from the last to the first, so that the backward, which begins with the first, finds some in L2.
 template <typename T, int U>
-__global__ void __launch_bounds__(256) ce_row_stats_stream_kernel(int64_t m, int64_t n, int trips, const T* __restrict__ x,
-                                                                  const int64_t* __restrict__ target, int64_t vocab_start,
-                                                                  float* __restrict__ out) {
+__global__ void __launch_bounds__(256) ce_row_stats_kernel(int64_t m, int64_t n, const T* __restrict__ x, const int64_t* __restrict__ target,
+                                                           int64_t vocab_start, float* __restrict__ out) {
     bmt::after_previous();
     constexpr int V = bmt::Vec16<T>::N;
     constexpr float L2E = 1.4426950408889634f;
-    __shared__ float sm_m[2][8], sm_s[2][8];
+    __shared__ float sm_m[8], sm_s[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t nv = n / V;
-    const int64_t my_rows = (int64_t)blockIdx.x < m ? (m - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    const int64_t chunks = my_rows * trips;
-    bmt::Vec16<T> a[U], b[U];
-    const auto load = [&](bmt::Vec16<T>(&v)[U], int64_t c) {
-        const int64_t row = blockIdx.x + (c / trips) * gridDim.x;
-        const int64_t base = (c % trips) * (int64_t)U * 256 + threadIdx.x;
-        const T* __restrict__ xr = x + row * n;
+    const int64_t row = m - 1 - (int64_t)blockIdx.x;
+    const T* __restrict__ xr = x + row * n;
+    const int64_t head = row_head<T>(xr, n), nv = (n - head) / V, tail = head + nv * V;
+    const int64_t t = threadIdx.x == 0 ? target[row] - vocab_start : -1;
+    const T* __restrict__ p = xr + head + (int64_t)threadIdx.x * V;
+    int64_t left = nv - threadIdx.x;              // this thread has a vector at p + u * 256 * V where u * 256 < left
+    // (a vector that is not there is not set to something either: that would wait for the load in its place)
+    struct Trip { bmt::Vec16<T> v[U]; int in; } a, b;
+    const auto load = [&](Trip& to) {
+        to.in = left > U * 256 ? U * 256 : (int)left;
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (base + u * 256 < nv) v[u] = bmt::ld16(xr + (base + u * 256) * V);
+            if (u * 256 < to.in) to.v[u] = bmt::ld16(p + u * 256 * V);
+        p += U * 256 * V;
+        left -= U * 256;
     };
-    float mx = -INFINITY, se = 0.f;
-    int par = 0;
-    const auto process = [&](bmt::Vec16<T>(&v)[U], int64_t c) {
-        const int64_t row = blockIdx.x + (c / trips) * gridDim.x;
-        const int trip = (int)(c % trips);
-        const int64_t base = (int64_t)trip * U * 256 + threadIdx.x;
+    // mx: largest logit so far; se: sum of 2^(x * log2e + off), off = -mx * log2e as it is rounded.  Taking the rounded product as the
+    // reference keeps the exponent exact to one rounding of the FMA; its distance from mx * log2e is made up for once, at the end.
+    float mx = -INFINITY, off = 0.f, se = 0.f;    // (off is 0 as long as all classes are hidden: -inf adds nothing)
+    const auto move_to = [&](float v) {
+        if (!(v > mx)) return;
+        const float o = -fmaxf(v * L2E, LOWEST);
+        if (mx != -INFINITY) se *= ex2(o - off);
+        mx = v;
+        off = o;
+    };
+    const auto add = [&](const Trip& from) {
         float lm = -INFINITY;
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (base + u * 256 < nv) lm = fmaxf(lm, packet_max(v[u]));
-        if (lm > mx) { se *= ex2((mx - lm) * L2E); mx = lm; }   // mx = -inf: se is 0 and stays 0 (0 * 2^-inf)
-        const float off = mx == -INFINITY ? 0.f : -fmaxf(mx * L2E, LOWEST);
+            if (u * 256 < from.in) lm = fmaxf(lm, packet_max(from.v[u]));
+        move_to(lm);
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (base + u * 256 < nv) {
+            if (u * 256 < from.in) {
 #pragma unroll
-                for (int k = 0; k < V; ++k) se += ex2(fmaf(bmt::Cvt<T>::to_f(v[u].v[k]), L2E, off));
+                for (int k = 0; k < V; ++k) se += ex2(fmaf(bmt::Cvt<T>::to_f(from.v[u].v[k]), L2E, off));
             }
-        if (trip == trips - 1) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float m2 = __shfl_xor_sync(0xffffffffu, mx, o), s2 = __shfl_xor_sync(0xffffffffu, se, o);
-                lse_combine(mx, se, m2, s2);
-            }
-            if (lane == 0) { sm_m[par][warp] = mx; sm_s[par][warp] = se; }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                float gm = sm_m[par][0], gs = sm_s[par][0];
-#pragma unroll
-                for (int i = 1; i < 8; ++i) lse_combine(gm, gs, sm_m[par][i], sm_s[par][i]);
-                const int64_t t = target[row] - vocab_start;
-                out[row] = gm;
-                out[m + row] = gs;
-                out[2 * m + row] = (t >= 0 && t < n) ? bmt::Cvt<T>::to_f(x[row * n + t]) : 0.f;
-            }
-            par ^= 1;
-            mx = -INFINITY;
-            se = 0.f;
-        }
     };
-    if (chunks > 0) load(a, 0);
-    for (int64_t c = 0; c < chunks; c += 2) {
-        if (c + 1 < chunks) load(b, c + 1);
-        process(a, c);
-        if (c + 1 < chunks) {
-            if (c + 2 < chunks) load(a, c + 2);
-            process(b, c + 1);
-        }
+    load(a);
+    T hit = bmt::Cvt<T>::from_f(0.f);
+    if (t >= 0 && t < n) hit = xr[t];
+    if ((int64_t)threadIdx.x < head + n - tail) {
+        const float f = bmt::Cvt<T>::to_f(xr[threadIdx.x < head ? threadIdx.x : tail + threadIdx.x - head]);
+        move_to(f);
+        se += ex2(fmaf(f, L2E, off));
+    }
+    for (;;) {
+        const bool more = left > 0;
+        if (more) load(b);
+        add(a);
+        if (!more) break;
+        const bool again = left > 0;
+        if (again) load(a);
+        add(b);
+        if (!again) break;
+    }
+    // one factor takes a thread's sum to the row's maximum, so that its error enters once
+    const float warp_most = bmt::warp_max(mx);
+    if (lane == 0) sm_m[warp] = warp_most;
+    __syncthreads();
+    float most = sm_m[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) most = fmaxf(most, sm_m[i]);
+    se = bmt::warp_sum(se == 0.f ? 0.f : se * ex2(-fmaf(most, L2E, off)));      // zero: no class that counts (a NaN is not lost)
+    if (lane == 0) sm_s[warp] = se;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        se = sm_s[0];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) se += sm_s[i];
+        out[row] = most;
+        out[m + row] = se;
+        out[2 * m + row] = bmt::Cvt<T>::to_f(hit);
     }
 }
 
@@ -299,36 +242,19 @@ extern "C" int bmt_ce_row_stats(int64_t m, int64_t n, const void* logits, int dt
                                 void* out, void* stream) {
     if (m <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
-    static const bool streaming = [] { const char* e = getenv("BMT_CE_STREAM"); return !(e && atoi(e) == 0); }();
-    if (streaming && dtype != BMT_DT_F32 && n % 8 == 0 && n >= 2048 && ((uintptr_t)logits & 15) == 0) {
-        const int64_t per_thread = (n / 8 + 255) / 256;
-        // vectors per trip: the size that leaves the fewest slots of the last trip empty, the larger one when it does not matter
-        // (50304 classes: 25 vectors a thread, 4 trips of 8 101 us, 5 trips of 5 96 us)
-        int u = 8, trips = (int)((per_thread + 7) / 8);
-        for (int c : {6, 5, 4}) {
-            const int n_trips = (int)((per_thread + c - 1) / c);
-            if (n_trips * c < trips * u) { u = c; trips = n_trips; }
-        }
-#define BMT_CE_STREAM(T, UU)                                                                                                   \
-        do {                                                                                                                   \
-            static int per_sm = 0;   /* resident CTAs per SM of this instantiation: the grid is exactly one wave */           \
-            if (!per_sm && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ce_row_stats_stream_kernel<T, UU>, 256, 0) != cudaSuccess || per_sm < 1)) \
-                per_sm = 2;                                                                                                    \
-            const int64_t cap = (int64_t)148 * per_sm;                                                                         \
-            bmt::launch(ce_row_stats_stream_kernel<T, UU>, (unsigned)(m < cap ? m : cap), 256, 0, s, 1,                                    \
-                m, n, trips, (const T*)logits, (const int64_t*)target, vocab_start, (float*)out);                              \
-        } while (0)
-#define BMT_CE_STREAM_U(T) \
-        do { if (u == 4) BMT_CE_STREAM(T, 4); else if (u == 5) BMT_CE_STREAM(T, 5); else if (u == 6) BMT_CE_STREAM(T, 6); else BMT_CE_STREAM(T, 8); } while (0)
-        if (dtype == BMT_DT_F16) BMT_CE_STREAM_U(__half); else BMT_CE_STREAM_U(__nv_bfloat16);
-#undef BMT_CE_STREAM_U
-#undef BMT_CE_STREAM
-        bmt_count_launch(1);
-        return (int)cudaGetLastError();
-    }
-    if (dtype == BMT_DT_F16) ce_row_stats_kernel<__half><<<(unsigned)m, 256, 0, s>>>(m, n, (const __half*)logits, (const int64_t*)target, vocab_start, (float*)out);
-    else if (dtype == BMT_DT_BF16) ce_row_stats_kernel<__nv_bfloat16><<<(unsigned)m, 256, 0, s>>>(m, n, (const __nv_bfloat16*)logits, (const int64_t*)target, vocab_start, (float*)out);
-    else ce_row_stats_kernel<float><<<(unsigned)m, 256, 0, s>>>(m, n, (const float*)logits, (const int64_t*)target, vocab_start, (float*)out);
+    const auto run = [&](auto* zero) {
+        using T = std::remove_pointer_t<decltype(zero)>;
+        const int64_t per_thread = (n / bmt::Vec16<T>::N + 255) / 256;
+        // 5 vectors in flight, 4 where that leaves fewer places of the last trip empty (8: 85 us instead of 68 at 4096 x 50304); short
+        // rows take no more than they have (4096 x 1000: 11.0 us with 1, 12.9 with 5)
+        const auto places = [&](int u) { return (per_thread + u - 1) / u * u; };
+        const auto kernel = per_thread <= 1 ? ce_row_stats_kernel<T, 1> : per_thread <= 2 ? ce_row_stats_kernel<T, 2>
+                          : places(4) < places(5) ? ce_row_stats_kernel<T, 4> : ce_row_stats_kernel<T, 5>;
+        bmt::launch(kernel, (unsigned)m, 256, 0, s, 1, m, n, (const T*)logits, (const int64_t*)target, vocab_start, (float*)out);
+    };
+    if (dtype == BMT_DT_F16) run((__half*)nullptr);
+    else if (dtype == BMT_DT_BF16) run((__nv_bfloat16*)nullptr);
+    else run((float*)nullptr);
     bmt_count_launch(1);
     return (int)cudaGetLastError();
 }
