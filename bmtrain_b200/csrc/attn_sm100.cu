@@ -57,28 +57,12 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// Two fp32 multiply-adds / adds in one instruction.
-__device__ __forceinline__ uint64_t pack_f2(float a, float b) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack_f2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
+using bmt::add_f2;
+using bmt::fma_f2;
+using bmt::mul_f2;
+using bmt::pack2;
+using bmt::pack_f2;
+using bmt::unpack_f2;
 // A from tensor memory: lane = row, every column holds two consecutive 16-bit elements of the reduction dimension.
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_c, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -101,16 +85,6 @@ template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setma
 
 // The lowest `n` of 32 bits (n may be outside [0, 32]).
 __device__ __forceinline__ uint32_t low_bits(int64_t n) { return n >= 32 ? 0xffffffffu : n <= 0 ? 0u : ((1u << (int)n) - 1u); }
-
-template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
-template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
-    __half2 h = __floats2half2_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&h);
-}
-template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&h);
-}
 
 // Packs a dense mask (b, sq, sk) of bytes into bits, once per call instead of once per head: one block per 128 x 128 tile.
 //   bits   (b, sq, key tiles, 4 words): the 128 keys of a tile as seen by one query (forward)

@@ -40,6 +40,57 @@ template <typename T> __device__ __forceinline__ void st16(T* p, const Vec16<T>&
     *reinterpret_cast<Vec16<T>*>(p) = x;
 }
 
+// Two fp32 multiply-adds / adds in one instruction.
+__device__ __forceinline__ uint64_t pack_f2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack_f2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Two 16-bit values that lie next to one another as a pair of fp32 values, and back.
+template <typename T> __device__ __forceinline__ uint64_t to_f2(uint32_t two);
+template <> __device__ __forceinline__ uint64_t to_f2<__half>(uint32_t two) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
+    return pack_f2(f.x, f.y);
+}
+template <> __device__ __forceinline__ uint64_t to_f2<__nv_bfloat16>(uint32_t two) {
+    return pack_f2(__uint_as_float(two << 16), __uint_as_float(two & 0xffff0000u));
+}
+template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
+template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
+    __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+}
+template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+}
+template <typename T> __device__ __forceinline__ uint32_t from_f2(uint64_t v) {
+    float a, b;
+    unpack_f2(v, a, b);
+    return pack2<T>(a, b);
+}
+__device__ __forceinline__ float sum_f2(uint64_t v) {
+    float a, b;
+    unpack_f2(v, a, b);
+    return a + b;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -1,13 +1,13 @@
 // LayerNorm / RMSNorm forward and backward for sm_100a.
 //
-// Forward: persistent grids whose warp teams hold a row in registers, take exact two-pass statistics over it and issue the
-// next row's loads ahead of the arithmetic.  Saves (mean, rstd) per row.
+// Forward: a team of warps per row, which holds it in registers and takes exact two-pass statistics over it.  Saves (mean, rstd) per row.
 // Backward: persistent grids (at most nblk CTAs) that get whole rows as bulk copies through a ring in shared memory, produce dx
 // and keep partial dgamma / dbeta in registers, written once to a (blocks x d) fp32 scratch that a second kernel folds.
 // Both also exist with one CTA per row, staged in shared memory (BMT_NORM_STAGED=1, and the combinations the others do not take).
 // (The reference calls F.layer_norm: example/layers/layernorm.py:29.)
 #include <math.h>
 #include <stdlib.h>
+#include <type_traits>
 
 #include "api.h"
 #include "common.cuh"
@@ -151,230 +151,123 @@ __global__ void __launch_bounds__(1024) norm_fold_kernel(int d, int nblk, const 
     }
 }
 
-// Forward with the row held in registers: WPR warps share a row (8 / WPR rows per CTA at a time), every lane keeps VPL
-// 16-byte vectors, all of whose loads are issued before the first use; statistics are exact two-pass sums over the
-// registers, reduced with shuffles (and one shared-memory exchange when WPR > 1).  A persistent grid strides over the
-// rows.
-template <typename T, int VPL, int WPR>
-__global__ void __launch_bounds__(NT, 2) norm_fwd_reg_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __restrict__ w,
-                                                          const T* __restrict__ b, float eps, int rms, T* __restrict__ y,
-                                                          float* __restrict__ stats) {
-    constexpr int RPC = 8 / WPR;                       // rows a CTA works on at a time
-    __shared__ float ex[2][8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int sub = warp % WPR, slot = warp / WPR;     // position inside the row's warp team, row slot inside the CTA
-    const int64_t groups = (rows + RPC - 1) / RPC;
-    for (int64_t gi = blockIdx.x; gi < groups; gi += gridDim.x) {
-        const int64_t r = gi * RPC + slot;
-        const bool live = r < rows;
-        float f[VPL][8];
-        float s = 0.f;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-            const int c = ((v * WPR + sub) * 32 + lane) * 8;
-            if (live && c < d) {
-                const bmt::Vec16<T> t = bmt::ld16(x + r * d + c);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) { f[v][k] = bmt::Cvt<T>::to_f(t.v[k]); s += f[v][k]; }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) f[v][k] = 0.f;
-            }
-        }
-        float mean = 0.f;
-        if (!rms) {
-            s = bmt::warp_sum(s);
-            if (WPR > 1) {
-                if (lane == 0) ex[0][warp] = s;
-                __syncthreads();
-                s = 0.f;
-#pragma unroll
-                for (int i = 0; i < WPR; ++i) s += ex[0][slot * WPR + i];
-            }
-            mean = s / d;
-        }
-        float q = 0.f;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-            const int c = ((v * WPR + sub) * 32 + lane) * 8;
-            if (c < d) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) { const float t = f[v][k] - mean; q += t * t; }
-            }
-        }
-        q = bmt::warp_sum(q);
-        if (WPR > 1) {
-            if (lane == 0) ex[1][warp] = q;
-            __syncthreads();
-            q = 0.f;
-#pragma unroll
-            for (int i = 0; i < WPR; ++i) q += ex[1][slot * WPR + i];
-        }
-        const float rstd = rsqrtf(q / d + eps);
-        if (live && sub == 0 && lane == 0) { stats[r] = mean; stats[rows + r] = rstd; }
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-            const int c = ((v * WPR + sub) * 32 + lane) * 8;
-            if (live && c < d) {
-                // weight and bias stay hot in L1 (a few KB re-read by every row); keeping them in registers instead would
-                // halve the number of resident warps and with it the bytes in flight
-                const bmt::Vec16<T> wv = bmt::ld16(w + c);
-                bmt::Vec16<T> bv, o;
-                if (b) bv = bmt::ld16(b + c);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    float t = (f[v][k] - mean) * rstd * bmt::Cvt<T>::to_f(wv.v[k]);
-                    if (b) t += bmt::Cvt<T>::to_f(bv.v[k]);
-                    o.v[k] = bmt::Cvt<T>::from_f(t);
-                }
-                bmt::st16(y + r * d + c, o);
-            }
-        }
-        if (WPR > 1) __syncthreads();   // the exchange slots are reused by the next group
-    }
-}
-
-// Streaming form of the kernel above: the row stays packed (16-byte vectors) in registers and the loads of the CTA's next
-// group of rows are issued before the arithmetic on the current one starts, so every warp has VPL loads in flight all the
-// time instead of only at the top of each row.  The exchange slots of a row's warp team alternate between two sets, which
-// saves the barrier at the end of a group.
-template <typename T, int VPL, int WPR>
-__global__ void __launch_bounds__(NT, VPL <= 4 ? 3 : 2) norm_fwd_stream_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __restrict__ w,
-                                                             const T* __restrict__ b, float eps, int rms, T* __restrict__ y,
-                                                             float* __restrict__ stats) {
+// Forward: a team of WPR warps has a row in its registers, a block one row or, if a warp is a team, four.  All loads are issued before
+// the first use; statistics are exact two-pass sums over the registers.  Bytes bound it once little is issued for an element: values are
+// worked on in pairs, blocks come and go instead of a resident grid striding over the rows with the next row's loads ahead of its
+// arithmetic (which left an SM 16 warps, and issued 19 instructions for an element).  16384 x 5120 bf16, RMSNorm: 66 us with the
+// resident grid, now 51 (6.6 TB/s); LayerNorm 85, now 54; 1024 x 2560 6.4, now 3.8.
+constexpr int FWD_WARPS(int wpr) { return wpr == 1 ? 4 : wpr; }
+template <typename T, int VPL, int WPR, bool RMS>
+__global__ void __launch_bounds__(FWD_WARPS(WPR) * 32) norm_fwd_row_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __restrict__ w,
+                                                                           const T* __restrict__ b, float eps, T* __restrict__ y,
+                                                                           float* __restrict__ stats) {
     bmt::after_previous();
-    constexpr int RPC = 8 / WPR;
-    __shared__ float ex[2][2][8];
+    constexpr int RPC = FWD_WARPS(WPR) / WPR;          // 1, or 4 teams without a barrier
+    __shared__ float ex[2][FWD_WARPS(WPR)];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = warp % WPR, slot = warp / WPR;
-    const int64_t groups = (rows + RPC - 1) / RPC;
-    bmt::Vec16<T> cur[VPL], nxt[VPL];
-    const auto load = [&](bmt::Vec16<T>(&v)[VPL], int64_t gi) {
-        const int64_t r = gi * RPC + slot;
-        if (r < rows) {
+    const int64_t r = (int64_t)blockIdx.x * RPC + slot;
+    const bool live = r < rows;                        // the same for a team
+    const int c0 = live ? (sub * 32 + lane) * 8 : d;   // the lane's vectors: columns c0 + i * WPR * 256 below d
+    const auto team_sum = [&](float v, int which) {
+        v = bmt::warp_sum(v);
+        if (WPR == 1) return v;
+        if (lane == 0) ex[which][warp] = v;
+        __syncthreads();
+        v = 0.f;
 #pragma unroll
-            for (int i = 0; i < VPL; ++i) {
-                const int c = ((i * WPR + sub) * 32 + lane) * 8;
-                if (c < d) v[i] = bmt::ld16(x + r * d + c);
-            }
-        }
+        for (int i = 0; i < WPR; ++i) v += ex[which][slot * WPR + i];
+        return v;
     };
-    int64_t gi = blockIdx.x;
-    if (gi < groups) load(cur, gi);
-    int par = 0;
-    for (; gi < groups; gi += gridDim.x, par ^= 1) {
-        if (gi + gridDim.x < groups) load(nxt, gi + gridDim.x);
-        const int64_t r = gi * RPC + slot;
-        const bool live = r < rows;
-        float mean = 0.f;
-        if (!rms) {
-            float s = 0.f;
+    const T* __restrict__ xr = x + r * d;
+    bmt::Vec16<T> raw[VPL];
 #pragma unroll
-            for (int i = 0; i < VPL; ++i) {
-                const int c = ((i * WPR + sub) * 32 + lane) * 8;
-                if (live && c < d) {
+    for (int i = 0; i < VPL; ++i)
+        if (c0 + i * WPR * 256 < d) raw[i] = bmt::ld16(xr + c0 + i * WPR * 256);
+    uint64_t f[VPL][4], acc = 0;
+    float mean = 0.f;
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) s += bmt::Cvt<T>::to_f(cur[i].v[k]);
+    for (int i = 0; i < VPL; ++i)
+        if (c0 + i * WPR * 256 < d) {
+            const uint32_t* u = reinterpret_cast<const uint32_t*>(raw[i].v);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                f[i][k] = bmt::to_f2<T>(u[k]);
+                acc = RMS ? bmt::fma_f2(f[i][k], f[i][k], acc) : bmt::add_f2(acc, f[i][k]);
+            }
+        }
+    if (!RMS) {
+        mean = team_sum(bmt::sum_f2(acc), 0) / d;
+        const uint64_t minus = bmt::pack_f2(-mean, -mean);
+        acc = 0;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i)
+            if (c0 + i * WPR * 256 < d) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    f[i][k] = bmt::add_f2(f[i][k], minus);
+                    acc = bmt::fma_f2(f[i][k], f[i][k], acc);
                 }
             }
-            s = bmt::warp_sum(s);
-            if (WPR > 1) {
-                if (lane == 0) ex[par][0][warp] = s;
-                __syncthreads();
-                s = 0.f;
-#pragma unroll
-                for (int i = 0; i < WPR; ++i) s += ex[par][0][slot * WPR + i];
-            }
-            mean = s / d;
-        }
-        float q = 0.f;
-#pragma unroll
-        for (int i = 0; i < VPL; ++i) {
-            const int c = ((i * WPR + sub) * 32 + lane) * 8;
-            if (live && c < d) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) { const float t = bmt::Cvt<T>::to_f(cur[i].v[k]) - mean; q += t * t; }
-            }
-        }
-        q = bmt::warp_sum(q);
-        if (WPR > 1) {
-            if (lane == 0) ex[par][1][warp] = q;
-            __syncthreads();
-            q = 0.f;
-#pragma unroll
-            for (int i = 0; i < WPR; ++i) q += ex[par][1][slot * WPR + i];
-        }
-        const float rstd = rsqrtf(q / d + eps);
-        if (live && sub == 0 && lane == 0) { stats[r] = mean; stats[rows + r] = rstd; }
-#pragma unroll
-        for (int i = 0; i < VPL; ++i) {
-            const int c = ((i * WPR + sub) * 32 + lane) * 8;
-            if (live && c < d) {
-                const bmt::Vec16<T> wv = bmt::ld16(w + c);   // a few KB re-read by every row: stays in L1
-                bmt::Vec16<T> bv, o;
-                if (b) bv = bmt::ld16(b + c);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    float t = (bmt::Cvt<T>::to_f(cur[i].v[k]) - mean) * rstd * bmt::Cvt<T>::to_f(wv.v[k]);
-                    if (b) t += bmt::Cvt<T>::to_f(bv.v[k]);
-                    o.v[k] = bmt::Cvt<T>::from_f(t);
-                }
-                bmt::st16(y + r * d + c, o);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < VPL; ++i) cur[i] = nxt[i];
     }
+    const float rstd = rsqrtf(team_sum(bmt::sum_f2(acc), 1) / d + eps);
+    if (live && sub == 0 && lane == 0) { stats[r] = mean; stats[rows + r] = rstd; }
+    const uint64_t by = bmt::pack_f2(rstd, rstd);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i)
+        if (const int c = c0 + i * WPR * 256; c < d) {
+            const bmt::Vec16<T> wv = bmt::ld16(w + c);       // a few KB that every row reads: in L1
+            bmt::Vec16<T> bv, o;
+            if (b) bv = bmt::ld16(b + c);
+            const uint32_t *uw = reinterpret_cast<const uint32_t*>(wv.v), *ub = reinterpret_cast<const uint32_t*>(bv.v);
+            uint32_t* uo = reinterpret_cast<uint32_t*>(o.v);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint64_t t = bmt::mul_f2(f[i][k], by), m = bmt::to_f2<T>(uw[k]);
+                uo[k] = bmt::from_f2<T>(b ? bmt::fma_f2(t, m, bmt::to_f2<T>(ub[k])) : bmt::mul_f2(t, m));
+            }
+            bmt::st16(y + r * d + c, o);
+        }
 }
 
 template <typename T, int VPL, int WPR>
-void launch_fwd_reg(int64_t rows, int d, const void* x, const void* w, const void* b, float eps, int rms, void* y, void* stats,
-                    cudaStream_t s) {
-    const int64_t groups = (rows + (8 / WPR) - 1) / (8 / WPR);
-    static const bool stream = [] { const char* e = getenv("BMT_NORM_STAGED"); return !(e && atoi(e) == 2); }();
-    if (stream) {
-        const int64_t cap = 148 * (VPL <= 4 ? 3 : 2);
-        const int64_t grid = groups < cap ? groups : cap;
-        if (groups <= cap)      // no striding: see `launch`
-            bmt::launch(norm_fwd_stream_kernel<T, VPL, WPR>, (unsigned)grid, NT, 0, s, 1, rows, d, (const T*)x, (const T*)w, (const T*)b, eps,
-                        rms, (T*)y, (float*)stats);
-        else
-            norm_fwd_stream_kernel<T, VPL, WPR><<<(unsigned)grid, NT, 0, s>>>(rows, d, (const T*)x, (const T*)w, (const T*)b, eps, rms,
-                                                                              (T*)y, (float*)stats);
-        return;
-    }
-    const int64_t grid = groups < 148 * 2 ? groups : 148 * 2;
-    norm_fwd_reg_kernel<T, VPL, WPR><<<(unsigned)grid, NT, 0, s>>>(rows, d, (const T*)x, (const T*)w, (const T*)b, eps, rms, (T*)y,
-                                                                    (float*)stats);
+void launch_fwd_row(int64_t rows, int d, const void* x, const void* w, const void* b, float eps, int rms, void* y, void* stats, cudaStream_t s) {
+    constexpr int RPC = FWD_WARPS(WPR) / WPR;
+    const auto kernel = rms ? norm_fwd_row_kernel<T, VPL, WPR, true> : norm_fwd_row_kernel<T, VPL, WPR, false>;
+    bmt::launch(kernel, (unsigned)((rows + RPC - 1) / RPC), FWD_WARPS(WPR) * 32, 0, s, 1, rows, d, (const T*)x, (const T*)w, (const T*)b, eps, (T*)y,
+                (float*)stats);
 }
 
-template <typename T, int WPR>
-bool fwd_reg_vpl(int vpl, int64_t rows, int d, const void* x, const void* w, const void* b, float eps, int rms, void* y, void* stats,
-                 cudaStream_t s) {
-    if (vpl <= 2) launch_fwd_reg<T, 2, WPR>(rows, d, x, w, b, eps, rms, y, stats, s);
-    else if (vpl <= 4) launch_fwd_reg<T, 4, WPR>(rows, d, x, w, b, eps, rms, y, stats, s);
-    else if (vpl <= 6) launch_fwd_reg<T, 6, WPR>(rows, d, x, w, b, eps, rms, y, stats, s);
-    else if (vpl <= 8) launch_fwd_reg<T, 8, WPR>(rows, d, x, w, b, eps, rms, y, stats, s);
-    else return false;
-    return true;
+// vpl: vectors a lane has to hold
+template <typename T, int WPR, typename... Args>
+void fwd_row(int vpl, Args... args) {
+    if constexpr (WPR < 8) {
+        if (vpl <= 1) return launch_fwd_row<T, 1, WPR>(args...);
+        if (vpl == 2) return launch_fwd_row<T, 2, WPR>(args...);
+    }
+    if (vpl <= 3) return launch_fwd_row<T, 3, WPR>(args...);
+    if (vpl == 4) return launch_fwd_row<T, 4, WPR>(args...);
+    if constexpr (WPR == 8) {
+        if (vpl == 6) return launch_fwd_row<T, 6, WPR>(args...);
+        if (vpl > 6) return launch_fwd_row<T, 8, WPR>(args...);
+    }
+    launch_fwd_row<T, 5, WPR>(args...);
 }
 
 template <typename T>
 int fwd(int64_t rows, int64_t d, const void* x, const void* w, const void* b, float eps, int rms, void* y, void* stats, cudaStream_t s) {
-    // smallest warp team that keeps at most 8 vectors (64 values) per lane
-    static const bool use_reg = [] { const char* e = getenv("BMT_NORM_STAGED"); return !(e && atoi(e) == 1); }();
-    if (use_reg && d <= 16384) {
-        const int wpr = d <= 2048 ? 1 : d <= 4096 ? 2 : d <= 8192 ? 4 : 8;
-        const int vpl = (int)((d + 256 * wpr - 1) / (256 * wpr));
-        bool done = false;
-        if (wpr == 1) done = fwd_reg_vpl<T, 1>(vpl, rows, (int)d, x, w, b, eps, rms, y, stats, s);
-        else if (wpr == 2) done = fwd_reg_vpl<T, 2>(vpl, rows, (int)d, x, w, b, eps, rms, y, stats, s);
-        else if (wpr == 4) done = fwd_reg_vpl<T, 4>(vpl, rows, (int)d, x, w, b, eps, rms, y, stats, s);
-        else done = fwd_reg_vpl<T, 8>(vpl, rows, (int)d, x, w, b, eps, rms, y, stats, s);
-        if (done) {
-            bmt_count_launch(1);
-            return (int)cudaGetLastError();
-        }
+    static const bool staged = [] { const char* e = getenv("BMT_NORM_STAGED"); return e && atoi(e) == 1; }();
+    if (!staged && d <= 16384) {
+        // the smallest team with at most 5 vectors a lane (8 warps: up to 8)
+        const int need = (int)((d + 255) / 256);       // vectors, in warps
+        const int wpr = need <= 5 ? 1 : need <= 10 ? 2 : need <= 20 ? 4 : 8, vpl = (need + wpr - 1) / wpr;
+        const auto run = [&](auto team) { fwd_row<T, decltype(team)::value>(vpl, rows, (int)d, x, w, b, eps, rms, y, stats, s); };
+        if (wpr == 1) run(std::integral_constant<int, 1>());
+        else if (wpr == 2) run(std::integral_constant<int, 2>());
+        else if (wpr == 4) run(std::integral_constant<int, 4>());
+        else run(std::integral_constant<int, 8>());
+        bmt_count_launch(1);
+        return (int)cudaGetLastError();
     }
     norm_fwd_kernel<T><<<(unsigned)rows, NT, d * sizeof(float), s>>>(rows, (int)d, (const T*)x, (const T*)w, (const T*)b, eps, rms, (T*)y, (float*)stats);
     bmt_count_launch(1);
@@ -388,8 +281,10 @@ int fwd(int64_t rows, int64_t d, const void* x, const void* w, const void* b, fl
 // registers and then working on it ran at 0.41 of the copy rate (16384 x 5120 RMS 193 us), one row ahead in registers at 0.48
 // (160 us): a load takes longer than a row's arithmetic.  So whole rows come as bulk copies into a ring of up to BWD_STAGES
 // stages in shared memory, refilled by one thread right behind the barrier that every row has anyway; the rows' statistics
-// are fetched for BWD_BATCH rows at a time: 124 us (LayerNorm 194 -> 171, bound by its arithmetic).  RMSNorm (RMS) has no bias
-// and drops the second accumulator.
+// are fetched for BWD_BATCH rows at a time: 124 us (LayerNorm 194 -> 171).  Then the instructions bound it, 33 for an element: columns
+// are worked on in pairs, the stage to refill is carried along instead of found by a 64-bit division in the thread that all others
+// wait for, and LayerNorm too has three vectors a lane (it reads the row from shared memory twice): 89 us, LayerNorm 98.
+// RMSNorm (RMS) has no bias and drops the second accumulator.
 constexpr int BWD_STAGES = 8, BWD_BATCH = 32;
 __device__ int g_norm_status = 0;   // 0, or (1 << 16) | blockIdx.x of the first CTA whose wait for a bulk copy ran out
 
@@ -408,6 +303,7 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
                        const float* __restrict__ stats, T* __restrict__ dx, float* __restrict__ partial, const T* __restrict__ dres) {
     bmt::after_previous();
     constexpr int RPC = BwdTeam<WPR>::RPC, WARPS = BwdTeam<WPR>::THREADS / 32;
+    constexpr bool AGAIN = VPL > (RMS ? 3 : 2);        // a row is read from shared memory again: no registers for it
     extern __shared__ __align__(128) uint8_t ring[];   // stages x {x, dy[, dres]} x RPC rows; 2 * d floats at the end of the kernel
     __shared__ __align__(8) uint64_t full[BWD_STAGES];
     __shared__ int late[2];                            // by parity of the row: a thread's wait for its copy ran out
@@ -417,8 +313,7 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
     const uint32_t part_bytes = (uint32_t)(RPC * d * 2), stage_bytes = part_bytes * (dres ? 3 : 2);
     const int64_t groups = (rows + RPC - 1) / RPC;
     const int64_t n_it = (int64_t)blockIdx.x < groups ? (groups - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    auto refill = [&](int64_t it) {                    // one thread: the rows of iteration `it` into its stage
-        const int st = (int)(it % stages);
+    auto refill = [&](int64_t it, int st) {            // one thread: the rows of iteration `it` into stage it % stages
         const int64_t r0 = (blockIdx.x + it * gridDim.x) * RPC;
         const uint32_t bytes = (uint32_t)((rows - r0 < RPC ? rows - r0 : RPC) * d * 2);
         const uint32_t bar = bmt_tc::smem_u32(&full[st]), dst = bmt_tc::smem_u32(ring) + st * stage_bytes;
@@ -431,16 +326,16 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
         for (int i = 0; i < stages; ++i) bmt_tc::mbar_init(&full[i], 1);
         bmt_tc::fence_barrier_init();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        for (int64_t it = 0; it < stages && it < n_it; ++it) refill(it);
+        for (int it = 0; it < stages && it < n_it; ++it) refill(it, it);
         late[0] = late[1] = 0;
     }
-    float dg[VPL][8], db[RMS ? 1 : VPL][8];
+    uint64_t dg[VPL][4], db[RMS ? 1 : VPL][4];         // pairs of columns
     bmt::Vec16<T> wv[VPL];
 #pragma unroll
     for (int v = 0; v < VPL; ++v) {
         const int c = ((v * WPR + sub) * 32 + lane) * 8;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) { dg[v][k] = 0.f; if (!RMS) db[v][k] = 0.f; }
+        for (int k = 0; k < 4; ++k) { dg[v][k] = 0; if (!RMS) db[v][k] = 0; }
         if (c < d) wv[v] = bmt::ld16(w + c);
     }
     __syncthreads();
@@ -464,7 +359,13 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
         const T* xs = reinterpret_cast<const T*>(ring + st * stage_bytes) + slot * d;
         const T* gs = reinterpret_cast<const T*>(ring + st * stage_bytes + part_bytes) + slot * d;
         bmt::Vec16<T> xv[VPL], gv[VPL];
-        float s1 = 0.f, s2 = 0.f;
+        const uint64_t by = bmt::pack_f2(rstd, rstd), minus = bmt::pack_f2(-mean, -mean);
+        const auto xhat = [&](uint32_t u) {
+            const uint64_t f = bmt::to_f2<T>(u);
+            return bmt::mul_f2(RMS ? f : bmt::add_f2(f, minus), by);
+        };
+        const auto words = [](const bmt::Vec16<T>& v) { return reinterpret_cast<const uint32_t*>(v.v); };
+        uint64_t t1 = 0, t2 = 0;
 #pragma unroll
         for (int v = 0; v < VPL; ++v) {
             const int c = ((v * WPR + sub) * 32 + lane) * 8;
@@ -472,17 +373,17 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
                 xv[v] = bmt::ld16(xs + c);
                 gv[v] = bmt::ld16(gs + c);
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const float xh = (bmt::Cvt<T>::to_f(xv[v].v[k]) - mean) * rstd;
-                    const float g = bmt::Cvt<T>::to_f(gv[v].v[k]);
-                    const float wg = g * bmt::Cvt<T>::to_f(wv[v].v[k]);
-                    if (!RMS) s1 += wg;
-                    s2 += wg * xh;
-                    dg[v][k] += g * xh;
-                    if (!RMS) db[v][k] += g;
+                for (int k = 0; k < 4; ++k) {
+                    const uint64_t xh = xhat(words(xv[v])[k]), g = bmt::to_f2<T>(words(gv[v])[k]);
+                    const uint64_t wg = bmt::mul_f2(g, bmt::to_f2<T>(words(wv[v])[k]));
+                    if (!RMS) t1 = bmt::add_f2(t1, wg);
+                    t2 = bmt::fma_f2(wg, xh, t2);
+                    dg[v][k] = bmt::fma_f2(g, xh, dg[v][k]);
+                    if (!RMS) db[v][k] = bmt::add_f2(db[v][k], g);
                 }
             }
         }
+        float s1 = bmt::sum_f2(t1), s2 = bmt::sum_f2(t2);
         if (!RMS) s1 = bmt::warp_sum(s1);
         s2 = bmt::warp_sum(s2);
         const int par = (int)(it & 1);
@@ -491,7 +392,7 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
         failed = late[par] != 0;                       // not written again before all have passed the next row's barrier
         if (failed) break;
         // every warp is through with the previous row: its stage takes the row `stages - 1` ahead of this one
-        if (threadIdx.x == 0 && it > 0 && it - 1 + stages < n_it) refill(it - 1 + stages);
+        if (threadIdx.x == 0 && it > 0 && it - 1 + stages < n_it) refill(it - 1 + stages, st == 0 ? stages - 1 : st - 1);
         if (WPR > 1) {
             s1 = s2 = 0.f;
 #pragma unroll
@@ -499,6 +400,7 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
         }
         s1 = s1 / d;
         s2 = s2 / d;
+        const uint64_t less1 = bmt::pack_f2(-s1, -s1), less2 = bmt::pack_f2(-s2, -s2);
         const T* ds = reinterpret_cast<const T*>(ring + st * stage_bytes + 2 * part_bytes) + slot * d;
 #pragma unroll
         for (int v = 0; v < VPL; ++v) {
@@ -506,14 +408,12 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
             if (live && c < d) {
                 bmt::Vec16<T> o, rv;
                 if (dres) rv = bmt::ld16(ds + c);
-                const bmt::Vec16<T> xc = VPL > 3 ? bmt::ld16(xs + c) : xv[v], gc = VPL > 3 ? bmt::ld16(gs + c) : gv[v];
+                const bmt::Vec16<T> xc = AGAIN ? bmt::ld16(xs + c) : xv[v], gc = AGAIN ? bmt::ld16(gs + c) : gv[v];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const float xh = (bmt::Cvt<T>::to_f(xc.v[k]) - mean) * rstd;
-                    const float wg = bmt::Cvt<T>::to_f(gc.v[k]) * bmt::Cvt<T>::to_f(wv[v].v[k]);
-                    float val = rstd * (wg - s1 - xh * s2);
-                    if (dres) val += bmt::Cvt<T>::to_f(rv.v[k]);
-                    o.v[k] = bmt::Cvt<T>::from_f(val);
+                for (int k = 0; k < 4; ++k) {
+                    const uint64_t xh = xhat(words(xc)[k]), g = bmt::to_f2<T>(words(gc)[k]), m = bmt::to_f2<T>(words(wv[v])[k]);
+                    const uint64_t t = bmt::fma_f2(xh, less2, RMS ? bmt::mul_f2(g, m) : bmt::fma_f2(g, m, less1));
+                    reinterpret_cast<uint32_t*>(o.v)[k] = bmt::from_f2<T>(dres ? bmt::fma_f2(t, by, bmt::to_f2<T>(words(rv)[k])) : bmt::mul_f2(t, by));
                 }
                 bmt::st16(dx + r * d + c, o);
             }
@@ -530,7 +430,7 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
 #pragma unroll
         for (int v = 0; v < VPL; ++v)
 #pragma unroll
-            for (int k = 0; k < 8; ++k) { dg[v][k] = NAN; if (!RMS) db[v][k] = NAN; }
+            for (int k = 0; k < 4; ++k) { dg[v][k] = bmt::pack_f2(NAN, NAN); if (!RMS) db[v][k] = bmt::pack_f2(NAN, NAN); }
     }
     // combine the RPC row slots of this CTA (slot 0 ends up with the CTA's column sums); every copy into the ring has landed
     float* fold = reinterpret_cast<float*>(ring);
@@ -544,7 +444,10 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
                 const int c = ((v * WPR + sub) * 32 + lane) * 8;
                 if (c < d) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) { fold[c + k] = dg[v][k]; if (!RMS) fold[d + c + k] = db[v][k]; }
+                    for (int k = 0; k < 4; ++k) {
+                        reinterpret_cast<uint64_t*>(fold + c)[k] = dg[v][k];
+                        if (!RMS) reinterpret_cast<uint64_t*>(fold + d + c)[k] = db[v][k];
+                    }
                 }
             }
         }
@@ -555,7 +458,10 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
                 const int c = ((v * WPR + sub) * 32 + lane) * 8;
                 if (c < d) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) { dg[v][k] += fold[c + k]; if (!RMS) db[v][k] += fold[d + c + k]; }
+                    for (int k = 0; k < 4; ++k) {
+                        dg[v][k] = bmt::add_f2(dg[v][k], reinterpret_cast<const uint64_t*>(fold + c)[k]);
+                        if (!RMS) db[v][k] = bmt::add_f2(db[v][k], reinterpret_cast<const uint64_t*>(fold + d + c)[k]);
+                    }
                 }
             }
         }
@@ -566,9 +472,9 @@ norm_bwd_stream_kernel(int64_t rows, int d, int stages, const T* __restrict__ x,
             const int c = ((v * WPR + sub) * 32 + lane) * 8;
             if (c < d) {
 #pragma unroll
-                for (int k = 0; k < 8; k += 4) {
-                    *reinterpret_cast<float4*>(pg + c + k) = make_float4(dg[v][k], dg[v][k + 1], dg[v][k + 2], dg[v][k + 3]);
-                    if (!RMS) *reinterpret_cast<float4*>(pb + c + k) = make_float4(db[v][k], db[v][k + 1], db[v][k + 2], db[v][k + 3]);
+                for (int k = 0; k < 4; k += 2) {
+                    *reinterpret_cast<ulonglong2*>(pg + c + 2 * k) = make_ulonglong2(dg[v][k], dg[v][k + 1]);
+                    if (!RMS) *reinterpret_cast<ulonglong2*>(pb + c + 2 * k) = make_ulonglong2(db[v][k], db[v][k + 1]);
                 }
             }
         }
@@ -595,8 +501,7 @@ int launch_bwd_stream(int64_t rows, int d, const void* x, const void* dy, const 
                                                            (float*)partial, (const T*)dres);
         return (int)grid;
     };
-    if constexpr (VPL == 3 && WPR < 16) return rms ? run(norm_bwd_stream_kernel<T, VPL, WPR, true>) : -31;   // LayerNorm: 2 vectors at most
-    else return rms ? run(norm_bwd_stream_kernel<T, VPL, WPR, true>) : run(norm_bwd_stream_kernel<T, VPL, WPR, false>);
+    return rms ? run(norm_bwd_stream_kernel<T, VPL, WPR, true>) : run(norm_bwd_stream_kernel<T, VPL, WPR, false>);
 }
 
 template <typename T, int WPR, typename... Args>
@@ -619,9 +524,9 @@ int bwd(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, c
     };
     static const bool use_reg = [] { const char* e = getenv("BMT_NORM_STAGED"); return !(e && atoi(e) == 1); }();
     if (use_reg && d <= 16384 && !(rms && db)) {
-        // the narrowest team with at most 3 vectors a lane, 2 with the bias sums (LayerNorm 16384 x 5120: 223 us with 3,
-        // 171 with 2); above 12288 / 8192 columns the widest team
-        const int64_t nv = (d + 255) / 256, most = rms ? 3 : 2;   // nv: vectors a lane of one warp would have
+        // the narrowest team with at most 3 vectors a lane (16384 x 5120: RMSNorm 118 us with 2 at most, 89 with 3; LayerNorm 132 and 98;
+        // 4 or 5 gain nothing more); above 12288 columns the widest team
+        const int64_t nv = (d + 255) / 256, most = 3;   // nv: vectors a lane of one warp would have
         const int wpr = nv <= most ? 1 : nv <= 2 * most ? 2 : nv <= 4 * most ? 4 : nv <= 8 * most ? 8 : 16;
         const int vpl = (int)((nv + wpr - 1) / wpr);
         const int blocks = wpr == 1 ? bwd_stream_vpl<T, 1>(vpl, rows, (int)d, x, dy, w, stats, rms, nblk, dx, partial, dres, s)
