@@ -38,6 +38,8 @@ int bmt_adam_bf16_multi(const BmtAdamTable* tab, float beta1, float beta2, float
 
 int bmt_has_inf_nan_multi(const BmtPtrTable* tab, int dtype, void* out_flag_u8, void* stream);
 int bmt_sq_norm_multi(const BmtPtrTable* tab, int dtype, void* out_f32, void* stream);
+// Zeros; tab->n counts bytes.
+int bmt_zero_multi(const BmtPtrTable* tab, void* stream);
 int bmt_scale_multi(const BmtPtrTable* tab, int dtype, const void* coef_f32, void* stream);
 
 int bmt_ce_row_stats(int64_t m, int64_t n, const void* logits, int dtype, const void* target_i64, int64_t vocab_start,

@@ -109,3 +109,23 @@ def multi_scale(tensors: Sequence[torch.Tensor], coef: torch.Tensor) -> None:
                 tab.p[j], tab.n[j] = t.data_ptr(), t.numel()
             _native.check(lib.bmt_scale_multi(ctypes.byref(tab), ctypes.c_int(_DT[dtype]), _native.ptr(coef),
                                               _native.stream_handle()), "grad-scale kernel")
+
+
+def multi_zero(tensors: Sequence[torch.Tensor]) -> None:
+    """``t.zero_()`` for every tensor: contiguous ones on the current device in one launch per <=24."""
+    flat = []
+    for t in tensors:
+        if (type(t) is torch.Tensor and t.is_cuda and t.layout is torch.strided and t.dtype in _DT and t.is_contiguous()
+                and t.device.index == torch.cuda.current_device()):
+            if t.numel():
+                flat.append(t)
+                torch.autograd.graph.increment_version(t)
+        else:
+            t.zero_()
+    for i in range(0, len(flat), _MAX):
+        chunk = flat[i:i + _MAX]
+        tab = _PtrTable()
+        tab.count = len(chunk)
+        for j, t in enumerate(chunk):
+            tab.p[j], tab.n[j] = t.data_ptr(), t.numel() * t.element_size()
+        _native.check(_native.cuda_lib().bmt_zero_multi(ctypes.byref(tab), _native.stream_handle()), "zero kernel")

@@ -14,7 +14,7 @@ from itertools import chain
 
 import torch
 
-from ..ops import adam as _adam
+from ..ops import adam as _adam, infnan as _infnan
 from ._distributed import state_dict_gather
 
 
@@ -34,6 +34,7 @@ def _zero_grad(optimizer, set_to_none: bool) -> None:
     A block's reduce-scatter produces a fresh partition gradient every step, so its old gradient is simply dropped
     (the next reduction then writes instead of accumulating) -- no zero-fill kernel per parameter and no read-modify-
     write in the reduction.  Other parameters are zeroed (or set to None) as ``torch.optim.Optimizer.zero_grad`` does."""
+    keep = []
     for group in optimizer.param_groups:
         for p in group["params"]:
             if p.grad is None:
@@ -49,7 +50,9 @@ def _zero_grad(optimizer, set_to_none: bool) -> None:
             else:
                 p.grad.detach_()
                 p.grad.requires_grad_(False)
-                p.grad.zero_()
+                keep.append(p.grad)
+    if keep:
+        _infnan.multi_zero(keep)
 
 
 class AdamOptimizer(torch.optim.Optimizer):
