@@ -952,6 +952,17 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     if (warp == 13) tmem_dealloc(tmem, 512);
 }
 
+// Row `w` of all (sample, token, head); divisions of 32 bits where they do (a 64-bit one is a hundred instructions, for 16 bytes a thread).
+struct Place { int64_t b, q; int head; };
+__device__ __forceinline__ Place place_of(int64_t w, int64_t rows, int64_t sq, int h) {
+    if (rows <= 0x7fffffff) {
+        const uint32_t n = (uint32_t)w, tok = n / (uint32_t)h, b = tok / (uint32_t)sq;
+        return {b, tok - b * (uint32_t)sq, (int)(n - tok * (uint32_t)h)};
+    }
+    const int64_t tok = w / h, b = tok / sq;
+    return {b, tok - b * sq, (int)(w - tok * h)};
+}
+
 // delta[b, h, q] = sum_d dO[b, q, h, d] * O[b, q, h, d], and zeros in the same row of the dQ accumulator (b, h, sq, d); 16
 // lanes per row (head dims up to 128 are 16 vectors of 8), two rows per warp.
 template <typename T>
@@ -961,9 +972,9 @@ __global__ void attn_delta_kernel(const T* o, int64_t o_tok, int64_t o_head, int
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
     const int c = (threadIdx.x & 15) * 8;
     const bool ok = w < rows;
-    const int64_t tok = ok ? w / h : 0;
-    const int head = ok ? (int)(w - tok * h) : 0;
-    const int64_t bb = tok / sq, qi = tok - bb * sq, row = (bb * h + head) * sq + qi;
+    const Place at = place_of(ok ? w : 0, rows, sq, h);
+    const int head = at.head;
+    const int64_t bb = at.b, qi = at.q, row = (bb * h + head) * sq + qi;
     float acc = 0.f;
     if (ok && c < d) {
         const bmt::Vec16<T> a = bmt::ld16(o + bb * o_batch + qi * o_tok + head * o_head + c), g = bmt::ld16(dout + bb * g_batch + qi * g_tok + head * g_head + c);
@@ -985,9 +996,9 @@ __global__ void attn_dq_convert_kernel(const float* acc, T* dq, int64_t q_tok, i
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
     const int c = (threadIdx.x & 15) * 8;
     if (w >= rows || c >= d) return;
-    const int64_t tok = w / h;
-    const int head = (int)(w - tok * h);
-    const int64_t bb = tok / sq, qi = tok - bb * sq;
+    const Place at = place_of(w, rows, sq, h);
+    const int head = at.head;
+    const int64_t bb = at.b, qi = at.q;
     const float4* src = reinterpret_cast<const float4*>(acc + ((bb * h + head) * sq + qi) * d + c);
     const float4 a0 = src[0], a1 = src[1];
     bmt::Vec16<T> o;
@@ -1098,7 +1109,12 @@ int run_bwd(int64_t batch, int64_t sq, int64_t sk, int h, int hk, int d, const v
                                                                               dks[2], (T*)dv, dvs[0], dvs[1], dvs[2]);
         bmt_count_launch(1);
     }
-    bmt::launch(attn_dq_convert_kernel<T>, row_blocks, 256, 0, st, 1, (const float*)dq_acc, (T*)dq, dqs[0], dqs[1], dqs[2], rows, sq, h, d);
+    // Long grids wait for the kernel before them to end instead of for its last CTAs to begin: the backward of 2x4096, 20 x 128
+    // causal 473 us so, 486 with blocks that sit on the SMs early; 2x512, 32 x 80 (2048 blocks) 41.4 and 40.1.
+    if (row_blocks > 4u * 8u * (unsigned)bmt::sm_count())
+        attn_dq_convert_kernel<T><<<row_blocks, 256, 0, st>>>((const float*)dq_acc, (T*)dq, dqs[0], dqs[1], dqs[2], rows, sq, h, d);
+    else
+        bmt::launch(attn_dq_convert_kernel<T>, row_blocks, 256, 0, st, 1, (const float*)dq_acc, (T*)dq, dqs[0], dqs[1], dqs[2], rows, sq, h, d);
     bmt_count_launch(2);
     return cudaGetLastError() == cudaSuccess ? 0 : -33;
 }
