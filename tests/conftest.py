@@ -1,3 +1,4 @@
+import gc
 import os
 import sys
 
@@ -9,6 +10,13 @@ os.environ.setdefault("BMT_QUIET", "1")
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200)")
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _models_of_earlier_modules_are_gone():
+    """Modules refer to their parameters and back, so a test's model lives until the collector runs: not in the middle of a later test that
+    compares how much memory is allocated."""
+    gc.collect()
 
 
 @pytest.fixture(scope="session")
