@@ -184,8 +184,10 @@ __global__ void __launch_bounds__(FWD_WARPS(WPR) * 32) norm_fwd_row_kernel(int64
 #pragma unroll
     for (int i = 0; i < VPL; ++i)
         if (c0 + i * WPR * 256 < d) raw[i] = bmt::ld16(xr + c0 + i * WPR * 256);
-    uint64_t f[VPL][4], acc = 0;
-    float mean = 0.f;
+    // the sums add one value after another, in a fixed order: a mean that differs in its last bit moves roundings of the result, and with
+    // them the signs of activations near zero
+    uint64_t f[VPL][4];
+    float sum = 0.f, mean = 0.f;
 #pragma unroll
     for (int i = 0; i < VPL; ++i)
         if (c0 + i * WPR * 256 < d) {
@@ -193,24 +195,29 @@ __global__ void __launch_bounds__(FWD_WARPS(WPR) * 32) norm_fwd_row_kernel(int64
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 f[i][k] = bmt::to_f2<T>(u[k]);
-                acc = RMS ? bmt::fma_f2(f[i][k], f[i][k], acc) : bmt::add_f2(acc, f[i][k]);
+                float lo, hi;
+                bmt::unpack_f2(f[i][k], lo, hi);
+                if (RMS) sum = fmaf(hi, hi, fmaf(lo, lo, sum));
+                else { sum += lo; sum += hi; }
             }
         }
     if (!RMS) {
-        mean = team_sum(bmt::sum_f2(acc), 0) / d;
+        mean = team_sum(sum, 0) / d;
         const uint64_t minus = bmt::pack_f2(-mean, -mean);
-        acc = 0;
+        sum = 0.f;
 #pragma unroll
         for (int i = 0; i < VPL; ++i)
             if (c0 + i * WPR * 256 < d) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     f[i][k] = bmt::add_f2(f[i][k], minus);
-                    acc = bmt::fma_f2(f[i][k], f[i][k], acc);
+                    float lo, hi;
+                    bmt::unpack_f2(f[i][k], lo, hi);
+                    sum = fmaf(hi, hi, fmaf(lo, lo, sum));
                 }
             }
     }
-    const float rstd = rsqrtf(team_sum(bmt::sum_f2(acc), 1) / d + eps);
+    const float rstd = rsqrtf(team_sum(sum, 1) / d + eps);
     if (live && sub == 0 && lane == 0) { stats[r] = mean; stats[rows + r] = rstd; }
     const uint64_t by = bmt::pack_f2(rstd, rstd);
 #pragma unroll
@@ -238,29 +245,27 @@ void launch_fwd_row(int64_t rows, int d, const void* x, const void* w, const voi
                 (float*)stats);
 }
 
-// vpl: vectors a lane has to hold
+// vpl: vectors a lane has to hold; wide teams have at least 5
 template <typename T, int WPR, typename... Args>
 void fwd_row(int vpl, Args... args) {
-    if constexpr (WPR < 8) {
+    if constexpr (WPR == 1) {
         if (vpl <= 1) return launch_fwd_row<T, 1, WPR>(args...);
         if (vpl == 2) return launch_fwd_row<T, 2, WPR>(args...);
+        if (vpl == 3) return launch_fwd_row<T, 3, WPR>(args...);
+        if (vpl == 4) return launch_fwd_row<T, 4, WPR>(args...);
     }
-    if (vpl <= 3) return launch_fwd_row<T, 3, WPR>(args...);
-    if (vpl == 4) return launch_fwd_row<T, 4, WPR>(args...);
-    if constexpr (WPR == 8) {
-        if (vpl == 6) return launch_fwd_row<T, 6, WPR>(args...);
-        if (vpl > 6) return launch_fwd_row<T, 8, WPR>(args...);
-    }
-    launch_fwd_row<T, 5, WPR>(args...);
+    if (vpl <= 5) launch_fwd_row<T, 5, WPR>(args...);
+    else if (vpl == 6) launch_fwd_row<T, 6, WPR>(args...);
+    else if (vpl == 7) launch_fwd_row<T, 7, WPR>(args...);
+    else launch_fwd_row<T, 8, WPR>(args...);
 }
 
 template <typename T>
 int fwd(int64_t rows, int64_t d, const void* x, const void* w, const void* b, float eps, int rms, void* y, void* stats, cudaStream_t s) {
     static const bool staged = [] { const char* e = getenv("BMT_NORM_STAGED"); return e && atoi(e) == 1; }();
     if (!staged && d <= 16384) {
-        // the smallest team with at most 5 vectors a lane (8 warps: up to 8)
-        const int need = (int)((d + 255) / 256);       // vectors, in warps
-        const int wpr = need <= 5 ? 1 : need <= 10 ? 2 : need <= 20 ? 4 : 8, vpl = (need + wpr - 1) / wpr;
+        // the smallest team with at most 8 vectors a lane
+        const int wpr = d <= 2048 ? 1 : d <= 4096 ? 2 : d <= 8192 ? 4 : 8, vpl = (int)((d + 256 * wpr - 1) / (256 * wpr));
         const auto run = [&](auto team) { fwd_row<T, decltype(team)::value>(vpl, rows, (int)d, x, w, b, eps, rms, y, stats, s); };
         if (wpr == 1) run(std::integral_constant<int, 1>());
         else if (wpr == 2) run(std::integral_constant<int, 2>());
