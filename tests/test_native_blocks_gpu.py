@@ -98,3 +98,26 @@ def test_hooks_and_partial_training_go_through_the_modules(bmt_gpu):
 
     assert block._native_module(args, only_reads_parameters(block._module), training=True) is None
     assert block._native_module([x.float()], True) is None
+
+
+@pytest.mark.parametrize("tokens,d,d_ff", [(370, 2560, 10240), (2272, 2496, 7936), (128, 256, 4096)])
+def test_products_below_a_relu_are_not_divided(bmt_gpu, tokens, d, d_ff):
+    """The block gives the bits that products of whole tiles give (the first two sizes are planned as divided ones elsewhere)."""
+    from bmtrain_b200.ops import gpt_block
+
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    dims = {"qkv": (3 * d, d), "out": (d, d), "fc1": (d_ff, d), "fc2": (d, d_ff)}
+    rnd = lambda *s: (0.02 * torch.randn(*s, generator=gen, device="cuda")).bfloat16()  # noqa: E731
+    params = {n + "_w": rnd(*s) for n, s in dims.items()} | {n + "_b": rnd(s[0]) for n, s in dims.items()}
+    for n in ("ln1", "ln2"):
+        params[n + "_w"], params[n + "_b"] = 1 + rnd(d), rnd(d)
+    order = ("ln1_w", "ln1_b", "qkv_w", "qkv_b", "out_w", "out_b", "ln2_w", "ln2_b", "fc1_w", "fc1_b", "fc2_w", "fc2_b")
+    x = torch.randn(1, tokens, d, generator=gen, device="cuda").bfloat16()
+
+    def ran(without):
+        run = gpt_block.Pass(x, None, [params[n].data_ptr() for n in order], d // 64, 64, d_ff, "relu", 1e-5, True)
+        if without:
+            run.tail = run.tail[:-2] + (0, 0)
+        return run.forward()
+
+    assert torch.equal(ran(False), ran(True))
