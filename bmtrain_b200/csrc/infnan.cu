@@ -77,9 +77,20 @@ template <typename T> __global__ void __launch_bounds__(THREADS) infnan_kernel(c
 template <typename T> __global__ void __launch_bounds__(THREADS) sqnorm_kernel(const __grid_constant__ ChunkTable c, float* out) {
     __shared__ float scratch[33];
     float acc = 0.f;
+    // a vector's squares come together first: added to the thread's sum one by one, some two thousand roundings of one sign were 1.4e-6 of
+    // the result with 300 M fp16 values (now a few 1e-7)
     walk<T, SCAN_U>(c, false, [&](T*, const bmt::Vec16<T>& x) {
+        constexpr int N = bmt::Vec16<T>::N;
+        float s[N];
 #pragma unroll
-        for (int k = 0; k < bmt::Vec16<T>::N; ++k) { const float f = bmt::Cvt<T>::to_f(x.v[k]); acc += f * f; }
+        for (int k = 0; k < N; ++k) s[k] = bmt::Cvt<T>::to_f(x.v[k]);
+#pragma unroll
+        for (int k = 0; k < N / 2; ++k) s[k] = fmaf(s[k], s[k], s[k + N / 2] * s[k + N / 2]);
+#pragma unroll
+        for (int n = N / 4; n > 0; n /= 2)
+#pragma unroll
+            for (int k = 0; k < n; ++k) s[k] += s[k + n];
+        acc += s[0];
     }, [&](T* p) { const float f = bmt::Cvt<T>::to_f(*p); acc += f * f; });
     acc = bmt::block_allreduce<false>(acc, scratch);
     if (threadIdx.x == 0 && acc != 0.f) atomicAdd(out, acc);
