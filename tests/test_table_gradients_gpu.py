@@ -75,3 +75,32 @@ def test_left_to_autograd(bmt_gpu):
     held.zero_()
     _loss(emb, ids, x).backward(retain_graph=False)
     assert (held.double() - want.double()).norm() <= 2.0 ** -9 * want.double().norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_same_bits_with_and_without_zeros_attached(bmt_gpu, dtype):
+    """A tied table: the first pass, which leaves the gradient to autograd, and passes that add to zeros in place."""
+    emb, p = _table(bmt_gpu, dtype=dtype)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    perm = lambda: torch.randperm(300, generator=gen, device="cuda")  # noqa: E731
+    ids = torch.cat([perm(), perm()[:107]])             # one or two tokens a row: their order does not matter
+    x = torch.randn(40, 64, generator=gen, device="cuda").to(dtype)
+    _loss(emb, ids, x).backward()
+    first, held = p.grad.clone(), p.grad
+    for _ in range(2):
+        held.zero_()
+        _loss(emb, ids, x).backward()
+        assert p.grad is held and torch.equal(held, first)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_sums_are_rounded_before_they_are_added(bmt_gpu, dtype):
+    from bmtrain_b200.ops import embedding as E
+
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    ids = torch.randint(0, 300, (500,), generator=gen, device="cuda")
+    ids[:40], ids[40:140] = 17, 33                      # rows of many tokens, one beyond the limit of the per-row teams
+    g = (torch.randint(-128, 128, (500, 64), generator=gen, device="cuda") / 64).to(dtype)      # sums exact in any order
+    held = torch.randn(300, 64, generator=gen, device="cuda").to(dtype)
+    want = (held.float() + E.embedding_backward(ids, g, 300).float()).to(dtype)
+    assert torch.equal(E.embedding_backward(ids, g, 300, add_to=held), want)
