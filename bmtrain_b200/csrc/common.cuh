@@ -129,34 +129,66 @@ __device__ __forceinline__ float ex2_approx(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-// log2 of the normal distribution function at -u (u >= 0), without its -u^2 / 2 log2(e) and log2(t), t = 1 / (1 + 0.4 u): a polynomial in t, fitted
-// for this file at Chebyshev nodes in 64 bits (the form of the complementary error function in Press et al., Numerical Recipes, 6.2).
-// Largest error 1.3e-7.  Taken this way the distribution keeps its relative accuracy on the negative side (1e-6 at -5), where
-// 1 + erf(x / sqrt 2) loses it (5e-2), and costs an exponential, a reciprocal and ten multiplications where erff set the pace
-// of what used it.
-__device__ __forceinline__ float normal_tail_log2(float t) {
-    float q = 0.27669891715049744f;
-    q = fmaf(q, t, -1.4162087440490723f);
-    q = fmaf(q, t, 2.8286075592041016f);
-    q = fmaf(q, t, -2.5461032390594482f);
-    q = fmaf(q, t, 0.795098066329956f);
-    q = fmaf(q, t, -0.2670532763004303f);
-    q = fmaf(q, t, 0.5381326079368591f);
-    q = fmaf(q, t, 1.4383363723754883f);
-    return fmaf(q, t, -2.647508144378662f);
+// GELU of pairs.  The normal distribution function comes in two forms, neither with erff, which sets the pace of what uses it:
+// Below 1.3: Phi(x) = 1/2 + x P(x^2), P fitted for this file in 64 bits behind its first coefficient, as that is rounded, weighted for the relative
+// error of Phi on the negative side (3e-9).
+// Above: Phi(-u) = t 2^(q(t)) exp(-u^2 / 2), t = 1 / (1 + 0.3 u), q fitted for this file in 64 bits (the form of the complementary error function in
+// Press et al., Numerical Recipes, 6.2; largest error 7e-8).  It keeps its relative accuracy on the negative side (2e-6 at -5, where
+// 1 + erf(x / sqrt 2) has 6e-2), but for small u it has errors of 5e-7.
+// Largest errors between -1.3 and 1.3, as with erff: x Phi(x) 3.5e-7 relative, Phi(x) + x phi(x) 1.4e-7 absolute.
+constexpr float HALF_LOG2E = 0.7213475204444817f, NORMAL_NEAR = 1.3f;
+__device__ __forceinline__ uint64_t both(float a) { return pack_f2(a, a); }
+__device__ __forceinline__ uint64_t normal_near(uint64_t x) {
+    const uint64_t s = mul_f2(x, x);
+    uint64_t p = both(5.271343753e-07f);
+    p = fma_f2(p, s, both(-9.379426047e-06f));
+    p = fma_f2(p, s, both(1.158123778e-04f));
+    p = fma_f2(p, s, both(-1.188031165e-03f));
+    p = fma_f2(p, s, both(9.974041022e-03f));
+    p = fma_f2(p, s, both(-6.649051607e-02f));
+    p = fma_f2(p, s, both(0.39894229173660278f));
+    return fma_f2(x, p, both(0.5f));
 }
-constexpr float HALF_LOG2E = 0.7213475204444817f;
-// x * Phi(x)
-__device__ __forceinline__ float gelu(float x) {
-    const float u = fabsf(x), t = rcp_approx_ftz(fmaf(u, 0.4f, 1.f));
-    const float tail = t * ex2_approx(fmaf(u * -HALF_LOG2E, u, normal_tail_log2(t)));
-    return x * (x >= 0.f ? 1.f - tail : tail);
+__device__ __forceinline__ uint64_t normal_far_log2(uint64_t t) {     // q, in units of log 2
+    uint64_t q = both(0.1297198086977005f);
+    q = fma_f2(q, t, both(-0.041672442108392715f));
+    q = fma_f2(q, t, both(-0.49322715401649475f));
+    q = fma_f2(q, t, both(0.32053878903388977f));
+    q = fma_f2(q, t, both(0.087591201066970825f));
+    q = fma_f2(q, t, both(0.62215578556060791f));
+    q = fma_f2(q, t, both(1.4390027523040771f));
+    return fma_f2(q, t, both(-3.0625312328338623f));
 }
-// Phi(x) + x * phi(x)
-__device__ __forceinline__ float gelu_grad(float x) {
-    const float u = fabsf(x), t = rcp_approx_ftz(fmaf(u, 0.4f, 1.f)), e = ex2_approx(u * -HALF_LOG2E * u);
-    const float tail = t * e * ex2_approx(normal_tail_log2(t));
-    return (x >= 0.f ? 1.f - tail : tail) + x * 0.3989422804014327f * e;
+__device__ __forceinline__ uint64_t ex2_f2(uint64_t v) {
+    float a, b;
+    unpack_f2(v, a, b);
+    return pack_f2(ex2_approx(a), ex2_approx(b));
+}
+// Phi(x) where Phi(-|x|) by the second form is `far`
+__device__ __forceinline__ uint64_t normal_of(uint64_t x, uint64_t far) {
+    float a, b, na, nb, fa, fb;
+    unpack_f2(x, a, b);
+    unpack_f2(normal_near(x), na, nb);
+    unpack_f2(far, fa, fb);
+    return pack_f2(fabsf(a) < NORMAL_NEAR ? na : a >= 0.f ? 1.f - fa : fa, fabsf(b) < NORMAL_NEAR ? nb : b >= 0.f ? 1.f - fb : fb);
+}
+__device__ __forceinline__ uint64_t abs_f2(uint64_t x) { return x & 0x7fffffff7fffffffull; }
+__device__ __forceinline__ uint64_t normal_t(uint64_t u) {
+    float a, b;
+    unpack_f2(fma_f2(u, both(0.3f), both(1.f)), a, b);
+    return pack_f2(rcp_approx_ftz(a), rcp_approx_ftz(b));
+}
+// x Phi(x)
+__device__ __forceinline__ uint64_t gelu(uint64_t x) {
+    const uint64_t u = abs_f2(x), t = normal_t(u);
+    const uint64_t far = mul_f2(t, ex2_f2(fma_f2(mul_f2(u, both(-HALF_LOG2E)), u, normal_far_log2(t))));
+    return mul_f2(x, normal_of(x, far));
+}
+// Phi(x) + x phi(x)
+__device__ __forceinline__ uint64_t gelu_grad(uint64_t x) {
+    const uint64_t u = abs_f2(x), t = normal_t(u), e = ex2_f2(mul_f2(mul_f2(u, both(-HALF_LOG2E)), u));
+    const uint64_t far = mul_f2(mul_f2(t, e), ex2_f2(normal_far_log2(t)));
+    return fma_f2(mul_f2(x, both(0.3989422804014327f)), e, normal_of(x, far));
 }
 
 // ---- dependent launches -------------------------------------------------------------------------------------------------------

@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256) colsum_multi_kernel(const __grid_constant
     }
 }
 
-// 4096 x 27648 bf16: 126 us with erff, 80 now (0.86 of the copy rate)
+// 4096 x 27648 bf16: 128 us with erff, 107 here; the instructions bound it, no longer the bytes (0.64 of the copy rate)
 template <typename T>
 __global__ void __launch_bounds__(EW_THREADS) gelu_kernel(int64_t n8, const T* __restrict__ x, T* __restrict__ out) {
     bmt::after_previous();
@@ -219,11 +219,10 @@ __global__ void __launch_bounds__(EW_THREADS) gelu_kernel(int64_t n8, const T* _
 #pragma unroll
     for (int i = 0; i < EW_U; ++i) {
         if (first + i * EW_THREADS >= n8) continue;
+        const uint32_t* in = reinterpret_cast<const uint32_t*>(v[i].v);
         bmt::Vec16<T> o;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            o.v[k] = bmt::Cvt<T>::from_f(bmt::gelu(bmt::Cvt<T>::to_f(v[i].v[k])));
-        }
+        for (int k = 0; k < 4; ++k) reinterpret_cast<uint32_t*>(o.v)[k] = bmt::from_f2<T>(bmt::gelu(bmt::to_f2<T>(in[k])));
         bmt::st16(out + (first + i * EW_THREADS) * 8, o);
     }
 }

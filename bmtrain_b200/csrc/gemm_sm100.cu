@@ -358,6 +358,13 @@ __device__ __forceinline__ bool wait_partials(uint32_t* flag, int64_t pitch, int
     return ok;
 }
 
+// v *= gelu'(e)
+__device__ __forceinline__ void mul_gelu_grad(float (&v)[8], const float (&e)[8]) {
+#pragma unroll
+    for (int i = 0; i < 8; i += 2)
+        bmt::unpack_f2(bmt::mul_f2(bmt::pack_f2(v[i], v[i + 1]), bmt::gelu_grad(bmt::pack_f2(e[i], e[i + 1]))), v[i], v[i + 1]);
+}
+
 // Epilogue of one warp's 32 rows of a tile: tensor memory -> (alpha, bias, activation, mask, residual, old C) -> global.
 // tcgen05.ld hands every thread one row; written out that way, a store instruction touches 32 rows with 16 bytes each, which
 // cost 5.5 to 8 us per 128 x 256 tile and made every weight gradient of a 1024-token block epilogue-bound (2560 x 8192 x 1024:
@@ -445,8 +452,11 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, con
                 float e[8];
                 unpack8<T>(cur[it], e);
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    v[it][i] = EXTRA == 1 ? (p.round_first ? bmt::Cvt<T>::to_f(bmt::Cvt<T>::from_f(v[it][i])) : v[it][i]) + e[i] : EXTRA == 2 ? (e[i] > 0.f ? v[it][i] : 0.f) : v[it][i] * bmt::gelu_grad(e[i]);
+                for (int i = 0; i < 8; ++i) {
+                    if (EXTRA == 1) v[it][i] = (p.round_first ? bmt::Cvt<T>::to_f(bmt::Cvt<T>::from_f(v[it][i])) : v[it][i]) + e[i];
+                    else if (EXTRA == 2) v[it][i] = e[i] > 0.f ? v[it][i] : 0.f;
+                }
+                if (EXTRA == 3) mul_gelu_grad(v[it], e);
             }
             if (col_ok && it * 8 + sub < rows) store8(dst + it * d_step + c * 32, v[it]);
         }
@@ -485,12 +495,17 @@ __device__ __forceinline__ void epilogue_rows_any(const GemmParams& p, TC* cbase
             for (int i = 0; i < 8; ++i) {
                 v[i] = v[i] * p.alpha + bias[i];
                 if (p.act == 1) v[i] = fmaxf(v[i], 0.f);
-                else if (p.act == 2) v[i] = bmt::gelu(v[i]);
+            }
+            if (p.act == 2) {
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) bmt::unpack_f2(bmt::gelu(bmt::pack_f2(v[i], v[i + 1])), v[i], v[i + 1]);
             }
             if (p.aux_mode) {
                 load_row8_dt(p.aux, p.bias_dtype, row * p.ld_aux + col, n_ok, a_vec, e);
+                if (p.aux_mode == 1) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = p.aux_mode == 1 ? (e[i] > 0.f ? v[i] : 0.f) : v[i] * bmt::gelu_grad(e[i]);
+                    for (int i = 0; i < 8; ++i) v[i] = e[i] > 0.f ? v[i] : 0.f;
+                } else mul_gelu_grad(v, e);
             }
             if (p.residual) {
                 load_row8_dt(p.residual, p.bias_dtype, row * p.ldr + col, n_ok, r_vec, e);
