@@ -114,12 +114,7 @@ template <bool IsMax> __device__ __forceinline__ float block_allreduce(float v, 
     return r;
 }
 
-__device__ __forceinline__ float rcp_approx(float x) {      // keeps subnormal results; relative error 2^-23
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ float rcp_approx_ftz(float x) {  // without the instructions that those take
+__device__ __forceinline__ float rcp_approx_ftz(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
