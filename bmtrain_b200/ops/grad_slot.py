@@ -18,11 +18,27 @@ def watched(param: torch.Tensor) -> bool:
     return bool(param._backward_hooks or param._post_accumulate_grad_hooks)
 
 
+def _nothing(*_):
+    pass
+
+
+def _node_watched(node) -> bool:
+    """Whether hooks sit on the node that accumulates into a leaf; wrappers that reduce gradients register them there.  They are kept in a
+    dictionary, to which only the handle of a hook leads (3 us)."""
+    for register in (node.register_hook, node.register_prehook):
+        handle = register(_nothing)
+        hooks = handle.hooks_dict_ref()
+        handle.remove()
+        if hooks:
+            return True
+    return False
+
+
 def attached(ctx, position: int, param: torch.Tensor) -> Optional[torch.Tensor]:
     """``param.grad`` if a backward that is running (``ctx``, whose input number ``position`` is the leaf ``param``) may add to it itself and
     return nothing to autograd, or None.  That is what autograd would do with a gradient that it got: the engine executes the leaf's
     accumulation in this very pass (a ``backward``, not a ``grad``, whose inputs if given contain the leaf), nothing watches the
-    parameter, no graph of the gradient is asked for, and the gradient is there, plain and of the parameter's type.  Only on the default
+    parameter or that node, no graph of the gradient is asked for, and the gradient is there, plain and of the parameter's type.  Only on the default
     stream: elsewhere it is the engine that orders the accumulation with the leaf's own stream."""
     g = param.grad
     if (g is None or not g.is_cuda or g.dtype != param.dtype or g.shape != param.shape or not g.is_contiguous() or g.requires_grad
@@ -33,9 +49,11 @@ def attached(ctx, position: int, param: torch.Tensor) -> Optional[torch.Tensor]:
     if getattr(node, "variable", None) is not param:
         return None
     try:
-        return g if torch._C._will_engine_execute_node(node) else None
+        if not torch._C._will_engine_execute_node(node) or _node_watched(node):
+            return None
     except RuntimeError:        # torch.autograd.grad asks for this leaf
         return None
+    return g
 
 
 def find(param: Optional[torch.Tensor]):

@@ -104,3 +104,22 @@ def test_sums_are_rounded_before_they_are_added(bmt_gpu, dtype):
     held = torch.randn(300, 64, generator=gen, device="cuda").to(dtype)
     want = (held.float() + E.embedding_backward(ids, g, 300).float()).to(dtype)
     assert torch.equal(E.embedding_backward(ids, g, 300, add_to=held), want)
+
+
+@pytest.mark.parametrize("kind", ["register_hook", "register_prehook"])
+def test_hooks_on_the_accumulation(bmt_gpu, kind):
+    """Hooks on the node that accumulates a table's gradient are given the gradient."""
+    emb, p = _table(bmt_gpu)
+    ids, x = torch.randint(0, 300, (50,), device="cuda"), torch.randn(8, 64, device="cuda").half()
+    _loss(emb, ids, x).backward()
+    want, held = p.grad.clone(), p.grad
+    node = p.expand_as(p).grad_fn.next_functions[0][0]
+    seen = []
+    handle = getattr(node, kind)(lambda *grads: seen.append(grads[-1][0]))
+    held.zero_()
+    _loss(emb, ids, x).backward()
+    handle.remove()
+    assert len(seen) == 1 and torch.equal(seen[0], want) and torch.equal(held, want)
+    held.zero_()
+    _loss(emb, ids, x).backward()               # nobody watches any more
+    assert len(seen) == 1 and p.grad is held and torch.equal(held, want)
