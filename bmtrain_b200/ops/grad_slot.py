@@ -53,6 +53,7 @@ def attached(ctx, position: int, param: torch.Tensor) -> Optional[torch.Tensor]:
             return None
     except RuntimeError:        # torch.autograd.grad asks for this leaf
         return None
+    torch.autograd.graph.increment_version(g)
     return g
 
 

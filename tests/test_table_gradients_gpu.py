@@ -123,3 +123,14 @@ def test_hooks_on_the_accumulation(bmt_gpu, kind):
     held.zero_()
     _loss(emb, ids, x).backward()               # nobody watches any more
     assert len(seen) == 1 and p.grad is held and torch.equal(held, want)
+
+
+def test_in_place_additions_are_counted(bmt_gpu):
+    emb, p = _table(bmt_gpu)
+    ids, x = torch.randint(0, 300, (50,), device="cuda"), torch.randn(8, 64, device="cuda").half()
+    _loss(emb, ids, x).backward()
+    weight = torch.ones(1, device="cuda", dtype=torch.float16, requires_grad=True)
+    product = (p.grad * weight).sum()           # keeps p.grad for its own backward
+    _loss(emb, ids, x).backward()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        product.backward()
