@@ -84,6 +84,11 @@ class Feedforward(DistributedModule):
         return self.w_out(h)
 
 
+def _has_bias(projection) -> bool:
+    own = getattr(projection, "_parameters", {})        # as it stands: read as an attribute, a parameter on its own is gathered
+    return (own["bias"] if "bias" in own else projection.bias) is not None
+
+
 @reads_parameters_only
 class TransformerEncoder(DistributedModule):
     """One pre-LN block."""
@@ -105,9 +110,8 @@ class TransformerEncoder(DistributedModule):
         return torch.is_tensor(hidden) and self._fused_ok(hidden) and not bmt_inspect.tensor.debug.get("_inspect_tensor", False)
 
     def _fused_ok(self, hidden: torch.Tensor) -> bool:
-        attn = self._modules["attn"]
-        return (hidden.is_cuda and hidden.dim() == 3 and config["tp_size"] == 1 and _FUSED_BLOCK
-                and attn._modules["project_qkv"]._parameters["bias"] is not None
+        attn = self.attn
+        return (hidden.is_cuda and hidden.dim() == 3 and config["tp_size"] == 1 and _FUSED_BLOCK and _has_bias(attn.project_qkv)
                 and hidden.dtype in (torch.float16, torch.bfloat16) and attn.dim_head % 8 == 0)
 
     # A ``Block`` whose module is this one, as it stands, has it computed by the native executor without autograd inside (see

@@ -121,3 +121,27 @@ def test_products_below_a_relu_are_not_divided(bmt_gpu, tokens, d, d_ff):
         return run.forward()
 
     assert torch.equal(ran(False), ran(True))
+
+
+class _Wrapped(torch.nn.Module):
+    """A projection whose parameters are not its own."""
+
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    weight = property(lambda self: self.inner.weight)
+    bias = property(lambda self: self.inner.bias)
+
+    def forward(self, x):
+        return self.inner(x)
+
+
+def test_block_with_a_wrapped_projection(bmt_gpu):
+    bmt = bmt_gpu
+    enc = _gpt(bmt, torch.float16, 256, 4, 64, 512, "relu", True)
+    bmt.init_parameters(enc)
+    x = torch.randn(1, 40, 256, device="cuda").half()
+    want = enc(x)
+    enc.attn.project_qkv = _Wrapped(enc.attn.project_qkv)
+    assert torch.equal(enc(x), want)
