@@ -120,8 +120,13 @@ class TransformerEncoder(DistributedModule):
         """The parameters in the executor's order if it takes these arguments, else None."""
         if not (torch.is_tensor(hidden) and self._fused_ok(hidden) and hidden.numel() > 0 and self._bmt_deferred_gather is None):
             return None
-        m, a = self._modules, self._modules["attn"]
+        m = self._modules
+        if not all(type(m[name]) is cls for name, cls in (("ln_attn", LayerNorm), ("attn", Attention), ("ln_ff", LayerNorm), ("ff", Feedforward))):
+            return None                                  # other submodules
+        a = m["attn"]
         attn, ff, (b, s, d), inner = a._modules, m["ff"]._modules, hidden.shape, a.num_heads * a.dim_head
+        if not all(type(mod) is Linear for mod in (attn["project_qkv"], attn["project_out"], ff["w_in"], ff["w_out"])):
+            return None
         if mask is not None and (not torch.is_tensor(mask) or mask.shape != (b, s, s) or mask.device != hidden.device):
             return None
         params = [p for mod in (m["ln_attn"], attn["project_qkv"], attn["project_out"], m["ln_ff"], ff["w_in"], ff["w_out"])

@@ -90,10 +90,13 @@ class LlamaBlock(DistributedModule):
         if not (torch.is_tensor(hidden) and hidden.is_cuda and hidden.dim() == 3 and hidden.numel() > 0 and config["tp_size"] == 1
                 and hidden.dtype in (torch.float16, torch.bfloat16) and _FUSED_BLOCK and os.environ.get("BMT_FLASH_ATTN", "1") != "0"):
             return None
-        m, a = self._modules, self._modules["attn"]
+        m = self._modules
+        if not all(type(m[name]) is cls for name, cls in (("ln_attn", RMSNorm), ("attn", LlamaAttention), ("ln_ff", RMSNorm), ("ff", LlamaMLP))):
+            return None                                  # other submodules
+        a = m["attn"]
         attn, ff, d = a._modules, m["ff"]._modules, hidden.shape[-1]
         linears = (attn["project_qkv"], attn["project_out"], ff["w_gate_up"], ff["w_out"])
-        if any(mod._parameters["bias"] is not None for mod in linears):
+        if any(type(mod) is not Linear or mod._parameters["bias"] is not None for mod in linears):
             return None
         params = [mod._parameters["weight"] for mod in (m["ln_attn"], *linears[:2], m["ln_ff"], *linears[2:])]
         shapes = [tuple(p._original_shape) for p in params]

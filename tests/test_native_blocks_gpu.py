@@ -145,3 +145,19 @@ def test_block_with_a_wrapped_projection(bmt_gpu):
     want = enc(x)
     enc.attn.project_qkv = _Wrapped(enc.attn.project_qkv)
     assert torch.equal(enc(x), want)
+
+
+def test_block_with_other_submodules(bmt_gpu):
+    """A Llama block with another feed-forward layer of this package runs its modules."""
+    from bmtrain_b200.models.gpt import Feedforward
+
+    bmt = bmt_gpu
+    inner = _llama(bmt, torch.bfloat16, 256, 4, 4, 64, 512)
+    inner.ff = Feedforward(256, 512, bias=False, dtype=torch.bfloat16)
+    block = bmt.Block(inner)
+    bmt.init_parameters(block)
+    x = torch.randn(1, 64, 256, device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad():
+        assert torch.equal(block(x), block(x))
+    y, dx, grads = _step(block, [x], torch.ones_like(x))
+    assert torch.isfinite(dx).all() and len(grads) == 6
