@@ -197,9 +197,10 @@ class _Bucket:
             self._layout = (sizes, gaps, where)
         return self._layout
 
-    def views_current(self) -> bool:
-        data = self.storage.data
-        return self._views_of == (data.data_ptr(), data.dtype, data.numel())
+    def points_local(self) -> bool:
+        """Whether every parameter is the view of the partition that ``local_views`` gives, whoever may have assigned to its ``data``."""
+        self._refresh_views()
+        return all(s.param.data_ptr() == at and s.param.dtype == self.storage.dtype for s, at in zip(self.slots, self._local_at))
 
     def _refresh_views(self) -> None:
         data = self.storage.data
@@ -207,6 +208,7 @@ class _Bucket:
         if self._views_of != key:
             # the views keep the memory they look at alive, so an equal address is the same memory
             self._local_views = [data[s.lo - self.begin:s.hi - self.begin] for s in self.slots]
+            self._local_at = [view.data_ptr() for view in self._local_views]
             self._full_views = None
             if self.comm.size == 1:
                 sizes, _, where = self.layout()
@@ -640,8 +642,8 @@ class Block(torch.nn.Module):
         self._resident = self._pointing = True
 
     def _point_to_local(self) -> None:
-        if not self._pointing and all(b.views_current() for b in self._buckets.values()):
-            return                               # they have not been made to point anywhere else
+        if not self._pointing and all(b.points_local() for b in self._buckets.values()):
+            return                               # nothing has made them point anywhere else
         self._pointing = False
         for b in self._buckets.values():
             for s, view in zip(b.slots, b.local_views()):
@@ -892,7 +894,7 @@ class Block(torch.nn.Module):
         try:
             return self._native_pass(native, args).forward()
         finally:
-            b.full = b.work = None
+            self._release_params()
 
     def _native_backward(self, native, args, grad_out):
         _, b, slots = native

@@ -161,3 +161,24 @@ def test_block_with_other_submodules(bmt_gpu):
         assert torch.equal(block(x), block(x))
     y, dx, grads = _step(block, [x], torch.ones_like(x))
     assert torch.isfinite(dx).all() and len(grads) == 6
+
+
+def test_parameters_show_the_partition_after_a_pass(bmt_gpu):
+    """Whatever was assigned to a parameter's ``data``: a pass computes with the partition, and afterwards the parameters are its views again."""
+    bmt = bmt_gpu
+    block = bmt.Block(_llama(bmt, torch.bfloat16, 256, 4, 4, 64, 512))
+    bmt.init_parameters(block)
+    x = torch.randn(1, 64, 256, device="cuda", dtype=torch.bfloat16)
+    _step(block, [x], torch.ones_like(x))
+    want = [p.data_ptr() for p in block.parameters()]
+    values = [p.detach().clone() for p in block.parameters()]
+    for training in (True, False):
+        for p in block.parameters():
+            p.data = p.data.clone().zero_()
+        if training:
+            _step(block, [x], torch.ones_like(x))
+        else:
+            with torch.no_grad():
+                block(x)
+        assert [p.data_ptr() for p in block.parameters()] == want
+        assert all(torch.equal(p.detach(), v) for p, v in zip(block.parameters(), values))
