@@ -157,11 +157,31 @@ class _Scratch:
         self.stream = stream
 
 
-def scratch() -> _Scratch:
-    """The current stream's.  Streams beyond the last ``_MOST_SCRATCH`` that came to have one give theirs back: to the allocator, which
-    hands it out again in the order of the same stream."""
+class _CapturedScratch:
+    """The same for one captured call: a graph may be replayed next to anything else, on any stream, so what its launches use belongs to it
+    (to its memory pool), and they set the counters to zero themselves.  GEMMs do not divide tiles there."""
+
+    __slots__ = ("buf", "index", "stream")
+    gemm = (0, 0)
+
+    def __init__(self, index, stream):
+        self.buf, self.index, self.stream = None, index, stream
+
+    @property
+    def colsum(self):
+        if self.buf is None:
+            self.buf = torch.empty(_COLSUM_BYTES, dtype=torch.uint8, device=torch.device("cuda", self.index))
+            self.buf[:4096].zero_()
+        return self.buf.data_ptr(), _COLSUM_BYTES
+
+
+def scratch():
+    """The current stream's, or the captured call's own.  Streams beyond the last ``_MOST_SCRATCH`` that came to have one give theirs back: to the
+    allocator, which hands it out again in the order of the same stream."""
     index = torch._C._cuda_getDevice()
     stream = torch._C._cuda_getCurrentRawStream(index)
+    if torch._C._cuda_isCurrentStreamCapturing():
+        return _CapturedScratch(index, stream)
     got = _scratch.get((index, stream))
     if got is None:
         if len(_scratch) >= _MOST_SCRATCH:

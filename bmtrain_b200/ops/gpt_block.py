@@ -127,7 +127,7 @@ class Pass:
         self.saved = torch.empty(total, dtype=torch.uint8, device=x.device)
         base = self.saved.data_ptr()
         at = {name: base + offset for name, offset in self.plan.items()}
-        work = self.scratch = _gemm.scratch()
+        self.scratch = _gemm.scratch()
         self.addresses = addresses
         self.head = (b, s, d, n_heads, d_head, d_ff, 0 if x.dtype == torch.float16 else 1, 1 if act == "relu" else 2, eps, 1 if causal else 0,
                      0 if self.mask8 is None else self.mask8.data_ptr())
@@ -135,7 +135,7 @@ class Pass:
         # fused attention: scores and probabilities never reach memory, one log-sum-exp per row is kept instead
         self.tail = (at["ln1"], at["stats1"], at["qkv"], get("probs", 0), (s + 7) // 8 * 8 if "probs" in at else 0, at["ctx"], at["h1"], at["ln2"],
                      at["stats2"], at["ff"], get("pre", 0), get("lse", 0), get("mask_packed", 0),
-                     *work.colsum, *work.gemm)
+                     0, 0, *self.scratch.gemm)         # forward adds no columns
 
     def forward(self) -> torch.Tensor:
         y = torch.empty_like(self.x)
@@ -165,9 +165,8 @@ class Pass:
         dx = torch.empty_like(self.x)
         g = _GRAD.pack(dy.data_ptr(), dx.data_ptr(), *grads, 1 if acc_weights else 0, *[at(n) for n in _WORK], nblk, at("dq_acc"), at("delta"),
                        1 if acc_small else 0, at("norm_partial2"))
-        scratch = _gemm.scratch()
-        if scratch is not self.scratch:         # another stream than the forward's
-            self.tail = self.tail[:-4] + (*scratch.colsum, *scratch.gemm)
+        scratch = _gemm.scratch()               # the forward may have been on another stream
+        self.tail = self.tail[:-4] + (*scratch.colsum, *scratch.gemm)
         _native.check(_native.entry("bmt_gpt_block_backward", "bbp")(self.describe(), g, scratch.stream), "GPT block backward")
         return dx
 
