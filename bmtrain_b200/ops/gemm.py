@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from typing import Optional
 
 import torch
@@ -136,7 +137,9 @@ def gemm_tn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
 
 _COLSUM_BYTES = 4 * (1024 + 2 * 1024 * 1024)
 _MOST_SCRATCH = 16
-_scratch = {}
+_scratch = {}                   # by device and stream, the one that was used last at the end
+_scratch_order = threading.Lock()
+_latest = (None, None)
 
 
 class _Scratch:
@@ -176,17 +179,24 @@ class _CapturedScratch:
 
 
 def scratch():
-    """The current stream's, or the captured call's own.  Streams beyond the last ``_MOST_SCRATCH`` that came to have one give theirs back: to the
+    """The current stream's, or the captured call's own.  Streams beyond the last ``_MOST_SCRATCH`` that used one give theirs back: to the
     allocator, which hands it out again in the order of the same stream."""
+    global _latest
     index = torch._C._cuda_getDevice()
     stream = torch._C._cuda_getCurrentRawStream(index)
     if torch._C._cuda_isCurrentStreamCapturing():
         return _CapturedScratch(index, stream)
-    got = _scratch.get((index, stream))
-    if got is None:
-        if len(_scratch) >= _MOST_SCRATCH:
-            _scratch.pop(next(iter(_scratch)), None)
-        got = _scratch[(index, stream)] = _Scratch(index, stream)
+    key, (last, got) = (index, stream), _latest
+    if last == key:
+        return got
+    with _scratch_order:
+        got = _scratch.pop(key, None)
+        if got is None:
+            if len(_scratch) >= _MOST_SCRATCH:
+                del _scratch[next(iter(_scratch))]
+            got = _Scratch(index, stream)
+        _scratch[key] = got
+        _latest = (key, got)
     return got
 
 

@@ -20,7 +20,24 @@ def streams(monkeypatch):
     monkeypatch.setattr(torch._C, "_cuda_isCurrentStreamCapturing", lambda: state["capturing"], raising=False)
     monkeypatch.setattr(gemm, "_Scratch", Made)
     monkeypatch.setattr(gemm, "_scratch", {})
+    monkeypatch.setattr(gemm, "_latest", (None, None), raising=False)
     return gemm, state
+
+
+def test_streams_in_use_keep_their_scratch(streams):
+    gemm, state = streams
+
+    def on(stream):
+        state["stream"] = stream
+        return gemm.scratch()
+
+    main = on(0)
+    for stream in range(1, 3 * gemm._MOST_SCRATCH):
+        assert on(stream).stream == stream
+        assert on(0) is main                    # used all the time, so it is never the one that goes
+        assert len(gemm._scratch) <= gemm._MOST_SCRATCH
+    assert on(3 * gemm._MOST_SCRATCH - 1).stream == 3 * gemm._MOST_SCRATCH - 1
+    assert len(state["made"]) == 3 * gemm._MOST_SCRATCH
 
 
 def test_nothing_that_a_capture_made_is_kept(streams):
