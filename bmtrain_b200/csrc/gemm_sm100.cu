@@ -1394,7 +1394,6 @@ int make_map_mn5(CUtensorMap* out, const void* ptr, int dtype, int64_t mn, int64
     return 0;
 }
 
-int g_num_sms = 0;
 // SMs that fused (compute + collective) kernels leave free.  Their CTAs wait for other ranks while they hold their SM; when
 // kernels of another parallel dimension (NCCL gathers of a ZeRO group) must be able to start next to them at any time, a
 // few SMs stay out of the fused grids so that such a kernel always finds room (bmt_gemm_reserve_sms).
@@ -1415,7 +1414,8 @@ struct TileChoice { int bn, cta2, sk_tiles, sk_workers; };
 constexpr int SK_MIN = 4, SK_MOST = 8;      // k-blocks of a range at least, CTAs per tile at most
 constexpr double SK_COST = 16000.0;
 
-TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn, int force_bn, int force_cta2, bool split) {
+// `sms`: that do math
+TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn, int force_bn, int force_cta2, bool split, int sms) {
     TileChoice best{0, 0, 0, 0}, best_split{0, 0, 0, 0};
     double best_cost = 1e30, best_split_cost = 1e30;
     const int64_t kblocks = (K + BK - 1) / BK;
@@ -1427,7 +1427,7 @@ TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn
         for (int bn = (b_mn ? 64 : 32) * ncta; bn <= 256; bn += step) {
             if (force_bn > 0 && bn != force_bn) continue;
             const int64_t tiles = ((M + BM * ncta - 1) / (BM * ncta)) * ((N + bn - 1) / bn) * batches;
-            const int64_t slots = g_num_sms / ncta;
+            const int64_t slots = sms / ncta;
             const int64_t waves = (tiles + slots - 1) / slots;
             const double mma = 2.05 * bn, load = 2.0 * (128 + bn / ncta);
             const double per_block = mma > load ? mma : load, fixed = 600.0 + 6.0 * bn;   // + fill/drain and epilogue
@@ -1452,15 +1452,15 @@ TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn
 }
 
 // The choice for a problem costs 2 to 4 us of divisions; a thread keeps its last ones.
-TileChoice planned_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn, int force_bn, int force_cta2, bool split) {
+TileChoice planned_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn, int force_bn, int force_cta2, bool split, int sms) {
     struct Plan { int64_t m, n, k, batches; int how, sms; TileChoice tc; };
     static thread_local Plan plans[256];
     const int how = 1 + (b_mn ? 1 : 0) + (split ? 2 : 0) + 4 * (force_cta2 + 1) + 16 * force_bn;
     const uint64_t hash = ((uint64_t)M * 0x9e3779b97f4a7c15ull) ^ ((uint64_t)N * 0xc2b2ae3d27d4eb4full) ^ ((uint64_t)K * 0x165667b19e3779f9ull) ^
                           ((uint64_t)batches * 0x27d4eb2f165667c5ull) ^ ((uint64_t)how * 0x85ebca77c2b2ae63ull);
     Plan& p = plans[(hash >> 40) & 255];
-    if (p.how != how || p.m != M || p.n != N || p.k != K || p.batches != batches || p.sms != g_num_sms)
-        p = Plan{M, N, K, batches, how, g_num_sms, pick_tile(M, N, K, batches, b_mn, force_bn, force_cta2, split)};
+    if (p.how != how || p.m != M || p.n != N || p.k != K || p.batches != batches || p.sms != sms)
+        p = Plan{M, N, K, batches, how, sms, pick_tile(M, N, K, batches, b_mn, force_bn, force_cta2, split, sms)};
     return p.tc;
 }
 
@@ -1476,6 +1476,21 @@ void set_split(GemmParams& p, const TileChoice& tc, int k_blocks) {
 // CTAs (pairs) of a launch with split tiles: whole tiles come only in full waves.
 int64_t whole_or_split(int64_t tiles, int64_t slots, const TileChoice& tc) { return tiles > tc.sk_tiles ? slots : tc.sk_workers; }
 
+// Once, whichever thread comes first.
+int prepare_kernels() {
+    static std::atomic<bool> done{false};
+    if (done.load(std::memory_order_acquire)) return 0;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    if (done.load(std::memory_order_relaxed)) return 0;
+    const int most = (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512);
+    for (const auto kernel : {gemm_tcgen05_kernel<false, 0>, gemm_tcgen05_kernel<true, 0>, gemm_tcgen05_kernel<false, 1>, gemm_tcgen05_kernel<false, 2>,
+                              gemm_tcgen05_kernel<false, 3>, gemm_tcgen05_kernel<true, 1>, gemm_tcgen05_kernel<true, 2>, gemm_tcgen05_kernel<true, 3>})
+        BMT_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    done.store(true, std::memory_order_release);
+    return 0;
+}
+
 int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fused = nullptr) {
     const int64_t m = g.m, n = g.n, k = g.k;
     const void* a = g.a; const void* b = g.b; void* c = g.c; const void* bias = g.bias;
@@ -1487,19 +1502,8 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     const float alpha = g.alpha;
     if (m <= 0 || n <= 0 || batch_inner <= 0 || batch_outer <= 0) return 0;
     if (k <= 0) return -20;
-    if (g_num_sms == 0) {
-        int dev = 0;
-        BMT_CUDA_OK(cudaGetDevice(&dev));
-        BMT_CUDA_OK(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
-        BMT_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - SMEM_FIXED + 1024 + 512)));
-    }
+    const int sms = bmt::sm_count();
+    if (const int rc = prepare_kernels()) return rc;
     static int force_bn = -1, force_cta2 = -2;
     if (force_bn < 0) { const char* e = getenv("BMT_GEMM_BN"); force_bn = e ? atoi(e) : 0; }
     if (force_cta2 == -2) { const char* e = getenv("BMT_GEMM_CTA2"); force_cta2 = e ? atoi(e) : -1; }
@@ -1510,19 +1514,17 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     p.a_mn = a_major; p.b_mn = b_major;
     const int comm_ctas = (fused && (fused->mode == 2 || fused->mode == 3)) ? fused->ag_ctas : 0;
     const int held_back = fused ? comm_ctas + g_reserved_sms : 0;
-    if (fused) g_num_sms -= held_back;  // tile choice for the CTAs that do math
     // a fused kernel can run as CTA pairs when its pusher CTAs pair up too and (mode 2) a rank's rows fill whole 256-row tiles
     const bool pair_ok = !fused || (comm_ctas % 2 == 0 && (fused->mode != 2 || fused->ag_rows % (2 * BM) == 0));
     // Split tiles need scratch whose flags nobody else uses.  A captured launch may be replayed next to any other, on any stream: there
     // the tiles stay whole.
-    bool split = !fused && g.scratch && k < (1 << 26) && g.scratch_bytes >= sk_bytes(g_num_sms, 256);
+    bool split = !fused && g.scratch && k < (1 << 26) && g.scratch_bytes >= sk_bytes(sms, 256);
     if (split) {
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) { cudaGetLastError(); split = false; }
     }
-    TileChoice tc = planned_tile(m, n, k, batch_inner * batch_outer, b_major != 0, force_bn, pair_ok ? force_cta2 : 0, split);
-    if (fused) g_num_sms += held_back;
-    if (tc.bn == 0) tc = pick_tile(m, n, k, batch_inner * batch_outer, b_major != 0, 0, -1, split);  // forced shape not applicable here
+    TileChoice tc = planned_tile(m, n, k, batch_inner * batch_outer, b_major != 0, force_bn, pair_ok ? force_cta2 : 0, split, sms - held_back);
+    if (tc.bn == 0) tc = pick_tile(m, n, k, batch_inner * batch_outer, b_major != 0, 0, -1, split, sms);  // forced shape not applicable here
     if (tc.bn == 0) return -22;
     p.bn = tc.bn;
     const int ncta = tc.cta2 ? 2 : 1;
@@ -1542,7 +1544,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
         set_split(p, tc, (int)((k + BK - 1) / BK));
         do p.sk_tag = g_sk_tag.fetch_add(1, std::memory_order_relaxed) + 1; while (p.sk_tag == 0);
         p.sk_flags = (uint32_t*)g.scratch;
-        p.sk_part = (float4*)((char*)g.scratch + (int64_t)g_num_sms * SK_WARPS * 4);
+        p.sk_part = (float4*)((char*)g.scratch + (int64_t)sms * SK_WARPS * 4);
         p.sk_slot = (uint32_t)(128 * ((p.bn + 31) / 32 * 32) / 4);
     }
     if (p.group_m > p.m_blocks) p.group_m = p.m_blocks;
@@ -1600,7 +1602,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     FusedComm none;
     memset(&none, 0, sizeof(none));
     if (fused) {
-        const int compute = (g_num_sms - held_back) / ncta;   // CTAs (or CTA pairs) that do math
+        const int compute = (sms - held_back) / ncta;   // CTAs (or CTA pairs) that do math
         const unsigned grid = (unsigned)(ncta * (tiles < compute ? tiles : compute)) + comm_ctas;
         FusedComm fc = *fused;
         if (fc.mode == 3) fc.bg_first_block = (int)(((fc.bg_first / k) / p.bn) % p.n_blocks);
@@ -1634,12 +1636,12 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
         return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
     }
     if (!tc.cta2) {
-        const unsigned grid = (unsigned)(tc.sk_tiles ? whole_or_split(tiles, g_num_sms, tc) : tiles < g_num_sms ? tiles : g_num_sms);
+        const unsigned grid = (unsigned)(tc.sk_tiles ? whole_or_split(tiles, sms, tc) : tiles < sms ? tiles : sms);
         const cudaError_t e = bmt::launch(gemm_tcgen05_kernel<false, 0>, grid, num_threads(0), smem, stream, 1, ma, mb, p, none);
         bmt_count_launch(1);
         return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
     }
-    const int64_t pairs = g_num_sms / 2;
+    const int64_t pairs = sms / 2;
     const unsigned grid = (unsigned)(2 * (tc.sk_tiles ? whole_or_split(tiles, pairs, tc) : tiles < pairs ? tiles : pairs));
     const cudaError_t e = bmt::launch(gemm_tcgen05_kernel<true, 0>, grid, num_threads(0), smem, stream, 2, ma, mb, p, none);
     bmt_count_launch(1);
@@ -1658,11 +1660,7 @@ extern "C" int bmt_gemm_reserve_sms(int n) {
 // Returns their number.  Host arithmetic only.
 extern "C" int bmt_gemm_plan(int64_t m, int64_t n, int64_t k, int b_major, int worker, int64_t* plan, int* items, int most) {
     const int sms = bmt::sm_count();
-    if (g_num_sms != 0 && g_num_sms != sms) return -1;
-    const int was = g_num_sms;
-    g_num_sms = sms;
-    const TileChoice tc = pick_tile(m, n, k, 1, b_major != 0, 0, -1, true);
-    g_num_sms = was;
+    const TileChoice tc = pick_tile(m, n, k, 1, b_major != 0, 0, -1, true, sms);
     const int ncta = tc.cta2 ? 2 : 1, k_blocks = (int)((k + BK - 1) / BK);
     const int64_t tiles = ((m + BM * ncta - 1) / (BM * ncta)) * ((n + tc.bn - 1) / tc.bn), slots = sms / ncta;
     const int64_t grid = tc.sk_tiles ? whole_or_split(tiles, slots, tc) : tiles < slots ? tiles : slots;
@@ -1780,14 +1778,12 @@ static int gemm_reduce_scatter_impl(const BmtGemmDesc* desc, int world, int rank
 
 // Number of CTAs the fused GEMM -> reduce-scatter launches for this problem (its completion counter advances by that much).
 extern "C" int bmt_gemm_rs_grid(int64_t m, int64_t n, int64_t k, int b_major) {
-    if (g_num_sms == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess) return -1;
-        if (cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
-    }
-    const TileChoice tc = pick_tile(m, n, k, 1, b_major != 0, 0, 0, false);
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return -1;
+    const int sms = bmt::sm_count();
+    const TileChoice tc = pick_tile(m, n, k, 1, b_major != 0, 0, 0, false, sms);
     const int64_t tiles = ((m + BM - 1) / BM) * ((n + tc.bn - 1) / tc.bn);
-    return (int)(tiles < g_num_sms ? tiles : g_num_sms);
+    return (int)(tiles < sms ? tiles : sms);
 }
 
 // all-gather -> GEMM over the rows of A (see FusedComm mode 2).  The gathered matrix (world * rows x K, pitch K) lives in
@@ -1822,7 +1818,7 @@ extern "C" int bmt_all_gather_gemm(const BmtGemmDesc* desc, int world, int rank,
 // CTA moves about 14 GB/s, all pushers together at most about 550 GB/s to remote destinations, and the math runs at
 // about 1.1 PFLOP/s on a full GPU.  push_bytes counts every destination (own copy included), remote_bytes the peers only.
 extern "C" int bmt_fused_comm_ctas(double flops, double push_bytes, double remote_bytes) {
-    static int sms = 0;   // not g_num_sms: that one doubles as the "kernel attributes are set" marker of launch_gemm
+    static int sms = 0;
     if (sms == 0) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess) return 16;
