@@ -371,6 +371,8 @@ int bmt_attn_status(void);
 
 // status word of the GEMM kernels: 0, or (role << 16 | cta) of the first CTA whose bounded wait ran out; reading clears it
 int bmt_gemm_status(void);
+// Waits as a GEMM waits for sums of another CTA until *flag is 1 (see bmt_gemm_status).
+int bmt_gemm_wait(void* flag_u32, void* stream);
 // Timing counters of the fused compute+collective GEMM kernels since the last call, in nanoseconds: out[0] sum over
 // compute CTAs of producer time spent waiting for other ranks' data, out[1] longest pusher CTA, out[2] longest CTA,
 // out[3] longest producer wait of one CTA, out[4] kernels counted, out[5] (GEMM -> reduce-scatter) longest wait for the

@@ -84,7 +84,19 @@ struct GemmParams {
     uint32_t* sk_flags;    // SK_WARPS words per CTA, zero between launches
     float4* sk_part;       // sk_slot 16-byte units per CTA
     uint32_t sk_slot;
+    int* host_status;      // pinned host memory, see gave_up
 };
+
+// A bounded wait has run out: what the CTA was to compute is missing.  Plain GEMMs report to the host as well, where the next launch finds it
+// without waiting for the device (fused ones have a status of their own, and their callers decide).
+template <bool FUSED> __device__ __forceinline__ void gave_up(int what, int* host_status) {
+    const int code = (what << 16) | (int)(blockIdx.x & 0xffff);
+    atomicCAS(&g_gemm_status, 0, code);
+    if (!FUSED) {
+        *reinterpret_cast<volatile int*>(host_status) = code;
+        __threadfence_system();
+    }
+}
 
 template <typename T> __device__ __forceinline__ void store8(T* dst, const float* v) {
     bmt::Vec16<T> o;
@@ -356,6 +368,14 @@ __device__ __forceinline__ bool wait_partials(uint32_t* flag, int64_t pitch, int
     ok = __all_sync(0xffffffffu, ok) != 0;
     __syncwarp();       // what lane 0 has acquired is there for the others
     return ok;
+}
+
+// This warp's part of a tile whose sums did not all arrive.
+template <typename T>
+__device__ __noinline__ void store_nan(const GemmParams& p, T* c, int64_t row0, int64_t n0, int64_t col_end, int lane, int first) {
+    const int64_t row_end = row0 + 32 < p.M ? row0 + 32 : p.M;
+    for (int64_t r = row0; r < row_end; ++r)
+        for (int64_t col = n0 + first * 32 + lane; col < col_end; col += 64) c[r * p.ldc + col] = bmt::Cvt<T>::from_f(NAN);
 }
 
 // v *= gelu'(e)
@@ -935,7 +955,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                 const int m0 = m_blk * (BM * NCTA) + (int)rank * BM;            // this CTA's rows of A
                 const int n0 = n_blk * p.bn + (int)(rank * bn_local);           // this CTA's rows of the B tile
                 for (int kb = it.kb0; kb < it.kb1; ++kb) {
-                    if (!mbar_wait_warp(empty0 + 8 * ps, pph ^ 1)) { ok = false; if (lane == 0) { atomicCAS(&g_gemm_status, 0, (1 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; } break; }
+                    if (!mbar_wait_warp(empty0 + 8 * ps, pph ^ 1)) { ok = false; if (lane == 0) { gave_up<FUSED != 0>(1, p.host_status); hdr->failed = 1; } break; }
                     const uint32_t sa = smem0 + ps * stage_bytes, sb = sa + a_bytes;
                     const int kx = kb * BK;
                     if (elect_one()) {
@@ -1006,11 +1026,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             for (Item it; ok && next_item(work, it); ++tcount) {
                 const uint32_t acc = tcount & 1;
                 const uint32_t acc_ph = (tcount >> 1) & 1;
-                if (!mbar_wait_warp(tempty0 + 8 * acc, acc_ph ^ 1)) { ok = false; if (lane == 0) { atomicCAS(&g_gemm_status, 0, (2 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; } break; }
+                if (!mbar_wait_warp(tempty0 + 8 * acc, acc_ph ^ 1)) { ok = false; if (lane == 0) { gave_up<FUSED != 0>(2, p.host_status); hdr->failed = 1; } break; }
                 tc_fence_after();
                 const uint32_t tmem_c = tmem_base + acc * p.bn;
                 for (int kb = it.kb0; kb < it.kb1; ++kb) {
-                    if (!mbar_wait_warp(full0 + 8 * cs, cph)) { ok = false; if (lane == 0) { atomicCAS(&g_gemm_status, 0, (3 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; } break; }
+                    if (!mbar_wait_warp(full0 + 8 * cs, cph)) { ok = false; if (lane == 0) { gave_up<FUSED != 0>(3, p.host_status); hdr->failed = 1; } break; }
                     tc_fence_after();
                     const uint32_t sa = smem0 + cs * stage_bytes;
                     const uint32_t a_lo = desc_lo(sa, a_lbo), b_lo = desc_lo(sa + a_bytes, b_lbo);
@@ -1071,7 +1091,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             const int bo = batch / (int)p.batch_inner, bi = batch - bo * (int)p.batch_inner;
             const uint32_t acc = tcount & 1;
             const uint32_t acc_ph = (tcount >> 1) & 1;
-            if (!mbar_wait_warp(smem_u32(&hdr->tmem_full[acc]), acc_ph)) { ok = false; if (lane == 0) atomicCAS(&g_gemm_status, 0, (4 << 16) | (blockIdx.x & 0xffff)); break; }
+            if (!mbar_wait_warp(smem_u32(&hdr->tmem_full[acc]), acc_ph)) { ok = false; if (lane == 0) gave_up<FUSED != 0>(4, p.host_status); break; }
             tc_fence_after();
             const int64_t row0 = (int64_t)m_blk * (BM * NCTA) + rank * BM + quarter * 32;
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * p.bn;
@@ -1154,7 +1174,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                     sk.count = first_tile - Work::first_of(p, first_tile, tile, k_blocks);
                     if (!wait_partials(flag - NCTA * SK_WARPS, NCTA * SK_WARPS, sk.count, p.sk_tag, lane)) {
                         ok = false;
-                        if (lane == 0) { atomicCAS(&g_gemm_status, 0, (12 << 16) | (blockIdx.x & 0xffff)); hdr->failed = 1; }
+                        if (lane == 0) { gave_up<FUSED != 0>(12, p.host_status); hdr->failed = 1; }
+                        if (p.c_dtype == BMT_DT_F16) store_nan(p, (__half*)p.c + coff, row0, n0, col_end, lane, first);
+                        else if (p.c_dtype == BMT_DT_BF16) store_nan(p, (__nv_bfloat16*)p.c + coff, row0, n0, col_end, lane, first);
+                        else store_nan(p, (float*)p.c + coff, row0, n0, col_end, lane, first);
                         break;
                     }
                     // the last item of this CTA: its loads have landed and its MMAs have read them
@@ -1476,6 +1499,9 @@ void set_split(GemmParams& p, const TileChoice& tc, int k_blocks) {
 // CTAs (pairs) of a launch with split tiles: whole tiles come only in full waves.
 int64_t whole_or_split(int64_t tiles, int64_t slots, const TileChoice& tc) { return tiles > tc.sk_tiles ? slots : tc.sk_workers; }
 
+// Where kernels report waits that ran out (see gave_up).
+int* g_host_status = nullptr;
+
 // Once, whichever thread comes first.
 int prepare_kernels() {
     static std::atomic<bool> done{false};
@@ -1487,6 +1513,12 @@ int prepare_kernels() {
     for (const auto kernel : {gemm_tcgen05_kernel<false, 0>, gemm_tcgen05_kernel<true, 0>, gemm_tcgen05_kernel<false, 1>, gemm_tcgen05_kernel<false, 2>,
                               gemm_tcgen05_kernel<false, 3>, gemm_tcgen05_kernel<true, 1>, gemm_tcgen05_kernel<true, 2>, gemm_tcgen05_kernel<true, 3>})
         BMT_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // allocates, which the first launch may have to do under a capture
+    BMT_CUDA_OK(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaHostAlloc((void**)&g_host_status, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    BMT_CUDA_OK(e);
+    *g_host_status = 0;
     done.store(true, std::memory_order_release);
     return 0;
 }
@@ -1504,6 +1536,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     if (k <= 0) return -20;
     const int sms = bmt::sm_count();
     if (const int rc = prepare_kernels()) return rc;
+    if (!fused && *(volatile int*)g_host_status != 0) return -60;     // until bmt_gemm_status has been read
     static int force_bn = -1, force_cta2 = -2;
     if (force_bn < 0) { const char* e = getenv("BMT_GEMM_BN"); force_bn = e ? atoi(e) : 0; }
     if (force_cta2 == -2) { const char* e = getenv("BMT_GEMM_CTA2"); force_cta2 = e ? atoi(e) : -1; }
@@ -1536,6 +1569,7 @@ int launch_gemm(const BmtGemmDesc& g, cudaStream_t stream, const FusedComm* fuse
     p.n_blocks = (int)((n + p.bn - 1) / p.bn);
     p.batch_inner = batch_inner; p.batch_outer = batch_outer; p.b_inner_div = b_inner_div > 0 ? b_inner_div : 1;
     p.c = c; p.ldc = ldc; p.c_bs0 = c_bs0; p.c_bs1 = c_bs1; p.c_dtype = c_dtype;
+    p.host_status = g_host_status;
     p.bias = bias; p.bias_dtype = ab_dtype; p.act = act; p.accumulate = accumulate; p.alpha = alpha;
     static int group_env = -1;
     if (group_env < 0) { const char* e = getenv("BMT_GEMM_GROUP_M"); group_env = e ? atoi(e) : 0; }
@@ -1906,5 +1940,16 @@ extern "C" int bmt_gemm_status(void) {
     int v = 0, zero = 0;
     if (cudaMemcpyFromSymbol(&v, g_gemm_status, sizeof(int)) != cudaSuccess) return -1;
     if (v) cudaMemcpyToSymbol(g_gemm_status, &zero, sizeof(int));
+    if (v && g_host_status) *g_host_status = 0;
     return v;
+}
+
+// The wait of a CTA for the sums of another, for a flag that the caller may or may not have set to 1: what a hand-over that fails does.
+__global__ void gemm_wait_kernel(uint32_t* flag, int* host_status) {
+    if (!wait_partials(flag, 0, 1, 1, (int)threadIdx.x) && threadIdx.x == 0) gave_up<false>(12, host_status);
+}
+extern "C" int bmt_gemm_wait(void* flag, void* stream) {
+    if (const int rc = prepare_kernels()) return rc;
+    gemm_wait_kernel<<<1, 32, 0, (cudaStream_t)stream>>>((uint32_t*)flag, g_host_status);
+    return (int)cudaGetLastError();
 }

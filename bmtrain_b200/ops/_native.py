@@ -83,5 +83,7 @@ def stream() -> int:
 
 
 def check(status: int, what: str) -> None:
+    if status == -60:
+        raise RuntimeError(f"{what}: not launched, since a CTA of an earlier GEMM gave up waiting and its result is incomplete (bmt_gemm_status)")
     if status != 0:
         raise RuntimeError(f"{what} failed with status {status}")
