@@ -124,66 +124,84 @@ __device__ __forceinline__ float ex2_approx(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-// GELU of pairs.  The normal distribution function comes in two forms, neither with erff, which sets the pace of what uses it:
+// GELU.  The normal distribution function comes in two forms, neither with erff, which sets the pace of what uses it:
 // Below 1.3: Phi(x) = 1/2 + x P(x^2), P fitted for this file in 64 bits behind its first coefficient, as that is rounded, weighted for the relative
 // error of Phi on the negative side (3e-9).
 // Above: Phi(-u) = t 2^(q(t)) exp(-u^2 / 2), t = 1 / (1 + 0.3 u), q fitted for this file in 64 bits (the form of the complementary error function in
 // Press et al., Numerical Recipes, 6.2; largest error 7e-8).  It keeps its relative accuracy on the negative side (2e-6 at -5, where
 // 1 + erf(x / sqrt 2) has 6e-2), but for small u it has errors of 5e-7.
 // Largest errors between -1.3 and 1.3, as with erff: x Phi(x) 3.5e-7 relative, Phi(x) + x phi(x) 1.4e-7 absolute.
+// One value or a pair at a time: pairs issue half as much, single ones take the constants as operands of the instructions (in pairs they sit in 30
+// registers, which the GEMM's epilogue does not have: all forms of it took 2 % longer).
 constexpr float HALF_LOG2E = 0.7213475204444817f, NORMAL_NEAR = 1.3f;
-__device__ __forceinline__ uint64_t both(float a) { return pack_f2(a, a); }
-__device__ __forceinline__ uint64_t normal_near(uint64_t x) {
-    const uint64_t s = mul_f2(x, x);
-    uint64_t p = both(5.271343753e-07f);
-    p = fma_f2(p, s, both(-9.379426047e-06f));
-    p = fma_f2(p, s, both(1.158123778e-04f));
-    p = fma_f2(p, s, both(-1.188031165e-03f));
-    p = fma_f2(p, s, both(9.974041022e-03f));
-    p = fma_f2(p, s, both(-6.649051607e-02f));
-    p = fma_f2(p, s, both(0.39894229173660278f));
-    return fma_f2(x, p, both(0.5f));
+template <typename V> struct Lanes;
+template <> struct Lanes<float> {
+    static __device__ __forceinline__ float all(float a) { return a; }
+    static __device__ __forceinline__ float fma(float a, float b, float c) { return fmaf(a, b, c); }
+    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+    static __device__ __forceinline__ float abs(float a) { return fabsf(a); }
+    static __device__ __forceinline__ float ex2(float a) { return ex2_approx(a); }
+    static __device__ __forceinline__ float rcp(float a) { return rcp_approx_ftz(a); }
+    // Phi(x) of its two forms: near(x), far(-|x|)
+    static __device__ __forceinline__ float pick(float x, float near, float far) { return fabsf(x) < NORMAL_NEAR ? near : x >= 0.f ? 1.f - far : far; }
+};
+template <> struct Lanes<uint64_t> {
+    typedef Lanes<float> One;
+    template <typename F> static __device__ __forceinline__ uint64_t each(uint64_t v, F f) {
+        float a, b;
+        unpack_f2(v, a, b);
+        return pack_f2(f(a), f(b));
+    }
+    static __device__ __forceinline__ uint64_t all(float a) { return pack_f2(a, a); }
+    static __device__ __forceinline__ uint64_t fma(uint64_t a, uint64_t b, uint64_t c) { return fma_f2(a, b, c); }
+    static __device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) { return mul_f2(a, b); }
+    static __device__ __forceinline__ uint64_t abs(uint64_t a) { return a & 0x7fffffff7fffffffull; }
+    static __device__ __forceinline__ uint64_t ex2(uint64_t v) { return each(v, [](float a) { return ex2_approx(a); }); }
+    static __device__ __forceinline__ uint64_t rcp(uint64_t v) { return each(v, [](float a) { return rcp_approx_ftz(a); }); }
+    static __device__ __forceinline__ uint64_t pick(uint64_t x, uint64_t near, uint64_t far) {
+        float a, b, na, nb, fa, fb;
+        unpack_f2(x, a, b);
+        unpack_f2(near, na, nb);
+        unpack_f2(far, fa, fb);
+        return pack_f2(One::pick(a, na, fa), One::pick(b, nb, fb));
+    }
+};
+template <typename V> __device__ __forceinline__ V normal_near(V x) {
+    typedef Lanes<V> L;
+    const V s = L::mul(x, x);
+    V p = L::all(5.271343753e-07f);
+    p = L::fma(p, s, L::all(-9.379426047e-06f));
+    p = L::fma(p, s, L::all(1.158123778e-04f));
+    p = L::fma(p, s, L::all(-1.188031165e-03f));
+    p = L::fma(p, s, L::all(9.974041022e-03f));
+    p = L::fma(p, s, L::all(-6.649051607e-02f));
+    p = L::fma(p, s, L::all(0.39894229173660278f));
+    return L::fma(x, p, L::all(0.5f));
 }
-__device__ __forceinline__ uint64_t normal_far_log2(uint64_t t) {     // q, in units of log 2
-    uint64_t q = both(0.1297198086977005f);
-    q = fma_f2(q, t, both(-0.041672442108392715f));
-    q = fma_f2(q, t, both(-0.49322715401649475f));
-    q = fma_f2(q, t, both(0.32053878903388977f));
-    q = fma_f2(q, t, both(0.087591201066970825f));
-    q = fma_f2(q, t, both(0.62215578556060791f));
-    q = fma_f2(q, t, both(1.4390027523040771f));
-    return fma_f2(q, t, both(-3.0625312328338623f));
-}
-__device__ __forceinline__ uint64_t ex2_f2(uint64_t v) {
-    float a, b;
-    unpack_f2(v, a, b);
-    return pack_f2(ex2_approx(a), ex2_approx(b));
-}
-// Phi(x) where Phi(-|x|) by the second form is `far`
-__device__ __forceinline__ uint64_t normal_of(uint64_t x, uint64_t far) {
-    float a, b, na, nb, fa, fb;
-    unpack_f2(x, a, b);
-    unpack_f2(normal_near(x), na, nb);
-    unpack_f2(far, fa, fb);
-    return pack_f2(fabsf(a) < NORMAL_NEAR ? na : a >= 0.f ? 1.f - fa : fa, fabsf(b) < NORMAL_NEAR ? nb : b >= 0.f ? 1.f - fb : fb);
-}
-__device__ __forceinline__ uint64_t abs_f2(uint64_t x) { return x & 0x7fffffff7fffffffull; }
-__device__ __forceinline__ uint64_t normal_t(uint64_t u) {
-    float a, b;
-    unpack_f2(fma_f2(u, both(0.3f), both(1.f)), a, b);
-    return pack_f2(rcp_approx_ftz(a), rcp_approx_ftz(b));
+template <typename V> __device__ __forceinline__ V normal_far_log2(V t) {     // q, in units of log 2
+    typedef Lanes<V> L;
+    V q = L::all(0.1297198086977005f);
+    q = L::fma(q, t, L::all(-0.041672442108392715f));
+    q = L::fma(q, t, L::all(-0.49322715401649475f));
+    q = L::fma(q, t, L::all(0.32053878903388977f));
+    q = L::fma(q, t, L::all(0.087591201066970825f));
+    q = L::fma(q, t, L::all(0.62215578556060791f));
+    q = L::fma(q, t, L::all(1.4390027523040771f));
+    return L::fma(q, t, L::all(-3.0625312328338623f));
 }
 // x Phi(x)
-__device__ __forceinline__ uint64_t gelu(uint64_t x) {
-    const uint64_t u = abs_f2(x), t = normal_t(u);
-    const uint64_t far = mul_f2(t, ex2_f2(fma_f2(mul_f2(u, both(-HALF_LOG2E)), u, normal_far_log2(t))));
-    return mul_f2(x, normal_of(x, far));
+template <typename V> __device__ __forceinline__ V gelu(V x) {
+    typedef Lanes<V> L;
+    const V u = L::abs(x), t = L::rcp(L::fma(u, L::all(0.3f), L::all(1.f)));
+    const V far = L::mul(t, L::ex2(L::fma(L::mul(u, L::all(-HALF_LOG2E)), u, normal_far_log2(t))));
+    return L::mul(x, L::pick(x, normal_near(x), far));
 }
 // Phi(x) + x phi(x)
-__device__ __forceinline__ uint64_t gelu_grad(uint64_t x) {
-    const uint64_t u = abs_f2(x), t = normal_t(u), e = ex2_f2(mul_f2(mul_f2(u, both(-HALF_LOG2E)), u));
-    const uint64_t far = mul_f2(mul_f2(t, e), ex2_f2(normal_far_log2(t)));
-    return fma_f2(mul_f2(x, both(0.3989422804014327f)), e, normal_of(x, far));
+template <typename V> __device__ __forceinline__ V gelu_grad(V x) {
+    typedef Lanes<V> L;
+    const V u = L::abs(x), t = L::rcp(L::fma(u, L::all(0.3f), L::all(1.f))), e = L::ex2(L::mul(L::mul(u, L::all(-HALF_LOG2E)), u));
+    const V far = L::mul(L::mul(t, e), L::ex2(normal_far_log2(t)));
+    return L::fma(L::mul(x, L::all(0.3989422804014327f)), e, L::pick(x, normal_near(x), far));
 }
 
 // ---- dependent launches -------------------------------------------------------------------------------------------------------

@@ -306,8 +306,10 @@ struct Partials {
 #pragma unroll
         for (int k = 0; k < SK_AHEAD; ++k) fetch();
     }
-    // r += the next piece of all slots
+    // r += the next piece of all slots.  count < 0: they did not all arrive, and every row gets a NaN in the first column of the piece (whole tiles of
+    // them, stored here or in the epilogue, cost the kernel registers, and 2 % of its time).
     __device__ __forceinline__ void add(uint32_t (&r)[32]) {
+        if (count < 0) r[0] = 0x7fffffffu;
         for (int k = 0; k < count; ++k) {
             float4 v[8];
             asm volatile("cp.async.wait_group %0;" ::"n"(SK_AHEAD - 1) : "memory");
@@ -368,21 +370,6 @@ __device__ __forceinline__ bool wait_partials(uint32_t* flag, int64_t pitch, int
     ok = __all_sync(0xffffffffu, ok) != 0;
     __syncwarp();       // what lane 0 has acquired is there for the others
     return ok;
-}
-
-// This warp's part of a tile whose sums did not all arrive.
-template <typename T>
-__device__ __noinline__ void store_nan(const GemmParams& p, T* c, int64_t row0, int64_t n0, int64_t col_end, int lane, int first) {
-    const int64_t row_end = row0 + 32 < p.M ? row0 + 32 : p.M;
-    for (int64_t r = row0; r < row_end; ++r)
-        for (int64_t col = n0 + first * 32 + lane; col < col_end; col += 64) c[r * p.ldc + col] = bmt::Cvt<T>::from_f(NAN);
-}
-
-// v *= gelu'(e)
-__device__ __forceinline__ void mul_gelu_grad(float (&v)[8], const float (&e)[8]) {
-#pragma unroll
-    for (int i = 0; i < 8; i += 2)
-        bmt::unpack_f2(bmt::mul_f2(bmt::pack_f2(v[i], v[i + 1]), bmt::gelu_grad(bmt::pack_f2(e[i], e[i + 1]))), v[i], v[i + 1]);
 }
 
 // Epilogue of one warp's 32 rows of a tile: tensor memory -> (alpha, bias, activation, mask, residual, old C) -> global.
@@ -475,8 +462,8 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, T* cbase, con
                 for (int i = 0; i < 8; ++i) {
                     if (EXTRA == 1) v[it][i] = (p.round_first ? bmt::Cvt<T>::to_f(bmt::Cvt<T>::from_f(v[it][i])) : v[it][i]) + e[i];
                     else if (EXTRA == 2) v[it][i] = e[i] > 0.f ? v[it][i] : 0.f;
+                    else v[it][i] *= bmt::gelu_grad(e[i]);
                 }
-                if (EXTRA == 3) mul_gelu_grad(v[it], e);
             }
             if (col_ok && it * 8 + sub < rows) store8(dst + it * d_step + c * 32, v[it]);
         }
@@ -515,17 +502,12 @@ __device__ __forceinline__ void epilogue_rows_any(const GemmParams& p, TC* cbase
             for (int i = 0; i < 8; ++i) {
                 v[i] = v[i] * p.alpha + bias[i];
                 if (p.act == 1) v[i] = fmaxf(v[i], 0.f);
-            }
-            if (p.act == 2) {
-#pragma unroll
-                for (int i = 0; i < 8; i += 2) bmt::unpack_f2(bmt::gelu(bmt::pack_f2(v[i], v[i + 1])), v[i], v[i + 1]);
+                else if (p.act == 2) v[i] = bmt::gelu(v[i]);
             }
             if (p.aux_mode) {
                 load_row8_dt(p.aux, p.bias_dtype, row * p.ld_aux + col, n_ok, a_vec, e);
-                if (p.aux_mode == 1) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) v[i] = e[i] > 0.f ? v[i] : 0.f;
-                } else mul_gelu_grad(v, e);
+                for (int i = 0; i < 8; ++i) v[i] = p.aux_mode == 1 ? (e[i] > 0.f ? v[i] : 0.f) : v[i] * bmt::gelu_grad(e[i]);
             }
             if (p.residual) {
                 load_row8_dt(p.residual, p.bias_dtype, row * p.ldr + col, n_ok, r_vec, e);
@@ -1175,13 +1157,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                     if (!wait_partials(flag - NCTA * SK_WARPS, NCTA * SK_WARPS, sk.count, p.sk_tag, lane)) {
                         ok = false;
                         if (lane == 0) { gave_up<FUSED != 0>(12, p.host_status); hdr->failed = 1; }
-                        if (p.c_dtype == BMT_DT_F16) store_nan(p, (__half*)p.c + coff, row0, n0, col_end, lane, first);
-                        else if (p.c_dtype == BMT_DT_BF16) store_nan(p, (__nv_bfloat16*)p.c + coff, row0, n0, col_end, lane, first);
-                        else store_nan(p, (float*)p.c + coff, row0, n0, col_end, lane, first);
-                        break;
-                    }
-                    // the last item of this CTA: its loads have landed and its MMAs have read them
-                    sk.start(smem_u32(smem) + (uint32_t)(warp - 2) * (SK_AHEAD * 4096) + lane * 16, first, 2, n_chunks);
+                        sk.count = -1;
+                    } else      // the last item of this CTA: its loads have landed and its MMAs have read them
+                        sk.start(smem_u32(smem) + (uint32_t)(warp - 2) * (SK_AHEAD * 4096) + lane * 16, first, 2, n_chunks);
                 }
                 if (p.c_dtype == BMT_DT_F16) epilogue_tile(p, (__half*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, sk, release);
                 else if (p.c_dtype == BMT_DT_BF16) epilogue_tile(p, (__nv_bfloat16*)p.c + coff, row0, n0, col_end, taddr, sbuf, lane, first, sk, release);
