@@ -200,7 +200,7 @@ class _Bucket:
     def points_local(self) -> bool:
         """Whether every parameter is the view of the partition that ``local_views`` gives, whoever may have assigned to its ``data``."""
         self._refresh_views()
-        return all(s.param.data_ptr() == at and s.param.dtype == self.storage.dtype for s, at in zip(self.slots, self._local_at))
+        return [(p.data_ptr(), p.dtype) for p in self._params] == self._local_at
 
     def _refresh_views(self) -> None:
         data = self.storage.data
@@ -208,7 +208,8 @@ class _Bucket:
         if self._views_of != key:
             # the views keep the memory they look at alive, so an equal address is the same memory
             self._local_views = [data[s.lo - self.begin:s.hi - self.begin] for s in self.slots]
-            self._local_at = [view.data_ptr() for view in self._local_views]
+            self._local_at = [(view.data_ptr(), view.dtype) for view in self._local_views]
+            self._params = [s.param for s in self.slots]
             self._full_views = None
             if self.comm.size == 1:
                 sizes, _, where = self.layout()
@@ -649,8 +650,9 @@ class Block(torch.nn.Module):
             for s, view in zip(b.slots, b.local_views()):
                 s.param.data = view
 
-    def _release_params(self) -> None:
-        self._point_to_local()
+    def _release_params(self, point: bool = True) -> None:
+        if point:
+            self._point_to_local()
         for b in self._buckets.values():
             sym = getattr(b, "full_sym", None)
             if sym is not None and b.full is not None:
@@ -894,7 +896,8 @@ class Block(torch.nn.Module):
         try:
             return self._native_pass(native, args).forward()
         finally:
-            self._release_params()
+            b.full = b.work = None
+            self._point_to_local()
 
     def _native_backward(self, native, args, grad_out):
         _, b, slots = native
@@ -938,7 +941,7 @@ class Block(torch.nn.Module):
             if not last:
                 return  # gradients keep accumulating in the full buffers until micro-batch 0
         self._scatter_grads()
-        self._release_params()
+        self._release_params(point=False)        # which that has done
 
     # ------------------------------------------------------------------ links
     def set_pre_module(self, pre_module) -> None:

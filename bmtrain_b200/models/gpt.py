@@ -84,9 +84,13 @@ class Feedforward(DistributedModule):
         return self.w_out(h)
 
 
-def _has_bias(projection) -> bool:
-    own = getattr(projection, "_parameters", {})        # as it stands: read as an attribute, a parameter on its own is gathered
-    return (own["bias"] if "bias" in own else projection.bias) is not None
+def _has_bias(attn) -> bool:
+    """Of the QKV projection.  Parameters are looked up as they stand: read as an attribute, one that is not in a block is gathered."""
+    qkv = attn._modules.get("project_qkv")
+    if qkv is None:
+        qkv = attn.project_qkv
+    own = getattr(qkv, "_parameters", {})
+    return (own["bias"] if "bias" in own else qkv.bias) is not None
 
 
 @reads_parameters_only
@@ -110,8 +114,10 @@ class TransformerEncoder(DistributedModule):
         return torch.is_tensor(hidden) and self._fused_ok(hidden) and not bmt_inspect.tensor.debug.get("_inspect_tensor", False)
 
     def _fused_ok(self, hidden: torch.Tensor) -> bool:
-        attn = self.attn
-        return (hidden.is_cuda and hidden.dim() == 3 and config["tp_size"] == 1 and _FUSED_BLOCK and _has_bias(attn.project_qkv)
+        attn = self._modules.get("attn")
+        if attn is None:
+            attn = self.attn
+        return (hidden.is_cuda and hidden.dim() == 3 and config["tp_size"] == 1 and _FUSED_BLOCK and _has_bias(attn)
                 and hidden.dtype in (torch.float16, torch.bfloat16) and attn.dim_head % 8 == 0)
 
     # A ``Block`` whose module is this one, as it stands, has it computed by the native executor without autograd inside (see
@@ -121,11 +127,12 @@ class TransformerEncoder(DistributedModule):
         if not (torch.is_tensor(hidden) and self._fused_ok(hidden) and hidden.numel() > 0 and self._bmt_deferred_gather is None):
             return None
         m = self._modules
-        if not all(type(m[name]) is cls for name, cls in (("ln_attn", LayerNorm), ("attn", Attention), ("ln_ff", LayerNorm), ("ff", Feedforward))):
+        if type(m["ln_attn"]) is not LayerNorm or type(m["attn"]) is not Attention or type(m["ln_ff"]) is not LayerNorm or type(m["ff"]) is not Feedforward:
             return None                                  # other submodules
         a = m["attn"]
         attn, ff, (b, s, d), inner = a._modules, m["ff"]._modules, hidden.shape, a.num_heads * a.dim_head
-        if not all(type(mod) is Linear for mod in (attn["project_qkv"], attn["project_out"], ff["w_in"], ff["w_out"])):
+        if (type(attn["project_qkv"]) is not Linear or type(attn["project_out"]) is not Linear or type(ff["w_in"]) is not Linear
+                or type(ff["w_out"]) is not Linear):
             return None
         if mask is not None and (not torch.is_tensor(mask) or mask.shape != (b, s, s) or mask.device != hidden.device):
             return None

@@ -91,7 +91,7 @@ class LlamaBlock(DistributedModule):
                 and hidden.dtype in (torch.float16, torch.bfloat16) and _FUSED_BLOCK and os.environ.get("BMT_FLASH_ATTN", "1") != "0"):
             return None
         m = self._modules
-        if not all(type(m[name]) is cls for name, cls in (("ln_attn", RMSNorm), ("attn", LlamaAttention), ("ln_ff", RMSNorm), ("ff", LlamaMLP))):
+        if type(m["ln_attn"]) is not RMSNorm or type(m["attn"]) is not LlamaAttention or type(m["ln_ff"]) is not RMSNorm or type(m["ff"]) is not LlamaMLP:
             return None                                  # other submodules
         a = m["attn"]
         attn, ff, d = a._modules, m["ff"]._modules, hidden.shape[-1]
