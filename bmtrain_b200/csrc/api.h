@@ -61,17 +61,11 @@ int bmt_norm_bwd(int64_t rows, int64_t d, const void* x, const void* dy, const v
 int bmt_norm_bwd_res(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, const void* stats, int rms,
                      int dtype, int nblk, void* dx, void* partial_2xnblkxd_f32, void* dw, void* db, const void* dres, void* stream);
 
-int bmt_norm_bwd_ex(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, const void* stats, int rms,
-                    int dtype, int nblk, void* dx, void* partial_2xnblkxd_f32, void* dw, void* db, const void* dres,
-                    int accumulate, void* stream);
-
 // 0, or (1 << 16 | CTA) of the first CTA of a norm backward whose bounded wait ran out (its weight gradient is NaN then); reading clears it
 int bmt_norm_status(void);
 
 int bmt_embedding_fwd(int64_t tokens, int64_t d, const void* ids_i64, const void* weight, int dtype, void* out, void* stream);
 int64_t bmt_embedding_bwd_scratch(int64_t tokens, int64_t rows);   // 32-bit words of scratch
-int bmt_embedding_bwd(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out, void* scratch,
-                      void* stream);
 // accumulate: added to what `out` holds
 int bmt_embedding_bwd_ex(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out, int accumulate,
                          void* scratch, void* stream);
@@ -100,7 +94,7 @@ typedef struct {
 #define BMT_MAX_COLSUMS 12
 // At most BMT_MAX_COLSUMS, n multiples of 8; scratch as of bmt_colsum_ex; accumulate: added to what the outputs hold.
 int bmt_colsum_multi(const BmtColsum* items, int count, int dtype, int accumulate, void* scratch, int64_t scratch_bytes, void* stream);
-// bmt_norm_bwd_ex without its last kernel: the weight's gradient is the column sums of the first *blocks rows of `partial` (fp32, d columns),
+// bmt_norm_bwd_res without its last kernel: the weight's gradient is the column sums of the first *blocks rows of `partial` (fp32, d columns),
 // the bias's of the *blocks rows behind them.
 int bmt_norm_bwd_partial(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, const void* stats, int rms, int dtype, int nblk,
                          void* dx, void* partial, const void* dres, int* blocks, void* stream);
@@ -194,7 +188,6 @@ typedef struct {
     void* norm_partial2;      // like norm_partial: one for each norm
 } BmtGptBlockGrad;
 
-int bmt_gpt_block_forward(const BmtGptBlock* blk, void* stream);
 int bmt_gpt_block_forward_steps(const BmtGptBlock* blk, int first_step, int last_step, void* stream);
 int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockGrad* g, void* stream);
 

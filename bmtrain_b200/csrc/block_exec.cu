@@ -134,8 +134,6 @@ extern "C" int bmt_gpt_block_forward_steps(const BmtGptBlock* blk, int first_ste
     return 0;
 }
 
-extern "C" int bmt_gpt_block_forward(const BmtGptBlock* blk, void* stream) { return bmt_gpt_block_forward_steps(blk, 1, 9, stream); }
-
 extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockGrad* grad, void* stream) {
     const BmtGptBlock& k = *blk;
     const BmtGptBlockGrad& w = *grad;

@@ -197,8 +197,3 @@ extern "C" int bmt_embedding_bwd_ex(int64_t tokens, int64_t d, int64_t rows, con
     bmt_count_launch(tokens > EMB_HOT ? 2 : 1);
     return (int)cudaGetLastError();
 }
-
-extern "C" int bmt_embedding_bwd(int64_t tokens, int64_t d, int64_t rows, const void* ids, const void* grad, int dtype, void* out,
-                                 void* scratch, void* stream) {
-    return bmt_embedding_bwd_ex(tokens, d, rows, ids, grad, dtype, out, 0, scratch, stream);
-}

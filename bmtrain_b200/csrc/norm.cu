@@ -122,10 +122,9 @@ __global__ void __launch_bounds__(NT) norm_bwd_kernel(int64_t rows, int d, const
 }
 
 // Fold the per-CTA partial sums: block = 32 columns x 32 row lanes, rows strided over the lanes, smem tree at the end.
-template <typename T, bool ACC = false>
+template <typename T>
 __global__ void __launch_bounds__(1024) norm_fold_kernel(int d, int nblk, const float* __restrict__ partial, T* __restrict__ dw, T* __restrict__ db) {
     bmt::after_previous();
-    // ACC: dw / db already hold gradients of earlier passes and are added to
     __shared__ float sa[32][33], sb[32][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int c = blockIdx.x * 32 + tx;
@@ -142,10 +141,6 @@ __global__ void __launch_bounds__(1024) norm_fold_kernel(int d, int nblk, const 
         float ra = 0.f, rb = 0.f;
 #pragma unroll 8
         for (int l = 0; l < 32; ++l) { ra += sa[l][tx]; rb += sb[l][tx]; }
-        if (ACC) {
-            ra += bmt::Cvt<T>::to_f(dw[c]);
-            if (db) rb += bmt::Cvt<T>::to_f(db[c]);
-        }
         dw[c] = bmt::Cvt<T>::from_f(ra);
         if (db) db[c] = bmt::Cvt<T>::from_f(rb);
     }
@@ -519,13 +514,12 @@ int bwd_stream_vpl(int vpl, Args... args) {
 
 template <typename T>
 int bwd(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, const void* stats, int rms, int nblk, void* dx,
-        void* partial, void* dw, void* db, cudaStream_t s, const void* dres = nullptr, bool acc = false, int* left = nullptr) {
+        void* partial, void* dw, void* db, cudaStream_t s, const void* dres = nullptr, int* left = nullptr) {
     // `left`: the sums are left in `partial`, as so many rows of them
     const auto fold = [&](int blocks) {
         if (left) { *left = blocks; return; }
         const unsigned g = (unsigned)((d + 31) / 32);
-        if (acc) bmt::launch(norm_fold_kernel<T, true>, g, dim3(32, 32), 0, s, 1, (int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
-        else bmt::launch(norm_fold_kernel<T>, g, dim3(32, 32), 0, s, 1, (int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
+        bmt::launch(norm_fold_kernel<T>, g, dim3(32, 32), 0, s, 1, (int)d, blocks, (const float*)partial, (T*)dw, (T*)db);
     };
     static const bool use_reg = [] { const char* e = getenv("BMT_NORM_STAGED"); return !(e && atoi(e) == 1); }();
     if (use_reg && d <= 16384 && !(rms && db)) {
@@ -580,25 +574,14 @@ extern "C" int bmt_norm_bwd_res(int64_t rows, int64_t d, const void* x, const vo
                                : bwd<__nv_bfloat16>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, dw, db, s, dres);
 }
 
-// Backward with residual-branch gradient and, when `accumulate` is set, dw / db += instead of =.
-extern "C" int bmt_norm_bwd_ex(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, const void* stats, int rms,
-                               int dtype, int nblk, void* dx, void* partial, void* dw, void* db, const void* dres, int accumulate,
-                               void* stream) {
-    if (rows <= 0) return 0;
-    if (d % 8 != 0 || d > NT * 8 * MAXIT || dtype == BMT_DT_F32) return -3;
-    cudaStream_t s = (cudaStream_t)stream;
-    return dtype == BMT_DT_F16 ? bwd<__half>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, dw, db, s, dres, accumulate != 0)
-                               : bwd<__nv_bfloat16>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, dw, db, s, dres, accumulate != 0);
-}
-
 extern "C" int bmt_norm_bwd_partial(int64_t rows, int64_t d, const void* x, const void* dy, const void* w, const void* stats, int rms, int dtype,
                                     int nblk, void* dx, void* partial, const void* dres, int* blocks, void* stream) {
     *blocks = 0;
     if (rows <= 0) return 0;
     if (d % 8 != 0 || d > NT * 8 * MAXIT || dtype == BMT_DT_F32) return -3;
     cudaStream_t s = (cudaStream_t)stream;
-    return dtype == BMT_DT_F16 ? bwd<__half>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, nullptr, nullptr, s, dres, false, blocks)
-                               : bwd<__nv_bfloat16>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, nullptr, nullptr, s, dres, false, blocks);
+    return dtype == BMT_DT_F16 ? bwd<__half>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, nullptr, nullptr, s, dres, blocks)
+                               : bwd<__nv_bfloat16>(rows, d, x, dy, w, stats, rms, nblk, dx, partial, nullptr, nullptr, s, dres, blocks);
 }
 
 // status of the norm backward: 0, or (1 << 16 | CTA) of the first CTA that gave up waiting for its rows; reading clears it
