@@ -1,6 +1,8 @@
-// Native executors for whole transformer blocks: pre-LN GPT and, below, the Llama-shaped one.  GPT: the whole forward (9 launches) or backward (15 launches) of a
+// Native executors for whole transformer blocks: pre-LN GPT and, below, the Llama-shaped one.  GPT: the whole forward or backward of a
 // transformer layer is issued from C++ by a single call, so the host cost per layer is a few microseconds instead
-// of one Python/autograd round trip per operator.  Every contraction goes to the tcgen05 GEMM (gemm_sm100.cu) with
+// of one Python/autograd round trip per operator.  Launches with the fused attention: 7 forward, one more with a mask and one more with GELU; 14
+// backward, 18 for more than 2048 tokens, whose bias gradients take a kernel each.  Two more either way with
+// scores in memory.  Every contraction goes to the tcgen05 GEMM (gemm_sm100.cu) with
 // fused epilogues: bias, ReLU, residual add, ReLU-mask / GELU-derivative on the dgrad path.
 // (The reference runs a block as ~40 separate PyTorch ops: example/layers/transformer.py:19-33.)
 #include <math.h>
@@ -68,7 +70,9 @@ extern "C" int bmt_gpt_block_forward_steps(const BmtGptBlock* blk, int first_ste
     const Dims q = dims_of(k);
     const int dt = k.dtype;
     // Below a ReLU no product is divided along its reduction: the sum's last bit moves roundings of the 16-bit results, ReLU inputs near zero
-    // change sides, and gradients of a bf16 model of three blocks move by 5 % (they are 6 % from the exact ones either way).
+    // change sides, and gradients of a bf16 model of three blocks move by 5 % (they are 6 % from the exact ones either way).  That keeps the bits
+    // that this executor gave before tiles were divided; a block that runs operator by operator (no biases, tensor parallelism, fused blocks
+    // switched off) has its products divided like any others, so it is as far from the exact result but not equal to the last bit.
     const auto product = [&](BmtGemmDesc& g) { return k.act == 1 ? bmt_gemm_ex(&g, stream) : gemm(k, g, stream); };
 #define STEP(n) if (first_step <= (n) && (n) <= last_step)
     // 1. LN1
@@ -233,7 +237,7 @@ extern "C" int bmt_gpt_block_backward(const BmtGptBlock* blk, const BmtGptBlockG
 }
 
 // ------------------------------------------------------------------------------------------------- Llama-shaped block
-// 9 launches forward, 17 to 18 backward.  The residual additions happen in the epilogues of the projections and in the norms'
+// 9 launches forward, 16 backward, one more where query heads share a key head and the kernel divides them.  The residual additions happen in the epilogues of the projections and in the norms'
 // backward (as operators of their own: six passes over (T, d) per block and step, 4 % of a block at 2048 x 8192).
 namespace {
 

@@ -182,3 +182,61 @@ def test_parameters_show_the_partition_after_a_pass(bmt_gpu):
                 block(x)
         assert [p.data_ptr() for p in block.parameters()] == want
         assert all(torch.equal(p.detach(), v) for p, v in zip(block.parameters(), values))
+
+
+def _launches(call):
+    import ctypes
+
+    from bmtrain_b200.ops import _native
+
+    lib = _native.cuda_lib()
+    lib.bmt_launch_count.restype = ctypes.c_int64
+    before = lib.bmt_launch_count()
+    call()
+    return lib.bmt_launch_count() - before
+
+
+@pytest.mark.parametrize("tokens,act,masked,forward,backward", [(300, "relu", False, 7, 14), (300, "gelu", True, 9, 14), (2056, "relu", False, 7, 18)])
+def test_launches_of_a_gpt_block(bmt_gpu, tokens, act, masked, forward, backward):
+    from bmtrain_b200.ops import gpt_block
+
+    d, f = 256, 512
+    shapes = [(d,), (d,), (3 * d, d), (3 * d,), (d, d), (d,), (d,), (d,), (f, d), (f,), (d, f), (d,)]
+    params = [torch.randn(*s, device="cuda").mul_(0.05).half() for s in shapes]
+    grads = [torch.empty_like(p) for p in params]
+    x = torch.randn(1, tokens, d, device="cuda").half()
+    mask = torch.ones(1, tokens, tokens, dtype=torch.bool, device="cuda") if masked else None
+    run = gpt_block.Pass(x, mask, [p.data_ptr() for p in params], 4, 64, f, act, 1e-5, True)
+    assert _launches(run.forward) == forward
+    assert _launches(lambda: run.backward(x, [g.data_ptr() for g in grads])) == backward
+
+
+@pytest.mark.parametrize("kv,backward", [(4, 16), (1, 17)])
+def test_launches_of_a_llama_block(bmt_gpu, kv, backward):
+    from bmtrain_b200.ops import llama_block
+
+    d, f, h, dh = 256, 512, 4, 64
+    shapes = [(d,), ((h + 2 * kv) * dh, d), (d, h * dh), (d,), (2 * f, d), (d, f)]
+    params = [torch.randn(*s, device="cuda").mul_(0.05).half() for s in shapes]
+    grads = [torch.empty_like(p) for p in params]
+    x = torch.randn(1, 300, d, device="cuda").half()
+    run = llama_block.Pass(x, [p.data_ptr() for p in params], h, kv, dh, f, 1e-5, 1e-5, 10000.0)
+    assert _launches(run.forward) == 9
+    assert _launches(lambda: run.backward(x, [g.data_ptr() for g in grads])) == backward
+
+
+def test_executor_and_operators_at_a_size_that_is_divided(bmt_gpu, monkeypatch):
+    """Below a ReLU the executor's products are whole and the operators' are divided: equal but for the rounding of sums."""
+    from bmtrain_b200.models import gpt
+
+    bmt, dtype = bmt_gpu, torch.bfloat16
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    enc = _gpt(bmt, dtype, 2560, 40, 64, 10240, "relu", True)
+    bmt.init_parameters(enc)
+    x = torch.randn(1, 370, 2560, generator=gen, device="cuda").to(dtype)
+    with torch.no_grad():
+        executor = enc(x)
+        monkeypatch.setattr(gpt, "_FUSED_BLOCK", False)
+        operators = enc(x)
+    # a chain of a dozen 16-bit intermediates
+    assert (executor.double() - operators.double()).norm() <= 12 * _UNIT[dtype] * operators.double().norm()
