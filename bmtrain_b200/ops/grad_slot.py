@@ -38,11 +38,11 @@ def attached(ctx, position: int, param: torch.Tensor) -> Optional[torch.Tensor]:
     """``param.grad`` if a backward that is running (``ctx``, whose input number ``position`` is the leaf ``param``) may add to it itself and
     return nothing to autograd, or None.  That is what autograd would do with a gradient that it got: the engine executes the leaf's
     accumulation in this very pass (a ``backward``, not a ``grad``, whose inputs if given contain the leaf), nothing watches the
-    parameter or that node, no graph of the gradient is asked for, and the gradient is there, plain and of the parameter's type.  Only on the default
+    parameter or that node, no graph of the gradient is asked for, and the gradient is there, plain, of the parameter's type and on a 16-byte boundary.  Only on the default
     stream: elsewhere it is the engine that orders the accumulation with the leaf's own stream."""
     g = param.grad
     if (g is None or not g.is_cuda or g.dtype != param.dtype or g.shape != param.shape or not g.is_contiguous() or g.requires_grad
-            or type(g) is not torch.Tensor or torch.is_grad_enabled() or watched(param)
+            or type(g) is not torch.Tensor or g.data_ptr() % 16 or torch.is_grad_enabled() or watched(param)
             or torch._C._cuda_getCurrentRawStream(g.device.index) != 0):
         return None
     node = ctx.next_functions[position][0]

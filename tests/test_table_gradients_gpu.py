@@ -134,3 +134,17 @@ def test_in_place_additions_are_counted(bmt_gpu):
     _loss(emb, ids, x).backward()
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         product.backward()
+
+
+def test_gradients_off_the_16_byte_boundary(bmt_gpu):
+    """A gradient that is a slice of a larger buffer, as programs that keep all gradients in one have it, is left to autograd."""
+    emb, p = _table(bmt_gpu)
+    ids, x = torch.randint(0, 300, (50,), device="cuda"), torch.randn(8, 64, device="cuda").half()
+    _loss(emb, ids, x).backward()
+    want = p.grad.clone()
+    for start in (1, 4, 7, 8):
+        buffer = torch.zeros(p.numel() + 32, device="cuda", dtype=p.dtype)
+        p.grad = buffer[start:start + p.numel()]
+        _loss(emb, ids, x).backward()
+        torch.cuda.synchronize()
+        assert torch.equal(p.grad, want) and not buffer[:start].any() and not buffer[start + p.numel():].any()
