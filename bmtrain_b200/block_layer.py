@@ -198,17 +198,18 @@ class _Bucket:
         return self._layout
 
     def points_local(self) -> bool:
-        """Whether every parameter is the view of the partition that ``local_views`` gives, whoever may have assigned to its ``data``."""
+        """Whether every parameter lies where ``local_views`` has it, whoever may have assigned to its ``data``."""
         self._refresh_views()
-        return [(p.data_ptr(), p.dtype) for p in self._params] == self._local_at
+        return list(map(torch.Tensor.data_ptr, self._params)) == self._local_at
 
     def _refresh_views(self) -> None:
-        data = self.storage.data
-        key = (data.data_ptr(), data.dtype, data.numel())
+        at = self.storage
+        key = (at.data_ptr(), at.dtype, at.numel())
         if self._views_of != key:
+            data = at.data
             # the views keep the memory they look at alive, so an equal address is the same memory
             self._local_views = [data[s.lo - self.begin:s.hi - self.begin] for s in self.slots]
-            self._local_at = [(view.data_ptr(), view.dtype) for view in self._local_views]
+            self._local_at = [view.data_ptr() for view in self._local_views]
             self._params = [s.param for s in self.slots]
             self._full_views = None
             if self.comm.size == 1:
