@@ -88,6 +88,7 @@ class LlamaBlock(DistributedModule):
     def _bmt_native_takes(self, hidden):
         """The parameters in the executor's order if it takes these arguments, else None."""
         if not (torch.is_tensor(hidden) and hidden.is_cuda and hidden.dim() == 3 and hidden.numel() > 0 and config["tp_size"] == 1
+                and hidden.is_contiguous()       # the result of the modules has the strides of what they are given
                 and hidden.dtype in (torch.float16, torch.bfloat16) and _FUSED_BLOCK and os.environ.get("BMT_FLASH_ATTN", "1") != "0"):
             return None
         m = self._modules

@@ -240,3 +240,19 @@ def test_executor_and_operators_at_a_size_that_is_divided(bmt_gpu, monkeypatch):
         operators = enc(x)
     # a chain of a dozen 16-bit intermediates
     assert (executor.double() - operators.double()).norm() <= 12 * _UNIT[dtype] * operators.double().norm()
+
+
+def test_strides_of_the_result(bmt_gpu, monkeypatch):
+    """A sequence-first hidden state seen as batch-first: the result lies in memory as that of the modules does."""
+    bmt = bmt_gpu
+    block = bmt.Block(_llama(bmt, torch.float16, 256, 4, 2, 64, 512))
+    bmt.init_parameters(block)
+    x = torch.randn(40, 3, 256, device="cuda").half().transpose(0, 1)
+    with torch.no_grad():
+        got, contiguous = block(x), block(x.contiguous())
+        assert block._native_module([x.contiguous()], True) is not None
+        monkeypatch.setattr(type(block), "_native_module", lambda *a, **k: None)
+        want = block(x)
+    assert got.stride() == want.stride() and contiguous.is_contiguous()
+    assert torch.equal(got, want) and torch.equal(contiguous, want)
+    got.transpose(0, 1).view(120, 256)
