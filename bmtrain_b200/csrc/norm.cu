@@ -156,7 +156,7 @@ template <typename T, int VPL, int WPR, bool RMS>
 __global__ void __launch_bounds__(FWD_WARPS(WPR) * 32) norm_fwd_row_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __restrict__ w,
                                                                            const T* __restrict__ b, float eps, T* __restrict__ y,
                                                                            float* __restrict__ stats) {
-    bmt::after_previous();
+    if (VPL > 1) bmt::after_previous();                // (see launch_fwd_row)
     constexpr int RPC = FWD_WARPS(WPR) / WPR;          // 1, or 4 teams without a barrier
     __shared__ float ex[2][FWD_WARPS(WPR)];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -232,12 +232,17 @@ __global__ void __launch_bounds__(FWD_WARPS(WPR) * 32) norm_fwd_row_kernel(int64
         }
 }
 
+// Rows of one vector a lane are launched normally: a block of four lives for less than a microsecond, and waiting for the kernel before it takes as
+// long (300000 x 256 RMSNorm 55 us so, 79 when launched early; 1000000 x 64 152 and 257; 100000 x 512, two vectors, 35 and 32).
 template <typename T, int VPL, int WPR>
 void launch_fwd_row(int64_t rows, int d, const void* x, const void* w, const void* b, float eps, int rms, void* y, void* stats, cudaStream_t s) {
     constexpr int RPC = FWD_WARPS(WPR) / WPR;
     const auto kernel = rms ? norm_fwd_row_kernel<T, VPL, WPR, true> : norm_fwd_row_kernel<T, VPL, WPR, false>;
-    bmt::launch(kernel, (unsigned)((rows + RPC - 1) / RPC), FWD_WARPS(WPR) * 32, 0, s, 1, rows, d, (const T*)x, (const T*)w, (const T*)b, eps, (T*)y,
-                (float*)stats);
+    const unsigned blocks = (unsigned)((rows + RPC - 1) / RPC);
+    if constexpr (VPL > 1)
+        bmt::launch(kernel, blocks, FWD_WARPS(WPR) * 32, 0, s, 1, rows, d, (const T*)x, (const T*)w, (const T*)b, eps, (T*)y, (float*)stats);
+    else
+        kernel<<<blocks, FWD_WARPS(WPR) * 32, 0, s>>>(rows, d, (const T*)x, (const T*)w, (const T*)b, eps, (T*)y, (float*)stats);
 }
 
 // vpl: vectors a lane has to hold; wide teams have at least 5
