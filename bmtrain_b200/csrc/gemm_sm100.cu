@@ -1410,15 +1410,19 @@ int g_reserved_sms = 0;
 // behind a long reduction and up to 10 where all SMs write and read their slots at once.  So the estimate has to win by 12 %
 // where there is less than a wave (1024 x 2560 x 8192 in the dgrad layout: 50 -> 43 us; 56 x 720 x 9144: 41 -> 19; 777 x 2560 x 7680,
 // estimated 11 % better, took 41 instead of 40) and by 2 % behind whole waves (4096 x 5120 x 27648: 807 -> 738 us;
-// 2048 x 57344 x 8192: 1256 -> 1208; 2560 x 8192 x 1024, not chosen, would take 44 instead of 38).
+// 2048 x 57344 x 8192: 1256 -> 1208; 2560 x 8192 x 1024, not chosen, would take 44 instead of 38).  A single row of tiles reads its large operand
+// once: where that lies along N, does not fit L2, and nearly all SMs have a whole wide tile of it, the memory is the bound and the tiles stay
+// whole (88 x 17944 x 24864 in the dgrad layout: 153 us, at 5.9 TB/s, against 176; 24 x 17752 x 16256: 91 and 118).  Not so in the other layout (80 x 16928
+// x 23016: 164 us divided, 212 whole) or with more rows (128 x 17456 x 16536: 123 and 146).
 struct TileChoice { int bn, cta2, sk_tiles, sk_workers; };
 constexpr int SK_MIN = 4, SK_MOST = 8;      // k-blocks of a range at least, CTAs per tile at most
 constexpr double SK_COST = 16000.0;
+constexpr double L2_BYTES = 126e6;
 
 // `sms`: that do math
 TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn, int force_bn, int force_cta2, bool split, int sms) {
     TileChoice best{0, 0, 0, 0}, best_split{0, 0, 0, 0};
-    double best_cost = 1e30, best_split_cost = 1e30;
+    double best_cost = 1e30, best_split_cost = 1e30, busy = 0.0;      // part of the SMs that `best` keeps busy, if it takes one wave
     const int64_t kblocks = (K + BK - 1) / BK;
     for (int cta2 = 0; cta2 <= 1; ++cta2) {
         if (force_cta2 >= 0 && cta2 != force_cta2) continue;
@@ -1433,7 +1437,7 @@ TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn
             const double mma = 2.05 * bn, load = 2.0 * (128 + bn / ncta);
             const double per_block = mma > load ? mma : load, fixed = 600.0 + 6.0 * bn;   // + fill/drain and epilogue
             const double cost = (double)waves * (kblocks * per_block + fixed);
-            if (cost < best_cost * 0.999) { best_cost = cost; best = TileChoice{bn, cta2, 0, 0}; }
+            if (cost < best_cost * 0.999) { best_cost = cost; best = TileChoice{bn, cta2, 0, 0}; busy = waves == 1 ? (double)tiles / slots : 0.0; }
             if (!split || tiles % slots == 0) continue;
             const bool behind = tiles > slots;              // behind whole waves
             const int64_t sk_tiles = tiles % slots + (behind ? slots : 0), total = sk_tiles * kblocks;
@@ -1449,6 +1453,8 @@ TileChoice pick_tile(int64_t M, int64_t N, int64_t K, int64_t batches, bool b_mn
             if (c < best_split_cost) { best_split_cost = c; best_split = TileChoice{bn, cta2, (int)sk_tiles, (int)workers}; }
         }
     }
+    const double bytes = 2.0 * batches * ((double)M * K + (double)N * K + (double)M * N);
+    if (b_mn && M <= 96 && best.bn >= 128 && busy >= 0.85 && bytes > L2_BYTES) return best;
     return best_split_cost < best_cost ? best_split : best;
 }
 
