@@ -160,8 +160,8 @@ void launch_rows(int64_t tokens, int64_t rows, int64_t d, const int64_t* ids, co
 
 }  // namespace
 
-// Rows of one vector a thread are launched normally: such a block lives for less than a microsecond, and waiting for the kernel before it takes as
-// long (65536 tokens, rows of 1024 16-bit values: 49 us so, 68 when launched early; of 5120: 195 and 192).
+// Many rows of one vector a thread are launched normally: such a block lives for less than a microsecond, and waiting for the kernel before it takes
+// as long (65536 tokens, rows of 1024 16-bit values: 49 us so, 68 when launched early; 8192 of 256: 8.3 and 9.2, 4096 alike; 65536 of 5120: 195 and 192).
 extern "C" int bmt_embedding_fwd(int64_t tokens, int64_t d, const void* ids, const void* weight, int dtype, void* out, void* stream) {
     if (tokens <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
@@ -169,7 +169,7 @@ extern "C" int bmt_embedding_fwd(int64_t tokens, int64_t d, const void* ids, con
         using T = std::remove_pointer_t<decltype(zero)>;
         constexpr int V = bmt::Vec16<T>::N;
         if (d % V) return -3;
-        if (d <= 128 * V) emb_fwd_kernel<T, false><<<(unsigned)tokens, 128, 0, s>>>(d, (const int64_t*)ids, (const T*)weight, (T*)out);
+        if (d <= 128 * V && tokens > 4096) emb_fwd_kernel<T, false><<<(unsigned)tokens, 128, 0, s>>>(d, (const int64_t*)ids, (const T*)weight, (T*)out);
         else bmt::launch(emb_fwd_kernel<T, true>, (unsigned)tokens, 128, 0, s, 1, d, (const int64_t*)ids, (const T*)weight, (T*)out);
         return 0;
     };

@@ -152,11 +152,11 @@ __global__ void __launch_bounds__(1024) norm_fold_kernel(int d, int nblk, const 
 // arithmetic (which left an SM 16 warps, and issued 19 instructions for an element).  16384 x 5120 bf16, RMSNorm: 66 us with the
 // resident grid, now 51 (6.6 TB/s); LayerNorm 85, now 54; 1024 x 2560 6.4, now 3.8.
 constexpr int FWD_WARPS(int wpr) { return wpr == 1 ? 4 : wpr; }
-template <typename T, int VPL, int WPR, bool RMS>
+template <typename T, int VPL, int WPR, bool RMS, bool EARLY>
 __global__ void __launch_bounds__(FWD_WARPS(WPR) * 32) norm_fwd_row_kernel(int64_t rows, int d, const T* __restrict__ x, const T* __restrict__ w,
                                                                            const T* __restrict__ b, float eps, T* __restrict__ y,
                                                                            float* __restrict__ stats) {
-    if (VPL > 1) bmt::after_previous();                // (see launch_fwd_row)
+    if (EARLY) bmt::after_previous();
     constexpr int RPC = FWD_WARPS(WPR) / WPR;          // 1, or 4 teams without a barrier
     __shared__ float ex[2][FWD_WARPS(WPR)];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -232,17 +232,19 @@ __global__ void __launch_bounds__(FWD_WARPS(WPR) * 32) norm_fwd_row_kernel(int64
         }
 }
 
-// Rows of one vector a lane are launched normally: a block of four lives for less than a microsecond, and waiting for the kernel before it takes as
-// long (300000 x 256 RMSNorm 55 us so, 79 when launched early; 1000000 x 64 152 and 257; 100000 x 512, two vectors, 35 and 32).
+// Many rows of one vector a lane are launched normally: a block of four lives for less than a microsecond, and waiting for the kernel before it takes
+// as long (300000 x 256 RMSNorm 55 us so, 79 when launched early; 100000 x 64 18 and 27, 30000 x 128 alike; 100000 x 512, two vectors, 35 and 32).
 template <typename T, int VPL, int WPR>
 void launch_fwd_row(int64_t rows, int d, const void* x, const void* w, const void* b, float eps, int rms, void* y, void* stats, cudaStream_t s) {
     constexpr int RPC = FWD_WARPS(WPR) / WPR;
-    const auto kernel = rms ? norm_fwd_row_kernel<T, VPL, WPR, true> : norm_fwd_row_kernel<T, VPL, WPR, false>;
     const unsigned blocks = (unsigned)((rows + RPC - 1) / RPC);
-    if constexpr (VPL > 1)
+    if (VPL > 1 || blocks <= 8192) {
+        const auto kernel = rms ? norm_fwd_row_kernel<T, VPL, WPR, true, true> : norm_fwd_row_kernel<T, VPL, WPR, false, true>;
         bmt::launch(kernel, blocks, FWD_WARPS(WPR) * 32, 0, s, 1, rows, d, (const T*)x, (const T*)w, (const T*)b, eps, (T*)y, (float*)stats);
-    else
+    } else if constexpr (VPL == 1) {
+        const auto kernel = rms ? norm_fwd_row_kernel<T, VPL, WPR, true, false> : norm_fwd_row_kernel<T, VPL, WPR, false, false>;
         kernel<<<blocks, FWD_WARPS(WPR) * 32, 0, s>>>(rows, d, (const T*)x, (const T*)w, (const T*)b, eps, (T*)y, (float*)stats);
+    }
 }
 
 // vpl: vectors a lane has to hold; wide teams have at least 5
